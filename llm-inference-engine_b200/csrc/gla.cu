@@ -73,7 +73,7 @@ template <typename T>
 __global__ void __launch_bounds__(kGlaThreads)
 gla_recurrent_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ decay, float *__restrict__ state, float *__restrict__ o,
                      const int *__restrict__ seq_start, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int heads,
-                     int dim, int vdim, int min_tokens) {
+                     int dim, int vdim, int min_tokens, int max_tokens) {
     extern __shared__ float sm[];
     float *S = sm;
     float *qs = S + (size_t)dim * kGlaCols;
@@ -85,7 +85,7 @@ gla_recurrent_kernel(const T *__restrict__ proj, int ld, const float *__restrict
     const int col = threadIdx.x % kGlaCols, rg = threadIdx.x / kGlaCols;
     constexpr int kRowGroups = kGlaThreads / kGlaCols;
     const int t0 = seq_start[s], t1 = seq_start[s + 1];
-    if (t1 - t0 < min_tokens) return;
+    if (t1 - t0 < min_tokens || t1 - t0 > max_tokens) return;
     const bool live = j0 + col < vdim;
     float *slot = state + (((size_t)seq_slot[s] * heads + h) * dim) * vdim;
     const bool fresh = seq_pos0[s] == 0;
@@ -133,7 +133,7 @@ template <typename T, int RR, int TB>
 __global__ void __launch_bounds__(256)
 gla_recurrent_reg_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ decay, float *__restrict__ state, float *__restrict__ o,
                          const int *__restrict__ seq_start, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int heads,
-                         int dim, int vdim, int min_tokens) {
+                         int dim, int vdim, int min_tokens, int max_tokens) {
     extern __shared__ __align__(16) float smf[];
     constexpr int DP = 32 * RR;                                  // padded rows
     constexpr int kStage = TB * DP * 4 + TB * kGlaCols;          // floats per stage: {a, k, q, -} [TB][DP] | v [TB][32]
@@ -144,7 +144,7 @@ gla_recurrent_reg_kernel(const T *__restrict__ proj, int ld, const float *__rest
     const bool producer = warp >= 4;                             // warps 4..7 stage the next block of tokens while warps 0..3 compute
     const int c0 = j0 + (warp & 3) * kGlaWarpCols;
     const int t0 = seq_start[s], t1 = seq_start[s + 1];
-    if (t1 - t0 < min_tokens) return;
+    if (t1 - t0 < min_tokens || t1 - t0 > max_tokens) return;
     float *slot = state + (((size_t)seq_slot[s] * heads + h) * dim) * vdim;
     const bool fresh = seq_pos0[s] == 0;
     const float qscale = rsqrtf((float)dim);
@@ -361,10 +361,10 @@ gla_step_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ de
 
 template <typename T, int RR, int TB>
 static void launch_gla_reg(const void *proj, int ld, const float *decay, float *state, float *o, const int *seq_start, const int *seq_pos0,
-                           const int *seq_slot, dim3 grid, int heads, int dim, int vdim, int min_tokens, cudaStream_t st) {
+                           const int *seq_slot, dim3 grid, int heads, int dim, int vdim, int min_tokens, int max_tokens, cudaStream_t st) {
     const size_t smem = 2 * ((size_t)TB * 32 * RR * 4 + (size_t)TB * kGlaCols) * sizeof(float);
     if (smem > 48 * 1024) cudaFuncSetAttribute(gla_recurrent_reg_kernel<T, RR, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    gla_recurrent_reg_kernel<T, RR, TB><<<grid, 256, smem, st>>>((const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim, min_tokens);
+    gla_recurrent_reg_kernel<T, RR, TB><<<grid, 256, smem, st>>>((const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim, min_tokens, max_tokens);
 }
 
 template <typename T>
@@ -428,7 +428,7 @@ int launch_gla_decay(int dtype, const void *proj, int ld, int col0, const void *
 }
 
 int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay, float *state, float *o, const int *seq_start,
-                         const int *seq_pos0, const int *seq_slot, int n_seqs, int heads, int dim, int vdim, cudaStream_t st, int kinds) {
+                         const int *seq_pos0, const int *seq_slot, int n_seqs, int heads, int dim, int vdim, cudaStream_t st, int kinds, int max_tokens) {
     if (n_seqs == 0) return B200_OK;
     // one-token portions take the step kernel (16-byte pieces of state rows: vdim a multiple of 4); the token-loop kernels then skip them
     const bool step = (kinds & kGlaOneToken) && vdim % 4 == 0 && (reinterpret_cast<size_t>(state) & 15) == 0 &&
@@ -451,17 +451,17 @@ int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay
     const dim3 grid((vdim + kGlaCols - 1) / kGlaCols, heads, n_seqs);
     if (dim <= 256) {
         B200_DISPATCH_DTYPE(dtype, {
-            if (dim <= 32) launch_gla_reg<T, 1, 16>(proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, grid, heads, dim, vdim, min_tokens, st);
-            else if (dim <= 64) launch_gla_reg<T, 2, 16>(proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, grid, heads, dim, vdim, min_tokens, st);
-            else if (dim <= 128) launch_gla_reg<T, 4, 16>(proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, grid, heads, dim, vdim, min_tokens, st);
-            else launch_gla_reg<T, 8, 8>(proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, grid, heads, dim, vdim, min_tokens, st);
+            if (dim <= 32) launch_gla_reg<T, 1, 16>(proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, grid, heads, dim, vdim, min_tokens, max_tokens, st);
+            else if (dim <= 64) launch_gla_reg<T, 2, 16>(proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, grid, heads, dim, vdim, min_tokens, max_tokens, st);
+            else if (dim <= 128) launch_gla_reg<T, 4, 16>(proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, grid, heads, dim, vdim, min_tokens, max_tokens, st);
+            else launch_gla_reg<T, 8, 8>(proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, grid, heads, dim, vdim, min_tokens, max_tokens, st);
         });
         return cuda_status("gla_recurrent launch");
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(gla_recurrent_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         gla_recurrent_kernel<T><<<grid, kGlaThreads, smem, st>>>((const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim,
-                                                                  vdim, min_tokens);
+                                                                  vdim, min_tokens, max_tokens);
     });
     return cuda_status("gla_recurrent launch");
 }

@@ -713,7 +713,8 @@ struct b200_hybrid {
     void *cat = nullptr, *xc = nullptr, *vkeep = nullptr;
     double *turns = nullptr;                    // the sinusoidal position vector's frequencies, formed by the first call after set_scratch
     bool turns_ready = false;
-    float *maps = nullptr;
+    float *maps = nullptr, *chunk = nullptr;
+    size_t chunk_floats = 0;
     int *meta = nullptr, *moe_i = nullptr;
     float *moe_f = nullptr;
     std::vector<int> host_meta;
@@ -722,7 +723,7 @@ struct b200_hybrid {
 namespace {
 
 struct Carve {
-    size_t x, f32a, f32b, xn, h, proj, mix, y, xg, u, yrows, us, ys, lqn, lqr, lql, lov, lpart, meta, moe_i, moe_f, rec, f32c, cat, xc, xs, turns, maps, vkeep, total;
+    size_t x, f32a, f32b, xn, h, proj, mix, y, xg, u, yrows, us, ys, lqn, lqr, lql, lov, lpart, meta, moe_i, moe_f, rec, f32c, cat, xc, xs, turns, maps, vkeep, chunk, total;
 };
 
 // rows of the input projection and columns of the output projection that ONE mixer owns
@@ -774,13 +775,16 @@ Carve carve(const b200_hybrid *m) {
     const b200_hybrid_config_t &c = m->cfg;
     const size_t T = (size_t)c.max_tokens, es = c.dtype == B200_F32 ? 4 : 2;
     size_t n_in = 1, n_mix = 1, n_f32 = 1, rows = 0, ff = 1, sff = 1, experts = 1, top = 1, lqn = 0, lqr = 0, lql = 0, lov = 0, lheads = 0, lpart = 0;
-    size_t n_rec = 0, n_heads = 0, n_cat = 0, n_gru = 0, n_vkeep = 0;
+    size_t n_rec = 0, n_heads = 0, n_cat = 0, n_gru = 0, n_vkeep = 0, n_chunk = 0;
     bool pre_norm = false;
     const size_t t_pad = (T + 127) / 128 * 128;  // rows per head of the latent mixer's grouped GEMMs
     for (int i = 0; i < c.num_layers; ++i) {
         if (!m->layer_set[i]) continue;
         const b200_hybrid_layer_t &l = m->layers[i];
         n_in = std::max(n_in, (size_t)n_in_of(l));
+        for (const b200_hybrid_layer_t *mx : {&l, l.side})
+            if (mx && (mx->mixer == B200_MIXER_GLA || mx->mixer == B200_MIXER_DELTA || mx->mixer == B200_MIXER_SSD || mx->mixer == B200_MIXER_LINEAR))
+                n_chunk = std::max(n_chunk, chunk_scratch_floats(mx->heads, mx->dim, c.max_tokens, c.max_seqs));
         n_mix = std::max(n_mix, (size_t)l.heads * std::max(l.dim, l.vdim));
         n_f32 = std::max(n_f32, (size_t)l.heads * std::max(l.dim, l.vdim));
         n_mix = std::max(n_mix, (size_t)l.heads * l.vdim);
@@ -849,7 +853,8 @@ Carve carve(const b200_hybrid *m) {
     k.turns = c.pos_base > 0.0f ? align256((size_t)(c.width + 1) / 2 * 8) : 0;
     k.maps = align256((T / kMingruChunk + (size_t)c.max_seqs) * kMingruMapRows * n_gru * 4);
     k.vkeep = align256(T * n_vkeep * es);
-    k.total = k.vkeep + k.maps + k.turns + k.xs + k.x + k.f32a + k.f32b + k.xn + k.h + k.proj + 2 * k.mix + k.y + k.xg + k.u + k.yrows + k.us + k.ys + k.lqn + k.lqr + 2 * k.lql +
+    k.chunk = align256(n_chunk * 4);
+    k.total = k.chunk + k.vkeep + k.maps + k.turns + k.xs + k.x + k.f32a + k.f32b + k.xn + k.h + k.proj + 2 * k.mix + k.y + k.xg + k.u + k.yrows + k.us + k.ys + k.lqn + k.lqr + 2 * k.lql +
               k.lov + k.lpart + k.meta + k.moe_i + k.moe_f + k.rec + k.f32c + k.cat + k.xc;
     return k;
 }
@@ -1084,6 +1089,7 @@ int b200_hybrid_set_scratch(b200_hybrid_t *m, void *ptr, size_t bytes) {
     m->turns = (double *)p, p += k.turns, m->turns_ready = false;
     m->maps = (float *)p, p += k.maps;
     m->vkeep = p, p += k.vkeep;
+    m->chunk = (float *)p, m->chunk_floats = k.chunk / 4, p += k.chunk;
     return B200_OK;
 }
 
@@ -1226,10 +1232,12 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     int n_tiles = 0, n_short = 0, n_chunks = 0, gla_kinds = 0;
     // minGRU chunks: at most 64 per portion (a chunk composes the maps of all chunks before it), of whole multiples of kMingruChunk tokens
     int longest = 0;
+    bool mid_portions = false;  // portions of several tokens that the token-parallel recurrences leave to the serial ones
     for (int s = 0; s < S; ++s) longest = std::max(longest, b->seq_start[s + 1] - b->seq_start[s]);
     const int chunk_tokens = std::max(1, (longest + 64 * kMingruChunk - 1) / (64 * kMingruChunk)) * kMingruChunk;
     for (int s = 0; s < S; ++s) {
         const int t0 = b->seq_start[s], t1 = b->seq_start[s + 1];
+        mid_portions |= t1 - t0 > 1 && t1 - t0 < kChunkMinTokens;
         gla_kinds |= t1 - t0 == 1 ? kGlaOneToken : (t1 - t0 > 1 ? kGlaManyTokens : 0);
         B200_REQUIRE(t1 >= t0 && b->seq_pos0[s] >= 0, "hybrid_forward: bad portion of sequence %d", s);
         B200_REQUIRE(b->seq_slot[s] >= 0 && b->seq_slot[s] < m->num_slots, "hybrid_forward: state slot %d outside [0, %d)", b->seq_slot[s], m->num_slots);
@@ -1331,6 +1339,25 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                                                                       c.embed_scale != 0.0f ? c.embed_scale : 1.0f); });
     }
 
+    // a recurrence over the batch: its token-parallel form for the long portions, where it takes the layer's sizes, and the serial form for the rest
+    auto recurrence = [&](auto chunked, auto serial) -> int {
+        int kinds = gla_kinds, max_tokens = kAnyTokens;
+        if (longest >= kChunkMinTokens) {
+            rc = chunked();
+            if (rc != B200_OK && rc != B200_ERR_UNSUPPORTED) return rc;
+            if (rc == B200_OK) {
+                max_tokens = kChunkMinTokens - 1;
+                if (!mid_portions) kinds &= ~kGlaManyTokens;
+            }
+        }
+        return kinds ? serial(kinds, max_tokens) : B200_OK;
+    };
+    auto decay_recurrence = [&](const b200_hybrid_layer_t &l, const MixerPlan &mp, int key_heads) -> int {
+        float *state = (float *)(m->state_pool + mp.state_off);
+        return recurrence([&] { return launch_chunk_decay(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, key_heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
+                          [&](int, int most) { return launch_decay_recurrent(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, key_heads, l.dim, l.vdim, st, gla_kinds == kGlaOneToken, most); });
+    };
+
     // one mixer of a shared-norm or pre-norm layer: reads its rows of the projection from column `col`, writes its heads into rows of `out`
     // (row stride out_ld: several mixers may fill one row of a shared output projection's input), scaled
     auto run_mixer = [&](const b200_hybrid_layer_t &l, const MixerPlan &mp, int n_in, int col, void *out_buf, int out_ld, float out_scale) -> int {
@@ -1371,8 +1398,9 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                 RUN(launch_delta_prep_direct(dt, m->proj, n_in, col, l.conv_w, l.conv, conv_state, l.decay_bias, l.a_log, m->rec, d_seq, d_pos, d_pos0, d_slot,
                                              NT, l.heads, l.kv_heads, l.dim, l.vdim, st));
             RUN(launch_conv_state_update(dt, m->proj, n_in, col, conv_state, l.conv, conv_channels(l), d_start, d_pos0, d_slot, S, st));
-            RUN(launch_delta_recurrent(m->rec, (float *)(m->state_pool + mp.state_off), m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.kv_heads, l.dim,
-                                       l.vdim, st, one_token));
+            float *state = (float *)(m->state_pool + mp.state_off);
+            RUN(recurrence([&] { return launch_chunk_delta(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.kv_heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
+                           [&](int, int most) { return launch_delta_recurrent(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.kv_heads, l.dim, l.vdim, st, one_token, most); }));
             if (l.decay_rank > 0) {
                 RUN(launch_head_output(dt, m->f32b, nullptr, nullptr, l.out_norm, 0, c.norm_eps, m->rec + lay.gate, lay.ld, nullptr, 0, out, out_ld, out_scale,
                                        NT, l.heads, l.vdim, st, l.gate_act));
@@ -1389,15 +1417,13 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             RUN(launch_ssd_prep(dt, m->proj, n_in, col, l.conv_w, l.conv_b, l.conv, conv_state, l.decay_bias, l.a_log, l.skip, m->rec, d_seq, d_pos, d_pos0,
                                 d_slot, NT, l.heads, l.kv_heads, l.dim, l.vdim, st));
             RUN(launch_conv_state_update(dt, m->proj, n_in, col + inner, conv_state, l.conv, conv_channels(l), d_start, d_pos0, d_slot, S, st));
-            RUN(launch_decay_recurrent(m->rec, (float *)(m->state_pool + mp.state_off), m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.kv_heads, l.dim,
-                                       l.vdim, st, one_token));
+            RUN(decay_recurrence(l, mp, l.kv_heads));
             RUN(launch_group_output(dt, m->f32b, m->rec + lay.skip, lay.ld, l.out_norm, c.norm_eps, (const char *)m->proj + (size_t)col * es, n_in, 1, 1, out,
                                     out_ld, NT, inner, l.norm_groups, st));
         } else if (l.mixer == B200_MIXER_LINEAR) {
             const int inner = l.heads * l.vdim;
             RUN(launch_linear_prep(dt, m->proj, n_in, col, l.head_decay, m->rec, NT, l.heads, l.dim, l.vdim, st));
-            RUN(launch_decay_recurrent(m->rec, (float *)(m->state_pool + mp.state_off), m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.heads, l.dim, l.vdim,
-                                       st, one_token));
+            RUN(decay_recurrence(l, mp, l.heads));
             RUN(launch_group_output(dt, m->f32b, nullptr, 0, l.out_norm, c.norm_eps, (const char *)m->proj + (size_t)(col + 2 * l.heads * l.dim + inner) * es,
                                     n_in, 0, 0, out, out_ld, NT, inner, 1, st));
         } else {
@@ -1652,8 +1678,9 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             const int hd = l.heads * l.dim, hv = l.heads * l.vdim;
             const char *gate = (const char *)m->proj + (size_t)(2 * hd + hv) * es;
             RUN(launch_gla_decay(dt, m->proj, lp.n_in, 2 * hd + 2 * hv, l.w_decay, l.decay_bias, l.tau, m->f32a, NT, l.decay_rank, hd, st));
-            RUN(launch_gla_recurrent(dt, m->proj, lp.n_in, m->f32a, (float *)(m->state_pool + lp.state_off), m->f32b, d_start, d_pos0, d_slot, S,
-                                     l.heads, l.dim, l.vdim, st, gla_kinds));
+            float *state = (float *)(m->state_pool + lp.state_off);
+            RUN(recurrence([&] { return launch_chunk_gla(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
+                           [&](int kinds, int most) { return launch_gla_recurrent(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, st, kinds, most); }));
             RUN(launch_gla_output(dt, m->f32b, l.out_norm, c.norm_eps, gate, lp.n_in, m->mix2, NT, l.heads, l.vdim, st));
             n_mixed = hv;
         }

@@ -69,6 +69,8 @@ int launch_scored_attention_tiles(int dtype, const void *q, const void *k_pool, 
                                   const int *tiles, int n_tiles, const int *block_table, int mpps, int heads, int kv_heads, int dim, int vdim,
                                   float scale, int window, int sigmoid, cudaStream_t st, ScoredOptions opt = ScoredOptions());
 
+constexpr int kAnyTokens = 0x7fffffff;  // max_tokens of the serial recurrences: portions with more tokens than this are left to chunk_recurrence.cu
+
 // recurrent.cu: column offsets of the fp32 row per token that the prep kernels write and the recurrences read.
 // launch_delta_prep scratch: lr (engine dtype) of tokens * (rank + gate_rank) elements + 256 bytes, za fp32 [tokens, heads*dim], zg fp32
 // [tokens, heads*vdim]
@@ -86,7 +88,7 @@ int launch_conv_state_update(int dtype, const void *proj, int ld, int col0, floa
                              const int *seq_pos0, const int *seq_slot, int n_seqs, cudaStream_t st);
 // one_token: the host knows that every portion of the batch is a single token (a decode batch)
 int launch_delta_recurrent(const float *rec, float *S, float *o, const int *seq_start, const int *seq_pos0, const int *seq_slot, int n_seqs,
-                           int heads, int kv_heads, int dim, int vdim, cudaStream_t st, int one_token = 0);
+                           int heads, int kv_heads, int dim, int vdim, cudaStream_t st, int one_token = 0, int max_tokens = kAnyTokens);
 int launch_mlstm_prep(int dtype, const void *proj, int ld, int col0, const float *b_in, float cap, float *rec, int tokens, int heads, int dim,
                       int vdim, cudaStream_t st);
 int launch_mlstm_recurrent(const float *rec, float *S, float *n_state, float *m_state, float *o, float *nq, float *m_out, const int *seq_start,
@@ -109,7 +111,7 @@ int launch_linear_prep(int dtype, const void *proj, int ld, int col0, const floa
                        cudaStream_t st);
 // S <- decay S + k v^T;  o = S^T q over every sequence's portion, from the tokens' DecayRow
 int launch_decay_recurrent(const float *rec, float *S, float *o, const int *seq_start, const int *seq_pos0, const int *seq_slot, int n_seqs,
-                           int heads, int kv_heads, int dim, int vdim, cudaStream_t st, int one_token = 0);
+                           int heads, int kv_heads, int dim, int vdim, cudaStream_t st, int one_token = 0, int max_tokens = kAnyTokens);
 // out[t, c] = T((o + skip)[t, c] (* act(gate) if gate_first) * rsqrt(mean over the column's group + eps) * w[c] (* act(gate) if not)),
 // `groups` equal groups of the `cols` columns; act = sigmoid (gate_act 0) or silu (1); skip may be NULL
 int launch_group_output(int dtype, const float *o, const float *skip, int skip_ld, const float *w, float eps, const void *gate, int gate_ld,
@@ -146,10 +148,23 @@ int launch_gla_decay(int dtype, const void *proj, int ld, int col0, const void *
 constexpr int kGlaOneToken = 1, kGlaManyTokens = 2;
 int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay, float *state, float *o, const int *seq_start,
                          const int *seq_pos0, const int *seq_slot, int n_seqs, int heads, int dim, int vdim, cudaStream_t st,
-                         int kinds = kGlaOneToken | kGlaManyTokens);
+                         int kinds = kGlaOneToken | kGlaManyTokens, int max_tokens = kAnyTokens);
 // out[t, h*vdim + j] = o[t,h,j] * rsqrt(mean_j o^2 + eps) * w[j] * silu(gate[t*gate_ld + h*vdim + j])
 int launch_gla_output(int dtype, const float *o, const float *w, float eps, const void *gate_in, int gate_ld, void *out, int tokens,
                       int heads, int vdim, cudaStream_t st);
+
+// chunk_recurrence.cu: the token-parallel form of the recurrences for portions of at least kChunkMinTokens tokens (shorter ones are skipped: the
+// serial kernels serve them with max_tokens = kChunkMinTokens - 1).  B200_ERR_UNSUPPORTED, nothing launched: sizes or alignments it does not take.
+// scratch: fp32, chunk_scratch_floats of the engine's limits (0: sizes it never takes); tokens / longest: of this call and of its longest portion
+constexpr int kChunkMinTokens = 64;
+size_t chunk_scratch_floats(int heads, int dim, int max_tokens, int max_seqs);
+int launch_chunk_gla(int dtype, const void *proj, int ld, const float *decay, float *state, float *o, const int *seq_start, const int *seq_pos0,
+                     const int *seq_slot, int n_seqs, int heads, int dim, int vdim, float *scratch, size_t scratch_floats, int tokens, int longest,
+                     cudaStream_t st);
+int launch_chunk_delta(const float *rec, float *state, float *o, const int *seq_start, const int *seq_pos0, const int *seq_slot, int n_seqs, int heads,
+                       int kv_heads, int dim, int vdim, float *scratch, size_t scratch_floats, int tokens, int longest, cudaStream_t st);
+int launch_chunk_decay(const float *rec, float *state, float *o, const int *seq_start, const int *seq_pos0, const int *seq_slot, int n_seqs, int heads,
+                       int kv_heads, int dim, int vdim, float *scratch, size_t scratch_floats, int tokens, int longest, cudaStream_t st);
 
 // moe.cu
 int launch_moe_route_sigmoid(const float *logits, int ld, int *sel_expert, float *sel_weight, float *shared_gate, int tokens,

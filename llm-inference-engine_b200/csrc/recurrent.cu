@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(256)
 column_recurrence_kernel(const float *__restrict__ rec, int rec_ld, int q_off, int k_off, int v_off, int a_off, int b_off,
                          float *__restrict__ S, float *__restrict__ n_state, float *__restrict__ m_state, float *__restrict__ o,
                          float *__restrict__ nq_out, float *__restrict__ m_out, const int *__restrict__ seq_start,
-                         const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int heads, int kv_heads, int dim, int vdim) {
+                         const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int heads, int kv_heads, int dim, int vdim, int max_tokens) {
     constexpr int RPT = DP / LANES, NV = MODE == 0 ? 3 : 2, TS = NV * DP + 4;
     static_assert(RPT >= 4 && RPT % 4 == 0 && RPT * CPT <= 128, "state tile per thread");
     extern __shared__ __align__(16) float stage[];  // [2][kRecTB][TS] | v [2][kRecTB][CB]
@@ -389,7 +389,7 @@ column_recurrence_kernel(const float *__restrict__ rec, int rec_ld, int q_off, i
     float *vs = stage + 2 * kRecTB * TS;
     const int s = blockIdx.z, h = blockIdx.y, g = h / (heads / kv_heads);
     const int t0 = seq_start[s], len = seq_start[s + 1] - t0;
-    if (len <= 0) return;
+    if (len <= 0 || len > max_tokens) return;
     const int pos0 = seq_pos0[s], slot = seq_slot[s];
     const int ncols = MODE == 1 ? vdim + 1 : vdim;
     const int cl = threadIdx.x / LANES * CPT, sub = threadIdx.x % LANES;  // first column within the CTA, lane within the column group
@@ -639,7 +639,7 @@ head_output_kernel(const float *__restrict__ o, const float *__restrict__ nq, co
 template <int DP, int LANES, int CPT, int MODE>
 static int launch_colrec_t(const float *rec, int rec_ld, int q_off, int k_off, int v_off, int a_off, int b_off, float *S, float *n_state,
                            float *m_state, float *o, float *nq, float *m_out, const int *seq_start, const int *seq_pos0, const int *seq_slot,
-                           int n_seqs, int heads, int kv_heads, int dim, int vdim, int one_token, cudaStream_t st) {
+                           int n_seqs, int heads, int kv_heads, int dim, int vdim, int one_token, int max_tokens, cudaStream_t st) {
     const int ncols = MODE == 1 ? vdim + 1 : vdim, groups = (ncols + CPT - 1) / CPT;
     // every CTA stages its head's key-side vectors for itself, so CTAs are as wide as the batch allows while about a hundred of them remain
     const long long threads = (long long)groups * LANES * heads * n_seqs;
@@ -655,7 +655,7 @@ static int launch_colrec_t(const float *rec, int rec_ld, int q_off, int k_off, i
     auto kern = column_recurrence_kernel<DP, LANES, CPT, MODE>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kern<<<dim3((ncols + cb - 1) / cb, heads, n_seqs), block, smem, st>>>(rec, rec_ld, q_off, k_off, v_off, a_off, b_off, S, n_state, m_state, o, nq, m_out,
-                                                                        seq_start, seq_pos0, seq_slot, heads, kv_heads, dim, vdim);
+                                                                        seq_start, seq_pos0, seq_slot, heads, kv_heads, dim, vdim, max_tokens);
     return cuda_status("column_recurrence launch");
 }
 
@@ -674,7 +674,7 @@ static int pick_lanes(int dp, int max_rows, long long groups) {
 template <int MODE>
 static int launch_colrec(const float *rec, int rec_ld, int q_off, int k_off, int v_off, int a_off, int b_off, float *S, float *n_state,
                          float *m_state, float *o, float *nq, float *m_out, const int *seq_start, const int *seq_pos0, const int *seq_slot,
-                         int n_seqs, int heads, int kv_heads, int dim, int vdim, int one_token, cudaStream_t st) {
+                         int n_seqs, int heads, int kv_heads, int dim, int vdim, int one_token, int max_tokens, cudaStream_t st) {
     if (n_seqs == 0) return B200_OK;
     if (dim > 512) {
         set_error("column recurrence: key size %d above 512", dim);
@@ -688,7 +688,7 @@ static int launch_colrec(const float *rec, int rec_ld, int q_off, int k_off, int
     const int lanes = pick_lanes(dp, 64, (long long)n_seqs * heads * ncols);
 #define B200_COLREC(D, L, C)  \
     if (dp == D && lanes == L && cpt == C) \
-        return launch_colrec_t<D, L, C, MODE>(rec, rec_ld, q_off, k_off, v_off, a_off, b_off, S, n_state, m_state, o, nq, m_out, seq_start, seq_pos0, seq_slot, n_seqs, heads, kv_heads, dim, vdim, one_token, st)
+        return launch_colrec_t<D, L, C, MODE>(rec, rec_ld, q_off, k_off, v_off, a_off, b_off, S, n_state, m_state, o, nq, m_out, seq_start, seq_pos0, seq_slot, n_seqs, heads, kv_heads, dim, vdim, one_token, max_tokens, st)
     B200_COLREC(16, 1, 1); B200_COLREC(16, 2, 1); B200_COLREC(16, 4, 1);
     B200_COLREC(32, 1, 1); B200_COLREC(32, 2, 1); B200_COLREC(32, 4, 1); B200_COLREC(32, 8, 1);
     B200_COLREC(64, 1, 1); B200_COLREC(64, 2, 1); B200_COLREC(64, 4, 1); B200_COLREC(64, 8, 1); B200_COLREC(64, 16, 1);
@@ -740,10 +740,10 @@ int launch_conv_state_update(int dtype, const void *proj, int ld, int col0, floa
 }
 
 int launch_delta_recurrent(const float *rec, float *S, float *o, const int *seq_start, const int *seq_pos0, const int *seq_slot, int n_seqs,
-                           int heads, int kv_heads, int dim, int vdim, cudaStream_t st, int one_token) {
+                           int heads, int kv_heads, int dim, int vdim, cudaStream_t st, int one_token, int max_tokens) {
     const DeltaRow lay = delta_row(heads, kv_heads, dim, vdim);
     return launch_colrec<0>(rec, lay.ld, lay.q, lay.k, lay.v, lay.decay, lay.beta, S, nullptr, nullptr, o, nullptr, nullptr, seq_start, seq_pos0,
-                            seq_slot, n_seqs, heads, kv_heads, dim, vdim, one_token, st);
+                            seq_slot, n_seqs, heads, kv_heads, dim, vdim, one_token, max_tokens, st);
 }
 
 int launch_mlstm_prep(int dtype, const void *proj, int ld, int col0, const float *b_in, float cap, float *rec, int tokens, int heads, int dim,
@@ -758,7 +758,7 @@ int launch_mlstm_recurrent(const float *rec, float *S, float *n_state, float *m_
                            const int *seq_pos0, const int *seq_slot, int n_seqs, int heads, int dim, int vdim, cudaStream_t st, int one_token) {
     const MlstmRow lay = mlstm_row(heads, dim, vdim);
     return launch_colrec<1>(rec, lay.ld, lay.q, lay.k, lay.v, lay.gi, lay.gf, S, n_state, m_state, o, nq, m_out, seq_start, seq_pos0, seq_slot,
-                            n_seqs, heads, heads, dim, vdim, one_token, st);
+                            n_seqs, heads, heads, dim, vdim, one_token, kAnyTokens, st);
 }
 
 int launch_head_output(int dtype, const float *o, const float *nq, const float *m_in, const float *w, int w_stride, float eps,
@@ -809,10 +809,10 @@ int launch_linear_prep(int dtype, const void *proj, int ld, int col0, const floa
 }
 
 int launch_decay_recurrent(const float *rec, float *S, float *o, const int *seq_start, const int *seq_pos0, const int *seq_slot, int n_seqs,
-                           int heads, int kv_heads, int dim, int vdim, cudaStream_t st, int one_token) {
+                           int heads, int kv_heads, int dim, int vdim, cudaStream_t st, int one_token, int max_tokens) {
     const DecayRow lay = decay_row(heads, kv_heads, dim, vdim);
     return launch_colrec<2>(rec, lay.ld, lay.q, lay.k, lay.v, lay.decay, lay.decay, S, nullptr, nullptr, o, nullptr, nullptr, seq_start, seq_pos0,
-                            seq_slot, n_seqs, heads, kv_heads, dim, vdim, one_token, st);
+                            seq_slot, n_seqs, heads, kv_heads, dim, vdim, one_token, max_tokens, st);
 }
 
 int launch_group_output(int dtype, const float *o, const float *skip, int skip_ld, const float *w, float eps, const void *gate, int gate_ld,
