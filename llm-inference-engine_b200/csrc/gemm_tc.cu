@@ -17,6 +17,7 @@
 #include "gemm_tc.cuh"
 
 #include <cuda.h>  // CUtensorMap (types only: the encoder is fetched through cudaGetDriverEntryPoint, no libcuda link dependency)
+#include <algorithm>
 #include <mutex>
 
 namespace b200 {
@@ -436,6 +437,209 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
 }
 
+// ------------------------------------------------------------------ CTA pairs (prefill shapes)
+// The same product with TWO SMs on one 256-row tile (tcgen05.mma.cta_group::2): each CTA of a cluster of two stages its own 128 rows of A and HALF
+// of the tile's B rows, and one instruction of the leader reads both halves -- per flop half the shared-memory writes and reads of B.  That traffic,
+// not the tensor pipe, is what the one-CTA form pays for (power as well as time: these launches run under the board's power cap).
+// Roles per CTA: warp 0 TMA producer, warp 1 MMA issuer (leader only), warps 2..9 epilogue of the CTA's own 128 rows (two warps per TMEM lane quarter,
+// one per half of the columns: a launch ends on an epilogue that nothing overlaps).  Every byte that either CTA loads is counted on the leader's
+// `full` barrier; `empty` and `tfull` are arrived at in both CTAs by multicast commits; both CTAs' epilogues release the leader's `tempty`.
+// Columns: the first n_wide column tiles are p.bn wide, the rest bn2: the last wave is cut so that it fills the pairs (choose_widths).
+// Measured: see pair_takes.
+struct GemmPairParams {
+    void *C;
+    int ldc, rowsA, rowsB, kb_total, tilesA, tiles;
+    int bn, bn2, n_wide;
+    int stages, is_bf16;
+    int swiglu_inter;  // as above: gate rows come from the leader's half of B, up rows from its peer's; tile widths count both
+};
+constexpr int kPairThreads = 320;
+constexpr int kPairStageBytes = 2 * kATileBytes;  // 128 rows of A, up to 128 rows of B
+
+__device__ unsigned int g_pair_wait_failed;  // a wait that gave up (seconds): the launch's results are not valid
+
+// false after a limit that no live launch reaches; the caller leaves its role loop
+__device__ __forceinline__ bool bar_wait_limited(uint32_t bar, uint32_t parity) {
+    for (int i = 0; i < (1 << 24); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    atomicExch(&g_pair_wait_failed, 1u);
+    return false;
+}
+__device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {  // the same shared-memory offset in CTA `rank` of the cluster
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t leader_bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+                 "l"(map), "r"(c0), "r"(c1), "r"(leader_bar)
+                 : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kPairThreads, 1)
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmB2, const GemmPairParams p) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (size_t)p.stages * kPairStageBytes);
+    const uint32_t full0 = s_u32(bars), empty0 = full0 + 8 * kMaxStages, tfull0 = empty0 + 8 * kMaxStages, tempty0 = tfull0 + 16;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kMaxStages + 4);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+
+    if (warp == 0 && lane == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB) : "memory");
+        for (int s = 0; s < p.stages; ++s) {
+            bar_init(full0 + 8 * s, 1);
+            bar_init(empty0 + 8 * s, 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            bar_init(tfull0 + 8 * a, 1);
+            bar_init(tempty0 + 8 * a, 16);  // eight epilogue warps of either CTA
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();  // the peer's barriers are initialised and its TMEM is allocated
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    pdl_wait();
+    pdl_launch_dependents();
+
+    auto width_of = [&](int tb) { return tb < p.n_wide ? p.bn : p.bn2; };
+    auto col_of = [&](int tb) {  // first output column (SwiGLU: half of a tile's width are output columns)
+        const int c = tb < p.n_wide ? tb * p.bn : p.n_wide * p.bn + (tb - p.n_wide) * p.bn2;
+        return p.swiglu_inter ? c >> 1 : c;
+    };
+
+    if (warp == 0) {
+        // ================================================= TMA producer: this CTA's rows of A, its half of the B rows
+        if (elect_one()) {
+            int it = 0;
+            bool live = true;
+            for (int item = pair; live && item < p.tiles; item += pairs) {
+                const int ta = item % p.tilesA, tb = item / p.tilesA, w = width_of(tb);
+                const int arow = ta * 2 * kBM + (int)rank * kBM;
+                const int brow = p.swiglu_inter ? (rank ? p.swiglu_inter : 0) + col_of(tb) : col_of(tb) + (int)rank * (w >> 1);
+                const CUtensorMap *mb = tb < p.n_wide ? &tmB : &tmB2;
+                for (int kb = 0; kb < p.kb_total; ++kb, ++it) {
+                    const int s = it % p.stages;
+                    live = bar_wait_limited(empty0 + 8 * s, ((it / p.stages) & 1) ^ 1);
+                    if (!live) break;
+                    const uint32_t sa = s_u32(smem + (size_t)s * kPairStageBytes), bar = in_cta(full0 + 8 * s, 0);
+                    if (rank == 0) bar_expect_tx(full0 + 8 * s, (uint32_t)(2 * (kATileBytes + (w >> 1) * kBK * 2)));
+                    tma_load_2d_pair(sa, &tmA, kb * kBK, arow, bar);
+                    tma_load_2d_pair(sa + kATileBytes, mb, kb * kBK, brow, bar);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ================================================= MMA issuer: the leader, for both
+        if (rank == 0) {
+            int it = 0, t = 0;
+            bool live = true;
+            for (int item = pair; live && item < p.tiles; item += pairs, ++t) {
+                const uint32_t idesc = instr_desc_f16(p.is_bf16 != 0, 2 * kBM, width_of(item / p.tilesA));
+                const int acc = t & 1;
+                live = bar_wait_limited(tempty0 + 8 * acc, ((t >> 1) & 1) ^ 1);
+                if (!live) break;
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
+                for (int kb = 0; kb < p.kb_total; ++kb, ++it) {
+                    const int s = it % p.stages;
+                    live = bar_wait_limited(full0 + 8 * s, (it / p.stages) & 1);
+                    if (!live) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t sa = s_u32(smem + (size_t)s * kPairStageBytes);
+                        const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + kATileBytes);
+#pragma unroll
+                        for (int k = 0; k < kBK / kUmmaK; ++k) tc_mma_f16_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        tc_commit_pair(empty0 + 8 * s);
+                        if (kb == p.kb_total - 1) tc_commit_pair(tfull0 + 8 * acc);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else {
+        // ================================================= epilogue: TMEM lane quarter q, one half of the columns
+        const int q = warp & 3, half = (warp - 2) >> 2;
+        T *C = reinterpret_cast<T *>(p.C);
+        int t = 0;
+        for (int item = pair; item < p.tiles; item += pairs, ++t) {
+            const int ta = item % p.tilesA, tb = item / p.tilesA, w = width_of(tb), acc = t & 1, col0 = col_of(tb);
+            if (!bar_wait_limited(tfull0 + 8 * acc, (t >> 1) & 1)) break;
+            tc_fence_after();
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 256);
+            const int i = ta * 2 * kBM + (int)rank * kBM + q * 32 + lane;
+            const int out_w = p.swiglu_inter ? w >> 1 : w;               // output columns of the tile, a multiple of 16
+            const int mid = (out_w >> 5) << 4;                            // this warp's share: [0, mid) or [mid, out_w), in steps of 16
+            for (int c = half ? mid : 0; c < (half ? out_w : mid); c += 16) {
+                uint32_t g[16];
+                tc_ld16(taddr + c, g);
+                const int valid = min(16, p.rowsB - (col0 + c));
+                if (p.swiglu_inter) {
+                    uint32_t u[16];
+                    tc_ld16(taddr + out_w + c, u);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) {  // (the same expression and roundings as the one-CTA epilogue)
+                        const float gf = round_to<T>(__uint_as_float(g[e])), uf = round_to<T>(__uint_as_float(u[e]));
+                        g[e] = __float_as_uint((gf / (1.0f + expf(-gf))) * uf);
+                    }
+                } else {
+                    tc_wait_ld();
+                }
+                if (i < p.rowsA && valid > 0) store_row16<T>(C + (size_t)i * p.ldc + col0 + c, g, valid);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(in_cta(tempty0 + 8 * acc, 0)) : "memory");
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();  // neither CTA leaves while the other may still read its shared memory or arrive at its barriers
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
+}
+
 // ------------------------------------------------------------------ host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -475,12 +679,71 @@ static unsigned int pow2_cols(int c) {
     return v;
 }
 
+// Column tiles of a pair launch: n_wide tiles of bn columns, the rest bn2 wide.  Tiles are dealt to the pairs in order, wide ones first, so pair 0 has
+// the most work; its load (columns, and what a tile costs beside its columns) is what a choice is judged by.  Widths are steps of 32 MMA columns.
+struct PairWidths { int bn, bn2, n_wide, n_tiles; long long cost; };
+static PairWidths choose_widths(int tiles_a, int cols, int pairs) {  // cols: MMA columns (SwiGLU: gate and up together)
+    constexpr int kTileCost = 24;
+    auto load = [&](int n1, int w1, int n2, int w2) {
+        const long long wide = (long long)tiles_a * n1, all = wide + (long long)tiles_a * n2;
+        const long long c1 = (wide + pairs - 1) / pairs, c = (all + pairs - 1) / pairs;
+        return c1 * (w1 + kTileCost) + (c - c1) * (w2 + kTileCost);
+    };
+    const int most = (cols + 255) / 256, back = std::max(1, (2 * pairs + tiles_a - 1) / tiles_a);
+    PairWidths best = {256, 256, most, most, load(most, 256, 0, 0)};
+    for (int n1 = std::max(0, most - 1 - back); n1 < most; ++n1)
+        for (int w2 = 224; w2 >= 64; w2 -= 32) {
+            const int n2 = (cols - n1 * 256 + w2 - 1) / w2;
+            const long long c = load(n1, 256, n2, w2);
+            if (c < best.cost) best = {256, w2, n1, n1 + n2, c};
+        }
+    return best;
+}
+
+// CTA pairs when their busiest pair finishes before the one-CTA form's busiest SM would.  Both are counted in columns of a row tile (a pair multiplies 256
+// rows in the time an SM takes for 128); per column the one-CTA form is the slower by its doubled B traffic (7B at 2048 tokens, all eight linears:
+// 1235 us against 1158), so row counts that 256-row tiles pad (1084 tokens: 1280 rows against 1152) stay with it.
+static bool pair_takes(int M, int cols, int sms) {
+    const int t128 = (M + kBM - 1) / kBM, t256 = (M + 2 * kBM - 1) / (2 * kBM), pairs = sms / 2;
+    if (cols < 256 || t256 * ((cols + 255) / 256) * 2 < pairs) return false;
+    long long one = 1LL << 60;
+    for (int bn : {256, 240, 224, 208, 192}) one = std::min(one, (long long)((t128 * ((cols + bn - 1) / bn) + sms - 1) / sms) * (bn + 24));
+    return choose_widths(t256, cols, pairs).cost * 16 <= one * 17;
+}
+
+static int launch_gemm_pair(const void *x, const void *w, void *y, int M, int N, int K, int dtype, int swiglu_inter, cudaStream_t st) {
+    const bool bf16 = dtype == B200_BF16;
+    const int cols = swiglu_inter ? 2 * swiglu_inter : N, sms = sm_count(), pairs = sms / 2;
+    GemmPairParams p = {};
+    p.C = y, p.ldc = swiglu_inter ? swiglu_inter : N, p.rowsA = M, p.rowsB = p.ldc;
+    p.kb_total = (K + kBK - 1) / kBK, p.is_bf16 = bf16 ? 1 : 0, p.swiglu_inter = swiglu_inter;
+    p.tilesA = (M + 2 * kBM - 1) / (2 * kBM);
+    const PairWidths pw = choose_widths(p.tilesA, cols, pairs);
+    p.bn = pw.bn, p.bn2 = pw.bn2, p.n_wide = pw.n_wide, p.tiles = p.tilesA * pw.n_tiles;
+    p.stages = 6;
+    const size_t smem = (size_t)p.stages * kPairStageBytes + 1024 + (2 * kMaxStages + 4) * 8 + 16;
+    CUtensorMap tmA, tmB, tmB2;
+    if (!make_map(&tmA, x, M, K, kBM, bf16) || !make_map(&tmB, w, cols, K, p.bn / 2, bf16) || !make_map(&tmB2, w, cols, K, p.bn2 / 2, bf16)) {
+        set_error("gemm_tc pair: cuTensorMapEncodeTiled failed (rows %d/%d, K %d)", M, cols, K);
+        return B200_ERR_CUDA;
+    }
+    const int grid = 2 * std::min(p.tiles, pairs);
+    auto launch = [&](auto kern) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        launch_pdl_cluster(kern, dim3(grid), dim3(kPairThreads), smem, st, true, 2u, tmA, tmB, tmB2, p);
+    };
+    if (bf16) launch(gemm_tc_pair_kernel<__nv_bfloat16>);
+    else launch(gemm_tc_pair_kernel<__half>);
+    return cuda_status("gemm_tc pair launch");
+}
+
 static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int N, int K, int dtype, int swiglu_inter, cudaStream_t st) {
     if (dtype != B200_BF16 && dtype != B200_F16) return B200_ERR_UNSUPPORTED;
     if (M < 1 || K % 8 != 0 || K < kBK || !aligned16(x) || !aligned16(w) || !y) return B200_ERR_UNSUPPORTED;
     const bool bf16 = dtype == B200_BF16;
     const bool swap = M <= 128;
     if (swiglu_inter && (swap || swiglu_inter < 128)) return B200_ERR_UNSUPPORTED;  // the fused epilogue exists for prefill-sized token counts
+    if (!swap && pair_takes(M, swiglu_inter ? 2 * swiglu_inter : N, sm_count())) return launch_gemm_pair(x, w, y, M, N, K, dtype, swiglu_inter, st);
     GemmTcParams p = {};
     p.C = y, p.ldc = N, p.K = K, p.swap = swap ? 1 : 0, p.is_bf16 = bf16 ? 1 : 0;
     p.swiglu_inter = swiglu_inter;

@@ -1,0 +1,149 @@
+"""The linears' tensor-core kernels at the edges of their tiles: the register-stationary GEMV (csrc/gemv_rs.cuh: one to sixteen tokens, every weight
+format, k slices that do not divide evenly, rows past the last unit, several parts) and the CTA-pair GEMM (csrc/gemm_tc.cu: rows past the last
+256-row tile, column tiles of two widths, k past the last stage), against the product in 64 bits; and the sampler's random numbers."""
+import math
+
+import pytest
+import torch
+
+import util
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+b200 = util.b200()
+# one rounding of the result to the output type; the sums themselves are fp32 (2^-24 per term of up to 16384 random signs: below a tenth of it)
+ROUND = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+
+
+def close(got, want, dtype, what):
+    scale = want.abs().max()
+    err = (got.double() - want).abs() - ROUND[dtype] * want.abs()
+    assert not torch.isnan(got).any(), what
+    assert float(err.max() / scale) < 2e-4, (what, float(err.max() / scale))  # 2e-4 of the largest: sums of up to 16384 products in fp32
+
+
+def quantised(gen, n, k, fmt, dtype):
+    """-> (codes, scales, zeros, dense weights in 64 bits)."""
+    if fmt == "fp8":
+        q = torch.randn(n, k, generator=gen, device=DEV).to(torch.float8_e4m3fn)
+        s = torch.rand(n, generator=gen, device=DEV) + 0.5
+        return q.view(torch.uint8), s, None, q.to(torch.float32).double() * s.double()[:, None]
+    codes = torch.randint(0, 256, (n, k // 2), generator=gen, device=DEV, dtype=torch.uint8)
+    s = (torch.rand(n, k // 128, generator=gen, device=DEV) + 0.5).to(dtype)
+    z = torch.randint(0, 16, (n, k // 128), generator=gen, device=DEV, dtype=torch.uint8)
+    q = torch.stack((codes & 15, codes >> 4), -1).reshape(n, k // 128, 128).double()
+    return codes, s, z, ((q - z.double()[..., None]) * s.double()[..., None]).reshape(n, k)
+
+
+@pytest.mark.parametrize("fmt", ["dense", "fp8", "int4"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("m", [1, 2, 3, 7, 8, 9, 15, 16])
+@pytest.mark.parametrize("k,n", [(128, 64), (384, 72), (2176, 1187 * 8), (4096, 40), (4224, 1184), (8192, 264), (11008, 2376), (14336, 8)])
+def test_linear_of_few_tokens(fmt, dtype, m, k, n):
+    gen = torch.Generator(device=DEV).manual_seed(m * 1000 + k + n)
+    x = torch.randn(m, k, generator=gen, device=DEV).to(dtype)
+    if fmt == "dense":
+        w = torch.randn(n, k, generator=gen, device=DEV).to(dtype)
+        got, dense = b200.linear(x, w), w.double()
+    else:
+        w, s, z, dense = quantised(gen, n, k, fmt, dtype)
+        got = b200.linear(x, w, w_format=b200.W_FP8 if fmt == "fp8" else b200.W_INT4, scales=s, zeros=z, group=128, N=n)
+    close(got, x.double() @ dense.T, dtype, (fmt, m, k, n))
+
+
+@pytest.mark.parametrize("n", [1, 7, 9, 1185])
+def test_linear_of_few_tokens_and_odd_rows(n):
+    """Row counts that are no multiple of a unit: the last unit's missing rows are neither fetched nor stored."""
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    x, w = torch.randn(6, 512, generator=gen, device=DEV).bfloat16(), torch.randn(n, 512, generator=gen, device=DEV).bfloat16()
+    out = torch.full((6 * n + 64,), 7.0, dtype=torch.bfloat16, device=DEV)
+    b200.linear(x, w, out=out[:6 * n].view(6, n))
+    close(out[:6 * n].view(6, n), x.double() @ w.double().T, torch.bfloat16, n)
+    assert bool((out[6 * n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("fmt", ["dense", "fp8", "int4"])
+@pytest.mark.parametrize("batch", [1, 2, 5, 8, 9, 16])
+def test_norm_on_the_fragments_matches_the_norm_kernel(fmt, batch):
+    """A layer whose norms run inside the linears (up to 16 tokens) against the same rows in a batch of 17 (norm kernel in front): rows agree to the
+    roundings of the layer's 16-bit intermediates."""
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    h, heads, kv, d, inter, rows = 1024, 8, 2, 128, 1408, 17
+
+    def lin(n, k):
+        if fmt == "dense":
+            return (torch.randn(n, k, generator=gen, device=DEV) / math.sqrt(k)).bfloat16()
+        q, s, z, _ = quantised(gen, n, k, fmt, torch.bfloat16)
+        return (q, s / math.sqrt(k), None) if fmt == "fp8" else (q, (s.float() / (5 * math.sqrt(k))).bfloat16(), z)
+
+    def vec(n):
+        return (1 + 0.2 * torch.randn(n, generator=gen, device=DEV)).bfloat16()
+
+    layers = [dict(g1=vec(h), g2=vec(h), o_bias=vec(h), qkv_bias=vec((heads + 2 * kv) * d), qkv=lin((heads + 2 * kv) * d, h), o=lin(h, heads * d),
+                   gate_up=lin(2 * inter, h), down=lin(h, inter)) for _ in range(2)]
+    wf = {"dense": b200.W_DENSE, "fp8": b200.W_FP8, "int4": b200.W_INT4}[fmt]
+    x = (2 * torch.randn(rows, h, generator=gen, device=DEV)).bfloat16()
+    k0, v0 = (torch.randn(2, rows, kv, 64, d, generator=gen, device=DEV).bfloat16() for _ in range(2))
+
+    def step(n):
+        dec = b200.Decoder(b200.DecoderConfig(h, heads, kv, d, inter, 2, 64, n, b200.BF16, wf, 128, 1e-6, d, 10000.0, 1, 0), DEV)
+        for i, w in enumerate(layers):
+            dec.set_layer(i, w)
+        hidden, kc, vc = x[:n].clone(), k0[:, :n].contiguous(), v0[:, :n].contiguous()
+        dec.step(hidden, kc, vc, 33)
+        torch.cuda.synchronize()
+        return hidden.double()
+
+    want, got = step(rows)[:batch], step(batch)
+    # per row: two layers of 16-bit intermediates summed in another order
+    rel = (got - want).norm(dim=-1) / want.norm(dim=-1)
+    assert float(rel.max()) < 1.5e-2, rel
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("m,k,n", [(256, 64, 9728), (250, 72, 9728), (512, 136, 4928), (769, 200, 4096), (1000, 1024, 4096), (1084, 320, 5136), (2048, 128, 4096),
+                                   (2047, 88, 2056), (4096, 64, 264), (129, 4096, 12288)])
+def test_linear_of_prompts(dtype, m, k, n):
+    """Pairs of CTAs on 256-row tiles where they serve: rows and columns past the last tile, two tile widths, a last stage that is mostly padding."""
+    gen = torch.Generator(device=DEV).manual_seed(m + k + n)
+    x, w = torch.randn(m, k, generator=gen, device=DEV).to(dtype), torch.randn(n, k, generator=gen, device=DEV).to(dtype)
+    out = torch.full((m * n + 64,), 7.0, dtype=dtype, device=DEV)
+    b200.linear(x, w, out=out[:m * n].view(m, n))
+    close(out[:m * n].view(m, n), x.double() @ w.double().T, dtype, (m, k, n))
+    assert bool((out[m * n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("m,k,inter", [(256, 64, 4864), (1000, 200, 2752), (2048, 128, 2688), (1084, 72, 5000), (300, 512, 1408)])
+def test_swiglu_of_prompts_is_the_two_launchers(m, k, inter):
+    """Gate and up halves of a tile come from the two CTAs of a pair: bit-identical to the linear followed by silu-and-mul."""
+    gen = torch.Generator(device=DEV).manual_seed(m + inter)
+    x, w = torch.randn(m, k, generator=gen, device=DEV).bfloat16(), torch.randn(2 * inter, k, generator=gen, device=DEV).bfloat16()
+    want = b200.silu_and_mul(b200.linear(x, w).view(m, 2, inter))
+    assert torch.equal(b200.linear_swiglu(x, w), want)
+
+
+@pytest.mark.parametrize("step", [1, 77, 123456])
+def test_sampled_ids_use_the_generators_own_numbers(step):
+    """Rows 0 .. 299 (all low digits of the subsequence, alone and together) and rows past 2^16: the ids that cuRAND's own first numbers give."""
+    for rows in (300, 65536 + 40):
+        gen = torch.Generator(device=DEV).manual_seed(step)
+        k = 8
+        ids = torch.arange(rows * k, dtype=torch.int32, device=DEV).reshape(rows, k)
+        vals = torch.sort(torch.randn(rows, k, generator=gen, device=DEV), -1, descending=True).values.contiguous()
+        u = b200.xorwow_uniform(rows, step, DEV)
+        weights = torch.exp(vals - vals[:, :1])
+        total = torch.zeros(rows, device=DEV)
+        for i in range(k):
+            total = total + weights[:, i]
+        left, want, done = u * total, ids[:, 0].clone(), torch.zeros(rows, dtype=torch.bool, device=DEV)
+        margin = torch.full((rows,), 9.0, device=DEV)
+        for i in range(k):
+            left = left - weights[:, i]
+            margin = torch.minimum(margin, left.abs())
+            hit = (left < 0) & ~done
+            want = torch.where(hit, ids[:, i], want)
+            done |= hit
+        seq, fin = torch.zeros(rows, dtype=torch.int32, device=DEV), torch.zeros(rows, dtype=torch.uint8, device=DEV)
+        got = b200.sampling(ids, vals.clone(), seq, fin, step, -1, rows * k)
+        clear = margin > 1e-5  # (a draw on the edge of two candidates may fall on either side of an ulp of exp)
+        assert bool((got == want)[clear].all()) and float(clear.float().mean()) > 0.99
