@@ -92,6 +92,9 @@ struct TpPush {
 // tp (optional, world > 1): `in` is replaced by the sum over ranks of tp->peer_x[*] (see TpExchange).
 int launch_norm_tp(int dtype, const void *in, void *out, const void *rin, void *rout, const void *bias, const void *gamma, float eps,
                    int tokens, int hidden, const TpExchange *tp, cudaStream_t st);
+// sampling.cu
+int launch_topk_draw(const float *logits, int *tmp_ids, float *tmp_vals, int *final_ids, float *final_vals, int *seq_len, uint8_t *finished, int *output_id, int rows,
+                     int vocab, int k, int step, int end_id, cudaStream_t st);
 // gamma == NULL: out = o + bias.  (norm.cu)
 int launch_norm_any(int dtype, const void *in, void *out, const void *rin, void *rout, const void *bias, const void *gamma,
                     float eps, int tokens, int hidden, cudaStream_t st);

@@ -816,10 +816,12 @@ int b200_lm_head_topk_sample(b200_decoder_t *dec, const void *hidden, const void
     }
     if (!topk_ids) return B200_OK;  // logits only
     B200_REQUIRE(tmp_ids && tmp_vals && topk_vals, "lm_head_topk_sample: null top-k buffer");
+    if (output_id && seq_len && finished && k >= 1 && k <= B200_TOPK_MAX_K && batch <= 65535)
+        return launch_topk_draw(logits, tmp_ids, tmp_vals, topk_ids, topk_vals, seq_len, finished, output_id, batch, vocab, k, step, end_id, st);
     rc = b200_topk(logits, tmp_ids, tmp_vals, topk_ids, topk_vals, batch, vocab, k, B200_F32, stream);
     if (rc != B200_OK || !output_id) return rc;
-    B200_REQUIRE(seq_len && finished, "lm_head_topk_sample: null sampling buffer");
-    return b200_sampling(topk_ids, topk_vals, seq_len, finished, output_id, batch, k, step, end_id, vocab, B200_F32, stream);
+    set_error("lm_head_topk_sample: null sampling buffer");
+    return B200_ERR_INVALID_ARG;
 }
 
 }  // extern "C"
