@@ -26,6 +26,7 @@
 //     order (deterministic), across K parts too, applies the FP8 row scale / SwiGLU (reference src/kernels/silu_and_mul.cu:6-41; a
 //     unit is then 4 gate rows interleaved with their 4 up rows) and stores -- or pushes the tensor-parallel partial (TpPush).
 #pragma once
+#include <algorithm>
 #include <type_traits>
 
 #include "gemv.cuh"
