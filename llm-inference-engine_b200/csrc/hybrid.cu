@@ -784,7 +784,7 @@ Carve carve(const b200_hybrid *m) {
         n_in = std::max(n_in, (size_t)n_in_of(l));
         for (const b200_hybrid_layer_t *mx : {&l, l.side})
             if (mx && (mx->mixer == B200_MIXER_GLA || mx->mixer == B200_MIXER_DELTA || mx->mixer == B200_MIXER_SSD || mx->mixer == B200_MIXER_LINEAR))
-                n_chunk = std::max(n_chunk, chunk_scratch_floats(mx->heads, mx->dim, c.max_tokens, c.max_seqs));
+                n_chunk = std::max(n_chunk, chunk_scratch_floats(mx->heads, mx->dim, mx->mixer == B200_MIXER_DELTA, c.max_tokens, c.max_seqs));
         n_mix = std::max(n_mix, (size_t)l.heads * std::max(l.dim, l.vdim));
         n_f32 = std::max(n_f32, (size_t)l.heads * std::max(l.dim, l.vdim));
         n_mix = std::max(n_mix, (size_t)l.heads * l.vdim);

@@ -4,6 +4,25 @@
 
 namespace b200 {
 
+// eight consecutive elements from a 16-byte boundary <-> fp32
+template <typename T> __device__ __forceinline__ void load8(const T *__restrict__ p, float *f) {
+    if constexpr (sizeof(T) == 2) {
+        unpack16<T>(ld_v4(p), f);
+    } else {
+        load_n<float, 4>(p, f);
+        load_n<float, 4>(p + 4, f + 4);
+    }
+}
+template <typename T> __device__ __forceinline__ void store8(T *__restrict__ p, const float *f) {
+    if constexpr (sizeof(T) == 2) {
+        st_v4(p, pack16<T>(f));
+    } else {
+        store_n<float, 4>(p, f);
+        store_n<float, 4>(p + 4, f + 4);
+    }
+}
+
+
 // attention_chunked.cu
 int launch_attn_qk_norm_cache(int dtype, const void *proj, int ld, void *q_out, void *k_pool, void *v_pool, const float *q_norm,
                               const float *k_norm, float eps, const int *tok_seq, const int *tok_pos, const int *block_table, int mpps,
@@ -157,7 +176,7 @@ int launch_gla_output(int dtype, const float *o, const float *w, float eps, cons
 // serial kernels serve them with max_tokens = kChunkMinTokens - 1).  B200_ERR_UNSUPPORTED, nothing launched: sizes or alignments it does not take.
 // scratch: fp32, chunk_scratch_floats of the engine's limits (0: sizes it never takes); tokens / longest: of this call and of its longest portion
 constexpr int kChunkMinTokens = 64;
-size_t chunk_scratch_floats(int heads, int dim, int max_tokens, int max_seqs);
+size_t chunk_scratch_floats(int heads, int dim, bool delta, int max_tokens, int max_seqs);
 int launch_chunk_gla(int dtype, const void *proj, int ld, const float *decay, float *state, float *o, const int *seq_start, const int *seq_pos0,
                      const int *seq_slot, int n_seqs, int heads, int dim, int vdim, float *scratch, size_t scratch_floats, int tokens, int longest,
                      cudaStream_t st);

@@ -99,6 +99,96 @@ delta_prep_kernel(const T *__restrict__ proj, int ld, int col0, const float *__r
     for (int h = threadIdx.x; h < heads; h += blockDim.x) out[lay.beta + h] = sigmoid_r(Elem<T>::to_f(row[h]));
 }
 
+// The same for prompt-sized batches of four taps: a thread takes EIGHT channels (one 16-byte piece of a projected row) of kPrepTokens consecutive
+// rows, `tiles` times.  It reads every row of its piece once -- the taps are rows it already holds -- and its channels' weights once, a channel's four in
+// one access: one CTA per token read each input once per tap and 64 KB of weights per token (100 us for 2911 tokens of 4096 channels, where the bytes
+// take 12), and weights fetched one by one for every eight rows still cost 1024 sectors a warp (65 us; now 44).  The unit norm of a head is a butterfly over the
+// dim / 8 lanes that hold it.  grid (row groups, channel groups + 1): the last group copies the low-rank inputs and the steps.
+constexpr int kPrepTokens = 8, kPrepTaps = 4;
+template <typename T>
+__global__ void __launch_bounds__(256)
+delta_prep_tile_kernel(const T *__restrict__ proj, int ld, int col0, const float *__restrict__ conv_w, const float *__restrict__ conv_state, int rank,
+                       int gate_rank, T *__restrict__ lr_a, T *__restrict__ lr_g, float *__restrict__ rec, DeltaRow lay, const int *__restrict__ tok_seq,
+                       const int *__restrict__ tok_pos, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int tokens, int heads, int kv_heads, int dim, int vdim,
+                       int tiles) {
+    __shared__ int s_pos[kPrepTokens], s_back[kPrepTokens], s_slot[kPrepTokens];  // position, rows of the own portion before it, state slot
+    const int nqk = kv_heads * dim, nv = heads * vdim, channels = 2 * nqk + nv;
+    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+    const bool copies = blockIdx.y + 1 == gridDim.y;
+    const bool mine = c < channels;      // (a head's lanes are all in range or all out: channels and heads are whole pieces)
+    const int cc = mine ? c : 0;
+    float w[kPrepTaps][8];               // w[b]: the weight of the input b tokens ago
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const float4 f = *reinterpret_cast<const float4 *>(conv_w + (size_t)(cc + e) * kPrepTaps);
+        w[3][e] = f.x, w[2][e] = f.y, w[1][e] = f.z, w[0][e] = f.w;
+    }
+    const bool is_q = cc < nqk, is_qk = cc < 2 * nqk;
+    const int lanes = dim / 8;           // lanes that hold one q or k head
+    float *dst0 = rec + (is_q ? lay.q + cc : (is_qk ? lay.k + cc - nqk : lay.v + cc - 2 * nqk));
+    for (int tile = 0; tile < tiles; ++tile) {
+        const int t0 = (blockIdx.x * tiles + tile) * kPrepTokens, nt = min(kPrepTokens, tokens - t0);
+        if (nt <= 0) return;
+        if (copies) {
+            for (int tt = 0; tt < nt; ++tt) {
+                const T *row = proj + (size_t)(t0 + tt) * ld + col0 + channels;  // step | decay-in | gate-in
+                for (int r = threadIdx.x; r < rank; r += blockDim.x) lr_a[(size_t)(t0 + tt) * rank + r] = row[heads + r];
+                for (int r = threadIdx.x; r < gate_rank; r += blockDim.x) lr_g[(size_t)(t0 + tt) * gate_rank + r] = row[heads + rank + r];
+                for (int h = threadIdx.x; h < heads; h += blockDim.x) rec[(size_t)(t0 + tt) * lay.ld + lay.beta + h] = sigmoid_r(Elem<T>::to_f(row[h]));
+            }
+            continue;
+        }
+        uint4 win[kPrepTokens + kPrepTaps - 1];  // rows t0 - 3 .. t0 + kPrepTokens - 1
+#pragma unroll
+        for (int r = 0; r < kPrepTokens + kPrepTaps - 1; ++r) win[r] = ld_v4(proj + (size_t)min(max(t0 + r - (kPrepTaps - 1), 0), tokens - 1) * ld + col0 + cc);
+        __syncthreads();
+        if (threadIdx.x < nt) {
+            const int seq = tok_seq[t0 + threadIdx.x], pos = tok_pos[t0 + threadIdx.x];
+            s_pos[threadIdx.x] = pos, s_back[threadIdx.x] = pos - seq_pos0[seq], s_slot[threadIdx.x] = seq_slot[seq];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int tt = 0; tt < kPrepTokens; ++tt) {
+            if (tt >= nt) break;
+            const int back = s_back[tt];
+            float acc[8] = {};
+#pragma unroll
+            for (int b = kPrepTaps - 1; b >= 0; --b) {  // oldest input first, as the one-token form adds them
+                float x[8];
+                if (b <= back) {
+                    unpack16<T>(win[tt + kPrepTaps - 1 - b], x);
+                } else if (s_pos[tt] - b >= 0) {        // stored by an earlier portion: its last inputs, the newest in the last row
+                    const float *st = conv_state + ((size_t)s_slot[tt] * (kPrepTaps - 1) + (kPrepTaps - 1 + back - b)) * channels + cc;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] = st[e];
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] = 0.0f;
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc[e] = fmaf(w[b][e], x[e], acc[e]);
+            }
+            float ss = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                acc[e] = acc[e] * sigmoid_r(acc[e]);
+                ss = fmaf(acc[e], acc[e], ss);
+            }
+            if (is_qk) {  // (the same for a whole warp)
+                for (int o = lanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                const float inv = rsqrtf(ss + 1e-6f) * (is_q ? rsqrtf((float)dim) : 1.0f);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc[e] *= inv;
+            }
+            if (mine) {
+                float4 *dst = reinterpret_cast<float4 *>(dst0 + (size_t)(t0 + tt) * lay.ld);
+                dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+            }
+        }
+    }
+}
+
 // The causal convolution of channel c at token t (packed row) / position pos: taps - 1 earlier inputs come from the portion's own rows,
 // from the slot's stored inputs (positions before pos0) or are zero (before position 0).  Every tap reads both places at an index that
 // always exists and keeps the one that is meant.
@@ -297,16 +387,30 @@ group_output_kernel(const float *__restrict__ o, const float *__restrict__ skip,
 // za fp32 [tokens, heads*dim] = w_decay . decay-in, zg fp32 [tokens, heads*vdim] = w_gate2 . gate-in (the products of the two low-rank
 // inputs) -> the token row's decay = exp(-exp(a_log[head]) * softplus(za + bias)) and gate pre-activation (the output kernel applies
 // the sigmoid)
+// (V4: four channels per access, where the heads' channels are whole pieces)
+template <bool V4>
 __global__ void __launch_bounds__(256)
 delta_finish_kernel(const float *__restrict__ za, const float *__restrict__ zg, const float *__restrict__ decay_bias, const float *__restrict__ a_log,
                     float *__restrict__ rec, DeltaRow lay, int heads, int dim, int vdim) {
+    constexpr int N = V4 ? 4 : 1;
     const int t = blockIdx.x, nd = heads * dim, nv = heads * vdim;
     float *out = rec + (size_t)t * lay.ld;
-    for (int c = threadIdx.x; c < nd; c += blockDim.x) {
-        const float z = za[(size_t)t * nd + c] + (decay_bias ? decay_bias[c] : 0.0f);
-        out[lay.decay + c] = expf(-expf(a_log[c / dim]) * softplus_r(z));
+    for (int c = threadIdx.x * N; c < nd; c += blockDim.x * N) {
+        float z[N], b[N];
+        load_n<float, N>(za + (size_t)t * nd + c, z);
+#pragma unroll
+        for (int e = 0; e < N; ++e) b[e] = 0.0f;
+        if (decay_bias) load_n<float, N>(decay_bias + c, b);
+        const float rate = -expf(a_log[c / dim]);
+#pragma unroll
+        for (int e = 0; e < N; ++e) z[e] = expf(rate * softplus_r(z[e] + b[e]));
+        store_n<float, N>(out + lay.decay + c, z);
     }
-    for (int c = threadIdx.x; c < nv; c += blockDim.x) out[lay.gate + c] = zg[(size_t)t * nv + c];
+    for (int c = threadIdx.x * N; c < nv; c += blockDim.x * N) {
+        float z[N];
+        load_n<float, N>(zg + (size_t)t * nv + c, z);
+        store_n<float, N>(out + lay.gate + c, z);
+    }
 }
 
 // After the convolutions have read it: the state's rows move up by the portion's length and its last inputs come in.  grid (channel
@@ -708,7 +812,20 @@ int launch_delta_prep(int dtype, const void *proj, int ld, int col0, const float
     const DeltaRow lay = delta_row(heads, kv_heads, dim, vdim);
     const size_t smem = ((size_t)2 * kv_heads * dim + heads * vdim) * sizeof(float), es = dtype == B200_F32 ? 4 : 2;
     void *lr_a = lr, *lr_g = (char *)lr + (((size_t)tokens * rank * es + 255) & ~(size_t)255);
-    B200_DISPATCH_DTYPE(dtype, {
+    // prompt-sized batches of a 16-bit engine: whole 16-byte pieces everywhere, and a head in 2 .. 32 lanes of one warp
+    const bool pieces = dtype != B200_F32 && tokens > 64 && taps == kPrepTaps && (dim == 16 || dim == 32 || dim == 64 || dim == 128 || dim == 256) && (heads * vdim) % 8 == 0 &&
+                        (2 * kv_heads * dim) % 256 == 0 && ld % 8 == 0 && col0 % 8 == 0 && all_aligned16({proj, rec, conv_w});
+    const int channels = 2 * kv_heads * dim + heads * vdim;
+    const int row_tiles = (tokens + kPrepTokens - 1) / kPrepTokens, groups = (channels / 8 + 255) / 256;
+    const int per = std::max(1, std::min(4, row_tiles * groups / (2 * sm_count())));  // tiles per CTA, two CTAs per SM left
+    const dim3 tile_grid((row_tiles + per - 1) / per, groups + 1);
+    if (pieces && dtype == B200_BF16)
+        delta_prep_tile_kernel<__nv_bfloat16><<<tile_grid, 256, 0, st>>>((const __nv_bfloat16 *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__nv_bfloat16 *)lr_a,
+                                                                         (__nv_bfloat16 *)lr_g, rec, lay, tok_seq, tok_pos, seq_pos0, seq_slot, tokens, heads, kv_heads, dim, vdim, per);
+    else if (pieces)
+        delta_prep_tile_kernel<__half><<<tile_grid, 256, 0, st>>>((const __half *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__half *)lr_a, (__half *)lr_g, rec, lay,
+                                                                  tok_seq, tok_pos, seq_pos0, seq_slot, tokens, heads, kv_heads, dim, vdim, per);
+    else B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         // few tokens: few CTAs, so each gets more threads (a thread's channels are a chain of load latencies)
         delta_prep_kernel<T><<<tokens, tokens <= 64 ? 1024 : 256, smem, st>>>((const T *)proj, ld, col0, conv_w, taps, conv_state, rank, gate_rank, (T *)lr_a, (T *)lr_g, rec, lay,
@@ -726,7 +843,8 @@ int launch_delta_prep(int dtype, const void *proj, int ld, int col0, const float
         if (rc == B200_ERR_UNSUPPORTED) rc = launch_proj_f32(dtype, xs[i], ks[i], dtype, ws[i], nullptr, zs[i], ns[i], tokens, ns[i], ks[i], st);
         if (rc != B200_OK) return rc;
     }
-    delta_finish_kernel<<<tokens, 256, 0, st>>>(za, zg, decay_bias, a_log, rec, lay, heads, dim, vdim);
+    const bool v4 = dim % 4 == 0 && (heads * vdim) % 4 == 0 && all_aligned16({za, zg, decay_bias, rec});
+    (v4 ? delta_finish_kernel<true> : delta_finish_kernel<false>)<<<tokens, 256, 0, st>>>(za, zg, decay_bias, a_log, rec, lay, heads, dim, vdim);
     return cuda_status("delta_finish launch");
 }
 
