@@ -475,6 +475,8 @@ int launch_chunked_attention_tiles(int dtype, const void *q, const void *k_pool,
         set_error("chunked_attention tiles: 16-bit dtypes and dim 64 / 128 only");
         return B200_ERR_UNSUPPORTED;
     }
+    const int rc = launch_chunked_attention_tc(dtype, q, k_pool, v_pool, sink, gate_in, gate_ld, out, tiles, n_tiles, block_table, mpps, heads, kv_heads, dim, scale, chunk, st);
+    if (rc != B200_ERR_UNSUPPORTED) return rc;
 #define B200_ATTN_TILES(TT, DD) \
     return launch_mma_t<TT, DD>(q, k_pool, v_pool, sink, gate_in, gate_ld, out, tiles, n_tiles, block_table, mpps, heads, kv_heads, scale, chunk, st)
     if (dtype == B200_BF16) {

@@ -698,6 +698,10 @@ int launch_latent_attention_tiles(int dtype, const void *ql, const void *qr, con
         set_error("latent_attention tiles: 16-bit dtypes, kv_rank and rot_dim multiples of 16, kv_rank <= 128, a multiple of 32 up to 256, or a multiple of 128");
         return B200_ERR_UNSUPPORTED;
     }
+    if (!by_head) {
+        const int rc = launch_latent_attention_tc(dtype, ql, qr, pool, sink, ol, tiles, n_tiles, block_table, mpps, t_pad, heads, kv_rank, rot_dim, scale, window, st);
+        if (rc != B200_ERR_UNSUPPORTED) return rc;
+    }
     const int nv = latent_value_blocks(kv_rank);
     dim3 grid(n_tiles, by_head ? (heads + kLatTileQ - 1) / kLatTileQ : heads, kv_rank / (16 * nv));
     // one-token tiles that do not fill the device: the key tiles of every token are shared out over up to 8 CTAs, whose partial results

@@ -593,6 +593,9 @@ int launch_scored_attention_tiles(int dtype, const void *q, const void *k_pool, 
         set_error("scored_attention tiles: 16-bit dtypes, dim and vdim of 32 / 64 / 128, a penalty only with a window");
         return B200_ERR_UNSUPPORTED;
     }
+    const int rc = launch_scored_attention_tc(dtype, q, k_pool, v_pool, dist_r1, dist_r2, gate_in, gate_ld, out, out_ld, out_scale, tiles, n_tiles, block_table, mpps, heads, kv_heads,
+                                              dim, vdim, scale, window, sigmoid, opt, st);
+    if (rc != B200_ERR_UNSUPPORTED) return rc;
 #define B200_SCORED_ARGS q, k_pool, v_pool, head_bias, dist_r1, dist_r2, gate_in, gate_ld, out, out_ld, out_scale, tiles, n_tiles, block_table, mpps, heads, kv_heads, scale, window, sigmoid, st, opt
 #define B200_SCORED_DV(TT, DK)                                                     \
     do {                                                                           \

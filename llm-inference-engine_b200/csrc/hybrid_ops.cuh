@@ -62,6 +62,12 @@ int launch_latent_gate(int dtype, const void *ov, const void *gate_in, int gate_
 // out [tokens, cols] = rmsnorm(in [tokens, ld] from its column 0 on) * w
 int launch_rms_rows(int dtype, const void *in, int ld, const float *w, float eps, void *out, int tokens, int cols, cudaStream_t st);
 
+// prompt_attn_tc.cu: the same attention on tcgen05 for the sizes that fill its tiles (B200_ERR_UNSUPPORTED, nothing launched, for others)
+int launch_chunked_attention_tc(int dtype, const void *q, const void *k_pool, const void *v_pool, const float *sink, const void *gate, int gate_ld, void *out,
+                                const int *tiles, int n_tiles, const int *block_table, int mpps, int heads, int kv_heads, int dim, float scale, int chunk, cudaStream_t st);
+int launch_latent_attention_tc(int dtype, const void *ql, const void *qr, const void *pool, const float *sink, void *ol, const int *tiles, int n_tiles,
+                               const int *block_table, int mpps, int t_pad, int heads, int kv_rank, int rot_dim, float scale, int window, cudaStream_t st);
+
 // attention_scored.cu: proj [tokens, ld] holds q (heads*dim), k (kv_heads*dim), v (kv_heads*vdim) from column col0 on; b_in (optional) is
 // counted from the same row.  q_out [tokens, heads*dim]; pools K [pages, kv_heads, page, dim], V [pages, kv_heads, page, vdim]
 // options of the prep step: rot_half: rotating pairs (i, i + rot_dims/2) instead of (2i, 2i+1); rot_factor > 0: long wavelengths are slowed
@@ -82,6 +88,10 @@ int launch_scored_attention(int dtype, const void *q, const void *k_pool, const 
                             const int *tok_pos, const int *block_table, int mpps, int tokens, int heads, int kv_heads, int dim, int vdim,
                             float scale, int window, int sigmoid, int max_keys, cudaStream_t st, const int *tok_list = nullptr,
                             ScoredOptions opt = ScoredOptions());
+// (on tcgen05, prompt_attn_tc.cu; B200_ERR_UNSUPPORTED, nothing launched, for sizes and options it does not take)
+int launch_scored_attention_tc(int dtype, const void *q, const void *k_pool, const void *v_pool, const float *dist_r1, const float *dist_r2, const void *gate, int gate_ld,
+                               void *out, int out_ld, float out_scale, const int *tiles, int n_tiles, const int *block_table, int mpps, int heads, int kv_heads, int dim, int vdim,
+                               float scale, int window, int sigmoid, ScoredOptions opt, cudaStream_t st);
 bool scored_attention_tiles_supported(int dtype, int dim, int vdim, int gate_ld, int out_ld, int window, bool penalty);
 int launch_scored_attention_tiles(int dtype, const void *q, const void *k_pool, const void *v_pool, const float *head_bias, const float *dist_r1,
                                   const float *dist_r2, const void *gate_in, int gate_ld, void *out, int out_ld, float out_scale,
