@@ -28,6 +28,7 @@
 //   latent mixer, q_rank > 0: down-projections -> row norm -> query up-projection -> as above, one gate per head
 // and at the end: final norm of the wanted rows -> LM head with fp32 logits (scaled, soft-capped).
 // Everything is stream-ordered and allocation-free; the only host->device traffic of a call is one copy of the batch description.
+#include "gemv.cuh"
 #include "hybrid_ops.cuh"
 
 #include <algorithm>
@@ -42,16 +43,29 @@ constexpr int kMingruChunk = 128;  // tokens of one chunk of the minGRU's scan (
 constexpr int kLatentHeadsPerTile = 16;  // latent layers with at least this many heads run a decoded token's heads as one tensor-core tile
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
+// x[t, :] = table[id] * scale, and its copy of the engine dtype at h2[t * h2_ld + :] (optional: what the first projection reads)
+// (eight columns per thread and step where rows are whole 16-byte pieces: 20 us for 3085 rows of 2048 one by one, now 12)
 template <typename T>
-__global__ void embed_f32_kernel(const int *__restrict__ ids, const T *__restrict__ table, float *__restrict__ x, T *__restrict__ h, int width,
-                                 int vocab, float scale) {
+__global__ void embed_rows_kernel(const int *__restrict__ ids, const T *__restrict__ table, float *__restrict__ x, T *__restrict__ h2, int h2_ld,
+                                  int width, int vocab, float scale, bool vec) {
     const int t = blockIdx.x;
     int id = ids[t];
     id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);  // the host has refused ids outside the vocabulary
+    if (vec) {
+        for (int c = threadIdx.x * 8; c < width; c += blockDim.x * 8) {
+            float v[8];
+            load8<T>(table + (size_t)id * width + c, v);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] *= scale;
+            store8<float>(x + (size_t)t * width + c, v);
+            if (h2) store8<T>(h2 + (size_t)t * h2_ld + c, v);
+        }
+        return;
+    }
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         const float v = Elem<T>::to_f(table[(size_t)id * width + c]) * scale;
         x[(size_t)t * width + c] = v;
-        if (h) h[(size_t)t * width + c] = Elem<T>::from_f(v);  // the 16-bit copy the first projection reads
+        if (h2) h2[(size_t)t * h2_ld + c] = Elem<T>::from_f(v);
     }
 }
 
@@ -72,14 +86,16 @@ postnorm_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, c
                                          reinterpret_cast<size_t>(h_out)) & 15) == 0;
     float ss = 0.0f;
     if (vec) {
+        // A thread's first piece stays in registers, its row and gains on their way while the block sums: with x fetched behind the sum a CTA spent two
+        // memory round trips in a row.
         const float sg = (!y_dense && y_shared) ? shared_gate[t] : 0.0f;
-        for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) {
-            float v[V];
+        auto gather = [&](int c, float *v) {
             if (y_dense) {
                 unpack16<T>(ld_v4(y_dense + (size_t)t * width + c), v);
             } else {
 #pragma unroll
                 for (int i = 0; i < V; ++i) v[i] = 0.0f;
+#pragma unroll 4
                 for (int k = 0; k < top; ++k) {
                     float f[V];
                     unpack16<T>(ld_v4(y_rows + (size_t)pair_row[(size_t)t * top + k] * width + c), f);
@@ -94,43 +110,62 @@ postnorm_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, c
                 }
             }
 #pragma unroll
-            for (int i = 0; i < V; i += 4) *reinterpret_cast<float4 *>(ys + c + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-#pragma unroll
             for (int i = 0; i < V; ++i) ss = fmaf(v[i], v[i], ss);
-        }
-    } else {
-        for (int c = threadIdx.x; c < width; c += blockDim.x) {
-            float v;
-            if (y_dense) {
-                v = Elem<T>::to_f(y_dense[(size_t)t * width + c]);
-            } else {
-                v = 0.0f;
-                for (int k = 0; k < top; ++k) v += Elem<T>::to_f(y_rows[(size_t)pair_row[(size_t)t * top + k] * width + c]);
-                if (y_shared) v = fmaf(shared_gate[t], Elem<T>::to_f(y_shared[(size_t)t * width + c]), v);
-            }
-            ys[c] = v;
-            ss = fmaf(v, v, ss);
-        }
-    }
-    ss = block_sum(ss, red);
-    const float inv = rsqrtf(ss / (float)width + eps);
-    if (vec) {
-        for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) {  // a thread reads back the pieces of ys it wrote
+        };
+        auto finish = [&](int c, const float *xs, const float *gs, const float *y, float inv) {
             float v[V];
 #pragma unroll
+            for (int i = 0; i < V; ++i) v[i] = xs[i] + y[i] * inv * gs[i];
+#pragma unroll
             for (int i = 0; i < V; i += 4) {
-                const float4 xv = *reinterpret_cast<const float4 *>(x + (size_t)t * width + c + i);
-                const float4 gv = *reinterpret_cast<const float4 *>(g + c + i);
-                const float4 yv = *reinterpret_cast<const float4 *>(ys + c + i);
-                const float4 r = make_float4(xv.x + yv.x * inv * gv.x, xv.y + yv.y * inv * gv.y, xv.z + yv.z * inv * gv.z, xv.w + yv.w * inv * gv.w);
+                const float4 r = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 *reinterpret_cast<float4 *>(x + (size_t)t * width + c + i) = r;
                 if (trace) *reinterpret_cast<float4 *>(trace + (size_t)t * width + c + i) = r;
-                v[i] = r.x, v[i + 1] = r.y, v[i + 2] = r.z, v[i + 3] = r.w;
             }
             if (h_out) st_v4(h_out + (size_t)t * width + c, pack16<T>(v));  // what the next sublayer's projections read (16-bit engines)
+        };
+        auto fetch = [&](const float *from, float *v) {
+#pragma unroll
+            for (int i = 0; i < V; i += 4) load_n<float, 4>(from + i, v + i);
+        };
+        const int c0 = threadIdx.x * V;
+        float y0[V], x0[V], g0[V];
+        if (c0 < width) {
+            fetch(x + (size_t)t * width + c0, x0);
+            fetch(g + c0, g0);
+            gather(c0, y0);
+        }
+        for (int c = c0 + blockDim.x * V; c < width; c += blockDim.x * V) {
+            float v[V];
+            gather(c, v);
+#pragma unroll
+            for (int i = 0; i < V; i += 4) store_n<float, 4>(ys + c + i, v + i);
+        }
+        const float inv = rsqrtf(block_sum(ss, red) / (float)width + eps);
+        if (c0 < width) finish(c0, x0, g0, y0, inv);
+        for (int c = c0 + blockDim.x * V; c < width; c += blockDim.x * V) {  // a thread reads back the pieces of ys it wrote
+            float xs[V], gs[V], y[V];
+            fetch(x + (size_t)t * width + c, xs);
+            fetch(g + c, gs);
+            fetch(ys + c, y);
+            finish(c, xs, gs, y, inv);
         }
         return;
     }
+    for (int c = threadIdx.x; c < width; c += blockDim.x) {
+        float v;
+        if (y_dense) {
+            v = Elem<T>::to_f(y_dense[(size_t)t * width + c]);
+        } else {
+            v = 0.0f;
+            for (int k = 0; k < top; ++k) v += Elem<T>::to_f(y_rows[(size_t)pair_row[(size_t)t * top + k] * width + c]);
+            if (y_shared) v = fmaf(shared_gate[t], Elem<T>::to_f(y_shared[(size_t)t * width + c]), v);
+        }
+        ys[c] = v;
+        ss = fmaf(v, v, ss);
+    }
+    ss = block_sum(ss, red);
+    const float inv = rsqrtf(ss / (float)width + eps);
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         const float v = x[(size_t)t * width + c] + ys[c] * inv * g[c];
         x[(size_t)t * width + c] = v;
@@ -357,7 +392,7 @@ proj_f32_kernel(const TX *__restrict__ x, int ldx, const TW *__restrict__ w, con
 template <typename TX, typename TW>
 __global__ void __launch_bounds__(256)
 proj_f32_small_kernel(const TX *__restrict__ x, int ldx, const TW *__restrict__ w, const float *__restrict__ bias, float *__restrict__ y, int ldy,
-                      int M, int N, int K) {
+                      int M, int N, int K, bool vec) {
     const int o = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (o >= M * N) return;
     const int mrow = o / N, n = o - mrow * N;
@@ -365,6 +400,24 @@ proj_f32_small_kernel(const TX *__restrict__ x, int ldx, const TW *__restrict__ 
     const TW *wr = w + (size_t)n * K;
     float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
     int k = lane;
+    if (vec) {  // eight consecutive k per lane and step, all of a row's loads in flight (one value per load: 16 round trips for 2048 k, 10.5 us; now 7)
+        constexpr int U = 4;
+        for (int k0 = lane * 8; k0 < K; k0 += U * 256) {
+            float f[U][8], g[U][8];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {  // (past the row's end: its last piece, not used)
+                load8(xr + min(k0 + 256 * u, K - 8), f[u]);
+                load8(wr + min(k0 + 256 * u, K - 8), g[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (k0 + 256 * u >= K) break;
+                a0 = fmaf(f[u][0], g[u][0], a0), a1 = fmaf(f[u][1], g[u][1], a1), a2 = fmaf(f[u][2], g[u][2], a2), a3 = fmaf(f[u][3], g[u][3], a3);
+                a0 = fmaf(f[u][4], g[u][4], a0), a1 = fmaf(f[u][5], g[u][5], a1), a2 = fmaf(f[u][6], g[u][6], a2), a3 = fmaf(f[u][7], g[u][7], a3);
+            }
+        }
+        k = K;
+    }
     for (; k + 96 < K; k += 128) {
         a0 = fmaf(Elem<TX>::to_f(xr[k]), Elem<TW>::to_f(wr[k]), a0);
         a1 = fmaf(Elem<TX>::to_f(xr[k + 32]), Elem<TW>::to_f(wr[k + 32]), a1);
@@ -427,8 +480,9 @@ int launch_proj_f32(int x_dtype, const void *x, int ldx, int w_dtype, const void
     if ((long long)M * N <= 8192) {
         const int grid = (M * N + 7) / 8;
         B200_DISPATCH_DTYPE(w_dtype, {
-            if (x_dtype == B200_F32) proj_f32_small_kernel<float, T><<<grid, 256, 0, st>>>((const float *)x, ldx, (const T *)w, bias, y, ldy, M, N, K);
-            else proj_f32_small_kernel<T, T><<<grid, 256, 0, st>>>((const T *)x, ldx, (const T *)w, bias, y, ldy, M, N, K);
+            const bool vec = K % 8 == 0 && ldx % 8 == 0 && all_aligned16({x, w});
+            if (x_dtype == B200_F32) proj_f32_small_kernel<float, T><<<grid, 256, 0, st>>>((const float *)x, ldx, (const T *)w, bias, y, ldy, M, N, K, vec);
+            else proj_f32_small_kernel<T, T><<<grid, 256, 0, st>>>((const T *)x, ldx, (const T *)w, bias, y, ldy, M, N, K, vec);
         });
         return cuda_status("proj_f32 (small) launch");
     }
@@ -463,53 +517,68 @@ int launch_proj_f32(int x_dtype, const void *x, int ldx, int w_dtype, const void
 }
 
 // ---- layers of one norm whose sublayers all read it (B200_NORM_LN_PARALLEL)
-// x[t, :] = table[id] * scale, and its copy of the engine dtype at h2[t * h2_ld + :] (optional)
-template <typename T>
-__global__ void embed_rows_kernel(const int *__restrict__ ids, const T *__restrict__ table, float *__restrict__ x, T *__restrict__ h2, int h2_ld,
-                                  int width, int vocab, float scale) {
-    const int t = blockIdx.x;
-    int id = ids[t];
-    id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);  // the host has refused ids outside the vocabulary
-    for (int c = threadIdx.x; c < width; c += blockDim.x) {
-        const float v = Elem<T>::to_f(table[(size_t)id * width + c]) * scale;
-        x[(size_t)t * width + c] = v;
-        if (h2) h2[(size_t)t * h2_ld + c] = Elem<T>::from_f(v);
-    }
-}
-
 // The residual step of such a layer and whatever the next layer run reads, in one kernel:
 //   v = (replace ? y32[t, :] : x[t, :] + y[t, :]) + bias;   x[t, :] = v;   trace[t, :] = v;
 //   h_out[t * h_ld + :] = ln ? T((v - mean) * rsqrt(var + eps) * w + b) : T(v)        (ln packed [w | b]; var = mean of squared deviations)
 // y, y32, bias, trace and h_out are optional.  The row waits in shared memory between the passes: mean first, then the deviations.
-template <typename T>
+// (V: columns per access; every row starts on a boundary of them)
+template <typename T, int V>
 __global__ void __launch_bounds__(256)
 ln_residual_kernel(float *__restrict__ x, const T *__restrict__ y, const float *__restrict__ y32, const float *__restrict__ bias, int replace,
                    const float *__restrict__ ln, float eps, int width, T *__restrict__ h_out, int h_ld, float *__restrict__ trace) {
     extern __shared__ __align__(16) float row[];  // [width]
     __shared__ float red[33];
     const int t = blockIdx.x;
+    const size_t at = (size_t)t * width;
     float sum = 0.0f;
-    for (int c = threadIdx.x; c < width; c += blockDim.x) {
-        float v = replace ? y32[(size_t)t * width + c] : x[(size_t)t * width + c] + (y ? Elem<T>::to_f(y[(size_t)t * width + c]) : 0.0f);
-        if (bias) v += bias[c];
-        if (replace || y || bias) x[(size_t)t * width + c] = v;
-        if (trace) trace[(size_t)t * width + c] = v;
-        row[c] = v;
-        sum += v;
+#pragma unroll 2
+    for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) {
+        float v[V], d[V];
+        load_n<float, V>((replace ? y32 : x) + at + c, v);
+        if (!replace && y) {
+            load_n<T, V>(y + at + c, d);
+#pragma unroll
+            for (int e = 0; e < V; ++e) v[e] += d[e];
+        }
+        if (bias) {
+            load_n<float, V>(bias + c, d);
+#pragma unroll
+            for (int e = 0; e < V; ++e) v[e] += d[e];
+        }
+        if (replace || y || bias) store_n<float, V>(x + at + c, v);
+        if (trace) store_n<float, V>(trace + at + c, v);
+        store_n<float, V>(row + c, v);
+#pragma unroll
+        for (int e = 0; e < V; ++e) sum += v[e];
     }
     if (!h_out) return;
+    T *h = h_out + (size_t)t * h_ld;
     if (!ln) {
-        for (int c = threadIdx.x; c < width; c += blockDim.x) h_out[(size_t)t * h_ld + c] = Elem<T>::from_f(row[c]);  // (a thread reads what it wrote)
+        for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) store_n<T, V>(h + c, row + c);  // (a thread reads what it wrote)
         return;
     }
     const float mean = block_sum(sum, red) / (float)width;
     float sq = 0.0f;
-    for (int c = threadIdx.x; c < width; c += blockDim.x) {
-        const float d = row[c] - mean;
-        sq = fmaf(d, d, sq);
+    for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) {
+        float v[V];
+        load_n<float, V>(row + c, v);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            const float d = v[e] - mean;
+            sq = fmaf(d, d, sq);
+        }
     }
     const float inv = rsqrtf(block_sum(sq, red) / (float)width + eps);
-    for (int c = threadIdx.x; c < width; c += blockDim.x) h_out[(size_t)t * h_ld + c] = Elem<T>::from_f(fmaf((row[c] - mean) * inv, ln[c], ln[width + c]));
+#pragma unroll 2
+    for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) {
+        float v[V], w[V], b[V];
+        load_n<float, V>(ln + c, w);
+        load_n<float, V>(ln + width + c, b);
+        load_n<float, V>(row + c, v);
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[e] = fmaf((v[e] - mean) * inv, w[e], b[e]);
+        store_n<T, V>(h + c, v);
+    }
 }
 
 // out[r * out_ld + c] = T(act(in[r * in_ld + gate_col + c]) * in[r * in_ld + up_col + c]): the gated feed-forward's inner row, read from
@@ -857,6 +926,15 @@ Carve carve(const b200_hybrid *m) {
     k.total = k.chunk + k.vkeep + k.maps + k.turns + k.xs + k.x + k.f32a + k.f32b + k.xn + k.h + k.proj + 2 * k.mix + k.y + k.xg + k.u + k.yrows + k.us + k.ys + k.lqn + k.lqr + 2 * k.lql +
               k.lov + k.lpart + k.meta + k.moe_i + k.moe_f + k.rec + k.f32c + k.cat + k.xc;
     return k;
+}
+
+// y fp32 [M, N] = x [M, K] w[N, K]^T for up to 16 rows of a 16-bit engine: the weight-streaming GEMVs
+int launch_rows_f32out(int dtype, const void *x, const void *w, float *y, int M, int N, int K, cudaStream_t st) {
+    if (dtype == B200_F32) return B200_ERR_UNSUPPORTED;
+    GemvArgs a = {};
+    a.w = w, a.x = x, a.y = y, a.y_f32 = 1;
+    a.M = M, a.K = K, a.N = N;
+    return launch_gemv_nk(a, dtype, WF_DENSE, false, st);
 }
 
 int linear(const b200_hybrid *m, const void *x, const void *w, void *y, int M, int K, int N, cudaStream_t st) {
@@ -1313,8 +1391,9 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     // the residual step of a shared-norm layer; it also writes what the next run reads: its normed input, or (before an entry step) x itself
     auto ln_residual = [&](const void *y, const float *y32, const float *bias, const float *ln, void *h_out, int h_ld, float *trace) -> int {
         B200_DISPATCH_DTYPE(dt, {
-            ln_residual_kernel<T><<<NT, 256, (size_t)width * sizeof(float), st>>>(m->x, (const T *)y, y32, bias, y32 ? 1 : 0, ln, c.norm_eps, width,
-                                                                                (T *)h_out, h_ld, trace);
+            const bool vec = width % 4 == 0 && h_ld % 4 == 0 && all_aligned16({m->x, y, y32, bias, ln, h_out, trace});
+            (vec ? ln_residual_kernel<T, 4> : ln_residual_kernel<T, 1>)<<<NT, 256, (size_t)width * sizeof(float), st>>>(
+                m->x, (const T *)y, y32, bias, y32 ? 1 : 0, ln, c.norm_eps, width, (T *)h_out, h_ld, trace);
         });
         return cuda_status("ln_residual launch");
     };
@@ -1324,19 +1403,20 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         if (m->plan[run].entry >= 0) return ln_residual(y, nullptr, bias, nullptr, m->xc, 2 * width, trace);
         return ln_residual(y, nullptr, bias, m->layers[m->plan[run].layer].pre1, m->h, width, trace);
     };
-    if (shared_norm) {
+    auto embed = [&](void *h2, int h2_ld) -> int {
+        const bool vec = width % 8 == 0 && h2_ld % 8 == 0 && all_aligned16({m->embedding, m->x, h2});
         B200_DISPATCH_DTYPE(dt, {
-            embed_rows_kernel<T><<<NT, 128, 0, st>>>(d_ids, (const T *)m->embedding, m->x, c.loop_times > 0 ? (T *)m->xc + width : nullptr, 2 * width, width,
-                                                    c.vocab, c.embed_scale != 0.0f ? c.embed_scale : 1.0f);
+            embed_rows_kernel<T><<<NT, 256, 0, st>>>(d_ids, (const T *)m->embedding, m->x, (T *)h2, h2_ld, width, c.vocab, c.embed_scale != 0.0f ? c.embed_scale : 1.0f, vec);
         });
+        return cuda_status("embed_rows launch");
+    };
+    if (shared_norm) {
+        RUN(embed(c.loop_times > 0 ? (char *)m->xc + (size_t)width * (f32 ? 4 : 2) : nullptr, 2 * width));
         RUN(hand_over(0, nullptr, nullptr, nullptr));
     } else if (pre_norm) {
-        B200_DISPATCH_DTYPE(dt, {
-            embed_rows_kernel<T><<<NT, 128, 0, st>>>(d_ids, (const T *)m->embedding, m->x, (T *)nullptr, 0, width, c.vocab, c.embed_scale != 0.0f ? c.embed_scale : 1.0f);
-        });
+        RUN(embed(nullptr, 0));
     } else if (!sum_norm) {
-    B200_DISPATCH_DTYPE(dt, { embed_f32_kernel<T><<<NT, 128, 0, st>>>(d_ids, (const T *)m->embedding, m->x, f32 ? nullptr : (T *)m->h, width, c.vocab,
-                                                                      c.embed_scale != 0.0f ? c.embed_scale : 1.0f); });
+        RUN(embed(f32 ? nullptr : m->h, width));
     }
 
     // a recurrence over the batch: its token-parallel form for the long portions, where it takes the layer's sizes, and the serial form for the rest
@@ -1648,7 +1728,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                     const int r = launch_gemm_tc_grouped(a, w, out, l.heads * t_pad, N, K, l.heads, d_lat_head128, d_lat_n128 + li, -1, dt, st);
                     if (r != B200_ERR_UNSUPPORTED) return r;
                 }
-                return launch_moe_grouped_gemm(dt, a, w, out, d_lat_head, d_lat_n + li, l.heads * tph, N, K, -1, st);
+                return launch_moe_grouped_gemm(dt, a, w, out, d_lat_head, d_lat_n + li, l.heads * tph, N, K, -1, st, std::min(NT, kMoeTileM));  // (NT <= 16: one tile per head)
             };
             RUN(head_product(m->lqn, l.w_uk_t, m->lql, l.kv_rank, l.dim));  // q into the latent space: ql[h] = qn[h] . W_uk,h
             const int max_keys = l.window > 0 ? std::min(l.window, mpps * kPageH) : mpps * kPageH;
@@ -1752,13 +1832,13 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         const int up_act = l.gated ? -1 : l.act;
         char *inner = (char *)m->u;
         if (tc) RUN(launch_gemm_tc_grouped(m->xg, l.w_up, m->u, max_rows, n_up, width, l.experts, tile_expert, n_live, up_act, dt, st));
-        else RUN(launch_moe_grouped_gemm(dt, m->xg, l.w_up, m->u, tile_expert, n_live, max_tiles, n_up, width, up_act, st));
+        else RUN(launch_moe_grouped_gemm(dt, m->xg, l.w_up, m->u, tile_expert, n_live, max_tiles, n_up, width, up_act, st, std::min(NT, kMoeTileM)));  // (a token chooses an expert once)
         if (l.gated) {
             inner += (size_t)max_rows * n_up * es;
             RUN(launch_gated_activation(dt, m->u, inner, max_rows, l.expert_ff, l.act, n_live, tile, st, l.act_limit, l.act_slope));
         }
         if (tc) RUN(launch_gemm_tc_grouped(inner, l.w_down, m->yrows, max_rows, width, l.expert_ff, l.experts, tile_expert, n_live, -1, dt, st));
-        else RUN(launch_moe_grouped_gemm(dt, inner, l.w_down, m->yrows, tile_expert, n_live, max_tiles, width, l.expert_ff, -1, st));
+        else RUN(launch_moe_grouped_gemm(dt, inner, l.w_down, m->yrows, tile_expert, n_live, max_tiles, width, l.expert_ff, -1, st, std::min(NT, kMoeTileM)));
         if (l.shared_ff > 0) {
             char *sin = (char *)m->us;
             RUN(linear(m, h2, l.w_shared_up, m->us, NT, width, inner_cols * l.shared_ff, st));
@@ -1790,7 +1870,8 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             else if (c.final_norm == B200_NORM_DYT_PRE_POST) final_dyt_rows_kernel<T><<<W, 256, 0, st>>>(m->x, d_want, m->final_norm, m->xn, f32 ? nullptr : (T *)m->h, width);
             else final_norm_rows_kernel<T><<<W, 256, 0, st>>>(m->x, d_want, m->final_norm, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
         });
-        rc = launch_dense_f32out(dt, m->h, m->lm_head, logits, W, c.vocab, width, st);
+        rc = W <= 16 ? launch_rows_f32out(dt, m->h, m->lm_head, logits, W, c.vocab, width, st) : B200_ERR_UNSUPPORTED;
+        if (rc == B200_ERR_UNSUPPORTED) rc = launch_dense_f32out(dt, m->h, m->lm_head, logits, W, c.vocab, width, st);
         if (rc == B200_ERR_UNSUPPORTED) rc = launch_proj_f32(B200_F32, m->xn, width, dt, m->lm_head, nullptr, logits, c.vocab, W, c.vocab, width, st);
         if (rc != B200_OK) return rc;
         const float lscale = c.logit_scale != 0.0f ? c.logit_scale : 1.0f;

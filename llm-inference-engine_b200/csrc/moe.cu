@@ -90,43 +90,86 @@ __global__ void moe_route_softmax_kernel(const float *__restrict__ logits, int l
     for (int k = lane; k < top; k += 32) sel_weight[(size_t)t * top + k] *= norm;
 }
 
-// one CTA.  Shared: count[E] | offset[E+1] | cursor[E]
+// One CTA.  Every warp counts its own stretch of the pairs in counters of its own, U loads in flight per lane: one counter per expert for all of them and
+// one load at a time made two chains of round trips (4096 tokens x 4 of 32 experts 32 -> 21 us, 16 tokens 10 -> 5.6 us).  The order of an expert's rows is
+// free: every row is the same product wherever it lies.  Shared: counters [warps][E] | total [E] | offset [E + 1]
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int *__restrict__ sel_expert, const float *__restrict__ sel_weight, int *__restrict__ row_token, float *__restrict__ row_weight,
                 int *__restrict__ tile_expert, int *__restrict__ pair_row, int *__restrict__ n_tiles, int pairs, int experts, int top, int tile) {
     // choices >= experts (identity experts) own no row: pair_row = -1
     extern __shared__ int si[];
-    int *count = si, *offset = si + experts, *cursor = offset + experts + 1;
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0, cursor[e] = 0;
+    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int *count = si, *total = count + warps * experts, *offset = total + experts;
+    for (int i = threadIdx.x; i < warps * experts; i += blockDim.x) count[i] = 0;
     __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x)
-        if (sel_expert[p] < experts) atomicAdd(&count[sel_expert[p]], 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int at = 0;
-        for (int e = 0; e < experts; ++e) {
-            offset[e] = at;
-            const int tiles = (count[e] + tile - 1) / tile;
-            for (int i = 0; i < tiles; ++i) tile_expert[at / tile + i] = e;
-            at += tiles * tile;
+    int *mine = count + warp * experts;
+    const int per = ((pairs + warps - 1) / warps + 31) / 32 * 32, lo = warp * per, hi = min(pairs, lo + per);
+    constexpr int U = 16;  // loads in flight per lane: one at a time, a warp's stretch was a chain of round trips to L2 (36 us)
+    int ex[U];
+    auto fetch = [&](int p0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int p = p0 + 32 * u + lane, e = p < hi ? sel_expert[p] : experts;
+            ex[u] = e < experts ? e : -1;
         }
-        offset[experts] = at;
-        *n_tiles = at / tile;
+    };
+    for (int p0 = lo; p0 < hi; p0 += 32 * U) {
+        fetch(p0);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (p0 + 32 * u >= hi) break;
+            if (ex[u] >= 0) atomicAdd(mine + ex[u], 1);
+        }
     }
     __syncthreads();
-    const int rows = offset[experts];
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) row_token[r] = -1, row_weight[r] = 0.0f;
-    __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-        const int e = sel_expert[p];
-        if (e >= experts) {
-            pair_row[p] = -1;
-            continue;
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+        int run = 0;
+        for (int w = 0; w < warps; ++w) {
+            const int n = count[w * experts + e];
+            count[w * experts + e] = run;
+            run += n;
         }
-        const int r = offset[e] + atomicAdd(&cursor[e], 1);
-        row_token[r] = p / top;
-        row_weight[r] = sel_weight[p];
-        pair_row[p] = r;
+        total[e] = run;
+    }
+    __syncthreads();
+    if (warp == 0) {  // first row of every expert: a running sum of whole tiles
+        int at = 0;
+        for (int e0 = 0; e0 < experts; e0 += 32) {
+            const int rows = e0 + lane < experts ? (total[e0 + lane] + tile - 1) / tile * tile : 0;
+            int sum = rows;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += up;
+            }
+            if (e0 + lane < experts) offset[e0 + lane] = at + sum - rows;
+            at += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) offset[experts] = at, *n_tiles = at / tile;
+    }
+    __syncthreads();
+    for (int e = warp; e < experts; e += warps) {
+        const int first = offset[e], end = offset[e + 1];
+        for (int i = first / tile + lane; i < end / tile; i += 32) tile_expert[i] = e;
+        for (int r = first + total[e] + lane; r < end; r += 32) row_token[r] = -1, row_weight[r] = 0.0f;  // padding
+    }
+    for (int p0 = lo; p0 < hi; p0 += 32 * U) {
+        if (hi - lo > 32 * U) fetch(p0);  // (else: what the first pass read)
+        float wt[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) wt[u] = p0 + 32 * u + lane < hi ? sel_weight[p0 + 32 * u + lane] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (p0 + 32 * u >= hi) break;
+            const int p = p0 + 32 * u + lane, e = ex[u];
+            if (e >= 0) {
+                const int r = offset[e] + atomicAdd(mine + e, 1);
+                row_token[r] = p / top;
+                row_weight[r] = wt[u];
+                pair_row[p] = r;
+            } else if (p < hi) {
+                pair_row[p] = -1;
+            }
+        }
     }
 }
 
@@ -479,10 +522,83 @@ moe_grouped_gemm_mma_kernel(const T *__restrict__ a, const T *__restrict__ w, TC
             }
 }
 
+// The grouped GEMM of a decode batch (at most 16 tokens, so at most 16 live rows at the head of every expert's tile): the time is the experts' weights,
+// and the kernel above -- 64 x 128 tiles through a ring of three 64-k stages, one CTA walking all of K -- waits for memory at every stage (2048 x 512
+// experts, 28 touched: 40 us up, 30 us down, for 59 MB each).  Here a warp owns a slice of up to 256 k and holds the tile's rows of it as mma.sync A
+// fragments; it reads its 8 weight rows of a unit straight into registers, 16 bytes per lane and 32-k block (k permuted inside a block alike for both
+// operands: a lane's 8 consecutive k are its fragments of two k-steps), the next unit's pieces in flight while it multiplies this one's.  KS warps share a
+// unit's k and meet in shared memory, NG units of a CTA run side by side (KS * NG >= 8 warps).
+// grid (unit groups, tiles); a CTA runs `steps` groups of NG units of 8 rows.  NT 1: at most 8 live rows, 2: at most 16.  A tile's rows start at its
+// number times tile_rows; rows >= M are neither read nor stored.  tile_expert and n_tiles NULL: one weight, every tile of the grid.
+// Measured (2048 x 512 experts, 16 tokens x 4 of 32, 59 MB): up and down 40 and 30 -> 19 us each.
+template <typename T, typename TC, int NT>
+__global__ void __launch_bounds__(512)
+moe_few_rows_kernel(const T *__restrict__ a, const T *__restrict__ w, TC *__restrict__ c, const int *__restrict__ tile_expert,
+                    const int *__restrict__ n_tiles, int tile_rows, int M, int N, int K, int act, int KS, int NG, int steps) {
+    if (n_tiles && (int)blockIdx.y >= *n_tiles) return;
+    constexpr int NB = 8;  // 32-k blocks of a slice
+    extern __shared__ __align__(16) float part[];  // [2][NG][KS][16 tokens x 8 rows]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int ng = warp / KS, ks = warp - ng * KS, blocks = K / 32;
+    const int first = blocks * ks / KS, nb = blocks * (ks + 1) / KS - first;
+    const T *wb = w + (tile_expert ? (size_t)tile_expert[blockIdx.y] * N * K : 0) + first * 32 + 8 * t;
+    const int m0 = blockIdx.y * tile_rows;
+    const T *ar = a + (size_t)m0 * K + first * 32 + 8 * t;
+    const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
+    uint4 av[NB], bv[NT == 2 ? NB : 1], wq[NB];
+    auto row_of = [&](int step) {  // this warp's weight row g of the unit; rows past N read the last one, whose result is not stored
+        return wb + (size_t)min(((int)blockIdx.x * steps + step) * NG * 8 + ng * 8 + g, N - 1) * K;
+    };
+    const T *next = row_of(0);
+#pragma unroll
+    for (int j = 0; j < NB; ++j) wq[j] = j < nb ? ld_stream_v4(next + 32 * j) : zero4;
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+        av[j] = j < nb && m0 + g < M ? ld_v4(ar + (size_t)g * K + 32 * j) : zero4;
+        if constexpr (NT == 2) bv[j] = j < nb && m0 + g + 8 < M ? ld_v4(ar + (size_t)(g + 8) * K + 32 * j) : zero4;
+    }
+    for (int step = 0; step < steps; ++step) {
+        const int unit0 = ((int)blockIdx.x * steps + step) * NG;
+        if (unit0 * 8 >= N) break;
+        float acc[4] = {}, acc2[4] = {};
+        const bool more = step + 1 < steps;
+        next = row_of(step + 1);
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+            const uint4 b = NT == 2 ? bv[j] : zero4;
+            const unsigned a0[4] = {av[j].x, b.x, av[j].y, b.y}, a1[4] = {av[j].z, b.z, av[j].w, b.w};
+            moe_mma<T>((j & 1) ? acc2 : acc, a0, wq[j].x, wq[j].y);
+            moe_mma<T>((j & 1) ? acc2 : acc, a1, wq[j].z, wq[j].w);
+            if (more && j < nb) wq[j] = ld_stream_v4(next + 32 * j);
+        }
+        float *p = part + (size_t)(step & 1) * NG * KS * 128;
+        float *mine = p + (size_t)(ng * KS + ks) * 128;
+        *reinterpret_cast<float2 *>(mine + g * 8 + 2 * t) = make_float2(acc[0] + acc2[0], acc[1] + acc2[1]);
+        if constexpr (NT == 2) *reinterpret_cast<float2 *>(mine + (g + 8) * 8 + 2 * t) = make_float2(acc[2] + acc2[2], acc[3] + acc2[3]);
+        __syncthreads();  // (two buffers: the next step's shares do not wait for this one's sums)
+        for (int i = threadIdx.x; i < NG * 64 * NT; i += blockDim.x) {
+            const int u = i / (64 * NT), e = i - u * 64 * NT, n = (unit0 + u) * 8 + (e & 7);
+            float v = 0.0f;
+            for (int x = 0; x < KS; ++x) v += p[(size_t)(u * KS + x) * 128 + e];
+            if (n < N && m0 + (e >> 3) < M) c[(size_t)(m0 + (e >> 3)) * N + n] = Elem<TC>::from_f(act >= 0 ? act_apply(v, act) : v);
+        }
+    }
+}
+
 // y fp32 [M, N] = x [M, K] (16-bit) * w[N, K]^T on the tensor cores, fp32 accumulation and fp32 result
 int launch_dense_f32out(int dtype, const void *x, const void *w, float *y, int M, int N, int K, cudaStream_t st) {
     if (M == 0) return B200_OK;
     if (dtype == B200_F32 || K % 8 != 0) return B200_ERR_UNSUPPORTED;
+    // few columns (a router's outputs): one tile of 64 rows per CTA would leave most SMs idle while each of its CTAs walks all of K; 16 rows per CTA, K
+    // shared by its warps (4096 rows x 33 columns of 2048 k: 35 -> 10 us)
+    if (N <= 128 && K % 32 == 0 && K >= 512 && K <= 4096 && aligned16(x) && aligned16(w)) {
+        const int KS = (K / 32 + 7) / 8, NG = KS >= 8 ? 1 : 8 / KS, steps = ((N + 7) / 8 + NG - 1) / NG;
+        const size_t smem = (size_t)2 * NG * KS * 128 * sizeof(float);
+        const dim3 few(1, (M + 15) / 16);
+        if (dtype == B200_BF16) moe_few_rows_kernel<__nv_bfloat16, float, 2><<<few, KS * NG * 32, smem, st>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
+        else moe_few_rows_kernel<__half, float, 2><<<few, KS * NG * 32, smem, st>>>((const __half *)x, (const __half *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
+        return cuda_status("dense_f32out (few columns) launch");
+    }
     const dim3 grid((N + kMN - 1) / kMN, (M + kMoeTileM - 1) / kMoeTileM);
     const size_t smem = (size_t)kMStages * (kMoeTileM + kMN) * kMK * 2;
     if (dtype == B200_BF16) {
@@ -564,8 +680,11 @@ int launch_poly_norm(int dtype, void *x, const float *coef, float eps, int rows,
 
 int launch_moe_plan(const int *sel_expert, const float *sel_weight, int *row_token, float *row_weight, int *tile_expert, int *pair_row,
                     int *n_tiles, int tokens, int experts, int top, int tile, cudaStream_t st) {
-    moe_plan_kernel<<<1, 1024, (size_t)(3 * experts + 1) * sizeof(int), st>>>(sel_expert, sel_weight, row_token, row_weight, tile_expert,
-                                                                             pair_row, n_tiles, tokens * top, experts, top, tile);
+    const int pairs = tokens * top;
+    const int warps = std::max(1, std::min({32, std::max(8, (pairs + 31) / 32), (int)(40 * 1024 / sizeof(int) / std::max(experts, 1))}));
+    const size_t smem = ((size_t)(warps + 2) * experts + 1) * sizeof(int);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    moe_plan_kernel<<<1, warps * 32, smem, st>>>(sel_expert, sel_weight, row_token, row_weight, tile_expert, pair_row, n_tiles, pairs, experts, top, tile);
     return cuda_status("moe_plan launch");
 }
 
@@ -577,8 +696,22 @@ int launch_moe_gather(int dtype, const float *x, const int *row_token, const flo
 }
 
 int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, const int *tile_expert, const int *n_tiles, int max_tiles,
-                            int N, int K, int act, cudaStream_t st) {
+                            int N, int K, int act, cudaStream_t st, int live_rows) {
     if (max_tiles == 0) return B200_OK;
+    // a decode batch: up to 16 live rows per tile, slices of K for 16 warps at most, whole 32-k blocks
+    if (dtype != B200_F32 && live_rows <= 16 && K % 32 == 0 && K <= 4096 && K >= 64 && N % 8 == 0 && aligned16(a) && aligned16(w)) {
+        const int KS = (K / 32 + 7) / 8, NG = KS >= 8 ? 1 : 8 / KS;
+        const int units = (N / 8 + NG - 1) / NG, steps = std::max(1, std::min(8, units * max_tiles / (4 * sm_count())));
+        const dim3 grid((units + steps - 1) / steps, max_tiles);
+        const size_t smem = (size_t)2 * NG * KS * 128 * sizeof(float);
+        auto go = [&](auto kern, auto *type) {
+            using T = std::remove_pointer_t<decltype(type)>;
+            kern<<<grid, KS * NG * 32, smem, st>>>((const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, kMoeTileM, max_tiles * kMoeTileM, N, K, act, KS, NG, steps);
+        };
+        if (dtype == B200_BF16) live_rows <= 8 ? go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 1>, (__nv_bfloat16 *)nullptr) : go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 2>, (__nv_bfloat16 *)nullptr);
+        else live_rows <= 8 ? go(moe_few_rows_kernel<__half, __half, 1>, (__half *)nullptr) : go(moe_few_rows_kernel<__half, __half, 2>, (__half *)nullptr);
+        return cuda_status("moe_few_rows launch");
+    }
     if (dtype != B200_F32 && K % 8 == 0) {
         const dim3 grid((N + kMN - 1) / kMN, max_tiles);
         const size_t smem = (size_t)kMStages * (kMoeTileM + kMN) * kMK * 2;
