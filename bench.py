@@ -579,13 +579,13 @@ def tp_parity_check(args, mod, tpmod, dist, dev, rank, world, fused):
 def dominant_linear_kernel(batch, wformat):
     """Name of the kernel the weight-streaming linears of a decode step dispatch to (decoder.cu norm_linear / plain_linear, gemv_f32.cu,
     linear.cu)."""
-    if batch == 1 or (wformat != "bf16" and batch <= 4):
-        return "gemv_nk_kernel" if wformat == "bf16" else "gemv_q_kernel"
+    if batch == 1 and wformat == "bf16":
+        return "gemv_nk_kernel"
     if batch <= 16:
-        return "gemv_mma_kernel"
+        return "gemv_rs_kernel"
     if wformat == "bf16":
         return "gemm_tc_kernel (tcgen05, swap-AB + stream-K)" if batch <= 128 else "gemm_tc_kernel (tcgen05)"
-    return "gemv_mma_kernel (passes of <= 16 tokens)" if batch <= 64 else "generic SIMT fallback"
+    return "gemv_rs_kernel (passes of <= 16 tokens)" if batch <= 64 else "generic SIMT fallback"
 
 
 def run_prefill(args, cfg, mod, dec, dev, dt, kc, vc, rank):
@@ -1644,10 +1644,10 @@ def main():
                 tmp_vals=torch.empty((B, 8, K_TOP), dtype=torch.float32, device=dev), topk_ids=torch.empty((B, K_TOP), dtype=torch.int32, device=dev),
                 topk_vals=torch.empty((B, K_TOP), dtype=torch.float32, device=dev), seq_len=torch.full((B,), ctx, dtype=torch.int32, device=dev),
                 finished=torch.zeros(B, dtype=torch.uint8, device=dev), output_id=torch.zeros(B, dtype=torch.int32, device=dev))
-    # embedding, per layer [norm,] QKV, attention, O, [norm,] gate/up, down (the two norms are fused into the GEMVs at batch 1), fold,
-    # [final norm,] LM head (16 tokens per pass), top-k x 2, sampling
-    fused_norm = B == 1 or (args.wformat != "bf16" and B <= 4)
-    launches_per_step = 1 + L * (5 if fused_norm else 7) + 1 + ((1 if B == 1 else 1 + (B + 15) // 16)) + 2 + 1
+    # embedding, per layer [norm,] QKV, attention, O, [norm,] gate/up, down (the two norms are fused into the dense GEMVs at batch 1), fold,
+    # [final norm,] LM head (16 tokens per pass), top-k x 2 (the second draws the sample)
+    fused_norm = B == 1 and args.wformat == "bf16"
+    launches_per_step = 1 + L * (5 if fused_norm else 7) + 1 + ((1 if B == 1 else 1 + (B + 15) // 16)) + 2
     tp_mode = "none"
     if tp > 1:
         tp_mode = "nccl all-reduce"
@@ -1668,7 +1668,7 @@ def main():
     sharded_head = None
     if tp > 1 and V % tp == 0 and not os.environ.get("B200_TP_REPLICATED_HEAD"):
         sharded_head = tpmod.VocabShardedHead(mod, dec, tpmod.shard_lm_head_rows(lm_head, rank, tp), V, rank, tp, B, K_TOP, dev)
-        launches_per_step += 8  # local top-k x 2, pack x 2, candidate copies x 2, index widen + gather (torch), merge top-k x 2 - replaced tail
+        launches_per_step += 9  # local top-k x 2, sampling, pack x 2, candidate copies x 2, index widen + gather (torch), merge top-k x 2 - replaced tail
 
     if args.mode == "prefill":
         run_prefill(args, cfg, mod, dec, dev, dt, kc, vc, rank)

@@ -126,14 +126,14 @@ __global__ void tp_begin_step_kernel(unsigned int *epoch) {
 // rows one fused GEMV launch can take: 16 for 16-bit models (tensor-core GEMV, gemv_mma.cuh), 4 for fp32 (SIMT GEMV)
 static int gemv_max_rows(const b200_decoder_config_t &c) { return c.dtype != B200_F32 ? 16 : 4; }
 
-// prologue (add residual / bias / RMSNorm) + linear (+ SwiGLU): fused GEMV for one token (fp32: up to 4), un-fused otherwise.
+// prologue (add residual / bias / RMSNorm) + linear (+ SwiGLU): fused GEMV for one dense token (fp32: up to 4), un-fused otherwise.
 // tp (optional): x is the fused all-reduce of every rank's partial (TpExchange) instead of a local tensor.
 static int norm_linear(b200_decoder *d, const void *x, const void *res_in, void *res_out, const void *bias, const void *gamma,
                        const b200_linear_weight_t &w, int K, int N, bool swiglu, void *y, int M, cudaStream_t st, const TpExchange *tp = nullptr) {
     const b200_decoder_config_t &c = d->cfg;
     const bool b16 = c.dtype != B200_F32;
-    // one token (any dtype), fp32 up to 4: the prologue runs inside the GEMV (SIMT kernels / gemv_q.cuh)
-    if (M == 1 || (!b16 && M <= 4)) {
+    // one dense token, fp32 up to 4 tokens: the prologue runs inside the GEMV (SIMT kernels)
+    if ((M == 1 && c.w_format == B200_W_DENSE) || (!b16 && M <= 4)) {
         GemvArgs a = {};
         a.w = w.w, a.scales = w.scales, a.zeros = w.zeros;
         a.x = x, a.y = y;

@@ -7,8 +7,6 @@ int launch_gemv_nk_bf16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st
 int launch_gemv_nk_f16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
 int launch_gemv_mma_bf16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
 int launch_gemv_mma_f16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
-int launch_gemv_q_bf16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
-int launch_gemv_q_f16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
 int launch_gemv_rs_bf16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
 int launch_gemv_rs_f16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
 int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStream_t st) {
@@ -17,21 +15,17 @@ int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStrea
         return B200_ERR_INVALID_ARG;
     }
     const bool b16 = dtype == B200_BF16 || dtype == B200_F16;
-    // 16-bit activations, 2..16 tokens, no prologue: the weights stream past activations in registers (gemv_rs.cuh; one token of quantised weights keeps the
-    // kernel with the prologue below, one dense token the SIMT kernel: a single row leaves the matrix instructions seven eighths empty)
-    if (b16 && a.M >= 2 && a.M <= 16) {
+    // 16-bit activations, no prologue: 2..16 tokens, and one token of quantised weights, past which the weights stream with the activations in registers
+    // (gemv_rs.cuh).  One dense token keeps the SIMT kernel and its fused norm: its weights alone fill the memory pipe, and the norm launch would come on
+    // top.  One quantised token, 4 layers, norm kernel + gemv_rs against the kernel with the fused norm that was here: 7B size FP8 266 / INT4 276 us against
+    // 262 / 280, 70B-shaped shard 227 / 236 against 250 / 271, 2048-wide 149 / 148 against 162 / 171.
+    if (b16 && (a.M >= 2 || fmt != WF_DENSE) && a.M <= 16) {
         const int rc = dtype == B200_BF16 ? launch_gemv_rs_bf16(a, fmt, swiglu, st) : launch_gemv_rs_f16(a, fmt, swiglu, st);
         if (rc != B200_ERR_UNSUPPORTED) return rc;
     }
-    // shapes whose ring does not fit beside it: activations in shared memory (gemv_mma.cuh)
-    if (b16 && a.M >= 2 && a.M <= 16) {
+    // what its ring leaves out (rows of more than 4096 k with so many outputs that their sums fill the SM): activations in shared memory (gemv_mma.cuh)
+    if (b16 && (a.M >= 2 || fmt != WF_DENSE) && a.M <= 16) {
         const int rc = dtype == B200_BF16 ? launch_gemv_mma_bf16(a, fmt, swiglu, st) : launch_gemv_mma_f16(a, fmt, swiglu, st);
-        if (rc != B200_ERR_UNSUPPORTED) return rc;
-    }
-    // weight-only quantised, 16-bit activations, one token (more where the kernels above refuse): dequant into mma fragments with the SIMT GEMV's fused
-    // prologue (gemv_q.cuh)
-    if (b16 && fmt != WF_DENSE && a.M <= 8) {
-        const int rc = dtype == B200_BF16 ? launch_gemv_q_bf16(a, fmt, swiglu, st) : launch_gemv_q_f16(a, fmt, swiglu, st);
         if (rc != B200_ERR_UNSUPPORTED) return rc;
     }
     if (a.M > 4) return B200_ERR_UNSUPPORTED;

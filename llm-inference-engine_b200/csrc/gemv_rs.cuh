@@ -13,7 +13,7 @@
 //   * rows longer than the slices reach (K > 4096) go in parts, the reducer adding the parts' tiles in shared memory.
 // The reducer adds the 16 warps' tiles in a fixed order (deterministic), applies the FP8 row scale / SwiGLU and stores, or pushes the tensor-parallel
 // partial, as in gemv_mma.cuh.
-// Measured, 4 layers of 7B size, us per decode step (gemv_mma.cuh / gemv_q.cuh before -> now): dense 2 tokens 430 -> 370, 8: 435 -> 375, 16 ragged 517 -> 447;
+// Measured, 4 layers of 7B size, us per decode step (the kernels before -> now): dense 2 tokens 430 -> 370, 8: 435 -> 375, 16 ragged 517 -> 447;
 // FP8 2: 328 -> 263, 4: 382 -> 261, 8: 388 -> 280, 16 ragged 520 -> 382; INT4 2: 383 -> 273, 4: 433 -> 276, 8: 573 -> 296, 16: 617 -> 451.  The gate / up
 // linear of 16 FP8 tokens (90 MB): 41 -> 25 us.  A norm on the fragments in front of the product was slower than a norm kernel: every CTA redid all rows
 // (16 dense tokens 490 against 449).

@@ -1,8 +1,10 @@
 #!/usr/bin/env python
 """Which kernel, how many passes over the weights and which ring geometry each linear of a decode step gets -- a Python MODEL of the host-side
 dispatch (no GPU): decoder.cu norm_linear / plain_linear (fused GEMV for M <= gemv_max_rows, un-fused otherwise), linear.cu:300-330
-(tcgen05 GEMM for dense M > 4, else GEMV passes of 8 / 4 rows), gemv_inst.cuh:32-60 (gemv_nk geometry) and gemv_q.cuh launch_gemv_q_inst.
-It restates those few formulas; when they change, this file must follow (tests/test_dispatch_plan.py pins the cases measured on the B200).
+(tcgen05 GEMM for dense M > 4, else GEMV passes of 8 / 4 rows), gemv_inst.cuh:32-60 (gemv_nk geometry) and gemv_rs.cuh gemv_rs_geometry.
+It restates those few formulas; when they change, this file must follow.  linear_plan is the dispatch without gemv_rs -- gemv_mma.cuh, which still takes
+what gemv_rs refuses, and the quantised GEMV with the fused prologue, whose place gemv_rs has taken -- and is kept for reading the profiles measured with
+it (tests/test_dispatch_plan.py pins those cases); decode_plan is the dispatch of today.
 usage: python scripts/dispatch_plan.py > profiles/<tag>_dispatch_plan.txt"""
 BUDGET = 224 * 1024
 GROUPS, GW, MAX_STAGES, ROWS, PIECE = 2, 8, 8, 2, 8192
@@ -101,6 +103,41 @@ def gemv_any(M, K, fmt):
     return gemv_nk_plan(M, K, fmt)
 
 
+RS_BLOCKS, RS_STAGES, SMS = 8, 12, 148
+
+
+def gemv_rs_plan(M, K, N, fmt, swiglu=False):
+    """gemv_rs.cuh gemv_rs_geometry (16-bit activations, 1..16 tokens): None when unsupported."""
+    if M < 1 or M > 16 or K % 128 or (fmt == "dense" and M == 1):
+        return None
+    dense, nt = fmt == "dense", 2 if M > 8 else 1
+    rows = 8 if dense else 16
+    units = -(-(N // 2) // (rows // 2)) if swiglu else -(-N // rows)
+    max_units = -(-units // max(1, min(SMS, units)))
+    groups = K // 128
+    parts = -(-groups * 4 // (MMA_WARPS * RS_BLOCKS))
+    part_k = -(-groups // parts) * 128
+    parts = -(-K // part_k)
+    row = {"dense": part_k * 2, "fp8": part_k, "int4": part_k // 2}[fmt]
+    stage = rows * (-(-row // 128) * 128 + (16 if fmt == "fp8" else 64))
+    tile, vals = (128, 128) if dense else (8 * nt * 20, 128 * nt)
+    fixed = (2 * RS_STAGES + 4) * 8 + 2 * MMA_WARPS * tile * 4 + (max_units * vals * 4 if parts > 1 else 0)
+    if fixed + 2 * stage > 226 * 1024:
+        return None
+    return dict(kernel="gemv_rs", pieces=parts, piece_bytes=row, stages=min((226 * 1024 - fixed) // stage, RS_STAGES), parts=parts, part_k=part_k)
+
+
+def decode_plan(M, K, N, fmt, fused_rows, swiglu=False):
+    """One linear of the decode step as gemv_f32.cu / linear.cu dispatch it: (path, passes over the weights, geometry)."""
+    step = M if M <= fused_rows else 16
+    plans = [gemv_rs_plan(min(step, M - m0), K, N, fmt, swiglu) for m0 in range(0, M, step)]
+    if all(plans) and (M <= fused_rows or (fmt != "dense" and M <= 64)):
+        if M <= fused_rows:
+            return ("norm_kernel + gemv_rs", 1, plans[0])
+        return (f"un-fused gemv_rs x {len(plans)} passes of <= {step} tokens", len(plans), plans[0])
+    return linear_plan(M, K, fmt, fused_rows)
+
+
 def linear_plan(M, K, fmt, fused_rows):
     """One linear of the decode step: (path, passes over the weights, geometry)."""
     if M <= fused_rows:
@@ -128,7 +165,7 @@ def step_plan(name, hidden, heads, kv_heads, d, inter, tp, batch, fmt):
               ("down", inter // tp, hidden)]
     lines = [f"{name}, batch {batch}, weights {fmt}" + (f", TP-{tp} (one rank)" if tp > 1 else "")]
     for lin, K, N in shapes:
-        path, passes, g = linear_plan(batch, K, fmt, fused_rows)
+        path, passes, g = decode_plan(batch, K, N, fmt, fused_rows, lin == "gate_up")
         geo = (f"pieces {g['pieces']} x {g['piece_bytes']} B, {g['stages']} stages" + (f", {g['parts']} activation parts of {g['part_k']} k" if g.get("parts") else "")) if g else "-"
         wbytes = K * N * {"dense": 2, "fp8": 1, "int4": 0.5}[fmt]
         lines.append(f"  {lin:8s} K={K:6d} N={N:6d}  {path:58s} weights read {passes} x {wbytes / 1e6:7.1f} MB   {geo}")
