@@ -19,6 +19,8 @@ __global__ void __launch_bounds__(256)
 attn_qk_norm_cache_kernel(const T *__restrict__ proj, int ld, T *__restrict__ q_out, T *__restrict__ k_pool, T *__restrict__ v_pool,
                           const float *__restrict__ q_norm, const float *__restrict__ k_norm, float eps, const int *__restrict__ tok_seq,
                           const int *__restrict__ tok_pos, const int *__restrict__ block_table, int mpps, int heads, int kv_heads, int dim) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[33];
     const int t = blockIdx.x;
     const int nq = heads * dim, nk = kv_heads * dim;
@@ -100,6 +102,8 @@ chunked_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const
                     const T *__restrict__ gate_in, int gate_ld, T *__restrict__ out, const int *__restrict__ tok_seq,
                     const int *__restrict__ tok_pos, const int *__restrict__ block_table, int mpps, int heads, int kv_heads, int dim,
                     float scale, int chunk, int max_keys, const int *__restrict__ tok_list) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ float sm[];
     const int t = tok_list ? tok_list[blockIdx.x] : blockIdx.x, h = blockIdx.y;
     const int g = h / (heads / kv_heads);
@@ -305,6 +309,8 @@ __global__ void __launch_bounds__(128)
 chunked_attn_mma_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const T *__restrict__ v_pool, const float *__restrict__ sink,
                         const T *__restrict__ gate_in, int gate_ld, T *__restrict__ out, const int4 *__restrict__ tiles,
                         const int *__restrict__ block_table, int mpps, int heads, int kv_heads, float scale, int chunk) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     T *qs = reinterpret_cast<T *>(smraw);     // [64][D]
     T *ks = qs + kTileQ * D;                  // [2][64][D]
@@ -457,7 +463,7 @@ static int launch_mma_t(const void *q, const void *k_pool, const void *v_pool, c
                         cudaStream_t st) {
     const size_t smem = (size_t)(kTileQ + 4 * kPage) * D * sizeof(T);
     cudaFuncSetAttribute(chunked_attn_mma_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    chunked_attn_mma_kernel<T, D><<<dim3(n_tiles, heads), 128, smem, st>>>((const T *)q, (const T *)k_pool, (const T *)v_pool, sink, (const T *)gate_in,
+    launch_pdl(chunked_attn_mma_kernel<T, D>, dim3(n_tiles, heads), dim3(128), smem, st, true, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink, (const T *)gate_in,
                                                                             gate_ld, (T *)out, (const int4 *)tiles, block_table, mpps, heads, kv_heads,
                                                                             scale, chunk);
     return cuda_status("chunked_attention (tensor core) launch");
@@ -493,7 +499,7 @@ int launch_attn_qk_norm_cache(int dtype, const void *proj, int ld, void *q_out, 
                               int tokens, int heads, int kv_heads, int dim, cudaStream_t st) {
     if (tokens == 0) return B200_OK;
     B200_DISPATCH_DTYPE(dtype, {
-        attn_qk_norm_cache_kernel<T><<<tokens, 256, 0, st>>>((const T *)proj, ld, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
+        launch_pdl(attn_qk_norm_cache_kernel<T>, dim3(tokens), dim3(256), 0, st, true, (const T *)proj, ld, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
                                                               tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim);
     });
     return cuda_status("attn_qk_norm_cache launch");
@@ -513,7 +519,7 @@ int launch_chunked_attention(int dtype, const void *q, const void *k_pool, const
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(chunked_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        chunked_attn_kernel<T><<<dim3(tokens, heads), threads, smem, st>>>((const T *)q, (const T *)k_pool, (const T *)v_pool, sink,
+        launch_pdl(chunked_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, true, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink,
                                                                             (const T *)gate_in, gate_ld, (T *)out, tok_seq, tok_pos,
                                                                             block_table, mpps, heads, kv_heads, dim, scale, chunk, max_keys, tok_list);
     });

@@ -31,6 +31,8 @@ scored_prep_kernel(const T *__restrict__ proj, int ld, int col0, const float *__
                    const int *__restrict__ tok_seq, const int *__restrict__ tok_pos, const int *__restrict__ block_table, int mpps, int heads,
                    int kv_heads, int dim, int vdim, int rot_dims, float rot_base, ScoredPrepOptions opt, T *__restrict__ v_keep,
                    const T *__restrict__ v_mix, float lambda) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ float rot[];  // cos [rot_dims/2] | sin [rot_dims/2]
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const int pos = tok_pos[t], half = rot_dims / 2;
@@ -117,6 +119,8 @@ scored_prep_vec_kernel(const T *__restrict__ proj, int ld, int col0, T *__restri
                        const float *__restrict__ q_norm, const float *__restrict__ k_norm, float eps, const int *__restrict__ tok_seq,
                        const int *__restrict__ tok_pos, const int *__restrict__ block_table, int mpps, int heads, int kv_heads, int dim, int vdim,
                        T *__restrict__ v_keep, const T *__restrict__ v_mix, float lambda) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int V = Elem<T>::kVec;
     const int t = blockIdx.x, pos = tok_pos[t], per = dim / V, n_qk = (heads + kv_heads) * per, n_v = kv_heads * vdim / V;
     const T *row = proj + (size_t)t * ld + col0;
@@ -189,6 +193,8 @@ scored_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const 
                    T *__restrict__ out, int out_ld, float out_scale, const int *__restrict__ tok_seq, const int *__restrict__ tok_pos,
                    const int *__restrict__ block_table, int mpps, int heads, int kv_heads, int dim, int vdim, float scale, int window,
                    int sigmoid, int max_keys, int part_floats, const int *__restrict__ tok_list, ScoredOptions opt) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ float sm[];
     const int t = tok_list ? tok_list[blockIdx.x] : blockIdx.x, h = blockIdx.y;
     const int g = h / (heads / kv_heads);
@@ -380,6 +386,8 @@ scored_attn_mma_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, co
                        const float *__restrict__ dist_r1, const float *__restrict__ dist_r2, const T *__restrict__ gate_in, int gate_ld,
                        T *__restrict__ out, int out_ld, float out_scale, const int4 *__restrict__ tiles, const int *__restrict__ block_table,
                        int mpps, int heads, int kv_heads, float scale, int window, int pen_len, ScoredOptions opt) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     T *qs = reinterpret_cast<T *>(smraw);       // [64][DK]
     T *ks = qs + kTileQS * DK;                  // [2][64][DK]
@@ -578,7 +586,7 @@ static int launch_scored_mma_t(const void *q, const void *k_pool, const void *v_
     const size_t smem = (size_t)(kTileQS + 2 * kPageS) * DK * sizeof(T) + (size_t)2 * kPageS * DV * sizeof(T) + (size_t)pen_len * sizeof(float);
     auto kern = sigmoid ? scored_attn_mma_kernel<T, DK, DV, 1> : scored_attn_mma_kernel<T, DK, DV, 0>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<dim3(n_tiles, heads), 128, smem, st>>>((const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, r1, r2, (const T *)gate_in, gate_ld,
+    launch_pdl(kern, dim3(n_tiles, heads), dim3(128), smem, st, true, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, r1, r2, (const T *)gate_in, gate_ld,
                                                   (T *)out, out_ld, out_scale, (const int4 *)tiles, block_table, mpps, heads, kv_heads, scale, window,
                                                   pen_len, opt);
     return cuda_status("scored_attention (tensor core) launch");
@@ -626,13 +634,12 @@ int launch_scored_prep(int dtype, const void *proj, int ld, int col0, const floa
         const int per = dim / V;
         if (rot_dims == 0 && !b_in && !opt.v_norm && dim % V == 0 && per <= 32 && (per & (per - 1)) == 0 && vdim % V == 0 && ld % V == 0 && col0 % V == 0 &&
             (q_norm == nullptr) == (k_norm == nullptr) && all_aligned16({proj, q_out, k_pool, v_pool, q_norm, k_norm, share.v_keep, share.v_mix})) {
-            scored_prep_vec_kernel<T><<<tokens, 128, 0, st>>>((const T *)proj, ld, col0, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
+            launch_pdl(scored_prep_vec_kernel<T>, dim3(tokens), dim3(128), 0, st, true, (const T *)proj, ld, col0, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
                                                               tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim, vdim, (T *)share.v_keep,
                                                               (const T *)share.v_mix, share.lambda);
             return cuda_status("scored_prep (vector) launch");
         }
-        scored_prep_kernel<T><<<tokens, 256, (size_t)std::max(rot_dims, 2) * sizeof(float), st>>>(
-            (const T *)proj, ld, col0, b_in, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps, tok_seq, tok_pos, block_table, mpps, heads,
+        launch_pdl(scored_prep_kernel<T>, dim3(tokens), dim3(256), (size_t)std::max(rot_dims, 2) * sizeof(float), st, true, (const T *)proj, ld, col0, b_in, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps, tok_seq, tok_pos, block_table, mpps, heads,
             kv_heads, dim, vdim, rot_dims, rot_base, opt, (T *)share.v_keep, (const T *)share.v_mix, share.lambda);
     });
     return cuda_status("scored_prep launch");
@@ -653,8 +660,7 @@ int launch_scored_attention(int dtype, const void *q, const void *k_pool, const 
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(scored_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        scored_attn_kernel<T><<<dim3(tokens, heads), threads, smem, st>>>(
-            (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, dist_r1, dist_r2, (const T *)gate_in, gate_ld, (T *)out, out_ld, out_scale,
+        launch_pdl(scored_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, true, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, dist_r1, dist_r2, (const T *)gate_in, gate_ld, (T *)out, out_ld, out_scale,
             tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim, vdim, scale, window, sigmoid, max_keys, (int)part, tok_list, opt);
     });
     return cuda_status("scored_attention launch");

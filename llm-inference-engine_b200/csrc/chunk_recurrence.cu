@@ -72,6 +72,8 @@ template <int CH> __device__ __forceinline__ void load_channels(const float *p, 
 template <typename TQ, int DK, bool DELTA>
 __global__ void __launch_bounds__(256)
 chunk_factors_kernel(const ChunkSource src, const ChunkMap map, float *__restrict__ blocks) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int P = DK + 4;  // row pitch: rows read by neighbouring lanes start four banks apart
     constexpr int CH = DK / 32;
     extern __shared__ __align__(16) float sm[];
@@ -266,6 +268,8 @@ __device__ __forceinline__ void cp16(void *smem, const void *gmem) {
 template <typename TQ, int DK, bool DELTA>
 __global__ void __launch_bounds__(DK * 2)
 chunk_scan_kernel(const ChunkSource src, const ChunkMap map, const float *__restrict__ blocks, float *__restrict__ state, float *__restrict__ o, int stages) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int NW = DK / 16, NT = NW * 32;
     constexpr int NY = DELTA ? 8 : 4;                         // 8-row tiles of [Kp; Qp] (linear attention: Qp alone)
     constexpr int VP = sizeof(TQ) == 2 ? 24 : 20;             // elements per staged value row (16-byte pieces, rows off the same bank)
@@ -439,8 +443,8 @@ int launch_chunks_t(const ChunkSource &src, ChunkMap map, float *scratch, size_t
     cudaFuncSetAttribute(sk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * stage + rest));
     for (map.first = 0; map.first < chunks; map.first += map.count) {
         const int n = std::min(map.count, chunks - map.first);
-        fk<<<dim3(n, map.heads, n_seqs), 256, smem_f, st>>>(src, map, scratch);
-        sk<<<dim3(map.vdim / kCols, map.heads, n_seqs), DK * 2, stages * stage + rest, st>>>(src, map, scratch, state, o, stages);
+        launch_pdl(fk, dim3(n, map.heads, n_seqs), dim3(256), smem_f, st, true, src, map, scratch);
+        launch_pdl(sk, dim3(map.vdim / kCols, map.heads, n_seqs), dim3(DK * 2), stages * stage + rest, st, true, src, map, scratch, state, o, stages);
     }
     return cuda_status("chunk recurrence launch");
 }

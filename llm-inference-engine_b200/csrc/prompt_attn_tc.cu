@@ -116,6 +116,8 @@ template <int DK, int DV, bool LATENT> struct PaShape {
 template <typename T, int DK, int DV, bool LATENT, bool BIASED>
 __global__ void __launch_bounds__(PaShape<DK, DV, LATENT>::kWarps * 32 + 64, 1)
 prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const PromptAttn p) {
+    pdl_launch_dependents();
+    pdl_wait();
     using Sh = PaShape<DK, DV, LATENT>;
     constexpr int WARPS = Sh::kWarps, WPR = WARPS / 4, ST = Sh::kStages, SC = kPage / WPR, OC = DV / WPR;  // keys / value columns per thread
     static_assert(SC % 16 == 0 && OC % 16 == 0, "TMEM is read 16 columns at a time");
@@ -428,7 +430,7 @@ int pa_launch(const PromptAttn &p, const void *k_pool, const void *v_pool, bool 
     auto kern = prompt_attn_tc_kernel<T, DK, DV, LATENT, BIASED>;
     const size_t smem = Sh::kSmem + 2 * p.pen_len * sizeof(float);
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<dim3(p.n_tiles, p.heads / 2), Sh::kWarps * 32 + 64, smem, st>>>(tmK, tmV, p);
+    launch_pdl(kern, dim3(p.n_tiles, p.heads / 2), dim3(Sh::kWarps * 32 + 64), smem, st, true, tmK, tmV, p);
     return cuda_status("prompt attention (tcgen05) launch");
 }
 
