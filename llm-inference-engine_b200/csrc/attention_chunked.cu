@@ -31,15 +31,30 @@ attn_qk_norm_cache_kernel(const T *__restrict__ proj, int ld, T *__restrict__ q_
                      ((reinterpret_cast<size_t>(proj) | reinterpret_cast<size_t>(q_out) | reinterpret_cast<size_t>(k_pool) |
                        reinterpret_cast<size_t>(v_pool) | reinterpret_cast<size_t>(q_norm) | reinterpret_cast<size_t>(k_norm)) & 15) == 0;
     float sq = 0.0f, sk = 0.0f;
+    const int pos = tok_pos[t];  // (on their way while the sums are formed)
+    const int page = block_table[(size_t)tok_seq[t] * mpps + pos / kPage];
+    constexpr int HELD = 2;  // a thread's first pieces stay in registers between the sums and the scaling
+    uint4 held[HELD];
     if (vec) {
-        for (int c = threadIdx.x * V; c < nq + nk; c += blockDim.x * V) {  // nq is a multiple of V: a piece is all q or all k
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) {
+            const int c = (threadIdx.x + i * blockDim.x) * V;
+            if (c < nq + nk) held[i] = ld_v4(row + c);
+        }
+        auto add = [&](int c, const uint4 &raw) {  // nq is a multiple of V: a piece is all q or all k
             float f[V];
-            unpack16<T>(ld_v4(row + c), f);
+            unpack16<T>(raw, f);
             float ss = 0.0f;
 #pragma unroll
             for (int e = 0; e < V; ++e) ss = fmaf(f[e], f[e], ss);
             if (c < nq) sq += ss; else sk += ss;
+        };
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) {
+            const int c = (threadIdx.x + i * blockDim.x) * V;
+            if (c < nq + nk) add(c, held[i]);
         }
+        for (int c = (threadIdx.x + HELD * blockDim.x) * V; c < nq + nk; c += blockDim.x * V) add(c, ld_v4(row + c));
     } else {
         for (int c = threadIdx.x; c < nq; c += blockDim.x) {
             const float v = Elem<T>::to_f(row[c]);
@@ -50,25 +65,29 @@ attn_qk_norm_cache_kernel(const T *__restrict__ proj, int ld, T *__restrict__ q_
             sk = fmaf(v, v, sk);
         }
     }
-    sq = block_sum(sq, red);
-    sk = block_sum(sk, red);
+    {  // both sums behind one barrier
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+        sq = warp_sum(sq), sk = warp_sum(sk);
+        if (lane == 0) red[warp] = sq, red[16 + warp] = sk;
+        __syncthreads();
+        sq = sk = 0.0f;
+        for (int i = 0; i < warps; ++i) sq += red[i], sk += red[16 + i];
+    }
     const float iq = q_norm ? rsqrtf(sq / (float)nq + eps) : 1.0f;
     const float ik = k_norm ? rsqrtf(sk / (float)nk + eps) : 1.0f;
-    const int pos = tok_pos[t];
-    const int page = block_table[(size_t)tok_seq[t] * mpps + pos / kPage];
     const int off = pos % kPage;
     if (vec) {
-        for (int c = threadIdx.x * V; c < nq + nk; c += blockDim.x * V) {
-            const uint4 raw = ld_v4(row + c);
+        auto finish = [&](int c, const uint4 &raw) {
             float f[V];
             unpack16<T>(raw, f);
             const bool is_q = c < nq;
             const float *nw = is_q ? q_norm : k_norm;
             if (nw) {
                 const float inv = is_q ? iq : ik;
-                const int cn = is_q ? c : c - nq;
+                float wv[V];
+                load_vec<V>(nw + (is_q ? c : c - nq), wv);
 #pragma unroll
-                for (int e = 0; e < V; ++e) f[e] = f[e] * inv * nw[cn + e];
+                for (int e = 0; e < V; ++e) f[e] = f[e] * inv * wv[e];
             }
             if (is_q) {
                 st_v4(q_out + (size_t)t * nq + c, nw ? pack16<T>(f) : raw);
@@ -78,7 +97,13 @@ attn_qk_norm_cache_kernel(const T *__restrict__ proj, int ld, T *__restrict__ q_
                 st_v4(k_pool + at, nw ? pack16<T>(f) : raw);
                 st_v4(v_pool + at, raw);
             }
+        };
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) {
+            const int c = (threadIdx.x + i * blockDim.x) * V;
+            if (c < nq + nk) finish(c, held[i]);
         }
+        for (int c = (threadIdx.x + HELD * blockDim.x) * V; c < nq + nk; c += blockDim.x * V) finish(c, ld_v4(row + c));
         return;
     }
     for (int c = threadIdx.x; c < nq; c += blockDim.x) {
@@ -101,20 +126,22 @@ __global__ void __launch_bounds__(512)
 chunked_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const T *__restrict__ v_pool, const float *__restrict__ sink,
                     const T *__restrict__ gate_in, int gate_ld, T *__restrict__ out, const int *__restrict__ tok_seq,
                     const int *__restrict__ tok_pos, const int *__restrict__ block_table, int mpps, int heads, int kv_heads, int dim,
-                    float scale, int chunk, int max_keys, const int *__restrict__ tok_list) {
+                    float scale, int chunk, int max_keys, const int *__restrict__ tok_list, int splits) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ float sm[];
-    const int t = tok_list ? tok_list[blockIdx.x] : blockIdx.x, h = blockIdx.y;
+    const int ti = blockIdx.x / splits, rank = blockIdx.x - ti * splits;  // (the CTAs of a cluster are neighbours along x)
+    const int t = tok_list ? tok_list[ti] : ti, h = blockIdx.y;
     const int g = h / (heads / kv_heads);
     const int pos = tok_pos[t];
-    const int first = chunk > 0 ? (pos / chunk) * chunk : 0;
-    const int nkeys = pos - first + 1;
+    const int first_all = chunk > 0 ? (pos / chunk) * chunk : 0, all = pos - first_all + 1;
+    const int lo = (int)((long long)all * rank / splits), nkeys = (int)((long long)all * (rank + 1) / splits) - lo, first = first_all + lo;  // this CTA's keys
     const int ngroups = (int)blockDim.x >= dim ? (int)blockDim.x / dim : 1;
     float *qs = sm;
     float *sc = qs + dim;
     float *part = sc + max_keys;
     float *red = part + max((size_t)ngroups * dim, (size_t)blockDim.x * 8);
+    float *stat = red + 33;  // [2]: this CTA's maximum and sum
     const int *bt = block_table + (size_t)tok_seq[t] * mpps;
     for (int c = threadIdx.x; c < dim; c += blockDim.x) qs[c] = Elem<T>::to_f(q[((size_t)t * heads + h) * dim + c]);
     __syncthreads();
@@ -184,8 +211,6 @@ chunked_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const
         sum += e;
     }
     sum = block_sum(sum, red);  // (its barriers also publish sc[])
-    if (sink) sum += expf(sink[h] - mx);
-    const float inv = 1.0f / sum;
 
     // ---- weighted sum of the values
     constexpr int V = Elem<T>::kVec;
@@ -248,14 +273,39 @@ chunked_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const
         }
         __syncthreads();
     }
-    for (int c = threadIdx.x; c < dim; c += blockDim.x) {
-        float o = part[c] * inv;
+    // ---- the cluster's shares: weights relative to the common maximum, columns dealt to its CTAs
+    float share[8], all_mx = mx, total = sum;  // share[r]: what CTA r's sums are scaled by
+    if (splits > 1) {
+        if (threadIdx.x == 0) stat[0] = mx, stat[1] = sum;
+        cluster_barrier();
+        float peer_mx[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) peer_mx[r] = r < splits ? peer_value(stat, r) : mx, all_mx = fmaxf(all_mx, peer_mx[r]);
+        total = 0.0f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            share[r] = expf(peer_mx[r] - all_mx);
+            if (r < splits) total = fmaf(peer_value(stat + 1, r), share[r], total);
+        }
+    }
+    if (sink) total += expf(sink[h] - all_mx);
+    const float inv = 1.0f / total;
+    for (int c = threadIdx.x * splits + rank; c < dim; c += blockDim.x * splits) {
+        float o = part[c];
+        if (splits > 1) {
+            o = 0.0f;
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                if (r < splits) o = fmaf(peer_value(part + c, r), share[r], o);
+        }
+        o *= inv;
         if (gate_in) {
             const float z = Elem<T>::to_f(gate_in[(size_t)t * gate_ld + h * dim + c]);
             o *= 1.0f / (1.0f + expf(-z));
         }
         out[((size_t)t * heads + h) * dim + c] = Elem<T>::from_f(o);
     }
+    if (splits > 1) cluster_barrier();  // no CTA leaves while another reads its shared memory
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------------
@@ -512,16 +562,17 @@ int launch_chunked_attention(int dtype, const void *q, const void *k_pool, const
     const int threads = max_keys >= 512 ? 512 : (max_keys >= 256 ? 256 : 128);  // long chunks: more keys in flight per CTA
     const int ngroups = threads >= dim ? threads / dim : 1;
     const size_t part = std::max((size_t)ngroups * dim, (size_t)threads * 8);  // key-group partial sums (scalar / 16-byte path)
-    const size_t smem = ((size_t)dim + max_keys + part + 33) * sizeof(float);
-    if (smem > 200 * 1024) {
+    const int splits = key_splits((long long)tokens * heads, max_keys), keys = (max_keys + splits - 1) / splits;
+    const size_t smem = ((size_t)dim + keys + part + 35) * sizeof(float);
+    if (((size_t)dim + max_keys + part + 33) * sizeof(float) > 200 * 1024) {  // (without splits: what is refused does not depend on the batch)
         set_error("chunked_attention: %d keys x dim %d do not fit the shared-memory score buffer", max_keys, dim);
         return B200_ERR_UNSUPPORTED;
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(chunked_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(chunked_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, true, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink,
-                                                                            (const T *)gate_in, gate_ld, (T *)out, tok_seq, tok_pos,
-                                                                            block_table, mpps, heads, kv_heads, dim, scale, chunk, max_keys, tok_list);
+        launch_pdl_cluster(chunked_attn_kernel<T>, dim3(tokens * splits, heads), dim3(threads), smem, st, true, (unsigned)splits, (const T *)q, (const T *)k_pool,
+                           (const T *)v_pool, sink, (const T *)gate_in, gate_ld, (T *)out, tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim, scale, chunk, keys,
+                           tok_list, splits);
     });
     return cuda_status("chunked_attention launch");
 }

@@ -433,15 +433,35 @@ static void launch_gla_reg(const void *proj, int ld, const float *decay, float *
 }
 
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 gla_output_kernel(const float *__restrict__ o, const float *__restrict__ w, float eps, const T *__restrict__ gate_in, int gate_ld,
-                  T *__restrict__ out, int heads, int vdim) {
+                  T *__restrict__ out, int heads, int vdim, int tokens, int by_warp) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float red[33];
+    constexpr int V = Elem<T>::kVec;
+    if (by_warp) {  // a warp per (token, head): rows of up to 32 pieces
+        const size_t idx = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+        if (idx >= (size_t)tokens * heads) return;
+        const int t = (int)(idx / heads), h = (int)(idx - (size_t)t * heads), j = (threadIdx.x & 31) * V;
+        float ov[V], gz[V], ss = 0.0f;
+        if (j < vdim) {
+            load_vec<V>(o + idx * vdim + j, ov);
+            unpack16<T>(ld_v4(gate_in + (size_t)t * gate_ld + h * vdim + j), gz);
+#pragma unroll
+            for (int e = 0; e < V; ++e) ss = fmaf(ov[e], ov[e], ss);
+        }
+        const float inv = rsqrtf(warp_sum(ss) / (float)vdim + eps);
+        if (j < vdim) {
+            float y[V];
+#pragma unroll
+            for (int e = 0; e < V; ++e) y[e] = ov[e] * inv * w[j + e] * (gz[e] / (1.0f + expf(-gz[e])));
+            st_v4(out + idx * vdim + j, pack16<T>(y));
+        }
+        return;
+    }
     const int t = blockIdx.x, h = blockIdx.y;
     const float *orow = o + ((size_t)t * heads + h) * vdim;
-    constexpr int V = Elem<T>::kVec;
     const T *grow = gate_in + (size_t)t * gate_ld + h * vdim;
     T *out_row = out + ((size_t)t * heads + h) * vdim;
     // 16-byte pieces when every row starts on a 16-byte boundary
@@ -545,9 +565,15 @@ int launch_gla_output(int dtype, const float *o, const float *w, float eps, cons
     if (tokens == 0) return B200_OK;
     B200_DISPATCH_DTYPE(dtype, {
         constexpr int V = Elem<T>::kVec;
+        // whole pieces, at most a warp of them per row: eight rows per CTA (one per CTA: 21 us for 32768 rows of 256, half of it CTAs coming and going)
+        if (vdim % V == 0 && vdim / V <= 32 && gate_ld % V == 0 && all_aligned16({o, gate_in, out})) {
+            launch_pdl(gla_output_kernel<T>, dim3((unsigned)(((size_t)tokens * heads + 7) / 8)), dim3(256), 0, st, true, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim,
+                       tokens, 1);
+            return cuda_status("gla_output launch");
+        }
         // rows that go in 16-byte pieces need one thread per piece; others keep 128 threads striding the row
         const int threads = (vdim % V == 0 && vdim / V <= 128) ? std::max(32, (vdim / V + 31) / 32 * 32) : 128;
-        launch_pdl(gla_output_kernel<T>, dim3(tokens, heads), dim3(threads), 0, st, true, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim);
+        launch_pdl(gla_output_kernel<T>, dim3(tokens, heads), dim3(threads), 0, st, true, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim, tokens, 0);
     });
     return cuda_status("gla_output launch");
 }

@@ -741,7 +741,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 head_output_kernel(const float *__restrict__ o, const float *__restrict__ nq, const float *__restrict__ m_in, const float *__restrict__ w,
                    int w_stride, float eps, const float *__restrict__ gate_f, int gate_f_ld, const T *__restrict__ gate_t, int gate_t_ld,
-                   T *__restrict__ out, int out_ld, float out_scale, int tokens, int heads, int vdim, int gate_act) {
+                   T *__restrict__ out, int out_ld, float out_scale, int tokens, int heads, int vdim, int gate_act, int vec) {
     pdl_launch_dependents();
     pdl_wait();
     const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -751,6 +751,25 @@ head_output_kernel(const float *__restrict__ o, const float *__restrict__ nq, co
     float inv_den = 1.0f;
     if (nq) inv_den = 1.0f / (fmaxf(fabsf(nq[idx]), expf(-m_in[idx])) + 1e-6f);
     float ss = 0.0f;
+    if (vec) {  // rows of up to 256 in pieces of eight per lane, held between the sum and the scaling (one by one: 21.5 us for 23288 rows of 256)
+        const int j = lane * 8;
+        float y[8], z[8], wv[8];
+        if (j < vdim) {
+            load8(src + j, y);
+            if (gate_f) load8(gate_f + (size_t)t * gate_f_ld + h * vdim + j, z);
+            else load8(gate_t + (size_t)t * gate_t_ld + h * vdim + j, z);
+            load8(w + h * w_stride + j, wv);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) ss = fmaf(y[e] * inv_den, y[e] * inv_den, ss);
+        }
+        const float inv = rsqrtf(warp_sum(ss) / (float)vdim + eps) * inv_den;
+        if (j < vdim) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] = y[e] * inv * wv[e] * (gate_act ? z[e] * sigmoid_r(z[e]) : sigmoid_r(z[e])) * out_scale;
+            store8(out + (size_t)t * out_ld + h * vdim + j, y);
+        }
+        return;
+    }
     for (int j = lane; j < vdim; j += 32) {
         const float y = src[j] * inv_den;
         ss = fmaf(y, y, ss);
@@ -906,9 +925,10 @@ int launch_head_output(int dtype, const float *o, const float *nq, const float *
                        int heads, int vdim, cudaStream_t st, int gate_act) {
     if (tokens == 0) return B200_OK;
     const int grid = (tokens * heads + 7) / 8;
+    const int vec = vdim % 8 == 0 && vdim <= 256 && w_stride % 4 == 0 && gate_f_ld % 4 == 0 && gate_t_ld % 8 == 0 && out_ld % 8 == 0 && all_aligned16({o, w, gate_f, gate_t, out});
     B200_DISPATCH_DTYPE(dtype, {
         launch_pdl(head_output_kernel<T>, dim3(grid), dim3(256), 0, st, true, o, nq, m_in, w, w_stride, eps, gate_f, gate_f_ld, (const T *)gate_t, gate_t_ld, (T *)out, out_ld,
-                                                   out_scale, tokens, heads, vdim, gate_act);
+                                                   out_scale, tokens, heads, vdim, gate_act, vec);
     });
     return cuda_status("head_output launch");
 }
