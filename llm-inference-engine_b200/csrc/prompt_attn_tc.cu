@@ -6,13 +6,15 @@
 // The mma.sync kernels reach a tenth of the tensor rate: operands go through registers, two CTAs per SM hide little of it.  Here one CTA takes the 64
 // tokens of a tile x TWO heads that share their keys (any two latent heads; two query heads of one kv head) as the 128 rows of an MMA, so a key page is
 // read from memory once for both:
-//   * producer warp: one page of 64 keys per ring stage (page-table look-up, one TMA box per 64 columns, 128-byte swizzle); chunked layers load the value
-//     page beside it, latent layers have their values in the first DV columns of the key rows: one tile serves both products;
+//   * producer warp: one page of 64 keys or values per ring stage (page-table look-up, one TMA box per 64 columns, 128-byte swizzle), in the order the
+//     products take them (K0 K1 V0 K2 V1 ...); latent layers have their values in the first DV columns of the key rows: one tile serves both products;
 //   * MMA warp: S = Q K^T (128 x 64, two TMEM buffers: the next page's scores are formed while the softmax works) and O += P V, V the MN-major operand,
 //     O in TMEM for the whole loop;
 //   * WARPS softmax warps: WARPS / 4 threads share a row; lazy rescale: O is scaled only when the running maximum grows by more than 2^8 (see
 //     context_attn_tc.cu, whose loop this follows); the sink is the initial maximum and sum; value rows past the tile's last query are zeroed, since a page's
 //     unwritten rows may hold anything and 0 * NaN would reach the accumulator.
+// A step is a chain (scores, TMEM read, row maximum, exponentials, P, product): two CTAs per SM, where shared memory holds them (not the latent rows),
+// fill each other's waits.
 // Measured against the mma.sync kernels, us per layer: chunked 175 -> 81 (4096 tokens, 16 heads of 128), latent 244 -> 72 (3085 tokens in two prompts, 16
 // heads, rank 192 + 64), scored with a distance penalty and a window of 1024 116 -> 75 (2911 tokens in three prompts, 16 heads of 128).
 #include "hybrid_ops.cuh"
@@ -108,19 +110,21 @@ __device__ __forceinline__ uint32_t pa_idesc(bool bf16, int n, bool b_mn_major) 
 template <int DK, int DV, bool LATENT> struct PaShape {
     static constexpr int kWarps = LATENT ? 16 : 8;                               // softmax warps
     static constexpr int kStages = 3;
-    static constexpr int kStage = (DK / 64 + (LATENT ? 0 : DV / 64)) * kKBox;     // bytes of a ring stage
+    static constexpr int kStage = DK / 64 * kKBox;                               // bytes of a ring stage: a key page, or a value page (DV == DK)
+    static constexpr int kCtas = LATENT ? 1 : 2;                                 // per SM
     static constexpr int kTmem = DV + 2 * kPage <= 256 ? 256 : 512;
     static constexpr size_t kSmem = 1024 + (size_t)(DK / 64) * kQBox + (size_t)kStages * kStage + kQBox + 256 + 2 * kQRows * (kWarps / 4) * sizeof(float);
 };
 
 template <typename T, int DK, int DV, bool LATENT, bool BIASED>
-__global__ void __launch_bounds__(PaShape<DK, DV, LATENT>::kWarps * 32 + 64, 1)
+__global__ void __launch_bounds__(PaShape<DK, DV, LATENT>::kWarps * 32 + 64, PaShape<DK, DV, LATENT>::kCtas)
 prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const PromptAttn p) {
     pdl_launch_dependents();
     pdl_wait();
     using Sh = PaShape<DK, DV, LATENT>;
     constexpr int WARPS = Sh::kWarps, WPR = WARPS / 4, ST = Sh::kStages, SC = kPage / WPR, OC = DV / WPR;  // keys / value columns per thread
     static_assert(SC % 16 == 0 && OC % 16 == 0, "TMEM is read 16 columns at a time");
+    static_assert(LATENT || DK == DV, "a ring stage holds a key or a value page");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char *sQ = smem, *ring = sQ + (DK / 64) * kQBox, *sP = ring + ST * Sh::kStage;
@@ -139,6 +143,9 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     if (p.window > 0) lo = max(0, pos0 - p.window + 1);
     if (p.chunk > 0) lo = max(lo, pos0 / p.chunk * p.chunk);
     const int page0 = lo / kPage, n = last / kPage + 1 - page0;
+    // ring items in the order the products take them: K0 K1 V0 K2 V1 ... (latent: every page once)
+    auto k_item = [&](int j) { return LATENT ? j : (j == 0 ? 0 : 2 * j - 1); };
+    auto v_item = [&](int j) { return LATENT ? j : (j + 1 < n ? 2 * j + 2 : 2 * j + 1); };
 
     if (warp == WARPS && lane == 0) {
         pa_init(q_full, WARPS);
@@ -167,26 +174,24 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         // ================================================= producer
         if (lane == 0) {
             const int *bt = p.block_table + (size_t)seq * p.mpps + page0;
-            for (int j = 0; j < n; ++j) {
-                const int s = j % ST;
+            for (int i = 0; i < (LATENT ? n : 2 * n); ++i) {
+                const int s = i % ST;
+                const bool value = !LATENT && i > 0 && (i == 2 * n - 1 || (i & 1) == 0);
+                const int j = LATENT ? i : (i == 0 ? 0 : (value ? (i == 2 * n - 1 ? n - 1 : i / 2 - 1) : (i + 1) / 2));
                 const int row = LATENT ? __ldg(bt + j) * kPage : (__ldg(bt + j) * p.kv_heads + h0 / p.group) * kPage;
-                pa_wait(empty0 + 8 * s, ((j / ST) & 1) ^ 1);
+                pa_wait(empty0 + 8 * s, ((i / ST) & 1) ^ 1);
                 const uint32_t d = pa_u32(ring + s * Sh::kStage), bar = full0 + 8 * s;
                 pa_expect(bar, Sh::kStage);
 #pragma unroll
-                for (int c = 0; c < DK / 64; ++c) pa_tma(d + c * kKBox, &tmK, 64 * c, row, bar);
-                if constexpr (!LATENT) {
-#pragma unroll
-                    for (int c = 0; c < DV / 64; ++c) pa_tma(d + (DK / 64 + c) * kKBox, &tmV, 64 * c, row, bar);
-                }
+                for (int c = 0; c < DK / 64; ++c) pa_tma(d + c * kKBox, value ? &tmV : &tmK, 64 * c, row, bar);
             }
         }
     } else if (warp == WARPS + 1) {
         // ================================================= MMA issuer
         const uint32_t id_qk = pa_idesc(p.is_bf16 != 0, kPage, false), id_pv = pa_idesc(p.is_bf16 != 0, DV, true);
         auto scores = [&](int j) {
-            const int s = j % ST, sb = j & 1;
-            pa_wait(full0 + 8 * s, (j / ST) & 1);
+            const int i = k_item(j), s = i % ST, sb = j & 1;
+            pa_wait(full0 + 8 * s, (i / ST) & 1);
             pa_wait(s_free0 + 8 * sb, ((j >> 1) & 1) ^ 1);
             pa_after();
             if (pa_elect()) {
@@ -194,6 +199,7 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 #pragma unroll
                 for (int k = 0; k < DK / 16; ++k)
                     pa_mma(tmem + (uint32_t)(sb * kPage), pa_desc(aq + (k / 4) * kQBox + (k % 4) * 32, 16), pa_desc(bk + (k / 4) * kKBox + (k % 4) * 32, 16), id_qk, k > 0 ? 1u : 0u);
+                if (!LATENT) pa_commit(empty0 + 8 * s);  // (a latent page still serves as the values)
                 pa_commit(s_full0 + 8 * sb);
             }
             __syncwarp();
@@ -202,11 +208,12 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         scores(0);
         for (int j = 0; j < n; ++j) {
             if (j + 1 < n) scores(j + 1);
-            const int s = j % ST;
+            const int i = v_item(j), s = i % ST;
+            if (!LATENT) pa_wait(full0 + 8 * s, (i / ST) & 1);
             pa_wait(p_ready, j & 1);
             pa_after();
             if (pa_elect()) {
-                const uint32_t ap = pa_u32(sP), bv = pa_u32(ring + s * Sh::kStage + (LATENT ? 0 : (DK / 64) * kKBox));
+                const uint32_t ap = pa_u32(sP), bv = pa_u32(ring + s * Sh::kStage);
 #pragma unroll
                 for (int k = 0; k < kPage / 16; ++k)
                     pa_mma(tmem + 2 * kPage, pa_desc(ap + k * 32, 16), pa_desc(bv + k * 16 * 128, kKBox), id_pv, (j > 0 || k > 0) ? 1u : 0u);
@@ -339,8 +346,9 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
             for (int q = 0; q < SC / 8; ++q) *reinterpret_cast<uint4 *>(prow + (((cg * (SC / 8) + q) ^ (row & 7)) << 4)) = packed[q];
             // value rows past the tile's last query: cleared by the threads of rows 0 .. 63 (the scores have been formed: a shared tile may go too)
             if (row < kPage && kp + row > last) {
-                pa_wait(full0 + 8 * (j % ST), (j / ST) & 1);
-                unsigned char *v = ring + (j % ST) * Sh::kStage + (LATENT ? 0 : (DK / 64) * kKBox) + row * 128;
+                const int i = v_item(j);
+                pa_wait(full0 + 8 * (i % ST), (i / ST) & 1);
+                unsigned char *v = ring + (i % ST) * Sh::kStage + row * 128;
                 for (int c = cg; c < DV / 8; c += WPR) *reinterpret_cast<uint4 *>(v + (c >> 3) * kKBox + ((c & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
