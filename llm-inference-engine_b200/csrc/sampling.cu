@@ -19,23 +19,24 @@ struct Cand {
 };
 __device__ __forceinline__ bool better(float v, int id, float v2, int id2) { return v > v2 || (v == v2 && id < id2); }
 
+// the best of a warp's candidates in two warp reductions: the largest value (as an unsigned key in the values' order, both zeros alike), then the lowest id
+// that has it.  The value handed back is that of the lane with the id, bit for bit
 __device__ __forceinline__ Cand warp_best(Cand c) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float v = __shfl_xor_sync(0xffffffffu, c.v, o);
-        const int id = __shfl_xor_sync(0xffffffffu, c.id, o);
-        if (better(v, id, c.v, c.id)) c.v = v, c.id = id;
-    }
-    return c;
+    const unsigned bits = __float_as_uint(c.v + 0.0f), key = bits & 0x80000000u ? ~bits : bits | 0x80000000u;
+    const unsigned best = __reduce_max_sync(0xffffffffu, key);
+    const int id = __reduce_min_sync(0xffffffffu, key == best ? c.id : INT_MAX);
+    const unsigned owner = __ballot_sync(0xffffffffu, key == best && c.id == id);
+    return Cand{__shfl_sync(0xffffffffu, c.v, __ffs(owner) - 1), id};
 }
 
-// sorted insertion into a thread-local list of k entries (descending)
-__device__ __forceinline__ void insert(float (&lv)[kMaxK], int (&li)[kMaxK], int k, float v, int id) {
-    if (!better(v, id, lv[k - 1], li[k - 1])) return;
-    lv[k - 1] = v, li[k - 1] = id;
+// sorted insertion into a thread-local list (descending).  The list always has kMaxK entries, whatever k is: an index that is not a constant would put it in
+// local memory (11 us for 8 rows of 32000, of which the reads take 2)
+__device__ __forceinline__ void insert(float (&lv)[kMaxK], int (&li)[kMaxK], float v, int id) {
+    if (!better(v, id, lv[kMaxK - 1], li[kMaxK - 1])) return;
+    lv[kMaxK - 1] = v, li[kMaxK - 1] = id;
 #pragma unroll
     for (int i = kMaxK - 1; i > 0; --i) {
-        if (i < k && better(lv[i], li[i], lv[i - 1], li[i - 1])) {
+        if (better(lv[i], li[i], lv[i - 1], li[i - 1])) {
             const float tv = lv[i];
             const int ti = li[i];
             lv[i] = lv[i - 1], li[i] = li[i - 1];
@@ -87,7 +88,7 @@ topk_stage1_kernel(const T *__restrict__ logits, int *__restrict__ tmp_ids, T *_
         for (int u = 0; u < U; ++u) v[u] = Elem<T>::to_f(p[min(base + u * kTopkThreads, hi - 1)]);
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (base + u * kTopkThreads < hi) insert(lv, li, k, v[u], base + u * kTopkThreads);
+            if (base + u * kTopkThreads < hi) insert(lv, li, v[u], base + u * kTopkThreads);
     }
     block_select(lv, li, k, sv, si, red);
     __syncthreads();
@@ -248,19 +249,18 @@ topk_stage2_kernel(const int *__restrict__ tmp_ids, const T *__restrict__ tmp_va
     pdl_wait();
     for (int i = threadIdx.x; i < B200_TOPK_BLOCKS * k; i += 64) {
         const int id = tmp_ids[(size_t)row * B200_TOPK_BLOCKS * k + i];
-        if (id >= 0) insert(lv, li, k, Elem<T>::to_f(tmp_vals[(size_t)row * B200_TOPK_BLOCKS * k + i]), id);
+        if (id >= 0) insert(lv, li, Elem<T>::to_f(tmp_vals[(size_t)row * B200_TOPK_BLOCKS * k + i]), id);
     }
     block_select(lv, li, k, sv, si, red);
+    if constexpr (DRAW) {
+        static_assert(sizeof(T) == sizeof(float), "the candidates are drawn from as they are stored");
+        if (threadIdx.x == 0)  // (it wrote sv and si)
+            draw_row<float>(uniform, si, sv, draw.seq_len + row, draw.finished + row, draw.output_id + row, k, draw.end_id, draw.vocab);
+    }
     __syncthreads();
     if (threadIdx.x < k) {
         final_ids[(size_t)row * k + threadIdx.x] = si[threadIdx.x];
         final_vals[(size_t)row * k + threadIdx.x] = Elem<T>::from_f(sv[threadIdx.x]);
-    }
-    if (DRAW) {
-        __syncthreads();  // the candidates as they were stored
-        if (threadIdx.x == 0)
-            draw_row<T>(uniform, final_ids + (size_t)row * k, final_vals + (size_t)row * k, draw.seq_len + row, draw.finished + row, draw.output_id + row, k, draw.end_id,
-                        draw.vocab);
     }
 }
 
