@@ -127,7 +127,8 @@ delta_prep_tile_kernel(const T *__restrict__ proj, int ld, int col0, const float
         const float4 f = *reinterpret_cast<const float4 *>(conv_w + (size_t)(cc + e) * kPrepTaps);
         w[3][e] = f.x, w[2][e] = f.y, w[1][e] = f.z, w[0][e] = f.w;
     }
-    const bool is_q = cc < nqk, is_qk = cc < 2 * nqk;
+    // (a lane past the last channel is neither: a warp that ends with value heads skips the heads' sums as a whole)
+    const bool is_q = mine && c < nqk, is_qk = mine && c < 2 * nqk;
     const int lanes = dim / 8;           // lanes that hold one q or k head
     float *dst0 = rec + (is_q ? lay.q + cc : (is_qk ? lay.k + cc - nqk : lay.v + cc - 2 * nqk));
     for (int tile = 0; tile < tiles; ++tile) {
