@@ -19,8 +19,6 @@ __global__ void __launch_bounds__(256)
 attn_qk_norm_cache_kernel(const T *__restrict__ proj, int ld, T *__restrict__ q_out, T *__restrict__ k_pool, T *__restrict__ v_pool,
                           const float *__restrict__ q_norm, const float *__restrict__ k_norm, float eps, const int *__restrict__ tok_seq,
                           const int *__restrict__ tok_pos, const int *__restrict__ block_table, int mpps, int heads, int kv_heads, int dim) {
-    pdl_launch_dependents();
-    pdl_wait();
     __shared__ float red[33];
     const int t = blockIdx.x;
     const int nq = heads * dim, nk = kv_heads * dim;
@@ -126,22 +124,18 @@ __global__ void __launch_bounds__(512)
 chunked_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const T *__restrict__ v_pool, const float *__restrict__ sink,
                     const T *__restrict__ gate_in, int gate_ld, T *__restrict__ out, const int *__restrict__ tok_seq,
                     const int *__restrict__ tok_pos, const int *__restrict__ block_table, int mpps, int heads, int kv_heads, int dim,
-                    float scale, int chunk, int max_keys, const int *__restrict__ tok_list, int splits) {
-    pdl_launch_dependents();
-    pdl_wait();
+                    float scale, int chunk, int max_keys, const int *__restrict__ tok_list) {
     extern __shared__ float sm[];
-    const int ti = blockIdx.x / splits, rank = blockIdx.x - ti * splits;  // (the CTAs of a cluster are neighbours along x)
-    const int t = tok_list ? tok_list[ti] : ti, h = blockIdx.y;
+    const int t = tok_list ? tok_list[blockIdx.x] : blockIdx.x, h = blockIdx.y;
     const int g = h / (heads / kv_heads);
     const int pos = tok_pos[t];
-    const int first_all = chunk > 0 ? (pos / chunk) * chunk : 0, all = pos - first_all + 1;
-    const int lo = (int)((long long)all * rank / splits), nkeys = (int)((long long)all * (rank + 1) / splits) - lo, first = first_all + lo;  // this CTA's keys
+    const int first = chunk > 0 ? (pos / chunk) * chunk : 0;
+    const int nkeys = pos - first + 1;
     const int ngroups = (int)blockDim.x >= dim ? (int)blockDim.x / dim : 1;
     float *qs = sm;
     float *sc = qs + dim;
     float *part = sc + max_keys;
     float *red = part + max((size_t)ngroups * dim, (size_t)blockDim.x * 8);
-    float *stat = red + 33;  // [2]: this CTA's maximum and sum
     const int *bt = block_table + (size_t)tok_seq[t] * mpps;
     for (int c = threadIdx.x; c < dim; c += blockDim.x) qs[c] = Elem<T>::to_f(q[((size_t)t * heads + h) * dim + c]);
     __syncthreads();
@@ -211,6 +205,8 @@ chunked_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const
         sum += e;
     }
     sum = block_sum(sum, red);  // (its barriers also publish sc[])
+    if (sink) sum += expf(sink[h] - mx);
+    const float inv = 1.0f / sum;
 
     // ---- weighted sum of the values
     constexpr int V = Elem<T>::kVec;
@@ -273,39 +269,14 @@ chunked_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const
         }
         __syncthreads();
     }
-    // ---- the cluster's shares: weights relative to the common maximum, columns dealt to its CTAs
-    float share[8], all_mx = mx, total = sum;  // share[r]: what CTA r's sums are scaled by
-    if (splits > 1) {
-        if (threadIdx.x == 0) stat[0] = mx, stat[1] = sum;
-        cluster_barrier();
-        float peer_mx[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) peer_mx[r] = r < splits ? peer_value(stat, r) : mx, all_mx = fmaxf(all_mx, peer_mx[r]);
-        total = 0.0f;
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            share[r] = expf(peer_mx[r] - all_mx);
-            if (r < splits) total = fmaf(peer_value(stat + 1, r), share[r], total);
-        }
-    }
-    if (sink) total += expf(sink[h] - all_mx);
-    const float inv = 1.0f / total;
-    for (int c = threadIdx.x * splits + rank; c < dim; c += blockDim.x * splits) {
-        float o = part[c];
-        if (splits > 1) {
-            o = 0.0f;
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-                if (r < splits) o = fmaf(peer_value(part + c, r), share[r], o);
-        }
-        o *= inv;
+    for (int c = threadIdx.x; c < dim; c += blockDim.x) {
+        float o = part[c] * inv;
         if (gate_in) {
             const float z = Elem<T>::to_f(gate_in[(size_t)t * gate_ld + h * dim + c]);
             o *= 1.0f / (1.0f + expf(-z));
         }
         out[((size_t)t * heads + h) * dim + c] = Elem<T>::from_f(o);
     }
-    if (splits > 1) cluster_barrier();  // no CTA leaves while another reads its shared memory
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------------
@@ -359,8 +330,6 @@ __global__ void __launch_bounds__(128)
 chunked_attn_mma_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const T *__restrict__ v_pool, const float *__restrict__ sink,
                         const T *__restrict__ gate_in, int gate_ld, T *__restrict__ out, const int4 *__restrict__ tiles,
                         const int *__restrict__ block_table, int mpps, int heads, int kv_heads, float scale, int chunk) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     T *qs = reinterpret_cast<T *>(smraw);     // [64][D]
     T *ks = qs + kTileQ * D;                  // [2][64][D]
@@ -513,7 +482,7 @@ static int launch_mma_t(const void *q, const void *k_pool, const void *v_pool, c
                         cudaStream_t st) {
     const size_t smem = (size_t)(kTileQ + 4 * kPage) * D * sizeof(T);
     cudaFuncSetAttribute(chunked_attn_mma_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(chunked_attn_mma_kernel<T, D>, dim3(n_tiles, heads), dim3(128), smem, st, true, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink, (const T *)gate_in,
+    launch_pdl(chunked_attn_mma_kernel<T, D>, dim3(n_tiles, heads), dim3(128), smem, st, false, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink, (const T *)gate_in,
                                                                             gate_ld, (T *)out, (const int4 *)tiles, block_table, mpps, heads, kv_heads,
                                                                             scale, chunk);
     return cuda_status("chunked_attention (tensor core) launch");
@@ -549,7 +518,7 @@ int launch_attn_qk_norm_cache(int dtype, const void *proj, int ld, void *q_out, 
                               int tokens, int heads, int kv_heads, int dim, cudaStream_t st) {
     if (tokens == 0) return B200_OK;
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(attn_qk_norm_cache_kernel<T>, dim3(tokens), dim3(256), 0, st, true, (const T *)proj, ld, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
+        launch_pdl(attn_qk_norm_cache_kernel<T>, dim3(tokens), dim3(256), 0, st, false, (const T *)proj, ld, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
                                                               tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim);
     });
     return cuda_status("attn_qk_norm_cache launch");
@@ -562,17 +531,16 @@ int launch_chunked_attention(int dtype, const void *q, const void *k_pool, const
     const int threads = max_keys >= 512 ? 512 : (max_keys >= 256 ? 256 : 128);  // long chunks: more keys in flight per CTA
     const int ngroups = threads >= dim ? threads / dim : 1;
     const size_t part = std::max((size_t)ngroups * dim, (size_t)threads * 8);  // key-group partial sums (scalar / 16-byte path)
-    const int splits = key_splits((long long)tokens * heads, max_keys), keys = (max_keys + splits - 1) / splits;
-    const size_t smem = ((size_t)dim + keys + part + 35) * sizeof(float);
-    if (((size_t)dim + max_keys + part + 33) * sizeof(float) > 200 * 1024) {  // (without splits: what is refused does not depend on the batch)
+    const size_t smem = ((size_t)dim + max_keys + part + 33) * sizeof(float);
+    if (smem > 200 * 1024) {
         set_error("chunked_attention: %d keys x dim %d do not fit the shared-memory score buffer", max_keys, dim);
         return B200_ERR_UNSUPPORTED;
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(chunked_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl_cluster(chunked_attn_kernel<T>, dim3(tokens * splits, heads), dim3(threads), smem, st, true, (unsigned)splits, (const T *)q, (const T *)k_pool,
-                           (const T *)v_pool, sink, (const T *)gate_in, gate_ld, (T *)out, tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim, scale, chunk, keys,
-                           tok_list, splits);
+        launch_pdl(chunked_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, false, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink,
+                                                                            (const T *)gate_in, gate_ld, (T *)out, tok_seq, tok_pos,
+                                                                            block_table, mpps, heads, kv_heads, dim, scale, chunk, max_keys, tok_list);
     });
     return cuda_status("chunked_attention launch");
 }

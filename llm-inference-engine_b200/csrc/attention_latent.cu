@@ -32,8 +32,6 @@ latent_prep_kernel(const T *__restrict__ proj, int ld, int q_col, int kv_col, T 
                    const float *__restrict__ kv_norm, float eps, const int *__restrict__ tok_seq, const int *__restrict__ tok_pos,
                    const int *__restrict__ block_table, int mpps, int t_pad, int heads, int dim, int rot_dim, int kv_rank, int rot_dims,
                    float rot_base, const T *__restrict__ kv_proj, int kv_ld, LatentRotation rt) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ float cs[];  // cos[half] | sin[half]
     __shared__ float red[33];
     const int t = blockIdx.x, half = rot_dims / 2;
@@ -160,8 +158,6 @@ latent_attn_kernel(const T *__restrict__ ql, const T *__restrict__ qr, const T *
                    T *__restrict__ ol, const int *__restrict__ tok_seq, const int *__restrict__ tok_pos, const int *__restrict__ block_table,
                    int mpps, int t_pad, int heads, int kv_rank, int rot_dim, float scale, int window, int max_keys, int part_floats,
                    const int *__restrict__ tok_list) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) float sm[];
     const int t = tok_list ? tok_list[blockIdx.x] : blockIdx.x, h = blockIdx.y;
     const int dk = kv_rank + rot_dim;
@@ -329,8 +325,6 @@ __global__ void __launch_bounds__(128)
 latent_attn_mma_kernel(const T *__restrict__ ql, const T *__restrict__ qr, const T *__restrict__ pool, const float *__restrict__ sink,
                        T *__restrict__ ol, const int4 *__restrict__ tiles, const int *__restrict__ block_table, int mpps, int t_pad, int heads,
                        int kv_rank, int rot_dim, int ld, float scale, int window, int by_head, int splits, float *__restrict__ part) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     T *qs = reinterpret_cast<T *>(smraw);  // [64][ld]
     T *ks = qs + kLatTileQ * ld;           // [2][64][ld]
@@ -496,8 +490,6 @@ latent_attn_mma_kernel(const T *__restrict__ ql, const T *__restrict__ qr, const
 template <typename T>
 __global__ void __launch_bounds__(128)
 latent_combine_kernel(const float *__restrict__ part, const int4 *__restrict__ tiles, T *__restrict__ ol, int t_pad, int heads, int kv_rank, int splits) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int h = blockIdx.y, t = tiles[blockIdx.x].y;
     const size_t stride = (size_t)kv_rank + 2;
     const float *p0 = part + ((size_t)blockIdx.x * splits * heads + h) * stride;
@@ -525,8 +517,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 latent_gate_kernel(const T *__restrict__ ov, const T *__restrict__ gate_in, int gate_ld, T *__restrict__ out, int t_pad, int heads, int vdim,
                    int head_gate) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x;
     constexpr int V = Elem<T>::kVec;
     if (!gate_in) {  // no gate
@@ -590,8 +580,6 @@ latent_gate_kernel(const T *__restrict__ ov, const T *__restrict__ gate_in, int 
 template <typename T>
 __global__ void __launch_bounds__(128)
 rms_rows_kernel(const T *__restrict__ in, int ld, const float *__restrict__ w, float eps, T *__restrict__ out, int tokens, int cols) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= tokens) return;
     constexpr int V = Elem<T>::kVec;
@@ -633,7 +621,7 @@ rms_rows_kernel(const T *__restrict__ in, int ld, const float *__restrict__ w, f
 
 int launch_rms_rows(int dtype, const void *in, int ld, const float *w, float eps, void *out, int tokens, int cols, cudaStream_t st) {
     if (tokens == 0) return B200_OK;
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(rms_rows_kernel<T>, dim3((tokens + 3) / 4), dim3(128), 0, st, true, (const T *)in, ld, w, eps, (T *)out, tokens, cols); });
+    B200_DISPATCH_DTYPE(dtype, { launch_pdl(rms_rows_kernel<T>, dim3((tokens + 3) / 4), dim3(128), 0, st, false, (const T *)in, ld, w, eps, (T *)out, tokens, cols); });
     return cuda_status("rms_rows launch");
 }
 
@@ -644,7 +632,7 @@ int launch_latent_prep(int dtype, const void *proj, int ld, int q_col, int kv_co
     if (tokens == 0) return B200_OK;
     const size_t smem = (size_t)std::max(rot_dims, 2) * sizeof(float);
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(latent_prep_kernel<T>, dim3(tokens), dim3(128), smem, st, true, (const T *)proj, ld, q_col, kv_col, (T *)qn, (T *)qr, (T *)pool, kv_norm, eps, tok_seq,
+        launch_pdl(latent_prep_kernel<T>, dim3(tokens), dim3(128), smem, st, false, (const T *)proj, ld, q_col, kv_col, (T *)qn, (T *)qr, (T *)pool, kv_norm, eps, tok_seq,
                                                         tok_pos, block_table, mpps, t_pad, heads, dim, rot_dim, kv_rank, rot_dims, rot_base,
                                                         (const T *)kv_proj, kv_ld, rot);
     });
@@ -667,7 +655,7 @@ int launch_latent_attention(int dtype, const void *ql, const void *qr, const voi
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(latent_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(latent_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, true, (const T *)ql, (const T *)qr, (const T *)pool, sink, (T *)ol, tok_seq,
+        launch_pdl(latent_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, false, (const T *)ql, (const T *)qr, (const T *)pool, sink, (T *)ol, tok_seq,
                                                                            tok_pos, block_table, mpps, t_pad, heads, kv_rank, rot_dim, scale,
                                                                            window, max_keys, (int)part, tok_list);
     });
@@ -694,11 +682,11 @@ static int launch_latent_mma_t(const void *ql, const void *qr, const void *pool,
     const int ld = (kv_rank + rot_dim + 63) / 64 * 64;
     const size_t smem = (size_t)3 * kLatTileQ * ld * sizeof(T);
     cudaFuncSetAttribute(latent_attn_mma_kernel<T, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(latent_attn_mma_kernel<T, NV>, dim3(grid), dim3(128), smem, st, true, (const T *)ql, (const T *)qr, (const T *)pool, sink, (T *)ol, (const int4 *)tiles,
+    launch_pdl(latent_attn_mma_kernel<T, NV>, dim3(grid), dim3(128), smem, st, false, (const T *)ql, (const T *)qr, (const T *)pool, sink, (T *)ol, (const int4 *)tiles,
                                                            block_table, mpps, t_pad, heads, kv_rank, rot_dim, ld, scale, window, by_head, splits,
                                                            splits > 1 ? part : nullptr);
     if (splits > 1)
-        launch_pdl(latent_combine_kernel<T>, dim3(grid.x, heads), dim3(128), 0, st, true, part, (const int4 *)tiles, (T *)ol, t_pad, heads, kv_rank, splits);
+        launch_pdl(latent_combine_kernel<T>, dim3(grid.x, heads), dim3(128), 0, st, false, part, (const int4 *)tiles, (T *)ol, t_pad, heads, kv_rank, splits);
     return cuda_status("latent_attention (tensor core) launch");
 }
 
@@ -747,7 +735,7 @@ int launch_latent_gate(int dtype, const void *ov, const void *gate_in, int gate_
                        cudaStream_t st, int head_gate) {
     if (tokens == 0) return B200_OK;
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(latent_gate_kernel<T>, dim3(tokens), dim3(256), 0, st, true, (const T *)ov, (const T *)gate_in, gate_ld, (T *)out, t_pad, heads, vdim, head_gate);
+        launch_pdl(latent_gate_kernel<T>, dim3(tokens), dim3(256), 0, st, false, (const T *)ov, (const T *)gate_in, gate_ld, (T *)out, t_pad, heads, vdim, head_gate);
     });
     return cuda_status("latent_gate launch");
 }

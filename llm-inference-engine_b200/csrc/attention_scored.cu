@@ -31,8 +31,6 @@ scored_prep_kernel(const T *__restrict__ proj, int ld, int col0, const float *__
                    const int *__restrict__ tok_seq, const int *__restrict__ tok_pos, const int *__restrict__ block_table, int mpps, int heads,
                    int kv_heads, int dim, int vdim, int rot_dims, float rot_base, ScoredPrepOptions opt, T *__restrict__ v_keep,
                    const T *__restrict__ v_mix, float lambda) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ float rot[];  // cos [rot_dims/2] | sin [rot_dims/2]
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const int pos = tok_pos[t], half = rot_dims / 2;
@@ -119,8 +117,6 @@ scored_prep_vec_kernel(const T *__restrict__ proj, int ld, int col0, T *__restri
                        const float *__restrict__ q_norm, const float *__restrict__ k_norm, float eps, const int *__restrict__ tok_seq,
                        const int *__restrict__ tok_pos, const int *__restrict__ block_table, int mpps, int heads, int kv_heads, int dim, int vdim,
                        T *__restrict__ v_keep, const T *__restrict__ v_mix, float lambda, const float *__restrict__ bias) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int V = Elem<T>::kVec;
     const int t = blockIdx.x, pos = tok_pos[t], per = dim / V, n_qk = (heads + kv_heads) * per, n_v = kv_heads * vdim / V;
     const T *row = proj + (size_t)t * ld + col0;
@@ -206,21 +202,17 @@ scored_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const 
                    const float *__restrict__ dist_r1, const float *__restrict__ dist_r2, const T *__restrict__ gate_in, int gate_ld,
                    T *__restrict__ out, int out_ld, float out_scale, const int *__restrict__ tok_seq, const int *__restrict__ tok_pos,
                    const int *__restrict__ block_table, int mpps, int heads, int kv_heads, int dim, int vdim, float scale, int window,
-                   int sigmoid, int max_keys, int part_floats, const int *__restrict__ tok_list, ScoredOptions opt, int splits) {
-    pdl_launch_dependents();
-    pdl_wait();
+                   int sigmoid, int max_keys, int part_floats, const int *__restrict__ tok_list, ScoredOptions opt) {
     extern __shared__ float sm[];
-    const int ti = blockIdx.x / splits, rank = blockIdx.x - ti * splits;  // (the CTAs of a cluster are neighbours along x)
-    const int t = tok_list ? tok_list[ti] : ti, h = blockIdx.y;
+    const int t = tok_list ? tok_list[blockIdx.x] : blockIdx.x, h = blockIdx.y;
     const int g = h / (heads / kv_heads);
     const int pos = tok_pos[t];
-    const int first_all = first_key(pos, window, opt.chunk), all = pos - first_all + 1;
-    const int lo = (int)((long long)all * rank / splits), nkeys = (int)((long long)all * (rank + 1) / splits) - lo, first = first_all + lo;  // this CTA's keys
+    const int first = first_key(pos, window, opt.chunk);
+    const int nkeys = pos - first + 1;
     float *qs = sm;
     float *sc = qs + dim;
     float *part = sc + max_keys;
     float *red = part + part_floats;
-    float *stat = red + 33;  // [2]: this CTA's maximum and sum
     const int *bt = block_table + (size_t)tok_seq[t] * mpps;
     for (int c = threadIdx.x; c < dim; c += blockDim.x) qs[c] = Elem<T>::to_f(q[((size_t)t * heads + h) * dim + c]);
     __syncthreads();
@@ -265,15 +257,18 @@ scored_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const 
             }
         }
     }
-    float sum = 0.0f;
+    float inv = 1.0f;
     if (!sigmoid) {
         mx = block_max(mx, red);
+        float sum = 0.0f;
         for (int j = threadIdx.x; j < nkeys; j += blockDim.x) {
             const float e = expf(sc[j] - mx);
             sc[j] = e;
             sum += e;
         }
         sum = block_sum(sum, red);  // (its barriers also publish sc[])
+        if (sunk) sum += expf(opt.sink[h] - mx);  // the sink: a logit with no key and no value, counted once
+        inv = 1.0f / sum;
     } else {
         __syncthreads();
     }
@@ -336,36 +331,11 @@ scored_attn_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, const 
             __syncthreads();
         }
     }
-    // ---- the cluster's shares: weights relative to the common maximum, columns dealt to its CTAs
-    float share[8], all_mx = mx, total = sum;  // share[r]: what CTA r's sums are scaled by
-    if (splits > 1) {
-        if (threadIdx.x == 0) stat[0] = mx, stat[1] = sum;
-        cluster_barrier();
-        float peer_mx[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) peer_mx[r] = r < splits ? peer_value(stat, r) : mx, all_mx = fmaxf(all_mx, peer_mx[r]);
-        total = 0.0f;
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            share[r] = sigmoid ? 1.0f : expf(peer_mx[r] - all_mx);
-            if (r < splits) total = fmaf(peer_value(stat + 1, r), share[r], total);
-        }
-    }
-    if (sunk) total += expf(opt.sink[h] - all_mx);  // the sink: a logit with no key and no value, counted once
-    const float inv = sigmoid ? 1.0f : 1.0f / total;
-    for (int c = threadIdx.x * splits + rank; c < vdim; c += blockDim.x * splits) {
-        float o = part[c];
-        if (splits > 1) {
-            o = 0.0f;
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-                if (r < splits) o = fmaf(peer_value(part + c, r), share[r], o);
-        }
-        o *= inv;
+    for (int c = threadIdx.x; c < vdim; c += blockDim.x) {
+        float o = part[c] * inv;
         if (gate_in) o *= sigmoid_f(Elem<T>::to_f(gate_in[(size_t)t * gate_ld + h * vdim + c]));
         out[(size_t)t * out_ld + h * vdim + c] = Elem<T>::from_f(o * out_scale);
     }
-    if (splits > 1) cluster_barrier();  // no CTA leaves while another reads its shared memory
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------------
@@ -424,8 +394,6 @@ scored_attn_mma_kernel(const T *__restrict__ q, const T *__restrict__ k_pool, co
                        const float *__restrict__ dist_r1, const float *__restrict__ dist_r2, const T *__restrict__ gate_in, int gate_ld,
                        T *__restrict__ out, int out_ld, float out_scale, const int4 *__restrict__ tiles, const int *__restrict__ block_table,
                        int mpps, int heads, int kv_heads, float scale, int window, int pen_len, ScoredOptions opt) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     T *qs = reinterpret_cast<T *>(smraw);       // [64][DK]
     T *ks = qs + kTileQS * DK;                  // [2][64][DK]
@@ -624,7 +592,7 @@ static int launch_scored_mma_t(const void *q, const void *k_pool, const void *v_
     const size_t smem = (size_t)(kTileQS + 2 * kPageS) * DK * sizeof(T) + (size_t)2 * kPageS * DV * sizeof(T) + (size_t)pen_len * sizeof(float);
     auto kern = sigmoid ? scored_attn_mma_kernel<T, DK, DV, 1> : scored_attn_mma_kernel<T, DK, DV, 0>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(kern, dim3(n_tiles, heads), dim3(128), smem, st, true, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, r1, r2, (const T *)gate_in, gate_ld,
+    launch_pdl(kern, dim3(n_tiles, heads), dim3(128), smem, st, false, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, r1, r2, (const T *)gate_in, gate_ld,
                                                   (T *)out, out_ld, out_scale, (const int4 *)tiles, block_table, mpps, heads, kv_heads, scale, window,
                                                   pen_len, opt);
     return cuda_status("scored_attention (tensor core) launch");
@@ -672,12 +640,12 @@ int launch_scored_prep(int dtype, const void *proj, int ld, int col0, const floa
         const int per = dim / V;
         if (rot_dims == 0 && !opt.v_norm && dim % V == 0 && per <= 32 && (per & (per - 1)) == 0 && vdim % V == 0 && ld % V == 0 && col0 % V == 0 &&
             (q_norm == nullptr) == (k_norm == nullptr) && all_aligned16({proj, b_in, q_out, k_pool, v_pool, q_norm, k_norm, share.v_keep, share.v_mix})) {
-            launch_pdl(scored_prep_vec_kernel<T>, dim3(tokens), dim3(128), 0, st, true, (const T *)proj, ld, col0, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
+            launch_pdl(scored_prep_vec_kernel<T>, dim3(tokens), dim3(128), 0, st, false, (const T *)proj, ld, col0, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
                                                               tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim, vdim, (T *)share.v_keep,
                                                               (const T *)share.v_mix, share.lambda, b_in);
             return cuda_status("scored_prep (vector) launch");
         }
-        launch_pdl(scored_prep_kernel<T>, dim3(tokens), dim3(256), (size_t)std::max(rot_dims, 2) * sizeof(float), st, true, (const T *)proj, ld, col0, b_in, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps, tok_seq, tok_pos, block_table, mpps, heads,
+        launch_pdl(scored_prep_kernel<T>, dim3(tokens), dim3(256), (size_t)std::max(rot_dims, 2) * sizeof(float), st, false, (const T *)proj, ld, col0, b_in, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps, tok_seq, tok_pos, block_table, mpps, heads,
             kv_heads, dim, vdim, rot_dims, rot_base, opt, (T *)share.v_keep, (const T *)share.v_mix, share.lambda);
     });
     return cuda_status("scored_prep launch");
@@ -691,16 +659,15 @@ int launch_scored_attention(int dtype, const void *q, const void *k_pool, const 
     const int threads = max_keys >= 512 ? 512 : (max_keys >= 256 ? 256 : 128);  // long contexts: more keys in flight per CTA
     const int ngroups = threads >= vdim ? threads / vdim : 1;
     const size_t part = std::max((size_t)ngroups * vdim, (size_t)threads * 8);  // key-group partial sums (scalar / 16-byte path)
-    const int splits = key_splits((long long)tokens * heads, max_keys), keys = (max_keys + splits - 1) / splits;
-    const size_t smem = ((size_t)dim + keys + part + 35) * sizeof(float);
-    if (((size_t)dim + max_keys + part + 33) * sizeof(float) > 200 * 1024) {  // (without splits: what is refused does not depend on the batch)
+    const size_t smem = ((size_t)dim + max_keys + part + 33) * sizeof(float);
+    if (smem > 200 * 1024) {
         set_error("scored_attention: %d keys x dim %d do not fit the shared-memory weight buffer", max_keys, dim);
         return B200_ERR_UNSUPPORTED;
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(scored_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl_cluster(scored_attn_kernel<T>, dim3(tokens * splits, heads), dim3(threads), smem, st, true, (unsigned)splits, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, dist_r1, dist_r2, (const T *)gate_in, gate_ld, (T *)out, out_ld, out_scale,
-            tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim, vdim, scale, window, sigmoid, keys, (int)part, tok_list, opt, splits);
+        launch_pdl(scored_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, false, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, dist_r1, dist_r2, (const T *)gate_in, gate_ld, (T *)out, out_ld, out_scale,
+            tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim, vdim, scale, window, sigmoid, max_keys, (int)part, tok_list, opt);
     });
     return cuda_status("scored_attention launch");
 }

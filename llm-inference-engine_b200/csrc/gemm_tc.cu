@@ -458,9 +458,9 @@ constexpr int kPairStageBytes = 2 * kATileBytes;  // 128 rows of A, up to 128 ro
 
 __device__ unsigned int g_pair_wait_failed;  // a wait that gave up (seconds): the launch's results are not valid
 
-// false after a limit that no live launch reaches; the caller leaves its role loop
+// false after 2^31 clocks (about a second; a try may sleep, so tries are no measure); the caller leaves its role loop
 __device__ __forceinline__ bool bar_wait_limited(uint32_t bar, uint32_t parity) {
-    for (int i = 0; i < (1 << 24); ++i) {
+    auto ready = [&]() -> bool {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -469,10 +469,16 @@ __device__ __forceinline__ bool bar_wait_limited(uint32_t bar, uint32_t parity) 
             : "=r"(ok)
             : "r"(bar), "r"(parity)
             : "memory");
-        if (ok) return true;
+        return ok != 0;
+    };
+    if (ready()) return true;
+    const uint32_t t0 = (uint32_t)clock();
+    while (!ready()) {
+        if ((uint32_t)clock() - t0 < 0x7fffffffu) continue;
+        atomicExch(&g_pair_wait_failed, 1u);
+        return false;
     }
-    atomicExch(&g_pair_wait_failed, 1u);
-    return false;
+    return true;
 }
 __device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {  // the same shared-memory offset in CTA `rank` of the cluster
     uint32_t r;

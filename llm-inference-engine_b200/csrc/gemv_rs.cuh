@@ -38,9 +38,14 @@ struct RsGeom {
     int max_units;      // units of the busiest CTA
 };
 
-// a wait that gives up after seconds, so that a fault elsewhere cannot hang the device
+// a wait that gives up after 2^31 clocks (about a second; a try may sleep, so tries are no measure), and with it every later wait of the CTA: a fault
+// elsewhere must not hang the device
+__device__ __forceinline__ volatile int &rs_gave_up() {
+    __shared__ volatile int v;
+    return v;
+}
 __device__ __forceinline__ void mbar_wait_limited(uint32_t bar, uint32_t parity) {
-    for (int i = 0; i < (1 << 24); ++i) {
+    auto ready = [&]() -> bool {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -49,7 +54,14 @@ __device__ __forceinline__ void mbar_wait_limited(uint32_t bar, uint32_t parity)
             : "=r"(ok)
             : "r"(bar), "r"(parity)
             : "memory");
-        if (ok) return;
+        return ok != 0;
+    };
+    if (ready()) return;
+    const uint32_t t0 = (uint32_t)clock();
+    while (!ready()) {
+        if ((uint32_t)clock() - t0 < 0x7fffffffu && !rs_gave_up()) continue;
+        rs_gave_up() = 1;
+        return;
     }
 }
 
@@ -117,6 +129,7 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
             if (++s == stages) s = 0;
         };
         if (lane == 0) {
+            rs_gave_up() = 0;
             for (int i = 0; i < stages; ++i) {
                 mbar_init(full0 + i * 8, 1);
                 mbar_init(empty0 + i * 8, kMmaWarps);

@@ -23,8 +23,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 gla_decay_kernel(const T *__restrict__ proj, int ld, int col0, const T *__restrict__ w, const float *__restrict__ bias, float inv_tau,
                  float *__restrict__ decay, int tokens, int rank, int channels) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) float lo[];  // [kDecayTokens][rank]: the tokens' low-rank vectors
     const int t0 = blockIdx.x * kDecayTokens;
     const int nt = min(kDecayTokens, tokens - t0);
@@ -96,8 +94,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 gla_decay_mma_kernel(const T *__restrict__ proj, int ld, int col0, const T *__restrict__ w, const float *__restrict__ bias, float inv_tau,
                      float *__restrict__ decay, int tokens, int rank, int channels, int steps) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int NB = 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, nb = rank / 32;
     const int t0 = blockIdx.x * 16 + g, t1 = t0 + 8;
@@ -133,8 +129,6 @@ __global__ void __launch_bounds__(kGlaThreads)
 gla_recurrent_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ decay, float *__restrict__ state, float *__restrict__ o,
                      const int *__restrict__ seq_start, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int heads,
                      int dim, int vdim, int min_tokens, int max_tokens) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ float sm[];
     float *S = sm;
     float *qs = S + (size_t)dim * kGlaCols;
@@ -195,8 +189,6 @@ __global__ void __launch_bounds__(256)
 gla_recurrent_reg_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ decay, float *__restrict__ state, float *__restrict__ o,
                          const int *__restrict__ seq_start, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int heads,
                          int dim, int vdim, int min_tokens, int max_tokens) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) float smf[];
     constexpr int DP = 32 * RR;                                  // padded rows
     constexpr int kStage = TB * DP * 4 + TB * kGlaCols;          // floats per stage: {a, k, q, -} [TB][DP] | v [TB][32]
@@ -362,8 +354,6 @@ __global__ void __launch_bounds__(256)
 gla_step_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ decay, float *__restrict__ state, float *__restrict__ o,
                 const int *__restrict__ seq_start, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int heads, int dim,
                 int vdim) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) float smf[];  // {a, k, q, -}[dim] | part[kStepRowGroups][kStepCols]
     const int s = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * kStepCols;
     const int t = seq_start[s];
@@ -429,15 +419,13 @@ static void launch_gla_reg(const void *proj, int ld, const float *decay, float *
                            const int *seq_slot, dim3 grid, int heads, int dim, int vdim, int min_tokens, int max_tokens, cudaStream_t st) {
     const size_t smem = 2 * ((size_t)TB * 32 * RR * 4 + (size_t)TB * kGlaCols) * sizeof(float);
     if (smem > 48 * 1024) cudaFuncSetAttribute(gla_recurrent_reg_kernel<T, RR, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(gla_recurrent_reg_kernel<T, RR, TB>, dim3(grid), dim3(256), smem, st, true, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim, min_tokens, max_tokens);
+    launch_pdl(gla_recurrent_reg_kernel<T, RR, TB>, dim3(grid), dim3(256), smem, st, false, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim, min_tokens, max_tokens);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256)
 gla_output_kernel(const float *__restrict__ o, const float *__restrict__ w, float eps, const T *__restrict__ gate_in, int gate_ld,
                   T *__restrict__ out, int heads, int vdim, int tokens, int by_warp) {
-    pdl_launch_dependents();
-    pdl_wait();
     __shared__ float red[33];
     constexpr int V = Elem<T>::kVec;
     if (by_warp) {  // a warp per (token, head): rows of up to 32 pieces
@@ -508,15 +496,15 @@ int launch_gla_decay(int dtype, const void *proj, int ld, int col0, const void *
         const int tiles = (tokens + 15) / 16, groups = (channels + 63) / 64;
         const int steps = std::max(1, std::min(groups, groups * tiles / (4 * sm_count())));  // about four CTAs per SM
         const dim3 grid(tiles, (groups + steps - 1) / steps);
-        if (dtype == B200_BF16) launch_pdl(gla_decay_mma_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, true, (const __nv_bfloat16 *)proj, ld, col0, (const __nv_bfloat16 *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels, steps);
-        else launch_pdl(gla_decay_mma_kernel<__half>, dim3(grid), dim3(256), 0, st, true, (const __half *)proj, ld, col0, (const __half *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels, steps);
+        if (dtype == B200_BF16) launch_pdl(gla_decay_mma_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, false, (const __nv_bfloat16 *)proj, ld, col0, (const __nv_bfloat16 *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels, steps);
+        else launch_pdl(gla_decay_mma_kernel<__half>, dim3(grid), dim3(256), 0, st, false, (const __half *)proj, ld, col0, (const __half *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels, steps);
         return cuda_status("gla_decay launch");
     }
     B200_DISPATCH_DTYPE(dtype, {
         // few token blocks (decoding): the channels are spread over CTAs as well
         const int nb = (tokens + kDecayTokens - 1) / kDecayTokens;
         const int cb = nb >= 64 ? 1 : (channels + 255) / 256;
-        launch_pdl(gla_decay_kernel<T>, dim3(nb, cb), dim3(256), (size_t)kDecayTokens * rank * sizeof(float), st, true, (const T *)proj, ld, col0, (const T *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels);
+        launch_pdl(gla_decay_kernel<T>, dim3(nb, cb), dim3(256), (size_t)kDecayTokens * rank * sizeof(float), st, false, (const T *)proj, ld, col0, (const T *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels);
     });
     return cuda_status("gla_decay launch");
 }
@@ -532,7 +520,7 @@ int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay
         const dim3 grid_step((vdim + kStepCols - 1) / kStepCols, heads, n_seqs);
         B200_DISPATCH_DTYPE(dtype, {
             if (smem_step > 48 * 1024) cudaFuncSetAttribute(gla_step_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_step);
-            launch_pdl(gla_step_kernel<T>, dim3(grid_step), dim3(256), smem_step, st, true, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim);
+            launch_pdl(gla_step_kernel<T>, dim3(grid_step), dim3(256), smem_step, st, false, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim);
         });
         if (!(kinds & kGlaManyTokens)) return cuda_status("gla_step launch");
     }
@@ -554,7 +542,7 @@ int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(gla_recurrent_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(gla_recurrent_kernel<T>, dim3(grid), dim3(kGlaThreads), smem, st, true, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim,
+        launch_pdl(gla_recurrent_kernel<T>, dim3(grid), dim3(kGlaThreads), smem, st, false, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim,
                                                                   vdim, min_tokens, max_tokens);
     });
     return cuda_status("gla_recurrent launch");
@@ -567,13 +555,13 @@ int launch_gla_output(int dtype, const float *o, const float *w, float eps, cons
         constexpr int V = Elem<T>::kVec;
         // whole pieces, at most a warp of them per row: eight rows per CTA (one per CTA: 21 us for 32768 rows of 256, half of it CTAs coming and going)
         if (vdim % V == 0 && vdim / V <= 32 && gate_ld % V == 0 && all_aligned16({o, gate_in, out})) {
-            launch_pdl(gla_output_kernel<T>, dim3((unsigned)(((size_t)tokens * heads + 7) / 8)), dim3(256), 0, st, true, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim,
+            launch_pdl(gla_output_kernel<T>, dim3((unsigned)(((size_t)tokens * heads + 7) / 8)), dim3(256), 0, st, false, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim,
                        tokens, 1);
             return cuda_status("gla_output launch");
         }
         // rows that go in 16-byte pieces need one thread per piece; others keep 128 threads striding the row
         const int threads = (vdim % V == 0 && vdim / V <= 128) ? std::max(32, (vdim / V + 31) / 32 * 32) : 128;
-        launch_pdl(gla_output_kernel<T>, dim3(tokens, heads), dim3(threads), 0, st, true, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim, tokens, 0);
+        launch_pdl(gla_output_kernel<T>, dim3(tokens, heads), dim3(threads), 0, st, false, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim, tokens, 0);
     });
     return cuda_status("gla_output launch");
 }

@@ -48,8 +48,6 @@ static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 template <typename T>
 __global__ void embed_rows_kernel(const int *__restrict__ ids, const T *__restrict__ table, float *__restrict__ x, T *__restrict__ h2, int h2_ld,
                                   int width, int vocab, float scale, bool vec) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x;
     int id = ids[t];
     id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);  // the host has refused ids outside the vocabulary
@@ -78,8 +76,6 @@ __global__ void __launch_bounds__(256)
 postnorm_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, const T *__restrict__ y_rows, const int *__restrict__ pair_row,
                          int top, const T *__restrict__ y_shared, const float *__restrict__ shared_gate, const float *__restrict__ g, float eps,
                          int width, float *__restrict__ trace, T *__restrict__ h_out) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) float ys[];  // [width]
     __shared__ float red[33];
     const int t = blockIdx.x;
@@ -213,8 +209,6 @@ sublayer_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, c
                          const float *__restrict__ shared_gate, const T *h_in, int norm, const float *__restrict__ post,
                          const float *__restrict__ ls, float eps, const float *__restrict__ pre, int width, float *__restrict__ trace, T *h_out,
                          int has_y, float branch_scale) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) float ys[];  // [width]
     __shared__ float red[33];
     constexpr int V = Elem<T>::kVec;
@@ -328,8 +322,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 final_dyt_rows_kernel(const float *__restrict__ x, const int *__restrict__ rows, const float *__restrict__ p, float *__restrict__ out,
                       T *__restrict__ out_t, int width) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int i = blockIdx.x;
     const float *xr = x + (size_t)rows[i] * width;
     const float alpha = p[2 * width];
@@ -341,8 +333,6 @@ final_dyt_rows_kernel(const float *__restrict__ x, const int *__restrict__ rows,
 }
 
 __global__ void softcap_kernel(float *__restrict__ logits, size_t n, float scale, float cap) {
-    pdl_launch_dependents();
-    pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float v = logits[i] * scale;
         logits[i] = cap > 0.0f ? cap * tanhf(v / cap) : v;
@@ -353,8 +343,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 final_norm_rows_kernel(const float *__restrict__ x, const int *__restrict__ rows, const float *__restrict__ g, float eps, float *__restrict__ out,
                        T *__restrict__ out_t, int width) {
-    pdl_launch_dependents();
-    pdl_wait();
     __shared__ float red[33];
     const int i = blockIdx.x;
     const float *xr = x + (size_t)rows[i] * width;
@@ -376,8 +364,6 @@ template <typename TX, typename TW, int PM>
 __global__ void __launch_bounds__(256)
 proj_f32_kernel(const TX *__restrict__ x, int ldx, const TW *__restrict__ w, const float *__restrict__ bias, float *__restrict__ y, int ldy, int M,
                 int N, int K, int cols_per_cta) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ float xs[];  // [PM][K]
     const int m0 = blockIdx.y * PM, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < PM * K; i += blockDim.x) {
@@ -407,8 +393,6 @@ template <typename TX, typename TW>
 __global__ void __launch_bounds__(256)
 proj_f32_small_kernel(const TX *__restrict__ x, int ldx, const TW *__restrict__ w, const float *__restrict__ bias, float *__restrict__ y, int ldy,
                       int M, int N, int K, bool vec) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int o = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (o >= M * N) return;
     const int mrow = o / N, n = o - mrow * N;
@@ -451,8 +435,6 @@ template <typename T, int PM>
 __global__ void __launch_bounds__(256)
 proj_f32_rows_kernel(const T *__restrict__ x, int ldx, const T *__restrict__ w, const float *__restrict__ bias, float *__restrict__ y, int ldy, int M,
                      int N, int K) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int V = Elem<T>::kVec;
     const int n = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= N) return;
@@ -489,7 +471,7 @@ static void launch_proj_f32_t(const void *x, int ldx, const void *w, const float
     int cols = (N * mt + 4 * 148 - 1) / (4 * 148);
     cols = cols < 8 ? 8 : (cols + 7) / 8 * 8;
     if (smem > 48 * 1024) cudaFuncSetAttribute(proj_f32_kernel<TX, TW, PM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(proj_f32_kernel<TX, TW, PM>, dim3((N + cols - 1) / cols, mt), dim3(256), smem, st, true, (const TX *)x, ldx, (const TW *)w, bias, y, ldy, M, N, K, cols);
+    launch_pdl(proj_f32_kernel<TX, TW, PM>, dim3((N + cols - 1) / cols, mt), dim3(256), smem, st, false, (const TX *)x, ldx, (const TW *)w, bias, y, ldy, M, N, K, cols);
 }
 
 int launch_proj_f32(int x_dtype, const void *x, int ldx, int w_dtype, const void *w, const float *bias, float *y, int ldy, int M, int N,
@@ -499,19 +481,19 @@ int launch_proj_f32(int x_dtype, const void *x, int ldx, int w_dtype, const void
         const int grid = (M * N + 7) / 8;
         B200_DISPATCH_DTYPE(w_dtype, {
             const bool vec = K % 8 == 0 && ldx % 8 == 0 && all_aligned16({x, w});
-            if (x_dtype == B200_F32) launch_pdl(proj_f32_small_kernel<float, T>, dim3(grid), dim3(256), 0, st, true, (const float *)x, ldx, (const T *)w, bias, y, ldy, M, N, K, vec);
-            else launch_pdl(proj_f32_small_kernel<T, T>, dim3(grid), dim3(256), 0, st, true, (const T *)x, ldx, (const T *)w, bias, y, ldy, M, N, K, vec);
+            if (x_dtype == B200_F32) launch_pdl(proj_f32_small_kernel<float, T>, dim3(grid), dim3(256), 0, st, false, (const float *)x, ldx, (const T *)w, bias, y, ldy, M, N, K, vec);
+            else launch_pdl(proj_f32_small_kernel<T, T>, dim3(grid), dim3(256), 0, st, false, (const T *)x, ldx, (const T *)w, bias, y, ldy, M, N, K, vec);
         });
         return cuda_status("proj_f32 (small) launch");
     }
     if (M <= 16 && x_dtype == w_dtype && w_dtype != B200_F32 && K % 8 == 0 && ldx % 8 == 0 && K >= 512 && aligned16(x) && aligned16(w)) {
         const int grid = (N + 7) / 8;
         if (w_dtype == B200_BF16) {
-            if (M <= 8) launch_pdl(proj_f32_rows_kernel<__nv_bfloat16, 8>, dim3(grid), dim3(256), 0, st, true, (const __nv_bfloat16 *)x, ldx, (const __nv_bfloat16 *)w, bias, y, ldy, M, N, K);
-            else launch_pdl(proj_f32_rows_kernel<__nv_bfloat16, 16>, dim3(grid), dim3(256), 0, st, true, (const __nv_bfloat16 *)x, ldx, (const __nv_bfloat16 *)w, bias, y, ldy, M, N, K);
+            if (M <= 8) launch_pdl(proj_f32_rows_kernel<__nv_bfloat16, 8>, dim3(grid), dim3(256), 0, st, false, (const __nv_bfloat16 *)x, ldx, (const __nv_bfloat16 *)w, bias, y, ldy, M, N, K);
+            else launch_pdl(proj_f32_rows_kernel<__nv_bfloat16, 16>, dim3(grid), dim3(256), 0, st, false, (const __nv_bfloat16 *)x, ldx, (const __nv_bfloat16 *)w, bias, y, ldy, M, N, K);
         } else {
-            if (M <= 8) launch_pdl(proj_f32_rows_kernel<__half, 8>, dim3(grid), dim3(256), 0, st, true, (const __half *)x, ldx, (const __half *)w, bias, y, ldy, M, N, K);
-            else launch_pdl(proj_f32_rows_kernel<__half, 16>, dim3(grid), dim3(256), 0, st, true, (const __half *)x, ldx, (const __half *)w, bias, y, ldy, M, N, K);
+            if (M <= 8) launch_pdl(proj_f32_rows_kernel<__half, 8>, dim3(grid), dim3(256), 0, st, false, (const __half *)x, ldx, (const __half *)w, bias, y, ldy, M, N, K);
+            else launch_pdl(proj_f32_rows_kernel<__half, 16>, dim3(grid), dim3(256), 0, st, false, (const __half *)x, ldx, (const __half *)w, bias, y, ldy, M, N, K);
         }
         return cuda_status("proj_f32 (rows) launch");
     }
@@ -544,8 +526,6 @@ template <typename T, int V>
 __global__ void __launch_bounds__(256)
 ln_residual_kernel(float *__restrict__ x, const T *__restrict__ y, const float *__restrict__ y32, const float *__restrict__ bias, int replace,
                    const float *__restrict__ ln, float eps, int width, T *__restrict__ h_out, int h_ld, float *__restrict__ trace) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) float row[];  // [width]
     __shared__ float red[33];
     const int t = blockIdx.x;
@@ -606,8 +586,6 @@ ln_residual_kernel(float *__restrict__ x, const T *__restrict__ y, const float *
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 gated_act_strided_kernel(const T *__restrict__ in, int in_ld, int gate_col, int up_col, T *__restrict__ out, int out_ld, int inner, int act) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int V = VEC ? Elem<T>::kVec : 1;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (c >= inner) return;
@@ -629,8 +607,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 final_ln_rows_kernel(const float *__restrict__ x, const int *__restrict__ rows, const float *__restrict__ p, int has_bias, float eps,
                      float *__restrict__ out, T *__restrict__ out_t, int width) {
-    pdl_launch_dependents();
-    pdl_wait();
     __shared__ float red[33];
     const int i = blockIdx.x;
     const float *xr = x + (size_t)rows[i] * width;
@@ -644,6 +620,53 @@ final_ln_rows_kernel(const float *__restrict__ x, const int *__restrict__ rows, 
         const float v = fmaf((xr[c] - mean) * inv, p[c], has_bias ? p[width + c] : 0.0f);
         out[(size_t)i * width + c] = v;
         if (out_t) out_t[(size_t)i * width + c] = Elem<T>::from_f(v);
+    }
+}
+
+// final_norm_rows / final_ln_rows for rows of up to 4096 columns in 16-byte pieces: the row is read once and stays in registers (a few rows mean a few CTAs,
+// and three passes of one value per load made 10 to 12 us of round trips).  LN: p = [w (width) | b (width), optional], else p = w
+template <typename T, bool LN>
+__global__ void __launch_bounds__(256)
+final_rows_kernel(const float *__restrict__ x, const int *__restrict__ rows, const float *__restrict__ p, int has_bias, float eps, float *__restrict__ out,
+                  T *__restrict__ out_t, int width) {
+    __shared__ float red[33];
+    const int i = blockIdx.x;
+    const float *xr = x + (size_t)rows[i] * width;
+    constexpr int HELD = 4;
+    float v[HELD][4], sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < HELD; ++j) {
+        const int c = (threadIdx.x + j * 256) * 4;
+        if (c < width) {
+            load_n<float, 4>(xr + c, v[j]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum = LN ? sum + v[j][e] : fmaf(v[j][e], v[j][e], sum);
+        }
+    }
+    sum = block_sum(sum, red);
+    const float mean = LN ? sum / (float)width : 0.0f;
+    if (LN) {
+        sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < HELD; ++j)
+            if ((threadIdx.x + j * 256) * 4 < width) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sum = fmaf(v[j][e] - mean, v[j][e] - mean, sum);
+            }
+        sum = block_sum(sum, red);
+    }
+    const float inv = rsqrtf(sum / (float)width + eps);
+#pragma unroll
+    for (int j = 0; j < HELD; ++j) {
+        const int c = (threadIdx.x + j * 256) * 4;
+        if (c >= width) continue;
+        float w[4], b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        load_n<float, 4>(p + c, w);
+        if (LN && has_bias) load_n<float, 4>(p + width + c, b);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[j][e] = LN ? fmaf((v[j][e] - mean) * inv, w[e], b[e]) : v[j][e] * inv * w[e];
+        store_n<float, 4>(out + (size_t)i * width + c, v[j]);
+        if (out_t) store_n<T, 4>(out_t + (size_t)i * width + c, v[j]);
     }
 }
 
@@ -665,8 +688,6 @@ stream_residual_kernel(float *xs, int S_any, const float *__restrict__ x_init, c
                        const float *__restrict__ na, const float *__restrict__ nb, float sa, float sb, const float *__restrict__ hc,
                        const float *__restrict__ hc_next, const float *__restrict__ ln_next, float eps, int width, T *__restrict__ h_out,
                        float *__restrict__ sum_out, float *__restrict__ trace) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) float row[];  // [width]
     __shared__ float red[33];
     constexpr int N = VEC ? 4 : 1, SM = SC > 0 ? SC : kMaxStreams;
@@ -1418,7 +1439,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     auto ln_residual = [&](const void *y, const float *y32, const float *bias, const float *ln, void *h_out, int h_ld, float *trace) -> int {
         B200_DISPATCH_DTYPE(dt, {
             const bool vec = width % 4 == 0 && h_ld % 4 == 0 && all_aligned16({m->x, y, y32, bias, ln, h_out, trace});
-            launch_pdl((vec ? ln_residual_kernel<T, 4> : ln_residual_kernel<T, 1>), dim3(NT), dim3(256), (size_t)width * sizeof(float), st, true, m->x, (const T *)y, y32, bias, y32 ? 1 : 0, ln, c.norm_eps, width, (T *)h_out, h_ld, trace);
+            launch_pdl((vec ? ln_residual_kernel<T, 4> : ln_residual_kernel<T, 1>), dim3(NT), dim3(256), (size_t)width * sizeof(float), st, false, m->x, (const T *)y, y32, bias, y32 ? 1 : 0, ln, c.norm_eps, width, (T *)h_out, h_ld, trace);
         });
         return cuda_status("ln_residual launch");
     };
@@ -1431,7 +1452,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     auto embed = [&](void *h2, int h2_ld) -> int {
         const bool vec = width % 8 == 0 && h2_ld % 8 == 0 && all_aligned16({m->embedding, m->x, h2});
         B200_DISPATCH_DTYPE(dt, {
-            launch_pdl(embed_rows_kernel<T>, dim3(NT), dim3(256), 0, st, true, d_ids, (const T *)m->embedding, m->x, (T *)h2, h2_ld, width, c.vocab, c.embed_scale != 0.0f ? c.embed_scale : 1.0f, vec);
+            launch_pdl(embed_rows_kernel<T>, dim3(NT), dim3(256), 0, st, false, d_ids, (const T *)m->embedding, m->x, (T *)h2, h2_ld, width, c.vocab, c.embed_scale != 0.0f ? c.embed_scale : 1.0f, vec);
         });
         return cuda_status("embed_rows launch");
     };
@@ -1549,7 +1570,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         // four columns per access when every row starts on a 16-byte boundary (the scratch buffers do; norm vectors and the trace are the caller's)
         const bool vec = width % 4 == 0 && ((reinterpret_cast<size_t>(na) | reinterpret_cast<size_t>(nb) | reinterpret_cast<size_t>(ln_next) |
                                               reinterpret_cast<size_t>(trace)) & 15) == 0;
-#define B200_STREAMS(SC, V) launch_pdl(stream_residual_kernel<T, SC, V>, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, true, \
+#define B200_STREAMS(SC, V) launch_pdl(stream_residual_kernel<T, SC, V>, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, false, \
     m->xs, n_streams, x_init, (const T *)ya, (const T *)yb, na, nb, sa, sb, hc, hc_next, ln_next, c.norm_eps, width, ln_next ? (T *)m->h : nullptr, sum_out, trace)
 #define B200_STREAMS_V(SC) do { if (vec) B200_STREAMS(SC, true); else B200_STREAMS(SC, false); } while (0)
         B200_DISPATCH_DTYPE(dt, {
@@ -1618,8 +1639,8 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                 const bool vec = lp.n_in % V == 0 && col % V == 0 && l.expert_ff % V == 0 && n_cat % V == 0 && ocol % V == 0;
                 const int per = vec ? V : 1;
                 const dim3 grid((l.expert_ff / per + 255) / 256, NT);
-                if (vec) launch_pdl(gated_act_strided_kernel<T, true>, dim3(grid), dim3(256), 0, st, true, (const T *)m->proj, lp.n_in, col, col + l.expert_ff, (T *)m->cat + ocol, n_cat, l.expert_ff, l.act);
-                else launch_pdl(gated_act_strided_kernel<T, false>, dim3(grid), dim3(256), 0, st, true, (const T *)m->proj, lp.n_in, col, col + l.expert_ff, (T *)m->cat + ocol, n_cat, l.expert_ff, l.act);
+                if (vec) launch_pdl(gated_act_strided_kernel<T, true>, dim3(grid), dim3(256), 0, st, false, (const T *)m->proj, lp.n_in, col, col + l.expert_ff, (T *)m->cat + ocol, n_cat, l.expert_ff, l.act);
+                else launch_pdl(gated_act_strided_kernel<T, false>, dim3(grid), dim3(256), 0, st, false, (const T *)m->proj, lp.n_in, col, col + l.expert_ff, (T *)m->cat + ocol, n_cat, l.expert_ff, l.act);
             });
             RUN(cuda_status("gated_act_strided launch"));
         }
@@ -1664,7 +1685,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     auto postnorm = [&](const void *y_dense, const void *y_rows, const int *pair_row, int top, const void *y_shared, const float *gate,
                         const float *g, float *trace) -> int {
         B200_DISPATCH_DTYPE(dt, {
-            launch_pdl(postnorm_residual_kernel<T>, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, true, m->x, (const T *)y_dense, (const T *)y_rows, pair_row, top,
+            launch_pdl(postnorm_residual_kernel<T>, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, false, m->x, (const T *)y_dense, (const T *)y_rows, pair_row, top,
                                                                                       (const T *)y_shared, gate, g, c.norm_eps, width, trace,
                                                                                       f32 ? nullptr : (T *)m->h);
         });
@@ -1679,7 +1700,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             const bool vec = width % Elem<T>::kVec == 0 && ((reinterpret_cast<size_t>(trace) | reinterpret_cast<size_t>(post) | reinterpret_cast<size_t>(ls) |
                                                               reinterpret_cast<size_t>(pre) | reinterpret_cast<size_t>(y_bias)) & 15) == 0;
             auto kern = vec ? sublayer_residual_kernel<T, true> : sublayer_residual_kernel<T, false>;
-            launch_pdl(kern, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, true, m->x, (const T *)y_dense, y_bias, (const T *)y_rows, pair_row, pair_weight, top,
+            launch_pdl(kern, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, false, m->x, (const T *)y_dense, y_bias, (const T *)y_rows, pair_row, pair_weight, top,
                                                                 (const T *)y_shared, gate, (const T *)m->h, norm, post, ls, c.norm_eps, pre, width, trace,
                                                                 (pre || !f32) ? (T *)m->h : nullptr, has_y ? 1 : 0,
                                                                 c.branch_scale != 0.0f ? c.branch_scale : 1.0f);
@@ -1890,10 +1911,15 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     if (W > 0) {
         // the wanted rows only: final norm (fp32 and, for 16-bit engines, a 16-bit copy in h), then the LM head with fp32 logits
         B200_DISPATCH_DTYPE(dt, {
-            if (c.final_norm == B200_NORM_LN_PARALLEL || c.final_norm == B200_NORM_LN_PRE || c.final_norm == B200_NORM_LN_POST)
-                launch_pdl(final_ln_rows_kernel<T>, dim3(W), dim3(256), 0, st, true, m->x, d_want, m->final_norm, c.final_norm != B200_NORM_LN_POST, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
-            else if (c.final_norm == B200_NORM_DYT_PRE_POST) launch_pdl(final_dyt_rows_kernel<T>, dim3(W), dim3(256), 0, st, true, m->x, d_want, m->final_norm, m->xn, f32 ? nullptr : (T *)m->h, width);
-            else launch_pdl(final_norm_rows_kernel<T>, dim3(W), dim3(256), 0, st, true, m->x, d_want, m->final_norm, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
+            const bool ln = c.final_norm == B200_NORM_LN_PARALLEL || c.final_norm == B200_NORM_LN_PRE || c.final_norm == B200_NORM_LN_POST;
+            const bool vec = width % 4 == 0 && width <= 4096 && c.final_norm != B200_NORM_DYT_PRE_POST && all_aligned16({m->x, m->final_norm, m->xn, m->h});
+            if (vec)
+                launch_pdl(ln ? final_rows_kernel<T, true> : final_rows_kernel<T, false>, dim3(W), dim3(256), 0, st, false, m->x, d_want, m->final_norm,
+                           c.final_norm != B200_NORM_LN_POST ? 1 : 0, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
+            else if (ln)
+                launch_pdl(final_ln_rows_kernel<T>, dim3(W), dim3(256), 0, st, false, m->x, d_want, m->final_norm, c.final_norm != B200_NORM_LN_POST, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
+            else if (c.final_norm == B200_NORM_DYT_PRE_POST) launch_pdl(final_dyt_rows_kernel<T>, dim3(W), dim3(256), 0, st, false, m->x, d_want, m->final_norm, m->xn, f32 ? nullptr : (T *)m->h, width);
+            else launch_pdl(final_norm_rows_kernel<T>, dim3(W), dim3(256), 0, st, false, m->x, d_want, m->final_norm, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
         });
         rc = W <= 16 ? launch_rows_f32out(dt, m->h, m->lm_head, logits, W, c.vocab, width, st) : B200_ERR_UNSUPPORTED;
         if (rc == B200_ERR_UNSUPPORTED) rc = launch_dense_f32out(dt, m->h, m->lm_head, logits, W, c.vocab, width, st);
@@ -1902,7 +1928,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         const float lscale = c.logit_scale != 0.0f ? c.logit_scale : 1.0f;
         if (c.logit_softcap > 0.0f || lscale != 1.0f) {
             const size_t n = (size_t)W * c.vocab;
-            launch_pdl(softcap_kernel, dim3((unsigned)std::min<size_t>((n + 255) / 256, 148 * 8)), dim3(256), 0, st, true, logits, n, lscale, c.logit_softcap);
+            launch_pdl(softcap_kernel, dim3((unsigned)std::min<size_t>((n + 255) / 256, 148 * 8)), dim3(256), 0, st, false, logits, n, lscale, c.logit_softcap);
         }
     }
 #undef RUN

@@ -23,24 +23,6 @@ template <typename T> __device__ __forceinline__ void store8(T *__restrict__ p, 
 }
 
 
-// ---- a (token, head) whose keys are shared out over the CTAs of a cluster (decoded tokens of the chunked and the scored attention)
-__device__ __forceinline__ void cluster_barrier() { asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ float peer_value(const float *smem, int rank) {  // the same shared variable in CTA `rank` of the cluster
-    uint32_t at;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(smem)), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
-    return v;
-}
-// CTAs per (token, head): one CTA walks 1024 keys in eight rounds of scores and four of values, each a round trip behind the block table's; with the keys
-// over a cluster a round or two are left (3 tokens x 16 heads, window of 1024: 41 -> 23 us).  Only while all CTAs run at once -- two of 512 threads per SM:
-// 16 tokens x 16 heads in twos were 31 us against 19 -- and each keeps a round of keys.
-inline int key_splits(long long rows, int max_keys) {
-    int n = 1;
-    while (n < 8 && rows * n * 2 <= 2LL * sm_count() && max_keys / (2 * n) >= 128) n *= 2;
-    return n;
-}
-
 // attention_chunked.cu
 int launch_attn_qk_norm_cache(int dtype, const void *proj, int ld, void *q_out, void *k_pool, void *v_pool, const float *q_norm,
                               const float *k_norm, float eps, const int *tok_seq, const int *tok_pos, const int *block_table, int mpps,

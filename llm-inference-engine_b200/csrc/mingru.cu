@@ -54,8 +54,6 @@ template <typename T, int N>
 __global__ void __launch_bounds__(32 * kSubs)
 mingru_chunk_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ bias, const float *__restrict__ state, float *__restrict__ maps,
                     const int4 *__restrict__ chunks, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int cols) {
-    pdl_launch_dependents();
-    pdl_wait();
     __shared__ float sa[kSubs][32 * N], sb[kSubs][32 * N];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = (blockIdx.x * 32 + lane) * N;
     const int4 ch = chunks[blockIdx.y];  // sequence, first packed row, tokens, index in its portion
@@ -104,8 +102,6 @@ template <typename T, int N>
 __global__ void __launch_bounds__(32 * kSubs)
 mingru_apply_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ bias, float *__restrict__ state, const float *__restrict__ maps,
                     T *__restrict__ out, const int4 *__restrict__ chunks, const int *__restrict__ seq_start, const int *__restrict__ seq_slot, int cols) {
-    pdl_launch_dependents();
-    pdl_wait();
     __shared__ float sa[kSubs][32 * N], sb[kSubs][32 * N];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = (blockIdx.x * 32 + lane) * N;
     const int4 ch = chunks[blockIdx.y];
@@ -173,8 +169,6 @@ template <typename T, int N>
 __global__ void __launch_bounds__(128)
 mingru_step_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ bias, float *__restrict__ state, T *__restrict__ out,
                    const int *__restrict__ seq_start, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int cols) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * N, q = blockIdx.y;
     const int t0 = seq_start[q], t1 = seq_start[q + 1];
     if (c >= cols || t1 == t0 || t1 - t0 >= kMingruShort) return;
@@ -212,12 +206,12 @@ int launch_mingru(int dtype, const void *proj, int ld, const float *bias, float 
             auto chunk = vec ? mingru_chunk_kernel<T, 4> : mingru_chunk_kernel<T, 1>;
             auto apply = vec ? mingru_apply_kernel<T, 4> : mingru_apply_kernel<T, 1>;
             const dim3 grid((cols + 32 * n - 1) / (32 * n), n_chunks);
-            launch_pdl(chunk, dim3(grid), dim3(32 * kSubs), 0, st, true, (const T *)proj, ld, bias, state, maps, ch, seq_pos0, seq_slot, cols);
-            launch_pdl(apply, dim3(grid), dim3(32 * kSubs), 0, st, true, (const T *)proj, ld, bias, state, maps, (T *)out, ch, seq_start, seq_slot, cols);
+            launch_pdl(chunk, dim3(grid), dim3(32 * kSubs), 0, st, false, (const T *)proj, ld, bias, state, maps, ch, seq_pos0, seq_slot, cols);
+            launch_pdl(apply, dim3(grid), dim3(32 * kSubs), 0, st, false, (const T *)proj, ld, bias, state, maps, (T *)out, ch, seq_start, seq_slot, cols);
         }
         if (n_short > 0) {
             auto step = vec ? mingru_step_kernel<T, 4> : mingru_step_kernel<T, 1>;
-            launch_pdl(step, dim3(blocks, n_seqs), dim3(threads), 0, st, true, (const T *)proj, ld, bias, state, (T *)out, seq_start, seq_pos0, seq_slot, cols);
+            launch_pdl(step, dim3(blocks, n_seqs), dim3(threads), 0, st, false, (const T *)proj, ld, bias, state, (T *)out, seq_start, seq_pos0, seq_slot, cols);
         }
     });
     return cuda_status("mingru launch");

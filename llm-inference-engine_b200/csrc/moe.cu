@@ -22,8 +22,6 @@ namespace b200 {
 // one warp per token
 __global__ void moe_route_sigmoid_kernel(const float *__restrict__ logits, int ld, int *__restrict__ sel_expert, float *__restrict__ sel_weight,
                                          float *__restrict__ shared_gate, int tokens, int experts, int top) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
     if (t >= tokens) return;
     const float *z = logits + (size_t)t * ld;
@@ -54,8 +52,6 @@ __global__ void moe_route_sigmoid_kernel(const float *__restrict__ logits, int l
 // logits, which order the scores and do not underflow.
 __global__ void moe_route_softmax_kernel(const float *__restrict__ logits, int ld, const float *__restrict__ bias, const float *__restrict__ logit_bias,
                                          int *__restrict__ sel_expert, float *__restrict__ sel_weight, int tokens, int outputs, int top) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
     if (t >= tokens) return;
     const float *row = logits + (size_t)t * ld;
@@ -100,8 +96,6 @@ __global__ void moe_route_softmax_kernel(const float *__restrict__ logits, int l
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int *__restrict__ sel_expert, const float *__restrict__ sel_weight, int *__restrict__ row_token, float *__restrict__ row_weight,
                 int *__restrict__ tile_expert, int *__restrict__ pair_row, int *__restrict__ n_tiles, int pairs, int experts, int top, int tile) {
-    pdl_launch_dependents();
-    pdl_wait();
     // choices >= experts (identity experts) own no row: pair_row = -1
     extern __shared__ int si[];
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -183,8 +177,6 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 moe_gather_kernel(const float *__restrict__ x, const int *__restrict__ row_token, const float *__restrict__ row_weight, T *__restrict__ xg,
                   const int *__restrict__ n_tiles, int width, int tile) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int r = blockIdx.x;
     if (r >= *n_tiles * tile) return;
     const int t = row_token[r];
@@ -216,8 +208,6 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 moe_gather_rows_kernel(const T *__restrict__ h, const int *__restrict__ row_token, T *__restrict__ xg, const int *__restrict__ n_tiles, int width,
                        int tile, const float *__restrict__ row_weight) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int r = blockIdx.x;
     if (r >= *n_tiles * tile) return;
     const int t = row_token[r];
@@ -264,8 +254,6 @@ __device__ __forceinline__ float gated_apply(float g, float u, int act, float li
 template <typename T>
 __global__ void gated_activation_kernel(const T *__restrict__ in, T *__restrict__ out, int rows, int inner, int act, const int *__restrict__ n_tiles,
                                         int tile, float limit, float slope) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int V = Elem<T>::kVec;
     const int live = n_tiles ? min(rows, *n_tiles * tile) : rows;
     if (inner % V == 0 && ((reinterpret_cast<size_t>(in) | reinterpret_cast<size_t>(out)) & 15) == 0) {
@@ -293,8 +281,6 @@ __global__ void gated_activation_kernel(const T *__restrict__ in, T *__restrict_
 // in place: x[r, c] = act(x[r, c] + bias[c]) (bias may be NULL, act < 0: none); 16-byte pieces when the rows start on 16-byte boundaries
 template <typename T>
 __global__ void bias_activation_kernel(T *__restrict__ x, const float *__restrict__ bias, size_t rows, int cols, int act) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int V = Elem<T>::kVec;
     if (cols % V == 0 && ((reinterpret_cast<size_t>(x) | reinterpret_cast<size_t>(bias)) & 15) == 0) {
         const int per_row = cols / V;
@@ -330,8 +316,6 @@ __global__ void bias_activation_kernel(T *__restrict__ x, const float *__restric
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 poly_norm_kernel(T *__restrict__ x, const float *__restrict__ coef, float eps, int cols) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int N = VEC ? Elem<T>::kVec : 1, KP = VEC ? 4 : 8;
     __shared__ float red[3][9];
     T *row = x + (size_t)blockIdx.x * cols;
@@ -403,8 +387,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 moe_grouped_gemm_kernel(const T *__restrict__ a, const T *__restrict__ w, T *__restrict__ c, const int *__restrict__ tile_expert,
                         const int *__restrict__ n_tiles, int N, int K, int act) {
-    pdl_launch_dependents();
-    pdl_wait();
     if ((int)blockIdx.y >= *n_tiles) return;
     __shared__ float As[kGK][kGT + 4];
     __shared__ float Bs[kGK][kGT + 4];
@@ -473,8 +455,6 @@ template <typename T, typename TC>
 __global__ void __launch_bounds__(128)
 moe_grouped_gemm_mma_kernel(const T *__restrict__ a, const T *__restrict__ w, TC *__restrict__ c, const int *__restrict__ tile_expert,
                             const int *__restrict__ n_tiles, int M, int N, int K, int act) {
-    pdl_launch_dependents();
-    pdl_wait();
     if (n_tiles && (int)blockIdx.y >= *n_tiles) return;
     extern __shared__ __align__(16) unsigned char smraw[];
     T *As = reinterpret_cast<T *>(smraw);               // [stages][64][64]
@@ -555,8 +535,6 @@ template <typename T, typename TC, int NT>
 __global__ void __launch_bounds__(512)
 moe_few_rows_kernel(const T *__restrict__ a, const T *__restrict__ w, TC *__restrict__ c, const int *__restrict__ tile_expert,
                     const int *__restrict__ n_tiles, int tile_rows, int M, int N, int K, int act, int KS, int NG, int steps) {
-    pdl_launch_dependents();
-    pdl_wait();
     if (n_tiles && (int)blockIdx.y >= *n_tiles) return;
     constexpr int NB = 8;  // 32-k blocks of a slice
     extern __shared__ __align__(16) float part[];  // [2][NG][KS][16 tokens x 8 rows]
@@ -617,18 +595,18 @@ int launch_dense_f32out(int dtype, const void *x, const void *w, float *y, int M
         const int KS = (K / 32 + 7) / 8, NG = KS >= 8 ? 1 : 8 / KS, steps = ((N + 7) / 8 + NG - 1) / NG;
         const size_t smem = (size_t)2 * NG * KS * 128 * sizeof(float);
         const dim3 few(1, (M + 15) / 16);
-        if (dtype == B200_BF16) launch_pdl(moe_few_rows_kernel<__nv_bfloat16, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, true, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
-        else launch_pdl(moe_few_rows_kernel<__half, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, true, (const __half *)x, (const __half *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
+        if (dtype == B200_BF16) launch_pdl(moe_few_rows_kernel<__nv_bfloat16, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, false, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
+        else launch_pdl(moe_few_rows_kernel<__half, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, false, (const __half *)x, (const __half *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
         return cuda_status("dense_f32out (few columns) launch");
     }
     const dim3 grid((N + kMN - 1) / kMN, (M + kMoeTileM - 1) / kMoeTileM);
     const size_t smem = (size_t)kMStages * (kMoeTileM + kMN) * kMK * 2;
     if (dtype == B200_BF16) {
         cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__nv_bfloat16, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(moe_grouped_gemm_mma_kernel<__nv_bfloat16, float>, dim3(grid), dim3(128), smem, st, true, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, M, N, K, -1);
+        launch_pdl(moe_grouped_gemm_mma_kernel<__nv_bfloat16, float>, dim3(grid), dim3(128), smem, st, false, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, M, N, K, -1);
     } else {
         cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__half, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(moe_grouped_gemm_mma_kernel<__half, float>, dim3(grid), dim3(128), smem, st, true, (const __half *)x, (const __half *)w, y, nullptr, nullptr, M, N, K, -1);
+        launch_pdl(moe_grouped_gemm_mma_kernel<__half, float>, dim3(grid), dim3(128), smem, st, false, (const __half *)x, (const __half *)w, y, nullptr, nullptr, M, N, K, -1);
     }
     return cuda_status("dense_f32out launch");
 }
@@ -636,8 +614,6 @@ int launch_dense_f32out(int dtype, const void *x, const void *w, float *y, int M
 // one 16-byte piece per thread; the last n % kVec elements (and everything, if x is not 16-byte aligned) one by one
 template <typename T>
 __global__ void activation_kernel(T *__restrict__ x, size_t n, int act, size_t n_vec) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int V = Elem<T>::kVec;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n_vec) {
@@ -655,21 +631,21 @@ __global__ void activation_kernel(T *__restrict__ x, size_t n, int act, size_t n
 int launch_moe_route_sigmoid(const float *logits, int ld, int *sel_expert, float *sel_weight, float *shared_gate, int tokens,
                              int experts, int top, cudaStream_t st) {
     if (tokens == 0) return B200_OK;
-    launch_pdl(moe_route_sigmoid_kernel, dim3((tokens + 3) / 4), dim3(128), 0, st, true, logits, ld, sel_expert, sel_weight, shared_gate, tokens, experts, top);
+    launch_pdl(moe_route_sigmoid_kernel, dim3((tokens + 3) / 4), dim3(128), 0, st, false, logits, ld, sel_expert, sel_weight, shared_gate, tokens, experts, top);
     return cuda_status("moe_route launch");
 }
 
 int launch_moe_route_softmax(const float *logits, int ld, const float *bias, int *sel_expert, float *sel_weight, int tokens, int outputs,
                              int top, cudaStream_t st, const float *logit_bias) {
     if (tokens == 0) return B200_OK;
-    launch_pdl(moe_route_softmax_kernel, dim3((tokens + 3) / 4), dim3(128), 0, st, true, logits, ld, bias, logit_bias, sel_expert, sel_weight, tokens, outputs, top);
+    launch_pdl(moe_route_softmax_kernel, dim3((tokens + 3) / 4), dim3(128), 0, st, false, logits, ld, bias, logit_bias, sel_expert, sel_weight, tokens, outputs, top);
     return cuda_status("moe_route (softmax) launch");
 }
 
 int launch_moe_gather_rows(int dtype, const void *h, const int *row_token, void *xg, const int *n_tiles, int max_rows, int width, int tile,
                            cudaStream_t st, const float *row_weight) {
     if (max_rows == 0) return B200_OK;
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(moe_gather_rows_kernel<T>, dim3(max_rows), dim3(128), 0, st, true, (const T *)h, row_token, (T *)xg, n_tiles, width, tile, row_weight); });
+    B200_DISPATCH_DTYPE(dtype, { launch_pdl(moe_gather_rows_kernel<T>, dim3(max_rows), dim3(128), 0, st, false, (const T *)h, row_token, (T *)xg, n_tiles, width, tile, row_weight); });
     return cuda_status("moe_gather_rows launch");
 }
 
@@ -678,7 +654,7 @@ int launch_gated_activation(int dtype, const void *in, void *out, int rows, int 
     if (rows == 0 || inner == 0) return B200_OK;
     const size_t n = (size_t)rows * inner / 4;
     const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 148 * 16));
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(gated_activation_kernel<T>, dim3(grid), dim3(256), 0, st, true, (const T *)in, (T *)out, rows, inner, act, n_tiles, tile, limit, slope); });
+    B200_DISPATCH_DTYPE(dtype, { launch_pdl(gated_activation_kernel<T>, dim3(grid), dim3(256), 0, st, false, (const T *)in, (T *)out, rows, inner, act, n_tiles, tile, limit, slope); });
     return cuda_status("gated_activation launch");
 }
 
@@ -686,7 +662,7 @@ int launch_bias_activation(int dtype, void *x, const float *bias, size_t rows, i
     if (rows == 0 || cols == 0) return B200_OK;
     const size_t n = rows * cols / 4;
     const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 148 * 16));
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(bias_activation_kernel<T>, dim3(grid), dim3(256), 0, st, true, (T *)x, bias, rows, cols, act); });
+    B200_DISPATCH_DTYPE(dtype, { launch_pdl(bias_activation_kernel<T>, dim3(grid), dim3(256), 0, st, false, (T *)x, bias, rows, cols, act); });
     return cuda_status("bias_activation launch");
 }
 
@@ -697,7 +673,7 @@ int launch_poly_norm(int dtype, void *x, const float *coef, float eps, int rows,
         const int per = vec ? Elem<T>::kVec : 1;
         const int threads = std::min(256, std::max(32, ((cols + per - 1) / per + 31) / 32 * 32));
         auto kern = vec ? poly_norm_kernel<T, true> : poly_norm_kernel<T, false>;
-        launch_pdl(kern, dim3(rows), dim3(threads), 0, st, true, (T *)x, coef, eps, cols);
+        launch_pdl(kern, dim3(rows), dim3(threads), 0, st, false, (T *)x, coef, eps, cols);
     });
     return cuda_status("poly_norm launch");
 }
@@ -708,14 +684,14 @@ int launch_moe_plan(const int *sel_expert, const float *sel_weight, int *row_tok
     const int warps = std::max(1, std::min({32, std::max(8, (pairs + 31) / 32), (int)(40 * 1024 / sizeof(int) / std::max(experts, 1))}));
     const size_t smem = ((size_t)(warps + 2) * experts + 1) * sizeof(int);
     if (smem > 48 * 1024) cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(moe_plan_kernel, dim3(1), dim3(warps * 32), smem, st, true, sel_expert, sel_weight, row_token, row_weight, tile_expert, pair_row, n_tiles, pairs, experts, top, tile);
+    launch_pdl(moe_plan_kernel, dim3(1), dim3(warps * 32), smem, st, false, sel_expert, sel_weight, row_token, row_weight, tile_expert, pair_row, n_tiles, pairs, experts, top, tile);
     return cuda_status("moe_plan launch");
 }
 
 int launch_moe_gather(int dtype, const float *x, const int *row_token, const float *row_weight, void *xg, const int *n_tiles,
                       int max_rows, int width, int tile, cudaStream_t st) {
     if (max_rows == 0) return B200_OK;
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(moe_gather_kernel<T>, dim3(max_rows), dim3(128), 0, st, true, x, row_token, row_weight, (T *)xg, n_tiles, width, tile); });
+    B200_DISPATCH_DTYPE(dtype, { launch_pdl(moe_gather_kernel<T>, dim3(max_rows), dim3(128), 0, st, false, x, row_token, row_weight, (T *)xg, n_tiles, width, tile); });
     return cuda_status("moe_gather launch");
 }
 
@@ -730,7 +706,7 @@ int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, co
         const size_t smem = (size_t)2 * NG * KS * 128 * sizeof(float);
         auto go = [&](auto kern, auto *type) {
             using T = std::remove_pointer_t<decltype(type)>;
-            launch_pdl(kern, dim3(grid), dim3(KS * NG * 32), smem, st, true, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, kMoeTileM, max_tiles * kMoeTileM, N, K, act, KS, NG, steps);
+            launch_pdl(kern, dim3(grid), dim3(KS * NG * 32), smem, st, false, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, kMoeTileM, max_tiles * kMoeTileM, N, K, act, KS, NG, steps);
         };
         if (dtype == B200_BF16) live_rows <= 8 ? go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 1>, (__nv_bfloat16 *)nullptr) : go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 2>, (__nv_bfloat16 *)nullptr);
         else live_rows <= 8 ? go(moe_few_rows_kernel<__half, __half, 1>, (__half *)nullptr) : go(moe_few_rows_kernel<__half, __half, 2>, (__half *)nullptr);
@@ -741,18 +717,18 @@ int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, co
         const size_t smem = (size_t)kMStages * (kMoeTileM + kMN) * kMK * 2;
         if (dtype == B200_BF16) {
             cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__nv_bfloat16, __nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            launch_pdl(moe_grouped_gemm_mma_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(grid), dim3(128), smem, st, true, (const __nv_bfloat16 *)a, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)c,
+            launch_pdl(moe_grouped_gemm_mma_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(grid), dim3(128), smem, st, false, (const __nv_bfloat16 *)a, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)c,
                                                                                                tile_expert, n_tiles, max_tiles * kMoeTileM, N, K, act);
         } else {
             cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__half, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            launch_pdl(moe_grouped_gemm_mma_kernel<__half, __half>, dim3(grid), dim3(128), smem, st, true, (const __half *)a, (const __half *)w, (__half *)c, tile_expert, n_tiles,
+            launch_pdl(moe_grouped_gemm_mma_kernel<__half, __half>, dim3(grid), dim3(128), smem, st, false, (const __half *)a, (const __half *)w, (__half *)c, tile_expert, n_tiles,
                                                                                  max_tiles * kMoeTileM, N, K, act);
         }
         return cuda_status("moe_grouped_gemm (tensor core) launch");
     }
     const dim3 grid((N + kGT - 1) / kGT, max_tiles);
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(moe_grouped_gemm_kernel<T>, dim3(grid), dim3(256), 0, st, true, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, N, K, act);
+        launch_pdl(moe_grouped_gemm_kernel<T>, dim3(grid), dim3(256), 0, st, false, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, N, K, act);
     });
     return cuda_status("moe_grouped_gemm launch");
 }
@@ -762,7 +738,7 @@ int launch_activation(int dtype, void *x, size_t n, int act, cudaStream_t st) {
     B200_DISPATCH_DTYPE(dtype, {
         const size_t n_vec = (reinterpret_cast<size_t>(x) & 15) == 0 ? n / Elem<T>::kVec : 0;
         const size_t threads = n_vec + (n - n_vec * Elem<T>::kVec);
-        launch_pdl(activation_kernel<T>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st, true, (T *)x, n, act, n_vec);
+        launch_pdl(activation_kernel<T>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st, false, (T *)x, n, act, n_vec);
     });
     return cuda_status("activation launch");
 }

@@ -52,17 +52,32 @@ __device__ __forceinline__ uint32_t pa_u32(const void *p) { return (uint32_t)__c
 __device__ __forceinline__ void pa_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
 __device__ __forceinline__ void pa_expect(uint32_t bar, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory"); }
 __device__ __forceinline__ void pa_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ uint32_t pa_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok;
+}
+__device__ unsigned int g_pa_wait_failed;  // a wait that gave up: the launch's results are not valid
+// gives up after 2^31 clocks (about a second; a try may sleep, so tries are no measure), and with it every later wait of the CTA: a fault elsewhere must
+// not hang the device
+__device__ __forceinline__ volatile int &pa_gave_up() {
+    __shared__ volatile int v;
+    return v;
+}
 __device__ __forceinline__ void pa_wait(uint32_t bar, uint32_t parity) {
-    for (int i = 0; i < (1 << 24); ++i) {  // gives up after seconds: a fault elsewhere must not hang the device
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return;
+    if (pa_try(bar, parity)) return;
+    const uint32_t t0 = (uint32_t)clock();
+    while (!pa_try(bar, parity)) {
+        if ((uint32_t)clock() - t0 < 0x7fffffffu && !pa_gave_up()) continue;
+        pa_gave_up() = 1;
+        atomicExch(&g_pa_wait_failed, 1u);
+        return;
     }
 }
 __device__ __forceinline__ void pa_tma(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
@@ -119,8 +134,6 @@ template <int DK, int DV, bool LATENT> struct PaShape {
 template <typename T, int DK, int DV, bool LATENT, bool BIASED>
 __global__ void __launch_bounds__(PaShape<DK, DV, LATENT>::kWarps * 32 + 64, PaShape<DK, DV, LATENT>::kCtas)
 prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const PromptAttn p) {
-    pdl_launch_dependents();
-    pdl_wait();
     using Sh = PaShape<DK, DV, LATENT>;
     constexpr int WARPS = Sh::kWarps, WPR = WARPS / 4, ST = Sh::kStages, SC = kPage / WPR, OC = DV / WPR;  // keys / value columns per thread
     static_assert(SC % 16 == 0 && OC % 16 == 0, "TMEM is read 16 columns at a time");
@@ -148,6 +161,7 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     auto v_item = [&](int j) { return LATENT ? j : (j + 1 < n ? 2 * j + 2 : 2 * j + 1); };
 
     if (warp == WARPS && lane == 0) {
+        pa_gave_up() = 0;
         pa_init(q_full, WARPS);
         for (int s = 0; s < ST; ++s) {
             pa_init(full0 + 8 * s, 1);
@@ -436,9 +450,10 @@ int pa_launch(const PromptAttn &p, const void *k_pool, const void *v_pool, bool 
     }
     using Sh = PaShape<DK, DV, LATENT>;
     auto kern = prompt_attn_tc_kernel<T, DK, DV, LATENT, BIASED>;
-    const size_t smem = Sh::kSmem + 2 * p.pen_len * sizeof(float);
+    // (biased logits: one CTA per SM)
+    const size_t smem = std::max<size_t>(Sh::kSmem + 2 * p.pen_len * sizeof(float), BIASED ? 120 * 1024 : 0);
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(kern, dim3(p.n_tiles, p.heads / 2), dim3(Sh::kWarps * 32 + 64), smem, st, true, tmK, tmV, p);
+    launch_pdl(kern, dim3(p.n_tiles, p.heads / 2), dim3(Sh::kWarps * 32 + 64), smem, st, false, tmK, tmV, p);
     return cuda_status("prompt attention (tcgen05) launch");
 }
 

@@ -60,8 +60,6 @@ delta_prep_kernel(const T *__restrict__ proj, int ld, int col0, const float *__r
                   int rank, int gate_rank, T *__restrict__ lr_a, T *__restrict__ lr_g, float *__restrict__ rec, DeltaRow lay,
                   const int *__restrict__ tok_seq, const int *__restrict__ tok_pos, const int *__restrict__ seq_pos0,
                   const int *__restrict__ seq_slot, int heads, int kv_heads, int dim, int vdim) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ float sh[];  // conv outputs [channels]
     const int t = blockIdx.x, s = tok_seq[t], pos = tok_pos[t], pos0 = seq_pos0[s], slot = seq_slot[s];
     const int nqk = kv_heads * dim, nv = heads * vdim, channels = 2 * nqk + nv;
@@ -113,8 +111,6 @@ delta_prep_tile_kernel(const T *__restrict__ proj, int ld, int col0, const float
                        int gate_rank, T *__restrict__ lr_a, T *__restrict__ lr_g, float *__restrict__ rec, DeltaRow lay, const int *__restrict__ tok_seq,
                        const int *__restrict__ tok_pos, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int tokens, int heads, int kv_heads, int dim, int vdim,
                        int tiles) {
-    pdl_launch_dependents();
-    pdl_wait();
     __shared__ int s_pos[kPrepTokens], s_back[kPrepTokens], s_slot[kPrepTokens];  // position, rows of the own portion before it, state slot
     const int nqk = kv_heads * dim, nv = heads * vdim, channels = 2 * nqk + nv;
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
@@ -221,8 +217,6 @@ delta_prep_direct_kernel(const T *__restrict__ proj, int ld, int col0, const flo
                          const float *__restrict__ decay_bias, const float *__restrict__ a_log, float *__restrict__ rec, DeltaRow lay,
                          const int *__restrict__ tok_seq, const int *__restrict__ tok_pos, const int *__restrict__ seq_pos0,
                          const int *__restrict__ seq_slot, int heads, int kv_heads, int dim, int vdim) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ float sh[];  // conv outputs [channels]
     const int t = blockIdx.x, s = tok_seq[t], pos = tok_pos[t], pos0 = seq_pos0[s], slot = seq_slot[s];
     const int nqk = kv_heads * dim, nv = heads * vdim, channels = 2 * nqk + nv;
@@ -264,8 +258,6 @@ ssd_prep_kernel(const T *__restrict__ proj, int ld, int col0, const float *__res
                 const float *__restrict__ skip_w, float *__restrict__ rec, DecayRow lay, const int *__restrict__ tok_seq,
                 const int *__restrict__ tok_pos, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int heads, int groups,
                 int state, int vdim) {
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ float sh[];  // dt [heads]
     const int t = blockIdx.x, s = tok_seq[t], pos = tok_pos[t], pos0 = seq_pos0[s], slot = seq_slot[s];
     const int inner = heads * vdim, gn = groups * state, channels = inner + 2 * gn;
@@ -300,8 +292,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 linear_prep_kernel(const T *__restrict__ proj, int ld, int col0, const float *__restrict__ head_decay, float *__restrict__ rec, DecayRow lay,
                    int heads, int dim, int vdim) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x, nqk = heads * dim, nv = heads * vdim;
     const T *row = proj + (size_t)t * ld + col0;
     float *out = rec + (size_t)t * lay.ld;
@@ -326,8 +316,6 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 group_output_kernel(const float *__restrict__ o, const float *__restrict__ skip, int skip_ld, const float *__restrict__ w, float eps,
                     const T *__restrict__ gate, int gate_ld, int gate_act, int gate_first, T *__restrict__ out, int out_ld, int cols, int groups) {
-    pdl_launch_dependents();
-    pdl_wait();
     __shared__ float red[33];
     constexpr int N = VEC ? 4 : 1, kKeep = VEC ? 2 : 8;
     const int t = blockIdx.x / groups, g = blockIdx.x - t * groups, per = cols / groups, c0 = g * per;
@@ -405,8 +393,6 @@ template <bool V4>
 __global__ void __launch_bounds__(256)
 delta_finish_kernel(const float *__restrict__ za, const float *__restrict__ zg, const float *__restrict__ decay_bias, const float *__restrict__ a_log,
                     float *__restrict__ rec, DeltaRow lay, int heads, int dim, int vdim) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int N = V4 ? 4 : 1;
     const int t = blockIdx.x, nd = heads * dim, nv = heads * vdim;
     float *out = rec + (size_t)t * lay.ld;
@@ -434,8 +420,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 conv_state_update_kernel(const T *__restrict__ proj, int ld, int col0, float *__restrict__ conv_state, int taps, int channels,
                          const int *__restrict__ seq_start, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int s = blockIdx.y, t0 = seq_start[s], len = seq_start[s + 1] - t0, pos0 = seq_pos0[s], keep = taps - 1;
     if (len <= 0) return;
     float *cst = conv_state + (size_t)seq_slot[s] * keep * channels;
@@ -454,8 +438,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 mlstm_prep_kernel(const T *__restrict__ proj, int ld, int col0, const float *__restrict__ b_in, float cap, float *__restrict__ rec, MlstmRow lay,
                   int heads, int dim, int vdim) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x;
     const T *row = proj + (size_t)t * ld + col0;
     const float *bias = b_in;  // counted from the mixer's own first row
@@ -505,8 +487,6 @@ column_recurrence_kernel(const float *__restrict__ rec, int rec_ld, int q_off, i
                          float *__restrict__ S, float *__restrict__ n_state, float *__restrict__ m_state, float *__restrict__ o,
                          float *__restrict__ nq_out, float *__restrict__ m_out, const int *__restrict__ seq_start,
                          const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int heads, int kv_heads, int dim, int vdim, int max_tokens) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int RPT = DP / LANES, NV = MODE == 0 ? 3 : 2, TS = NV * DP + 4;
     static_assert(RPT >= 4 && RPT % 4 == 0 && RPT * CPT <= 128, "state tile per thread");
     extern __shared__ __align__(16) float stage[];  // [2][kRecTB][TS] | v [2][kRecTB][CB]
@@ -743,8 +723,6 @@ __global__ void __launch_bounds__(256)
 head_output_kernel(const float *__restrict__ o, const float *__restrict__ nq, const float *__restrict__ m_in, const float *__restrict__ w,
                    int w_stride, float eps, const float *__restrict__ gate_f, int gate_f_ld, const T *__restrict__ gate_t, int gate_t_ld,
                    T *__restrict__ out, int out_ld, float out_scale, int tokens, int heads, int vdim, int gate_act, int vec) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (idx >= tokens * heads) return;
     const int t = idx / heads, h = idx - t * heads;
@@ -800,7 +778,7 @@ static int launch_colrec_t(const float *rec, int rec_ld, int q_off, int k_off, i
     const size_t smem = ((size_t)2 * kRecTB * (NV * DP + 4) + (size_t)2 * kRecTB * cb) * sizeof(float);
     auto kern = column_recurrence_kernel<DP, LANES, CPT, MODE>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(kern, dim3((ncols + cb - 1) / cb, heads, n_seqs), dim3(block), smem, st, true, rec, rec_ld, q_off, k_off, v_off, a_off, b_off, S, n_state, m_state, o, nq, m_out,
+    launch_pdl(kern, dim3((ncols + cb - 1) / cb, heads, n_seqs), dim3(block), smem, st, false, rec, rec_ld, q_off, k_off, v_off, a_off, b_off, S, n_state, m_state, o, nq, m_out,
                                                                         seq_start, seq_pos0, seq_slot, heads, kv_heads, dim, vdim, max_tokens);
     return cuda_status("column_recurrence launch");
 }
@@ -862,15 +840,15 @@ int launch_delta_prep(int dtype, const void *proj, int ld, int col0, const float
     const int per = std::max(1, std::min(4, row_tiles * groups / (2 * sm_count())));  // tiles per CTA, two CTAs per SM left
     const dim3 tile_grid((row_tiles + per - 1) / per, groups + 1);
     if (pieces && dtype == B200_BF16)
-        launch_pdl(delta_prep_tile_kernel<__nv_bfloat16>, dim3(tile_grid), dim3(256), 0, st, true, (const __nv_bfloat16 *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__nv_bfloat16 *)lr_a,
+        launch_pdl(delta_prep_tile_kernel<__nv_bfloat16>, dim3(tile_grid), dim3(256), 0, st, false, (const __nv_bfloat16 *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__nv_bfloat16 *)lr_a,
                                                                          (__nv_bfloat16 *)lr_g, rec, lay, tok_seq, tok_pos, seq_pos0, seq_slot, tokens, heads, kv_heads, dim, vdim, per);
     else if (pieces)
-        launch_pdl(delta_prep_tile_kernel<__half>, dim3(tile_grid), dim3(256), 0, st, true, (const __half *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__half *)lr_a, (__half *)lr_g, rec, lay,
+        launch_pdl(delta_prep_tile_kernel<__half>, dim3(tile_grid), dim3(256), 0, st, false, (const __half *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__half *)lr_a, (__half *)lr_g, rec, lay,
                                                                   tok_seq, tok_pos, seq_pos0, seq_slot, tokens, heads, kv_heads, dim, vdim, per);
     else B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         // few tokens: few CTAs, so each gets more threads (a thread's channels are a chain of load latencies)
-        launch_pdl(delta_prep_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), smem, st, true, (const T *)proj, ld, col0, conv_w, taps, conv_state, rank, gate_rank, (T *)lr_a, (T *)lr_g, rec, lay,
+        launch_pdl(delta_prep_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), smem, st, false, (const T *)proj, ld, col0, conv_w, taps, conv_state, rank, gate_rank, (T *)lr_a, (T *)lr_g, rec, lay,
                                                        tok_seq, tok_pos, seq_pos0, seq_slot, heads, kv_heads, dim, vdim);
     });
     int rc = cuda_status("delta_prep launch");
@@ -886,7 +864,7 @@ int launch_delta_prep(int dtype, const void *proj, int ld, int col0, const float
         if (rc != B200_OK) return rc;
     }
     const bool v4 = dim % 4 == 0 && (heads * vdim) % 4 == 0 && all_aligned16({za, zg, decay_bias, rec});
-    launch_pdl((v4 ? delta_finish_kernel<true> : delta_finish_kernel<false>), dim3(tokens), dim3(256), 0, st, true, za, zg, decay_bias, a_log, rec, lay, heads, dim, vdim);
+    launch_pdl((v4 ? delta_finish_kernel<true> : delta_finish_kernel<false>), dim3(tokens), dim3(256), 0, st, false, za, zg, decay_bias, a_log, rec, lay, heads, dim, vdim);
     return cuda_status("delta_finish launch");
 }
 
@@ -894,7 +872,7 @@ int launch_conv_state_update(int dtype, const void *proj, int ld, int col0, floa
                              const int *seq_pos0, const int *seq_slot, int n_seqs, cudaStream_t st) {
     if (n_seqs == 0 || taps <= 1) return B200_OK;
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(conv_state_update_kernel<T>, dim3((channels + 255) / 256, n_seqs), dim3(256), 0, st, true, (const T *)proj, ld, col0, conv_state, taps, channels, seq_start, seq_pos0, seq_slot);
+        launch_pdl(conv_state_update_kernel<T>, dim3((channels + 255) / 256, n_seqs), dim3(256), 0, st, false, (const T *)proj, ld, col0, conv_state, taps, channels, seq_start, seq_pos0, seq_slot);
     });
     return cuda_status("conv_state_update launch");
 }
@@ -910,7 +888,7 @@ int launch_mlstm_prep(int dtype, const void *proj, int ld, int col0, const float
                       int vdim, cudaStream_t st) {
     if (tokens == 0) return B200_OK;
     const MlstmRow lay = mlstm_row(heads, dim, vdim);
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(mlstm_prep_kernel<T>, dim3(tokens), dim3(256), 0, st, true, (const T *)proj, ld, col0, b_in, cap, rec, lay, heads, dim, vdim); });
+    B200_DISPATCH_DTYPE(dtype, { launch_pdl(mlstm_prep_kernel<T>, dim3(tokens), dim3(256), 0, st, false, (const T *)proj, ld, col0, b_in, cap, rec, lay, heads, dim, vdim); });
     return cuda_status("mlstm_prep launch");
 }
 
@@ -928,7 +906,7 @@ int launch_head_output(int dtype, const float *o, const float *nq, const float *
     const int grid = (tokens * heads + 7) / 8;
     const int vec = vdim % 8 == 0 && vdim <= 256 && w_stride % 4 == 0 && gate_f_ld % 4 == 0 && gate_t_ld % 8 == 0 && out_ld % 8 == 0 && all_aligned16({o, w, gate_f, gate_t, out});
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(head_output_kernel<T>, dim3(grid), dim3(256), 0, st, true, o, nq, m_in, w, w_stride, eps, gate_f, gate_f_ld, (const T *)gate_t, gate_t_ld, (T *)out, out_ld,
+        launch_pdl(head_output_kernel<T>, dim3(grid), dim3(256), 0, st, false, o, nq, m_in, w, w_stride, eps, gate_f, gate_f_ld, (const T *)gate_t, gate_t_ld, (T *)out, out_ld,
                                                    out_scale, tokens, heads, vdim, gate_act, vec);
     });
     return cuda_status("head_output launch");
@@ -942,7 +920,7 @@ int launch_delta_prep_direct(int dtype, const void *proj, int ld, int col0, cons
     const size_t smem = ((size_t)2 * kv_heads * dim + heads * vdim) * sizeof(float);
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_direct_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(delta_prep_direct_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), smem, st, true, (const T *)proj, ld, col0, conv_w, taps, conv_state, decay_bias, a_log, rec,
+        launch_pdl(delta_prep_direct_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), smem, st, false, (const T *)proj, ld, col0, conv_w, taps, conv_state, decay_bias, a_log, rec,
                                                                                    lay, tok_seq, tok_pos, seq_pos0, seq_slot, heads, kv_heads, dim, vdim);
     });
     return cuda_status("delta_prep_direct launch");
@@ -954,7 +932,7 @@ int launch_ssd_prep(int dtype, const void *proj, int ld, int col0, const float *
     if (tokens == 0) return B200_OK;
     const DecayRow lay = decay_row(heads, groups, state, vdim);
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(ssd_prep_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), (size_t)heads * sizeof(float), st, true, (const T *)proj, ld, col0, conv_w, conv_b, taps, conv_state, dt_bias,
+        launch_pdl(ssd_prep_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), (size_t)heads * sizeof(float), st, false, (const T *)proj, ld, col0, conv_w, conv_b, taps, conv_state, dt_bias,
                                                                                                    a_log, skip_w, rec, lay, tok_seq, tok_pos, seq_pos0, seq_slot,
                                                                                                    heads, groups, state, vdim);
     });
@@ -965,7 +943,7 @@ int launch_linear_prep(int dtype, const void *proj, int ld, int col0, const floa
                        cudaStream_t st) {
     if (tokens == 0) return B200_OK;
     const DecayRow lay = decay_row(heads, heads, dim, vdim);
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(linear_prep_kernel<T>, dim3(tokens), dim3(256), 0, st, true, (const T *)proj, ld, col0, head_decay, rec, lay, heads, dim, vdim); });
+    B200_DISPATCH_DTYPE(dtype, { launch_pdl(linear_prep_kernel<T>, dim3(tokens), dim3(256), 0, st, false, (const T *)proj, ld, col0, head_decay, rec, lay, heads, dim, vdim); });
     return cuda_status("linear_prep launch");
 }
 
@@ -986,7 +964,7 @@ int launch_group_output(int dtype, const float *o, const float *skip, int skip_l
     const int pieces = vec ? per / 4 : per, threads = pieces <= 64 ? 32 : (pieces <= 128 ? 64 : (pieces <= 256 ? 128 : 256));
     B200_DISPATCH_DTYPE(dtype, {
         auto kern = vec ? group_output_kernel<T, true> : group_output_kernel<T, false>;
-        launch_pdl(kern, dim3(tokens * groups), dim3(threads), 0, st, true, o, skip, skip_ld, w, eps, (const T *)gate, gate_ld, gate_act, gate_first, (T *)out, out_ld, cols, groups);
+        launch_pdl(kern, dim3(tokens * groups), dim3(threads), 0, st, false, o, skip, skip_ld, w, eps, (const T *)gate, gate_ld, gate_act, gate_first, (T *)out, out_ld, cols, groups);
     });
     return cuda_status("group_output launch");
 }

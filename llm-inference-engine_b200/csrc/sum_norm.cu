@@ -76,8 +76,6 @@ __global__ void __launch_bounds__(512)
 sum_norm_kernel(float *x, const T *__restrict__ y_dense, const T *__restrict__ y_rows, const int *__restrict__ pair_row, int top,
                 const T *__restrict__ y_shared, const float *__restrict__ shared_gate, float alpha, const float *__restrict__ g, float eps, int width,
                 float *__restrict__ trace, T *__restrict__ h_out, RingConv own, RingConv next, int one_token, PortionMap pm) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int N = VEC ? Elem<T>::kVec : 1, KP = VEC ? 2 : 8;
     __shared__ float red[33];
     const int t = blockIdx.x, s = pm.tok_seq[t], pos = pm.tok_pos[t];
@@ -163,8 +161,6 @@ sum_norm_kernel(float *x, const T *__restrict__ y_dense, const T *__restrict__ y
 
 // turns[i] = base^(-2i / width) / (2 pi): turns per position of channels 2i and 2i + 1
 __global__ void pos_turns_kernel(double *__restrict__ turns, int width, float base) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (2 * i < width) turns[i] = exp2(-2.0 * (double)i / (double)width * log2((double)base)) * 0.15915494309189533577;
 }
@@ -176,8 +172,6 @@ template <typename T, int N>
 __global__ void __launch_bounds__(256)
 embed_pos_kernel(const int *__restrict__ ids, const T *__restrict__ table, float *__restrict__ x, T *__restrict__ h_out, int width, int vocab,
                  float scale, const double *__restrict__ turns, RingConv next, int one_token, PortionMap pm) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * N;
     if (c >= width) return;
     int id = ids[t];
@@ -215,8 +209,6 @@ constexpr int kConvRun = 8;
 template <typename T, int TAPS, int N>
 __global__ void __launch_bounds__(256)
 conv_input_kernel(const float *__restrict__ x, T *__restrict__ h, int width, int tokens, RingConv cv, PortionMap pm) {
-    pdl_launch_dependents();
-    pdl_wait();
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * N;
     if (c >= width) return;
     const int taps = TAPS > 0 ? TAPS : cv.taps, keep = taps - 1;
@@ -287,14 +279,14 @@ int launch_sum_norm(int dtype, float *x, const void *y_dense, const void *y_rows
         const int per = vec ? Elem<T>::kVec : 1;
         const int threads = std::min(512, std::max(32, ((width + per - 1) / per + 31) / 32 * 32));
         auto kern = vec ? sum_norm_kernel<T, true> : sum_norm_kernel<T, false>;
-        launch_pdl(kern, dim3(tokens), dim3(threads), 0, st, true, x, (const T *)y_dense, (const T *)y_rows, pair_row, top, (const T *)y_shared, shared_gate, alpha, g, eps, width,
+        launch_pdl(kern, dim3(tokens), dim3(threads), 0, st, false, x, (const T *)y_dense, (const T *)y_rows, pair_row, top, (const T *)y_shared, shared_gate, alpha, g, eps, width,
                                          trace, (T *)h_out, own, next, one_token, pm);
     });
     return cuda_status("sum_norm launch");
 }
 
 int launch_pos_turns(double *turns, int width, float base, cudaStream_t st) {
-    launch_pdl(pos_turns_kernel, dim3((width + 511) / 512), dim3(256), 0, st, true, turns, width, base);
+    launch_pdl(pos_turns_kernel, dim3((width + 511) / 512), dim3(256), 0, st, false, turns, width, base);
     return cuda_status("pos_turns launch");
 }
 
@@ -306,7 +298,7 @@ int launch_embed_pos(int dtype, const int *ids, const void *table, float *x, voi
         const int cols = vec ? width / 4 : width;
         const int threads = std::min(256, (cols + 31) / 32 * 32);
         auto kern = vec ? embed_pos_kernel<T, 4> : embed_pos_kernel<T, 1>;
-        launch_pdl(kern, dim3(tokens, (cols + threads - 1) / threads), dim3(threads), 0, st, true, ids, (const T *)table, x, (T *)h_out, width, vocab, scale, turns, next,
+        launch_pdl(kern, dim3(tokens, (cols + threads - 1) / threads), dim3(threads), 0, st, false, ids, (const T *)table, x, (T *)h_out, width, vocab, scale, turns, next,
                                                                                one_token, pm);
     });
     return cuda_status("embed_pos launch");
@@ -319,7 +311,7 @@ static void launch_conv_taps(const float *x, void *h, int width, RingConv cv, Po
     const int threads = std::min(256, (cols + 31) / 32 * 32);
     const dim3 grid((tokens + kConvRun - 1) / kConvRun, (cols + threads - 1) / threads);
     auto kern = vec ? conv_input_kernel<T, TAPS, 4> : conv_input_kernel<T, TAPS, 1>;
-    launch_pdl(kern, dim3(grid), dim3(threads), 0, st, true, x, (T *)h, width, tokens, cv, pm);
+    launch_pdl(kern, dim3(grid), dim3(threads), 0, st, false, x, (T *)h, width, tokens, cv, pm);
 }
 
 int launch_conv_input(int dtype, const float *x, void *h, int width, RingConv cv, PortionMap pm, int tokens, cudaStream_t st) {

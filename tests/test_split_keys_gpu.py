@@ -1,5 +1,5 @@
-"""Decoded tokens whose keys are shared out over a cluster of CTAs (csrc/attention_chunked.cu, csrc/attention_scored.cu): contexts shorter than the
-cluster, uneven shares, blocks and windows that end inside a share; against the float64 restatements of the designs, pools poisoned with NaN."""
+"""Decoded tokens of the per-token attention kernels (csrc/attention_chunked.cu, csrc/attention_scored.cu): contexts of a few keys and of several
+rounds of the block, blocks and windows that end inside a page; against the float64 restatements of the designs, pools poisoned with NaN."""
 import importlib
 
 import numpy as np
