@@ -13,8 +13,8 @@
 //   * WARPS softmax warps: WARPS / 4 threads share a row; lazy rescale: O is scaled only when the running maximum grows by more than 2^8 (see
 //     context_attn_tc.cu, whose loop this follows); the sink is the initial maximum and sum; value rows past the tile's last query are zeroed, since a page's
 //     unwritten rows may hold anything and 0 * NaN would reach the accumulator.
-// A step is a chain (scores, TMEM read, row maximum, exponentials, P, product): two CTAs per SM, where shared memory holds them (not the latent rows),
-// fill each other's waits.
+// A step is a chain (scores, TMEM read, row maximum, exponentials, P, product): two CTAs per SM fill each other's waits (not for latent rows, which are too
+// large, nor for logits with a penalty).
 // Measured against the mma.sync kernels, us per layer: chunked 175 -> 81 (4096 tokens, 16 heads of 128), latent 244 -> 72 (3085 tokens in two prompts, 16
 // heads, rank 192 + 64), scored with a distance penalty and a window of 1024 116 -> 75 (2911 tokens in three prompts, 16 heads of 128).
 #include "hybrid_ops.cuh"
