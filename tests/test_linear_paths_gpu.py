@@ -64,8 +64,8 @@ def test_linear_of_few_tokens_and_odd_rows(n):
 
 @pytest.mark.parametrize("fmt", ["dense", "fp8", "int4"])
 @pytest.mark.parametrize("batch", [1, 2, 5, 8, 9, 16])
-def test_norm_on_the_fragments_matches_the_norm_kernel(fmt, batch):
-    """A layer whose norms run inside the linears (up to 16 tokens) against the same rows in a batch of 17 (norm kernel in front): rows agree to the
+def test_few_tokens_match_the_same_rows_in_a_larger_batch(fmt, batch):
+    """Layers of up to 16 tokens (streamed weights; one dense token: norms inside the linears) against the same rows in a batch of 17: rows agree to the
     roundings of the layer's 16-bit intermediates."""
     gen = torch.Generator(device=DEV).manual_seed(3)
     h, heads, kv, d, inter, rows = 1024, 8, 2, 128, 1408, 17
