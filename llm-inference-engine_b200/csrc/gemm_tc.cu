@@ -570,6 +570,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     tma_load_2d_pair(sa + kATileBytes, mb, kb * kBK, brow, bar);
                 }
             }
+            // The leader's last commits arrive at `empty` of both CTAs and nobody refills those stages: each CTA waits for its own here, since the
+            // closing cluster barrier does not order them and a late one would land in the shared memory of whatever runs on this SM next
+            for (int i = max(0, it - p.stages); live && i < it; ++i) live = bar_wait_limited(empty0 + 8 * (i % p.stages), (i / p.stages) & 1);
         }
     } else if (warp == 1) {
         // ================================================= MMA issuer: the leader, for both

@@ -113,6 +113,23 @@ def test_linear_of_prompts(dtype, m, k, n):
     assert bool((out[m * n:] == 7.0).all())
 
 
+@pytest.mark.parametrize("k", [64, 384, 448, 1024])
+def test_pairs_leave_nothing_under_way(k):
+    """Launches of CTA pairs whose k blocks are fewer than, as many as and more than the ring's stages, each with kernels behind it that hold barriers in the
+    same shared memory: an arrival that outlived its CTA would complete a phase of theirs too early.  Every launch gives the first one's bits."""
+    gen = torch.Generator(device=DEV).manual_seed(k)
+    rand = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()  # noqa: E731
+    x, w, few, odd = rand(512, k), rand(9728, k), rand(6, 2048), rand(200, 2048)
+    w2 = rand(1024, 2048)
+    first = None
+    for _ in range(200):
+        got = (b200.linear(x, w), b200.linear(few, w2), b200.linear(odd, w2))
+        first = first or got
+        assert all(torch.equal(a, b) for a, b in zip(got, first))
+    for (a, b), got in zip(((x, w), (few, w2), (odd, w2)), first):
+        close(got, a.double() @ b.double().T, torch.bfloat16, k)
+
+
 @pytest.mark.parametrize("m,k,inter", [(256, 64, 4864), (1000, 200, 2752), (2048, 128, 2688), (1084, 72, 5000), (300, 512, 1408)])
 def test_swiglu_of_prompts_is_the_two_launchers(m, k, inter):
     """Gate and up halves of a tile come from the two CTAs of a pair: bit-identical to the linear followed by silu-and-mul."""
