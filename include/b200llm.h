@@ -67,6 +67,18 @@ int b200_abi_version(void);
 /* Number of SMs of the current device (grid sizing is a multiple of this). */
 int b200_sm_count(void);
 
+/* ---- waits inside kernels --------------------------------------------------------------------------
+ * The kernels that hand tiles from one part of a CTA to another wait on barriers, and a wait lasts about a second at most.  One that runs
+ * out means a fault elsewhere: the kernel stores NaN for what it could not form, returns, and leaves its code in a word that every later
+ * call reports as B200_ERR_CUDA.  Kernels replayed from a graph make no calls: read b200_wait_error() where the program synchronises.
+ *   b200_wait_error(clear): the code (0: none); clear != 0 takes it back.
+ *   b200_wait_limit(clocks): limit for launches of the calling thread, in SM clocks; 0: every wait runs out at once; anything above the
+ *     default of 2^31 - 1 is the default.  For tests of a program's own error handling.
+ *   b200_wait_probe(stream): launches a kernel whose wait can only run out. */
+int b200_wait_error(int clear);
+void b200_wait_limit(unsigned int clocks);
+int b200_wait_probe(b200_stream_t stream);
+
 /* ---- library workspace (split-K partials, split-KV partials, tickets) -------------------------------
  * Launchers never allocate.  The workspace is either handed over by the caller or allocated once by
  * b200_workspace_ensure() (cudaMalloc; call it outside stream capture). */

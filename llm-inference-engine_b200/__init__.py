@@ -120,6 +120,9 @@ SIGNATURES = {
     "b200_last_error_string": [],
     "b200_abi_version": [],
     "b200_sm_count": [],
+    "b200_wait_error": [_I],
+    "b200_wait_limit": [C.c_uint],
+    "b200_wait_probe": [_P],
     "b200_workspace_default_bytes": [],
     "b200_workspace_set": [_P, _SZ],
     "b200_workspace_ensure": [_SZ],
@@ -233,7 +236,7 @@ SIGNATURES = {
     "b200_batcher_hybrid_workspace_bytes": [_P, _I, _I],
     "b200_batcher_step_hybrid": [_P, _P, _I, _I, _I, _P, _SZ, C.POINTER(C.c_int), _P],
 }
-_RESTYPES = {"b200_last_error_string": C.c_char_p, "b200_workspace_default_bytes": _SZ, "b200_decoder_create": _P,
+_RESTYPES = {"b200_last_error_string": C.c_char_p, "b200_wait_limit": None, "b200_workspace_default_bytes": _SZ, "b200_decoder_create": _P,
              "b200_decoder_destroy": None, "b200_decoder_scratch_bytes": _SZ, "b200_decoder_prefill_scratch_bytes": _SZ,
              "b200_decoder_tp_buffer_bytes": _SZ, "b200_generate_workspace_bytes": _SZ, "b200_batcher_create": _P,
              "b200_batcher_destroy": None, "b200_batcher_plan_array": C.POINTER(C.c_int), "b200_batcher_workspace_bytes": _SZ,
@@ -266,6 +269,12 @@ def check(rc):
 # ------------------------------------------------------------------ torch plumbing (device memory + streams only)
 def _torch():
     import torch
+def wait_error(clear=False):
+    """The code of a wait inside a kernel that ran out since the last clear (0: none): results since then are not valid, and every call raises until it
+    is cleared.  Replayed graphs make no calls, so a program that replays them reads this where it synchronises."""
+    return lib().b200_wait_error(int(clear))
+
+
 
     return torch
 

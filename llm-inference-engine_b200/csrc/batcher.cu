@@ -632,6 +632,7 @@ int b200_batcher_step(b200_batcher_t *b, b200_decoder_t *dec, const b200_generat
         if (cudaMemcpyAsync(sampled_p.data(), output_id, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return fail(cuda_status("batcher_step D2H (prefill)"));
+        if ((rc = wait_status("batcher_step (prefill)")) != B200_OK) return fail(rc);
     }
     // ---- running sequences: one decode step, every row at its own position, through the block table
     if (plan.n_decode > 0) {
@@ -650,6 +651,7 @@ int b200_batcher_step(b200_batcher_t *b, b200_decoder_t *dec, const b200_generat
         if (cudaMemcpyAsync(sampled_d.data(), output_id, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return fail(cuda_status("batcher_step D2H (decode)"));
+        if ((rc = wait_status("batcher_step (decode)")) != B200_OK) return fail(rc);
     }
     const int fin = b200_batcher_commit(b, sampled_p.data(), sampled_d.data(), p->end_id);
     if (fin < 0) return fin;
@@ -755,6 +757,7 @@ int b200_batcher_step_hybrid(b200_batcher_t *b, b200_hybrid_t *model, int vocab,
     } else if (cudaStreamSynchronize(as_stream(stream)) != cudaSuccess) {
         return fail(cuda_status("batcher_step_hybrid sync"));
     }
+    if ((rc = wait_status("batcher_step_hybrid")) != B200_OK) return fail(rc);
     const int fin = b200_batcher_commit_mixed(b, sampled.data(), end_id);
     if (fin < 0) return fin;
     if (n_finished) *n_finished = fin;

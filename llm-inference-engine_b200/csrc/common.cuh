@@ -17,8 +17,19 @@ namespace b200 {
 
 // ------------------------------------------------------------------ error plumbing (host)
 void set_error(const char *fmt, ...);
-int cuda_status(const char *what);  // cudaGetLastError() -> B200_OK / B200_ERR_CUDA (+ message)
+int cuda_status(const char *what);  // cudaGetLastError(), then wait_status() -> B200_OK / B200_ERR_CUDA (+ message)
 int sm_count();
+
+// Waits inside kernels have a limit: a fault elsewhere must not hang the device.  A kernel whose wait runs out stores NaN in place of what it could not
+// form, waits for its own copies, leaves its code in the process's wait word (mapped host memory) and returns; every later call of the library on the host
+// reports the word until b200_wait_error(1) clears it.  (Replayed graphs make no calls: their owner reads b200_wait_error().)
+enum WaitCode : unsigned int { kWaitGemvRs = 1, kWaitGemmPair = 2, kWaitPromptAttn = 3, kWaitProbe = 4 };
+struct WaitGuard {          // kernel argument
+    unsigned int *word;     // the wait word as the device sees it, or NULL
+    unsigned int clocks;    // limit of one wait; 0: every wait runs out at once
+};
+WaitGuard wait_guard();             // for launches made by the calling thread
+int wait_status(const char *what);  // the wait word -> B200_OK / B200_ERR_CUDA (+ message)
 
 #define B200_REQUIRE(cond, ...)                 \
     do {                                        \
@@ -138,6 +149,54 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// ------------------------------------------------------------------ waits that end (see WaitGuard)
+constexpr unsigned int kWaitClocks = 0x7fffffffu;  // about a second
+// what one try counts at most: a try may sleep, so tries are no measure of time -- nor are clocks while the context is off the device
+constexpr unsigned int kWaitStep = 1u << 24;
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// one flag per CTA, cleared by the thread that initialises its barriers: a wait that has run out ends every later one of the CTA
+__device__ __forceinline__ volatile int &cta_gave_up() {
+    __shared__ volatile int v;
+    return v;
+}
+// what a wait does when its first try fails, out of line: the waits stand in loops whose code should stay small (inline in the GEMV: 1 to 3 % of a decode step)
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, unsigned int *word, unsigned int clocks, unsigned int code) {
+    for (uint32_t spent = 0, last = (uint32_t)clock(); spent < clocks && !cta_gave_up();) {
+        if (mbar_try(bar, parity)) return true;
+        const uint32_t now = (uint32_t)clock();
+        spent += min(now - last, kWaitStep), last = now;
+    }
+    cta_gave_up() = 1;
+    if (word) {
+        *reinterpret_cast<volatile unsigned int *>(word) = code;
+        __threadfence_system();
+    }
+    return false;
+}
+__device__ __forceinline__ bool mbar_wait_guarded(uint32_t bar, uint32_t parity, const WaitGuard &wg, unsigned int code) {
+    if (wg.clocks != 0 && mbar_try(bar, parity)) return true;
+    return mbar_wait_slow(bar, parity, wg.word, wg.clocks, code);
+}
+// for what the CTA has under way itself when it leaves (copies into its shared memory, products that read it): whatever has run out before
+static __device__ __noinline__ bool mbar_drain(uint32_t bar, uint32_t parity) {
+    for (uint32_t spent = 0, last = (uint32_t)clock(); spent < kWaitClocks;) {
+        if (mbar_try(bar, parity)) return true;
+        const uint32_t now = (uint32_t)clock();
+        spent += min(now - last, kWaitStep), last = now;
+    }
+    return false;
 }
 
 // ------------------------------------------------------------------ element traits

@@ -452,34 +452,11 @@ struct GemmPairParams {
     int bn, bn2, n_wide;
     int stages, is_bf16;
     int swiglu_inter;  // as above: gate rows come from the leader's half of B, up rows from its peer's; tile widths count both
+    WaitGuard wait;
 };
 constexpr int kPairThreads = 320;
 constexpr int kPairStageBytes = 2 * kATileBytes;  // 128 rows of A, up to 128 rows of B
 
-__device__ unsigned int g_pair_wait_failed;  // a wait that gave up (seconds): the launch's results are not valid
-
-// false after 2^31 clocks (about a second; a try may sleep, so tries are no measure); the caller leaves its role loop
-__device__ __forceinline__ bool bar_wait_limited(uint32_t bar, uint32_t parity) {
-    auto ready = [&]() -> bool {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        return ok != 0;
-    };
-    if (ready()) return true;
-    const uint32_t t0 = (uint32_t)clock();
-    while (!ready()) {
-        if ((uint32_t)clock() - t0 < 0x7fffffffu) continue;
-        atomicExch(&g_pair_wait_failed, 1u);
-        return false;
-    }
-    return true;
-}
 __device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {  // the same shared-memory offset in CTA `rank` of the cluster
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
@@ -492,6 +469,9 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
 }
 __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void tc_commit_leader(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -513,6 +493,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (size_t)p.stages * kPairStageBytes);
     const uint32_t full0 = s_u32(bars), empty0 = full0 + 8 * kMaxStages, tfull0 = empty0 + 8 * kMaxStages, tempty0 = tfull0 + 16;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kMaxStages + 4);
+    const uint32_t drain = tempty0 + 24;  // (behind the TMEM slot)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -529,6 +510,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             bar_init(tfull0 + 8 * a, 1);
             bar_init(tempty0 + 8 * a, 16);  // eight epilogue warps of either CTA
         }
+        bar_init(drain, 1);
+        cta_gave_up() = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -544,6 +527,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     pdl_wait();
     pdl_launch_dependents();
 
+    // a wait that runs out: no more copies, no more products, NaN for the tiles that are left, and the other CTA's waits on them run out in turn
+    auto wait = [&](uint32_t bar, uint32_t parity) { return mbar_wait_guarded(bar, parity, p.wait, kWaitGemmPair); };
     auto width_of = [&](int tb) { return tb < p.n_wide ? p.bn : p.bn2; };
     auto col_of = [&](int tb) {  // first output column (SwiGLU: half of a tile's width are output columns)
         const int c = tb < p.n_wide ? tb * p.bn : p.n_wide * p.bn + (tb - p.n_wide) * p.bn2;
@@ -562,7 +547,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 const CUtensorMap *mb = tb < p.n_wide ? &tmB : &tmB2;
                 for (int kb = 0; kb < p.kb_total; ++kb, ++it) {
                     const int s = it % p.stages;
-                    live = bar_wait_limited(empty0 + 8 * s, ((it / p.stages) & 1) ^ 1);
+                    live = wait(empty0 + 8 * s, ((it / p.stages) & 1) ^ 1);
                     if (!live) break;
                     const uint32_t sa = s_u32(smem + (size_t)s * kPairStageBytes), bar = in_cta(full0 + 8 * s, 0);
                     if (rank == 0) bar_expect_tx(full0 + 8 * s, (uint32_t)(2 * (kATileBytes + (w >> 1) * kBK * 2)));
@@ -572,45 +557,48 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
             // The leader's last commits arrive at `empty` of both CTAs and nobody refills those stages: each CTA waits for its own here, since the
             // closing cluster barrier does not order them and a late one would land in the shared memory of whatever runs on this SM next
-            for (int i = max(0, it - p.stages); live && i < it; ++i) live = bar_wait_limited(empty0 + 8 * (i % p.stages), (i / p.stages) & 1);
+            for (int i = max(0, it - p.stages); live && i < it; ++i) live = wait(empty0 + 8 * (i % p.stages), (i / p.stages) & 1);
+            // (given up: both CTAs' copies are counted here, and the peer stays until the leader has seen them land)
+            for (int i = max(0, it - p.stages); !live && rank == 0 && i < it; ++i)
+                if (!mbar_drain(full0 + 8 * (i % p.stages), (i / p.stages) & 1)) break;
         }
     } else if (warp == 1) {
         // ================================================= MMA issuer: the leader, for both
-        if (rank == 0) {
+        if (rank == 0 && elect_one()) {
             int it = 0, t = 0;
             bool live = true;
             for (int item = pair; live && item < p.tiles; item += pairs, ++t) {
                 const uint32_t idesc = instr_desc_f16(p.is_bf16 != 0, 2 * kBM, width_of(item / p.tilesA));
                 const int acc = t & 1;
-                live = bar_wait_limited(tempty0 + 8 * acc, ((t >> 1) & 1) ^ 1);
+                live = wait(tempty0 + 8 * acc, ((t >> 1) & 1) ^ 1);
                 if (!live) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
                 for (int kb = 0; kb < p.kb_total; ++kb, ++it) {
                     const int s = it % p.stages;
-                    live = bar_wait_limited(full0 + 8 * s, (it / p.stages) & 1);
+                    live = wait(full0 + 8 * s, (it / p.stages) & 1);
                     if (!live) break;
                     tc_fence_after();
-                    if (elect_one()) {
-                        const uint32_t sa = s_u32(smem + (size_t)s * kPairStageBytes);
-                        const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + kATileBytes);
+                    const uint32_t sa = s_u32(smem + (size_t)s * kPairStageBytes);
+                    const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + kATileBytes);
 #pragma unroll
-                        for (int k = 0; k < kBK / kUmmaK; ++k) tc_mma_f16_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                        tc_commit_pair(empty0 + 8 * s);
-                        if (kb == p.kb_total - 1) tc_commit_pair(tfull0 + 8 * acc);
-                    }
-                    __syncwarp();
+                    for (int k = 0; k < kBK / kUmmaK; ++k) tc_mma_f16_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    tc_commit_pair(empty0 + 8 * s);
+                    if (kb == p.kb_total - 1) tc_commit_pair(tfull0 + 8 * acc);
                 }
             }
+            tc_commit_leader(drain);  // no product reads either CTA's shared memory when the pair leaves
+            mbar_drain(drain, 0);
         }
     } else {
         // ================================================= epilogue: TMEM lane quarter q, one half of the columns
         const int q = warp & 3, half = (warp - 2) >> 2;
         T *C = reinterpret_cast<T *>(p.C);
         int t = 0;
+        bool live = true;
         for (int item = pair; item < p.tiles; item += pairs, ++t) {
             const int ta = item % p.tilesA, tb = item / p.tilesA, w = width_of(tb), acc = t & 1, col0 = col_of(tb);
-            if (!bar_wait_limited(tfull0 + 8 * acc, (t >> 1) & 1)) break;
+            live = live && __all_sync(0xffffffffu, wait(tfull0 + 8 * acc, (t >> 1) & 1));
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 256);
             const int i = ta * 2 * kBM + (int)rank * kBM + q * 32 + lane;
@@ -631,6 +619,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     }
                 } else {
                     tc_wait_ld();
+                }
+                if (!live) {
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) g[e] = 0x7fc00000u;
                 }
                 if (i < p.rowsA && valid > 0) store_row16<T>(C + (size_t)i * p.ldc + col0 + c, g, valid);
             }
@@ -729,7 +721,7 @@ static int launch_gemm_pair(const void *x, const void *w, void *y, int M, int N,
     p.tilesA = (M + 2 * kBM - 1) / (2 * kBM);
     const PairWidths pw = choose_widths(p.tilesA, cols, pairs);
     p.bn = pw.bn, p.bn2 = pw.bn2, p.n_wide = pw.n_wide, p.tiles = p.tilesA * pw.n_tiles;
-    p.stages = 6;
+    p.stages = 6, p.wait = wait_guard();
     const size_t smem = (size_t)p.stages * kPairStageBytes + 1024 + (2 * kMaxStages + 4) * 8 + 16;
     CUtensorMap tmA, tmB, tmB2;
     if (!make_map(&tmA, x, M, K, kBM, bf16) || !make_map(&tmB, w, cols, K, p.bn / 2, bf16) || !make_map(&tmB2, w, cols, K, p.bn2 / 2, bf16)) {

@@ -36,34 +36,8 @@ struct RsGeom {
     int row_stride;     // bytes between the rows of a stage
     int stage_bytes, stages;
     int max_units;      // units of the busiest CTA
+    WaitGuard wait;
 };
-
-// a wait that gives up after 2^31 clocks (about a second; a try may sleep, so tries are no measure), and with it every later wait of the CTA: a fault
-// elsewhere must not hang the device
-__device__ __forceinline__ volatile int &rs_gave_up() {
-    __shared__ volatile int v;
-    return v;
-}
-__device__ __forceinline__ void mbar_wait_limited(uint32_t bar, uint32_t parity) {
-    auto ready = [&]() -> bool {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        return ok != 0;
-    };
-    if (ready()) return;
-    const uint32_t t0 = (uint32_t)clock();
-    while (!ready()) {
-        if ((uint32_t)clock() - t0 < 0x7fffffffu && !rs_gave_up()) continue;
-        rs_gave_up() = 1;
-        return;
-    }
-}
 
 // 8 activations of T in k order -> the A fragments' halves: dense as they are; quantised formats in f16, INT4 with the pairs its dequantisation makes
 template <typename T, int FMT> __device__ __forceinline__ uint4 rs_fragment(const uint4 raw) {
@@ -108,6 +82,14 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
     float *outacc = reinterpret_cast<float *>(smem + off);  // [unit][VALS], parts > 1 only
     const uint32_t ring_u32 = smem_u32(ring);
 
+    // Whatever stops in the CTA, the reducer's wait for the next tile runs out, and that ends all other waits: the compute warps run through what they have
+    // (their barriers count on it), the producer stops, and what the reducer stores from then on is NaN.  Only the reducer keeps the time: the limit inside
+    // every wait made the loops' code larger and a decode step 1 to 3 % slower.
+    auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
+        while (!mbar_try(bar, parity))
+            if (cta_gave_up()) return false;
+        return true;
+    };
     auto unit_row = [&](int u, int r) -> int { return kSwiGLU ? ((r & 1) ? a.inter : 0) + (R / 2) * u + (r >> 1) : R * u + r; };
     auto row_ok = [&](int u, int r) -> bool { return kSwiGLU ? ((R / 2) * u + (r >> 1) < a.inter) : (R * u + r < N); };
 
@@ -129,7 +111,7 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
             if (++s == stages) s = 0;
         };
         if (lane == 0) {
-            rs_gave_up() = 0;
+            cta_gave_up() = 0;
             for (int i = 0; i < stages; ++i) {
                 mbar_init(full0 + i * 8, 1);
                 mbar_init(empty0 + i * 8, kMmaWarps);
@@ -143,13 +125,17 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
         __syncwarp();
         while (item < stages && item < my_items) issue_next();  // the weights do not depend on the previous kernel
         __syncthreads();                                         // publishes the barriers
+        pdl_wait();  // (nothing here reads what the kernel in front writes: the limit of the waits below starts when it is done)
         int e_s = 0, e_ph = 0;
         while (item < my_items) {
-            mbar_wait_limited(empty0 + e_s * 8, e_ph);
+            if (!__all_sync(0xffffffffu, wait(empty0 + e_s * 8, e_ph))) break;
             if (++e_s == stages) e_s = 0, e_ph ^= 1;
             fence_proxy_async();
             issue_next();
         }
+        // the CTA stays until its last copies have landed, whether or not somebody still waits for them
+        for (int i = max(0, item - stages); i < item; ++i)
+            if (!mbar_drain(full0 + i % stages * 8, (i / stages) & 1)) break;
         return;
     }
     if (warp > kMmaWarps) {
@@ -167,7 +153,7 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) s8[i] = (p + 1 == parts && row_ok(u, r0 + i)) ? __ldg(reinterpret_cast<const float *>(a.scales) + unit_row(u, r0 + i)) : 1.0f;
                 }
-                mbar_wait_limited(ready0 + b * 8, (h >> 1) & 1);
+                const bool lost = !mbar_wait_guarded(ready0 + b * 8, (h >> 1) & 1, geo.wait, kWaitGemvRs) || cta_gave_up();  // (set before whatever the warps hand over without having waited)
                 constexpr int PASSES = VALS / 128;
                 float4 sums[PASSES];
 #pragma unroll
@@ -199,6 +185,7 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
                         }
                     }
                     if (m >= a.M) continue;
+                    if (lost) v.x = v.y = v.z = v.w = __int_as_float(0x7fc00000);
                     float o[4] = {v.x, v.y, v.z, v.w};
                     if constexpr (FMT == WF_FP8) {
 #pragma unroll
@@ -310,7 +297,7 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
         for (int un = 0; un < my_units; ++un, ++h) {
             // dense: [token g (+8)][row 2t (+1)], two chains; quantised: [row g (+8)][token 2t (+1)], acc2: tokens 8 .. 15
             float acc[4] = {}, acc2[4] = {};
-            mbar_wait_limited(full0 + s * 8, ph);
+            (void)wait(full0 + s * 8, ph);
             uint32_t za = 0, zb = 0;
             const int src = (un & 1) * 16 + g;  // the lane that fetched row g of this unit
             if constexpr (FMT == WF_INT4) {
@@ -399,7 +386,7 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
             if (++s == stages) s = 0, ph ^= 1;
             // ---- hand this warp's tile of the (part, unit) to the reducer (double-buffered slot)
             const int b = h & 1;
-            if (h >= 2) mbar_wait_limited(free0 + b * 8, ((h >> 1) - 1) & 1);
+            if (h >= 2) (void)wait(free0 + b * 8, ((h >> 1) - 1) & 1);
             float *slot = tiles + ((size_t)b * kMmaWarps + warp) * TILE;
             if constexpr (kDense) {
                 *reinterpret_cast<float2 *>(slot + g * R + 2 * t) = make_float2(acc[0] + acc2[0], acc[1] + acc2[1]);
@@ -438,6 +425,7 @@ inline bool gemv_rs_geometry(int M, int K, int max_units, int fmt, RsGeom *out) 
     g.stage_bytes = rs_rows(fmt == WF_DENSE) * g.row_stride;
     const size_t budget = 226 * 1024, fixed = gemv_rs_fixed_smem(g, fmt == WF_DENSE, M > 8 ? 2 : 1);
     if (fixed + (size_t)2 * g.stage_bytes > budget) return false;
+    g.wait = wait_guard();
     g.stages = (int)((budget - fixed) / g.stage_bytes);
     if (g.stages > kRsMaxStages) g.stages = kRsMaxStages;
     *out = g;

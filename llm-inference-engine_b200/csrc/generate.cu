@@ -166,6 +166,7 @@ int b200_generate_ragged(b200_decoder_t *dec, const b200_generate_params_t *p, c
             if (cudaMemcpyAsync(poll.data(), out_dev, poll.size() * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
                 cudaStreamSynchronize(st) != cudaSuccess)
                 return cuda_status("generate poll");
+            if ((rc = wait_status("generate")) != B200_OK) return rc;
             bool all = true;
             for (int b = 0; b < batch && all; ++b) {
                 bool hit = false;
@@ -191,6 +192,7 @@ int b200_generate_ragged(b200_decoder_t *dec, const b200_generate_params_t *p, c
     if (cudaMemcpyAsync(host.data(), out_dev, host.size() * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         return cuda_status("generate D2H");
+    if ((rc = wait_status("generate")) != B200_OK) return rc;
     for (int b = 0; b < batch; ++b) {
         int n = 0;
         while (n < produced && host[(size_t)b * N + n] != p->end_id) ++n;

@@ -46,40 +46,13 @@ struct PromptAttn {
     int out_ld, pen_len;
     float out_scale;
     const float *dist_r1, *dist_r2, *slope;
+    WaitGuard wait;
 };
 
 __device__ __forceinline__ uint32_t pa_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void pa_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
 __device__ __forceinline__ void pa_expect(uint32_t bar, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory"); }
 __device__ __forceinline__ void pa_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ uint32_t pa_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok;
-}
-__device__ unsigned int g_pa_wait_failed;  // a wait that gave up: the launch's results are not valid
-// gives up after 2^31 clocks (about a second; a try may sleep, so tries are no measure), and with it every later wait of the CTA: a fault elsewhere must
-// not hang the device
-__device__ __forceinline__ volatile int &pa_gave_up() {
-    __shared__ volatile int v;
-    return v;
-}
-__device__ __forceinline__ void pa_wait(uint32_t bar, uint32_t parity) {
-    if (pa_try(bar, parity)) return;
-    const uint32_t t0 = (uint32_t)clock();
-    while (!pa_try(bar, parity)) {
-        if ((uint32_t)clock() - t0 < 0x7fffffffu && !pa_gave_up()) continue;
-        pa_gave_up() = 1;
-        atomicExch(&g_pa_wait_failed, 1u);
-        return;
-    }
-}
 __device__ __forceinline__ void pa_tma(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar)
                  : "memory");
@@ -109,11 +82,6 @@ __device__ __forceinline__ float pa_ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ bool pa_elect() {
-    uint32_t pred;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
-    return pred != 0;
-}
 // 128-byte-swizzled operands (8-row atoms of 1024 bytes): K-major, and MN-major with `box` bytes between groups of 64 columns
 __device__ __forceinline__ uint64_t pa_desc(uint32_t addr, uint32_t box) {
     return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)(box >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
@@ -142,7 +110,7 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char *sQ = smem, *ring = sQ + (DK / 64) * kQBox, *sP = ring + ST * Sh::kStage;
     uint64_t *bars = reinterpret_cast<uint64_t *>(sP + kQBox);
-    const uint32_t q_full = pa_u32(bars), full0 = q_full + 8, empty0 = full0 + 8 * ST, s_full0 = empty0 + 8 * ST, s_free0 = s_full0 + 16, p_ready = s_free0 + 16, pv_done = p_ready + 8;
+    const uint32_t q_full = pa_u32(bars), full0 = q_full + 8, empty0 = full0 + 8 * ST, s_full0 = empty0 + 8 * ST, s_free0 = s_full0 + 16, p_ready = s_free0 + 16, pv_done = p_ready + 8, drain = pv_done + 8;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 16);
     float *red = reinterpret_cast<float *>(bars + 32);  // [2][128][WPR]
     float *pen = red + 2 * kQRows * WPR;                // [2][pen_len] (BIASED): the penalty of either head in base-2 units
@@ -161,7 +129,7 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     auto v_item = [&](int j) { return LATENT ? j : (j + 1 < n ? 2 * j + 2 : 2 * j + 1); };
 
     if (warp == WARPS && lane == 0) {
-        pa_gave_up() = 0;
+        cta_gave_up() = 0;
         pa_init(q_full, WARPS);
         for (int s = 0; s < ST; ++s) {
             pa_init(full0 + 8 * s, 1);
@@ -173,6 +141,7 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         }
         pa_init(p_ready, WARPS);
         pa_init(pv_done, 1);
+        pa_init(drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == WARPS + 1) {
@@ -183,50 +152,57 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     __syncthreads();
     pa_after();
     const uint32_t tmem = *tmem_slot;  // columns: S0 [0, 64) S1 [64, 128) O [128, 128 + DV)
+    // a wait that runs out ends all of the CTA's: no more copies, no more products; the softmax warps go through their tiles (they meet at named barriers)
+    // and store NaN
+    auto wait = [&](uint32_t bar, uint32_t parity) { return mbar_wait_guarded(bar, parity, p.wait, kWaitPromptAttn); };
 
     if (warp == WARPS) {
         // ================================================= producer
         if (lane == 0) {
             const int *bt = p.block_table + (size_t)seq * p.mpps + page0;
-            for (int i = 0; i < (LATENT ? n : 2 * n); ++i) {
+            int i = 0;
+            bool live = true;
+            for (; i < (LATENT ? n : 2 * n); ++i) {
                 const int s = i % ST;
                 const bool value = !LATENT && i > 0 && (i == 2 * n - 1 || (i & 1) == 0);
                 const int j = LATENT ? i : (i == 0 ? 0 : (value ? (i == 2 * n - 1 ? n - 1 : i / 2 - 1) : (i + 1) / 2));
                 const int row = LATENT ? __ldg(bt + j) * kPage : (__ldg(bt + j) * p.kv_heads + h0 / p.group) * kPage;
-                pa_wait(empty0 + 8 * s, ((i / ST) & 1) ^ 1);
+                live = wait(empty0 + 8 * s, ((i / ST) & 1) ^ 1);
+                if (!live) break;
                 const uint32_t d = pa_u32(ring + s * Sh::kStage), bar = full0 + 8 * s;
                 pa_expect(bar, Sh::kStage);
 #pragma unroll
                 for (int c = 0; c < DK / 64; ++c) pa_tma(d + c * kKBox, value ? &tmV : &tmK, 64 * c, row, bar);
             }
+            // the CTA stays until its last copies have landed and, if all is well, their stages have been released
+            for (int j = max(0, i - ST); j < i; ++j) {
+                if (!mbar_drain(full0 + 8 * (j % ST), (j / ST) & 1)) break;
+                if (live) live = wait(empty0 + 8 * (j % ST), (j / ST) & 1);
+            }
         }
     } else if (warp == WARPS + 1) {
-        // ================================================= MMA issuer
-        const uint32_t id_qk = pa_idesc(p.is_bf16 != 0, kPage, false), id_pv = pa_idesc(p.is_bf16 != 0, DV, true);
-        auto scores = [&](int j) {
-            const int i = k_item(j), s = i % ST, sb = j & 1;
-            pa_wait(full0 + 8 * s, (i / ST) & 1);
-            pa_wait(s_free0 + 8 * sb, ((j >> 1) & 1) ^ 1);
-            pa_after();
-            if (pa_elect()) {
+        // ================================================= MMA issuer: one thread
+        if (lane == 0) {
+            const uint32_t id_qk = pa_idesc(p.is_bf16 != 0, kPage, false), id_pv = pa_idesc(p.is_bf16 != 0, DV, true);
+            auto scores = [&](int j) -> bool {
+                const int i = k_item(j), s = i % ST, sb = j & 1;
+                if (!wait(full0 + 8 * s, (i / ST) & 1) || !wait(s_free0 + 8 * sb, ((j >> 1) & 1) ^ 1)) return false;
+                pa_after();
                 const uint32_t aq = pa_u32(sQ), bk = pa_u32(ring + s * Sh::kStage);
 #pragma unroll
                 for (int k = 0; k < DK / 16; ++k)
                     pa_mma(tmem + (uint32_t)(sb * kPage), pa_desc(aq + (k / 4) * kQBox + (k % 4) * 32, 16), pa_desc(bk + (k / 4) * kKBox + (k % 4) * 32, 16), id_qk, k > 0 ? 1u : 0u);
                 if (!LATENT) pa_commit(empty0 + 8 * s);  // (a latent page still serves as the values)
                 pa_commit(s_full0 + 8 * sb);
-            }
-            __syncwarp();
-        };
-        pa_wait(q_full, 0);
-        scores(0);
-        for (int j = 0; j < n; ++j) {
-            if (j + 1 < n) scores(j + 1);
-            const int i = v_item(j), s = i % ST;
-            if (!LATENT) pa_wait(full0 + 8 * s, (i / ST) & 1);
-            pa_wait(p_ready, j & 1);
-            pa_after();
-            if (pa_elect()) {
+                return true;
+            };
+            bool live = wait(q_full, 0) && scores(0);
+            for (int j = 0; live && j < n; ++j) {
+                if (j + 1 < n && !scores(j + 1)) break;
+                const int i = v_item(j), s = i % ST;
+                if (!LATENT && !wait(full0 + 8 * s, (i / ST) & 1)) break;
+                if (!wait(p_ready, j & 1)) break;
+                pa_after();
                 const uint32_t ap = pa_u32(sP), bv = pa_u32(ring + s * Sh::kStage);
 #pragma unroll
                 for (int k = 0; k < kPage / 16; ++k)
@@ -234,7 +210,8 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                 pa_commit(empty0 + 8 * s);
                 pa_commit(pv_done);
             }
-            __syncwarp();
+            pa_commit(drain);  // no product reads shared memory or writes TMEM when the CTA leaves
+            mbar_drain(drain, 0);
         }
     } else {
         // ================================================= softmax + epilogue: row = head half x token; WPR threads per row
@@ -286,7 +263,7 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         for (int j = 0; j < n; ++j) {
             const int sb = j & 1, kp = (page0 + j) * kPage, k0 = kp + cg * SC;
             uint32_t r[SC];
-            pa_wait(s_full0 + 8 * sb, (j >> 1) & 1);
+            (void)wait(s_full0 + 8 * sb, (j >> 1) & 1);
             pa_after();
 #pragma unroll
             for (int c = 0; c < SC; c += 16) pa_ld16(lane_addr + (uint32_t)(sb * kPage + cg * SC + c), r + c);
@@ -328,7 +305,7 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                     const float corr = need ? pa_ex2(m_use - m_run) : 1.0f;
                     if (need) m_use = m_run;
                     l *= corr;
-                    pa_wait(pv_done, (j - 1) & 1);
+                    (void)wait(pv_done, (j - 1) & 1);
                     pa_after();
 #pragma unroll
                     for (int c = 0; c < OC; c += 16) {
@@ -354,14 +331,14 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                 }
                 packed[q] = pack16<T>(pf);
             }
-            if (j > 0) pa_wait(pv_done, (j - 1) & 1);  // the previous product has read P
+            if (j > 0) (void)wait(pv_done, (j - 1) & 1);  // the previous product has read P
             unsigned char *prow = sP + row * 128;
 #pragma unroll
             for (int q = 0; q < SC / 8; ++q) *reinterpret_cast<uint4 *>(prow + (((cg * (SC / 8) + q) ^ (row & 7)) << 4)) = packed[q];
             // value rows past the tile's last query: cleared by the threads of rows 0 .. 63 (the scores have been formed: a shared tile may go too)
             if (row < kPage && kp + row > last) {
                 const int i = v_item(j);
-                pa_wait(full0 + 8 * (i % ST), (i / ST) & 1);
+                (void)wait(full0 + 8 * (i % ST), (i / ST) & 1);
                 unsigned char *v = ring + (i % ST) * Sh::kStage + row * 128;
                 for (int c = cg; c < DV / 8; c += WPR) *reinterpret_cast<uint4 *>(v + (c >> 3) * kKBox + ((c & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
             }
@@ -376,7 +353,7 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 #pragma unroll
         for (int c = 0; c < WPR; ++c) sum += rx[c];
         const float inv = LATENT ? 1.0f / sum : p.out_scale / sum;
-        pa_wait(pv_done, (n - 1) & 1);
+        const bool lost = !wait(pv_done, (n - 1) & 1) || cta_gave_up();  // (set before anything that was formed without having waited is handed on)
         pa_after();
 #pragma unroll
         for (int c = 0; c < OC; c += 16) {
@@ -387,7 +364,7 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                 const int col = cg * OC + c;
                 float f[16];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) f[e] = __uint_as_float(acc[e]) * inv;
+                for (int e = 0; e < 16; ++e) f[e] = lost ? __int_as_float(0x7fc00000) : __uint_as_float(acc[e]) * inv;
                 T *dst;
                 if constexpr (LATENT) {
                     dst = static_cast<T *>(p.out) + ((size_t)head * p.t_pad + row0 + tok) * DV + col;
@@ -442,8 +419,9 @@ bool pa_map(CUtensorMap *map, const void *ptr, int cols, bool bf16) {
 }
 
 template <typename T, int DK, int DV, bool LATENT, bool BIASED>
-int pa_launch(const PromptAttn &p, const void *k_pool, const void *v_pool, bool bf16, cudaStream_t st) {
+int pa_launch(PromptAttn p, const void *k_pool, const void *v_pool, bool bf16, cudaStream_t st) {
     CUtensorMap tmK, tmV;
+    p.wait = wait_guard();
     if (!pa_map(&tmK, k_pool, DK, bf16) || !pa_map(&tmV, v_pool, LATENT ? DK : DV, bf16)) {
         set_error("prompt attention: cuTensorMapEncodeTiled failed");
         return B200_ERR_CUDA;

@@ -1,6 +1,7 @@
 // runtime.cu -- error plumbing, device queries and the library workspace of libb200llm.so.
 #include "common.cuh"
 
+#include <atomic>
 #include <mutex>
 
 #ifndef B200_NO_NVTX
@@ -26,9 +27,54 @@ void set_error(const char *fmt, ...) {
 
 int cuda_status(const char *what) {
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) return B200_OK;
+    if (e == cudaSuccess) return wait_status(what);
     set_error("%s: %s", what, cudaGetErrorString(e));
     return B200_ERR_CUDA;
+}
+
+// The wait word of the process, made by the first launch that needs it.
+static std::atomic<unsigned int *> g_wait_word{nullptr};
+static thread_local unsigned int t_wait_clocks = kWaitClocks;
+static unsigned int *wait_word() {
+    static std::once_flag once;
+    std::call_once(once, [] {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (the launch may be one that is being captured)
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+            *static_cast<unsigned int *>(p) = 0;
+            g_wait_word.store(static_cast<unsigned int *>(p), std::memory_order_release);
+        } else {
+            cudaGetLastError();
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    });
+    return g_wait_word.load(std::memory_order_acquire);
+}
+WaitGuard wait_guard() { return {wait_word(), t_wait_clocks}; }  // (one address for host and devices: unified addressing)
+
+static unsigned int wait_code() {
+    unsigned int *w = g_wait_word.load(std::memory_order_acquire);
+    return w ? *reinterpret_cast<volatile unsigned int *>(w) : 0u;
+}
+int wait_status(const char *what) {
+    const unsigned int code = wait_code();
+    if (code == 0) return B200_OK;
+    static const char *const names[] = {"", "the streaming GEMV", "the CTA-pair GEMM", "the prompt attention", "the wait probe"};
+    set_error("%s: a wait inside %s ran out; results since then are not valid (b200_wait_error(1) clears this)", what, code <= kWaitProbe ? names[code] : "a kernel");
+    return B200_ERR_CUDA;
+}
+
+// a barrier that nothing arrives at: what is left of a kernel whose producer never comes
+__global__ void wait_probe_kernel(WaitGuard wait) {
+    __shared__ __align__(8) unsigned long long bar;
+    const uint32_t addr = (uint32_t)__cvta_generic_to_shared(&bar);
+    if (threadIdx.x == 0) {
+        cta_gave_up() = 0;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(addr) : "memory");
+    }
+    __syncthreads();
+    mbar_wait_guarded(addr, 0, wait, kWaitProbe);
 }
 
 int sm_count() {
@@ -78,6 +124,17 @@ extern "C" {
 const char *b200_last_error_string(void) { return g_err; }
 int b200_abi_version(void) { return B200LLM_ABI_VERSION; }
 int b200_sm_count(void) { return sm_count(); }
+
+int b200_wait_error(int clear) {
+    const unsigned int code = wait_code();
+    if (clear && code) *reinterpret_cast<volatile unsigned int *>(g_wait_word.load(std::memory_order_acquire)) = 0;
+    return (int)code;
+}
+void b200_wait_limit(unsigned int clocks) { t_wait_clocks = clocks < kWaitClocks ? clocks : kWaitClocks; }
+int b200_wait_probe(b200_stream_t stream) {
+    wait_probe_kernel<<<1, 64, 0, as_stream(stream)>>>(wait_guard());
+    return cuda_status("wait_probe launch");
+}
 
 size_t b200_workspace_default_bytes(void) { return (size_t)64 << 20; }
 
