@@ -78,8 +78,8 @@ topk_stage1_kernel(const T *__restrict__ logits, int *__restrict__ tmp_ids, T *_
     int li[kMaxK];
 #pragma unroll
     for (int i = 0; i < kMaxK; ++i) lv[i] = -INFINITY, li[i] = INT_MAX;
-    pdl_launch_dependents();  // the merge is small: it takes its place (and its random numbers) while this runs
     pdl_wait();
+    pdl_launch_dependents();  // the merge is small: it takes its place (and its random numbers) while this runs
     const T *p = logits + (size_t)row * vocab;
     constexpr int U = 16;  // loads in flight per thread: a block's share of 32000 logits is 16 per thread, one round trip instead of 16
     for (int base = lo + threadIdx.x; base < hi; base += U * kTopkThreads) {
@@ -243,10 +243,10 @@ topk_stage2_kernel(const int *__restrict__ tmp_ids, const T *__restrict__ tmp_va
     int li[kMaxK];
 #pragma unroll
     for (int i = 0; i < kMaxK; ++i) lv[i] = -INFINITY, li[i] = INT_MAX;
-    if (!DRAW) pdl_launch_dependents();
     float uniform = 0.0f;
     if (DRAW && threadIdx.x == 0) uniform = first_uniform((unsigned long long)draw.step, (unsigned int)row);
     pdl_wait();
+    if (!DRAW) pdl_launch_dependents();
     for (int i = threadIdx.x; i < B200_TOPK_BLOCKS * k; i += 64) {
         const int id = tmp_ids[(size_t)row * B200_TOPK_BLOCKS * k + i];
         if (id >= 0) insert(lv, li, Elem<T>::to_f(tmp_vals[(size_t)row * B200_TOPK_BLOCKS * k + i]), id);
