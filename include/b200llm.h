@@ -765,6 +765,15 @@ int b200_mlstm_recurrent(const float *rec, float *state, float *n_state, float *
 int b200_decay_recurrent(const float *rec, float *state, float *o, const int *seq_start, const int *seq_pos0, const int *seq_slot,
                          int n_seqs, int heads, int kv_heads, int dim, int vdim, b200_stream_t stream);
 
+/* The three recurrences above over portions of 64 tokens and more, 32 tokens at a time (shorter portions are left as they are: the launchers above take
+ * them).  kind: B200_MIXER_GLA (rows = proj, kv_heads = heads), B200_MIXER_DELTA or B200_MIXER_LINEAR (rows = rec, fp32: dtype B200_F32, ld and decay unused).
+ * dim 64 or 128, vdim a multiple of 16, rows in 16-byte pieces; B200_ERR_UNSUPPORTED otherwise.  scratch: DEVICE, of at least
+ * b200_chunk_recurrence_scratch_bytes (0: sizes it never takes); tokens / longest: of this call, of its longest portion. */
+size_t b200_chunk_recurrence_scratch_bytes(int kind, int heads, int dim, int max_tokens, int max_seqs);
+int b200_chunk_recurrence(int kind, const void *rows, int ld, const float *decay, float *state, float *o, const int *seq_start, const int *seq_pos0,
+                          const int *seq_slot, int n_seqs, int heads, int kv_heads, int dim, int vdim, void *scratch, size_t scratch_bytes, int tokens,
+                          int longest, int dtype, b200_stream_t stream);
+
 /* The minGRU recurrence (B200_MIXER_MINGRU).  proj [tokens, ld] of `dtype`: z | u | gate (cols each); bias fp32 [2*cols] for z and u, or
  * NULL; state fp32 [num_slots, cols]; out [tokens, cols] of `dtype`.  Portions of 8 tokens or more are described by `chunks`, DEVICE int4
  * {sequence, first packed row, tokens, index in its portion} (a portion's chunks in order and complete; 16-byte aligned); maps: fp32 scratch

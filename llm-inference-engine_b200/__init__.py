@@ -220,6 +220,8 @@ SIGNATURES = {
     "b200_scored_attention_tiles_paged": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _F, _P, _I, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P],
     "b200_delta_rule_recurrent": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "b200_mlstm_recurrent": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
+    "b200_chunk_recurrence_scratch_bytes": [_I, _I, _I, _I, _I],
+    "b200_chunk_recurrence": [_I, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _SZ, _I, _I, _I, _P],
     "b200_decay_recurrent": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "b200_mingru": [_P, _I, _P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P],
     "b200_poly_norm": [_P, _P, _F, _I, _I, _I, _P],
@@ -241,7 +243,7 @@ _RESTYPES = {"b200_last_error_string": C.c_char_p, "b200_wait_limit": None, "b20
              "b200_decoder_tp_buffer_bytes": _SZ, "b200_generate_workspace_bytes": _SZ, "b200_batcher_create": _P,
              "b200_batcher_destroy": None, "b200_batcher_plan_array": C.POINTER(C.c_int), "b200_batcher_workspace_bytes": _SZ,
              "b200_hybrid_create": _P, "b200_hybrid_destroy": None, "b200_hybrid_scratch_bytes": _SZ, "b200_hybrid_kv_pool_bytes": _SZ,
-             "b200_hybrid_state_pool_bytes": _SZ, "b200_batcher_hybrid_workspace_bytes": _SZ}
+             "b200_hybrid_state_pool_bytes": _SZ, "b200_chunk_recurrence_scratch_bytes": _SZ, "b200_batcher_hybrid_workspace_bytes": _SZ}
 
 _lib = None
 
@@ -266,15 +268,15 @@ def check(rc):
         raise B200Error(f"b200 status {rc}: {lib().b200_last_error_string().decode()}")
 
 
-# ------------------------------------------------------------------ torch plumbing (device memory + streams only)
-def _torch():
-    import torch
 def wait_error(clear=False):
     """The code of a wait inside a kernel that ran out since the last clear (0: none): results since then are not valid, and every call raises until it
     is cleared.  Replayed graphs make no calls, so a program that replays them reads this where it synchronises."""
     return lib().b200_wait_error(int(clear))
 
 
+# ------------------------------------------------------------------ torch plumbing (device memory + streams only)
+def _torch():
+    import torch
 
     return torch
 
