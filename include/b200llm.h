@@ -773,6 +773,10 @@ size_t b200_chunk_recurrence_scratch_bytes(int kind, int heads, int dim, int max
 int b200_chunk_recurrence(int kind, const void *rows, int ld, const float *decay, float *state, float *o, const int *seq_start, const int *seq_pos0,
                           const int *seq_slot, int n_seqs, int heads, int kv_heads, int dim, int vdim, void *scratch, size_t scratch_bytes, int tokens,
                           int longest, int dtype, b200_stream_t stream);
+/* decay fp32 [tokens, channels] = sigmoid(W_decay x + bias)^(1/tau), x the `rank` columns of proj [tokens, ld] from column col0 on, W_decay
+ * [channels, rank] of `dtype`, bias fp32 or NULL: the decays of B200_MIXER_GLA. */
+int b200_gla_decay(const void *proj, int ld, int col0, const void *w_decay, const float *bias, float tau, float *decay, int tokens, int rank, int channels,
+                   int dtype, b200_stream_t stream);
 
 /* The minGRU recurrence (B200_MIXER_MINGRU).  proj [tokens, ld] of `dtype`: z | u | gate (cols each); bias fp32 [2*cols] for z and u, or
  * NULL; state fp32 [num_slots, cols]; out [tokens, cols] of `dtype`.  Portions of 8 tokens or more are described by `chunks`, DEVICE int4

@@ -222,6 +222,7 @@ SIGNATURES = {
     "b200_mlstm_recurrent": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     "b200_chunk_recurrence_scratch_bytes": [_I, _I, _I, _I, _I],
     "b200_chunk_recurrence": [_I, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _SZ, _I, _I, _I, _P],
+    "b200_gla_decay": [_P, _I, _I, _P, _P, _F, _P, _I, _I, _I, _I, _P],
     "b200_decay_recurrent": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "b200_mingru": [_P, _I, _P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P],
     "b200_poly_norm": [_P, _P, _F, _I, _I, _I, _P],

@@ -111,7 +111,12 @@ gla_decay_mma_kernel(const T *__restrict__ proj, int ld, int col0, const T *__re
         float z[4] = {};
 #pragma unroll
         for (int j = 0; j < NB; ++j)
-            if (j < nb) decay_mma<T>(z, lo[j], hi[j], ld_v4(wr + 32 * j));
+            if (j < nb) {  // (32 products at a time: what the instruction adds up is cut off, not rounded, and one chain through the rank let that grow)
+                float part[4] = {};
+                decay_mma<T>(part, lo[j], hi[j], ld_v4(wr + 32 * j));
+#pragma unroll
+                for (int e = 0; e < 4; ++e) z[e] += part[e];
+            }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int c = c0 + 2 * t + (e & 1), tok = e < 2 ? t0 : t1;
@@ -576,4 +581,11 @@ extern "C" int b200_gla_recurrent(const void *proj, int ld, const float *decay, 
     B200_REQUIRE(proj && decay && state && o && seq_start && seq_pos0 && seq_slot, "gla_recurrent: null pointer");
     B200_REQUIRE(n_seqs >= 0 && heads > 0 && dim > 0 && vdim > 0 && ld >= 2 * heads * dim + heads * vdim, "gla_recurrent: bad shape");
     return launch_gla_recurrent(dtype, proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, n_seqs, heads, dim, vdim, as_stream(stream));
+}
+
+extern "C" int b200_gla_decay(const void *proj, int ld, int col0, const void *w_decay, const float *bias, float tau, float *decay, int tokens, int rank,
+                              int channels, int dtype, b200_stream_t stream) {
+    B200_REQUIRE(proj && w_decay && decay, "gla_decay: null pointer");
+    B200_REQUIRE(tokens >= 0 && rank > 0 && channels > 0 && col0 >= 0 && ld >= col0 + rank && tau > 0.0f, "gla_decay: bad shape");
+    return launch_gla_decay(dtype, proj, ld, col0, w_decay, bias, tau, decay, tokens, rank, channels, as_stream(stream));
 }

@@ -178,3 +178,22 @@ def test_no_further_from_64_bits_than_the_serial_kernels(kind, dim, decays, lens
         errors.append([float((got.double() - w).norm() / w.norm()) for got, w in zip((o, state), want)])
     # (the same roundings in another order: 5 % for the spread of two samples of a few thousand values)
     assert all(c <= 1.05 * s for s, c in zip(*errors)), errors
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("rank", [32, 64, 256])
+def test_decays_on_the_tensor_cores(dtype, rank):
+    """Against 64 bits, beside the general kernel (which takes columns that do not start on a 16-byte boundary)."""
+    T, channels, tau = 515, 1000, 16.0
+    gen = torch.Generator(device=DEV).manual_seed(rank)
+    rand = lambda *s: torch.randn(*s, generator=gen, device=DEV)  # noqa: E731
+    x, w, bias = rand(T, rank).to(dtype), (2 * rand(channels, rank) / rank ** 0.5).to(dtype), rand(channels)
+    want = torch.exp(torch.nn.functional.logsigmoid(x.double() @ w.double().T + bias.double()) / tau)
+    errors = []
+    for col0 in (1, 8):
+        proj = torch.zeros(T, rank + 8, dtype=dtype, device=DEV)
+        proj[:, col0:col0 + rank] = x
+        got = torch.zeros(T, channels, device=DEV)
+        b200.check(b200.lib().b200_gla_decay(proj.data_ptr(), rank + 8, col0, w.data_ptr(), bias.data_ptr(), tau, got.data_ptr(), T, rank, channels, b200.dtype_code(x), b200.stream()))
+        errors.append(float((got.double().log() - want.log()).norm() / want.log().norm()))
+    assert errors[1] <= 1.02 * errors[0], errors
