@@ -30,6 +30,9 @@ norm_kernel(const T *in, T *out, const T *residual_in, T *residual_out, const T 
     T *rout = residual_out ? residual_out + (size_t)row * hidden : nullptr;
 
     pdl_wait();
+    // (at once: the linear behind fills its ring with weights while this kernel works.  Released behind the row's loads, a 7B step of one FP8 token, whose
+    // norms stand in front of the linears, took 246 us where the norms inside the linears had taken 243)
+    pdl_launch_dependents();
     const unsigned int tp_want = kTp ? tp_flag(tp.epoch, tp.seq) : 0u;
     // pre-norm value of vector i: o (+ residual); residual_out <- that; (+ bias)
     auto prenorm = [&](int i, float *f) {
@@ -93,7 +96,6 @@ norm_kernel(const T *in, T *out, const T *residual_in, T *residual_out, const T 
         if constexpr (kVec) st_v4(o + (size_t)i * V, pack16<T>(f));
         else o[i] = Elem<T>::from_f(f[0]);
     }
-    pdl_launch_dependents();
     ss = block_sum(ss, red);
     const float r = rsqrtf(ss / (float)hidden + eps);
 #pragma unroll
