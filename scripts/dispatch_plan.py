@@ -1,14 +1,12 @@
 #!/usr/bin/env python
 """Which kernel, how many passes over the weights and which ring geometry each linear of a decode step gets -- a Python MODEL of the host-side
-dispatch (no GPU): decoder.cu norm_linear / plain_linear (fused GEMV for M <= gemv_max_rows, un-fused otherwise), linear.cu:300-330
-(tcgen05 GEMM for dense M > 4, else GEMV passes of 8 / 4 rows), gemv_inst.cuh:32-60 (gemv_nk geometry) and gemv_rs.cuh gemv_rs_geometry.
-It restates those few formulas; when they change, this file must follow.  linear_plan is the dispatch without gemv_rs -- gemv_mma.cuh, which still takes
-what gemv_rs refuses, and the quantised GEMV with the fused prologue, whose place gemv_rs has taken -- and is kept for reading the profiles measured with
-it (tests/test_dispatch_plan.py pins those cases); decode_plan is the dispatch of today.
+dispatch (no GPU): decoder.cu norm_linear (norm inside the GEMV for one dense token, a norm kernel in front otherwise), gemv_f32.cu launch_gemv_nk
+(gemv_rs, what its ring refuses on gemv_mma, the SIMT GEMV for up to 4 tokens), linear.cu (GEMV passes, tcgen05 GEMM for dense M > 16), gemv_inst.cuh,
+gemv_rs.cuh gemv_rs_geometry and gemv_mma.cuh gemv_mma_geometry.  It restates those few formulas; when they change, this file must follow
+(tests/test_dispatch_plan.py).
 usage: python scripts/dispatch_plan.py > profiles/<tag>_dispatch_plan.txt"""
 BUDGET = 224 * 1024
 GROUPS, GW, MAX_STAGES, ROWS, PIECE = 2, 8, 8, 2, 8192
-Q_ROWS, Q_TOK = 16, 8
 MMA_WARPS, MMA_ROWS = 16, 8
 WARPS = GROUPS * GW
 
@@ -31,20 +29,6 @@ def gemv_nk_plan(M, K, fmt, ebytes=2):
     if fixed + 3 * per_stage > BUDGET:
         return None
     return dict(kernel="gemv_nk", pieces=pieces, piece_bytes=piece_bytes, stages=min((BUDGET - fixed) // per_stage, MAX_STAGES))
-
-
-def gemv_q_plan(M, K, fmt):
-    """gemv_q.cuh launch_gemv_q_t / launch_gemv_q_inst (16-bit activations): None when unsupported."""
-    if fmt not in ("fp8", "int4") or M < 1 or M > Q_TOK or K % 128:
-        return None
-    xs_stride = K + (16 if fmt == "fp8" else 32)
-    fixed = (M * xs_stride * 2 + 127) // 128 * 128 + GROUPS * (2 * MAX_STAGES + 4) * 8 + WARPS * 2 * Q_ROWS * Q_TOK * 4
-    for piece in (2048, 1024):
-        per_stage = GROUPS * Q_ROWS * (piece + 16)
-        if fixed + 3 * per_stage <= BUDGET:
-            k_per_piece = piece * (1 if fmt == "fp8" else 2)
-            return dict(kernel="gemv_q", pieces=-(-K // k_per_piece), piece_bytes=piece, stages=min((BUDGET - fixed) // per_stage, MAX_STAGES))
-    return None
 
 
 def gemv_mma_plan(M, K, fmt, max_units=8):
@@ -89,20 +73,6 @@ def gemv_mma_plan(M, K, fmt, max_units=8):
     return best
 
 
-def gemv_any(M, K, fmt):
-    """gemv_f32.cu launch_gemv_nk for a 16-bit model: the tensor-core GEMV for 2..16 dense tokens and 5..16 quantised ones, the round-1
-    quantised kernel for 1..4 quantised tokens (fused prologue), the SIMT kernel for one dense token."""
-    if 2 <= M <= 16 and (fmt == "dense" or M > 4):
-        g = gemv_mma_plan(M, K, fmt)
-        if g:
-            return g
-    if fmt != "dense" and M <= 8:
-        g = gemv_q_plan(M, K, fmt)
-        if g:
-            return g
-    return gemv_nk_plan(M, K, fmt)
-
-
 RS_BLOCKS, RS_STAGES, SMS = 8, 12, 148
 
 
@@ -127,33 +97,33 @@ def gemv_rs_plan(M, K, N, fmt, swiglu=False):
     return dict(kernel="gemv_rs", pieces=parts, piece_bytes=row, stages=min((226 * 1024 - fixed) // stage, RS_STAGES), parts=parts, part_k=part_k)
 
 
-def decode_plan(M, K, N, fmt, fused_rows, swiglu=False):
-    """One linear of the decode step as gemv_f32.cu / linear.cu dispatch it: (path, passes over the weights, geometry)."""
-    step = M if M <= fused_rows else 16
-    plans = [gemv_rs_plan(min(step, M - m0), K, N, fmt, swiglu) for m0 in range(0, M, step)]
-    if all(plans) and (M <= fused_rows or (fmt != "dense" and M <= 64)):
-        if M <= fused_rows:
-            return ("norm_kernel + gemv_rs", 1, plans[0])
-        return (f"un-fused gemv_rs x {len(plans)} passes of <= {step} tokens", len(plans), plans[0])
-    return linear_plan(M, K, fmt, fused_rows)
-
-
-def linear_plan(M, K, fmt, fused_rows):
-    """One linear of the decode step: (path, passes over the weights, geometry)."""
-    if M <= fused_rows:
-        g = gemv_any(M, K, fmt)
-        if g:  # gemv_nk / gemv_q run the norm / residual / TP-reduce prologue themselves; gemv_mma takes plain activations (norm_kernel in front)
-            return (("norm_kernel + " if g["kernel"] == "gemv_mma" else "fused ") + g["kernel"], 1, g)
-    if M <= 16:  # linear.cu: one GEMV pass for decode batches
-        g = gemv_any(M, K, fmt)
+def gemv_any(M, K, N, fmt, swiglu=False):
+    """gemv_f32.cu launch_gemv_nk for a 16-bit model."""
+    if M <= 16 and (M >= 2 or fmt != "dense"):
+        rows = 16 if fmt == "fp8" else 8
+        units = -(-(N // 2) // (rows // 2)) if swiglu else -(-N // rows)
+        g = gemv_rs_plan(M, K, N, fmt, swiglu) or gemv_mma_plan(M, K, fmt, -(-units // max(1, min(SMS, units))))
         if g:
-            return ("un-fused " + g["kernel"], 1, g)
+            return g
+    return gemv_nk_plan(M, K, fmt)
+
+
+def linear_plan(M, K, N, fmt, fused_rows=16, swiglu=False):
+    """One linear of the decode step: (path, passes over the weights, geometry)."""
+    if M == 1 and fmt == "dense":  # the norm / residual / tensor-parallel prologue inside the GEMV
+        g = gemv_nk_plan(M, K, fmt)
+        if g:
+            return ("fused " + g["kernel"], 1, g)
+    if M <= fused_rows:
+        g = gemv_any(M, K, N, fmt, swiglu)
+        if g:
+            return ("norm_kernel + " + g["kernel"], 1, g)
     if fmt == "dense" and M > 4:
         return ("un-fused gemm_tc (tcgen05, swap-AB stream-K)" if M <= 128 else "un-fused gemm_tc", 1, None)
-    for step in (16, 8, 4):  # linear.cu: quantised weights up to 64 tokens in passes
-        if M > 4 * step or M > 64:
+    for step in (16, 8, 4):  # linear.cu: quantised weights in passes
+        if M > (8 if step == 16 else 4) * step:
             continue
-        plans = [gemv_any(min(step, M - m0), K, fmt) for m0 in range(0, M, step)]
+        plans = [gemv_any(min(step, M - m0), K, N, fmt) for m0 in range(0, M, step)]
         if all(plans):
             return (f"un-fused {plans[0]['kernel']} x {len(plans)} passes of <= {step} tokens", len(plans), plans[0])
     return ("un-fused generic SIMT fallback (launch_simt, linear.cu)", 1, None)
@@ -165,7 +135,7 @@ def step_plan(name, hidden, heads, kv_heads, d, inter, tp, batch, fmt):
               ("down", inter // tp, hidden)]
     lines = [f"{name}, batch {batch}, weights {fmt}" + (f", TP-{tp} (one rank)" if tp > 1 else "")]
     for lin, K, N in shapes:
-        path, passes, g = decode_plan(batch, K, N, fmt, fused_rows, lin == "gate_up")
+        path, passes, g = linear_plan(batch, K, N, fmt, fused_rows, lin == "gate_up")
         geo = (f"pieces {g['pieces']} x {g['piece_bytes']} B, {g['stages']} stages" + (f", {g['parts']} activation parts of {g['part_k']} k" if g.get("parts") else "")) if g else "-"
         wbytes = K * N * {"dense": 2, "fp8": 1, "int4": 0.5}[fmt]
         lines.append(f"  {lin:8s} K={K:6d} N={N:6d}  {path:58s} weights read {passes} x {wbytes / 1e6:7.1f} MB   {geo}")

@@ -1,9 +1,10 @@
-"""scripts/dispatch_plan.py restates the host-side kernel selection (decoder.cu / linear.cu / gemv_inst.cuh / gemv_q.cuh) so that the plan of a
-decode step can be read without a GPU.  These cases pin it to geometries that were observed on the B200 (six 16 KB stages per
-group for the bf16 GEMV at batch 1; the 3-stage ring of the quantised kernel; 8 tokens of a K = 11008 row do not fit) so the model cannot
-drift silently from the numbers the design document quotes."""
+"""scripts/dispatch_plan.py restates the host-side kernel selection (decoder.cu / gemv_f32.cu / linear.cu / gemv_inst.cuh / gemv_rs.cuh / gemv_mma.cuh) so that
+the plan of a decode step can be read without a GPU.  These cases pin it to the geometries of the dispatch (six 16 KB stages per group for the bf16 GEMV at
+one token; whole-unit stages of gemv_rs, whose ring and sums share the SM; the sizes gemv_rs refuses)."""
 import os
 import sys
+
+import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, os.path.join(ROOT, "scripts"))
@@ -17,32 +18,51 @@ def test_dense_batch1_geometry_matches_the_design_document():
     assert g["pieces"] == 3 and g["piece_bytes"] % 512 == 0 and g["pieces"] * g["piece_bytes"] >= 11008 * 2
 
 
-def test_quantised_round1_kernel_geometry_is_still_modelled():
-    assert dp.gemv_q_plan(1, 4096, "int4") == dict(kernel="gemv_q", pieces=1, piece_bytes=2048, stages=3)
-    assert dp.gemv_q_plan(8, 11008, "fp8") is None and dp.gemv_q_plan(8, 11008, "int4") is None  # 176 KB of activations: no ring fits
+@pytest.mark.parametrize("fmt", ["dense", "fp8", "int4"])
+@pytest.mark.parametrize("k", [128, 4096, 4224, 11008, 28672])
+@pytest.mark.parametrize("m", [1, 2, 8, 9, 16])
+def test_streaming_gemv_geometry(fmt, k, m):
+    """Parts cover the row in whole groups of 128 that a warp's eight blocks reach, and at least two stages fit beside the tiles and the parts' sums."""
+    g = dp.gemv_rs_plan(m, k, 4096, fmt)
+    if fmt == "dense" and m == 1:
+        assert g is None
+        return
+    assert g["parts"] == max(1, -(-k // 4096)) and g["part_k"] % 128 == 0 and g["part_k"] <= 16 * 8 * 32
+    assert g["parts"] * g["part_k"] >= k > (g["parts"] - 1) * g["part_k"]
+    rows, nt = (8 if fmt == "dense" else 16), (2 if m > 8 else 1)
+    stage = rows * (-(-g["piece_bytes"] // 128) * 128 + (16 if fmt == "fp8" else 64))
+    tile, sums = (128, 128) if fmt == "dense" else (160 * nt, 128 * nt)
+    units = -(-(-(-4096 // rows)) // 148)
+    assert 2 <= g["stages"] <= 12
+    assert g["stages"] * stage + 28 * 8 + 2 * 16 * tile * 4 + (units * sums * 4 if g["parts"] > 1 else 0) <= 226 * 1024
 
 
-def test_tensor_core_gemv_reads_the_weights_once_up_to_16_tokens():
-    """gemv_mma.cuh: activations staged in K parts of 64 KiB, so K = 8192 and K = 11008 keep a >= 4-stage ring at 8 and at 16 tokens; every
-    decode batch up to 16 is ONE pass over the weights, in every format (round 1: 2 passes at batch 16, 4 for the K = 11008 down projection)."""
-    for m, k in ((2, 4096), (8, 4096), (16, 4096), (8, 8192), (8, 11008), (16, 11008)):  # incl. the 70B-shaped hidden size and the 7B down projection
-        g = dp.gemv_mma_plan(m, k, "dense")
-        assert g and g["stages"] >= 3 and g["parts"] * g["part_k"] >= k, (m, k, g)
-        assert (m + 1) * (g["part_k"] + 32) * 2 + g["stages"] * 8 * (g["piece_bytes"] + 64) <= 226 * 1024  # the staged part and the ring share the SM
-    assert dp.gemv_mma_plan(8, 4096, "dense")["parts"] == 1 and dp.gemv_mma_plan(16, 4096, "dense")["parts"] == 2
-    assert dp.gemv_mma_plan(8, 8192, "dense")["parts"] == 2  # 8 tokens x 8192 k do not fit beside a ring: two parts of 4096
+def test_streaming_gemv_stages():
+    """16 tokens at K = 4096: two 64 KB FP8 stages beside the tiles, five INT4 ones, three dense ones; K = 11008 goes in three parts."""
+    stages = {fmt: dp.gemv_rs_plan(16, 4096, 4096, fmt)["stages"] for fmt in ("dense", "fp8", "int4")}
+    assert stages == {"dense": 3, "fp8": 2, "int4": 5}
+    assert dp.gemv_rs_plan(16, 11008, 4096, "fp8")["parts"] == 3
+
+
+def test_decode_batches_read_the_weights_once():
+    """Every decode batch up to 16 is ONE pass over the weights, in every format, behind a norm kernel; one dense token keeps the norm inside the GEMV."""
     for fmt in ("dense", "fp8", "int4"):
-        for m in (2, 8, 16):
-            for k in (4096, 11008):
-                path, passes, geo = dp.linear_plan(m, k, fmt, fused_rows=16)
-                want = "fused gemv_q" if (fmt != "dense" and m <= 4) else "norm_kernel + gemv_mma"
+        for m in (1, 2, 4, 8, 16):
+            for k, n in ((4096, 12288), (11008, 4096), (8192, 1280)):
+                path, passes, geo = dp.linear_plan(m, k, n, fmt)
+                want = "fused gemv_nk" if fmt == "dense" and m == 1 else "norm_kernel + gemv_rs"
                 assert passes == 1 and path == want, (fmt, m, k, path)
-    assert dp.linear_plan(1, 4096, "dense", fused_rows=16)[0] == "fused gemv_nk"  # a single dense token stays on the SIMT kernel
-    assert dp.linear_plan(1, 4096, "int4", fused_rows=16)[0] == "fused gemv_q"  # up to 4 quantised tokens: the kernel with the fused prologue
-    path, passes, _ = dp.linear_plan(32, 4096, "fp8", fused_rows=16)
-    assert passes == 2 and "16 tokens" in path
+    path, passes, _ = dp.linear_plan(32, 4096, 4096, "fp8")
+    assert passes == 2 and path == "un-fused gemv_rs x 2 passes of <= 16 tokens"
+
+
+def test_sums_of_a_vocabulary_leave_no_ring():
+    """Rows of more than 4096 k with vocabulary-sized outputs: the parts' sums fill the SM, and the kernel with the activations in shared memory takes over."""
+    assert dp.linear_plan(16, 8192, 128256, "fp8")[0] == "norm_kernel + gemv_rs"
+    path, passes, geo = dp.linear_plan(16, 8192, 152064, "fp8")
+    assert (path, passes) == ("norm_kernel + gemv_mma", 1) and geo["parts"] * geo["part_k"] >= 8192 and geo["stages"] >= 3
 
 
 def test_dense_batches_beyond_16_go_to_the_tensor_core_gemm():
     for m in (17, 32, 128):
-        assert dp.linear_plan(m, 4096, "dense", fused_rows=16)[0].startswith("un-fused gemm_tc")
+        assert dp.linear_plan(m, 4096, 4096, "dense")[0].startswith("un-fused gemm_tc")
