@@ -62,6 +62,34 @@ def test_linear_of_few_tokens_and_odd_rows(n):
     assert bool((out[6 * n:] == 7.0).all())
 
 
+@pytest.mark.parametrize("fmt,n", [("dense", 192000), ("fp8", 152064), ("int4", 290000)])
+def test_linear_whose_sums_leave_no_ring(fmt, n):
+    """Vocabulary-sized outputs of rows of 8192 k, 16 tokens: sizes that stay with the kernel whose activations are in shared memory (csrc/gemv_mma.cuh), and
+    (INT4) that neither takes at once: two passes of eight tokens."""
+    m, k, step = 16, 8192, 16000
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    x = torch.randn(m, k, generator=gen, device=DEV).bfloat16()
+    kw = {}
+    if fmt == "dense":
+        w = torch.empty(n, k, dtype=torch.bfloat16, device=DEV).normal_(generator=gen)
+    elif fmt == "fp8":
+        w = torch.randint(0, 0x70, (n, k), generator=gen, device=DEV, dtype=torch.uint8) | (torch.randint(0, 2, (n, k), generator=gen, device=DEV, dtype=torch.uint8) << 7)
+        kw = dict(w_format=b200.W_FP8, scales=torch.rand(n, generator=gen, device=DEV) + 0.5, N=n)
+    else:
+        w = torch.randint(0, 256, (n, k // 2), generator=gen, device=DEV, dtype=torch.uint8)
+        kw = dict(w_format=b200.W_INT4, scales=(torch.rand(n, k // 128, generator=gen, device=DEV) + 0.5).bfloat16(),
+                  zeros=torch.randint(0, 16, (n, k // 128), generator=gen, device=DEV, dtype=torch.uint8), group=128, N=n)
+    got = b200.linear(x, w, **kw)
+    for r in range(0, n, step):
+        part = w[r:r + step]
+        if fmt == "fp8":
+            part = part.view(torch.float8_e4m3fn).to(torch.float32) * kw["scales"][r:r + step, None]
+        elif fmt == "int4":
+            q = torch.stack((part & 15, part >> 4), -1).reshape(len(part), k // 128, 128).float() - kw["zeros"][r:r + step, :, None].float()
+            part = (q * kw["scales"][r:r + step, :, None].float()).reshape(len(part), k)
+        close(got[:, r:r + step], x.double() @ part.double().T, torch.bfloat16, (fmt, r))
+
+
 @pytest.mark.parametrize("fmt", ["dense", "fp8", "int4"])
 @pytest.mark.parametrize("batch", [1, 2, 5, 8, 9, 16])
 def test_few_tokens_match_the_same_rows_in_a_larger_batch(fmt, batch):
