@@ -482,7 +482,7 @@ static int launch_mma_t(const void *q, const void *k_pool, const void *v_pool, c
                         cudaStream_t st) {
     const size_t smem = (size_t)(kTileQ + 4 * kPage) * D * sizeof(T);
     cudaFuncSetAttribute(chunked_attn_mma_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(chunked_attn_mma_kernel<T, D>, dim3(n_tiles, heads), dim3(128), smem, st, false, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink, (const T *)gate_in,
+    launch_plain(chunked_attn_mma_kernel<T, D>, dim3(n_tiles, heads), dim3(128), smem, st, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink, (const T *)gate_in,
                                                                             gate_ld, (T *)out, (const int4 *)tiles, block_table, mpps, heads, kv_heads,
                                                                             scale, chunk);
     return cuda_status("chunked_attention (tensor core) launch");
@@ -518,7 +518,7 @@ int launch_attn_qk_norm_cache(int dtype, const void *proj, int ld, void *q_out, 
                               int tokens, int heads, int kv_heads, int dim, cudaStream_t st) {
     if (tokens == 0) return B200_OK;
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(attn_qk_norm_cache_kernel<T>, dim3(tokens), dim3(256), 0, st, false, (const T *)proj, ld, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
+        launch_plain(attn_qk_norm_cache_kernel<T>, dim3(tokens), dim3(256), 0, st, (const T *)proj, ld, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
                                                               tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim);
     });
     return cuda_status("attn_qk_norm_cache launch");
@@ -538,7 +538,7 @@ int launch_chunked_attention(int dtype, const void *q, const void *k_pool, const
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(chunked_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(chunked_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, false, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink,
+        launch_plain(chunked_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink,
                                                                             (const T *)gate_in, gate_ld, (T *)out, tok_seq, tok_pos,
                                                                             block_table, mpps, heads, kv_heads, dim, scale, chunk, max_keys, tok_list);
     });

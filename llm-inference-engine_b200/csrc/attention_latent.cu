@@ -621,7 +621,7 @@ rms_rows_kernel(const T *__restrict__ in, int ld, const float *__restrict__ w, f
 
 int launch_rms_rows(int dtype, const void *in, int ld, const float *w, float eps, void *out, int tokens, int cols, cudaStream_t st) {
     if (tokens == 0) return B200_OK;
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(rms_rows_kernel<T>, dim3((tokens + 3) / 4), dim3(128), 0, st, false, (const T *)in, ld, w, eps, (T *)out, tokens, cols); });
+    B200_DISPATCH_DTYPE(dtype, { launch_plain(rms_rows_kernel<T>, dim3((tokens + 3) / 4), dim3(128), 0, st, (const T *)in, ld, w, eps, (T *)out, tokens, cols); });
     return cuda_status("rms_rows launch");
 }
 
@@ -632,7 +632,7 @@ int launch_latent_prep(int dtype, const void *proj, int ld, int q_col, int kv_co
     if (tokens == 0) return B200_OK;
     const size_t smem = (size_t)std::max(rot_dims, 2) * sizeof(float);
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(latent_prep_kernel<T>, dim3(tokens), dim3(128), smem, st, false, (const T *)proj, ld, q_col, kv_col, (T *)qn, (T *)qr, (T *)pool, kv_norm, eps, tok_seq,
+        launch_plain(latent_prep_kernel<T>, dim3(tokens), dim3(128), smem, st, (const T *)proj, ld, q_col, kv_col, (T *)qn, (T *)qr, (T *)pool, kv_norm, eps, tok_seq,
                                                         tok_pos, block_table, mpps, t_pad, heads, dim, rot_dim, kv_rank, rot_dims, rot_base,
                                                         (const T *)kv_proj, kv_ld, rot);
     });
@@ -655,7 +655,7 @@ int launch_latent_attention(int dtype, const void *ql, const void *qr, const voi
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(latent_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(latent_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, false, (const T *)ql, (const T *)qr, (const T *)pool, sink, (T *)ol, tok_seq,
+        launch_plain(latent_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, (const T *)ql, (const T *)qr, (const T *)pool, sink, (T *)ol, tok_seq,
                                                                            tok_pos, block_table, mpps, t_pad, heads, kv_rank, rot_dim, scale,
                                                                            window, max_keys, (int)part, tok_list);
     });
@@ -682,11 +682,11 @@ static int launch_latent_mma_t(const void *ql, const void *qr, const void *pool,
     const int ld = (kv_rank + rot_dim + 63) / 64 * 64;
     const size_t smem = (size_t)3 * kLatTileQ * ld * sizeof(T);
     cudaFuncSetAttribute(latent_attn_mma_kernel<T, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(latent_attn_mma_kernel<T, NV>, dim3(grid), dim3(128), smem, st, false, (const T *)ql, (const T *)qr, (const T *)pool, sink, (T *)ol, (const int4 *)tiles,
+    launch_plain(latent_attn_mma_kernel<T, NV>, dim3(grid), dim3(128), smem, st, (const T *)ql, (const T *)qr, (const T *)pool, sink, (T *)ol, (const int4 *)tiles,
                                                            block_table, mpps, t_pad, heads, kv_rank, rot_dim, ld, scale, window, by_head, splits,
                                                            splits > 1 ? part : nullptr);
     if (splits > 1)
-        launch_pdl(latent_combine_kernel<T>, dim3(grid.x, heads), dim3(128), 0, st, false, part, (const int4 *)tiles, (T *)ol, t_pad, heads, kv_rank, splits);
+        launch_plain(latent_combine_kernel<T>, dim3(grid.x, heads), dim3(128), 0, st, part, (const int4 *)tiles, (T *)ol, t_pad, heads, kv_rank, splits);
     return cuda_status("latent_attention (tensor core) launch");
 }
 
@@ -735,7 +735,7 @@ int launch_latent_gate(int dtype, const void *ov, const void *gate_in, int gate_
                        cudaStream_t st, int head_gate) {
     if (tokens == 0) return B200_OK;
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(latent_gate_kernel<T>, dim3(tokens), dim3(256), 0, st, false, (const T *)ov, (const T *)gate_in, gate_ld, (T *)out, t_pad, heads, vdim, head_gate);
+        launch_plain(latent_gate_kernel<T>, dim3(tokens), dim3(256), 0, st, (const T *)ov, (const T *)gate_in, gate_ld, (T *)out, t_pad, heads, vdim, head_gate);
     });
     return cuda_status("latent_gate launch");
 }

@@ -592,7 +592,7 @@ static int launch_scored_mma_t(const void *q, const void *k_pool, const void *v_
     const size_t smem = (size_t)(kTileQS + 2 * kPageS) * DK * sizeof(T) + (size_t)2 * kPageS * DV * sizeof(T) + (size_t)pen_len * sizeof(float);
     auto kern = sigmoid ? scored_attn_mma_kernel<T, DK, DV, 1> : scored_attn_mma_kernel<T, DK, DV, 0>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(kern, dim3(n_tiles, heads), dim3(128), smem, st, false, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, r1, r2, (const T *)gate_in, gate_ld,
+    launch_plain(kern, dim3(n_tiles, heads), dim3(128), smem, st, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, r1, r2, (const T *)gate_in, gate_ld,
                                                   (T *)out, out_ld, out_scale, (const int4 *)tiles, block_table, mpps, heads, kv_heads, scale, window,
                                                   pen_len, opt);
     return cuda_status("scored_attention (tensor core) launch");
@@ -640,12 +640,12 @@ int launch_scored_prep(int dtype, const void *proj, int ld, int col0, const floa
         const int per = dim / V;
         if (rot_dims == 0 && !opt.v_norm && dim % V == 0 && per <= 32 && (per & (per - 1)) == 0 && vdim % V == 0 && ld % V == 0 && col0 % V == 0 &&
             (q_norm == nullptr) == (k_norm == nullptr) && all_aligned16({proj, b_in, q_out, k_pool, v_pool, q_norm, k_norm, share.v_keep, share.v_mix})) {
-            launch_pdl(scored_prep_vec_kernel<T>, dim3(tokens), dim3(128), 0, st, false, (const T *)proj, ld, col0, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
+            launch_plain(scored_prep_vec_kernel<T>, dim3(tokens), dim3(128), 0, st, (const T *)proj, ld, col0, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps,
                                                               tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim, vdim, (T *)share.v_keep,
                                                               (const T *)share.v_mix, share.lambda, b_in);
             return cuda_status("scored_prep (vector) launch");
         }
-        launch_pdl(scored_prep_kernel<T>, dim3(tokens), dim3(256), (size_t)std::max(rot_dims, 2) * sizeof(float), st, false, (const T *)proj, ld, col0, b_in, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps, tok_seq, tok_pos, block_table, mpps, heads,
+        launch_plain(scored_prep_kernel<T>, dim3(tokens), dim3(256), (size_t)std::max(rot_dims, 2) * sizeof(float), st, (const T *)proj, ld, col0, b_in, (T *)q_out, (T *)k_pool, (T *)v_pool, q_norm, k_norm, eps, tok_seq, tok_pos, block_table, mpps, heads,
             kv_heads, dim, vdim, rot_dims, rot_base, opt, (T *)share.v_keep, (const T *)share.v_mix, share.lambda);
     });
     return cuda_status("scored_prep launch");
@@ -666,7 +666,7 @@ int launch_scored_attention(int dtype, const void *q, const void *k_pool, const 
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(scored_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(scored_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, false, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, dist_r1, dist_r2, (const T *)gate_in, gate_ld, (T *)out, out_ld, out_scale,
+        launch_plain(scored_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, dist_r1, dist_r2, (const T *)gate_in, gate_ld, (T *)out, out_ld, out_scale,
             tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim, vdim, scale, window, sigmoid, max_keys, (int)part, tok_list, opt);
     });
     return cuda_status("scored_attention launch");

@@ -531,8 +531,8 @@ int launch_chunks_t(const ChunkSource &src, ChunkMap map, float *scratch, size_t
     cudaFuncSetAttribute(sk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem);
     for (map.first = 0; map.first < chunks; map.first += map.count) {
         const int n = std::min(map.count, chunks - map.first);
-        launch_pdl(fk, dim3(n, map.heads, n_seqs), dim3(256), smem_f, st, false, src, map, scratch);
-        launch_pdl(sk, dim3(map.vdim / kCols, map.heads, n_seqs), dim3(DK * 2), scan_smem, st, false, src, map, scratch, state, o);
+        launch_plain(fk, dim3(n, map.heads, n_seqs), dim3(256), smem_f, st, src, map, scratch);
+        launch_plain(sk, dim3(map.vdim / kCols, map.heads, n_seqs), dim3(DK * 2), scan_smem, st, src, map, scratch, state, o);
     }
     return cuda_status("chunk recurrence launch");
 }

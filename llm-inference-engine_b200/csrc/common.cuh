@@ -143,6 +143,11 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl, Args... args) {
     return launch_pdl_cluster(kernel, grid, block, smem, stream, pdl, 1u, args...);
 }
+// in plain stream order: starts when everything in front is done
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_plain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_pdl_cluster(kernel, grid, block, smem, stream, false, 1u, args...);
+}
 
 #ifdef __CUDACC__
 // ------------------------------------------------------------------ PDL (device)

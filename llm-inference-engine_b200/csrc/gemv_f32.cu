@@ -17,8 +17,8 @@ int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStrea
     const bool b16 = dtype == B200_BF16 || dtype == B200_F16;
     // 16-bit activations, no prologue: 2..16 tokens, and one token of quantised weights, past which the weights stream with the activations in registers
     // (gemv_rs.cuh).  One dense token keeps the SIMT kernel and its fused norm: its weights alone fill the memory pipe, and the norm launch would come on
-    // top.  One quantised token, 4 layers, norm kernel + gemv_rs against the kernel with the fused norm that was here: 7B size FP8 266 / INT4 276 us against
-    // 262 / 280, 70B-shaped shard 227 / 236 against 250 / 271, 2048-wide 149 / 148 against 162 / 171.
+    // top.  One quantised token, 4 layers, norm kernel + gemv_rs against the kernel with the fused norm that was here (ctx 1024): 7B size FP8 238 / INT4 249 us
+    // against 245 / 268, 70B-shaped shard 204 / 222 against 230 / 255, 2048-wide 130 / 131 against 142 / 159.
     if (b16 && (a.M >= 2 || fmt != WF_DENSE) && a.M <= 16) {
         const int rc = dtype == B200_BF16 ? launch_gemv_rs_bf16(a, fmt, swiglu, st) : launch_gemv_rs_f16(a, fmt, swiglu, st);
         if (rc != B200_ERR_UNSUPPORTED) return rc;

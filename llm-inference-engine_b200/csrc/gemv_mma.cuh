@@ -1,3 +1,4 @@
+// (Today gemv_rs.cuh takes these calls; this kernel serves what its ring leaves out: rows of more than 4096 k with vocabulary-sized outputs.)
 // gemv_mma.cuh -- the decode-shaped linear for 2..16 tokens on the tensor cores: y[M,N] = x[M,K] * W^T, W packed [N,K], dense 16-bit,
 // FP8-e4m3 (W8A16) or INT4-g128 (W4A16) weights.  Reference: launchLinearGemm (src/kernels/linear.cu:10-87) at the decode shapes of
 // src/layers/self_attention.cpp:79-86,131-138 and src/layers/ffn.cpp:105-139, with the quantisation the README plans (README.md:36-39).

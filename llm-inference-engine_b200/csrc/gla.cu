@@ -424,7 +424,7 @@ static void launch_gla_reg(const void *proj, int ld, const float *decay, float *
                            const int *seq_slot, dim3 grid, int heads, int dim, int vdim, int min_tokens, int max_tokens, cudaStream_t st) {
     const size_t smem = 2 * ((size_t)TB * 32 * RR * 4 + (size_t)TB * kGlaCols) * sizeof(float);
     if (smem > 48 * 1024) cudaFuncSetAttribute(gla_recurrent_reg_kernel<T, RR, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(gla_recurrent_reg_kernel<T, RR, TB>, dim3(grid), dim3(256), smem, st, false, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim, min_tokens, max_tokens);
+    launch_plain(gla_recurrent_reg_kernel<T, RR, TB>, dim3(grid), dim3(256), smem, st, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim, min_tokens, max_tokens);
 }
 
 template <typename T>
@@ -501,15 +501,15 @@ int launch_gla_decay(int dtype, const void *proj, int ld, int col0, const void *
         const int tiles = (tokens + 15) / 16, groups = (channels + 63) / 64;
         const int steps = std::max(1, std::min(groups, groups * tiles / (4 * sm_count())));  // about four CTAs per SM
         const dim3 grid(tiles, (groups + steps - 1) / steps);
-        if (dtype == B200_BF16) launch_pdl(gla_decay_mma_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, false, (const __nv_bfloat16 *)proj, ld, col0, (const __nv_bfloat16 *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels, steps);
-        else launch_pdl(gla_decay_mma_kernel<__half>, dim3(grid), dim3(256), 0, st, false, (const __half *)proj, ld, col0, (const __half *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels, steps);
+        if (dtype == B200_BF16) launch_plain(gla_decay_mma_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, (const __nv_bfloat16 *)proj, ld, col0, (const __nv_bfloat16 *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels, steps);
+        else launch_plain(gla_decay_mma_kernel<__half>, dim3(grid), dim3(256), 0, st, (const __half *)proj, ld, col0, (const __half *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels, steps);
         return cuda_status("gla_decay launch");
     }
     B200_DISPATCH_DTYPE(dtype, {
         // few token blocks (decoding): the channels are spread over CTAs as well
         const int nb = (tokens + kDecayTokens - 1) / kDecayTokens;
         const int cb = nb >= 64 ? 1 : (channels + 255) / 256;
-        launch_pdl(gla_decay_kernel<T>, dim3(nb, cb), dim3(256), (size_t)kDecayTokens * rank * sizeof(float), st, false, (const T *)proj, ld, col0, (const T *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels);
+        launch_plain(gla_decay_kernel<T>, dim3(nb, cb), dim3(256), (size_t)kDecayTokens * rank * sizeof(float), st, (const T *)proj, ld, col0, (const T *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels);
     });
     return cuda_status("gla_decay launch");
 }
@@ -525,7 +525,7 @@ int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay
         const dim3 grid_step((vdim + kStepCols - 1) / kStepCols, heads, n_seqs);
         B200_DISPATCH_DTYPE(dtype, {
             if (smem_step > 48 * 1024) cudaFuncSetAttribute(gla_step_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_step);
-            launch_pdl(gla_step_kernel<T>, dim3(grid_step), dim3(256), smem_step, st, false, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim);
+            launch_plain(gla_step_kernel<T>, dim3(grid_step), dim3(256), smem_step, st, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim);
         });
         if (!(kinds & kGlaManyTokens)) return cuda_status("gla_step launch");
     }
@@ -547,7 +547,7 @@ int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay
     }
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(gla_recurrent_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(gla_recurrent_kernel<T>, dim3(grid), dim3(kGlaThreads), smem, st, false, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim,
+        launch_plain(gla_recurrent_kernel<T>, dim3(grid), dim3(kGlaThreads), smem, st, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim,
                                                                   vdim, min_tokens, max_tokens);
     });
     return cuda_status("gla_recurrent launch");
@@ -560,13 +560,13 @@ int launch_gla_output(int dtype, const float *o, const float *w, float eps, cons
         constexpr int V = Elem<T>::kVec;
         // whole pieces, at most a warp of them per row: eight rows per CTA (one per CTA: 21 us for 32768 rows of 256, half of it CTAs coming and going)
         if (vdim % V == 0 && vdim / V <= 32 && gate_ld % V == 0 && all_aligned16({o, gate_in, out})) {
-            launch_pdl(gla_output_kernel<T>, dim3((unsigned)(((size_t)tokens * heads + 7) / 8)), dim3(256), 0, st, false, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim,
+            launch_plain(gla_output_kernel<T>, dim3((unsigned)(((size_t)tokens * heads + 7) / 8)), dim3(256), 0, st, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim,
                        tokens, 1);
             return cuda_status("gla_output launch");
         }
         // rows that go in 16-byte pieces need one thread per piece; others keep 128 threads striding the row
         const int threads = (vdim % V == 0 && vdim / V <= 128) ? std::max(32, (vdim / V + 31) / 32 * 32) : 128;
-        launch_pdl(gla_output_kernel<T>, dim3(tokens, heads), dim3(threads), 0, st, false, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim, tokens, 0);
+        launch_plain(gla_output_kernel<T>, dim3(tokens, heads), dim3(threads), 0, st, o, w, eps, (const T *)gate_in, gate_ld, (T *)out, heads, vdim, tokens, 0);
     });
     return cuda_status("gla_output launch");
 }

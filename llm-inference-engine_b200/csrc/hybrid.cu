@@ -471,7 +471,7 @@ static void launch_proj_f32_t(const void *x, int ldx, const void *w, const float
     int cols = (N * mt + 4 * 148 - 1) / (4 * 148);
     cols = cols < 8 ? 8 : (cols + 7) / 8 * 8;
     if (smem > 48 * 1024) cudaFuncSetAttribute(proj_f32_kernel<TX, TW, PM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(proj_f32_kernel<TX, TW, PM>, dim3((N + cols - 1) / cols, mt), dim3(256), smem, st, false, (const TX *)x, ldx, (const TW *)w, bias, y, ldy, M, N, K, cols);
+    launch_plain(proj_f32_kernel<TX, TW, PM>, dim3((N + cols - 1) / cols, mt), dim3(256), smem, st, (const TX *)x, ldx, (const TW *)w, bias, y, ldy, M, N, K, cols);
 }
 
 int launch_proj_f32(int x_dtype, const void *x, int ldx, int w_dtype, const void *w, const float *bias, float *y, int ldy, int M, int N,
@@ -481,19 +481,19 @@ int launch_proj_f32(int x_dtype, const void *x, int ldx, int w_dtype, const void
         const int grid = (M * N + 7) / 8;
         B200_DISPATCH_DTYPE(w_dtype, {
             const bool vec = K % 8 == 0 && ldx % 8 == 0 && all_aligned16({x, w});
-            if (x_dtype == B200_F32) launch_pdl(proj_f32_small_kernel<float, T>, dim3(grid), dim3(256), 0, st, false, (const float *)x, ldx, (const T *)w, bias, y, ldy, M, N, K, vec);
-            else launch_pdl(proj_f32_small_kernel<T, T>, dim3(grid), dim3(256), 0, st, false, (const T *)x, ldx, (const T *)w, bias, y, ldy, M, N, K, vec);
+            if (x_dtype == B200_F32) launch_plain(proj_f32_small_kernel<float, T>, dim3(grid), dim3(256), 0, st, (const float *)x, ldx, (const T *)w, bias, y, ldy, M, N, K, vec);
+            else launch_plain(proj_f32_small_kernel<T, T>, dim3(grid), dim3(256), 0, st, (const T *)x, ldx, (const T *)w, bias, y, ldy, M, N, K, vec);
         });
         return cuda_status("proj_f32 (small) launch");
     }
     if (M <= 16 && x_dtype == w_dtype && w_dtype != B200_F32 && K % 8 == 0 && ldx % 8 == 0 && K >= 512 && aligned16(x) && aligned16(w)) {
         const int grid = (N + 7) / 8;
         if (w_dtype == B200_BF16) {
-            if (M <= 8) launch_pdl(proj_f32_rows_kernel<__nv_bfloat16, 8>, dim3(grid), dim3(256), 0, st, false, (const __nv_bfloat16 *)x, ldx, (const __nv_bfloat16 *)w, bias, y, ldy, M, N, K);
-            else launch_pdl(proj_f32_rows_kernel<__nv_bfloat16, 16>, dim3(grid), dim3(256), 0, st, false, (const __nv_bfloat16 *)x, ldx, (const __nv_bfloat16 *)w, bias, y, ldy, M, N, K);
+            if (M <= 8) launch_plain(proj_f32_rows_kernel<__nv_bfloat16, 8>, dim3(grid), dim3(256), 0, st, (const __nv_bfloat16 *)x, ldx, (const __nv_bfloat16 *)w, bias, y, ldy, M, N, K);
+            else launch_plain(proj_f32_rows_kernel<__nv_bfloat16, 16>, dim3(grid), dim3(256), 0, st, (const __nv_bfloat16 *)x, ldx, (const __nv_bfloat16 *)w, bias, y, ldy, M, N, K);
         } else {
-            if (M <= 8) launch_pdl(proj_f32_rows_kernel<__half, 8>, dim3(grid), dim3(256), 0, st, false, (const __half *)x, ldx, (const __half *)w, bias, y, ldy, M, N, K);
-            else launch_pdl(proj_f32_rows_kernel<__half, 16>, dim3(grid), dim3(256), 0, st, false, (const __half *)x, ldx, (const __half *)w, bias, y, ldy, M, N, K);
+            if (M <= 8) launch_plain(proj_f32_rows_kernel<__half, 8>, dim3(grid), dim3(256), 0, st, (const __half *)x, ldx, (const __half *)w, bias, y, ldy, M, N, K);
+            else launch_plain(proj_f32_rows_kernel<__half, 16>, dim3(grid), dim3(256), 0, st, (const __half *)x, ldx, (const __half *)w, bias, y, ldy, M, N, K);
         }
         return cuda_status("proj_f32 (rows) launch");
     }
@@ -1439,7 +1439,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     auto ln_residual = [&](const void *y, const float *y32, const float *bias, const float *ln, void *h_out, int h_ld, float *trace) -> int {
         B200_DISPATCH_DTYPE(dt, {
             const bool vec = width % 4 == 0 && h_ld % 4 == 0 && all_aligned16({m->x, y, y32, bias, ln, h_out, trace});
-            launch_pdl((vec ? ln_residual_kernel<T, 4> : ln_residual_kernel<T, 1>), dim3(NT), dim3(256), (size_t)width * sizeof(float), st, false, m->x, (const T *)y, y32, bias, y32 ? 1 : 0, ln, c.norm_eps, width, (T *)h_out, h_ld, trace);
+            launch_plain((vec ? ln_residual_kernel<T, 4> : ln_residual_kernel<T, 1>), dim3(NT), dim3(256), (size_t)width * sizeof(float), st, m->x, (const T *)y, y32, bias, y32 ? 1 : 0, ln, c.norm_eps, width, (T *)h_out, h_ld, trace);
         });
         return cuda_status("ln_residual launch");
     };
@@ -1452,7 +1452,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     auto embed = [&](void *h2, int h2_ld) -> int {
         const bool vec = width % 8 == 0 && h2_ld % 8 == 0 && all_aligned16({m->embedding, m->x, h2});
         B200_DISPATCH_DTYPE(dt, {
-            launch_pdl(embed_rows_kernel<T>, dim3(NT), dim3(256), 0, st, false, d_ids, (const T *)m->embedding, m->x, (T *)h2, h2_ld, width, c.vocab, c.embed_scale != 0.0f ? c.embed_scale : 1.0f, vec);
+            launch_plain(embed_rows_kernel<T>, dim3(NT), dim3(256), 0, st, d_ids, (const T *)m->embedding, m->x, (T *)h2, h2_ld, width, c.vocab, c.embed_scale != 0.0f ? c.embed_scale : 1.0f, vec);
         });
         return cuda_status("embed_rows launch");
     };
@@ -1570,7 +1570,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         // four columns per access when every row starts on a 16-byte boundary (the scratch buffers do; norm vectors and the trace are the caller's)
         const bool vec = width % 4 == 0 && ((reinterpret_cast<size_t>(na) | reinterpret_cast<size_t>(nb) | reinterpret_cast<size_t>(ln_next) |
                                               reinterpret_cast<size_t>(trace)) & 15) == 0;
-#define B200_STREAMS(SC, V) launch_pdl(stream_residual_kernel<T, SC, V>, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, false, \
+#define B200_STREAMS(SC, V) launch_plain(stream_residual_kernel<T, SC, V>, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, \
     m->xs, n_streams, x_init, (const T *)ya, (const T *)yb, na, nb, sa, sb, hc, hc_next, ln_next, c.norm_eps, width, ln_next ? (T *)m->h : nullptr, sum_out, trace)
 #define B200_STREAMS_V(SC) do { if (vec) B200_STREAMS(SC, true); else B200_STREAMS(SC, false); } while (0)
         B200_DISPATCH_DTYPE(dt, {
@@ -1639,8 +1639,8 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                 const bool vec = lp.n_in % V == 0 && col % V == 0 && l.expert_ff % V == 0 && n_cat % V == 0 && ocol % V == 0;
                 const int per = vec ? V : 1;
                 const dim3 grid((l.expert_ff / per + 255) / 256, NT);
-                if (vec) launch_pdl(gated_act_strided_kernel<T, true>, dim3(grid), dim3(256), 0, st, false, (const T *)m->proj, lp.n_in, col, col + l.expert_ff, (T *)m->cat + ocol, n_cat, l.expert_ff, l.act);
-                else launch_pdl(gated_act_strided_kernel<T, false>, dim3(grid), dim3(256), 0, st, false, (const T *)m->proj, lp.n_in, col, col + l.expert_ff, (T *)m->cat + ocol, n_cat, l.expert_ff, l.act);
+                if (vec) launch_plain(gated_act_strided_kernel<T, true>, dim3(grid), dim3(256), 0, st, (const T *)m->proj, lp.n_in, col, col + l.expert_ff, (T *)m->cat + ocol, n_cat, l.expert_ff, l.act);
+                else launch_plain(gated_act_strided_kernel<T, false>, dim3(grid), dim3(256), 0, st, (const T *)m->proj, lp.n_in, col, col + l.expert_ff, (T *)m->cat + ocol, n_cat, l.expert_ff, l.act);
             });
             RUN(cuda_status("gated_act_strided launch"));
         }
@@ -1685,7 +1685,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     auto postnorm = [&](const void *y_dense, const void *y_rows, const int *pair_row, int top, const void *y_shared, const float *gate,
                         const float *g, float *trace) -> int {
         B200_DISPATCH_DTYPE(dt, {
-            launch_pdl(postnorm_residual_kernel<T>, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, false, m->x, (const T *)y_dense, (const T *)y_rows, pair_row, top,
+            launch_plain(postnorm_residual_kernel<T>, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, m->x, (const T *)y_dense, (const T *)y_rows, pair_row, top,
                                                                                       (const T *)y_shared, gate, g, c.norm_eps, width, trace,
                                                                                       f32 ? nullptr : (T *)m->h);
         });
@@ -1700,7 +1700,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             const bool vec = width % Elem<T>::kVec == 0 && ((reinterpret_cast<size_t>(trace) | reinterpret_cast<size_t>(post) | reinterpret_cast<size_t>(ls) |
                                                               reinterpret_cast<size_t>(pre) | reinterpret_cast<size_t>(y_bias)) & 15) == 0;
             auto kern = vec ? sublayer_residual_kernel<T, true> : sublayer_residual_kernel<T, false>;
-            launch_pdl(kern, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, false, m->x, (const T *)y_dense, y_bias, (const T *)y_rows, pair_row, pair_weight, top,
+            launch_plain(kern, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, m->x, (const T *)y_dense, y_bias, (const T *)y_rows, pair_row, pair_weight, top,
                                                                 (const T *)y_shared, gate, (const T *)m->h, norm, post, ls, c.norm_eps, pre, width, trace,
                                                                 (pre || !f32) ? (T *)m->h : nullptr, has_y ? 1 : 0,
                                                                 c.branch_scale != 0.0f ? c.branch_scale : 1.0f);
@@ -1914,12 +1914,12 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             const bool ln = c.final_norm == B200_NORM_LN_PARALLEL || c.final_norm == B200_NORM_LN_PRE || c.final_norm == B200_NORM_LN_POST;
             const bool vec = width % 4 == 0 && width <= 4096 && c.final_norm != B200_NORM_DYT_PRE_POST && all_aligned16({m->x, m->final_norm, m->xn, m->h});
             if (vec)
-                launch_pdl(ln ? final_rows_kernel<T, true> : final_rows_kernel<T, false>, dim3(W), dim3(256), 0, st, false, m->x, d_want, m->final_norm,
+                launch_plain(ln ? final_rows_kernel<T, true> : final_rows_kernel<T, false>, dim3(W), dim3(256), 0, st, m->x, d_want, m->final_norm,
                            c.final_norm != B200_NORM_LN_POST ? 1 : 0, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
             else if (ln)
-                launch_pdl(final_ln_rows_kernel<T>, dim3(W), dim3(256), 0, st, false, m->x, d_want, m->final_norm, c.final_norm != B200_NORM_LN_POST, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
-            else if (c.final_norm == B200_NORM_DYT_PRE_POST) launch_pdl(final_dyt_rows_kernel<T>, dim3(W), dim3(256), 0, st, false, m->x, d_want, m->final_norm, m->xn, f32 ? nullptr : (T *)m->h, width);
-            else launch_pdl(final_norm_rows_kernel<T>, dim3(W), dim3(256), 0, st, false, m->x, d_want, m->final_norm, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
+                launch_plain(final_ln_rows_kernel<T>, dim3(W), dim3(256), 0, st, m->x, d_want, m->final_norm, c.final_norm != B200_NORM_LN_POST, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
+            else if (c.final_norm == B200_NORM_DYT_PRE_POST) launch_plain(final_dyt_rows_kernel<T>, dim3(W), dim3(256), 0, st, m->x, d_want, m->final_norm, m->xn, f32 ? nullptr : (T *)m->h, width);
+            else launch_plain(final_norm_rows_kernel<T>, dim3(W), dim3(256), 0, st, m->x, d_want, m->final_norm, c.norm_eps, m->xn, f32 ? nullptr : (T *)m->h, width);
         });
         rc = W <= 16 ? launch_rows_f32out(dt, m->h, m->lm_head, logits, W, c.vocab, width, st) : B200_ERR_UNSUPPORTED;
         if (rc == B200_ERR_UNSUPPORTED) rc = launch_dense_f32out(dt, m->h, m->lm_head, logits, W, c.vocab, width, st);
@@ -1928,7 +1928,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         const float lscale = c.logit_scale != 0.0f ? c.logit_scale : 1.0f;
         if (c.logit_softcap > 0.0f || lscale != 1.0f) {
             const size_t n = (size_t)W * c.vocab;
-            launch_pdl(softcap_kernel, dim3((unsigned)std::min<size_t>((n + 255) / 256, 148 * 8)), dim3(256), 0, st, false, logits, n, lscale, c.logit_softcap);
+            launch_plain(softcap_kernel, dim3((unsigned)std::min<size_t>((n + 255) / 256, 148 * 8)), dim3(256), 0, st, logits, n, lscale, c.logit_softcap);
         }
     }
 #undef RUN

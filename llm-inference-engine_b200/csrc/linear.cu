@@ -1,9 +1,9 @@
 // linear.cu -- b200_linear / b200_batched_gemm and the weight packing helpers.
 //
 // Dispatch of y[M,N] = x[M,K] * W (reference src/kernels/linear.cu:10-158):
-//   M <= 4, W packed [N,K] (dense / FP8 / INT4)  -> gemv_nk_kernel  (gemv.cuh; TMA-bulk weight streaming)
+//   M <= 16 (fp32: 4), W packed [N,K] (dense / FP8 / INT4) -> launch_gemv_nk (gemv_f32.cu: gemv_rs.cuh, gemv_mma.cuh, gemv.cuh; TMA-bulk weight streaming)
 //   M <= 4, W dense  [K,N] (the reference's own memory order) -> gemv_kn_kernel (this file)
-//   M  > 4, 16-bit activations, W packed [N,K]   -> tcgen05 / TMEM tensor-core GEMM (gemm_tc.cu)
+//   M > 16, 16-bit activations, dense W packed [N,K] -> tcgen05 / TMEM tensor-core GEMM (gemm_tc.cu)
 //   everything else                              -> gemm_simt_kernel (tiled fp32-accumulate fallback, this file)
 #include <stdlib.h>
 
@@ -353,7 +353,7 @@ int b200_linear(const void *x, const void *w, const void *scales, const void *ze
         int done = 0, rc = B200_OK;
         const bool b16 = dtype != B200_F32;
         // weight-streaming GEMV in passes of `step` tokens (one pass = one read of the weights): 16-bit activations take 16 tokens per pass on
-        // the tensor-core GEMV (gemv_mma.cuh: dense, FP8, INT4), fp32 4 on the SIMT GEMV
+        // the tensor-core GEMVs (gemv_rs.cuh, gemv_mma.cuh: dense, FP8, INT4), fp32 4 on the SIMT GEMV
         auto gemv_passes = [&](int step) -> int {
             for (int m0 = 0; m0 < M; m0 += step) {
                 GemvArgs a = {};
@@ -379,7 +379,7 @@ int b200_linear(const void *x, const void *w, const void *scales, const void *ze
             else if (rc != B200_ERR_UNSUPPORTED) return rc;
         }
         // quantised weights up to 128 tokens: passes of 16 (4 passes over packed INT4 move what one pass over bf16 moves); smaller steps
-        // for the shapes only the older kernels take.  (Prefill-sized quantised linears inside the engine: dequantise + tcgen05 GEMM,
+        // for outputs whose sums fill the SM at 16 tokens.  (Prefill-sized quantised linears inside the engine: dequantise + tcgen05 GEMM,
         // decoder.cu prefill_linear.)
         for (int step = b16 ? 16 : 4; !done && step >= 4 && M <= 128; step = step == 16 ? 8 : step - 4) {
             if (M > (step == 16 ? 8 : 4) * step) continue;

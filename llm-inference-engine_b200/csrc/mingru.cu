@@ -206,12 +206,12 @@ int launch_mingru(int dtype, const void *proj, int ld, const float *bias, float 
             auto chunk = vec ? mingru_chunk_kernel<T, 4> : mingru_chunk_kernel<T, 1>;
             auto apply = vec ? mingru_apply_kernel<T, 4> : mingru_apply_kernel<T, 1>;
             const dim3 grid((cols + 32 * n - 1) / (32 * n), n_chunks);
-            launch_pdl(chunk, dim3(grid), dim3(32 * kSubs), 0, st, false, (const T *)proj, ld, bias, state, maps, ch, seq_pos0, seq_slot, cols);
-            launch_pdl(apply, dim3(grid), dim3(32 * kSubs), 0, st, false, (const T *)proj, ld, bias, state, maps, (T *)out, ch, seq_start, seq_slot, cols);
+            launch_plain(chunk, dim3(grid), dim3(32 * kSubs), 0, st, (const T *)proj, ld, bias, state, maps, ch, seq_pos0, seq_slot, cols);
+            launch_plain(apply, dim3(grid), dim3(32 * kSubs), 0, st, (const T *)proj, ld, bias, state, maps, (T *)out, ch, seq_start, seq_slot, cols);
         }
         if (n_short > 0) {
             auto step = vec ? mingru_step_kernel<T, 4> : mingru_step_kernel<T, 1>;
-            launch_pdl(step, dim3(blocks, n_seqs), dim3(threads), 0, st, false, (const T *)proj, ld, bias, state, (T *)out, seq_start, seq_pos0, seq_slot, cols);
+            launch_plain(step, dim3(blocks, n_seqs), dim3(threads), 0, st, (const T *)proj, ld, bias, state, (T *)out, seq_start, seq_pos0, seq_slot, cols);
         }
     });
     return cuda_status("mingru launch");

@@ -527,7 +527,7 @@ moe_grouped_gemm_mma_kernel(const T *__restrict__ a, const T *__restrict__ w, TC
 // experts, 28 touched: 40 us up, 30 us down, for 59 MB each).  Here a warp owns a slice of up to 256 k and holds the tile's rows of it as mma.sync A
 // fragments; it reads its 8 weight rows of a unit straight into registers, 16 bytes per lane and 32-k block (k permuted inside a block alike for both
 // operands: a lane's 8 consecutive k are its fragments of two k-steps), the next unit's pieces in flight while it multiplies this one's.  KS warps share a
-// unit's k and meet in shared memory, NG units of a CTA run side by side (KS * NG >= 8 warps).
+// unit's k and meet in shared memory, NG units of a CTA run side by side (5 to 16 warps).
 // grid (unit groups, tiles); a CTA runs `steps` groups of NG units of 8 rows.  NT 1: at most 8 live rows, 2: at most 16.  A tile's rows start at its
 // number times tile_rows; rows >= M are neither read nor stored.  tile_expert and n_tiles NULL: one weight, every tile of the grid.
 // Measured (2048 x 512 experts, 16 tokens x 4 of 32, 59 MB): up and down 40 and 30 -> 19 us each.
@@ -595,18 +595,18 @@ int launch_dense_f32out(int dtype, const void *x, const void *w, float *y, int M
         const int KS = (K / 32 + 7) / 8, NG = KS >= 8 ? 1 : 8 / KS, steps = ((N + 7) / 8 + NG - 1) / NG;
         const size_t smem = (size_t)2 * NG * KS * 128 * sizeof(float);
         const dim3 few(1, (M + 15) / 16);
-        if (dtype == B200_BF16) launch_pdl(moe_few_rows_kernel<__nv_bfloat16, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, false, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
-        else launch_pdl(moe_few_rows_kernel<__half, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, false, (const __half *)x, (const __half *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
+        if (dtype == B200_BF16) launch_plain(moe_few_rows_kernel<__nv_bfloat16, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
+        else launch_plain(moe_few_rows_kernel<__half, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, (const __half *)x, (const __half *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
         return cuda_status("dense_f32out (few columns) launch");
     }
     const dim3 grid((N + kMN - 1) / kMN, (M + kMoeTileM - 1) / kMoeTileM);
     const size_t smem = (size_t)kMStages * (kMoeTileM + kMN) * kMK * 2;
     if (dtype == B200_BF16) {
         cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__nv_bfloat16, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(moe_grouped_gemm_mma_kernel<__nv_bfloat16, float>, dim3(grid), dim3(128), smem, st, false, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, M, N, K, -1);
+        launch_plain(moe_grouped_gemm_mma_kernel<__nv_bfloat16, float>, dim3(grid), dim3(128), smem, st, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, M, N, K, -1);
     } else {
         cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__half, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(moe_grouped_gemm_mma_kernel<__half, float>, dim3(grid), dim3(128), smem, st, false, (const __half *)x, (const __half *)w, y, nullptr, nullptr, M, N, K, -1);
+        launch_plain(moe_grouped_gemm_mma_kernel<__half, float>, dim3(grid), dim3(128), smem, st, (const __half *)x, (const __half *)w, y, nullptr, nullptr, M, N, K, -1);
     }
     return cuda_status("dense_f32out launch");
 }
@@ -631,21 +631,21 @@ __global__ void activation_kernel(T *__restrict__ x, size_t n, int act, size_t n
 int launch_moe_route_sigmoid(const float *logits, int ld, int *sel_expert, float *sel_weight, float *shared_gate, int tokens,
                              int experts, int top, cudaStream_t st) {
     if (tokens == 0) return B200_OK;
-    launch_pdl(moe_route_sigmoid_kernel, dim3((tokens + 3) / 4), dim3(128), 0, st, false, logits, ld, sel_expert, sel_weight, shared_gate, tokens, experts, top);
+    launch_plain(moe_route_sigmoid_kernel, dim3((tokens + 3) / 4), dim3(128), 0, st, logits, ld, sel_expert, sel_weight, shared_gate, tokens, experts, top);
     return cuda_status("moe_route launch");
 }
 
 int launch_moe_route_softmax(const float *logits, int ld, const float *bias, int *sel_expert, float *sel_weight, int tokens, int outputs,
                              int top, cudaStream_t st, const float *logit_bias) {
     if (tokens == 0) return B200_OK;
-    launch_pdl(moe_route_softmax_kernel, dim3((tokens + 3) / 4), dim3(128), 0, st, false, logits, ld, bias, logit_bias, sel_expert, sel_weight, tokens, outputs, top);
+    launch_plain(moe_route_softmax_kernel, dim3((tokens + 3) / 4), dim3(128), 0, st, logits, ld, bias, logit_bias, sel_expert, sel_weight, tokens, outputs, top);
     return cuda_status("moe_route (softmax) launch");
 }
 
 int launch_moe_gather_rows(int dtype, const void *h, const int *row_token, void *xg, const int *n_tiles, int max_rows, int width, int tile,
                            cudaStream_t st, const float *row_weight) {
     if (max_rows == 0) return B200_OK;
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(moe_gather_rows_kernel<T>, dim3(max_rows), dim3(128), 0, st, false, (const T *)h, row_token, (T *)xg, n_tiles, width, tile, row_weight); });
+    B200_DISPATCH_DTYPE(dtype, { launch_plain(moe_gather_rows_kernel<T>, dim3(max_rows), dim3(128), 0, st, (const T *)h, row_token, (T *)xg, n_tiles, width, tile, row_weight); });
     return cuda_status("moe_gather_rows launch");
 }
 
@@ -654,7 +654,7 @@ int launch_gated_activation(int dtype, const void *in, void *out, int rows, int 
     if (rows == 0 || inner == 0) return B200_OK;
     const size_t n = (size_t)rows * inner / 4;
     const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 148 * 16));
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(gated_activation_kernel<T>, dim3(grid), dim3(256), 0, st, false, (const T *)in, (T *)out, rows, inner, act, n_tiles, tile, limit, slope); });
+    B200_DISPATCH_DTYPE(dtype, { launch_plain(gated_activation_kernel<T>, dim3(grid), dim3(256), 0, st, (const T *)in, (T *)out, rows, inner, act, n_tiles, tile, limit, slope); });
     return cuda_status("gated_activation launch");
 }
 
@@ -662,7 +662,7 @@ int launch_bias_activation(int dtype, void *x, const float *bias, size_t rows, i
     if (rows == 0 || cols == 0) return B200_OK;
     const size_t n = rows * cols / 4;
     const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 148 * 16));
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(bias_activation_kernel<T>, dim3(grid), dim3(256), 0, st, false, (T *)x, bias, rows, cols, act); });
+    B200_DISPATCH_DTYPE(dtype, { launch_plain(bias_activation_kernel<T>, dim3(grid), dim3(256), 0, st, (T *)x, bias, rows, cols, act); });
     return cuda_status("bias_activation launch");
 }
 
@@ -673,7 +673,7 @@ int launch_poly_norm(int dtype, void *x, const float *coef, float eps, int rows,
         const int per = vec ? Elem<T>::kVec : 1;
         const int threads = std::min(256, std::max(32, ((cols + per - 1) / per + 31) / 32 * 32));
         auto kern = vec ? poly_norm_kernel<T, true> : poly_norm_kernel<T, false>;
-        launch_pdl(kern, dim3(rows), dim3(threads), 0, st, false, (T *)x, coef, eps, cols);
+        launch_plain(kern, dim3(rows), dim3(threads), 0, st, (T *)x, coef, eps, cols);
     });
     return cuda_status("poly_norm launch");
 }
@@ -684,14 +684,14 @@ int launch_moe_plan(const int *sel_expert, const float *sel_weight, int *row_tok
     const int warps = std::max(1, std::min({32, std::max(8, (pairs + 31) / 32), (int)(40 * 1024 / sizeof(int) / std::max(experts, 1))}));
     const size_t smem = ((size_t)(warps + 2) * experts + 1) * sizeof(int);
     if (smem > 48 * 1024) cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(moe_plan_kernel, dim3(1), dim3(warps * 32), smem, st, false, sel_expert, sel_weight, row_token, row_weight, tile_expert, pair_row, n_tiles, pairs, experts, top, tile);
+    launch_plain(moe_plan_kernel, dim3(1), dim3(warps * 32), smem, st, sel_expert, sel_weight, row_token, row_weight, tile_expert, pair_row, n_tiles, pairs, experts, top, tile);
     return cuda_status("moe_plan launch");
 }
 
 int launch_moe_gather(int dtype, const float *x, const int *row_token, const float *row_weight, void *xg, const int *n_tiles,
                       int max_rows, int width, int tile, cudaStream_t st) {
     if (max_rows == 0) return B200_OK;
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(moe_gather_kernel<T>, dim3(max_rows), dim3(128), 0, st, false, x, row_token, row_weight, (T *)xg, n_tiles, width, tile); });
+    B200_DISPATCH_DTYPE(dtype, { launch_plain(moe_gather_kernel<T>, dim3(max_rows), dim3(128), 0, st, x, row_token, row_weight, (T *)xg, n_tiles, width, tile); });
     return cuda_status("moe_gather launch");
 }
 
@@ -706,7 +706,7 @@ int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, co
         const size_t smem = (size_t)2 * NG * KS * 128 * sizeof(float);
         auto go = [&](auto kern, auto *type) {
             using T = std::remove_pointer_t<decltype(type)>;
-            launch_pdl(kern, dim3(grid), dim3(KS * NG * 32), smem, st, false, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, kMoeTileM, max_tiles * kMoeTileM, N, K, act, KS, NG, steps);
+            launch_plain(kern, dim3(grid), dim3(KS * NG * 32), smem, st, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, kMoeTileM, max_tiles * kMoeTileM, N, K, act, KS, NG, steps);
         };
         if (dtype == B200_BF16) live_rows <= 8 ? go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 1>, (__nv_bfloat16 *)nullptr) : go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 2>, (__nv_bfloat16 *)nullptr);
         else live_rows <= 8 ? go(moe_few_rows_kernel<__half, __half, 1>, (__half *)nullptr) : go(moe_few_rows_kernel<__half, __half, 2>, (__half *)nullptr);
@@ -717,18 +717,18 @@ int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, co
         const size_t smem = (size_t)kMStages * (kMoeTileM + kMN) * kMK * 2;
         if (dtype == B200_BF16) {
             cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__nv_bfloat16, __nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            launch_pdl(moe_grouped_gemm_mma_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(grid), dim3(128), smem, st, false, (const __nv_bfloat16 *)a, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)c,
+            launch_plain(moe_grouped_gemm_mma_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(grid), dim3(128), smem, st, (const __nv_bfloat16 *)a, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)c,
                                                                                                tile_expert, n_tiles, max_tiles * kMoeTileM, N, K, act);
         } else {
             cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__half, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            launch_pdl(moe_grouped_gemm_mma_kernel<__half, __half>, dim3(grid), dim3(128), smem, st, false, (const __half *)a, (const __half *)w, (__half *)c, tile_expert, n_tiles,
+            launch_plain(moe_grouped_gemm_mma_kernel<__half, __half>, dim3(grid), dim3(128), smem, st, (const __half *)a, (const __half *)w, (__half *)c, tile_expert, n_tiles,
                                                                                  max_tiles * kMoeTileM, N, K, act);
         }
         return cuda_status("moe_grouped_gemm (tensor core) launch");
     }
     const dim3 grid((N + kGT - 1) / kGT, max_tiles);
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(moe_grouped_gemm_kernel<T>, dim3(grid), dim3(256), 0, st, false, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, N, K, act);
+        launch_plain(moe_grouped_gemm_kernel<T>, dim3(grid), dim3(256), 0, st, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, N, K, act);
     });
     return cuda_status("moe_grouped_gemm launch");
 }
@@ -738,7 +738,7 @@ int launch_activation(int dtype, void *x, size_t n, int act, cudaStream_t st) {
     B200_DISPATCH_DTYPE(dtype, {
         const size_t n_vec = (reinterpret_cast<size_t>(x) & 15) == 0 ? n / Elem<T>::kVec : 0;
         const size_t threads = n_vec + (n - n_vec * Elem<T>::kVec);
-        launch_pdl(activation_kernel<T>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st, false, (T *)x, n, act, n_vec);
+        launch_plain(activation_kernel<T>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st, (T *)x, n, act, n_vec);
     });
     return cuda_status("activation launch");
 }

@@ -778,7 +778,7 @@ static int launch_colrec_t(const float *rec, int rec_ld, int q_off, int k_off, i
     const size_t smem = ((size_t)2 * kRecTB * (NV * DP + 4) + (size_t)2 * kRecTB * cb) * sizeof(float);
     auto kern = column_recurrence_kernel<DP, LANES, CPT, MODE>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(kern, dim3((ncols + cb - 1) / cb, heads, n_seqs), dim3(block), smem, st, false, rec, rec_ld, q_off, k_off, v_off, a_off, b_off, S, n_state, m_state, o, nq, m_out,
+    launch_plain(kern, dim3((ncols + cb - 1) / cb, heads, n_seqs), dim3(block), smem, st, rec, rec_ld, q_off, k_off, v_off, a_off, b_off, S, n_state, m_state, o, nq, m_out,
                                                                         seq_start, seq_pos0, seq_slot, heads, kv_heads, dim, vdim, max_tokens);
     return cuda_status("column_recurrence launch");
 }
@@ -840,15 +840,15 @@ int launch_delta_prep(int dtype, const void *proj, int ld, int col0, const float
     const int per = std::max(1, std::min(4, row_tiles * groups / (2 * sm_count())));  // tiles per CTA, two CTAs per SM left
     const dim3 tile_grid((row_tiles + per - 1) / per, groups + 1);
     if (pieces && dtype == B200_BF16)
-        launch_pdl(delta_prep_tile_kernel<__nv_bfloat16>, dim3(tile_grid), dim3(256), 0, st, false, (const __nv_bfloat16 *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__nv_bfloat16 *)lr_a,
+        launch_plain(delta_prep_tile_kernel<__nv_bfloat16>, dim3(tile_grid), dim3(256), 0, st, (const __nv_bfloat16 *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__nv_bfloat16 *)lr_a,
                                                                          (__nv_bfloat16 *)lr_g, rec, lay, tok_seq, tok_pos, seq_pos0, seq_slot, tokens, heads, kv_heads, dim, vdim, per);
     else if (pieces)
-        launch_pdl(delta_prep_tile_kernel<__half>, dim3(tile_grid), dim3(256), 0, st, false, (const __half *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__half *)lr_a, (__half *)lr_g, rec, lay,
+        launch_plain(delta_prep_tile_kernel<__half>, dim3(tile_grid), dim3(256), 0, st, (const __half *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__half *)lr_a, (__half *)lr_g, rec, lay,
                                                                   tok_seq, tok_pos, seq_pos0, seq_slot, tokens, heads, kv_heads, dim, vdim, per);
     else B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         // few tokens: few CTAs, so each gets more threads (a thread's channels are a chain of load latencies)
-        launch_pdl(delta_prep_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), smem, st, false, (const T *)proj, ld, col0, conv_w, taps, conv_state, rank, gate_rank, (T *)lr_a, (T *)lr_g, rec, lay,
+        launch_plain(delta_prep_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), smem, st, (const T *)proj, ld, col0, conv_w, taps, conv_state, rank, gate_rank, (T *)lr_a, (T *)lr_g, rec, lay,
                                                        tok_seq, tok_pos, seq_pos0, seq_slot, heads, kv_heads, dim, vdim);
     });
     int rc = cuda_status("delta_prep launch");
@@ -864,7 +864,7 @@ int launch_delta_prep(int dtype, const void *proj, int ld, int col0, const float
         if (rc != B200_OK) return rc;
     }
     const bool v4 = dim % 4 == 0 && (heads * vdim) % 4 == 0 && all_aligned16({za, zg, decay_bias, rec});
-    launch_pdl((v4 ? delta_finish_kernel<true> : delta_finish_kernel<false>), dim3(tokens), dim3(256), 0, st, false, za, zg, decay_bias, a_log, rec, lay, heads, dim, vdim);
+    launch_plain((v4 ? delta_finish_kernel<true> : delta_finish_kernel<false>), dim3(tokens), dim3(256), 0, st, za, zg, decay_bias, a_log, rec, lay, heads, dim, vdim);
     return cuda_status("delta_finish launch");
 }
 
@@ -872,7 +872,7 @@ int launch_conv_state_update(int dtype, const void *proj, int ld, int col0, floa
                              const int *seq_pos0, const int *seq_slot, int n_seqs, cudaStream_t st) {
     if (n_seqs == 0 || taps <= 1) return B200_OK;
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(conv_state_update_kernel<T>, dim3((channels + 255) / 256, n_seqs), dim3(256), 0, st, false, (const T *)proj, ld, col0, conv_state, taps, channels, seq_start, seq_pos0, seq_slot);
+        launch_plain(conv_state_update_kernel<T>, dim3((channels + 255) / 256, n_seqs), dim3(256), 0, st, (const T *)proj, ld, col0, conv_state, taps, channels, seq_start, seq_pos0, seq_slot);
     });
     return cuda_status("conv_state_update launch");
 }
@@ -888,7 +888,7 @@ int launch_mlstm_prep(int dtype, const void *proj, int ld, int col0, const float
                       int vdim, cudaStream_t st) {
     if (tokens == 0) return B200_OK;
     const MlstmRow lay = mlstm_row(heads, dim, vdim);
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(mlstm_prep_kernel<T>, dim3(tokens), dim3(256), 0, st, false, (const T *)proj, ld, col0, b_in, cap, rec, lay, heads, dim, vdim); });
+    B200_DISPATCH_DTYPE(dtype, { launch_plain(mlstm_prep_kernel<T>, dim3(tokens), dim3(256), 0, st, (const T *)proj, ld, col0, b_in, cap, rec, lay, heads, dim, vdim); });
     return cuda_status("mlstm_prep launch");
 }
 
@@ -906,7 +906,7 @@ int launch_head_output(int dtype, const float *o, const float *nq, const float *
     const int grid = (tokens * heads + 7) / 8;
     const int vec = vdim % 8 == 0 && vdim <= 256 && w_stride % 4 == 0 && gate_f_ld % 4 == 0 && gate_t_ld % 8 == 0 && out_ld % 8 == 0 && all_aligned16({o, w, gate_f, gate_t, out});
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(head_output_kernel<T>, dim3(grid), dim3(256), 0, st, false, o, nq, m_in, w, w_stride, eps, gate_f, gate_f_ld, (const T *)gate_t, gate_t_ld, (T *)out, out_ld,
+        launch_plain(head_output_kernel<T>, dim3(grid), dim3(256), 0, st, o, nq, m_in, w, w_stride, eps, gate_f, gate_f_ld, (const T *)gate_t, gate_t_ld, (T *)out, out_ld,
                                                    out_scale, tokens, heads, vdim, gate_act, vec);
     });
     return cuda_status("head_output launch");
@@ -920,7 +920,7 @@ int launch_delta_prep_direct(int dtype, const void *proj, int ld, int col0, cons
     const size_t smem = ((size_t)2 * kv_heads * dim + heads * vdim) * sizeof(float);
     B200_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_direct_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_pdl(delta_prep_direct_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), smem, st, false, (const T *)proj, ld, col0, conv_w, taps, conv_state, decay_bias, a_log, rec,
+        launch_plain(delta_prep_direct_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), smem, st, (const T *)proj, ld, col0, conv_w, taps, conv_state, decay_bias, a_log, rec,
                                                                                    lay, tok_seq, tok_pos, seq_pos0, seq_slot, heads, kv_heads, dim, vdim);
     });
     return cuda_status("delta_prep_direct launch");
@@ -932,7 +932,7 @@ int launch_ssd_prep(int dtype, const void *proj, int ld, int col0, const float *
     if (tokens == 0) return B200_OK;
     const DecayRow lay = decay_row(heads, groups, state, vdim);
     B200_DISPATCH_DTYPE(dtype, {
-        launch_pdl(ssd_prep_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), (size_t)heads * sizeof(float), st, false, (const T *)proj, ld, col0, conv_w, conv_b, taps, conv_state, dt_bias,
+        launch_plain(ssd_prep_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), (size_t)heads * sizeof(float), st, (const T *)proj, ld, col0, conv_w, conv_b, taps, conv_state, dt_bias,
                                                                                                    a_log, skip_w, rec, lay, tok_seq, tok_pos, seq_pos0, seq_slot,
                                                                                                    heads, groups, state, vdim);
     });
@@ -943,7 +943,7 @@ int launch_linear_prep(int dtype, const void *proj, int ld, int col0, const floa
                        cudaStream_t st) {
     if (tokens == 0) return B200_OK;
     const DecayRow lay = decay_row(heads, heads, dim, vdim);
-    B200_DISPATCH_DTYPE(dtype, { launch_pdl(linear_prep_kernel<T>, dim3(tokens), dim3(256), 0, st, false, (const T *)proj, ld, col0, head_decay, rec, lay, heads, dim, vdim); });
+    B200_DISPATCH_DTYPE(dtype, { launch_plain(linear_prep_kernel<T>, dim3(tokens), dim3(256), 0, st, (const T *)proj, ld, col0, head_decay, rec, lay, heads, dim, vdim); });
     return cuda_status("linear_prep launch");
 }
 
@@ -964,7 +964,7 @@ int launch_group_output(int dtype, const float *o, const float *skip, int skip_l
     const int pieces = vec ? per / 4 : per, threads = pieces <= 64 ? 32 : (pieces <= 128 ? 64 : (pieces <= 256 ? 128 : 256));
     B200_DISPATCH_DTYPE(dtype, {
         auto kern = vec ? group_output_kernel<T, true> : group_output_kernel<T, false>;
-        launch_pdl(kern, dim3(tokens * groups), dim3(threads), 0, st, false, o, skip, skip_ld, w, eps, (const T *)gate, gate_ld, gate_act, gate_first, (T *)out, out_ld, cols, groups);
+        launch_plain(kern, dim3(tokens * groups), dim3(threads), 0, st, o, skip, skip_ld, w, eps, (const T *)gate, gate_ld, gate_act, gate_first, (T *)out, out_ld, cols, groups);
     });
     return cuda_status("group_output launch");
 }

@@ -279,14 +279,14 @@ int launch_sum_norm(int dtype, float *x, const void *y_dense, const void *y_rows
         const int per = vec ? Elem<T>::kVec : 1;
         const int threads = std::min(512, std::max(32, ((width + per - 1) / per + 31) / 32 * 32));
         auto kern = vec ? sum_norm_kernel<T, true> : sum_norm_kernel<T, false>;
-        launch_pdl(kern, dim3(tokens), dim3(threads), 0, st, false, x, (const T *)y_dense, (const T *)y_rows, pair_row, top, (const T *)y_shared, shared_gate, alpha, g, eps, width,
+        launch_plain(kern, dim3(tokens), dim3(threads), 0, st, x, (const T *)y_dense, (const T *)y_rows, pair_row, top, (const T *)y_shared, shared_gate, alpha, g, eps, width,
                                          trace, (T *)h_out, own, next, one_token, pm);
     });
     return cuda_status("sum_norm launch");
 }
 
 int launch_pos_turns(double *turns, int width, float base, cudaStream_t st) {
-    launch_pdl(pos_turns_kernel, dim3((width + 511) / 512), dim3(256), 0, st, false, turns, width, base);
+    launch_plain(pos_turns_kernel, dim3((width + 511) / 512), dim3(256), 0, st, turns, width, base);
     return cuda_status("pos_turns launch");
 }
 
@@ -298,7 +298,7 @@ int launch_embed_pos(int dtype, const int *ids, const void *table, float *x, voi
         const int cols = vec ? width / 4 : width;
         const int threads = std::min(256, (cols + 31) / 32 * 32);
         auto kern = vec ? embed_pos_kernel<T, 4> : embed_pos_kernel<T, 1>;
-        launch_pdl(kern, dim3(tokens, (cols + threads - 1) / threads), dim3(threads), 0, st, false, ids, (const T *)table, x, (T *)h_out, width, vocab, scale, turns, next,
+        launch_plain(kern, dim3(tokens, (cols + threads - 1) / threads), dim3(threads), 0, st, ids, (const T *)table, x, (T *)h_out, width, vocab, scale, turns, next,
                                                                                one_token, pm);
     });
     return cuda_status("embed_pos launch");
@@ -311,7 +311,7 @@ static void launch_conv_taps(const float *x, void *h, int width, RingConv cv, Po
     const int threads = std::min(256, (cols + 31) / 32 * 32);
     const dim3 grid((tokens + kConvRun - 1) / kConvRun, (cols + threads - 1) / threads);
     auto kern = vec ? conv_input_kernel<T, TAPS, 4> : conv_input_kernel<T, TAPS, 1>;
-    launch_pdl(kern, dim3(grid), dim3(threads), 0, st, false, x, (T *)h, width, tokens, cv, pm);
+    launch_plain(kern, dim3(grid), dim3(threads), 0, st, x, (T *)h, width, tokens, cv, pm);
 }
 
 int launch_conv_input(int dtype, const float *x, void *h, int width, RingConv cv, PortionMap pm, int tokens, cudaStream_t st) {
