@@ -19,6 +19,9 @@ namespace b200 {
 void set_error(const char *fmt, ...);
 int cuda_status(const char *what);  // cudaGetLastError(), then wait_status() -> B200_OK / B200_ERR_CUDA (+ message)
 int sm_count();
+// Raises the dynamic shared memory that a launch of this kernel may ask for, once per device, to the most that any of its launches asks for: the limit belongs
+// to the function, so a thread that set its own smaller size would make another thread's next launch fail.
+bool allow_smem(const void *kernel, size_t most);
 
 // Waits inside kernels have a limit: a fault elsewhere must not hang the device.  A kernel whose wait runs out stores NaN in place of what it could not
 // form, waits for its own copies, leaves its code in the process's wait word (mapped host memory) and returns; every later call of the library on the host

@@ -27,6 +27,7 @@ constexpr int kBK = 64;    // K elements per stage = one 128-byte swizzle row of
 constexpr int kUmmaK = 16; // K per tcgen05.mma for 16-bit inputs
 constexpr int kTcThreads = 192;
 constexpr int kMaxStages = 8;
+constexpr size_t kTcSmem = 200 * 1024 + 1024 /*alignment slack*/ + (2 * kMaxStages + 4) * 8 + 16;  // of a CTA, at most
 constexpr int kATileBytes = kBM * kBK * 2;
 
 struct GemmTcParams {
@@ -730,7 +731,7 @@ static int launch_gemm_pair(const void *x, const void *w, void *y, int M, int N,
     }
     const int grid = 2 * std::min(p.tiles, pairs);
     auto launch = [&](auto kern) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(reinterpret_cast<const void *>(kern), smem);
         launch_pdl_cluster(kern, dim3(grid), dim3(kPairThreads), smem, st, true, 2u, tmA, tmB, tmB2, p);
     };
     if (bf16) launch(gemm_tc_pair_kernel<__nv_bfloat16>);
@@ -812,7 +813,7 @@ static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int
     p.acc_stride = p.bn > 128 ? 256 : p.bn;
     p.tmem_cols = pow2_cols(p.acc_bufs == 2 ? p.acc_stride + p.bn : p.bn);
     const int stage_bytes = kATileBytes + p.bn * kBK * 2;
-    int stages = (int)((200 * 1024) / stage_bytes);
+    int stages = (int)((200 * 1024) / stage_bytes);  // (kTcSmem)
     if (stages > kMaxStages) stages = kMaxStages;
     if (stages < 2) return B200_ERR_UNSUPPORTED;
     p.stages = stages;
@@ -824,7 +825,7 @@ static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int
         return B200_ERR_CUDA;
     }
     auto launch = [&](auto kern) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(reinterpret_cast<const void *>(kern), kTcSmem);
         launch_pdl(kern, dim3(grid), dim3(kTcThreads), smem, st, true, tmA, tmB, p);
     };
     if (bf16) launch(gemm_tc_kernel<__nv_bfloat16>);
@@ -863,7 +864,7 @@ int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, 
     p.acc_stride = p.bn > 128 ? 256 : p.bn;
     p.tmem_cols = pow2_cols(p.acc_bufs == 2 ? p.acc_stride + p.bn : p.bn);
     const int stage_bytes = kATileBytes + p.bn * kBK * 2;
-    int stages = (int)((200 * 1024) / stage_bytes);
+    int stages = (int)((200 * 1024) / stage_bytes);  // (kTcSmem)
     if (stages > kMaxStages) stages = kMaxStages;
     if (stages < 2) return B200_ERR_UNSUPPORTED;
     p.stages = stages;
@@ -874,7 +875,7 @@ int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, 
         return B200_ERR_CUDA;
     }
     auto launch = [&](auto kern) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(reinterpret_cast<const void *>(kern), kTcSmem);
         launch_pdl(kern, dim3(grid), dim3(kTcThreads), smem, st, true, tmA, tmB, p);
     };
     if (bf16) launch(gemm_tc_kernel<__nv_bfloat16>);

@@ -10,15 +10,7 @@ namespace b200 {
 template <typename T, int FMT, int MB, bool SW, int XV>
 static int launch_gemv_geom(const GemvArgs &a, const GemvGeom &g, size_t smem, cudaStream_t st) {
     auto kern = gemv_nk_kernel<T, FMT, MB, SW, XV>;
-    static thread_local size_t cached_smem[64] = {0};  // per device, per instantiation: opt in to large dynamic smem once
-    int dev = 0;
-    cudaGetDevice(&dev);
-    dev &= 63;
-    if (cached_smem[dev] < smem) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return cuda_status("gemv cudaFuncSetAttribute");
-        cached_smem[dev] = smem;
-    }
+    if (!allow_smem(reinterpret_cast<const void *>(kern), 224 * 1024)) return cuda_status("gemv cudaFuncSetAttribute");
     const int units = SW ? a.inter : (a.N + 1) / 2;
     int grid = sm_count();
     const int need = (units + g.groups - 1) / g.groups;

@@ -559,14 +559,7 @@ template <typename T, int FMT, bool SW, int NT>
 static int launch_gemv_mma_inst(const GemvArgs &a, const MmaGeom &g, int grid, cudaStream_t st) {
     auto kern = gemv_mma_kernel<T, FMT, SW, NT, FMT == WF_FP8 ? 2 : 1>;
     const size_t smem = gemv_mma_smem(g);
-    static thread_local size_t cached_smem[64] = {0};  // per device, per instantiation
-    int dev = 0;
-    cudaGetDevice(&dev);
-    dev &= 63;
-    if (cached_smem[dev] < smem) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return cuda_status("gemv_mma cudaFuncSetAttribute");
-        cached_smem[dev] = smem;
-    }
+    if (!allow_smem(reinterpret_cast<const void *>(kern), 226 * 1024)) return cuda_status("gemv_mma cudaFuncSetAttribute");
     launch_pdl(kern, dim3(grid), dim3(kMmaThreads), smem, st, true, a, g);
     return cuda_status("gemv_mma launch");
 }

@@ -23,6 +23,7 @@
 namespace b200 {
 
 constexpr int kRsMaxStages = 12;
+constexpr size_t kRsSmem = 226 * 1024;  // dynamic shared memory of a CTA, at most
 constexpr int kRsBlocks = 8;            // 32-k blocks of a part that a warp holds (4 registers each at up to 8 tokens, 8 above)
 // Dense weights: a unit is 8 rows, the activations are the MMA's A operand (16 tokens), the weights its B.  Quantised weights: a unit is 16 rows and the
 // weights are A -- up to 8 tokens fill B, more take a second one, the dequantised rows serve both -- so that what a unit costs beside its weights
@@ -423,7 +424,7 @@ inline bool gemv_rs_geometry(int M, int K, int max_units, int fmt, RsGeom *out) 
     // (FP8: 128) bytes of each -- fall on different banks
     g.row_stride = (int)((bytes + 127) / 128 * 128) + (fmt == WF_FP8 ? 16 : 64);
     g.stage_bytes = rs_rows(fmt == WF_DENSE) * g.row_stride;
-    const size_t budget = 226 * 1024, fixed = gemv_rs_fixed_smem(g, fmt == WF_DENSE, M > 8 ? 2 : 1);
+    const size_t budget = kRsSmem, fixed = gemv_rs_fixed_smem(g, fmt == WF_DENSE, M > 8 ? 2 : 1);
     if (fixed + (size_t)2 * g.stage_bytes > budget) return false;
     g.wait = wait_guard();
     g.stages = (int)((budget - fixed) / g.stage_bytes);
@@ -436,14 +437,7 @@ template <typename T, int FMT, bool SW, int NT>
 static int launch_gemv_rs_inst(const GemvArgs &a, const RsGeom &g, int grid, cudaStream_t st) {
     auto kern = gemv_rs_kernel<T, FMT, SW, NT>;
     const size_t smem = gemv_rs_fixed_smem(g, FMT == WF_DENSE, NT) + (size_t)g.stages * g.stage_bytes;
-    static thread_local size_t cached_smem[64] = {0};  // per device, per instantiation
-    int dev = 0;
-    cudaGetDevice(&dev);
-    dev &= 63;
-    if (cached_smem[dev] < smem) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return cuda_status("gemv_rs cudaFuncSetAttribute");
-        cached_smem[dev] = smem;
-    }
+    if (!allow_smem(reinterpret_cast<const void *>(kern), kRsSmem)) return cuda_status("gemv_rs cudaFuncSetAttribute");
     launch_pdl(kern, dim3(grid), dim3(kMmaThreads), smem, st, true, a, g);
     return cuda_status("gemv_rs launch");
 }

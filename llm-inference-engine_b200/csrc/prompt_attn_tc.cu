@@ -33,6 +33,7 @@ constexpr int kQBox = kQRows * 128;        // bytes of 64 columns of Q or of P
 constexpr int kKBox = kPage * 128;         // bytes of 64 columns of a key / value page
 constexpr float kLog2eP = 1.4426950408889634f;
 constexpr float kRescale = 8.0f;           // log2 domain
+constexpr int kMaxPenalty = 8192;          // longest window with a distance penalty (its table is in shared memory)
 
 struct PromptAttn {
     const void *q, *qr;        // latent: q [heads, t_pad, DV], qr [tokens, heads, DK - DV];  chunked: q [tokens, heads * DK]
@@ -431,7 +432,7 @@ int pa_launch(PromptAttn p, const void *k_pool, const void *v_pool, bool bf16, c
     // (logits with a penalty: one CTA per SM.  Two ran only while the launches of this path overlapped, an order that stopped for a reason not found and was
     // taken back with them; the form has not been shown sound by itself)
     const size_t smem = std::max<size_t>(Sh::kSmem + 2 * p.pen_len * sizeof(float), BIASED ? 120 * 1024 : 0);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(reinterpret_cast<const void *>(kern), std::max<size_t>(Sh::kSmem + (BIASED ? 2 * (kMaxPenalty + 64) * sizeof(float) : 0), BIASED ? 120 * 1024 : 0));
     launch_plain(kern, dim3(p.n_tiles, p.heads / 2), dim3(Sh::kWarps * 32 + 64), smem, st, tmK, tmV, p);
     return cuda_status("prompt attention (tcgen05) launch");
 }
@@ -455,7 +456,7 @@ int launch_scored_attention_tc(int dtype, const void *q, const void *k_pool, con
                                void *out, int out_ld, float out_scale, const int *tiles, int n_tiles, const int *block_table, int mpps, int heads, int kv_heads, int dim, int vdim,
                                float scale, int window, int sigmoid, ScoredOptions opt, cudaStream_t st) {
     if ((dtype != B200_BF16 && dtype != B200_F16) || dim != 128 || vdim != 128 || sigmoid || opt.softcap > 0.0f || heads / kv_heads % 2 != 0 || !(scale > 0.0f)) return B200_ERR_UNSUPPORTED;
-    if (dist_r1 && !(window > 0 && window <= 8192)) return B200_ERR_UNSUPPORTED;
+    if (dist_r1 && !(window > 0 && window <= kMaxPenalty)) return B200_ERR_UNSUPPORTED;
     if (!all_aligned16({q, k_pool, v_pool, gate, out, tiles}) || (gate && gate_ld % 8 != 0) || out_ld % 8 != 0) return B200_ERR_UNSUPPORTED;
     if (n_tiles == 0) return B200_OK;
     PromptAttn p = {};

@@ -3,6 +3,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <unordered_set>
 
 #ifndef B200_NO_NVTX
 #include <nvtx3/nvToolsExt.h>
@@ -87,6 +88,23 @@ int sm_count() {
         cached[dev] = n;
     }
     return cached[dev];
+}
+
+bool allow_smem(const void *kernel, size_t most) {
+    static std::mutex mu;
+    static std::unordered_set<const void *> raised[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    static thread_local std::unordered_set<const void *> seen[64];  // (what this thread has found raised: no lock on a hot path)
+    dev &= 63;
+    if (seen[dev].count(kernel)) return true;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!raised[dev].count(kernel)) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return false;
+        raised[dev].insert(kernel);
+    }
+    seen[dev].insert(kernel);
+    return true;
 }
 
 // One workspace per device: [tickets (kTickets x u32, zeroed once, self-resetting) | scratch].
