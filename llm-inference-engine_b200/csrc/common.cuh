@@ -22,6 +22,11 @@ int sm_count();
 // Raises the dynamic shared memory that a launch of this kernel may ask for, once per device, to the most that any of its launches asks for: the limit belongs
 // to the function, so a thread that set its own smaller size would make another thread's next launch fail.
 bool allow_smem(const void *kernel, size_t most);
+}  // namespace b200
+struct CUtensorMap_st;
+namespace b200 {
+// Tensor map of a rows x cols matrix of a 16-bit type whose rows follow one another: boxes of box_rows x 64 columns, 128-byte swizzle, zeros past the edge.
+bool tile_map(CUtensorMap_st *map, const void *ptr, size_t rows, int cols, int box_rows, bool bf16);
 
 // Waits inside kernels have a limit: a fault elsewhere must not hang the device.  A kernel whose wait runs out stores NaN in place of what it could not
 // form, waits for its own copies, leaves its code in the process's wait word (mapped host memory) and returns; every later call of the library on the host

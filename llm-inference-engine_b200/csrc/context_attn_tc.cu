@@ -30,7 +30,6 @@
 
 #include <cuda.h>
 #include <float.h>
-#include <mutex>
 
 namespace b200 {
 
@@ -466,35 +465,6 @@ context_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *sym = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(sym);
-        else
-            cudaGetLastError();
-    });
-    return fn;
-}
-// rows x 128 matrix of a 16-bit type, boxes of 128 rows x 64 columns, 128-byte swizzle
-static bool make_map(CUtensorMap *map, const void *ptr, size_t rows, bool bf16, int box_rows = 128) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return false;
-    cuuint64_t dims[2] = {(cuuint64_t)kD, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)kD * 2};
-    cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 }  // namespace catc
 
 // q [B, H, max_q_len, 128]; k/v: LAYER base of the cache [B, Hkv, S, 128]; out [T, H, 128]; seq_off [B] (device).
@@ -511,8 +481,8 @@ int launch_context_attention_tc(const void *q, const void *k_layer, const void *
     CUtensorMap tmQ, tmK, tmV;
     const size_t kv_rows = block_table ? (size_t)num_pages * kv_head_num * 64 : (size_t)batch * kv_head_num * max_seq_len;
     const int kv_box = block_table ? 64 : 128;
-    if (!make_map(&tmQ, q, (size_t)batch * head_num * max_q_len, bf16) || !make_map(&tmK, k_layer, kv_rows, bf16, kv_box) ||
-        !make_map(&tmV, v_layer, kv_rows, bf16, kv_box)) {
+    if (!tile_map(&tmQ, q, (size_t)batch * head_num * max_q_len, kD, 128, bf16) || !tile_map(&tmK, k_layer, kv_rows, kD, kv_box, bf16) ||
+        !tile_map(&tmV, v_layer, kv_rows, kD, kv_box, bf16)) {
         set_error("context_attention: cuTensorMapEncodeTiled failed");
         return B200_ERR_CUDA;
     }

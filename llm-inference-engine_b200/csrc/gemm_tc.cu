@@ -16,9 +16,8 @@
 // (self-resetting ticket) adds the slots in a fixed order (deterministic, no atomics on data).
 #include "gemm_tc.cuh"
 
-#include <cuda.h>  // CUtensorMap (types only: the encoder is fetched through cudaGetDriverEntryPoint, no libcuda link dependency)
+#include <cuda.h>  // CUtensorMap
 #include <algorithm>
-#include <mutex>
 
 namespace b200 {
 
@@ -643,38 +642,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 }
 
 // ------------------------------------------------------------------ host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *sym = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(sym);
-        else
-            cudaGetLastError();
-    });
-    return fn;
-}
-
-// 2-D K-major tensor map: dims {K, rows}, row pitch K * 2 bytes, box {64, box_rows}, 128-byte swizzle, zero fill out of bounds.
-static bool make_map(CUtensorMap *map, const void *ptr, int rows, int K, int box_rows, bool bf16) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return false;
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(ptr), dims, strides,
-              box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 static unsigned int pow2_cols(int c) {
     unsigned int v = 32;
     while ((int)v < c) v <<= 1;
@@ -725,7 +692,7 @@ static int launch_gemm_pair(const void *x, const void *w, void *y, int M, int N,
     p.stages = 6, p.wait = wait_guard();
     const size_t smem = (size_t)p.stages * kPairStageBytes + 1024 + (2 * kMaxStages + 4) * 8 + 16;
     CUtensorMap tmA, tmB, tmB2;
-    if (!make_map(&tmA, x, M, K, kBM, bf16) || !make_map(&tmB, w, cols, K, p.bn / 2, bf16) || !make_map(&tmB2, w, cols, K, p.bn2 / 2, bf16)) {
+    if (!tile_map(&tmA, x, M, K, kBM, bf16) || !tile_map(&tmB, w, cols, K, p.bn / 2, bf16) || !tile_map(&tmB2, w, cols, K, p.bn2 / 2, bf16)) {
         set_error("gemm_tc pair: cuTensorMapEncodeTiled failed (rows %d/%d, K %d)", M, cols, K);
         return B200_ERR_CUDA;
     }
@@ -820,7 +787,7 @@ static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int
     const size_t smem = (size_t)stages * stage_bytes + 1024 /*alignment slack*/ + (2 * kMaxStages + 4) * 8 + 16;
 
     CUtensorMap tmA, tmB;
-    if (!make_map(&tmA, a_ptr, p.rowsA, K, kBM, bf16) || !make_map(&tmB, b_ptr, rows_b_map, K, swiglu_inter ? p.swiglu_hw : p.bn, bf16)) {
+    if (!tile_map(&tmA, a_ptr, p.rowsA, K, kBM, bf16) || !tile_map(&tmB, b_ptr, rows_b_map, K, swiglu_inter ? p.swiglu_hw : p.bn, bf16)) {
         set_error("gemm_tc: cuTensorMapEncodeTiled failed (rows %d/%d, K %d)", p.rowsA, p.rowsB, K);
         return B200_ERR_CUDA;
     }
@@ -870,7 +837,7 @@ int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, 
     p.stages = stages;
     const size_t smem = (size_t)stages * stage_bytes + 1024 + (2 * kMaxStages + 4) * 8 + 16;
     CUtensorMap tmA, tmB;
-    if (!make_map(&tmA, a, max_rows, K, kBM, bf16) || !make_map(&tmB, w, experts * N, K, p.bn, bf16)) {
+    if (!tile_map(&tmA, a, max_rows, K, kBM, bf16) || !tile_map(&tmB, w, experts * N, K, p.bn, bf16)) {
         set_error("gemm_tc grouped: cuTensorMapEncodeTiled failed (rows %d, experts %d x %d, K %d)", max_rows, experts, N, K);
         return B200_ERR_CUDA;
     }

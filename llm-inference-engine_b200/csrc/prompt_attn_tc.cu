@@ -21,7 +21,6 @@
 
 #include <cuda.h>
 #include <algorithm>
-#include <mutex>
 
 namespace b200 {
 
@@ -394,29 +393,10 @@ prompt_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     }
 }
 
-typedef CUresult (*PaEncode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
-                             CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-PaEncode pa_encode() {
-    static PaEncode fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *sym = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess) fn = reinterpret_cast<PaEncode>(sym);
-        else cudaGetLastError();
-    });
-    return fn;
-}
 // the pool as a matrix of `cols`-wide rows in boxes of one page x 64 columns.  Its row count is not known here: the block table names the rows that are
 // asked for, and those exist
 bool pa_map(CUtensorMap *map, const void *ptr, int cols, bool bf16) {
-    PaEncode fn = pa_encode();
-    if (!fn) return false;
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)1 << 30};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-    cuuint32_t box[2] = {64, (cuuint32_t)kPage}, estr[2] = {1, 1};
-    return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return tile_map(map, ptr, (size_t)1 << 30, cols, kPage, bf16);
 }
 
 template <typename T, int DK, int DV, bool LATENT, bool BIASED>

@@ -1,6 +1,7 @@
 // runtime.cu -- error plumbing, device queries and the library workspace of libb200llm.so.
 #include "common.cuh"
 
+#include <cuda.h>  // CUtensorMap: types only, the encoder comes through cudaGetDriverEntryPoint (no libcuda to link)
 #include <atomic>
 #include <mutex>
 #include <unordered_set>
@@ -105,6 +106,29 @@ bool allow_smem(const void *kernel, size_t most) {
     }
     seen[dev].insert(kernel);
     return true;
+}
+
+bool tile_map(CUtensorMap *map, const void *ptr, size_t rows, int cols, int box_rows, bool bf16) {
+    typedef CUresult (*Encode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
+                               CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void *sym = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &found) != cudaSuccess) cudaGetLastError(), sym = nullptr;
+        return sym && found == cudaDriverEntryPointSuccess ? reinterpret_cast<Encode>(sym) : nullptr;
+    }();
+    if (!encode) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, steps[2] = {1, 1};
+    auto make = [&] {
+        return encode(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, steps,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    if (make() == CUDA_SUCCESS) return true;
+    // The encoder is the driver's and wants a current context, which the runtime binds to a thread with its first call that needs one: in a thread whose first
+    // call is this one there is none yet.
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && make() == CUDA_SUCCESS;
 }
 
 // One workspace per device: [tickets (kTickets x u32, zeroed once, self-resetting) | scratch].
