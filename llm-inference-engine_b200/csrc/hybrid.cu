@@ -1356,13 +1356,14 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     static_assert(kShortPortion == kMingruShort, "one list of short portions serves both");
     int n_tiles = 0, n_short = 0, n_chunks = 0, gla_kinds = 0;
     // minGRU chunks: at most 64 per portion (a chunk composes the maps of all chunks before it), of whole multiples of kMingruChunk tokens
-    int longest = 0;
+    int longest = 0, long_tokens = 0;  // long_tokens: of the portions that the token-parallel recurrences can take
     bool mid_portions = false;  // portions of several tokens that the token-parallel recurrences leave to the serial ones
     for (int s = 0; s < S; ++s) longest = std::max(longest, b->seq_start[s + 1] - b->seq_start[s]);
     const int chunk_tokens = std::max(1, (longest + 64 * kMingruChunk - 1) / (64 * kMingruChunk)) * kMingruChunk;
     for (int s = 0; s < S; ++s) {
         const int t0 = b->seq_start[s], t1 = b->seq_start[s + 1];
         mid_portions |= t1 - t0 > 1 && t1 - t0 < kChunkMinTokens;
+        if (t1 - t0 >= kChunkMinTokens) long_tokens += t1 - t0;
         gla_kinds |= t1 - t0 == 1 ? kGlaOneToken : (t1 - t0 > 1 ? kGlaManyTokens : 0);
         B200_REQUIRE(t1 >= t0 && b->seq_pos0[s] >= 0, "hybrid_forward: bad portion of sequence %d", s);
         B200_REQUIRE(b->seq_slot[s] >= 0 && b->seq_slot[s] < m->num_slots, "hybrid_forward: state slot %d outside [0, %d)", b->seq_slot[s], m->num_slots);
@@ -1465,10 +1466,10 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         RUN(embed(f32 ? nullptr : m->h, width));
     }
 
-    // a recurrence over the batch: its token-parallel form for the long portions, where it takes the layer's sizes, and the serial form for the rest
-    auto recurrence = [&](auto chunked, auto serial) -> int {
+    // a recurrence over the batch: its token-parallel form for the long portions, where it takes the layer's sizes and is the faster one, and the serial form for the rest
+    auto recurrence = [&](const b200_hybrid_layer_t &l, auto chunked, auto serial) -> int {
         int kinds = gla_kinds, max_tokens = kAnyTokens;
-        if (longest >= kChunkMinTokens) {
+        if (chunk_pays(l.mixer == B200_MIXER_GLA, l.heads, l.vdim, longest, long_tokens, sm_count())) {
             rc = chunked();
             if (rc != B200_OK && rc != B200_ERR_UNSUPPORTED) return rc;
             if (rc == B200_OK) {
@@ -1480,7 +1481,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     };
     auto decay_recurrence = [&](const b200_hybrid_layer_t &l, const MixerPlan &mp, int key_heads) -> int {
         float *state = (float *)(m->state_pool + mp.state_off);
-        return recurrence([&] { return launch_chunk_decay(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, key_heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
+        return recurrence(l, [&] { return launch_chunk_decay(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, key_heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
                           [&](int, int most) { return launch_decay_recurrent(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, key_heads, l.dim, l.vdim, st, gla_kinds == kGlaOneToken, most); });
     };
 
@@ -1525,7 +1526,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                                              NT, l.heads, l.kv_heads, l.dim, l.vdim, st));
             RUN(launch_conv_state_update(dt, m->proj, n_in, col, conv_state, l.conv, conv_channels(l), d_start, d_pos0, d_slot, S, st));
             float *state = (float *)(m->state_pool + mp.state_off);
-            RUN(recurrence([&] { return launch_chunk_delta(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.kv_heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
+            RUN(recurrence(l, [&] { return launch_chunk_delta(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.kv_heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
                            [&](int, int most) { return launch_delta_recurrent(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.kv_heads, l.dim, l.vdim, st, one_token, most); }));
             if (l.decay_rank > 0) {
                 RUN(launch_head_output(dt, m->f32b, nullptr, nullptr, l.out_norm, 0, c.norm_eps, m->rec + lay.gate, lay.ld, nullptr, 0, out, out_ld, out_scale,
@@ -1805,7 +1806,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             const char *gate = (const char *)m->proj + (size_t)(2 * hd + hv) * es;
             RUN(launch_gla_decay(dt, m->proj, lp.n_in, 2 * hd + 2 * hv, l.w_decay, l.decay_bias, l.tau, m->f32a, NT, l.decay_rank, hd, st));
             float *state = (float *)(m->state_pool + lp.state_off);
-            RUN(recurrence([&] { return launch_chunk_gla(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
+            RUN(recurrence(l, [&] { return launch_chunk_gla(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
                            [&](int kinds, int most) { return launch_gla_recurrent(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, st, kinds, most); }));
             RUN(launch_gla_output(dt, m->f32b, l.out_norm, c.norm_eps, gate, lp.n_in, m->mix2, NT, l.heads, l.vdim, st));
             n_mixed = hv;

@@ -186,6 +186,19 @@ int launch_gla_output(int dtype, const float *o, const float *w, float eps, cons
 // serial kernels serve them with max_tokens = kChunkMinTokens - 1).  B200_ERR_UNSUPPORTED, nothing launched: sizes or alignments it does not take.
 // scratch: fp32, chunk_scratch_floats of the engine's limits (0: sizes it never takes); tokens / longest: of this call and of its longest portion
 constexpr int kChunkMinTokens = 64;
+// Whether a batch is faster so: the form trades one dependent step per token for more multiply-adds, so it wins while the portions are long and the CTAs few.
+// The work counted is that of the scan's CTAs (16 columns of one head's state and portion) and the factors' (about 8 more per head), with as many portions as
+// the longest would make of the batch's long tokens.  Measured (B200, serial against factors + scan, us; dim 128 or 64, vdim 64 to 256, 1 to 16 portions):
+//   <= 2 units of work per SM: one portion of 64 tokens 23.6 / 23.2 (GLA), 26.6 / 29.7 (delta), of 96 27.6 / 25.6 and 35.6 / 33.6 (at other sizes up to 1.1 times
+//   as long), of 128 34.8 / 27.6 and 45.0 / 37.7: from 128 tokens on never slower, at 512 0.4 to 0.83 of the serial time
+//   above that, 128 tokens: up to 1.11 times as long (delta 40.9 / 44.0), 256: 0.53 to 1.0 while the limit below holds
+//   limit: GLA (whose serial step is the cheaper one) 3 per SM: 56.3 / 50.1 at 2.6, but 82.9 / 87.0 at 5.2; the others 6: delta 273 / 237, decay alone 182 / 161
+//   at 5.2, but 141 / 138 and 93 / 95 at 6.9 and 200 / 235 and 130 / 163 at 13.8
+inline bool chunk_pays(bool gla, int heads, int vdim, int longest, int long_tokens, int sms) {
+    if (longest < 128) return false;
+    const long long work = (long long)heads * (vdim / 16 + 8) * long_tokens, unit = (long long)sms * longest;
+    return work <= unit * 2 || (longest >= 256 && work <= unit * (gla ? 3 : 6));
+}
 size_t chunk_scratch_floats(int heads, int dim, bool delta, int max_tokens, int max_seqs);
 int launch_chunk_gla(int dtype, const void *proj, int ld, const float *decay, float *state, float *o, const int *seq_start, const int *seq_pos0,
                      const int *seq_slot, int n_seqs, int heads, int dim, int vdim, float *scratch, size_t scratch_floats, int tokens, int longest,

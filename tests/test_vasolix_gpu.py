@@ -506,3 +506,19 @@ def test_sizes_that_fit_every_vector(dtype, tol):
         want = want_logits(config, W, req[name])
         per_pos = np.linalg.norm(got[name] - want, axis=-1) / np.linalg.norm(want, axis=-1)
         assert np.median(per_pos) < tol and per_pos.max() < 5 * tol, (name, float(np.median(per_pos)), float(per_pos.max()))
+
+
+@pytest.mark.parametrize("heads,schedule", [
+    (2, [[("a", 127), ("b", 63)], [("a", 128), ("b", 64), ("c", 63), ("d", 1)], [("a", 1), ("b", 65), ("c", 1), ("d", 130)]]),  # around 128 tokens
+    (24, [[("a", 256)], [("a", 64), ("b", 256)], [("b", 130), ("c", 131), ("d", 129)], [("a", 1), ("c", 64)]]),                 # work around the limits
+], ids=["length", "work"])
+def test_recurrence_on_both_sides_of_the_token_parallel_rule(heads, schedule):
+    """One request after another through serial and token-parallel recurrences, beside portions that stay serial: the state goes from one to the other."""
+    config = ref.make_config([ref.gla_layer(heads=heads, dim=64, vdim=64), ref.attention_layer(heads=2, kv_heads=1, dim=16, size=90, scale=0.25)], width=64)
+    W, packed = ref.make_weights(config, seed=101)
+    total = {}
+    for step in schedule:
+        for name, n in step:
+            total[name] = total.get(name, 0) + n
+    req = {name: tokens_of(config, n, 1 + i) for i, (name, n) in enumerate(total.items())}
+    check_all(replay(session(config, packed, pool_tokens=2048), req, schedule), config, W, req, 5e-5)
