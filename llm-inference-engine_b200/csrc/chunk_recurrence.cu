@@ -14,8 +14,8 @@
 // here first (182 us for the first case below, 203 for the second): 22 of 24 bits and sums that are cut off put read-outs up to 2.1 and states up to 5 times
 // as far from 64 bits as the serial kernels'; now 0.46 to 1.05 times (fp32 vectors, dim 64 and 128, 64 to 4096 tokens, decays near 1, around 0.7 and 0.15).
 // tcgen05 has no fp32 form.
-// Measured (B200, 8 heads, dim 128, vdim 256; factors + scan against the serial kernel): linear attention of 4096 tokens 38 + 321 against 690 us, delta rule of
-// 1500, 511 and 900 tokens 41 + 293 against 401.
+// Measured (B200, 8 heads, dim 128, vdim 256; factors + scan against the serial kernel): linear attention of 4096 tokens 37 + 326 against 690 us, delta rule of
+// 1500, 511 and 900 tokens 40 + 289 against 401.
 #include "hybrid_ops.cuh"
 
 #include <algorithm>
