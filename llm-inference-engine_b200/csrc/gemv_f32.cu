@@ -7,6 +7,8 @@ int launch_gemv_nk_bf16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st
 int launch_gemv_nk_f16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
 int launch_gemv_mma_bf16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
 int launch_gemv_mma_f16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
+int launch_gemv_qd_bf16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
+int launch_gemv_qd_f16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
 int launch_gemv_rs_bf16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
 int launch_gemv_rs_f16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
 int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStream_t st) {
@@ -15,10 +17,15 @@ int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStrea
         return B200_ERR_INVALID_ARG;
     }
     const bool b16 = dtype == B200_BF16 || dtype == B200_F16;
-    // 16-bit activations, no prologue: 2..16 tokens, and one token of quantised weights, past which the weights stream with the activations in registers
+    // up to 8 tokens of INT4 weights: weights straight from global memory into registers (gemv_qd.cuh, with both sides' times)
+    if (b16 && fmt == WF_INT4 && a.M <= 8) {
+        const int rc = dtype == B200_BF16 ? launch_gemv_qd_bf16(a, fmt, swiglu, st) : launch_gemv_qd_f16(a, fmt, swiglu, st);
+        if (rc != B200_ERR_UNSUPPORTED) return rc;
+    }
+    // 16-bit activations, no prologue: 2..16 tokens, and one token of FP8 weights, past which the weights stream with the activations in registers
     // (gemv_rs.cuh).  One dense token keeps the SIMT kernel and its fused norm: its weights alone fill the memory pipe, and the norm launch would come on
-    // top.  One quantised token, 4 layers, norm kernel + gemv_rs against the kernel with the fused norm that was here (ctx 1024): 7B size FP8 238 / INT4 249 us
-    // against 245 / 268, 70B-shaped shard 204 / 222 against 230 / 255, 2048-wide 130 / 131 against 142 / 159.
+    // top.  One FP8 token, 4 layers, norm kernel + gemv_rs against the kernel with the fused norm that was here (ctx 1024): 7B size 238 us against 245, 70B-shaped
+    // shard 204 against 230, 2048-wide 130 against 142.
     if (b16 && (a.M >= 2 || fmt != WF_DENSE) && a.M <= 16) {
         const int rc = dtype == B200_BF16 ? launch_gemv_rs_bf16(a, fmt, swiglu, st) : launch_gemv_rs_f16(a, fmt, swiglu, st);
         if (rc != B200_ERR_UNSUPPORTED) return rc;

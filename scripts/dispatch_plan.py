@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Which kernel, how many passes over the weights and which ring geometry each linear of a decode step gets -- a Python MODEL of the host-side
 dispatch (no GPU): decoder.cu norm_linear (norm inside the GEMV for one dense token, a norm kernel in front otherwise), gemv_f32.cu launch_gemv_nk
-(gemv_rs, what its ring refuses on gemv_mma, the SIMT GEMV for up to 4 tokens), linear.cu (GEMV passes, tcgen05 GEMM for dense M > 16), gemv_inst.cuh,
+(gemv_qd for up to 8 tokens of INT4, gemv_rs, what its ring refuses on gemv_mma, the SIMT GEMV for up to 4 tokens), linear.cu (GEMV passes, tcgen05 GEMM for dense M > 16), gemv_inst.cuh,
 gemv_rs.cuh gemv_rs_geometry and gemv_mma.cuh gemv_mma_geometry.  It restates those few formulas; when they change, this file must follow
 (tests/test_dispatch_plan.py).
 usage: python scripts/dispatch_plan.py > profiles/<tag>_dispatch_plan.txt"""
@@ -97,8 +97,23 @@ def gemv_rs_plan(M, K, N, fmt, swiglu=False):
     return dict(kernel="gemv_rs", pieces=parts, piece_bytes=row, stages=min((226 * 1024 - fixed) // stage, RS_STAGES), parts=parts, part_k=part_k)
 
 
+def gemv_qd_plan(M, K, N, fmt, swiglu=False):
+    """gemv_qd.cuh launch_gemv_qd_t (INT4 in groups of 128, 1..8 tokens): None when unsupported.  It is the form of gemv_rs whose ring is in registers."""
+    if fmt != "int4" or M < 1 or M > 8 or K % 128:
+        return None
+    units = -(-(N // 2) // 8) if swiglu else -(-N // 16)
+    warps = 16 if K >= 8192 or (K >= 4096 and units <= 2 * SMS) else 8
+    smem = M * (2 * K + 64) + 256 + 2 * warps * 160 * 4
+    if smem > 160 * 1024 * warps // 16:
+        return None
+    return dict(kernel="gemv_rs", form="gemv_qd", warps=warps, pieces=1, piece_bytes=K // 2, stages=2, smem=smem)
+
+
 def gemv_any(M, K, N, fmt, swiglu=False):
     """gemv_f32.cu launch_gemv_nk for a 16-bit model."""
+    g = gemv_qd_plan(M, K, N, fmt, swiglu)
+    if g:
+        return g
     if M <= 16 and (M >= 2 or fmt != "dense"):
         rows = 16 if fmt == "fp8" else 8
         units = -(-(N // 2) // (rows // 2)) if swiglu else -(-N // rows)

@@ -62,6 +62,30 @@ def test_linear_of_few_tokens_and_odd_rows(n):
     assert bool((out[6 * n:] == 7.0).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("m,k,n", [(1, 128, 1), (8, 640, 31), (3, 1920, 2369), (8, 2176, 4743), (2, 4096, 17), (5, 4096, 4737), (8, 4224, 2384), (1, 8320, 4743), (6, 8192, 16),
+                                   (6, 11008, 24), (7, 11008, 24), (2, 28672, 48), (3, 28672, 48)])
+def test_int4_weights_streamed_into_registers(dtype, m, k, n):
+    """csrc/gemv_qd.cuh: every zero point of a byte, activations with a mean or tiny (2^-12), odd group counts per warp and warps without groups, rows past the
+    last unit, activations that only just fit (or no longer do)."""
+    gen = torch.Generator(device=DEV).manual_seed(m + k + n)
+    q, s, _, _ = quantised(gen, n, k, "int4", dtype)
+    s *= 2.0 ** -11  # the largest result, 28672 products of 270 and activations of mean 4, stays below 65504
+    z = torch.randint(0, 256, (n, k // 128), generator=gen, device=DEV, dtype=torch.uint8)
+    z[::2] &= 15
+    codes = torch.stack((q & 15, q >> 4), -1).reshape(n, k // 128, 128).double()
+    dense = ((codes - z.double()[..., None]) * s.double()[..., None]).reshape(n, k)
+    for mean, scale in ((4.0, 1.0), (0.0, 2.0 ** -12)):
+        x = ((torch.randn(m, k, generator=gen, device=DEV) + mean) * scale).to(dtype)
+        out = torch.full((m * n + 64,), 7.0, dtype=dtype, device=DEV)
+        got = b200.linear(x, q, w_format=b200.W_INT4, scales=s, zeros=z, group=128, N=n, out=out[:m * n].view(m, n)).double()
+        # one rounding of the result; fp32 sums: 2^-24 of the terms' sizes for each of a group's 8 products, the groups' and the warps' sums (28672 k: 14 + 16)
+        x16 = x.half().double()  # the activations as the tensor cores take them
+        bound = ROUND[dtype] * (x16 @ dense.T).abs() + 38 * 2.0 ** -24 * x16.abs() @ ((codes - z.double()[..., None]).abs() * s.double()[..., None]).reshape(n, k).T + 2.0 ** -24
+        assert bool(((got - x16 @ dense.T).abs() <= bound).all()), (mean, float(((got - x16 @ dense.T).abs() / bound).max()))
+        assert bool((out[m * n:] == 7.0).all())
+
+
 @pytest.mark.parametrize("fmt,n", [("dense", 192000), ("fp8", 152064), ("int4", 290000)])
 def test_linear_whose_sums_leave_no_ring(fmt, n):
     """Vocabulary-sized outputs of rows of 8192 k, 16 tokens: sizes that stay with the kernel whose activations are in shared memory (csrc/gemv_mma.cuh), and
