@@ -14,11 +14,12 @@
 // here first (182 us for the first case below, 203 for the second): 22 of 24 bits and sums that are cut off put read-outs up to 2.1 and states up to 5 times
 // as far from 64 bits as the serial kernels'; now 0.46 to 1.05 times (fp32 vectors, dim 64 and 128, 64 to 4096 tokens, decays near 1, around 0.7 and 0.15).
 // tcgen05 has no fp32 form.
-// Measured (B200, 8 heads, dim 128, vdim 256; factors + scan against the serial kernel): linear attention of 4096 tokens 37 + 326 against 690 us, delta rule of
-// 1500, 511 and 900 tokens 40 + 289 against 401.
+// Measured (B200, 8 heads, dim 128, vdim 256; factors + scan against the serial kernel): linear attention of 4096 tokens 39 + 218 against 690 us, delta rule of
+// 1500, 511 and 900 tokens 42 + 212 against 401.
 #include "hybrid_ops.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace b200 {
 
@@ -27,12 +28,14 @@ namespace {
 constexpr int kC = 32;      // tokens per chunk
 constexpr int kCols = 16;   // columns of S per CTA of the scan (the M of its matrix instructions)
 
-// one (chunk, head) block, rows as they are: Qp [kC x DK], (delta rule: Kp [kC x DK]), Ke [kC x DK], P [kC x kC], p_C [DK], (Tb [kC x kC])
+// one (chunk, head) block, rows as the scan has them in shared memory: Qp, (delta rule: Kp,) Ke [kC][kP], P [kC][kTP], p_C [DK], (Tb [kC][kTP])
+constexpr int kTP = 40;  // floats per row of P and Tb and per column of V^T
 template <int DK, bool DELTA> struct Block {
-    static constexpr int kQp = 0, kKp = kC * DK, kKe = (DELTA ? 2 : 1) * kC * DK, kP = kKe + kC * DK, kG = kP + kC * kC, kTb = kG + DK;
-    static constexpr int kFloats = kTb + (DELTA ? kC * kC : 0);
+    static constexpr int kP = DK + 8;  // floats per row of the factors and per column of S^T: rows start 8 banks apart
+    static constexpr int kQp = 0, kKp = kC * kP, kKe = (DELTA ? 2 : 1) * kC * kP, kPm = kKe + kC * kP, kG = kPm + kC * kTP, kTb = kG + DK;
+    static constexpr int kFloats = kTb + (DELTA ? kC * kTP : 0);
 };
-__host__ __device__ constexpr int block_floats(int dk, bool delta) { return (delta ? 3 : 2) * kC * dk + (delta ? 2 : 1) * kC * kC + dk; }
+__host__ __device__ constexpr int block_floats(int dk, bool delta) { return (delta ? 3 : 2) * kC * (dk + 8) + (delta ? 2 : 1) * kC * kTP + dk; }
 
 // where a head's vectors of a token are: q, k, v rows of one array of type TQ (element offsets), the decays in an fp32 array
 struct ChunkSource {
@@ -191,7 +194,7 @@ chunk_factors_kernel(const ChunkSource src, const ChunkMap map, float *__restric
 #pragma unroll 4
         for (int t = 15; t >= 0; --t) {  // g: after token t, to the end of the half
             const int row = 16 * half + t;
-            blk[B::kKe + row * DK + i] = (float)((double)ks[row * P + i] * (g * after));
+            blk[B::kKe + row * B::kP + i] = (float)((double)ks[row * P + i] * (g * after));
             g *= (double)gs[row * P + i];
         }
         g = 1.0;
@@ -201,8 +204,8 @@ chunk_factors_kernel(const ChunkSource src, const ChunkMap map, float *__restric
             const float k = ks[row * P + i], q = qs[row * P + i];
             g *= (double)gs[row * P + i];
             const double p = before * g;
-            if (DELTA) blk[B::kKp + row * DK + i] = (float)((double)k * p);
-            blk[B::kQp + row * DK + i] = (float)((double)q * p);
+            if (DELTA) blk[B::kKp + row * B::kP + i] = (float)((double)k * p);
+            blk[B::kQp + row * B::kP + i] = (float)((double)q * p);
             // the operands of the block below the diagonal replace the raw rows: targets from its start here, sources carried to the first half's end below
             if (half) ks[row * P + i] = k * (float)g, qs[row * P + i] = q * (float)g;
         }
@@ -242,11 +245,11 @@ chunk_factors_kernel(const ChunkSource src, const ChunkMap map, float *__restric
 #pragma unroll
             for (int r = 0; r < t; ++r) d[r & 3] = fmaf(-As[t * 36 + r], x[r], d[r & 3]);
             x[t] = bs[t] * ((d[0] + d[1]) + (d[2] + d[3]));
-            blk[B::kTb + t * kC + lane] = x[t];
+            blk[B::kTb + t * kTP + lane] = x[t];
         }
     } else {
         const int first = DELTA ? 32 : 0;
-        for (int idx = tid - first; idx < kC * kC; idx += 256 - first) blk[B::kP + idx] = Ps[(idx >> 5) * 36 + (idx & 31)];
+        for (int idx = tid - first; idx < kC * kC; idx += 256 - first) blk[B::kPm + (idx >> 5) * kTP + (idx & 31)] = Ps[(idx >> 5) * 36 + (idx & 31)];
     }
 }
 
@@ -264,70 +267,99 @@ __device__ __forceinline__ void cp16(void *smem, const void *gmem) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// What bounds it: shared memory.  Per chunk the products are (2 or 3) x 32 x DK x 16 multiply-adds of operands that are used once, so they are shared out by how
-// little each reads again:
-//   read   [Kp; Qp] S   a warp takes 8 columns and a quarter of the rows; 16 lanes share a row, a lane holds its DK / 16 rows of S for the 8 columns in
-//                       registers and reads each row of the factors once; eight shuffles fold the lanes' sums into one column per lane pair
-//   solve  Tb R, P u    a thread takes a token and two columns, over the tokens up to its own
-//   update S            a warp takes 16 rows of S, a lane 2 rows x 4 columns in registers for the whole portion: S <- p_C S, then one multiply-add per token in
-//                       the tokens' order (the decayed, smaller ones first), and S^T goes to shared memory for the next read
-// One stage of the block: its first part (Qp, Kp, V) is free behind the read and the second (the rest) behind the update, so either arrives while the other
-// is used, and two CTAs share an SM.
-template <typename TQ, int DK, bool DELTA> struct Scan {
+// What bounds it: fp32 multiply-adds and shared memory, about evenly: per chunk (2 or 3) x 32 x DK x 16 multiply-adds and as many again for the update, of
+// operands that are used once.  Products are thread tiles, so that an operand read serves four multiply-adds:
+//   read   [Kp; Qp] S   4 rows x 4 columns per thread over a quarter of k (linear attention: an eighth, and P V joins as 32 more k), four lanes' sums folded
+//                       into four outputs of each
+//   solve  Tb R, P u    a token and two columns per thread, over the tokens up to its own
+//   update S            4 rows x 2 columns per thread, held in registers for the whole portion: S <- p_C S, then one multiply-add per token in the tokens'
+//                       order (the decayed, smaller ones first), and S^T goes to shared memory for the next read
+// A warp's 16-byte reads have at most eight addresses in each half, on different banks (pitches of 8 or 4 modulo 32 floats).  Linear attention's read and
+// update touch different copies of S^T, so a chunk has two barriers; its factors have two stages.  The delta rule has three barriers and one stage, whose first
+// part (Qp, Kp) is free behind the read and the second (the rest) behind the update, so either arrives while the other is used.  Two CTAs share an SM.
+// Measured (the sizes above): 218 and 212 us; a row of the factors at a time, folded by eight shuffles, 16-byte reads that shared no addresses between
+// neighbouring lanes, values waited for within their chunk and factors copied row by row: 326 and 289 us.  Linear attention with read and update in different
+// warps of one CTA: 209 us, but 238 against 220 (with the factors) for four portions of 1024.
+template <int DK, bool DELTA> struct Scan {
     using B = Block<DK, DELTA>;
-    static constexpr int kSP = DK + 4;                             // floats per column of S^T
-    static constexpr int kUP = 20;                                 // floats per token of R, u, Qp S
-    static constexpr int kVP = sizeof(TQ) == 2 ? 24 : 20;          // elements per staged value row
-    static constexpr int kV = B::kFloats, kS = kV + kC * kVP * (int)sizeof(TQ) / 4, kR = kS + kCols * kSP, kQ = kR + kC * kUP, kU = kQ + kC * kUP;
-    static constexpr int kFloats = kU + kC * kUP;                  // of shared memory
+    static constexpr int kP = B::kP, kStage = B::kFloats;
+    static constexpr int kStages = DELTA ? 1 : 2;
+    static constexpr int KW = DELTA ? 1 : DK / 64;      // warps that share the k of a row group (linear attention)
+    static constexpr int kS = kStages * kStage, kV = kS + kStages * kCols * kP, kR = kV + kStages * kCols * kTP;
+    static constexpr int kUP = 36;                      // floats per column of R^T, (Qp S)^T, u^T: 4 banks apart, for eight columns at a time
+    static constexpr int kPart = 20;                    // floats per token of the partial outputs
+    static constexpr int kFloats = kR + (DELTA ? 3 * kCols * kUP : KW * kC * kPart);
 };
 
 template <typename TQ, int DK, bool DELTA>
 __global__ void __launch_bounds__(DK * 2, 2)
 chunk_scan_kernel(const ChunkSource src, const ChunkMap map, const float *__restrict__ blocks, float *__restrict__ state, float *__restrict__ o) {
-    using Sh = Scan<TQ, DK, DELTA>;
+    using Sh = Scan<DK, DELTA>;
     using B = Block<DK, DELTA>;
-    constexpr int NT = DK * 2, NW = NT / 32, KJ = DK / 64;    // threads, warps, 16-byte pieces of a row per lane
-    constexpr int ROWS = DELTA ? 2 * kC : kC, PER = ROWS / (NW / 2);  // rows of [Kp; Qp], of a warp
+    constexpr int NT = DK * 2, NW = NT / 32, P = Sh::kP, TP = kTP, UP = Sh::kUP, RW = DK / 32;  // threads, warps, pitches, warps that share the rows of S
     extern __shared__ __align__(16) float sm[];
-    TQ *vs = reinterpret_cast<TQ *>(sm + Sh::kV);
-    float *St = sm + Sh::kS, *R = sm + Sh::kR, *Qs = sm + Sh::kQ, *U = sm + Sh::kU;
+    float *const St = sm + Sh::kS, *const VT = sm + Sh::kV, *const RT = sm + Sh::kR, *const QT = RT + kCols * UP, *const UT = QT + kCols * UP;
     const int s = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * kCols;
     const int start = map.seq_start[s], len = map.seq_start[s + 1] - start;
     if (len < map.min_tokens || map.first * kC >= len) return;
     const int n_chunks = min(map.count, (len + kC - 1) / kC - map.first);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const float *blk = blocks + ((size_t)block_base(map, s) * map.heads + h) * B::kFloats;
-    auto load = [&](int c, int from, int to) {
-        const float *b = blk + (size_t)c * map.heads * B::kFloats;
-        for (int i = from / 4 + tid; i < to / 4; i += NT) cp16(sm + 4 * i, b + 4 * i);
+    // floats [from, to) of chunk c's block into its stage
+    auto load = [&](int c, auto from, auto to) {
+        constexpr int at = decltype(from)::value, n = (decltype(to)::value - at) / 4;
+        const float *b = blk + (size_t)c * map.heads * B::kFloats + at + 4 * tid;
+        float *st = sm + (c % Sh::kStages) * Sh::kStage + at + 4 * tid;
+#pragma unroll
+        for (int i = 0; i < (n + NT - 1) / NT; ++i)
+            if ((i + 1) * NT <= n || tid + i * NT < n) cp16(st + 4 * i * NT, b + 4 * i * NT);
     };
-    auto load_first = [&](int c) {
-        load(c, 0, B::kKe);
-        constexpr int per = kCols * (int)sizeof(TQ) / 16;      // 16-byte pieces per value row
-        for (int i = tid; i < kC * per; i += NT) {
-            const int t = min((map.first + c) * kC + i / per, len - 1), e = i % per * (16 / (int)sizeof(TQ));  // past the end: a live row, which no key meets
-            cp16(vs + (i / per) * Sh::kVP + e, static_cast<const TQ *>(src.rows) + (size_t)(start + t) * src.ld + src.v_off + h * map.vdim + j0 + e);
+    constexpr std::integral_constant<int, 0> first{};          // (delta rule: the parts of a block, see below)
+    constexpr std::integral_constant<int, B::kKe> second{};
+    constexpr std::integral_constant<int, B::kFloats> end{};
+    // values: a thread's two columns of one or two tokens, on their way in registers for two chunks (32 bytes of every row: one chunk ahead, linear attention
+    // waited for them, 60 of 320 us), then columns of V^T
+    constexpr int VN = kC * 8 / NT;
+    using Pair = typename std::conditional<sizeof(TQ) == 2, uint32_t, float2>::type;
+    Pair vreg[2][VN];  // of this chunk's successor and the one behind it, as they come: a conversion at the load would wait for it
+    auto load_values = [&](int c, Pair (&to)[VN]) {
+#pragma unroll
+        for (int x = 0; x < VN; ++x) {
+            const int t = min((map.first + c) * kC + (tid >> 3) + x * (NT / 8), len - 1);  // past the end: a live row, which no key meets
+            const TQ *v = static_cast<const TQ *>(src.rows) + (size_t)(start + t) * src.ld + src.v_off + h * map.vdim + j0 + 2 * (tid & 7);
+            to[x] = *reinterpret_cast<const Pair *>(v);  // (aligned: rows and segments start on 16-byte boundaries)
         }
-        cp_commit();
     };
-    load_first(0);
-    // this lane's part of S: rows r0, r0 + 1, columns c0 .. c0 + 3
-    const int r0 = 16 * w + 2 * (lane & 7), c0 = 4 * (lane >> 3);
-    float S[2][4], S0[2][4];
-    float *slot = state + ((size_t)map.seq_slot[s] * map.heads + h) * DK * map.vdim + j0;
+    auto put_values = [&](int c, const Pair (&from)[VN]) {
+        float *to = VT + (c % Sh::kStages) * kCols * TP;
+#pragma unroll
+        for (int x = 0; x < VN; ++x) {
+            const int t = (tid >> 3) + x * (NT / 8), e = 2 * (tid & 7);
+            const TQ *v = reinterpret_cast<const TQ *>(&from[x]);
+            to[e * TP + t] = Elem<TQ>::to_f(v[0]), to[(e + 1) * TP + t] = Elem<TQ>::to_f(v[1]);
+        }
+    };
+    if constexpr (DELTA) load(0, first, second);
+    else load(0, first, end);
+    cp_commit();
+    load_values(0, vreg[1]);
+    load_values(1, vreg[0]);
+    put_values(0, vreg[1]);
+    // this lane's part of S: rows r0 .. r0 + 3, columns cp and cp + 8
+    const int r0 = 4 * ((lane >> 1 & 1) + 2 * (lane >> 3) + 8 * (w % RW)), cp = (lane & 1) + 2 * (lane >> 2 & 1) + 4 * (w / RW);
+    float S[4][2], S0[4][2];
+    float *slot = state + ((size_t)map.seq_slot[s] * map.heads + h) * DK * map.vdim + j0 + cp;
     const bool fresh = map.first == 0 && map.seq_pos0[s] == 0;
 #pragma unroll
-    for (int x = 0; x < 2; ++x)
+    for (int x = 0; x < 4; ++x)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[x][e] = fresh ? 0.0f : slot[(size_t)(r0 + x) * map.vdim + c0 + e];
-    auto publish = [&]() {
+        for (int e = 0; e < 2; ++e) S[x][e] = fresh ? 0.0f : slot[(size_t)(r0 + x) * map.vdim + 8 * e];
+    auto publish = [&](int c) {  // for chunk c to read
+        float *to = St + (c % Sh::kStages) * kCols * P;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) *reinterpret_cast<float2 *>(St + (c0 + e) * Sh::kSP + r0) = make_float2(S[0][e], S[1][e]);
+        for (int e = 0; e < 2; ++e) *reinterpret_cast<float4 *>(to + (cp + 8 * e) * P + r0) = make_float4(S[0][e], S[1][e], S[2][e], S[3][e]);
     };
-    publish();
-    const int t = tid / 8 % kC, cp = 2 * (tid & 7);            // a thread's token and columns of the solve (64-row states: of half the tokens)
-    constexpr int TS = NT / 8;                                 // tokens per pass of the solve
+    publish(0);
 
     // The products multiply a token's vectors with those of the whole chunk, by zero where one must not see the other: an infinity or a NaN could reach what
     // came before it (0 x inf), and P and Tb gather sums that the serial kernels form token by token.  A chunk whose state or read-outs are not all finite
@@ -335,183 +367,251 @@ chunk_scan_kernel(const ChunkSource src, const ChunkMap map, const float *__rest
     bool bad = false;
     auto again = [&](int c) {
         const int hk = h / map.group;
-        auto total = [&](float (&p)[4], float *buf) {          // sums over the rows of S for this lane's columns; buf [NW][kCols]
+        auto total = [&](float (&p)[2], float *buf) {          // sums over the rows of S for this lane's columns; buf [RW][kCols]
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
+            for (int e = 0; e < 2; ++e) {
 #pragma unroll
-                for (int x = 1; x < 8; x <<= 1) p[e] += __shfl_xor_sync(0xffffffffu, p[e], x);
-                if ((lane & 7) == 0) buf[w * kCols + c0 + e] = p[e];
+                for (int x = 2; x < 32; x <<= x == 2 ? 2 : 1) p[e] += __shfl_xor_sync(0xffffffffu, p[e], x);  // (the lane bits of r0: 1, 3, 4)
+                if ((lane & 26) == 0) buf[w % RW * kCols + cp + 8 * e] = p[e];
             }
             __syncthreads();
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
+            for (int e = 0; e < 2; ++e) {
                 p[e] = 0.0f;
-                for (int x = 0; x < NW; ++x) p[e] += buf[x * kCols + c0 + e];
+                for (int x = 0; x < RW; ++x) p[e] += buf[x * kCols + cp + 8 * e];
             }
         };
 #pragma unroll
-        for (int x = 0; x < 2; ++x)
+        for (int x = 0; x < 4; ++x)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) S[x][e] = S0[x][e];
+            for (int e = 0; e < 2; ++e) S[x][e] = S0[x][e];
         for (int tt = (map.first + c) * kC, end = min(len, tt + kC); tt < end; ++tt) {
             const size_t tok = (size_t)(start + tt);
             const TQ *row = static_cast<const TQ *>(src.rows) + tok * src.ld;
             const float *dec = src.decay + tok * src.decay_ld + src.decay_off + (src.decay_dim == 1 ? h : h * DK);
-            float k[2], q[2], p[4] = {}, u[4];
+            float k[4], q[4], p[2] = {}, u[2];
 #pragma unroll
-            for (int x = 0; x < 2; ++x) {
+            for (int x = 0; x < 4; ++x) {
                 k[x] = Elem<TQ>::to_f(row[src.k_off + hk * DK + r0 + x]), q[x] = Elem<TQ>::to_f(row[src.q_off + hk * DK + r0 + x]) * src.q_scale;
                 const float d = src.decay_dim == 1 ? dec[0] : dec[r0 + x];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
+                for (int e = 0; e < 2; ++e) {
                     S[x][e] *= d;
                     p[e] = fmaf(S[x][e], k[x], p[e]);
                 }
             }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) u[e] = Elem<TQ>::to_f(row[src.v_off + h * map.vdim + j0 + c0 + e]);
+            for (int e = 0; e < 2; ++e) u[e] = Elem<TQ>::to_f(row[src.v_off + h * map.vdim + j0 + cp + 8 * e]);
             if (DELTA) {
-                total(p, Qs);
+                total(p, RT + RW * kCols);
                 const float beta = src.beta[tok * src.beta_ld + h];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) u[e] = beta * (u[e] - p[e]);
+                for (int e = 0; e < 2; ++e) u[e] = beta * (u[e] - p[e]);
             }
-            float y[4] = {};
+            float y[2] = {};
 #pragma unroll
-            for (int x = 0; x < 2; ++x)
+            for (int x = 0; x < 4; ++x)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
+                for (int e = 0; e < 2; ++e) {
                     S[x][e] = fmaf(k[x], u[e], S[x][e]);
                     y[e] = fmaf(S[x][e], q[x], y[e]);
                 }
-            total(y, R);
-            if (w == 0 && (lane & 7) == 0) {
+            total(y, RT);
+            if (w % RW == 0 && (lane & 26) == 0) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) o[(tok * map.heads + h) * map.vdim + j0 + c0 + e] = y[e];
+                for (int e = 0; e < 2; ++e) o[(tok * map.heads + h) * map.vdim + j0 + cp + 8 * e] = y[e];
             }
             if (!DELTA) __syncthreads();  // (the delta rule's first sum stands between two uses of the second's places)
         }
-        publish();
+        publish(c + 1);
         __syncthreads();
     };
-    static_assert(NW * kCols <= kC * Sh::kUP, "the sums of `again` fit where the chunk's were");
+    static_assert(2 * RW * kCols <= Sh::kFloats - Sh::kR, "the sums of `again` fit where the chunk's were");
+
+    // sums of 4 rows x 4 columns over this lane's k: a[i] rows of the first operand, b[j] columns of the second, `step` floats from one access to the next
+    auto tile = [&](float2 (&acc)[4][4], const float *const (&a)[4], const float *const (&b)[4], int n, int step) {
+#pragma unroll 4
+        for (int x = 0; x < n; ++x) {
+            float4 f[4], g[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) f[i] = *reinterpret_cast<const float4 *>(a[i] + x * step), g[i] = *reinterpret_cast<const float4 *>(b[i] + x * step);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    acc[i][j] = fma2(make_float2(f[i].z, f[i].w), make_float2(g[j].z, g[j].w), fma2(make_float2(f[i].x, f[i].y), make_float2(g[j].x, g[j].y), acc[i][j]));
+        }
+    };
+    // four lanes (bits 3 and 4) fold their 16 sums: a lane ends with row ks of the tile
+    auto fold4 = [&](const float2 (&acc)[4][4], float (&y)[4]) {
+        const bool hi = lane & 16, lo = lane & 8;
+        float m[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float u = acc[i][j].x + acc[i][j].y, v = acc[2 + i][j].x + acc[2 + i][j].y;
+                m[i][j] = (hi ? v : u) + __shfl_xor_sync(0xffffffffu, hi ? u : v, 16);
+            }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = (lo ? m[1][j] : m[0][j]) + __shfl_xor_sync(0xffffffffu, lo ? m[0][j] : m[1][j], 8);
+    };
+    // A 16-byte access of a warp takes two cycles where lanes share addresses with the lane beside them (bit 0) or the one after it (bit 1), four where they do not
+    // (measured): rows are shared across bit 0, columns across bit 1, and the four lanes of a sum lie eight apart.
+    const int ks = lane >> 3, cg = (lane & 1) + 2 * (lane >> 2 & 1), rg = lane >> 1 & 1;
+    auto row_of = [&](int g, int i) { return 8 * g + rg + 2 * i; };
+    auto col_of = [&](int j) { return cg + 4 * j; };
+    // the delta rule's sums over the sources of a token, row t of `rows` with columns st_c and st_c + 8 of x: a thread's own, over the tokens up to its own.  The
+    // last four hold the largest terms: they come last, behind `base`, one rounding a term (folded with the others, states came out 1.2 to 1.4 times as far from
+    // 64 bits as the serial kernels').  As 4 x 4 tiles over eight lanes this took 2400 instructions of a chunk's 9400 in selects and shuffles.
+    const int st_t = (lane & 1) + 2 * (lane >> 4) + 4 * w, st_c = lane >> 1 & 7;
+    auto solve = [&](const float *rows, const float *x, int t, float2 y) -> float2 {
+        float2 a = make_float2(0.0f, 0.0f), b = a;
+        const int last = t & ~3;
+#pragma unroll 2
+        for (int s4 = 0; s4 < last; s4 += 4) {
+            const float4 f = *reinterpret_cast<const float4 *>(rows + t * TP + s4);
+            const float4 u = *reinterpret_cast<const float4 *>(x + st_c * UP + s4), v = *reinterpret_cast<const float4 *>(x + (st_c + 8) * UP + s4);
+            a = fma2(make_float2(f.z, f.w), make_float2(u.z, u.w), fma2(make_float2(f.x, f.y), make_float2(u.x, u.y), a));
+            b = fma2(make_float2(f.z, f.w), make_float2(v.z, v.w), fma2(make_float2(f.x, f.y), make_float2(v.x, v.y), b));
+        }
+        y.x += a.x + a.y, y.y += b.x + b.y;
+        const float4 f = *reinterpret_cast<const float4 *>(rows + t * TP + last);
+        const float4 u = *reinterpret_cast<const float4 *>(x + st_c * UP + last), v = *reinterpret_cast<const float4 *>(x + (st_c + 8) * UP + last);
+        y = fma2(make_float2(f.x, f.x), make_float2(u.x, v.x), y), y = fma2(make_float2(f.y, f.y), make_float2(u.y, v.y), y);
+        return fma2(make_float2(f.w, f.w), make_float2(u.w, v.w), fma2(make_float2(f.z, f.z), make_float2(u.z, v.z), y));
+    };
 
     for (int c = 0; c < n_chunks; ++c) {
+        const float *const stage = sm + (c % Sh::kStages) * Sh::kStage, *const Sc = St + (c % Sh::kStages) * kCols * P, *const Vc = VT + (c % Sh::kStages) * kCols * TP;
         cp_wait_all();
-        if (__syncthreads_or(bad)) again(c - 1);               // (also: S^T and the first part are there, the second part is free)
+        if (__syncthreads_or(bad)) again(c - 1);               // (also: S^T, V^T and the (first part of the) stage are there; what they replace is free)
         bad = false;
 #pragma unroll
-        for (int x = 0; x < 2; ++x)
+        for (int x = 0; x < 4; ++x)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) S0[x][e] = S[x][e];
-        load(c, B::kKe, B::kFloats);
+            for (int e = 0; e < 2; ++e) S0[x][e] = S[x][e];
+        if constexpr (DELTA) load(c, second, end);
+        else if (c + 1 < n_chunks) load(c + 1, first, end);
         cp_commit();
-        {   // read: rows `half` + 2 i of this warp's, 8 columns
-            const int half = lane >> 4, l16 = lane & 15, cg = 8 * (w & 1);
-            float4 Sr[8][KJ];
+        load_values(c + 2, vreg[1]);
+        // ---- read
+        if constexpr (DELTA) {
+            for (int g = w; g < 2 * kC / 8; g += NW) {         // rows 0 .. kC - 1 are Qp's, then Kp's
+                float2 acc[4][4] = {};
+                const float *a[4], *b[4];
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
+                for (int i = 0; i < 4; ++i) a[i] = stage + row_of(g, i) * P + 4 * ks, b[i] = Sc + col_of(i) * P + 4 * ks;
+                tile(acc, a, b, DK / 16, 16);
+                float y[4];
+                fold4(acc, y);
+                const int row = row_of(g, ks);
 #pragma unroll
-                for (int j = 0; j < KJ; ++j) Sr[e][j] = *reinterpret_cast<const float4 *>(St + (cg + e) * Sh::kSP + 64 * j + 4 * l16);
-            const int col = cg + (lane >> 1 & 4) + (lane >> 1 & 2) + (lane >> 1 & 1);  // the column whose sum this lane ends with
-#pragma unroll 4
-            for (int i = 0; i < PER / 2; ++i) {
-                const int row = (w >> 1) * PER + 2 * i + half;  // (delta rule: rows kC .. are Kp's)
-                float2 a2[8] = {};
-#pragma unroll
-                for (int j = 0; j < KJ; ++j) {
-                    const float4 f = *reinterpret_cast<const float4 *>(sm + B::kQp + row * DK + 64 * j + 4 * l16);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) a2[e] = fma2(make_float2(f.z, f.w), make_float2(Sr[e][j].z, Sr[e][j].w), fma2(make_float2(f.x, f.y), make_float2(Sr[e][j].x, Sr[e][j].y), a2[e]));
-                }
-                float a[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) a[e] = a2[e].x + a2[e].y;
-                const bool b8 = lane & 8, b4 = lane & 4, b2 = lane & 2;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) a[e] = (b8 ? a[e + 4] : a[e]) + __shfl_xor_sync(0xffffffffu, b8 ? a[e] : a[e + 4], 8);
-#pragma unroll
-                for (int e = 0; e < 2; ++e) a[e] = (b4 ? a[e + 2] : a[e]) + __shfl_xor_sync(0xffffffffu, b4 ? a[e] : a[e + 2], 4);
-                a[0] = (b2 ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, b2 ? a[0] : a[1], 2);
-                a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
-                if ((lane & 1) == 0) {
-                    if (DELTA && row >= kC) R[(row - kC) * Sh::kUP + col] = Elem<TQ>::to_f(vs[(row - kC) * Sh::kVP + col]) - a[0];
-                    else Qs[row * Sh::kUP + col] = a[0];
+                for (int j = 0; j < 4; ++j) {
+                    if (row >= kC) RT[col_of(j) * UP + row - kC] = Vc[col_of(j) * TP + row - kC] - y[j];
+                    else QT[col_of(j) * UP + row] = y[j];
                 }
             }
-            if (!DELTA)
-                for (int i = tid; i < kC * kCols; i += NT) U[i / kCols * Sh::kUP + i % kCols] = Elem<TQ>::to_f(vs[i / kCols * Sh::kVP + i % kCols]);
-        }
-        cp_wait_all();
-        __syncthreads();                                       // R, Qp S (and u) are there, so is the second part; the first part is free
-        if (c + 1 < n_chunks) load_first(c + 1);
-        // sums over the tokens up to t of a row of Tb or P with two columns of R or u; `base` joins in front of the last group (see the update)
-        auto solve = [&](const float *rows, const float *x, int tt, float2 base) -> float2 {
-            float2 y = make_float2(0.0f, 0.0f);
-            auto group = [&](int s4) {
-                const float4 f = *reinterpret_cast<const float4 *>(rows + tt * kC + s4);
-                const float ff[4] = {f.x, f.y, f.z, f.w};
+            cp_wait_all();
+            __syncthreads();                                   // R, Qp S are there, so is the second part; Qp, Kp, S^T and V^T are free
+            if (c + 1 < n_chunks) load(c + 1, first, second);
+            cp_commit();
 #pragma unroll
-                for (int e = 0; e < 4; ++e) y = fma2(make_float2(ff[e], ff[e]), *reinterpret_cast<const float2 *>(x + (s4 + e) * Sh::kUP + cp), y);
-            };
-            const int last = tt & ~3;
-#pragma unroll 2
-            for (int s4 = 0; s4 < last; s4 += 4) group(s4);
-            y.x += base.x, y.y += base.y;
-            group(last);
-            return y;
-        };
-        if (DELTA) {
-#pragma unroll
-            for (int tt = t; tt < kC; tt += TS) *reinterpret_cast<float2 *>(U + tt * Sh::kUP + cp) = solve(sm + B::kTb, R, tt, make_float2(0.0f, 0.0f));
+            for (int t = st_t; t < kC; t += 4 * NW) {
+                const float2 u = solve(stage + B::kTb, RT, t, make_float2(0.0f, 0.0f));
+                UT[st_c * UP + t] = u.x, UT[(st_c + 8) * UP + t] = u.y;
+            }
             __syncthreads();
+        } else {
+            constexpr int KW = Sh::KW;
+            const int g = w / KW, kw = w % KW;                 // row group, share of k
+            float2 acc[4][4] = {};
+            const float *a[4], *b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = stage + row_of(g, i) * P + kw * (DK / KW) + 4 * ks, b[i] = Sc + col_of(i) * P + kw * (DK / KW) + 4 * ks;
+            tile(acc, a, b, DK / KW / 16, 16);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = stage + B::kPm + row_of(g, i) * TP + kw * (kC / KW) + 4 * ks, b[i] = Vc + col_of(i) * TP + kw * (kC / KW) + 4 * ks;
+            tile(acc, a, b, kC / KW / 16, 16);
+            float y[4];
+            fold4(acc, y);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) RT[(kw * kC + row_of(g, ks)) * Sh::kPart + col_of(j)] = y[j];
         }
-        {   // update
-            // all but the last four of the chunk's tokens are added up apart from the state: with decays near 1 their sum is smaller than it and so are its
+        {   // ---- update
+            // all but the chunk's last (up to four) tokens are added up apart from the state: with decays near 1 their sum is smaller than it and so are its
             // roundings, with strong ones the last tokens are nearly all of it and round once
-            const int live = min(kC, len - (map.first + c) * kC), apart = max(live - 4, 0);
+            const int last = (min(kC, len - (map.first + c) * kC) - 1) & ~3;  // (tokens past the end: keys of zero)
+            constexpr int VP = DELTA ? UP : TP;
+            const float *const Ke = stage + B::kKe + r0, *const U = DELTA ? UT : Vc;
             float2 d[2][2] = {};
-            auto add = [&](int x, float2 (&to)[2][2]) {
-                const float2 k = *reinterpret_cast<const float2 *>(sm + B::kKe + x * DK + r0);
-                const float4 u = *reinterpret_cast<const float4 *>(U + x * Sh::kUP + c0);
-                const float2 k0 = make_float2(k.x, k.x), k1 = make_float2(k.y, k.y), lo = make_float2(u.x, u.y), hi = make_float2(u.z, u.w);
-                to[0][0] = fma2(k0, lo, to[0][0]), to[0][1] = fma2(k0, hi, to[0][1]);
-                to[1][0] = fma2(k1, lo, to[1][0]), to[1][1] = fma2(k1, hi, to[1][1]);
+            auto add = [&](int x) {
+                const float4 u0 = *reinterpret_cast<const float4 *>(U + cp * VP + x), u1 = *reinterpret_cast<const float4 *>(U + (cp + 8) * VP + x);
+                const float a0[4] = {u0.x, u0.y, u0.z, u0.w}, a1[4] = {u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float4 k = *reinterpret_cast<const float4 *>(Ke + (x + i) * P);
+                    const float2 lo = make_float2(k.x, k.y), hi = make_float2(k.z, k.w), v0 = make_float2(a0[i], a0[i]), v1 = make_float2(a1[i], a1[i]);
+                    d[0][0] = fma2(lo, v0, d[0][0]), d[0][1] = fma2(hi, v0, d[0][1]);
+                    d[1][0] = fma2(lo, v1, d[1][0]), d[1][1] = fma2(hi, v1, d[1][1]);
+                }
             };
-#pragma unroll 4
-            for (int x = 0; x < apart; ++x) add(x, d);
-            const float2 p = *reinterpret_cast<const float2 *>(sm + B::kG + r0);
+#pragma unroll 2
+            for (int x = 0; x < last; x += 4) add(x);
+            const float4 p = *reinterpret_cast<const float4 *>(stage + B::kG + r0);
 #pragma unroll
-            for (int x = 0; x < 2; ++x)
+            for (int e = 0; e < 2; ++e) {
+                d[e][0] = fma2(make_float2(p.x, p.y), make_float2(S[0][e], S[1][e]), d[e][0]);
+                d[e][1] = fma2(make_float2(p.z, p.w), make_float2(S[2][e], S[3][e]), d[e][1]);
+            }
+            add(last);
 #pragma unroll
-                for (int e = 0; e < 2; ++e) d[x][e] = fma2(make_float2(x ? p.y : p.x, x ? p.y : p.x), make_float2(S[x][2 * e], S[x][2 * e + 1]), d[x][e]);
-#pragma unroll 4
-            for (int x = apart; x < live; ++x) add(x, d);
+            for (int e = 0; e < 2; ++e) S[0][e] = d[e][0].x, S[1][e] = d[e][0].y, S[2][e] = d[e][1].x, S[3][e] = d[e][1].y;
 #pragma unroll
-            for (int x = 0; x < 2; ++x)
+            for (int x = 0; x < 4; ++x)
 #pragma unroll
-                for (int e = 0; e < 2; ++e) S[x][2 * e] = d[x][e].x, S[x][2 * e + 1] = d[x][e].y;
+                for (int e = 0; e < 2; ++e) bad |= !(fabsf(S[x][e]) < INFINITY);
+            publish(c + 1);
+            if (c + 1 < n_chunks) put_values(c + 1, vreg[0]);
 #pragma unroll
-            for (int x = 0; x < 2; ++x)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) bad |= !(fabsf(S[x][e]) < INFINITY);
-            publish();
+            for (int x = 0; x < VN; ++x) vreg[0][x] = vreg[1][x];
         }
+        // ---- read-outs
+        auto finite = [&](float2 y) { return fabsf(y.x) < INFINITY && fabsf(y.y) < INFINITY; };
+        auto out = [&](int t) { return o + ((size_t)(start + (map.first + c) * kC + t) * map.heads + h) * map.vdim + j0; };
+        const int live = min(kC, len - (map.first + c) * kC);
+        if constexpr (DELTA) {
 #pragma unroll
-        for (int tt = t; tt < kC; tt += TS) {                  // read-outs
-            const float2 y = solve(sm + B::kP, U, tt, *reinterpret_cast<const float2 *>(Qs + tt * Sh::kUP + cp));
-            const int at = (map.first + c) * kC + tt;
-            if (at < len) {
-                *reinterpret_cast<float2 *>(o + ((size_t)(start + at) * map.heads + h) * map.vdim + j0 + cp) = y;
-                bad |= !(fabsf(y.x) < INFINITY) || !(fabsf(y.y) < INFINITY);
+            for (int t = st_t; t < kC; t += 4 * NW) {
+                const float2 y = solve(stage + B::kPm, UT, t, make_float2(QT[st_c * UP + t], QT[(st_c + 8) * UP + t]));
+                if (t < live) {
+                    out(t)[st_c] = y.x, out(t)[st_c + 8] = y.y;
+                    bad |= !finite(y);
+                }
+            }
+        } else {
+            __syncthreads();                                   // the partial sums are there
+#pragma unroll
+            for (int x = 0; x < VN; ++x) {
+                const int t = (tid >> 3) + x * (NT / 8), e = 2 * (tid & 7);
+                float2 y = *reinterpret_cast<const float2 *>(RT + t * Sh::kPart + e);
+#pragma unroll
+                for (int kw = 1; kw < Sh::KW; ++kw) {
+                    const float2 z = *reinterpret_cast<const float2 *>(RT + (kw * kC + t) * Sh::kPart + e);
+                    y.x += z.x, y.y += z.y;
+                }
+                if (t < live) {
+                    *reinterpret_cast<float2 *>(out(t) + e) = y;
+                    bad |= !finite(y);
+                }
             }
         }
     }
     if (__syncthreads_or(bad)) again(n_chunks - 1);
 #pragma unroll
-    for (int x = 0; x < 2; ++x)
+    for (int x = 0; x < 4; ++x)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) slot[(size_t)(r0 + x) * map.vdim + c0 + e] = S[x][e];
+        for (int e = 0; e < 2; ++e) slot[(size_t)(r0 + x) * map.vdim + 8 * e] = S[x][e];
 }
 
 template <typename TQ, int DK, bool DELTA>
@@ -524,7 +624,7 @@ int launch_chunks_t(const ChunkSource &src, ChunkMap map, float *scratch, size_t
     map.count = map.packed ? chunks : (int)std::min<size_t>(fit / n_seqs, chunks);
     if (map.count == 0) return B200_ERR_UNSUPPORTED;
     const size_t smem_f = (size_t)(3 * kC * (DK + 4) + 2 * kC * 36 + 4 * DK + kC) * sizeof(float);
-    const size_t scan_smem = Scan<TQ, DK, DELTA>::kFloats * sizeof(float);
+    const size_t scan_smem = Scan<DK, DELTA>::kFloats * sizeof(float);
     auto fk = chunk_factors_kernel<TQ, DK, DELTA>;
     auto sk = chunk_scan_kernel<TQ, DK, DELTA>;
     cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f);

@@ -180,6 +180,14 @@ def test_no_further_from_64_bits_than_the_serial_kernels(kind, dim, decays, lens
     assert all(c <= 1.05 * s for s, c in zip(*errors)), errors
 
 
+@pytest.mark.parametrize("kind", ["gla", "delta", "linear"])
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("tail", [1, 2, 3, 4, 5, 8, 27, 28, 29, 31, 32, 33])
+def test_last_chunks_of_every_length(kind, dim, tail):
+    """The scan's update takes tokens in fours and the last four apart: portions that end anywhere in a chunk, beside one that ends with it."""
+    test_no_further_from_64_bits_than_the_serial_kernels(kind, dim, "mixed", (96 + tail, 64))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
 @pytest.mark.parametrize("rank", [32, 64, 256])
 def test_decays_on_the_tensor_cores(dtype, rank):
