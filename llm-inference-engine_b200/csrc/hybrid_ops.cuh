@@ -221,6 +221,15 @@ constexpr int kMoeTileM = 64;  // rows of one expert are padded to whole tiles o
 // n_tiles: device int.
 int launch_moe_plan(const int *sel_expert, const float *sel_weight, int *row_token, float *row_weight, int *tile_expert, int *pair_row,
                     int *n_tiles, int tokens, int experts, int top, int tile, cudaStream_t st);
+// launch_moe_route_sigmoid and launch_moe_plan in one, for prompts; `counts`: moe_route_plan_bytes of scratch.  B200_ERR_UNSUPPORTED: take the two
+size_t moe_route_plan_bytes(int tokens, int experts);
+int launch_moe_route_plan(const float *logits, int ld, int *sel_expert, float *sel_weight, float *shared_gate, int *counts, int *row_token, float *row_weight,
+                          int *tile_expert, int *pair_row, int *n_tiles, int tokens, int experts, int top, int tile, cudaStream_t st);
+// launch_moe_route_sigmoid, launch_moe_plan and launch_moe_gather in one, for a decode batch whose experts run in moe_few_rows_kernel: of every tile only the
+// first tile_live rows are written.  B200_ERR_UNSUPPORTED: take the three
+int launch_moe_few_plan(int dtype, const float *logits, int ld, const float *x, void *xg, int *pair_row, int *tile_expert, int *tile_live, int *n_tiles,
+                        float *shared_gate, int tokens, int experts, int top, int width, cudaStream_t st);
+bool moe_few_rows_takes(int dtype, int live_rows, int N, int K, const void *a, const void *w);
 // xg[row, :] = T(weight[row] * x[token[row], :]) (zeros for padding rows): the routing weight multiplies the expert's INPUT
 int launch_moe_gather(int dtype, const float *x, const int *row_token, const float *row_weight, void *xg, const int *n_tiles,
                       int max_rows, int width, int tile, cudaStream_t st);
@@ -239,9 +248,9 @@ int launch_bias_activation(int dtype, void *x, const float *bias, size_t rows, i
 int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, int N, int K, int experts, const int *tile_expert,
                            const int *n_live, int act, int dtype, cudaStream_t st);
 // c[row, n] = act?(sum_k a[row, k] * w[tile_expert[row / kMoeTileM]][n, k]);  rows >= n_tiles * kMoeTileM are skipped
-// live_rows: rows at the head of every tile that a caller reads afterwards (the others may stay unwritten)
+// live_rows: rows at the head of every tile that a caller reads afterwards (the others may stay unwritten); tile_live (moe_few_rows_takes): each tile's own number
 int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, const int *tile_expert, const int *n_tiles, int max_tiles,
-                            int N, int K, int act, cudaStream_t st, int live_rows = kMoeTileM);
+                            int N, int K, int act, cudaStream_t st, int live_rows = kMoeTileM, const int *tile_live = nullptr);
 // y fp32 [M, N] = x [M, K] * w[N, K]^T for 16-bit x and w on the tensor cores (fp32 accumulation, fp32 result); B200_ERR_UNSUPPORTED for
 // fp32 engines and K not a multiple of 8 (the caller falls back to launch_proj_f32)
 int launch_dense_f32out(int dtype, const void *x, const void *w, float *y, int M, int N, int K, cudaStream_t st);

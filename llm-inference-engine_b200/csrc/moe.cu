@@ -173,6 +173,205 @@ moe_plan_kernel(const int *__restrict__ sel_expert, const float *__restrict__ se
     }
 }
 
+// The `top` largest of a token's logits by one warp, the smaller index first among equals, as moe_route_sigmoid_kernel chooses: z[j] is logit lane + 32 j
+// (a NaN, and what is past the last expert, is never chosen; with nothing left to choose the index is 0x7fffffff and the weight that of -inf).  Logits in an
+// order that unsigned integers keep, so that a choice is two reductions in hardware and not five rounds of two shuffles.
+template <int J, typename Put>
+__device__ __forceinline__ void choose_sigmoid(const float (&z)[J], int lane, int experts, int top, Put put) {
+    unsigned key[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const unsigned b = __float_as_uint(z[j] + 0.0f);  // (-0 and +0 are equal)
+        key[j] = lane + 32 * j < experts && z[j] == z[j] ? ((b & 0x80000000u) ? ~b : b | 0x80000000u) : 0u;
+    }
+    for (int k = 0; k < top; ++k) {
+        unsigned mine = key[0];
+#pragma unroll
+        for (int j = 1; j < J; ++j) mine = max(mine, key[j]);
+        const unsigned best = __reduce_max_sync(0xffffffffu, mine);
+        unsigned at = 0x7fffffffu;
+#pragma unroll
+        for (int j = J - 1; j >= 0; --j)
+            if (best != 0u && key[j] == best) at = lane + 32 * j;
+        at = __reduce_min_sync(0xffffffffu, at);
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+            if (lane + 32 * j == (int)at) key[j] = 0u;
+        const float v = best == 0u ? -INFINITY : __uint_as_float((best & 0x80000000u) ? best & 0x7fffffffu : ~best);
+        put(k, (int)at, 1.0f / (1.0f + expf(-v)));  // sigmoid is monotone: the largest logit has the largest score
+    }
+}
+
+// A decode batch (at most 16 tokens, 128 choices, 256 experts): choice, plan and gather in one launch.  Every CTA chooses for all tokens -- 16 rows of logits, a
+// microsecond -- and knows the plan from that alone: an expert that was chosen owns one tile, in the experts' order, its rows are its pairs in order.  CTA b
+// gathers tile b, its live rows only (moe_few_rows_kernel reads no others).  Bound: latency, one chain of logits -> rows.
+// Measured (16 tokens, 4 of 32 experts, width 2048): three launches 5.4 + 6.1 + 4.3 us -> 7.5.
+constexpr int kFewTokens = 16, kFewPairs = 128, kFewExperts = 256;
+template <typename T>
+__global__ void __launch_bounds__(256)
+moe_few_plan_kernel(const float *__restrict__ logits, int ld, const float *__restrict__ x, T *__restrict__ xg, int *__restrict__ pair_row,
+                    int *__restrict__ tile_expert, int *__restrict__ tile_live, int *__restrict__ n_tiles, float *__restrict__ shared_gate, int tokens, int experts,
+                    int top, int width) {
+    __shared__ __align__(16) int sel[kFewPairs];
+    __shared__ int list[kFewPairs];
+    __shared__ float weight[kFewPairs];
+    __shared__ unsigned chosen[kFewExperts / 32];
+    __shared__ int live;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pairs = tokens * top;
+    constexpr int J = kFewExperts / 32, V = Elem<T>::kVec;
+    float z[2][J];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < J; ++j) z[i][j] = warp + 8 * i < tokens && lane + 32 * j < experts ? logits[(size_t)(warp + 8 * i) * ld + lane + 32 * j] : 0.0f;
+    if (threadIdx.x < kFewPairs) sel[threadIdx.x] = -1;
+    if (threadIdx.x < kFewExperts / 32) chosen[threadIdx.x] = 0u;
+    if (threadIdx.x == 0) live = 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        if (warp + 8 * i < tokens)
+            choose_sigmoid(z[i], lane, experts, top, [&](int k, int e, float w) {
+                if (lane == 0) {
+                    sel[(warp + 8 * i) * top + k] = e, weight[(warp + 8 * i) * top + k] = w;
+                    if (e < experts) atomicOr(&chosen[e >> 5], 1u << (e & 31));
+                }
+            });
+    __syncthreads();
+    auto tile_of = [&](int e) {  // experts chosen before e
+        int n = __popc(chosen[e >> 5] & ((1u << (e & 31)) - 1u));
+        for (int q = 0; q < e >> 5; ++q) n += __popc(chosen[q]);
+        return n;
+    };
+    const int p = threadIdx.x;
+    if (p < pairs) {
+        const int e = sel[p];
+        int rank = 0, count = 0;
+#pragma unroll 8
+        for (int q = 0; q < pairs; q += 4) {
+            const int4 v = *reinterpret_cast<const int4 *>(sel + q);
+            const int same[4] = {v.x == e, v.y == e, v.z == e, v.w == e};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) rank += q + i < p ? same[i] : 0, count += same[i];
+        }
+        const int tile = e < experts ? tile_of(e) : -1;
+        if (tile == (int)blockIdx.x) list[rank] = p, live = count;
+        if (blockIdx.x == 0) {
+            pair_row[p] = tile >= 0 ? tile * kMoeTileM + rank : -1;
+            if (tile >= 0 && rank == 0) tile_expert[tile] = e, tile_live[tile] = count;
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        int n = 0;
+        for (int q = 0; q < kFewExperts / 32; ++q) n += __popc(chosen[q]);
+        *n_tiles = n;
+    }
+    if (blockIdx.x == 0 && shared_gate && threadIdx.x < tokens) shared_gate[threadIdx.x] = 1.0f / (1.0f + expf(-logits[(size_t)threadIdx.x * ld + experts]));
+    __syncthreads();
+    for (int r0 = 0; r0 < live; r0 += 4) {  // four rows in flight
+        for (int c = threadIdx.x * V; c < width; c += 256 * V) {
+            float f[4][V];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (r0 + i < live) load_vec<V>(x + (size_t)(list[r0 + i] / top) * width + c, f[i]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (r0 + i < live) {
+                    const float w = weight[list[r0 + i]];
+#pragma unroll
+                    for (int e = 0; e < V; ++e) f[i][e] *= w;
+                    st_v4(xg + ((size_t)blockIdx.x * kMoeTileM + r0 + i) * width + c, pack16<T>(f[i]));
+                }
+        }
+    }
+}
+
+// Prompts: choice and count, then the plan, each by many CTAs.  A CTA chooses for kRouteTokens tokens and leaves its count per expert; a CTA of the plan adds up the
+// counts of all (a few KB), so it knows where every expert starts and where its own pairs of it go.  The order of an expert's rows is free.  Measured (4096
+// tokens, 4 of 32 experts): choice by a warp per token and the plan of one CTA (moe_plan_kernel) 7.6 + 21 us -> 7.1 + 7.3.
+constexpr int kRouteTokens = 32, kRouteExperts = 128;
+__global__ void __launch_bounds__(256)
+moe_route_count_kernel(const float *__restrict__ logits, int ld, int *__restrict__ sel_expert, float *__restrict__ sel_weight, float *__restrict__ shared_gate,
+                       int *__restrict__ counts, int tokens, int experts, int top) {
+    __shared__ int count[kRouteExperts];
+    constexpr int J = kRouteExperts / 32, PER = kRouteTokens / 8;
+    const int lane = threadIdx.x & 31, first = blockIdx.x * kRouteTokens + (threadIdx.x >> 5) * PER;
+    float z[PER][J], gate = 0.0f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+#pragma unroll
+        for (int j = 0; j < J; ++j) z[i][j] = first + i < tokens && lane + 32 * j < experts ? logits[(size_t)(first + i) * ld + lane + 32 * j] : 0.0f;
+    if (shared_gate && lane < PER && first + lane < tokens) gate = logits[(size_t)(first + lane) * ld + experts];
+    for (int e = threadIdx.x; e < experts; e += 256) count[e] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+        if (first + i < tokens)
+            choose_sigmoid(z[i], lane, experts, top, [&](int k, int e, float w) {
+                if (lane == 0) {
+                    sel_expert[(size_t)(first + i) * top + k] = e, sel_weight[(size_t)(first + i) * top + k] = w;
+                    if (e < experts) atomicAdd(&count[e], 1);
+                }
+            });
+    if (shared_gate && lane < PER && first + lane < tokens) shared_gate[first + lane] = 1.0f / (1.0f + expf(-gate));
+    __syncthreads();
+    for (int e = threadIdx.x; e < experts; e += 256) counts[(size_t)blockIdx.x * experts + e] = count[e];
+}
+__global__ void __launch_bounds__(256)
+moe_place_kernel(const int *__restrict__ sel_expert, const float *__restrict__ sel_weight, const int *__restrict__ counts, int *__restrict__ row_token,
+                 float *__restrict__ row_weight, int *__restrict__ tile_expert, int *__restrict__ pair_row, int *__restrict__ n_tiles, int pairs, int experts, int top,
+                 int tile) {
+    __shared__ int total[kRouteExperts], next[kRouteExperts], offset[kRouteExperts + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, blocks = gridDim.x;
+    for (int e = threadIdx.x; e < experts; e += 256) total[e] = next[e] = 0;
+    __syncthreads();
+    for (int i0 = threadIdx.x; i0 < blocks * experts; i0 += 8 * 256) {  // (eight loads in flight)
+        int v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = i0 + 256 * u < blocks * experts ? counts[i0 + 256 * u] : 0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (v[u] > 0) {
+                const int b = (i0 + 256 * u) / experts, e = i0 + 256 * u - b * experts;
+                atomicAdd(&total[e], v[u]);
+                if (b < (int)blockIdx.x) atomicAdd(&next[e], v[u]);
+            }
+    }
+    __syncthreads();
+    if (warp == 0) {  // first row of every expert: a running sum of whole tiles
+        int at = 0;
+        for (int e0 = 0; e0 < experts; e0 += 32) {
+            const int rows = e0 + lane < experts ? (total[e0 + lane] + tile - 1) / tile * tile : 0;
+            int sum = rows;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += up;
+            }
+            if (e0 + lane < experts) offset[e0 + lane] = at + sum - rows;
+            at += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) offset[experts] = at;
+        if (lane == 0 && blockIdx.x == 0) *n_tiles = at / tile;
+    }
+    __syncthreads();
+    for (int e = blockIdx.x + blocks * warp; e < experts; e += blocks * 8) {
+        const int first = offset[e], end = offset[e + 1];
+        for (int i = first / tile + lane; i < end / tile; i += 32) tile_expert[i] = e;
+        for (int r = first + total[e] + lane; r < end; r += 32) row_token[r] = -1, row_weight[r] = 0.0f;  // padding
+    }
+    const int lo = blockIdx.x * kRouteTokens * top, hi = min(pairs, lo + kRouteTokens * top);
+    for (int p = lo + threadIdx.x; p < hi; p += 256) {
+        const int e = sel_expert[p];
+        const float w = sel_weight[p];
+        if (e < experts) {
+            const int r = offset[e] + atomicAdd(&next[e], 1);
+            row_token[r] = p / top, row_weight[r] = w, pair_row[p] = r;
+        } else {
+            pair_row[p] = -1;
+        }
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128)
 moe_gather_kernel(const float *__restrict__ x, const int *__restrict__ row_token, const float *__restrict__ row_weight, T *__restrict__ xg,
@@ -529,58 +728,63 @@ moe_grouped_gemm_mma_kernel(const T *__restrict__ a, const T *__restrict__ w, TC
 // operands: a lane's 8 consecutive k are its fragments of two k-steps), the next unit's pieces in flight while it multiplies this one's.  KS warps share a
 // unit's k and meet in shared memory, NG units of a CTA run side by side (5 to 16 warps).
 // grid (unit groups, tiles); a CTA runs `steps` groups of NG units of 8 rows.  NT 1: at most 8 live rows, 2: at most 16.  A tile's rows start at its
-// number times tile_rows; rows >= M are neither read nor stored.  tile_expert and n_tiles NULL: one weight, every tile of the grid.
-// Measured (2048 x 512 experts, 16 tokens x 4 of 32, 59 MB): up and down 40 and 30 -> 19 us each.
+// number times tile_rows; rows >= M, or from tile_live on (a 16-row read of every CTA was 40 % of what it took from L2 beside its weights), are neither read nor
+// stored.  tile_expert and n_tiles NULL: one weight, every tile of the grid.
+// Measured (2048 x 512 experts, 16 tokens x 4 of 32, 59 MB): up and down 40 and 30 -> 19 us each; live rows only, eight at a time, CTAs of one wave: 14.5.
 template <typename T, typename TC, int NT>
 __global__ void __launch_bounds__(512)
 moe_few_rows_kernel(const T *__restrict__ a, const T *__restrict__ w, TC *__restrict__ c, const int *__restrict__ tile_expert,
-                    const int *__restrict__ n_tiles, int tile_rows, int M, int N, int K, int act, int KS, int NG, int steps) {
+                    const int *__restrict__ n_tiles, const int *__restrict__ tile_live, int tile_rows, int M, int N, int K, int act, int KS, int NG, int steps) {
     if (n_tiles && (int)blockIdx.y >= *n_tiles) return;
+    const int live = tile_live ? tile_live[blockIdx.y] : min(8 * NT, M - (int)blockIdx.y * tile_rows);
     constexpr int NB = 8;  // 32-k blocks of a slice
     extern __shared__ __align__(16) float part[];  // [2][NG][KS][16 tokens x 8 rows]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int ng = warp / KS, ks = warp - ng * KS, blocks = K / 32;
     const int first = blocks * ks / KS, nb = blocks * (ks + 1) / KS - first;
     const T *wb = w + (tile_expert ? (size_t)tile_expert[blockIdx.y] * N * K : 0) + first * 32 + 8 * t;
-    const int m0 = blockIdx.y * tile_rows;
-    const T *ar = a + (size_t)m0 * K + first * 32 + 8 * t;
     const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
     uint4 av[NB], bv[NT == 2 ? NB : 1], wq[NB];
     auto row_of = [&](int step) {  // this warp's weight row g of the unit; rows past N read the last one, whose result is not stored
         return wb + (size_t)min(((int)blockIdx.x * steps + step) * NG * 8 + ng * 8 + g, N - 1) * K;
     };
-    const T *next = row_of(0);
+    for (int r0 = 0; r0 < live; r0 += 8 * NT) {  // (a second pass over the weights where more than 8 NT of a tile's rows are live)
+        const int m0 = blockIdx.y * tile_rows + r0, rows = live - r0;
+        const T *ar = a + (size_t)m0 * K + first * 32 + 8 * t;
+        const T *next = row_of(0);
 #pragma unroll
-    for (int j = 0; j < NB; ++j) wq[j] = j < nb ? ld_stream_v4(next + 32 * j) : zero4;
-#pragma unroll
-    for (int j = 0; j < NB; ++j) {
-        av[j] = j < nb && m0 + g < M ? ld_v4(ar + (size_t)g * K + 32 * j) : zero4;
-        if constexpr (NT == 2) bv[j] = j < nb && m0 + g + 8 < M ? ld_v4(ar + (size_t)(g + 8) * K + 32 * j) : zero4;
-    }
-    for (int step = 0; step < steps; ++step) {
-        const int unit0 = ((int)blockIdx.x * steps + step) * NG;
-        if (unit0 * 8 >= N) break;
-        float acc[4] = {}, acc2[4] = {};
-        const bool more = step + 1 < steps;
-        next = row_of(step + 1);
+        for (int j = 0; j < NB; ++j) wq[j] = j < nb ? ld_stream_v4(next + 32 * j) : zero4;
 #pragma unroll
         for (int j = 0; j < NB; ++j) {
-            const uint4 b = NT == 2 ? bv[j] : zero4;
-            const unsigned a0[4] = {av[j].x, b.x, av[j].y, b.y}, a1[4] = {av[j].z, b.z, av[j].w, b.w};
-            moe_mma<T>((j & 1) ? acc2 : acc, a0, wq[j].x, wq[j].y);
-            moe_mma<T>((j & 1) ? acc2 : acc, a1, wq[j].z, wq[j].w);
-            if (more && j < nb) wq[j] = ld_stream_v4(next + 32 * j);
+            av[j] = j < nb && g < rows ? ld_v4(ar + (size_t)g * K + 32 * j) : zero4;
+            if constexpr (NT == 2) bv[j] = j < nb && g + 8 < rows ? ld_v4(ar + (size_t)(g + 8) * K + 32 * j) : zero4;
         }
-        float *p = part + (size_t)(step & 1) * NG * KS * 128;
-        float *mine = p + (size_t)(ng * KS + ks) * 128;
-        *reinterpret_cast<float2 *>(mine + g * 8 + 2 * t) = make_float2(acc[0] + acc2[0], acc[1] + acc2[1]);
-        if constexpr (NT == 2) *reinterpret_cast<float2 *>(mine + (g + 8) * 8 + 2 * t) = make_float2(acc[2] + acc2[2], acc[3] + acc2[3]);
-        __syncthreads();  // (two buffers: the next step's shares do not wait for this one's sums)
-        for (int i = threadIdx.x; i < NG * 64 * NT; i += blockDim.x) {
-            const int u = i / (64 * NT), e = i - u * 64 * NT, n = (unit0 + u) * 8 + (e & 7);
-            float v = 0.0f;
-            for (int x = 0; x < KS; ++x) v += p[(size_t)(u * KS + x) * 128 + e];
-            if (n < N && m0 + (e >> 3) < M) c[(size_t)(m0 + (e >> 3)) * N + n] = Elem<TC>::from_f(act >= 0 ? act_apply(v, act) : v);
+        if (r0 > 0) __syncthreads();  // (the last pass's shares have been added up)
+        for (int step = 0; step < steps; ++step) {
+            const int unit0 = ((int)blockIdx.x * steps + step) * NG;
+            if (unit0 * 8 >= N) break;
+            float acc[4] = {}, acc2[4] = {};
+            const bool more = step + 1 < steps;
+            next = row_of(step + 1);
+#pragma unroll
+            for (int j = 0; j < NB; ++j) {
+                const uint4 b = NT == 2 ? bv[j] : zero4;
+                const unsigned a0[4] = {av[j].x, b.x, av[j].y, b.y}, a1[4] = {av[j].z, b.z, av[j].w, b.w};
+                moe_mma<T>((j & 1) ? acc2 : acc, a0, wq[j].x, wq[j].y);
+                moe_mma<T>((j & 1) ? acc2 : acc, a1, wq[j].z, wq[j].w);
+                if (more && j < nb) wq[j] = ld_stream_v4(next + 32 * j);
+            }
+            float *p = part + (size_t)(step & 1) * NG * KS * 128;
+            float *mine = p + (size_t)(ng * KS + ks) * 128;
+            *reinterpret_cast<float2 *>(mine + g * 8 + 2 * t) = make_float2(acc[0] + acc2[0], acc[1] + acc2[1]);
+            if constexpr (NT == 2) *reinterpret_cast<float2 *>(mine + (g + 8) * 8 + 2 * t) = make_float2(acc[2] + acc2[2], acc[3] + acc2[3]);
+            __syncthreads();  // (two buffers: the next step's shares do not wait for this one's sums)
+            for (int i = threadIdx.x; i < NG * 64 * NT; i += blockDim.x) {
+                const int u = i / (64 * NT), e = i - u * 64 * NT, n = (unit0 + u) * 8 + (e & 7);
+                float v = 0.0f;
+                for (int x = 0; x < KS; ++x) v += p[(size_t)(u * KS + x) * 128 + e];
+                if (n < N && (e >> 3) < rows) c[(size_t)(m0 + (e >> 3)) * N + n] = Elem<TC>::from_f(act >= 0 ? act_apply(v, act) : v);
+            }
         }
     }
 }
@@ -595,8 +799,8 @@ int launch_dense_f32out(int dtype, const void *x, const void *w, float *y, int M
         const int KS = (K / 32 + 7) / 8, NG = KS >= 8 ? 1 : 8 / KS, steps = ((N + 7) / 8 + NG - 1) / NG;
         const size_t smem = (size_t)2 * NG * KS * 128 * sizeof(float);
         const dim3 few(1, (M + 15) / 16);
-        if (dtype == B200_BF16) launch_plain(moe_few_rows_kernel<__nv_bfloat16, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
-        else launch_plain(moe_few_rows_kernel<__half, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, (const __half *)x, (const __half *)w, y, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
+        if (dtype == B200_BF16) launch_plain(moe_few_rows_kernel<__nv_bfloat16, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
+        else launch_plain(moe_few_rows_kernel<__half, float, 2>, dim3(few), dim3(KS * NG * 32), smem, st, (const __half *)x, (const __half *)w, y, nullptr, nullptr, nullptr, 16, M, N, K, -1, KS, NG, steps);
         return cuda_status("dense_f32out (few columns) launch");
     }
     const dim3 grid((N + kMN - 1) / kMN, (M + kMoeTileM - 1) / kMoeTileM);
@@ -688,6 +892,26 @@ int launch_moe_plan(const int *sel_expert, const float *sel_weight, int *row_tok
     return cuda_status("moe_plan launch");
 }
 
+int launch_moe_few_plan(int dtype, const float *logits, int ld, const float *x, void *xg, int *pair_row, int *tile_expert, int *tile_live, int *n_tiles,
+                        float *shared_gate, int tokens, int experts, int top, int width, cudaStream_t st) {
+    if (tokens > kFewTokens || tokens * top > kFewPairs || experts > kFewExperts || dtype == B200_F32 || width % 8 != 0 || !all_aligned16({x, xg})) return B200_ERR_UNSUPPORTED;
+    const int tiles = std::min(experts, tokens * top);
+    if (dtype == B200_BF16) launch_plain(moe_few_plan_kernel<__nv_bfloat16>, dim3(tiles), dim3(256), 0, st, logits, ld, x, (__nv_bfloat16 *)xg, pair_row, tile_expert, tile_live, n_tiles, shared_gate, tokens, experts, top, width);
+    else launch_plain(moe_few_plan_kernel<__half>, dim3(tiles), dim3(256), 0, st, logits, ld, x, (__half *)xg, pair_row, tile_expert, tile_live, n_tiles, shared_gate, tokens, experts, top, width);
+    return cuda_status("moe_few_plan launch");
+}
+
+size_t moe_route_plan_bytes(int tokens, int experts) { return (size_t)((tokens + kRouteTokens - 1) / kRouteTokens) * experts * sizeof(int); }
+int launch_moe_route_plan(const float *logits, int ld, int *sel_expert, float *sel_weight, float *shared_gate, int *counts, int *row_token, float *row_weight,
+                          int *tile_expert, int *pair_row, int *n_tiles, int tokens, int experts, int top, int tile, cudaStream_t st) {
+    // (below 512 tokens one CTA plans in less than the second launch's time; a table of more than 64 K counts would be read by every CTA of the plan)
+    const int blocks = (tokens + kRouteTokens - 1) / kRouteTokens;
+    if (tokens < 512 || experts > kRouteExperts || blocks * experts > 65536) return B200_ERR_UNSUPPORTED;
+    launch_plain(moe_route_count_kernel, dim3(blocks), dim3(256), 0, st, logits, ld, sel_expert, sel_weight, shared_gate, counts, tokens, experts, top);
+    launch_plain(moe_place_kernel, dim3(blocks), dim3(256), 0, st, sel_expert, sel_weight, counts, row_token, row_weight, tile_expert, pair_row, n_tiles, tokens * top, experts, top, tile);
+    return cuda_status("moe_route_plan launch");
+}
+
 int launch_moe_gather(int dtype, const float *x, const int *row_token, const float *row_weight, void *xg, const int *n_tiles,
                       int max_rows, int width, int tile, cudaStream_t st) {
     if (max_rows == 0) return B200_OK;
@@ -695,21 +919,25 @@ int launch_moe_gather(int dtype, const float *x, const int *row_token, const flo
     return cuda_status("moe_gather launch");
 }
 
+bool moe_few_rows_takes(int dtype, int live_rows, int N, int K, const void *a, const void *w) {
+    return dtype != B200_F32 && live_rows <= 16 && K % 32 == 0 && K <= 4096 && K >= 64 && N % 8 == 0 && aligned16(a) && aligned16(w);
+}
+
 int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, const int *tile_expert, const int *n_tiles, int max_tiles,
-                            int N, int K, int act, cudaStream_t st, int live_rows) {
+                            int N, int K, int act, cudaStream_t st, int live_rows, const int *tile_live) {
     if (max_tiles == 0) return B200_OK;
     // a decode batch: up to 16 live rows per tile, slices of K for 16 warps at most, whole 32-k blocks
-    if (dtype != B200_F32 && live_rows <= 16 && K % 32 == 0 && K <= 4096 && K >= 64 && N % 8 == 0 && aligned16(a) && aligned16(w)) {
+    if (moe_few_rows_takes(dtype, live_rows, N, K, a, w)) {
         const int KS = (K / 32 + 7) / 8, NG = KS >= 8 ? 1 : 8 / KS;
-        const int units = (N / 8 + NG - 1) / NG, steps = std::max(1, std::min(8, units * max_tiles / (4 * sm_count())));
+        const int units = (N / 8 + NG - 1) / NG, steps = std::max(1, std::min(8, units * max_tiles / (2 * sm_count())));
         const dim3 grid((units + steps - 1) / steps, max_tiles);
         const size_t smem = (size_t)2 * NG * KS * 128 * sizeof(float);
         auto go = [&](auto kern, auto *type) {
             using T = std::remove_pointer_t<decltype(type)>;
-            launch_plain(kern, dim3(grid), dim3(KS * NG * 32), smem, st, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, kMoeTileM, max_tiles * kMoeTileM, N, K, act, KS, NG, steps);
+            launch_plain(kern, dim3(grid), dim3(KS * NG * 32), smem, st, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, tile_live, kMoeTileM, max_tiles * kMoeTileM, N, K, act, KS, NG, steps);
         };
-        if (dtype == B200_BF16) live_rows <= 8 ? go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 1>, (__nv_bfloat16 *)nullptr) : go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 2>, (__nv_bfloat16 *)nullptr);
-        else live_rows <= 8 ? go(moe_few_rows_kernel<__half, __half, 1>, (__half *)nullptr) : go(moe_few_rows_kernel<__half, __half, 2>, (__half *)nullptr);
+        if (dtype == B200_BF16) live_rows <= 8 || tile_live ? go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 1>, (__nv_bfloat16 *)nullptr) : go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 2>, (__nv_bfloat16 *)nullptr);
+        else live_rows <= 8 || tile_live ? go(moe_few_rows_kernel<__half, __half, 1>, (__half *)nullptr) : go(moe_few_rows_kernel<__half, __half, 2>, (__half *)nullptr);
         return cuda_status("moe_few_rows launch");
     }
     if (dtype != B200_F32 && K % 8 == 0) {

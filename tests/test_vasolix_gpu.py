@@ -522,3 +522,37 @@ def test_recurrence_on_both_sides_of_the_token_parallel_rule(heads, schedule):
             total[name] = total.get(name, 0) + n
     req = {name: tokens_of(config, n, 1 + i) for i, (name, n) in enumerate(total.items())}
     check_all(replay(session(config, packed, pool_tokens=2048), req, schedule), config, W, req, 5e-5)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 16])
+@pytest.mark.parametrize("experts,top", [(1, 1), (3, 3), (8, 8), (40, 4), (256, 2)])
+def test_decode_batches_plan_their_experts_in_one_launch(dtype, n, experts, top):
+    """Up to 16 tokens of a 16-bit engine: choice, plan and gather of csrc/moe.cu's moe_few_plan_kernel, experts on their tiles' live rows.  Every expert chosen by
+    every token (up to 16 live rows of a tile: two passes), or a few of many (most tiles one row), against the float64 model."""
+    config = ref.make_config([ref.gla_layer(mlp=ref.moe(experts=experts, top=top, ff=64, shared_ff=64))], width=64)
+    W, packed = ref.make_weights(config, seed=experts)
+    req = {f"r{i}": tokens_of(config, 23, 100 + i) for i in range(n)}
+    sess = session(config, packed, dtype=dtype, pool_tokens=64 * n, max_seqs=n)
+    got = replay(sess, req, [[(k, 20) for k in req]] + [[(k, 1) for k in req]] * 3)
+    for name in req:
+        want = want_logits(config, W, req[name])
+        per_pos = (np.linalg.norm(got[name] - want, axis=-1) / np.linalg.norm(want, axis=-1))[20:]
+        assert np.median(per_pos) < 4e-2, (name, per_pos)
+        if experts == top:  # (no close routing calls)
+            assert per_pos.max() < 0.15, (name, per_pos)
+
+
+@pytest.mark.parametrize("tokens", [511, 512, 513, 900])
+@pytest.mark.parametrize("experts,top", [(3, 3), (32, 4), (33, 1), (128, 8), (129, 2)])
+def test_prompts_plan_their_experts_in_many_ctas(tokens, experts, top):
+    """Prompts on both sides of 512 tokens, expert counts on both sides of a warp's and of the kernel's limit (csrc/moe.cu: moe_route_count_kernel, moe_place_kernel;
+    moe_plan_kernel beyond), the last CTA's tokens partly there; fp32, against the float64 model's residual stream."""
+    config = ref.make_config([ref.gla_layer(mlp=ref.moe(experts=experts, top=top, ff=8, shared_ff=8))])
+    W, packed = ref.make_weights(config, seed=experts)
+    toks = tokens_of(config, tokens, 1)
+    sess = session(config, packed, pool_tokens=1024, max_seqs=1, max_batch_tokens=1024)
+    _, trace = sess.feed([(sess.open(), toks, [tokens - 1])], trace=True)
+    res = []
+    ref.forward(config, W, toks, res)
+    assert ref.rel_err(trace[0].cpu().numpy(), res[0].numpy()) < 2e-5
