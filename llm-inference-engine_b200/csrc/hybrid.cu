@@ -1874,7 +1874,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         const bool weigh_x = !softmax && !sum_norm;  // sigmoid scores weigh the experts' inputs: the fp32 residual row, or (sum_norm) the convolved row the router read
         int *tile_live = nullptr;
         rc = B200_ERR_UNSUPPORTED;
-        if (weigh_x && !l.gated && !tc && moe_few_rows_takes(dt, NT, n_up, width, m->xg, l.w_up) && moe_few_rows_takes(dt, NT, width, l.expert_ff, m->u, l.w_down)) {
+        if (weigh_x && !l.gated && !tc && moe_few_rows_takes(dt, 1, n_up, width, m->xg, l.w_up) && moe_few_rows_takes(dt, 1, width, l.expert_ff, m->u, l.w_down)) {
             rc = launch_moe_few_plan(dt, m->f32a, outputs, m->x, m->xg, pair_row, tile_expert, row_token, n_live, gate, NT, l.experts, l.top, width, st);
             if (rc == B200_OK) tile_live = row_token;  // (its place: the rows' tokens are not needed)
         } else if (!softmax && moe_route_plan_bytes(NT, l.experts) <= (size_t)max_rows * width * es) {  // (the counts lie where the gather puts its rows)

@@ -202,12 +202,13 @@ __device__ __forceinline__ void choose_sigmoid(const float (&z)[J], int lane, in
     }
 }
 
-// A decode batch (at most 16 tokens, 128 choices, 256 experts): choice, plan and gather in one launch.  Every CTA chooses for all tokens -- 16 rows of logits, a
+// A decode batch (at most 64 tokens, 256 choices, 256 experts): choice, plan and gather in one launch.  Every CTA chooses for all tokens -- 16 rows of logits, a
 // microsecond -- and knows the plan from that alone: an expert that was chosen owns one tile, in the experts' order, its rows are its pairs in order.  CTA b
 // gathers tile b, its live rows only (moe_few_rows_kernel reads no others).  Bound: latency, one chain of logits -> rows.
-// Measured (16 tokens, 4 of 32 experts, width 2048): three launches 5.4 + 6.1 + 4.3 us -> 7.5.
-constexpr int kFewTokens = 16, kFewPairs = 128, kFewExperts = 256;
-template <typename T>
+// Measured (16 tokens, 4 of 32 experts, width 2048): three launches 5.4 + 6.1 + 4.3 us -> 7.5.  A whole Vasolix-shaped decode step of 17 / 32 / 64 requests, whose
+// experts otherwise run on 64-row tiles: 761 / 853 / 1034 -> 571 / 674 / 932 us.
+constexpr int kFewTokens = 64, kFewPairs = 256, kFewExperts = 256;
+template <typename T, int J>  // J: logits of a token per lane
 __global__ void __launch_bounds__(256)
 moe_few_plan_kernel(const float *__restrict__ logits, int ld, const float *__restrict__ x, T *__restrict__ xg, int *__restrict__ pair_row,
                     int *__restrict__ tile_expert, int *__restrict__ tile_live, int *__restrict__ n_tiles, float *__restrict__ shared_gate, int tokens, int experts,
@@ -218,18 +219,19 @@ moe_few_plan_kernel(const float *__restrict__ logits, int ld, const float *__res
     __shared__ unsigned chosen[kFewExperts / 32];
     __shared__ int live;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pairs = tokens * top;
-    constexpr int J = kFewExperts / 32, V = Elem<T>::kVec;
-    float z[2][J];
+    constexpr int V = Elem<T>::kVec, PER = kFewTokens / 8;
+    float z[PER][J];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < PER; ++i)
 #pragma unroll
         for (int j = 0; j < J; ++j) z[i][j] = warp + 8 * i < tokens && lane + 32 * j < experts ? logits[(size_t)(warp + 8 * i) * ld + lane + 32 * j] : 0.0f;
-    if (threadIdx.x < kFewPairs) sel[threadIdx.x] = -1;
+    sel[threadIdx.x] = -1;
+    static_assert(kFewPairs == 256, "a thread per pair");
     if (threadIdx.x < kFewExperts / 32) chosen[threadIdx.x] = 0u;
     if (threadIdx.x == 0) live = 0;
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < PER; ++i)
         if (warp + 8 * i < tokens)
             choose_sigmoid(z[i], lane, experts, top, [&](int k, int e, float w) {
                 if (lane == 0) {
@@ -896,8 +898,15 @@ int launch_moe_few_plan(int dtype, const float *logits, int ld, const float *x, 
                         float *shared_gate, int tokens, int experts, int top, int width, cudaStream_t st) {
     if (tokens > kFewTokens || tokens * top > kFewPairs || experts > kFewExperts || dtype == B200_F32 || width % 8 != 0 || !all_aligned16({x, xg})) return B200_ERR_UNSUPPORTED;
     const int tiles = std::min(experts, tokens * top);
-    if (dtype == B200_BF16) launch_plain(moe_few_plan_kernel<__nv_bfloat16>, dim3(tiles), dim3(256), 0, st, logits, ld, x, (__nv_bfloat16 *)xg, pair_row, tile_expert, tile_live, n_tiles, shared_gate, tokens, experts, top, width);
-    else launch_plain(moe_few_plan_kernel<__half>, dim3(tiles), dim3(256), 0, st, logits, ld, x, (__half *)xg, pair_row, tile_expert, tile_live, n_tiles, shared_gate, tokens, experts, top, width);
+    auto go = [&](auto kern, auto *out) { launch_plain(kern, dim3(tiles), dim3(256), 0, st, logits, ld, x, out, pair_row, tile_expert, tile_live, n_tiles, shared_gate, tokens, experts, top, width); };
+    auto with = [&](auto *out) {
+        using T = std::remove_pointer_t<decltype(out)>;
+        if (experts <= 32) go(moe_few_plan_kernel<T, 1>, out);
+        else if (experts <= 128) go(moe_few_plan_kernel<T, 4>, out);
+        else go(moe_few_plan_kernel<T, 8>, out);
+    };
+    if (dtype == B200_BF16) with((__nv_bfloat16 *)xg);
+    else with((__half *)xg);
     return cuda_status("moe_few_plan launch");
 }
 
@@ -927,7 +936,7 @@ int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, co
                             int N, int K, int act, cudaStream_t st, int live_rows, const int *tile_live) {
     if (max_tiles == 0) return B200_OK;
     // a decode batch: up to 16 live rows per tile, slices of K for 16 warps at most, whole 32-k blocks
-    if (moe_few_rows_takes(dtype, live_rows, N, K, a, w)) {
+    if (moe_few_rows_takes(dtype, tile_live ? 1 : live_rows, N, K, a, w)) {
         const int KS = (K / 32 + 7) / 8, NG = KS >= 8 ? 1 : 8 / KS;
         const int units = (N / 8 + NG - 1) / NG, steps = std::max(1, std::min(8, units * max_tiles / (2 * sm_count())));
         const dim3 grid((units + steps - 1) / steps, max_tiles);

@@ -525,22 +525,22 @@ def test_recurrence_on_both_sides_of_the_token_parallel_rule(heads, schedule):
 
 
 @pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
-@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 16])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 16, 17, 32, 64, 65])
 @pytest.mark.parametrize("experts,top", [(1, 1), (3, 3), (8, 8), (40, 4), (256, 2)])
 def test_decode_batches_plan_their_experts_in_one_launch(dtype, n, experts, top):
-    """Up to 16 tokens of a 16-bit engine: choice, plan and gather of csrc/moe.cu's moe_few_plan_kernel, experts on their tiles' live rows.  Every expert chosen by
-    every token (up to 16 live rows of a tile: two passes), or a few of many (most tiles one row), against the float64 model."""
+    """Up to 64 tokens of a 16-bit engine: choice, plan and gather of csrc/moe.cu's moe_few_plan_kernel, experts on their tiles' live rows.  Every expert chosen by
+    every token (up to 64 live rows of a tile: eight passes; 8 of 8: more pairs than it takes from 33 tokens on), or a few of many (most tiles one row), and 65 tokens,
+    which it leaves alone, against the float64 model."""
     config = ref.make_config([ref.gla_layer(mlp=ref.moe(experts=experts, top=top, ff=64, shared_ff=64))], width=64)
     W, packed = ref.make_weights(config, seed=experts)
     req = {f"r{i}": tokens_of(config, 23, 100 + i) for i in range(n)}
-    sess = session(config, packed, dtype=dtype, pool_tokens=64 * n, max_seqs=n)
+    sess = session(config, packed, dtype=dtype, pool_tokens=64 * n, max_seqs=n, max_batch_tokens=2048)
     got = replay(sess, req, [[(k, 20) for k in req]] + [[(k, 1) for k in req]] * 3)
-    for name in req:
-        want = want_logits(config, W, req[name])
-        per_pos = (np.linalg.norm(got[name] - want, axis=-1) / np.linalg.norm(want, axis=-1))[20:]
-        assert np.median(per_pos) < 4e-2, (name, per_pos)
-        if experts == top:  # (no close routing calls)
-            assert per_pos.max() < 0.15, (name, per_pos)
+    wants = {k: want_logits(config, W, req[k]) for k in req}
+    per_pos = np.concatenate([(np.linalg.norm(got[k] - wants[k], axis=-1) / np.linalg.norm(wants[k], axis=-1))[20:] for k in req])
+    assert np.median(per_pos) < 4e-2, np.sort(per_pos)  # (16-bit rounding may flip a close choice of one token: it stays that token's)
+    if experts == top:  # (no close calls)
+        assert per_pos.max() < 0.15, np.sort(per_pos)
 
 
 @pytest.mark.parametrize("tokens", [511, 512, 513, 900])
