@@ -17,8 +17,8 @@ int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStrea
         return B200_ERR_INVALID_ARG;
     }
     const bool b16 = dtype == B200_BF16 || dtype == B200_F16;
-    // up to 8 tokens of INT4 weights: weights straight from global memory into registers (gemv_qd.cuh, with both sides' times)
-    if (b16 && fmt == WF_INT4 && a.M <= 8) {
+    // up to 8 tokens of INT4 weights, dense rows of at most 3072 k: straight from global memory into registers (gemv_qd.cuh, with both sides' times)
+    if (b16 && fmt != WF_FP8) {
         const int rc = dtype == B200_BF16 ? launch_gemv_qd_bf16(a, fmt, swiglu, st) : launch_gemv_qd_f16(a, fmt, swiglu, st);
         if (rc != B200_ERR_UNSUPPORTED) return rc;
     }

@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Which kernel, how many passes over the weights and which ring geometry each linear of a decode step gets -- a Python MODEL of the host-side
 dispatch (no GPU): decoder.cu norm_linear (norm inside the GEMV for one dense token, a norm kernel in front otherwise), gemv_f32.cu launch_gemv_nk
-(gemv_qd for up to 8 tokens of INT4, gemv_rs, what its ring refuses on gemv_mma, the SIMT GEMV for up to 4 tokens), linear.cu (GEMV passes, tcgen05 GEMM for dense M > 16), gemv_inst.cuh,
+(gemv_qd for up to 8 tokens of INT4 and short dense rows, gemv_rs, what its ring refuses on gemv_mma, the SIMT GEMV for up to 4 tokens), linear.cu (GEMV passes, tcgen05 GEMM for dense M > 16), gemv_inst.cuh,
 gemv_rs.cuh gemv_rs_geometry and gemv_mma.cuh gemv_mma_geometry.  It restates those few formulas; when they change, this file must follow
 (tests/test_dispatch_plan.py).
 usage: python scripts/dispatch_plan.py > profiles/<tag>_dispatch_plan.txt"""
@@ -98,15 +98,19 @@ def gemv_rs_plan(M, K, N, fmt, swiglu=False):
 
 
 def gemv_qd_plan(M, K, N, fmt, swiglu=False):
-    """gemv_qd.cuh launch_gemv_qd_t (INT4 in groups of 128, 1..8 tokens): None when unsupported.  It is the form of gemv_rs whose ring is in registers."""
-    if fmt != "int4" or M < 1 or M > 8 or K % 128:
+    """gemv_qd.cuh launch_gemv_qd_t (INT4 in groups of 128 of 1..8 tokens, short dense rows of 1..16): None when unsupported.  It is the form of gemv_rs
+    whose ring is in registers."""
+    dense = fmt == "dense"
+    if fmt == "fp8" or M < 1 or M > (16 if dense else 8) or K % 128 or (dense and K > 3072):
         return None
-    units = -(-(N // 2) // 8) if swiglu else -(-N // 16)
-    warps = 16 if K >= 8192 or (K >= 4096 and units <= 2 * SMS) else 8
-    smem = M * (2 * K + 64) + 256 + 2 * warps * 160 * 4
-    if smem > 160 * 1024 * warps // 16:
+    if dense:
+        warps = 16 if (K >= 2048 if M > 8 else K > 2048) else 8
+    else:
+        warps = 16 if K >= 8192 else 8
+    smem = M * (2 * K + 64) + 256 + 2 * warps * (16 if M > 8 else 8) * 20 * 4
+    if smem > (108 if dense else 160) * 1024 * warps // 16:
         return None
-    return dict(kernel="gemv_rs", form="gemv_qd", warps=warps, pieces=1, piece_bytes=K // 2, stages=2, smem=smem)
+    return dict(kernel="gemv_rs", form="gemv_qd", warps=warps, pieces=1, piece_bytes=K * 2 if dense else K // 2, stages=2, smem=smem)
 
 
 def gemv_any(M, K, N, fmt, swiglu=False):
