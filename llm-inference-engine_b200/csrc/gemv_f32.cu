@@ -1,6 +1,7 @@
 #include <stdlib.h>
 
 #include "gemv_inst.cuh"
+#include "gemv_sr.cuh"
 namespace b200 {
 int launch_gemv_nk_f32(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st) { return launch_gemv_t<float, false>(a, fmt, swiglu, st); }
 int launch_gemv_nk_bf16(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st);
@@ -36,6 +37,11 @@ int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStrea
         if (rc != B200_ERR_UNSUPPORTED) return rc;
     }
     if (a.M > 4) return B200_ERR_UNSUPPORTED;
+    // one token of short rows (fp32: up to four) and its norm: whole rows per warp (gemv_sr.cuh, with both sides' times)
+    {
+        const int rc = dtype == B200_F32 ? launch_gemv_sr_t<float>(a, fmt, swiglu, st) : dtype == B200_BF16 ? launch_gemv_sr_t<__nv_bfloat16>(a, fmt, swiglu, st) : dtype == B200_F16 ? launch_gemv_sr_t<__half>(a, fmt, swiglu, st) : B200_ERR_UNSUPPORTED;
+        if (rc != B200_ERR_UNSUPPORTED) return rc;
+    }
     switch (dtype) {
         case B200_F32: return launch_gemv_nk_f32(a, fmt, swiglu, st);
         case B200_F16: return launch_gemv_nk_f16(a, fmt, swiglu, st);

@@ -238,7 +238,7 @@ static int launch_gemv_qd_inst(const GemvArgs &a, int units, cudaStream_t st) {
     auto kern = gemv_qd_kernel<T, FMT, SW, NT, NW>;
     const size_t smem = gemv_qd_smem(a.M, a.K, NW);
     if (smem > qd_smem(FMT, NW)) return B200_ERR_UNSUPPORTED;
-    if (!allow_smem(reinterpret_cast<const void *>(kern), qd_smem(FMT, NW))) return cuda_status("gemv_qd cudaFuncSetAttribute");
+    if (!allow_smem(reinterpret_cast<const void *>(kern), qd_smem(FMT, NW), qd_smem(FMT, 16) + 2048)) return cuda_status("gemv_qd cudaFuncSetAttribute");
     launch_pdl(kern, dim3(std::max(1, std::min(units, 16 / NW * sm_count()))), dim3(NW * 32), smem, st, true, a);
     return cuda_status("gemv_qd launch");
 }

@@ -3,6 +3,7 @@
 
 #include <cuda.h>  // CUtensorMap: types only, the encoder comes through cudaGetDriverEntryPoint (no libcuda to link)
 #include <atomic>
+#include <algorithm>
 #include <mutex>
 #include <unordered_set>
 
@@ -91,7 +92,7 @@ int sm_count() {
     return cached[dev];
 }
 
-bool allow_smem(const void *kernel, size_t most) {
+bool allow_smem(const void *kernel, size_t most, size_t per_sm) {
     static std::mutex mu;
     static std::unordered_set<const void *> raised[64];
     int dev = 0;
@@ -102,6 +103,7 @@ bool allow_smem(const void *kernel, size_t most) {
     std::lock_guard<std::mutex> lk(mu);
     if (!raised[dev].count(kernel)) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return false;
+        if (per_sm > 0 && cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)std::min<size_t>(100, (per_sm * 100 + (228 << 10) - 1) / (228 << 10))) != cudaSuccess) return false;
         raised[dev].insert(kernel);
     }
     seen[dev].insert(kernel);

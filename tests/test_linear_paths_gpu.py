@@ -62,6 +62,19 @@ def test_linear_of_few_tokens_and_odd_rows(n):
     assert bool((out[6 * n:] == 7.0).all())
 
 
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("k,n", [(128, 1), (512, 7), (1408, 296), (1536, 2369), (1664, 4738), (3072, 31), (3200, 297)])
+def test_fp32_rows_of_a_few_tokens(m, k, n):
+    """csrc/gemv_sr.cuh: rows that are no whole number of a warp's slots, row counts around the SMs and their warps, odd ones, and the lengths it leaves alone."""
+    gen = torch.Generator(device=DEV).manual_seed(m + k + n)
+    x, w = torch.randn(m, k, generator=gen, device=DEV), torch.randn(n, k, generator=gen, device=DEV)
+    out = torch.full((m * n + 64,), 7.0, device=DEV)
+    got = b200.linear(x, w, out=out[:m * n].view(m, n))
+    # chains of at most k / 128 products a lane, then the lanes: each rounding 2^-24 of the terms' sizes
+    assert bool(((got.double() - x.double() @ w.double().T).abs() <= (k / 128 + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)).all())
+    assert bool((out[m * n:] == 7.0).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
 @pytest.mark.parametrize("m,k,n", [(1, 128, 1), (8, 640, 31), (3, 1920, 2369), (8, 2176, 4743), (2, 4096, 17), (5, 4096, 4737), (8, 4224, 2384), (1, 8320, 4743), (6, 8192, 16),
                                    (6, 11008, 24), (7, 11008, 24), (2, 28672, 48), (3, 28672, 48)])
