@@ -131,6 +131,8 @@ def linear_plan(M, K, N, fmt, fused_rows=16, swiglu=False):
     """One linear of the decode step: (path, passes over the weights, geometry)."""
     if M == 1 and fmt == "dense":  # the norm / residual / tensor-parallel prologue inside the GEMV
         g = gemv_nk_plan(M, K, fmt)
+        if g and K <= 3072 and K % 256 == 0:  # gemv_sr.cuh launch_gemv_sr_t: the form of gemv_nk with whole rows per warp
+            g = dict(kernel="gemv_nk", form="gemv_sr", pieces=1, piece_bytes=K * 2, stages=2)
         if g:
             return ("fused " + g["kernel"], 1, g)
     if M <= fused_rows:
