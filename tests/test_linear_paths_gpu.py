@@ -99,6 +99,22 @@ def test_int4_weights_streamed_into_registers(dtype, m, k, n):
         assert bool((out[m * n:] == 7.0).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("k", [128, 640, 1152, 1920, 2048, 2176, 3968, 4096, 4224, 4352, 5120, 7168, 8192, 8832, 11008, 12416, 14336, 28672])
+def test_int4_token_has_the_same_bits_beside_any_others(dtype, k):
+    """1 to 8 tokens, whichever form of csrc/gemv_qd.cuh holds their activations, or csrc/gemv_rs.cuh where none does (11008 k from 7 tokens on, 28672 from 3 on)."""
+    for n in (17, 300, 4743):
+        gen = torch.Generator(device=DEV).manual_seed(k + n)
+        x = torch.randn(8, k, generator=gen, device=DEV).to(dtype)
+        q, s, z, _ = quantised(gen, n, k, "int4", dtype)
+        run = lambda t: b200.linear(t, q, w_format=b200.W_INT4, scales=s, zeros=z, group=128, N=n)  # noqa: B023,E731
+        s *= 2.0 ** -8
+        all8 = run(x)
+        for m in range(1, 8):
+            assert torch.equal(run(x[:m].contiguous()), all8[:m]), (n, m)
+        assert torch.equal(run(x[5:].contiguous()), all8[5:]), n
+
+
 @pytest.mark.parametrize("fmt,n", [("dense", 192000), ("fp8", 152064), ("int4", 290000)])
 def test_linear_whose_sums_leave_no_ring(fmt, n):
     """Vocabulary-sized outputs of rows of 8192 k, 16 tokens: sizes that stay with the kernel whose activations are in shared memory (csrc/gemv_mma.cuh), and
