@@ -9,14 +9,15 @@
 //     of products keep the tensor pipe from waiting for its own results.  (K = 4096, N = 12288, where this takes 8.5 us: two buffers of four groups 10.6, one
 //     group at a time in three CTAs per SM 9.2);
 //   * 16 warps per SM, as two CTAs where both hold the activations, so that a unit's sum does not stop all of them (K = 4096, N = 12288 8.5 us with two against 9.4
-//     with one, K = 2048, N = 5376 2.8 against 4.9), else as one;
+//     with one, K = 2048, N = 5376 2.8 against 4.9), else as one: longer rows (K > 4096, dense > 2048) and more tokens;
 //   * the first weights and parameters are requested before griddepcontrol.wait; one __syncthreads per unit (and part, below): the warps leave their tiles in one of
 //     two buffers, the first threads add them in a fixed order (deterministic).
-// INT4: a token's result does not depend on how many are beside it, though the form does.
-//   * Everything is summed in the order of gemv_rs.cuh, which takes the tokens that no form holds (K = 11008 from 7 on).  Fragments, dequantisation and
+// A token's result does not depend on how many are beside it, though the form does:
+//   * INT4: everything is summed in the order of gemv_rs.cuh, which takes the tokens that no form holds (K = 11008 from 7 on).  Fragments, dequantisation and
 //     arithmetic are its own: exact integers in f16, fp32 sums, the group's scale once per 128 k; then parts of at most 32 groups, of every part 16 slices, of every
 //     slice a tile.  So a part of a long row costs a barrier: K = 11008, N = 4096 10.3 us where one sum over each warp's whole slice took 9.3, K = 8192, N = 10240 14.9
 //     for 13.8; all parts' tiles at once behind one barrier 10.6 and 14.4.
+//   * dense: the sums of eight warps in order, or of sixteen two by two, which are the same where a warp of eight has at most two groups (K <= 2048).
 // Dense weights: a launch's start rather than its instructions; its CTAs wait for no barrier and no ring.  Their sums are shorter chains in the tensor cores than
 // gemv_rs.cuh's (fp32 outputs of K = 4096: 1.08e-7 from 64 bits against 1.42e-7).
 // (Codes multiplied as they are, as subnormal f16, with the zero points' part taken off afterwards, need five instructions instead of nine for eight weights and
@@ -25,7 +26,7 @@
 // 5.1 / 5.5 / 6.0 -> 4.0 / 4.9 / 5.2, N = 22016 16.7 / 17.4 / 17.7 -> 13.3 / 14.2 / 16.5; K = 11008, N = 4096 12.0 / 12.6 / 14.0 -> 10.3 / 11.4 / gemv_rs;
 // K = 8192, N = 10240 17.6 / 18.2 / 19.6 -> 14.9 / 16.0 / 17.6; K = 5120, N = 5120 9.6 / 9.8 / 10.2 -> 8.9 / 9.6 / 10.4 (its 20 groups a part are one or two to a slot).
 // Dense, 1 (gemv.cuh) / 8 / 16 tokens (gemv_rs.cuh -> here): K = 2048: N = 6176 7.3 / 7.6 / 9.0 -> 5.3 / 6.0 / 6.6, N = 2048 3.8 / 3.6 / 4.3 -> 2.6 / 3.0 / 3.5;
-// K = 1024, N = 1536 3.1 / 2.8 / 3.2 -> 1.8 / 1.9 / 2.4.
+// K = 1024, N = 1536 3.1 / 2.8 / 3.2 -> 1.8 / 1.9 / 2.4; K = 1536, N = 3072 4.4 / 4.1 / 5.0 -> 2.6 / 3.0 / 3.9; K = 3072, N = 3072 5.7 / 5.9 / 7.1 -> 4.2 / 4.8 / 5.9.
 #pragma once
 #include "gemv_rs.cuh"
 
@@ -42,10 +43,11 @@ constexpr int kQdTileRow = 20;          // fp32 values of a token in a warp's ti
 // groups of 128 k per slot: INT4 two of them (2 KB of 16 rows), dense weights one (4 KB)
 __host__ __device__ constexpr int qd_groups(int fmt) { return fmt == WF_INT4 ? 2 : 1; }
 // What a warp's slot is.  INT4 (a slice has at most two groups, where rows have at most 2048 k one): its two slices; one of its two slices; its only slice of a part.
-// Dense: a group of its slice
-enum { QD_TWO_SLICES, QD_SLICE, QD_PART, QD_DENSE };
-// dynamic shared memory of an SM's one CTA of 16 warps or two of 8, at most: what is in flight (64 KB, dense 128) needs L1 beside it
-__host__ __device__ constexpr size_t qd_smem(int mode, int warps) { return (size_t)(mode == QD_DENSE ? 108 : 160) * 1024 * warps / 16; }
+// Dense: a group of its slice, with at most 108 KB of shared memory per SM, or 148
+enum { QD_TWO_SLICES, QD_SLICE, QD_PART, QD_DENSE, QD_DENSE_LARGE };
+// Dynamic shared memory of an SM's one CTA of 16 warps or two of 8, at most: what is in flight (64 KB, dense 128) needs L1 beside it.  With 148 KB dense loads no
+// longer have all of theirs: K = 2048, N = 6176 of 1 / 8 / 16 tokens 5.8 / 6.5 / 6.7 us for 5.3 / 6.0 / 6.6; for K = 3072 and 16 tokens, which 108 KB do not hold, 5.9 (gemv_rs 7.1)
+__host__ __device__ constexpr size_t qd_smem(int mode, int warps) { return (size_t)(mode == QD_DENSE ? 108 : mode == QD_DENSE_LARGE ? 148 : 160) * 1024 * warps / 16; }
 
 template <typename T, int FMT, bool kSwiGLU, int NT, int NW, int MODE>
 __global__ void __launch_bounds__(NW * 32, 16 / NW)
@@ -164,8 +166,13 @@ gemv_qd_kernel(const GemvArgs a) {
             const int r = lane & 15, m = warp * 2 + (lane >> 4);
             const float *mine = red + (size_t)(h & 1) * TILES * TILE + m * kQdTileRow + r;
             float v = 0.0f;
+            if constexpr (kDense && NW == 16) {  // (a warp of the other form has the groups of two of these)
 #pragma unroll
-            for (int w2 = 0; w2 < TILES; ++w2) v += mine[(size_t)w2 * TILE];
+                for (int w2 = 0; w2 < TILES; w2 += 2) v += mine[(size_t)w2 * TILE] + mine[(size_t)(w2 + 1) * TILE];
+            } else {
+#pragma unroll
+                for (int w2 = 0; w2 < TILES; ++w2) v += mine[(size_t)w2 * TILE];
+            }
             if constexpr (MODE == QD_PART) {
                 v += sum, sum = last ? 0.0f : v;
                 if (!last) {
@@ -321,12 +328,13 @@ static int launch_gemv_qd_t(const GemvArgs &a, int fmt, bool swiglu, cudaStream_
     }
     // Dense rows of at most 3072 k: there the start is most of a launch.  Longer ones fill gemv_rs.cuh's 200 KB ring before their wait, behind an attention or a
     // norm kernel, where this holds 128 KB (four layers, 2 / 8 tokens: 7B size 386 / 377 us there, 403 / 411 here; 2048 wide 155 / 169 there, 149 / 150 here; a
-    // 70B-shaped shard, whose down projection has 3584 k, 286 / 296 there, 330 / 344 with it here and 273 / 287 without).  A vocabulary's fp32 logits of more than
-    // 8 tokens stay there as well (50257 x 2048, 16 tokens: 58.1 us a head there, 59.0 here).
-    if (a.K > 3072 || (a.M > 8 && a.y_f32)) return B200_ERR_UNSUPPORTED;
-    const bool wide = a.M > 8 ? a.K >= 2048 : a.K > 2048;
+    // 70B-shaped shard, whose down projection has 3584 k, 286 / 296 there, 330 / 344 with it here and 273 / 287 without).  A vocabulary's fp32 logits of 16 rows, norm and
+    // top-k included: 1024 x 32000 41.7 us there, 30.3 here; 2048 x 32000 41.9 and 41.7; 2048 x 50257 58.2 and 59.6.
+    if (a.K > 3072) return B200_ERR_UNSUPPORTED;
+    const bool wide = a.K > 2048 || !fits(QD_DENSE, 8);
 #define B200_QD_GO(SW) (a.M <= 8 ? (wide ? launch_gemv_qd_inst<T, WF_DENSE, SW, 1, 16, QD_DENSE>(a, units, st) : launch_gemv_qd_inst<T, WF_DENSE, SW, 1, 8, QD_DENSE>(a, units, st)) \
-                        : wide ? launch_gemv_qd_inst<T, WF_DENSE, SW, 2, 16, QD_DENSE>(a, units, st) : launch_gemv_qd_inst<T, WF_DENSE, SW, 2, 8, QD_DENSE>(a, units, st))
+                        : !wide ? launch_gemv_qd_inst<T, WF_DENSE, SW, 2, 8, QD_DENSE>(a, units, st) : fits(QD_DENSE, 16) ? launch_gemv_qd_inst<T, WF_DENSE, SW, 2, 16, QD_DENSE>(a, units, st) \
+                        : launch_gemv_qd_inst<T, WF_DENSE, SW, 2, 16, QD_DENSE_LARGE>(a, units, st))
     return swiglu ? B200_QD_GO(true) : B200_QD_GO(false);
 #undef B200_QD_GO
 }

@@ -115,6 +115,44 @@ def test_int4_token_has_the_same_bits_beside_any_others(dtype, k):
         assert torch.equal(run(x[5:].contiguous()), all8[5:]), n
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("k", [128, 640, 1024, 1152, 1536, 1920, 2048, 2176, 2688, 3072, 3200, 4096, 5120, 11008])
+def test_dense_token_has_the_same_bits_beside_any_others(dtype, k):
+    """2 to 16 tokens, in csrc/gemv_qd.cuh (to 3072 k) and in csrc/gemv_rs.cuh."""
+    for n in (17, 300, 4743):
+        gen = torch.Generator(device=DEV).manual_seed(k + n)
+        x, w = (torch.randn(r, k, generator=gen, device=DEV).to(dtype) for r in (16, n))
+        all16 = b200.linear(x, w)
+        for m in range(2, 16):
+            assert torch.equal(b200.linear(x[:m].contiguous(), w), all16[:m]), (n, m)
+        assert torch.equal(b200.linear(x[5:].contiguous(), w), all16[5:]), n
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("hidden", [1024, 2048, 3072, 4096])
+def test_logits_of_a_row_have_the_same_bits_beside_any_others(dtype, hidden):
+    """The head's fp32 logits, norm in front, of 2 to 16 rows, and of 17 to 24, whose last pass has 1 to 8 rows (one row has a kernel of its own)."""
+    gen = torch.Generator(device=DEV).manual_seed(hidden)
+    vocab, k = 1003, 5
+    x, gamma, head = (torch.randn(*s, generator=gen, device=DEV).to(dtype) for s in ((24, hidden), (hidden,), (vocab, hidden)))
+    code = {torch.bfloat16: b200.BF16, torch.float16: b200.F16}[dtype]
+    engine = b200.Decoder(b200.DecoderConfig(hidden, hidden // 128, hidden // 128, 128, 256, 1, 64, 24, code, b200.W_DENSE, 128, 1e-6, 128, 10000.0, 1, 0), DEV)
+
+    def logits(rows):
+        b = len(rows)
+        z = lambda *s, dtype=torch.int32: torch.zeros(*s, dtype=dtype, device=DEV)  # noqa: E731
+        bufs = dict(logits=z(b, vocab, dtype=torch.float32), tmp_ids=z(b, b200.TOPK_BLOCKS, k), tmp_vals=z(b, b200.TOPK_BLOCKS, k, dtype=torch.float32),
+                    topk_ids=z(b, k), topk_vals=z(b, k, dtype=torch.float32), seq_len=z(b), finished=z(b, dtype=torch.uint8), output_id=z(b))
+        engine.lm_head_topk_sample(rows.clone(), gamma, head, bufs, k, 7, 2)
+        return bufs["logits"]
+
+    all16 = logits(x[:16])
+    for m in (2, 3, 7, 8, 9, 12, 15):
+        assert torch.equal(logits(x[:m]), all16[:m]), m
+    all24 = logits(x)
+    assert torch.equal(all24[:16], all16) and torch.equal(logits(x[:19])[16:], all24[16:19])
+
+
 @pytest.mark.parametrize("fmt,n", [("dense", 192000), ("fp8", 152064), ("int4", 290000)])
 def test_linear_whose_sums_leave_no_ring(fmt, n):
     """Vocabulary-sized outputs of rows of 8192 k, 16 tokens: sizes that stay with the kernel whose activations are in shared memory (csrc/gemv_mma.cuh), and
