@@ -5,9 +5,10 @@
 // (4 numbers of 1024 for a lane), hands every pair of rows through two barriers to a reducer warp and starts with a ring's worth of barriers and bulk copies.
 // Here a warp owns whole rows, two at a time (SwiGLU: a gate row and its up row), and streams them into registers; nothing is shared between warps but the
 // activations, and the first 8 KB of every warp are on their way before griddepcontrol.wait.  Units are dealt over the SMs first, then over an SM's warps.
-// A lane adds 4 (16-bit: 8) chains of products, the warp adds the lanes: fp32 multiply-adds in a fixed order, whatever rows are beside (deterministic).
-// Measured (four layers, us per step, gemv.cuh -> here): fp32, 1024 wide, feed-forward 1408, 1 / 2 / 4 tokens 95 / 184 / 238 -> 81 / 132 / 163; 2048 wide, 2688,
-// 2 / 4 tokens 250 / 328 -> 216 / 278; bf16, 2048 wide, 1 token 161 -> 140.  With gemv.cuh's prologue, one token's norm after another: 1024 wide 85 / 178 / 239.
+// A lane adds 4 (16-bit: 8) chains of products, the warp adds the lanes: fp32 multiply-adds in a fixed order (deterministic).  Neither that order nor the norm's
+// depends on the number of tokens: a token's result has the same bits whatever is beside it.
+// Measured (four layers, context 129, us per step, gemv.cuh -> here): fp32, 1024 wide, feed-forward 1408, 1 / 2 / 3 / 4 tokens 96 / 141 / 175 / 194 -> 81 / 96 / 122 / 130;
+// bf16, 2048 wide, 1 token 133 -> 102.  With gemv.cuh's prologue, one token's norm after another, 2 and 4 fp32 tokens gained little: 184 -> 178 and 238 -> 239, another context.
 #pragma once
 #include "gemv.cuh"
 
@@ -20,7 +21,7 @@ __global__ void __launch_bounds__(kSrWarps * 32, 2)
 gemv_sr_kernel(const GemvArgs a) {
     constexpr int V = Elem<T>::kVec, C = V / 4;
     extern __shared__ __align__(16) float xs[];  // [MB][K]; 16-bit: the halves of a warp's 256 numbers apart, so that 16-byte reads of neighbours touch
-    __shared__ float red[kSrWarps];
+    __shared__ float red[MB][kSrWarps];
     GemvArgs b = a;
     b.tp.world = 0;  // (never set here: the exchange's registers are not wanted)
     const int K = a.K, N = a.N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -55,27 +56,35 @@ gemv_sr_kernel(const GemvArgs a) {
     {   // Activations, one token per 8 / MB warps: x (+ residual) -> T; residual_out <- that (CTA 0); (+ bias) -> T; norm, rounded where the un-fused kernels round
         constexpr int TT = kSrWarps * 32 / MB;  // threads of a token
         const int m = threadIdx.x / TT, t = threadIdx.x - m * TT;
-        float ss = 0.0f;
+        float ss[MB] = {};  // squares, summed as by 8 warps whatever MB is: a token's norm has the same bits beside any others
         auto place = [&](int i, int c) { return reinterpret_cast<float4 *>(xs + (size_t)m * K + (i >> 5) * 32 * V + c * 128 + (i & 31) * 4); };
         if (m < a.M) {
-#pragma unroll 4
-            for (int i = t; i < K / V; i += TT) {
-                float f[V];
-                gemv_prenorm_vec<T>(b, 0u, m, i, f, true);
+#pragma unroll (4 / MB)
+            for (int i0 = t; i0 < K / V; i0 += MB * TT) {
 #pragma unroll
-                for (int j = 0; j < V; ++j) ss = fmaf(f[j], f[j], ss);
+                for (int w = 0; w < MB; ++w) {
+                    const int i = i0 + w * TT;
+                    if (i >= K / V) break;
+                    float f[V];
+                    gemv_prenorm_vec<T>(b, 0u, m, i, f, true);
 #pragma unroll
-                for (int c = 0; c < C; ++c) *place(i, c) = make_float4(f[4 * c], f[4 * c + 1], f[4 * c + 2], f[4 * c + 3]);
+                    for (int j = 0; j < V; ++j) ss[w] = fmaf(f[j], f[j], ss[w]);
+#pragma unroll
+                    for (int c = 0; c < C; ++c) *place(i, c) = make_float4(f[4 * c], f[4 * c + 1], f[4 * c + 2], f[4 * c + 3]);
+                }
             }
         }
         if (norm) {  // (every thread scales what it has written)
-            ss = warp_sum(ss);
-            if (lane == 0) red[warp] = ss;
-            __syncthreads();
-            ss = 0.0f;
 #pragma unroll
-            for (int w = 0; w < kSrWarps / MB; ++w) ss += red[m * (kSrWarps / MB) + w];
-            const float rs = rsqrtf(ss / (float)K + a.eps);
+            for (int w = 0; w < MB; ++w) {
+                ss[w] = warp_sum(ss[w]);
+                if (lane == 0) red[m][w * (kSrWarps / MB) + warp % (kSrWarps / MB)] = ss[w];
+            }
+            __syncthreads();
+            float total = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kSrWarps; ++w) total += red[m][w];
+            const float rs = rsqrtf(total / (float)K + a.eps);
             if (m < a.M) {
 #pragma unroll 4
                 for (int i = t; i < K / V; i += TT) {
@@ -101,14 +110,13 @@ gemv_sr_kernel(const GemvArgs a) {
         for (int i = 0; i < kSrRing; ++i) {
             if (u >= units) break;
 #pragma unroll
-            for (int j = 0; j < kSrSlot; ++j) {
-                if (at * kSrSlot + j >= pieces) break;
-                float w[2][V];
-                unpack16<T>(ring[i].w[j][0], w[0]), unpack16<T>(ring[i].w[j][1], w[1]);
+            for (int m = 0; m < MB; ++m) {
+                if (MB > 1 && m >= a.M) break;
 #pragma unroll
-                for (int m = 0; m < MB; ++m) {
-                    if (MB > 1 && m >= a.M) break;
-                    float x[V];
+                for (int j = 0; j < kSrSlot; ++j) {
+                    if (at * kSrSlot + j >= pieces) break;
+                    float w[2][V], x[V];
+                    unpack16<T>(ring[i].w[j][0], w[0]), unpack16<T>(ring[i].w[j][1], w[1]);
 #pragma unroll
                     for (int c = 0; c < C; ++c)
                         load_vec<4>(xs + (size_t)m * K + (at * kSrSlot + j) * 32 * V + c * 128 + lane * 4, x + 4 * c);
@@ -153,12 +161,13 @@ gemv_sr_kernel(const GemvArgs a) {
     }
 }
 
-// The rows' length says whether a launch is mostly its start (it alone, so that a row's bits do not depend on the rows beside it): one fp32 token of 2048 / 2688 k
-// has 16 to 44 MB per linear, for which gemv.cuh holds 192 KB per SM in flight (four layers 188 us there, 194 here).
+// The rows' length says whether a launch is mostly its start -- it alone, so that a token's bits do not depend on those beside it: one fp32 token of 2048 / 2688 k has
+// 16 to 44 MB per linear, for which gemv.cuh holds 192 KB per SM in flight (four layers 188 us there, 194 here), so 2 to 4 of them run there too (four layers,
+// context 129, 2 / 4 tokens 208 / 286 us there, 177 / 238 here).
 // B200_ERR_UNSUPPORTED (no error text): other formats, long rows, rows that are no whole number of a warp's pieces, tensor-parallel ends
 template <typename T>
 static int launch_gemv_sr_t(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st) {
-    if (fmt != WF_DENSE || a.M < 1 || a.M > (sizeof(T) == 4 ? 4 : 1) || a.K > (sizeof(T) == 4 && a.M == 1 ? 1536 : 3072) || a.K % (32 * Elem<T>::kVec) != 0 || !all_aligned16({a.w, a.x})) return B200_ERR_UNSUPPORTED;
+    if (fmt != WF_DENSE || a.M < 1 || a.M > (sizeof(T) == 4 ? 4 : 1) || a.K > (sizeof(T) == 4 ? 1536 : 3072) || a.K % (32 * Elem<T>::kVec) != 0 || !all_aligned16({a.w, a.x})) return B200_ERR_UNSUPPORTED;
     if (a.tp.world > 1 || a.push.n > 0 || (a.norm && !all_aligned16({a.res_in, a.res_out, a.bias, a.gamma}))) return B200_ERR_UNSUPPORTED;
     const int units = swiglu ? a.inter : (a.N + 1) / 2, sms = sm_count();
     const dim3 grid(units <= sms ? std::max(1, units) : units <= sms * kSrWarps ? sms : 2 * sms);

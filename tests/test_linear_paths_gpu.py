@@ -153,6 +153,32 @@ def test_logits_of_a_row_have_the_same_bits_beside_any_others(dtype, hidden):
     assert torch.equal(all24[:16], all16) and torch.equal(logits(x[:19])[16:], all24[16:19])
 
 
+@pytest.mark.parametrize("k", [128, 512, 1024, 1408, 1536, 1664, 2048, 2688, 3072, 4096])
+def test_fp32_token_has_the_same_bits_beside_any_others(k):
+    """1 to 4 tokens, in csrc/gemv_sr.cuh (to 1536 k) and in csrc/gemv.cuh; and a decode step, whose linears norm their tokens: hidden size k, one layer."""
+    for n in (17, 300, 4743):
+        gen = torch.Generator(device=DEV).manual_seed(k + n)
+        x, w = torch.randn(4, k, generator=gen, device=DEV), torch.randn(n, k, generator=gen, device=DEV)
+        all4 = b200.linear(x, w)
+        for m in (1, 2, 3):
+            assert torch.equal(b200.linear(x[:m].contiguous(), w), all4[:m]), (n, m)
+        assert torch.equal(b200.linear(x[3:].contiguous(), w), all4[3:]), n
+    gen = torch.Generator(device=DEV).manual_seed(k)
+    r = lambda *s: torch.randn(*s, generator=gen, device=DEV) / math.sqrt(s[-1])  # noqa: E731
+    heads, inter = k // 128, k + 128
+    layer = dict(g1=r(k) + 1, g2=r(k) + 1, qkv=r(3 * heads * 128, k), o=r(k, heads * 128), gate_up=r(2 * inter, k), down=r(k, inter))
+    x, cache = torch.randn(4, k, generator=gen, device=DEV), torch.randn(2, 1, 4, heads, 64, 128, generator=gen, device=DEV)
+    got = []
+    for m in (4, 1, 2, 3):
+        dec = b200.Decoder(b200.DecoderConfig(k, heads, heads, 128, inter, 1, 64, m, b200.F32, b200.W_DENSE, 128, 1e-6, 128, 10000.0, 1, 0), DEV)
+        dec.set_layer(0, layer)
+        hidden = x[:m].clone()
+        dec.step(hidden, cache[0, :, :m].contiguous(), cache[1, :, :m].contiguous(), 33)
+        got.append(hidden)
+    for y in got[1:]:
+        assert torch.equal(y, got[0][:len(y)]), len(y)
+
+
 @pytest.mark.parametrize("fmt,n", [("dense", 192000), ("fp8", 152064), ("int4", 290000)])
 def test_linear_whose_sums_leave_no_ring(fmt, n):
     """Vocabulary-sized outputs of rows of 8192 k, 16 tokens: sizes that stay with the kernel whose activations are in shared memory (csrc/gemv_mma.cuh), and
