@@ -7,6 +7,8 @@
 // activations, and the first 8 KB of every warp are on their way before griddepcontrol.wait.  Units are dealt over the SMs first, then over an SM's warps.
 // A lane adds 4 (16-bit: 8) chains of products, the warp adds the lanes: fp32 multiply-adds in a fixed order (deterministic).  Neither that order nor the norm's
 // depends on the number of tokens: a token's result has the same bits whatever is beside it.
+// fp32 sums: relative to 64 bits 8.7e-8 / 8.9e-8 / 9.0e-8 at 1024 / 1408 / 1536 k (8192 rows of normal numbers; gemv.cuh 9.4e-8 / 9.1e-8 / 9.2e-8; all of a lane's
+// products of one chain in a row 9.1e-8 / 9.5e-8 / 9.6e-8, and 2 to 4 tokens 1 to 4 % less time).
 // Measured (four layers, context 129, us per step, gemv.cuh -> here): fp32, 1024 wide, feed-forward 1408, 1 / 2 / 3 / 4 tokens 96 / 141 / 175 / 194 -> 81 / 96 / 122 / 130;
 // bf16, 2048 wide, 1 token 133 -> 102.  With gemv.cuh's prologue, one token's norm after another, 2 and 4 fp32 tokens gained little: 184 -> 178 and 238 -> 239, another context.
 #pragma once
@@ -105,6 +107,8 @@ gemv_sr_kernel(const GemvArgs a) {
 
     int u = warp * gridDim.x + blockIdx.x, at = 0;
     float acc[MB][2][V] = {};
+    // fp32: a slot's products are summed before they join the row's, chains of 4 and of K / 512 terms instead of one of K / 128
+    constexpr bool kSplit = sizeof(T) == 4;
     while (u < units) {
 #pragma unroll
         for (int i = 0; i < kSrRing; ++i) {
@@ -112,6 +116,8 @@ gemv_sr_kernel(const GemvArgs a) {
 #pragma unroll
             for (int m = 0; m < MB; ++m) {
                 if (MB > 1 && m >= a.M) break;
+                float part[2][V] = {};
+                float(&to)[2][V] = kSplit ? part : acc[m];
 #pragma unroll
                 for (int j = 0; j < kSrSlot; ++j) {
                     if (at * kSrSlot + j >= pieces) break;
@@ -123,7 +129,13 @@ gemv_sr_kernel(const GemvArgs a) {
 #pragma unroll
                     for (int r = 0; r < 2; ++r)
 #pragma unroll
-                        for (int v = 0; v < V; ++v) acc[m][r][v] = fmaf(w[r][v], x[v], acc[m][r][v]);
+                        for (int v = 0; v < V; ++v) to[r][v] = fmaf(w[r][v], x[v], to[r][v]);
+                }
+                if constexpr (kSplit) {
+#pragma unroll
+                    for (int r = 0; r < 2; ++r)
+#pragma unroll
+                        for (int v = 0; v < V; ++v) acc[m][r][v] += part[r][v];
                 }
             }
             load(ring[i]);

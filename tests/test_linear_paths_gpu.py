@@ -179,6 +179,23 @@ def test_fp32_token_has_the_same_bits_beside_any_others(k):
         assert torch.equal(y, got[0][:len(y)]), len(y)
 
 
+@pytest.mark.parametrize("m", [1, 2, 4])
+@pytest.mark.parametrize("k", [512, 1024, 1408, 1536])
+def test_fp32_sums_round_no_more_often_than_they_need(m, k):
+    """csrc/gemv_sr.cuh's distance from 64 bits over 8192 rows.  A sum of j random terms has variance j (a term's: 1); rounding it adds s^2 j, s^2 = 2^-46 / 12 times
+    the mean of 1 / mantissa^2 (0.541 for mantissas spread over their logarithm).  A lane's four chains: slots of four products (1 + 2 + 3 + 4), which join one
+    another (4 (2 + .. + S) for S = k / 512); then four chains to one (2 additions of a half, one of all: twice k over all lanes) and five rounds over the
+    lanes (k each).  One chain of k / 128 products (1 + .. + k / 128) instead comes out 1.05 times as far at 1408 and 1536 k.  Sums of normal products have
+    mantissas a little nearer to 1 than that: a tenth more, against 5 % measured."""
+    pieces = k // 128
+    chains = sum(10 if s + 4 <= pieces else sum(range(1, pieces - s + 1)) for s in range(0, pieces, 4)) + sum(min(4 * i, pieces) for i in range(2, (pieces + 3) // 4 + 1))
+    model = math.sqrt(2.0 ** -46 / 12 * 0.541 * (128 * chains / k + 2 + 5))
+    gen = torch.Generator(device=DEV).manual_seed(m + k)
+    x, w = torch.randn(m, k, generator=gen, device=DEV), torch.randn(8192, k, generator=gen, device=DEV)
+    want = x.double() @ w.double().T
+    assert float((b200.linear(x, w).double() - want).norm() / want.norm()) < 1.08 * model
+
+
 @pytest.mark.parametrize("fmt,n", [("dense", 192000), ("fp8", 152064), ("int4", 290000)])
 def test_linear_whose_sums_leave_no_ring(fmt, n):
     """Vocabulary-sized outputs of rows of 8192 k, 16 tokens: sizes that stay with the kernel whose activations are in shared memory (csrc/gemv_mma.cuh), and
