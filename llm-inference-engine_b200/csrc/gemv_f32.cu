@@ -19,8 +19,7 @@ int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStrea
     }
     const bool b16 = dtype == B200_BF16 || dtype == B200_F16;
     // up to 8 tokens of INT4 weights, dense rows of at most 3072 k: straight from global memory into registers (gemv_qd.cuh, with both sides' times)
-    // (it has no waits on a barrier of its own: a thread that has set their limit to zero, so that they run out, gets the kernels that have)
-    if (b16 && fmt != WF_FP8 && wait_guard().clocks != 0) {
+    if (b16 && fmt != WF_FP8) {
         const int rc = dtype == B200_BF16 ? launch_gemv_qd_bf16(a, fmt, swiglu, st) : launch_gemv_qd_f16(a, fmt, swiglu, st);
         if (rc != B200_ERR_UNSUPPORTED) return rc;
     }

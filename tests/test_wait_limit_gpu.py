@@ -55,10 +55,8 @@ def test_a_barrier_that_nothing_arrives_at():
     assert bool((b200.linear(x, w) == 256).all())
 
 
-@pytest.mark.parametrize("fmt", ["dense", "fp8", "int4"])
-@pytest.mark.parametrize("m", [2, 13])
-@pytest.mark.parametrize("k,n", [(256, 40), (2048, 4736), (8192, 2400)])
-def test_streaming_gemv(fmt, m, k, n):
+def streamed(fmt, m, k, n):
+    """A linear's call."""
     gen = torch.Generator(device=DEV).manual_seed(k + n + m)
     x = torch.randn(m, k, generator=gen, device=DEV).bfloat16()
     kw = {}
@@ -70,11 +68,32 @@ def test_streaming_gemv(fmt, m, k, n):
     else:
         w = torch.randint(0, 256, (n, k // 2), generator=gen, device=DEV, dtype=torch.uint8)
         kw = dict(w_format=b200.W_INT4, scales=torch.ones(n, k // 128, device=DEV).bfloat16(), zeros=torch.full((n, k // 128), 8, device=DEV, dtype=torch.uint8), group=128, N=n)
-    call = lambda: b200.linear(x, w, **kw)  # noqa: E731
+    return lambda: b200.linear(x, w, **kw)
+
+
+@pytest.mark.parametrize("fmt,m,k,n", [("fp8", m, k, n) for m in (2, 13) for k, n in ((256, 40), (2048, 4736), (8192, 2400))]
+                         + [("int4", 13, k, n) for k, n in ((256, 40), (2048, 4736), (8192, 2400))] + [("int4", 8, 11008, 2400)]
+                         + [("dense", m, k, n) for m in (2, 13) for k, n in ((3200, 40), (4096, 4736), (8192, 2400))])
+def test_streaming_gemv(fmt, m, k, n):
+    call = streamed(fmt, m, k, n)
     want = call()
     got = run_out(call, GEMV)
     assert bool(torch.isnan(got).all())
     assert torch.equal(call(), want) and not bool(torch.isnan(want).any())
+
+
+@pytest.mark.parametrize("fmt,m,k,n", [("int4", m, k, n) for m in (1, 2, 8) for k, n in ((256, 40), (2048, 4736), (8192, 2400))]
+                         + [("dense", m, k, n) for m in (1, 2, 13) for k, n in ((256, 40), (2048, 4736), (3072, 2400))])
+def test_linears_without_a_wait(fmt, m, k, n):
+    """The limit is no choice between kernels: a linear that streams into registers waits for no barrier, whatever the limit."""
+    call = streamed(fmt, m, k, n)
+    want = call()
+    b200.lib().b200_wait_limit(0)
+    got = call()
+    b200.lib().b200_wait_limit(2 ** 32 - 1)
+    torch.cuda.synchronize()
+    assert b200.wait_error() == 0
+    assert torch.equal(got, want) and not bool(torch.isnan(want).any())
 
 
 @pytest.mark.parametrize("m,k,n", [(512, 64, 4928), (2048, 128, 4096)])
