@@ -54,6 +54,46 @@ def test_experts_of_few_tokens(monkeypatch, dtype, tol, u, width, ff, experts, t
         assert open_rows.mean() <= (0.0 if experts == top else 0.6 if n >= 8 else 1.0), (n, open_rows)
 
 
+def ordered(h, W, p, ml):
+    """The router's choice among equals and among what is not finite: the largest logits, of equals the smaller index first, a NaN never; what then is missing has
+    no weight (its expert here is 0)."""
+    logits, top = (h @ W[p + "router"].T).tolist(), ml["router"]["top"]
+    chosen, weight = torch.zeros(len(logits), top, dtype=torch.long), torch.zeros(len(logits), top, dtype=torch.float64)
+    for t, row in enumerate(logits):
+        for k, e in enumerate(sorted((e for e in range(len(row)) if row[e] == row[e]), key=lambda e: (-row[e], e))[:top]):
+            chosen[t, k], weight[t, k] = e, 0.0 if row[e] == -math.inf else 1.0 / (1.0 + math.exp(-row[e]))
+    return chosen, weight
+
+
+@pytest.mark.parametrize("dtype,tol", [("bfloat16", 4e-2), ("float16", 6e-3), ("float32", 2e-5)])
+@pytest.mark.parametrize("experts,top", [(3, 3), (7, 4), (32, 6), (33, 6), (128, 6), (200, 4)])
+def test_choices_among_equals_and_what_is_not_finite(monkeypatch, dtype, tol, experts, top):
+    """Every routing kernel of csrc/moe.cu: decode batches (16-bit, up to 64 tokens), prompts from 512 tokens on, and what lies between.  A router row has one weight, on
+    a channel that is large and of either sign: equal weights give equal logits, 0 and -0 too, an infinite one plus or minus infinity, a NaN NaN."""
+    layer = ref.attention_layer(heads=2, kv_heads=1, dim=16, size=50, mlp=ref.moe(experts=experts, top=top, ff=32, shared_ff=32))
+    config = ref.make_config([layer], width=64, vocab=80)
+    W, packed = ref.make_weights(config, seed=4)
+    values = ([math.nan, 0.25, math.inf] if experts == 3 else [math.nan, 0.5, -0.0, 0.5, 0.0, -0.5, math.inf] if experts == 7 else
+              [0.5, -0.5, math.nan, 0.0, math.inf, -0.0, -0.5, 0.5, 0.0, 0.0, 0.25, -math.inf, math.inf] + [[0.0, 0.25, -0.25, -0.0][e % 4] for e in range(13, experts)])
+    router = torch.zeros(experts, 64)
+    router[:, 5] = torch.tensor(values)
+    packed["l0.mlp.router"] = router.to(torch.bfloat16)
+    packed["embed"][:, 5] = torch.where(torch.arange(80) % 3 == 0, -4.0, 4.0).to(torch.bfloat16)
+    for name in ("l0.mlp.router", "embed"):
+        W[name] = packed[name].to(torch.float64)
+    model = importlib.import_module("llm-inference-engine_b200.models.vasolix").VasolixModel(config, packed, dtype=dtype, device="cuda:0", max_tokens=640, max_seqs=2,
+                                                                                              max_pages_per_seq=10)
+    serving = importlib.import_module("llm-inference-engine_b200.serving")
+    monkeypatch.setattr(ref, "route", ordered)
+    for n in (1, 2, 9, 40, 64, 65, 512, 600):
+        toks = np.random.default_rng(n).integers(0, 80, n).tolist()
+        sess = serving.Session(model, 1280, max_seqs=2, max_batch_tokens=640, poison=True)
+        got = sess.feed([(sess.open(), toks, range(n))]).cpu().numpy()
+        want = ref.forward(config, W, toks).numpy()
+        err = np.linalg.norm(got - want, axis=-1) / np.linalg.norm(want, axis=-1)
+        assert (err < tol).all(), (n, err.max())
+
+
 @pytest.mark.parametrize("dtype,tol", [("bfloat16", 4e-2), ("float16", 6e-3)])
 @pytest.mark.parametrize("n", [8, 9, 16])
 def test_same_experts_for_every_token_of_a_decode_batch(dtype, tol, n):
