@@ -1877,11 +1877,13 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         const int n_up = inner_cols * l.expert_ff;
         float *gate = l.shared_ff > 0 ? shared_gate : nullptr;
         const bool weigh_x = !softmax && !sum_norm;  // sigmoid scores weigh the experts' inputs: the fp32 residual row, or (sum_norm) the convolved row the router read
-        int *tile_live = nullptr;
+        int *tile_live = nullptr, live_rows = std::min(NT, kMoeTileM);  // (a token chooses an expert once)
         rc = B200_ERR_UNSUPPORTED;
         if (weigh_x && !l.gated && !tc && moe_few_rows_takes(dt, 1, n_up, width, m->xg, l.w_up) && moe_few_rows_takes(dt, 1, width, l.expert_ff, m->u, l.w_down)) {
             rc = launch_moe_few_plan(dt, m->f32a, outputs, m->x, m->xg, pair_row, tile_expert, row_token, n_live, gate, NT, l.experts, l.top, width, st);
-            if (rc == B200_OK) tile_live = row_token;  // (its place: the rows' tokens are not needed)
+            // eight rows a pass, or sixteen where many experts have more than eight: a pass reads an expert's weights (4 layers, 8 / 16 rows, us a step: 3 of 3 experts, 16 and
+            // 64 tokens 367 / 351 and 825 / 789; 8 of 32, 24 tokens 661 / 623; 4 of 32, 32 tokens 630 / 615, 24 tokens 593 / 596; 2 of 8, 12 tokens 348 / 351)
+            if (rc == B200_OK) tile_live = row_token, live_rows = NT > 8 && pairs > 4 * l.experts ? 16 : 8;  // (its place: the rows' tokens are not needed)
         } else if (!softmax && moe_route_plan_bytes(NT, l.experts) <= (size_t)max_rows * width * es) {  // (the counts lie where the gather puts its rows)
             rc = launch_moe_route_plan(m->f32a, outputs, sel_expert, sel_weight, gate, (int *)m->xg, row_token, row_weight, tile_expert, pair_row, n_live, NT, l.experts, l.top, tile, st);
         }
@@ -1896,13 +1898,13 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         const int up_act = l.gated ? -1 : l.act;
         char *inner = (char *)m->u;
         if (tc) RUN(launch_gemm_tc_grouped(m->xg, l.w_up, m->u, max_rows, n_up, width, l.experts, tile_expert, n_live, up_act, dt, st));
-        else RUN(launch_moe_grouped_gemm(dt, m->xg, l.w_up, m->u, tile_expert, n_live, max_tiles, n_up, width, up_act, st, std::min(NT, kMoeTileM), tile_live));  // (a token chooses an expert once)
+        else RUN(launch_moe_grouped_gemm(dt, m->xg, l.w_up, m->u, tile_expert, n_live, max_tiles, n_up, width, up_act, st, live_rows, tile_live));
         if (l.gated) {
             inner += (size_t)max_rows * n_up * es;
             RUN(launch_gated_activation(dt, m->u, inner, max_rows, l.expert_ff, l.act, n_live, tile, st, l.act_limit, l.act_slope));
         }
         if (tc) RUN(launch_gemm_tc_grouped(inner, l.w_down, m->yrows, max_rows, width, l.expert_ff, l.experts, tile_expert, n_live, -1, dt, st));
-        else RUN(launch_moe_grouped_gemm(dt, inner, l.w_down, m->yrows, tile_expert, n_live, max_tiles, width, l.expert_ff, -1, st, std::min(NT, kMoeTileM), tile_live));
+        else RUN(launch_moe_grouped_gemm(dt, inner, l.w_down, m->yrows, tile_expert, n_live, max_tiles, width, l.expert_ff, -1, st, live_rows, tile_live));
         if (l.shared_ff > 0) {
             char *sin = (char *)m->us;
             RUN(linear(m, h2, l.w_shared_up, m->us, NT, width, inner_cols * l.shared_ff, st));

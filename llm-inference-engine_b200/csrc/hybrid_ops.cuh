@@ -248,7 +248,8 @@ int launch_bias_activation(int dtype, void *x, const float *bias, size_t rows, i
 int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, int N, int K, int experts, const int *tile_expert,
                            const int *n_live, int act, int dtype, cudaStream_t st);
 // c[row, n] = act?(sum_k a[row, k] * w[tile_expert[row / kMoeTileM]][n, k]);  rows >= n_tiles * kMoeTileM are skipped
-// live_rows: rows at the head of every tile that a caller reads afterwards (the others may stay unwritten); tile_live (moe_few_rows_takes): each tile's own number
+// live_rows: rows at the head of every tile that a caller reads afterwards (the others may stay unwritten); tile_live (moe_few_rows_takes): each tile's own number, taken 8 or
+// 16 (live_rows) at a time
 int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, const int *tile_expert, const int *n_tiles, int max_tiles,
                             int N, int K, int act, cudaStream_t st, int live_rows = kMoeTileM, const int *tile_live = nullptr);
 // y fp32 [M, N] = x [M, K] * w[N, K]^T for 16-bit x and w on the tensor cores (fp32 accumulation, fp32 result); B200_ERR_UNSUPPORTED for

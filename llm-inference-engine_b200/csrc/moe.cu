@@ -936,7 +936,7 @@ int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, co
                             int N, int K, int act, cudaStream_t st, int live_rows, const int *tile_live) {
     if (max_tiles == 0) return B200_OK;
     // a decode batch: up to 16 live rows per tile, slices of K for 16 warps at most, whole 32-k blocks
-    if (moe_few_rows_takes(dtype, tile_live ? 1 : live_rows, N, K, a, w)) {
+    if (moe_few_rows_takes(dtype, live_rows, N, K, a, w)) {
         const int KS = (K / 32 + 7) / 8, NG = KS >= 8 ? 1 : 8 / KS;
         const int units = (N / 8 + NG - 1) / NG, steps = std::max(1, std::min(8, units * max_tiles / (2 * sm_count())));
         const dim3 grid((units + steps - 1) / steps, max_tiles);
@@ -945,8 +945,8 @@ int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, co
             using T = std::remove_pointer_t<decltype(type)>;
             launch_plain(kern, dim3(grid), dim3(KS * NG * 32), smem, st, (const T *)a, (const T *)w, (T *)c, tile_expert, n_tiles, tile_live, kMoeTileM, max_tiles * kMoeTileM, N, K, act, KS, NG, steps);
         };
-        if (dtype == B200_BF16) live_rows <= 8 || tile_live ? go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 1>, (__nv_bfloat16 *)nullptr) : go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 2>, (__nv_bfloat16 *)nullptr);
-        else live_rows <= 8 || tile_live ? go(moe_few_rows_kernel<__half, __half, 1>, (__half *)nullptr) : go(moe_few_rows_kernel<__half, __half, 2>, (__half *)nullptr);
+        if (dtype == B200_BF16) live_rows <= 8 ? go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 1>, (__nv_bfloat16 *)nullptr) : go(moe_few_rows_kernel<__nv_bfloat16, __nv_bfloat16, 2>, (__nv_bfloat16 *)nullptr);
+        else live_rows <= 8 ? go(moe_few_rows_kernel<__half, __half, 1>, (__half *)nullptr) : go(moe_few_rows_kernel<__half, __half, 2>, (__half *)nullptr);
         return cuda_status("moe_few_rows launch");
     }
     if (dtype != B200_F32 && K % 8 == 0) {

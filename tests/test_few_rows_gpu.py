@@ -94,6 +94,33 @@ def test_choices_among_equals_and_what_is_not_finite(monkeypatch, dtype, tol, ex
         assert (err < tol).all(), (n, err.max())
 
 
+@pytest.mark.parametrize("dtype,tol,u", [("bfloat16", 4e-2, 2.0 ** -8), ("float16", 6e-3, 2.0 ** -11)])
+@pytest.mark.parametrize("experts,top", [(40, 4), (256, 2), (8, 4), (32, 8), (12, 4)])
+def test_sparse_choices_of_decode_batches(monkeypatch, dtype, tol, u, experts, top):
+    """Up to 64 tokens whose choices scatter over the experts: tiles of one row to about thirty, in passes of eight rows or sixteen (12 and 32 experts: either, by the
+    number of tokens); every row whose choice is not open within 16-bit rounding.  The embeddings lean towards the router's rows, so that most choices are sure."""
+    layer = ref.attention_layer(heads=2, kv_heads=1, dim=16, size=50, mlp=ref.moe(experts=experts, top=top, ff=96, shared_ff=64))
+    config = ref.make_config([layer], width=512, vocab=80)
+    W, packed = ref.make_weights(config, seed=3)
+    gen = torch.Generator().manual_seed(experts)
+    router = W["l0.mlp.router"]
+    meant = torch.stack([torch.randperm(experts, generator=gen)[:top] for _ in range(80)])
+    lean = torch.zeros(80, experts, dtype=torch.float64).scatter_(1, meant, 12.0) @ torch.nn.functional.normalize(router, dim=-1)
+    packed["embed"] = (W["embed"] + lean).to(torch.bfloat16)
+    W["embed"] = packed["embed"].to(torch.float64)
+    model = importlib.import_module("llm-inference-engine_b200.models.vasolix").VasolixModel(config, packed, dtype=dtype, device="cuda:0", max_tokens=128, max_seqs=20,
+                                                                                              max_pages_per_seq=2)
+    serving = importlib.import_module("llm-inference-engine_b200.serving")
+    for n in (9, 12, 13, 16, 17, 24, 25, 32, 33, 63, 64, 65):
+        toks = np.random.default_rng(n).integers(0, 80, n).tolist()
+        sess = serving.Session(model, 2560, max_seqs=20, max_batch_tokens=128, poison=True)
+        got = sess.feed([(sess.open(), toks, range(n))]).cpu().numpy()
+        want, open_rows = ambiguous_rows(monkeypatch, config, W, toks, u)
+        err = np.linalg.norm(got - want, axis=-1) / np.linalg.norm(want, axis=-1)
+        assert (err[~open_rows] < tol).all(), (n, err, open_rows)
+        assert open_rows.mean() <= 0.3, (n, open_rows)
+
+
 @pytest.mark.parametrize("dtype,tol", [("bfloat16", 4e-2), ("float16", 6e-3)])
 @pytest.mark.parametrize("n", [8, 9, 16])
 def test_same_experts_for_every_token_of_a_decode_batch(dtype, tol, n):
