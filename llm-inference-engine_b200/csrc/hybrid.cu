@@ -1884,7 +1884,8 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             // eight rows a pass, or sixteen where many experts have more than eight: a pass reads an expert's weights (4 layers, 8 / 16 rows, us a step: 3 of 3 experts, 16 and
             // 64 tokens 367 / 351 and 825 / 789; 8 of 32, 24 tokens 661 / 623; 4 of 32, 32 tokens 630 / 615, 24 tokens 593 / 596; 2 of 8, 12 tokens 348 / 351)
             if (rc == B200_OK) tile_live = row_token, live_rows = NT > 8 && pairs > 4 * l.experts ? 16 : 8;  // (its place: the rows' tokens are not needed)
-        } else if (!softmax && moe_route_plan_bytes(NT, l.experts) <= (size_t)max_rows * width * es) {  // (the counts lie where the gather puts its rows)
+        }
+        if (rc == B200_ERR_UNSUPPORTED && !softmax && moe_route_plan_bytes(NT, l.experts) <= (size_t)max_rows * width * es) {  // (the counts lie where the gather puts its rows)
             rc = launch_moe_route_plan(m->f32a, outputs, sel_expert, sel_weight, gate, (int *)m->xg, row_token, row_weight, tile_expert, pair_row, n_live, NT, l.experts, l.top, tile, st);
         }
         if (rc != B200_OK && rc != B200_ERR_UNSUPPORTED) return rc;

@@ -122,6 +122,27 @@ def test_sparse_choices_of_decode_batches(monkeypatch, dtype, tol, u, experts, t
 
 
 @pytest.mark.parametrize("dtype,tol", [("bfloat16", 4e-2), ("float16", 6e-3)])
+@pytest.mark.parametrize("n", [511, 512, 1000, 1023])
+def test_prompts_of_one_expert_each(monkeypatch, dtype, tol, n):
+    """16-bit prompts of fewer than 1024 pairs, whose experts run on 64-row tiles: from 512 tokens on their choice and their plan run in many CTAs."""
+    layer = ref.attention_layer(heads=2, kv_heads=1, dim=16, size=50, mlp=ref.moe(experts=5, top=1, ff=64, shared_ff=64))
+    config = ref.make_config([layer], width=64, vocab=80)
+    W, packed = ref.make_weights(config, seed=2)
+    model = importlib.import_module("llm-inference-engine_b200.models.vasolix").VasolixModel(config, packed, dtype=dtype, device="cuda:0", max_tokens=1024, max_seqs=1,
+                                                                                              max_pages_per_seq=16)
+    toks = np.random.default_rng(n).integers(0, 80, n).tolist()
+    sess = importlib.import_module("llm-inference-engine_b200.serving").Session(model, 1024, max_seqs=1, max_batch_tokens=1024, poison=True)
+    rid = sess.open()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        got = sess.feed([(rid, toks, range(n))]).cpu().numpy()
+    kernels = " ".join(e.key for e in prof.key_averages())
+    assert ("moe_route_count_kernel" in kernels) == (n >= 512) and ("moe_plan_kernel" in kernels) == (n < 512), kernels
+    want, open_rows = ambiguous_rows(monkeypatch, config, W, toks, 2.0 ** -8 if dtype == "bfloat16" else 2.0 ** -11)
+    err = np.linalg.norm(got - want, axis=-1) / np.linalg.norm(want, axis=-1)
+    assert (err[~open_rows] < tol).all() and open_rows.mean() <= 0.6
+
+
+@pytest.mark.parametrize("dtype,tol", [("bfloat16", 4e-2), ("float16", 6e-3)])
 @pytest.mark.parametrize("n", [8, 9, 16])
 def test_same_experts_for_every_token_of_a_decode_batch(dtype, tol, n):
     """n sequences of one and the same token: every row of the two experts' tiles is live, the last one too."""
