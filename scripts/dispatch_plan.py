@@ -1,8 +1,9 @@
 #!/usr/bin/env python
 """Which kernel, how many passes over the weights and which ring geometry each linear of a decode step gets -- a Python MODEL of the host-side
 dispatch (no GPU): decoder.cu norm_linear (norm inside the GEMV for one dense token, a norm kernel in front otherwise), gemv_f32.cu launch_gemv_nk
-(gemv_qd for up to 8 tokens of INT4 and short dense rows, gemv_rs, what its ring refuses on gemv_mma, the SIMT GEMV for up to 4 tokens), linear.cu (GEMV passes, tcgen05 GEMM for dense M > 16), gemv_inst.cuh,
-gemv_rs.cuh gemv_rs_geometry and gemv_mma.cuh gemv_mma_geometry.  It restates those few formulas; when they change, this file must follow
+(gemv_qd for up to 8 tokens of INT4 and short dense rows, gemv_rs, what its ring refuses on gemv_mma, gemv_sr for one token of short rows, the SIMT GEMV for up
+to 4 tokens), linear.cu (GEMV passes, tcgen05 GEMM for dense M > 16), gemv_inst.cuh, gemv_qd.cuh launch_gemv_qd_t, gemv_sr.cuh launch_gemv_sr_t, gemv_rs.cuh
+gemv_rs_geometry and gemv_mma.cuh gemv_mma_geometry.  It restates those few formulas; when they change, this file must follow
 (tests/test_dispatch_plan.py).
 usage: python scripts/dispatch_plan.py > profiles/<tag>_dispatch_plan.txt"""
 BUDGET = 224 * 1024
@@ -98,25 +99,35 @@ def gemv_rs_plan(M, K, N, fmt, swiglu=False):
 
 
 def gemv_qd_plan(M, K, N, fmt, swiglu=False):
-    """gemv_qd.cuh launch_gemv_qd_t (INT4 in groups of 128 of 1..8 tokens, short dense rows of 1..16): None when unsupported.  It is the form of gemv_rs
-    whose ring is in registers."""
+    """gemv_qd.cuh launch_gemv_qd_t (16-bit activations; INT4 in groups of 128 of 1..8 tokens, dense rows of at most 3072 k of 1..16): None when unsupported.
+    warps: of a CTA (8: two CTAs per SM); barriers: of a unit of 16 rows."""
     dense = fmt == "dense"
-    if fmt == "fp8" or M < 1 or M > (16 if dense else 8) or K % 128 or (dense and K > 3072):
+    if fmt == "fp8" or M < 1 or M > (16 if dense else 8) or K % 128 or (dense and K > 3072) or (swiglu and N // 2 % 8):
         return None
-    if dense:
-        warps = 16 if (K >= 2048 if M > 8 else K > 2048) else 8
-    else:
-        warps = 16 if K >= 8192 else 8
-    smem = M * (2 * K + 64) + 256 + 2 * warps * (16 if M > 8 else 8) * 20 * 4
-    if smem > (108 if dense else 160) * 1024 * warps // 16:
+
+    def smem(warps):
+        return M * (2 * K + 64) + 256 + 2 * (warps if dense else 16) * (16 if M > 8 else 8) * 20 * 4
+
+    budget = (108 if dense else 160) * 1024
+    warps = 16 if K > (2048 if dense else 4096) or smem(8) > budget // 2 else 8
+    if dense and warps == 16 and smem(16) > budget:
+        budget = 148 * 1024
+    if smem(warps) > budget * warps // 16:
         return None
-    return dict(kernel="gemv_rs", form="gemv_qd", warps=warps, pieces=1, piece_bytes=K * 2 if dense else K // 2, stages=2, smem=smem)
+    return dict(kernel="gemv_qd", warps=warps, smem=smem(warps), budget=budget, barriers=1 if dense or warps == 8 else -(-K // 4096))
 
 
-def gemv_any(M, K, N, fmt, swiglu=False):
-    """gemv_f32.cu launch_gemv_nk for a 16-bit model."""
+def gemv_sr_plan(M, K, ebytes=2):
+    """gemv_sr.cuh launch_gemv_sr_t (dense rows, norm in front or not; one 16-bit token, one to four fp32 tokens): None when unsupported."""
+    if M < 1 or M > (1 if ebytes == 2 else 4) or K > (3072 if ebytes == 2 else 1536) or K % (32 * 16 // ebytes):
+        return None
+    return dict(kernel="gemv_sr", smem=(M if M <= 2 else 4) * K * 4 + K * ebytes)
+
+
+def gemv_any(M, K, N, fmt, swiglu=False, push=False):
+    """gemv_f32.cu launch_gemv_nk for a 16-bit model; push: a tensor-parallel rank's partial, which the kernels with a ring of registers leave to the others."""
     g = gemv_qd_plan(M, K, N, fmt, swiglu)
-    if g:
+    if g and not push:
         return g
     if M <= 16 and (M >= 2 or fmt != "dense"):
         rows = 16 if fmt == "fp8" else 8
@@ -124,19 +135,17 @@ def gemv_any(M, K, N, fmt, swiglu=False):
         g = gemv_rs_plan(M, K, N, fmt, swiglu) or gemv_mma_plan(M, K, fmt, -(-units // max(1, min(SMS, units))))
         if g:
             return g
-    return gemv_nk_plan(M, K, fmt)
+    return (fmt == "dense" and not push and gemv_sr_plan(M, K)) or gemv_nk_plan(M, K, fmt)
 
 
-def linear_plan(M, K, N, fmt, fused_rows=16, swiglu=False):
+def linear_plan(M, K, N, fmt, fused_rows=16, swiglu=False, push=False):
     """One linear of the decode step: (path, passes over the weights, geometry)."""
     if M == 1 and fmt == "dense":  # the norm / residual / tensor-parallel prologue inside the GEMV
-        g = gemv_nk_plan(M, K, fmt)
-        if g and K <= 3072 and K % 256 == 0:  # gemv_sr.cuh launch_gemv_sr_t: the form of gemv_nk with whole rows per warp
-            g = dict(kernel="gemv_nk", form="gemv_sr", pieces=1, piece_bytes=K * 2, stages=2)
+        g = (not push and gemv_sr_plan(M, K)) or gemv_nk_plan(M, K, fmt)
         if g:
             return ("fused " + g["kernel"], 1, g)
     if M <= fused_rows:
-        g = gemv_any(M, K, N, fmt, swiglu)
+        g = gemv_any(M, K, N, fmt, swiglu, push)
         if g:
             return ("norm_kernel + " + g["kernel"], 1, g)
     if fmt == "dense" and M > 4:
@@ -156,8 +165,13 @@ def step_plan(name, hidden, heads, kv_heads, d, inter, tp, batch, fmt):
               ("down", inter // tp, hidden)]
     lines = [f"{name}, batch {batch}, weights {fmt}" + (f", TP-{tp} (one rank)" if tp > 1 else "")]
     for lin, K, N in shapes:
-        path, passes, g = linear_plan(batch, K, N, fmt, fused_rows, lin == "gate_up")
-        geo = (f"pieces {g['pieces']} x {g['piece_bytes']} B, {g['stages']} stages" + (f", {g['parts']} activation parts of {g['part_k']} k" if g.get("parts") else "")) if g else "-"
+        path, passes, g = linear_plan(batch, K, N, fmt, fused_rows, lin == "gate_up", tp > 1 and lin in ("o", "down"))
+        if g and g["kernel"] == "gemv_qd":
+            geo = f"ring of registers, {16 // g['warps']} CTAs of {g['warps']} warps per SM, barriers per 16 rows: {g['barriers']}"
+        elif g and g["kernel"] == "gemv_sr":
+            geo = "ring of registers, 2 CTAs of 8 warps per SM, a row per warp"
+        else:
+            geo = (f"pieces {g['pieces']} x {g['piece_bytes']} B, {g['stages']} stages" + (f", {g['parts']} activation parts of {g['part_k']} k" if g.get("parts") else "")) if g else "-"
         wbytes = K * N * {"dense": 2, "fp8": 1, "int4": 0.5}[fmt]
         lines.append(f"  {lin:8s} K={K:6d} N={N:6d}  {path:58s} weights read {passes} x {wbytes / 1e6:7.1f} MB   {geo}")
     return lines
