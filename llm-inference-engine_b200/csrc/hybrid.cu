@@ -71,7 +71,6 @@ __global__ void embed_rows_kernel(const int *__restrict__ ids, const T *__restri
 
 // x[t, :] += rmsnorm(y[t, :]) * g (and h_out[t, :] = T(x[t, :]) for the next projection), where y is either a dense row (y_dense) or the mixture
 //   sum_k y_rows[pair_row[t*top + k], :] + shared_gate[t] * y_shared[t, :].   trace (optional) receives the new x.
-// (pair_row -1: a choice that found no expert left, with NaN among the router's logits; it adds nothing)
 template <typename T>
 __global__ void __launch_bounds__(256)
 postnorm_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, const T *__restrict__ y_rows, const int *__restrict__ pair_row,
@@ -98,9 +97,8 @@ postnorm_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, c
                 for (int i = 0; i < V; ++i) v[i] = 0.0f;
 #pragma unroll 4
                 for (int k = 0; k < top; ++k) {
-                    const int r = pair_row[(size_t)t * top + k];
                     float f[V];
-                    unpack16<T>(r >= 0 ? ld_v4(y_rows + (size_t)r * width + c) : make_uint4(0u, 0u, 0u, 0u), f);
+                    unpack16<T>(ld_v4(y_rows + (size_t)pair_row[(size_t)t * top + k] * width + c), f);
 #pragma unroll
                     for (int i = 0; i < V; ++i) v[i] += f[i];
                 }
@@ -160,10 +158,7 @@ postnorm_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, c
             v = Elem<T>::to_f(y_dense[(size_t)t * width + c]);
         } else {
             v = 0.0f;
-            for (int k = 0; k < top; ++k) {
-                const int r = pair_row[(size_t)t * top + k];
-                if (r >= 0) v += Elem<T>::to_f(y_rows[(size_t)r * width + c]);
-            }
+            for (int k = 0; k < top; ++k) v += Elem<T>::to_f(y_rows[(size_t)pair_row[(size_t)t * top + k] * width + c]);
             if (y_shared) v = fmaf(shared_gate[t], Elem<T>::to_f(y_shared[(size_t)t * width + c]), v);
         }
         ys[c] = v;

@@ -31,7 +31,7 @@ __global__ void moe_route_sigmoid_kernel(const float *__restrict__ logits, int l
         for (int e = lane; e < experts; e += 32) {
             bool taken = false;
             for (int p = 0; p < k; ++p) taken |= sel_expert[(size_t)t * top + p] == e;
-            const float v = z[e];
+            const float v = z[e] == z[e] ? z[e] : -INFINITY;  // (NaN is chosen last, with weight 0: every choice has a row)
             if (!taken && (v > best || (v == best && e < bi))) best = v, bi = e;
         }
         for (int o = 16; o > 0; o >>= 1) {
@@ -174,15 +174,15 @@ moe_plan_kernel(const int *__restrict__ sel_expert, const float *__restrict__ se
 }
 
 // The `top` largest of a token's logits by one warp, the smaller index first among equals, as moe_route_sigmoid_kernel chooses: z[j] is logit lane + 32 j
-// (a NaN, and what is past the last expert, is never chosen; with nothing left to choose the index is 0x7fffffff and the weight that of -inf).  Logits in an
-// order that unsigned integers keep, so that a choice is two reductions in hardware and not five rounds of two shuffles.
+// (a NaN counts as -inf, and there are at least `top` experts).  Logits in an order that unsigned integers keep, so that a choice is two reductions in hardware
+// and not five rounds of two shuffles.
 template <int J, typename Put>
 __device__ __forceinline__ void choose_sigmoid(const float (&z)[J], int lane, int experts, int top, Put put) {
     unsigned key[J];
 #pragma unroll
     for (int j = 0; j < J; ++j) {
         const unsigned b = __float_as_uint(z[j] + 0.0f);  // (-0 and +0 are equal)
-        key[j] = lane + 32 * j < experts && z[j] == z[j] ? ((b & 0x80000000u) ? ~b : b | 0x80000000u) : 0u;
+        key[j] = lane + 32 * j >= experts ? 0u : z[j] != z[j] ? 0x007fffffu : (b & 0x80000000u) ? ~b : b | 0x80000000u;  // (0: past the last expert, or taken)
     }
     for (int k = 0; k < top; ++k) {
         unsigned mine = key[0];
@@ -192,12 +192,12 @@ __device__ __forceinline__ void choose_sigmoid(const float (&z)[J], int lane, in
         unsigned at = 0x7fffffffu;
 #pragma unroll
         for (int j = J - 1; j >= 0; --j)
-            if (best != 0u && key[j] == best) at = lane + 32 * j;
+            if (key[j] == best) at = lane + 32 * j;
         at = __reduce_min_sync(0xffffffffu, at);
 #pragma unroll
         for (int j = 0; j < J; ++j)
             if (lane + 32 * j == (int)at) key[j] = 0u;
-        const float v = best == 0u ? -INFINITY : __uint_as_float((best & 0x80000000u) ? best & 0x7fffffffu : ~best);
+        const float v = __uint_as_float((best & 0x80000000u) ? best & 0x7fffffffu : ~best);
         put(k, (int)at, 1.0f / (1.0f + expf(-v)));  // sigmoid is monotone: the largest logit has the largest score
     }
 }
@@ -236,7 +236,7 @@ moe_few_plan_kernel(const float *__restrict__ logits, int ld, const float *__res
             choose_sigmoid(z[i], lane, experts, top, [&](int k, int e, float w) {
                 if (lane == 0) {
                     sel[(warp + 8 * i) * top + k] = e, weight[(warp + 8 * i) * top + k] = w;
-                    if (e < experts) atomicOr(&chosen[e >> 5], 1u << (e & 31));
+                    atomicOr(&chosen[e >> 5], 1u << (e & 31));
                 }
             });
     __syncthreads();
@@ -256,11 +256,11 @@ moe_few_plan_kernel(const float *__restrict__ logits, int ld, const float *__res
 #pragma unroll
             for (int i = 0; i < 4; ++i) rank += q + i < p ? same[i] : 0, count += same[i];
         }
-        const int tile = e < experts ? tile_of(e) : -1;
+        const int tile = tile_of(e);
         if (tile == (int)blockIdx.x) list[rank] = p, live = count;
         if (blockIdx.x == 0) {
-            pair_row[p] = tile >= 0 ? tile * kMoeTileM + rank : -1;
-            if (tile >= 0 && rank == 0) tile_expert[tile] = e, tile_live[tile] = count;
+            pair_row[p] = tile * kMoeTileM + rank;
+            if (rank == 0) tile_expert[tile] = e, tile_live[tile] = count;
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -312,7 +312,7 @@ moe_route_count_kernel(const float *__restrict__ logits, int ld, int *__restrict
             choose_sigmoid(z[i], lane, experts, top, [&](int k, int e, float w) {
                 if (lane == 0) {
                     sel_expert[(size_t)(first + i) * top + k] = e, sel_weight[(size_t)(first + i) * top + k] = w;
-                    if (e < experts) atomicAdd(&count[e], 1);
+                    atomicAdd(&count[e], 1);
                 }
             });
     if (shared_gate && lane < PER && first + lane < tokens) shared_gate[first + lane] = 1.0f / (1.0f + expf(-gate));
@@ -365,12 +365,8 @@ moe_place_kernel(const int *__restrict__ sel_expert, const float *__restrict__ s
     for (int p = lo + threadIdx.x; p < hi; p += 256) {
         const int e = sel_expert[p];
         const float w = sel_weight[p];
-        if (e < experts) {
-            const int r = offset[e] + atomicAdd(&next[e], 1);
-            row_token[r] = p / top, row_weight[r] = w, pair_row[p] = r;
-        } else {
-            pair_row[p] = -1;
-        }
+        const int r = offset[e] + atomicAdd(&next[e], 1);
+        row_token[r] = p / top, row_weight[r] = w, pair_row[p] = r;
     }
 }
 

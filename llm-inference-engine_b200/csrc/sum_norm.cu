@@ -90,9 +90,8 @@ sum_norm_kernel(float *x, const T *__restrict__ y_dense, const T *__restrict__ y
 #pragma unroll
             for (int i = 0; i < N; ++i) v[i] = 0.0f;
             for (int k = 0; k < top; ++k) {
-                const int r = pair_row[(size_t)t * top + k];
-                float f[N] = {};
-                if (r >= 0) ld_t<T, N>(y_rows + (size_t)r * width + c, f);
+                float f[N];
+                ld_t<T, N>(y_rows + (size_t)pair_row[(size_t)t * top + k] * width + c, f);
 #pragma unroll
                 for (int i = 0; i < N; ++i) v[i] += f[i];
             }
