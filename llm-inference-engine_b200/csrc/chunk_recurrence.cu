@@ -26,7 +26,7 @@ namespace b200 {
 namespace {
 
 constexpr int kC = 32;      // tokens per chunk
-constexpr int kCols = 16;   // columns of S per CTA of the scan (the M of its matrix instructions)
+constexpr int kCols = 16;   // columns of S per CTA of the scan
 
 // one (chunk, head) block, rows as the scan has them in shared memory: Qp, (delta rule: Kp,) Ke [kC][kP], P [kC][kTP], p_C [DK], (Tb [kC][kTP])
 constexpr int kTP = 40;  // floats per row of P and Tb and per column of V^T

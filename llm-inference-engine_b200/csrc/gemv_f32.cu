@@ -18,7 +18,7 @@ int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStrea
         return B200_ERR_INVALID_ARG;
     }
     const bool b16 = dtype == B200_BF16 || dtype == B200_F16;
-    // up to 8 tokens of INT4 weights, dense rows of at most 3072 k: straight from global memory into registers (gemv_qd.cuh, with both sides' times)
+    // up to 8 tokens of INT4 weights, up to 16 of dense rows of at most 3072 k: straight from global memory into registers (gemv_qd.cuh, with both sides' times)
     if (b16 && fmt != WF_FP8) {
         const int rc = dtype == B200_BF16 ? launch_gemv_qd_bf16(a, fmt, swiglu, st) : launch_gemv_qd_f16(a, fmt, swiglu, st);
         if (rc != B200_ERR_UNSUPPORTED) return rc;
@@ -37,7 +37,7 @@ int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStrea
         if (rc != B200_ERR_UNSUPPORTED) return rc;
     }
     if (a.M > 4) return B200_ERR_UNSUPPORTED;
-    // one token of short rows (fp32: up to four) and its norm: whole rows per warp (gemv_sr.cuh, with both sides' times)
+    // one token of short rows (fp32: up to four), norm in front or not: whole rows per warp (gemv_sr.cuh, with both sides' times)
     {
         const int rc = dtype == B200_F32 ? launch_gemv_sr_t<float>(a, fmt, swiglu, st) : dtype == B200_BF16 ? launch_gemv_sr_t<__nv_bfloat16>(a, fmt, swiglu, st) : dtype == B200_F16 ? launch_gemv_sr_t<__half>(a, fmt, swiglu, st) : B200_ERR_UNSUPPORTED;
         if (rc != B200_ERR_UNSUPPORTED) return rc;

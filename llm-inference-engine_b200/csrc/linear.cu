@@ -1,7 +1,7 @@
 // linear.cu -- b200_linear / b200_batched_gemm and the weight packing helpers.
 //
 // Dispatch of y[M,N] = x[M,K] * W (reference src/kernels/linear.cu:10-158):
-//   M <= 16 (fp32: 4), W packed [N,K] (dense / FP8 / INT4) -> launch_gemv_nk (gemv_f32.cu: gemv_qd.cuh, gemv_rs.cuh, gemv_mma.cuh, gemv.cuh)
+//   M <= 16 (fp32: 4), W packed [N,K] (dense / FP8 / INT4) -> launch_gemv_nk (gemv_f32.cu: gemv_qd.cuh, gemv_rs.cuh, gemv_mma.cuh, gemv_sr.cuh, gemv.cuh)
 //   M <= 4, W dense  [K,N] (the reference's own memory order) -> gemv_kn_kernel (this file)
 //   M > 16, 16-bit activations, dense W packed [N,K] -> tcgen05 / TMEM tensor-core GEMM (gemm_tc.cu)
 //   everything else                              -> gemm_simt_kernel (tiled fp32-accumulate fallback, this file)

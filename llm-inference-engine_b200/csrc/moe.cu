@@ -205,8 +205,8 @@ __device__ __forceinline__ void choose_sigmoid(const float (&z)[J], int lane, in
 // A decode batch (at most 64 tokens, 256 choices, 256 experts): choice, plan and gather in one launch.  Every CTA chooses for all tokens -- 16 rows of logits, a
 // microsecond -- and knows the plan from that alone: an expert that was chosen owns one tile, in the experts' order, its rows are its pairs in order.  CTA b
 // gathers tile b, its live rows only (moe_few_rows_kernel reads no others).  Bound: latency, one chain of logits -> rows.
-// Measured (16 tokens, 4 of 32 experts, width 2048): three launches 5.4 + 6.1 + 4.3 us -> 7.5.  A whole Vasolix-shaped decode step of 17 / 32 / 64 requests, whose
-// experts otherwise run on 64-row tiles: 761 / 853 / 1034 -> 571 / 674 / 932 us.
+// Measured (16 tokens, 4 of 32 experts, width 2048, under the profiler): three launches 5.4 + 6.1 + 4.3 us -> 9.7 (7.5 with two tokens a warp, which end at 16).
+// A Vasolix-shaped decode step of four layers, 17 / 32 / 64 requests, whose experts otherwise run on 64-row tiles: 753 / 804 / 937 -> 551 / 628 / 786 us.
 constexpr int kFewTokens = 64, kFewPairs = 256, kFewExperts = 256;
 template <typename T, int J>  // J: logits of a token per lane
 __global__ void __launch_bounds__(256)
@@ -728,7 +728,7 @@ moe_grouped_gemm_mma_kernel(const T *__restrict__ a, const T *__restrict__ w, TC
 // grid (unit groups, tiles); a CTA runs `steps` groups of NG units of 8 rows.  NT 1: at most 8 live rows, 2: at most 16.  A tile's rows start at its
 // number times tile_rows; rows >= M, or from tile_live on (a 16-row read of every CTA was 40 % of what it took from L2 beside its weights), are neither read nor
 // stored.  tile_expert and n_tiles NULL: one weight, every tile of the grid.
-// Measured (2048 x 512 experts, 16 tokens x 4 of 32, 59 MB): up and down 40 and 30 -> 19 us each; live rows only, eight at a time, CTAs of one wave: 14.5.
+// Measured (2048 x 512 experts, 16 tokens x 4 of 32, 59 MB): up and down 40 and 30 -> 19 us each; live rows only, eight at a time, CTAs of one wave: 13.6.
 template <typename T, typename TC, int NT>
 __global__ void __launch_bounds__(512)
 moe_few_rows_kernel(const T *__restrict__ a, const T *__restrict__ w, TC *__restrict__ c, const int *__restrict__ tile_expert,
