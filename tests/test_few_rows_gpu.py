@@ -55,8 +55,8 @@ def test_experts_of_few_tokens(monkeypatch, dtype, tol, u, width, ff, experts, t
 
 
 def ordered(h, W, p, ml):
-    """The router's choice among equals and among what is not finite: the largest logits, of equals the smaller index first, a NaN never; what then is missing has
-    no weight (its expert here is 0)."""
+    """The router's choice among equals and among what is not finite: the largest logits, of equals the smaller index first; minus infinity and NaN have no weight
+    (which of them is chosen makes no difference: a NaN is left out here, and expert 0 stands in its place)."""
     logits, top = (h @ W[p + "router"].T).tolist(), ml["router"]["top"]
     chosen, weight = torch.zeros(len(logits), top, dtype=torch.long), torch.zeros(len(logits), top, dtype=torch.float64)
     for t, row in enumerate(logits):
@@ -135,11 +135,13 @@ def test_prompts_of_one_expert_each(monkeypatch, dtype, tol, n):
     rid = sess.open()
     with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
         got = sess.feed([(rid, toks, range(n))]).cpu().numpy()
-    kernels = " ".join(e.key for e in prof.key_averages())
-    assert ("moe_route_count_kernel" in kernels) == (n >= 512) and ("moe_plan_kernel" in kernels) == (n < 512), kernels
     want, open_rows = ambiguous_rows(monkeypatch, config, W, toks, 2.0 ** -8 if dtype == "bfloat16" else 2.0 ** -11)
     err = np.linalg.norm(got - want, axis=-1) / np.linalg.norm(want, axis=-1)
     assert (err[~open_rows] < tol).all() and open_rows.mean() <= 0.6
+    kernels = " ".join(e.key for e in prof.key_averages())
+    if "kernel" not in kernels:
+        pytest.skip("no launch was recorded: the route is not seen")
+    assert ("moe_route_count_kernel" in kernels) == (n >= 512) and ("moe_plan_kernel" in kernels) == (n < 512), kernels
 
 
 @pytest.mark.parametrize("dtype,tol", [("bfloat16", 4e-2), ("float16", 6e-3)])
