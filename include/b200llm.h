@@ -119,6 +119,10 @@ int b200_linear(const void *x, const void *w, const void *scales, const void *ze
                 int M, int K, int N, int dtype, int w_format, int w_layout, int group,
                 b200_stream_t stream);
 
+/* y[M,N] = act(x . W^T + bias), W dense [N,K]: the sum is rounded to the type, then takes bias [N] (fp32 or NULL) and act (b200_act_t up to B200_ACT_RELU, -1:
+ * none), rounded again */
+int b200_linear_act(const void *x, const void *w, const float *bias, void *y, int M, int K, int N, int act, int dtype, b200_stream_t stream);
+
 /* launchLinearGemm (gate_up) + launchSiluAndMul in ONE kernel for prefill-sized token counts (src/layers/ffn.cpp:105-129,
  * src/kernels/silu_and_mul.cu:6-41): act[M, inter] = silu(x . Wgate^T) * (x . Wup^T), w_gate_up dense `dtype` [2*inter, K] (gate rows
  * first, the engine's packed layout).  Bit-identical to b200_linear followed by b200_silu_and_mul (gate and up are rounded to `dtype`

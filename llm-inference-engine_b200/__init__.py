@@ -130,6 +130,7 @@ SIGNATURES = {
     "b200_fused_add_bias_residual_rmsnorm": [_P, _P, _P, _P, _F, _I, _I, _I, _P],
     "b200_add_residual": [_P, _P, _I, _I, _I, _P],
     "b200_linear": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+    "b200_linear_act": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "b200_linear_swiglu": [_P, _P, _P, _I, _I, _I, _I, _P],
     "b200_batched_gemm": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "b200_quantize_fp8": [_P, _P, _P, _I, _I, _I, _P],
@@ -335,6 +336,16 @@ def linear(x, w, layout=LAYOUT_NK, w_format=W_DENSE, scales=None, zeros=None, gr
     if layout == LAYOUT_KN or M > 4:
         ensure_workspace()  # split-K partials
     check(lib().b200_linear(ptr(x), ptr(w), ptr(scales), ptr(zeros), ptr(y), M, K, N, dtype_code(x), w_format, layout, group, stream()))
+    return y
+
+
+def linear_act(x, w, bias=None, act=-1):
+    """act(x . W^T + bias) (b200_linear_act): w [N, K] dense, bias [N] fp32 or None, act a b200_act_t number or -1."""
+    torch = _torch()
+    M, K = x.shape
+    y = torch.empty((M, w.shape[0]), dtype=x.dtype, device=x.device)
+    ensure_workspace()
+    check(lib().b200_linear_act(ptr(x), ptr(w), ptr(bias), ptr(y), M, K, w.shape[0], act, dtype_code(x), stream()))
     return y
 
 

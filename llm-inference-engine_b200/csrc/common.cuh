@@ -472,6 +472,14 @@ __device__ __forceinline__ float act_apply(float v, int act) {
     return 0.5f * v * (1.0f + tanhf(c * (v + 0.044715f * v * v * v)));
 }
 
+// A linear's result with a bias and an activation (b200_act_t, -1: none) on it: what a separate pass over the stored row of T makes of it, rounded as that pass
+// finds it, so that the two agree in every bit.
+template <typename T> __device__ __forceinline__ float bias_act(float v, const float *bias, size_t n, int act) {
+    v = round_to<T>(v);
+    if (bias) v += __ldg(bias + n);
+    return act >= 0 ? act_apply(v, act) : v;
+}
+
 // ------------------------------------------------------------------ reductions
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

@@ -31,6 +31,7 @@ int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStrea
         const int rc = dtype == B200_BF16 ? launch_gemv_rs_bf16(a, fmt, swiglu, st) : launch_gemv_rs_f16(a, fmt, swiglu, st);
         if (rc != B200_ERR_UNSUPPORTED) return rc;
     }
+    if (a.finish) return B200_ERR_UNSUPPORTED;
     // what its ring leaves out (rows of more than 4096 k with so many outputs that their sums fill the SM): activations in shared memory (gemv_mma.cuh)
     if (b16 && (a.M >= 2 || fmt != WF_DENSE) && a.M <= 16) {
         const int rc = dtype == B200_BF16 ? launch_gemv_mma_bf16(a, fmt, swiglu, st) : launch_gemv_mma_f16(a, fmt, swiglu, st);

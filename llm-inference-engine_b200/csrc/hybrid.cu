@@ -10,11 +10,11 @@
 //   latent mixer:     split + rotation + latent-row norm + pool append -> grouped GEMM over the heads (q into the latent space) -> windowed
 //                     sink attention over the latent rows -> grouped GEMM over the heads (value up-projection) -> gate -> output projection
 //   post-norm + residual add (fp32)
-//   dense ff:         b200_linear up -> bias + act -> b200_linear down (its bias joins the residual kernel)
+//   dense ff:         b200_linear_act up (bias + act in its ending) -> b200_linear down (its bias joins the residual kernel)
 //   moe (softmax):    router (fp32) -> route -> plan -> gather rows -> grouped gate|up -> act(gate) * up -> grouped down; shared expert alike;
 //                     combine (weights on the outputs, identity experts return the input) + norm + residual add, one kernel
 //   moe:              router + shared gate (fp32) -> route -> plan -> gather (weight on the input) -> grouped up (+act) -> grouped down
-//                     shared expert: b200_linear up -> act -> b200_linear down
+//                     shared expert: b200_linear_act up -> b200_linear down
 //                     combine (sum of the token's expert rows + gate * shared) + post-norm + residual add, one kernel
 // (B200_NORM_LN_POST: x += m * layernorm(mixer(x)) * g1, x += m * layernorm(ff(x)) * g2 runs in the same loop; so does the scored attention mixer:
 //   per-head q/k norm + values + pool append -> attention -> output projection)
@@ -988,6 +988,10 @@ int linear(const b200_hybrid *m, const void *x, const void *w, void *y, int M, i
     return b200_linear(x, w, nullptr, nullptr, y, M, K, N, m->cfg.dtype, B200_W_DENSE, B200_LAYOUT_NK, 0, (b200_stream_t)st);
 }
 
+int linear_act(const b200_hybrid *m, const void *x, const void *w, void *y, int M, int K, int N, const float *bias, int act, cudaStream_t st) {
+    return b200_linear_act(x, w, bias, y, M, K, N, act, m->cfg.dtype, (b200_stream_t)st);
+}
+
 }  // namespace
 
 extern "C" {
@@ -1831,19 +1835,19 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         const int inner_cols = l.gated ? 2 : 1;
         if (l.mlp == B200_MLP_DENSE) {
             char *up = (char *)m->us, *act = up;
-            RUN(linear(m, h2, l.w_up, up, NT, width, inner_cols * l.expert_ff, st));
+            const bool ends = !l.gated && l.act != B200_ACT_POLYNORM;  // (the linear's own ending)
+            if (ends) RUN(linear_act(m, h2, l.w_up, up, NT, width, l.expert_ff, l.b_up, l.act, st));
+            else RUN(linear(m, h2, l.w_up, up, NT, width, inner_cols * l.expert_ff, st));
             if (l.gated) {
                 act = up + (size_t)NT * 2 * l.expert_ff * es;
                 if (l.b_up) RUN(launch_bias_activation(dt, up, l.b_up, NT, 2 * l.expert_ff, -1, st));
                 RUN(launch_gated_activation(dt, up, act, NT, l.expert_ff, l.act, nullptr, 0, st, l.act_limit, l.act_slope));
-            } else if (l.act == B200_ACT_POLYNORM) {
+            } else if (!ends) {
                 RUN(launch_poly_norm(dt, up, l.act_coef, c.norm_eps, NT, l.expert_ff, st));
-            } else {
-                RUN(launch_bias_activation(dt, up, l.b_up, NT, l.expert_ff, l.act, st));
             }
-            RUN(linear(m, act, l.w_down, m->ys, NT, l.expert_ff, width, st));
+            if (sum_norm && l.b_down) RUN(linear_act(m, act, l.w_down, m->ys, NT, l.expert_ff, width, l.b_down, -1, st));
+            else RUN(linear(m, act, l.w_down, m->ys, NT, l.expert_ff, width, st));
             if (sum_norm) {
-                if (l.b_down) RUN(launch_bias_activation(dt, m->ys, l.b_down, NT, width, -1, st));
                 RUN(sum_step(li, 1, m->ys, nullptr, nullptr, nullptr, nullptr, trace));
             } else if (dyt) RUN(residual(true, m->ys, l.b_down, nullptr, nullptr, nullptr, 0, nullptr, nullptr, l.norm, l.post2, l.ls2, pre, trace));
             else RUN(residual(true, m->ys, l.b_down, nullptr, nullptr, nullptr, 0, nullptr, nullptr, l.norm, l.norm2, nullptr, nullptr, trace));
@@ -1903,12 +1907,12 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         else RUN(launch_moe_grouped_gemm(dt, inner, l.w_down, m->yrows, tile_expert, n_live, max_tiles, width, l.expert_ff, -1, st, live_rows, tile_live));
         if (l.shared_ff > 0) {
             char *sin = (char *)m->us;
-            RUN(linear(m, h2, l.w_shared_up, m->us, NT, width, inner_cols * l.shared_ff, st));
             if (l.gated) {
+                RUN(linear(m, h2, l.w_shared_up, m->us, NT, width, 2 * l.shared_ff, st));
                 sin += (size_t)NT * 2 * l.shared_ff * es;
                 RUN(launch_gated_activation(dt, m->us, sin, NT, l.shared_ff, l.act, nullptr, 0, st, l.act_limit, l.act_slope));
             } else {
-                RUN(launch_activation(dt, m->us, (size_t)NT * l.shared_ff, l.act, st));
+                RUN(linear_act(m, h2, l.w_shared_up, m->us, NT, width, l.shared_ff, nullptr, l.act, st));
             }
             RUN(linear(m, sin, l.w_shared_down, m->ys, NT, l.shared_ff, width, st));
         }

@@ -255,8 +255,6 @@ int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, co
 // y fp32 [M, N] = x [M, K] * w[N, K]^T for 16-bit x and w on the tensor cores (fp32 accumulation, fp32 result); B200_ERR_UNSUPPORTED for
 // fp32 engines and K not a multiple of 8 (the caller falls back to launch_proj_f32)
 int launch_dense_f32out(int dtype, const void *x, const void *w, float *y, int M, int N, int K, cudaStream_t st);
-// in place: x = act(x)
-int launch_activation(int dtype, void *x, size_t n, int act, cudaStream_t st);
 
 // hybrid.cu
 // y[m, n] (fp32) = sum_k x[m*ldx + k] * w[n*K + k] (+ bias[n]);  x of type TX (fp32 when x_dtype == B200_F32), w of `w_dtype`
