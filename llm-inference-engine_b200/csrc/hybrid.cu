@@ -833,13 +833,14 @@ struct b200_hybrid {
     size_t chunk_floats = 0;
     int *meta = nullptr, *moe_i = nullptr;
     float *moe_f = nullptr;
+    float *tpart = nullptr;  // decoded tokens' key shares (attention_token.cu)
     std::vector<int> host_meta;
 };
 
 namespace {
 
 struct Carve {
-    size_t x, f32a, f32b, xn, h, proj, mix, y, xg, u, yrows, us, ys, lqn, lqr, lql, lov, lpart, meta, moe_i, moe_f, rec, f32c, cat, xc, xs, turns, maps, vkeep, chunk, total;
+    size_t x, f32a, f32b, xn, h, proj, mix, y, xg, u, yrows, us, ys, lqn, lqr, lql, lov, lpart, meta, moe_i, moe_f, rec, f32c, cat, xc, xs, turns, maps, vkeep, chunk, tpart, total;
 };
 
 // rows of the input projection and columns of the output projection that ONE mixer owns
@@ -891,7 +892,7 @@ Carve carve(const b200_hybrid *m) {
     const b200_hybrid_config_t &c = m->cfg;
     const size_t T = (size_t)c.max_tokens, es = c.dtype == B200_F32 ? 4 : 2;
     size_t n_in = 1, n_mix = 1, n_f32 = 1, rows = 0, ff = 1, sff = 1, experts = 1, top = 1, lqn = 0, lqr = 0, lql = 0, lov = 0, lheads = 0, lpart = 0;
-    size_t n_rec = 0, n_heads = 0, n_cat = 0, n_gru = 0, n_vkeep = 0, n_chunk = 0;
+    size_t n_rec = 0, n_heads = 0, n_cat = 0, n_gru = 0, n_vkeep = 0, n_chunk = 0, n_tpart = 0;
     bool pre_norm = false;
     const size_t t_pad = (T + 127) / 128 * 128;  // rows per head of the latent mixer's grouped GEMMs
     for (int i = 0; i < c.num_layers; ++i) {
@@ -901,6 +902,9 @@ Carve carve(const b200_hybrid *m) {
         for (const b200_hybrid_layer_t *mx : {&l, l.side})
             if (mx && (mx->mixer == B200_MIXER_GLA || mx->mixer == B200_MIXER_DELTA || mx->mixer == B200_MIXER_SSD || mx->mixer == B200_MIXER_LINEAR))
                 n_chunk = std::max(n_chunk, chunk_scratch_floats(mx->heads, mx->dim, mx->mixer == B200_MIXER_DELTA, c.max_tokens, c.max_seqs));
+        for (const b200_hybrid_layer_t *mx : {&l, l.side})
+            if (mx && c.dtype != B200_F32 && (mx->mixer == B200_MIXER_ATTN_CHUNKED || mx->mixer == B200_MIXER_ATTN_SCORED))
+                n_tpart = std::max(n_tpart, token_attention_part_floats(mx->mixer == B200_MIXER_ATTN_CHUNKED ? mx->dim : mx->vdim));
         n_mix = std::max(n_mix, (size_t)l.heads * std::max(l.dim, l.vdim));
         n_f32 = std::max(n_f32, (size_t)l.heads * std::max(l.dim, l.vdim));
         n_mix = std::max(n_mix, (size_t)l.heads * l.vdim);
@@ -955,10 +959,11 @@ Carve carve(const b200_hybrid *m) {
     // meta: attention tiles [4 * (T/64 + S), padded] | ids | tok_seq | tok_pos | want | short-portion token list [T each] | seq_start [S+1] |
     //       pos0 | slot [S each] | block table [S * mpps]
     //       | chunks of the minGRU mixer [4 * (T/64 + S)]
-    //       | latent mixers: one-token tiles of the short portions [4 * T] | head of every row tile of 64 and of 128 [heads * t_pad / 64,
+    //       | one-token tiles of the short portions [4 * T] | latent mixers: head of every row tile of 64 and of 128 [heads * t_pad / 64,
     //         heads * t_pad / 128] | live row tiles per layer, of 64 and of 128 [layers each]
+    //       | arrivals of the decoded tokens' key shares [kTokenShareCtas], zeros
     k.meta = align256((8 * (T / 64 + (size_t)c.max_seqs + 1) + 5 * T + 3 * (size_t)c.max_seqs + 1 + (size_t)c.max_seqs * c.max_pages_per_seq +
-                       (lheads ? 4 * T : 0) + 2 * lheads * (t_pad / 64) + 2 * (size_t)c.num_layers) * 4);
+                       4 * T + 2 * lheads * (t_pad / 64) + 2 * (size_t)c.num_layers + kTokenShareCtas) * 4);
     // moe ints: sel_expert | pair_row [T*top each] | row_token [rows] | tile_expert [rows / tile] | n_tiles
     k.moe_i = align256((2 * T * top + rows + rows / kMoeTileM + 4) * 4);
     // moe floats: sel_weight [T*top] | row_weight [rows] | shared_gate [T]
@@ -970,7 +975,8 @@ Carve carve(const b200_hybrid *m) {
     k.maps = align256((T / kMingruChunk + (size_t)c.max_seqs) * kMingruMapRows * n_gru * 4);
     k.vkeep = align256(T * n_vkeep * es);
     k.chunk = align256(n_chunk * 4);
-    k.total = k.chunk + k.vkeep + k.maps + k.turns + k.xs + k.x + k.f32a + k.f32b + k.xn + k.h + k.proj + 2 * k.mix + k.y + k.xg + k.u + k.yrows + k.us + k.ys + k.lqn + k.lqr + 2 * k.lql +
+    k.tpart = align256(n_tpart * 4);
+    k.total = k.tpart + k.chunk + k.vkeep + k.maps + k.turns + k.xs + k.x + k.f32a + k.f32b + k.xn + k.h + k.proj + 2 * k.mix + k.y + k.xg + k.u + k.yrows + k.us + k.ys + k.lqn + k.lqr + 2 * k.lql +
               k.lov + k.lpart + k.meta + k.moe_i + k.moe_f + k.rec + k.f32c + k.cat + k.xc;
     return k;
 }
@@ -1219,6 +1225,7 @@ int b200_hybrid_set_scratch(b200_hybrid_t *m, void *ptr, size_t bytes) {
     m->maps = (float *)p, p += k.maps;
     m->vkeep = p, p += k.vkeep;
     m->chunk = (float *)p, m->chunk_floats = k.chunk / 4, p += k.chunk;
+    m->tpart = k.tpart ? (float *)p : nullptr, p += k.tpart;
     return B200_OK;
 }
 
@@ -1331,20 +1338,18 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     // latent mixers: their per-head products are grouped GEMMs over [heads, t_pad, *]; row tile i belongs to head i / (tiles per head).
     // Prompt-sized batches of a 16-bit engine take 128-row tiles on the tcgen05 grouped GEMM, others 64-row tiles on mma.sync / SIMT.
     int lat_heads = 0;
-    bool lat_by_head = false;  // some latent layer runs its short portions as one-token tiles over 64 heads
     for (int i = 0; i < c.num_layers; ++i) {
         const b200_hybrid_layer_t &l = m->layers[i];
         if (l.mixer != B200_MIXER_LATENT) continue;
         lat_heads = std::max(lat_heads, l.heads);
-        lat_by_head |= l.heads >= kLatentHeadsPerTile && latent_attention_tiles_supported(c.dtype, l.kv_rank, l.rot_dim);
     }
     const bool lat_tc = c.dtype != B200_F32 && NT >= 256;
     const int t_pad = lat_tc ? (NT + 127) / 128 * 128 : (NT + kMoeTileM - 1) / kMoeTileM * kMoeTileM;
     const int tph = t_pad / kMoeTileM, tph128 = lat_tc ? t_pad / 128 : 0;
     bool any_mingru = false;
     for (int i = 0; i < c.num_layers; ++i) any_mingru |= m->layers[i].mixer == B200_MIXER_MINGRU;
-    const size_t n_tile_ints = 4 * ((size_t)NT / 64 + S + 1), n_chunk_ints = any_mingru ? n_tile_ints : 0, n_stile_ints = lat_by_head ? (size_t)4 * NT : 0;
-    hm.assign(n_tile_ints + n_chunk_ints + n_stile_ints + (size_t)5 * NT + 3 * S + 1 + (size_t)S * mpps + (size_t)lat_heads * (tph + tph128) + 2 * c.num_layers, 0);
+    const size_t n_tile_ints = 4 * ((size_t)NT / 64 + S + 1), n_chunk_ints = any_mingru ? n_tile_ints : 0, n_stile_ints = (size_t)4 * NT;
+    hm.assign(n_tile_ints + n_chunk_ints + n_stile_ints + (size_t)5 * NT + 3 * S + 1 + (size_t)S * mpps + (size_t)lat_heads * (tph + tph128) + 2 * c.num_layers + kTokenShareCtas, 0);
     int *h_tiles = hm.data(), *h_chunks = h_tiles + n_tile_ints, *h_stiles = h_chunks + n_chunk_ints, *h_ids = h_stiles + n_stile_ints, *h_seq = h_ids + NT, *h_pos = h_seq + NT,
         *h_want = h_pos + NT, *h_short = h_want + NT, *h_start = h_short + NT, *h_pos0 = h_start + S + 1, *h_slot = h_pos0 + S, *h_bt = h_slot + S,
         *h_lat_head = h_bt + (size_t)S * mpps, *h_lat_head128 = h_lat_head + (size_t)lat_heads * tph,
@@ -1358,7 +1363,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     // prompt portions go to the tensor-core attention in tiles of <= 64 consecutive tokens, short ones (decoded tokens) to the per-token kernel
     constexpr int kShortPortion = 8;
     static_assert(kShortPortion == kMingruShort, "one list of short portions serves both");
-    int n_tiles = 0, n_short = 0, n_chunks = 0, gla_kinds = 0;
+    int n_tiles = 0, n_short = 0, n_chunks = 0, gla_kinds = 0, last_short = 0;
     // minGRU chunks: at most 64 per portion (a chunk composes the maps of all chunks before it), of whole multiples of kMingruChunk tokens
     int longest = 0, long_tokens = 0;  // long_tokens: of the portions that the token-parallel recurrences can take
     bool mid_portions = false;  // portions of several tokens that the token-parallel recurrences leave to the serial ones
@@ -1381,11 +1386,10 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         for (int t = t0; t < t1; ++t) h_seq[t] = s, h_pos[t] = b->seq_pos0[s] + (t - t0);
         if (t1 - t0 < kShortPortion) {
             for (int t = t0; t < t1; ++t) {
-                if (lat_by_head) {
-                    int *tl = h_stiles + 4 * n_short;
-                    tl[0] = s, tl[1] = t, tl[2] = 1, tl[3] = h_pos[t];
-                }
+                int *tl = h_stiles + 4 * n_short;
+                tl[0] = s, tl[1] = t, tl[2] = 1, tl[3] = h_pos[t];
                 h_short[n_short++] = t;
+                last_short = std::max(last_short, h_pos[t]);
             }
         } else {
             for (int t = t0; t < t1; t += 64, ++n_tiles) {
@@ -1417,6 +1421,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
               *d_want = d_pos + NT, *d_short = d_want + NT, *d_start = d_short + NT, *d_pos0 = d_start + S + 1, *d_slot = d_pos0 + S, *d_bt = d_slot + S,
               *d_lat_head = d_bt + (size_t)S * mpps, *d_lat_head128 = d_lat_head + (size_t)lat_heads * tph,
               *d_lat_n = d_lat_head128 + (size_t)lat_heads * tph128, *d_lat_n128 = d_lat_n + c.num_layers;
+    unsigned int *const tickets = (unsigned int *)(m->meta + hm.size() - kTokenShareCtas);
 
     const int dt = c.dtype, width = c.width;
     const bool f32 = dt == B200_F32;
@@ -1510,11 +1515,17 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                                    l.kv_heads, l.dim, l.vdim, l.rot_dims, l.rot_base, st, opt, share));
             int max_keys = l.window > 0 ? std::min(l.window, mpps * kPageH) : mpps * kPageH;
             if (l.chunk > 0) max_keys = std::min(max_keys, l.chunk);
+            const int seen = std::min(max_keys, last_short + 1);  // keys of a decoded token, at most
+            TokenAttn ta{m->mix, kp, vp, l.head_bias, l.dist_r1, l.dist_r2, l.dist_slope, l.sink, gate, n_in, out, out_ld, out_scale, l.scale, l.softcap, (const int4 *)d_stiles, d_bt, mpps,
+                         l.heads, l.kv_heads, l.dim, l.vdim, l.window, l.chunk, sig, m->tpart, tickets};
             if (scored_attention_tiles_supported(dt, l.dim, l.vdim, n_in, out_ld, l.window, l.dist_r1 != nullptr)) {
                 RUN(launch_scored_attention_tiles(dt, m->mix, kp, vp, l.head_bias, l.dist_r1, l.dist_r2, gate, n_in, out, out_ld, out_scale, d_tiles, n_tiles,
                                                   d_bt, mpps, l.heads, l.kv_heads, l.dim, l.vdim, l.scale, l.window, sig, st, so));
-                RUN(launch_scored_attention(dt, m->mix, kp, vp, l.head_bias, l.dist_r1, l.dist_r2, gate, n_in, out, out_ld, out_scale, d_seq, d_pos, d_bt,
-                                            mpps, n_short, l.heads, l.kv_heads, l.dim, l.vdim, l.scale, l.window, sig, max_keys, st, d_short, so));
+                rc = launch_token_attention(dt, ta, n_short, seen, st);
+                if (rc == B200_ERR_UNSUPPORTED)
+                    rc = launch_scored_attention(dt, m->mix, kp, vp, l.head_bias, l.dist_r1, l.dist_r2, gate, n_in, out, out_ld, out_scale, d_seq, d_pos, d_bt,
+                                                 mpps, n_short, l.heads, l.kv_heads, l.dim, l.vdim, l.scale, l.window, sig, max_keys, st, d_short, so);
+                if (rc != B200_OK) return rc;
             } else {
                 RUN(launch_scored_attention(dt, m->mix, kp, vp, l.head_bias, l.dist_r1, l.dist_r2, gate, n_in, out, out_ld, out_scale, d_seq, d_pos, d_bt,
                                             mpps, NT, l.heads, l.kv_heads, l.dim, l.vdim, l.scale, l.window, sig, max_keys, st, nullptr, so));
@@ -1747,8 +1758,15 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             if (chunked_attention_tiles_supported(dt, l.dim, lp.n_in)) {
                 RUN(launch_chunked_attention_tiles(dt, m->mix, m->kv_pool + lp.k_off, m->kv_pool + lp.v_off, l.sink, gate, lp.n_in, m->mix2, d_tiles,
                                                    n_tiles, d_bt, mpps, l.heads, l.kv_heads, l.dim, l.scale, l.chunk, st));
-                RUN(launch_chunked_attention(dt, m->mix, m->kv_pool + lp.k_off, m->kv_pool + lp.v_off, l.sink, gate, lp.n_in, m->mix2, d_seq, d_pos,
-                                             d_bt, mpps, n_short, l.heads, l.kv_heads, l.dim, l.scale, l.chunk, max_keys, st, d_short));
+                TokenAttn ta{m->mix, m->kv_pool + lp.k_off, m->kv_pool + lp.v_off};
+                ta.sink = l.sink, ta.gate = gate, ta.gate_ld = lp.n_in, ta.out = m->mix2, ta.out_ld = hd, ta.scale = l.scale;
+                ta.tokens = (const int4 *)d_stiles, ta.block_table = d_bt, ta.mpps = mpps;
+                ta.heads = l.heads, ta.kv_heads = l.kv_heads, ta.dim = ta.vdim = l.dim, ta.chunk = l.chunk, ta.part = m->tpart, ta.tickets = tickets;
+                rc = launch_token_attention(dt, ta, n_short, std::min(max_keys, last_short + 1), st);
+                if (rc == B200_ERR_UNSUPPORTED)
+                    rc = launch_chunked_attention(dt, m->mix, m->kv_pool + lp.k_off, m->kv_pool + lp.v_off, l.sink, gate, lp.n_in, m->mix2, d_seq, d_pos,
+                                                  d_bt, mpps, n_short, l.heads, l.kv_heads, l.dim, l.scale, l.chunk, max_keys, st, d_short);
+                if (rc != B200_OK) return rc;
             } else {
                 RUN(launch_chunked_attention(dt, m->mix, m->kv_pool + lp.k_off, m->kv_pool + lp.v_off, l.sink, gate, lp.n_in, m->mix2, d_seq, d_pos,
                                              d_bt, mpps, NT, l.heads, l.kv_heads, l.dim, l.scale, l.chunk, max_keys, st));

@@ -36,6 +36,25 @@ int launch_chunked_attention_tiles(int dtype, const void *q, const void *k_pool,
                                    int gate_ld, void *out, const int *tiles, int n_tiles, const int *block_table, int mpps, int heads,
                                    int kv_heads, int dim, float scale, int chunk, cudaStream_t st);
 
+// attention_token.cu: attention of decoded tokens (or of any listed tokens), the masks and scores of the chunked and of the scored attention
+struct TokenAttn {
+    const void *q, *k_pool, *v_pool;  // q [tokens, heads, dim]; pools [pages][kv_heads][page][dim or vdim]
+    const float *head_bias = nullptr, *dist_r1 = nullptr, *dist_r2 = nullptr, *slope = nullptr, *sink = nullptr;  // per query head, as in attention_scored.cu
+    const void *gate = nullptr;       // sigmoid gate's pre-activations [tokens, gate_ld]
+    int gate_ld = 0;
+    void *out = nullptr;              // [tokens, out_ld]
+    int out_ld = 0;
+    float out_scale = 1.0f, scale = 1.0f, softcap = 0.0f;
+    const int4 *tokens = nullptr;     // {sequence, row, 1, position} of every token to do
+    const int *block_table = nullptr;
+    int mpps = 0, heads = 0, kv_heads = 0, dim = 0, vdim = 0, window = 0, chunk = 0, sigmoid = 0;
+    float *part = nullptr;            // scratch of token_attention_part_floats
+    unsigned int *tickets = nullptr;  // [kTokenShareCtas], zero, and zero again afterwards
+};
+constexpr int kMaxTokenShares = 16, kTokenShareCtas = 296;
+size_t token_attention_part_floats(int vdim);
+int launch_token_attention(int dtype, const TokenAttn &a, int tokens, int max_keys, cudaStream_t st);
+
 // attention_latent.cu
 // other rotations than pairs (i, i + rot_dims/2) by pos * rot_base^(-2i/rot_dims): pairs: (2i, 2i+1); turns: DEVICE [rot_dims/2] turns per
 // position of every pair instead of the powers of rot_base; amp multiplies cosine and sine

@@ -1,0 +1,76 @@
+"""Attention of decoded tokens by key head (csrc/attention_token.cu) against the float64 restatements: query heads per key head on both sides of every block of
+heads (1, 2, 3, 4, 5, 8, 9), head sizes of 64, 128 and 256, contexts of one key, of a share's edge (31, 32, 33), of a page's (63, 64, 65) and of more shares than
+one; batches whose tokens share out their keys beside batches that do not; portions of several decoded tokens; windows, blocks, a sink, distance penalties and
+un-normalised weights."""
+import importlib
+
+import numpy as np
+import pytest
+import torch
+
+import fedovik_oracle
+import vasolix_oracle
+
+pytestmark = pytest.mark.gpu
+TOL = {"bfloat16": 4e-2, "float16": 6e-3}  # as the other tests of 16-bit engines: rounding of a layer's rows, eight or eleven bits
+
+
+def run(name, ref, config, dtype, contexts, steps, seqs):
+    W, packed = ref.make_weights(config, seed=5)
+    cls = {"vasolix": "VasolixModel", "fedovik": "FedovikModel"}[name]
+    longest = max(contexts) + steps
+    model = getattr(importlib.import_module("llm-inference-engine_b200.models." + name), cls)(config, packed, dtype=dtype, device="cuda:0", max_tokens=2048, max_seqs=seqs,
+                                                                                              max_pages_per_seq=(longest + 63) // 64)
+    serving = importlib.import_module("llm-inference-engine_b200.serving")
+    sess = serving.Session(model, (longest + 64) * seqs, max_seqs=seqs, max_batch_tokens=2048, poison=True)
+    toks = [np.random.default_rng(i).integers(0, config["vocab"], n + steps).tolist() for i, n in enumerate(contexts)]
+    ids = [sess.open() for _ in contexts]
+    for i, n in enumerate(contexts):
+        if n:
+            sess.feed([(ids[i], toks[i][:n], [])])
+    got = [[] for _ in contexts]
+    at = list(contexts)
+    while any(a < len(t) for a, t in zip(at, toks)):
+        some = [i for i in range(len(toks)) if at[i] < len(toks[i])]
+        take = {i: min(1 + (i + at[i]) % 3, len(toks[i]) - at[i]) for i in some}  # portions of one to three tokens
+        out = sess.feed([(ids[i], toks[i][at[i]:at[i] + take[i]], list(range(take[i]))) for i in some]).cpu().numpy()
+        o = 0
+        for i in some:
+            got[i].append(out[o:o + take[i]])
+            o += take[i]
+            at[i] += take[i]
+    for i, n in enumerate(contexts):
+        want = ref.forward(config, W, toks[i])
+        want = (want[0] if isinstance(want, tuple) else want).numpy()[n:]
+        lg = np.concatenate(got[i])
+        assert not np.isnan(lg).any()
+        err = np.linalg.norm(lg - want, axis=-1) / np.linalg.norm(want, axis=-1)
+        assert err.max() < TOL[dtype], (n, int(err.argmax()), float(err.max()))
+
+
+EDGES = [0, 1, 30, 31, 32, 62, 63, 64, 95, 290]
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("heads,kv,dim,chunk", [(1, 1, 64, 40), (2, 1, 128, 64), (6, 2, 64, 100), (4, 1, 128, 1000), (5, 1, 64, 200), (8, 1, 64, 33), (9, 1, 64, 128), (2, 2, 256, 96)])
+def test_blocks_of_positions_with_a_sink(dtype, heads, kv, dim, chunk):
+    config = vasolix_oracle.make_config([vasolix_oracle.attention_layer(heads=heads, kv_heads=kv, dim=dim, size=chunk, scale=dim ** -0.5)], width=64)
+    run("vasolix", vasolix_oracle, config, dtype, EDGES, 5, 10)
+    run("vasolix", vasolix_oracle, config, dtype, [700], 4, 1)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("heads,kv,dim,vdim,window", [(2, 1, 32, 64, 33), (4, 2, 64, 128, 64), (3, 1, 96, 64, 200), (8, 2, 128, 128, 500), (8, 1, 64, 256, 70)])
+def test_windows_with_a_distance_penalty(dtype, heads, kv, dim, vdim, window):
+    layer = fedovik_oracle.pair_layer(heads=heads, kv_heads=kv, dim=dim, vdim=vdim, window=window, mlp=fedovik_oracle.dense())
+    config = fedovik_oracle.make_config([layer], width=64)
+    run("fedovik", fedovik_oracle, config, dtype, EDGES, 5, 10)
+    run("fedovik", fedovik_oracle, config, dtype, [600], 4, 1)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(4, 2, 64, 64), (3, 1, 32, 128)])
+def test_unnormalised_weights(dtype, heads, kv, dim, vdim):
+    config = fedovik_oracle.make_config([fedovik_oracle.attention_layer(heads=heads, kv_heads=kv, dim=dim, vdim=vdim)], width=64)
+    run("fedovik", fedovik_oracle, config, dtype, EDGES, 5, 10)
+    run("fedovik", fedovik_oracle, config, dtype, [400], 4, 1)
