@@ -12,6 +12,7 @@
 // The residual stream rotates over engine-owned buffers so that no kernel writes a tensor another CTA of the same kernel
 // still reads.
 #include "attention_decode.cuh"
+#include "gemm_tc.cuh"
 #include "gemv.cuh"
 
 #include <math.h>
@@ -51,8 +52,6 @@ int launch_prefill_qkv_rope_cache(void *q, void *k_layer, void *v_layer, const v
 
 int launch_dequant_vec(const void *w, const void *scales, const void *zeros, void *dst, int N, int K, int w_format, int group, int dtype,
                        cudaStream_t st);  // linear.cu
-int launch_gemm_tc(const void *x, const void *w, void *y, int M, int N, int K, int dtype, cudaStream_t st);  // gemm_tc.cu
-int launch_gemm_tc_swiglu(const void *x, const void *w, void *act, int M, int inter, int K, int dtype, cudaStream_t st);  // gemm_tc.cu
 
 static size_t align_up(size_t v) { return (v + 255) & ~(size_t)255; }
 // A kernel never writes the residual buffer other CTAs of the same launch still read: outputs go to the next buffer of the rotation.
@@ -662,12 +661,17 @@ static int prefill_impl(b200_decoder_t *dec, void *hidden, void *k_cache, void *
     int rc = b200_cal_padding_offset(padding_offset, cum, input_len, batch, max_q_len, stream);
     if (rc != B200_OK) return rc;
     void *wdq = base + off[11];
+    // quantised weights through scratch: FP8 from where its passes cost more (7B, two layers: 70 tokens 478 us against 627 in five passes, 48 about 460 in three),
+    // INT4 where the passes end (its weights lose bits on this way)
+    const bool fp8 = c.w_format == B200_W_FP8E4M3;
+    const bool quant_gemm = c.w_format != B200_W_DENSE && c.dtype != B200_F32 && T > (fp8 ? 48 : 128);
     auto linear = [&](const void *x, const b200_linear_weight_t &w, void *out, int K, int N) {
-        // FP8 / INT4 at prefill sizes: dequantise the linear into scratch (one vectorised pass), then the tcgen05 GEMM -- the tensor-core
-        // path north_star asks for; round 1 fell to a SIMT kernel here
-        if (c.w_format != B200_W_DENSE && c.dtype != B200_F32 && T > 128) {
-            int r = launch_dequant_vec(w.w, w.scales, w.zeros, wdq, N, K, c.w_format, c.group, c.dtype, st);
-            if (r == B200_OK) r = launch_gemm_tc(x, wdq, out, T, N, K, c.dtype, st);
+        // FP8 / INT4 at prefill sizes: the linear's weights into scratch as 16-bit numbers (one vectorised pass), then the tcgen05 GEMM.  FP8 codes are exact there and
+        // the rows' scales multiply the GEMM's sums; INT4 weights are rounded with their groups' scales.  Fewer tokens: the decode kernels' passes of 16 tokens over
+        // the packed weights.
+        if (quant_gemm) {
+            int r = launch_dequant_vec(w.w, fp8 ? nullptr : w.scales, w.zeros, wdq, N, K, c.w_format, c.group, c.dtype, st);
+            if (r == B200_OK) r = launch_gemm_tc(x, wdq, out, T, N, K, c.dtype, st, fp8 ? (const float *)w.scales : nullptr);
             if (r != B200_ERR_UNSUPPORTED) return r;
         }
         return b200_linear(x, w.w, w.scales, w.zeros, out, T, K, N, c.dtype, c.w_format, B200_LAYOUT_NK, c.group, stream);
@@ -713,18 +717,17 @@ static int prefill_impl(b200_decoder_t *dec, void *hidden, void *k_cache, void *
         // residual += attention output; (+ o bias); xn = RMSNorm
         rc = launch_norm_any(c.dtype, y, xn, res, res, w.o_bias, w.ffn_norm_gamma, c.rmsnorm_eps, T, h, st);
         if (rc != B200_OK) return rc;
-        // gate_up + SwiGLU: one tensor-core GEMM whose epilogue applies the activation (16-bit, T > 128; quantised weights: dequantised
-        // into scratch first); otherwise the two launchers
+        // gate_up + SwiGLU: one tensor-core GEMM whose epilogue applies the activation (16-bit, T > 16; quantised weights as above); otherwise the two launchers
         rc = B200_ERR_UNSUPPORTED;
-        if (c.dtype != B200_F32 && T > 128) {
+        if (c.dtype != B200_F32 && (c.w_format == B200_W_DENSE ? T > 16 : quant_gemm)) {
             const void *wgu = w.gate_up.w;
             if (c.w_format != B200_W_DENSE) {
-                rc = launch_dequant_vec(w.gate_up.w, w.gate_up.scales, w.gate_up.zeros, wdq, 2 * c.inter_size, h, c.w_format, c.group, c.dtype, st);
+                rc = launch_dequant_vec(w.gate_up.w, fp8 ? nullptr : w.gate_up.scales, w.gate_up.zeros, wdq, 2 * c.inter_size, h, c.w_format, c.group, c.dtype, st);
                 if (rc != B200_OK && rc != B200_ERR_UNSUPPORTED) return rc;
                 wgu = rc == B200_OK ? wdq : nullptr;
                 rc = B200_ERR_UNSUPPORTED;
             }
-            if (wgu) rc = launch_gemm_tc_swiglu(xn, wgu, act, T, c.inter_size, h, c.dtype, st);
+            if (wgu) rc = launch_gemm_tc_swiglu(xn, wgu, act, T, c.inter_size, h, c.dtype, st, fp8 ? (const float *)w.gate_up.scales : nullptr);
         }
         if (rc == B200_ERR_UNSUPPORTED) {
             if ((rc = linear(xn, w.gate_up, gu, h, 2 * c.inter_size)) != B200_OK) return rc;

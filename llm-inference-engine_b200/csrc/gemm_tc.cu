@@ -1,10 +1,6 @@
 // gemm_tc.cu -- tcgen05 / TMEM tensor-core GEMM for sm_100a: D[i,j] = sum_k A[i,k] * B[j,k], both operands K-major.
 //
-// Serves the two GEMM-shaped cases of launchLinearGemm (reference src/kernels/linear.cu:10-87) with W packed [N,K]:
-//   * prefill / context linears (M = tokens >= 129):  A = x [M,K],  B = W [N,K],  C[i,j]      (tensor-pipe bound)
-//   * batched decode linears   (5 <= M <= 128):       A = W [N,K],  B = x [M,K],  C[j,i]      ("swap-AB": the weight rows
-//     fill the 128-row MMA M dimension, the few tokens are the MMA N dimension; HBM bound -> stream-K: the tiles x k-blocks
-//     space is cut into one equal contiguous range per SM so that every SM streams the same number of weight bytes)
+// Serves launchLinearGemm (reference src/kernels/linear.cu:10-87) with W packed [N,K] beyond the decode kernels' 16 tokens: A = x [M,K], B = W [N,K], C[i,j].
 //
 // Structure (one persistent CTA per SM, 192 threads, warp-specialised):
 //   warp 0   TMA producer: cp.async.bulk.tensor 2-D tiles (128B swizzle) of A and B into a ring of smem stages, mbarrier tx counts
@@ -12,8 +8,10 @@
 //            accumulate in TMEM), tcgen05.commit releases the smem stage / publishes the accumulator
 //   warp 2-5 epilogue: tcgen05.ld the accumulator (each warp owns its 32-lane TMEM quarter), convert, store; double-buffered
 //            accumulators so the epilogue of tile t overlaps the MMAs of tile t+1
-// Tiles shared by several CTAs (stream-K) exchange fp32 partials through the library workspace; the last CTA to arrive at a tile
-// (self-resetting ticket) adds the slots in a fixed order (deterministic, no atomics on data).
+// What bounds it: the operand rows that a tile loads -- L2 to shared memory at 75 bytes a nanosecond and SM -- and, with few rows, the round trip of a ring of
+// stages.  So few tokens take narrow tiles (up to 128 tokens and N = 2048: 16 columns on 128 SMs), and where a narrow tile would load the tokens' rows too often or
+// walk too long a k (N = 4096, K = 11008), two CTAs of a cluster share a tile's k: each leaves its sums in its shared memory and adds up its part of the columns of
+// both, in rank order (deterministic; no memory traffic).  plan_tiles weighs the forms.
 #include "gemm_tc.cuh"
 
 #include <cuda.h>  // CUtensorMap
@@ -25,22 +23,21 @@ constexpr int kBM = 128;   // UMMA M
 constexpr int kBK = 64;    // K elements per stage = one 128-byte swizzle row of a 16-bit type
 constexpr int kUmmaK = 16; // K per tcgen05.mma for 16-bit inputs
 constexpr int kTcThreads = 192;
-constexpr int kMaxStages = 8;
-constexpr size_t kTcSmem = 200 * 1024 + 1024 /*alignment slack*/ + (2 * kMaxStages + 4) * 8 + 16;  // of a CTA, at most
+constexpr int kMaxStages = 24;
 constexpr int kATileBytes = kBM * kBK * 2;
+constexpr size_t kRingBytes = 200 * 1024;  // of stages, at most
+constexpr size_t kTcExtra = 1024 /*alignment slack*/ + (2 * kMaxStages + 4) * 8 + 16;
+constexpr size_t kTcSmem = kRingBytes + kATileBytes + kTcExtra;  // of a CTA, at most (a product reads 128 rows of A from a stage that may hold fewer)
 
 struct GemmTcParams {
     void *C;
-    float *partial;
-    unsigned int *tickets;
     int ldc;
     int rowsA, rowsB, K;
     int tilesA, tiles, kb_total;
-    int streamk;   // 0: whole tiles dealt round-robin; 1: the tiles x k-blocks space cut into gridDim.x equal contiguous ranges
-    int maxslots;  // stream-K: partial slots reserved per tile
+    int splits;    // CTAs of a cluster that share the k of one tile (then a CTA has one tile), or 1: tiles are dealt round-robin
     int bn;        // UMMA N: rows of B per tile, multiple of 16, <= 256
+    int a_rows;    // rows of A that a stage loads: all 128, or fewer where A has fewer (what lies below them in a stage fills accumulator rows that nobody stores)
     int stages;
-    int swap;      // 0: C[i*ldc + j]   1: C[j*ldc + i]
     int is_bf16;
     int acc_bufs;  // TMEM accumulators (2 when 2*bn <= 512)
     int acc_stride;  // TMEM columns between the accumulators: bn, or 256 for the 192..240-column tiles (power-of-two placement)
@@ -56,44 +53,24 @@ struct GemmTcParams {
     const int *tile_expert;
     const int *n_live;
     int act;        // b200_act_t applied to the result before it is stored, -1: none (plain and grouped GEMM, not the SwiGLU epilogue)
+    const float *scale;  // of every row of B (fp32, NULL: none): the sums are multiplied by it, before anything else
     int finish;     // 1: the result is rounded and takes `bias` (bias_act) before its activation (plain GEMM, A = activations)
     const float *bias;
 };
 
-// One contiguous piece of work of a CTA: k-blocks [kb0, kb1) of one output tile.  nslots > 1: the tile is shared with
-// other CTAs; this CTA's partial goes to slot `slot` and the last arriver (ticket) adds the slots in order.
+// A CTA's pieces of work: k-blocks [kb0, kb1) of output tiles.
 struct Seg {
-    int tile, kb0, kb1, slot, nslots;
+    int tile, kb0, kb1;
 };
 struct SegIter {
     const GemmTcParams &p;
-    long long g, gend, total;
-    int item, G;
-    __device__ SegIter(const GemmTcParams &pp) : p(pp) {
-        G = gridDim.x;
-        total = (long long)p.tiles * p.kb_total;
-        item = blockIdx.x;
-        g = start(blockIdx.x);
-        gend = start(blockIdx.x + 1);
-    }
-    __device__ long long start(int c) const { return (long long)c * total / G; }
-    __device__ int owner(long long gg) const { return (int)(((gg + 1) * G + total - 1) / total) - 1; }  // max c: start(c) <= gg
+    int item;
+    __device__ SegIter(const GemmTcParams &pp) : p(pp), item(blockIdx.x / pp.splits) {}
     __device__ bool next(Seg &s) {
-        if (!p.streamk) {
-            if (item >= p.tiles) return false;
-            s.tile = item, s.kb0 = 0, s.kb1 = p.kb_total, s.slot = 0, s.nslots = 1;
-            item += G;
-            return true;
-        }
-        if (g >= gend) return false;
-        s.tile = (int)(g / p.kb_total);
-        s.kb0 = (int)(g - (long long)s.tile * p.kb_total);
-        const long long len = min((long long)(p.kb_total - s.kb0), gend - g);
-        s.kb1 = s.kb0 + (int)len;
-        const int first = owner((long long)s.tile * p.kb_total), last = owner((long long)(s.tile + 1) * p.kb_total - 1);
-        s.slot = (int)blockIdx.x - first;
-        s.nslots = last - first + 1;
-        g += len;
+        if (item >= p.tiles) return false;
+        const int rank = blockIdx.x % p.splits;
+        s.tile = item, s.kb0 = p.kb_total * rank / p.splits, s.kb1 = p.kb_total * (rank + 1) / p.splits;
+        item += gridDim.x / p.splits;
         return true;
     }
 };
@@ -195,6 +172,26 @@ template <typename T> __device__ __forceinline__ void store_row16(T *dst, const 
     }
 }
 
+// the numbers of 16 consecutive columns, the first n0 of `cols` (past the last: the last)
+__device__ __forceinline__ void columns16(const float *p, int n0, int cols, float (&b)[16]) {
+    if ((reinterpret_cast<size_t>(p + n0) & 15) == 0 && n0 + 16 <= cols) {
+#pragma unroll
+        for (int e = 0; e < 16; e += 4) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(p + n0 + e));
+            b[e] = v.x, b[e + 1] = v.y, b[e + 2] = v.z, b[e + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) b[e] = __ldg(p + min(n0 + e, cols - 1));
+    }
+}
+__device__ __forceinline__ void scale16(uint32_t (&r)[16], const float *scale, int n0, int cols) {
+    float b[16];
+    columns16(scale, n0, cols, b);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * b[e]);
+}
+
 // bias_act on 16 consecutive outputs of one row, the first of them column n0 of `cols`.  The choice of the activation stands outside the columns (inside, an
 // epilogue outlasted the products it should hide behind: a layer of 3085 rows with a biased up projection of 8192 columns 638 us, now 572), the biases come in 16-byte loads where they can.
 template <typename T> __device__ __forceinline__ void finish16(uint32_t (&r)[16], const float *bias, int n0, int cols, int act) {
@@ -202,16 +199,10 @@ template <typename T> __device__ __forceinline__ void finish16(uint32_t (&r)[16]
 #pragma unroll
     for (int e = 0; e < 16; ++e) v[e] = round_to<T>(__uint_as_float(r[e]));
     if (bias) {
-        if ((reinterpret_cast<size_t>(bias + n0) & 15) == 0 && n0 + 16 <= cols) {
+        float b[16];
+        columns16(bias, n0, cols, b);
 #pragma unroll
-            for (int e = 0; e < 16; e += 4) {
-                const float4 b = __ldg(reinterpret_cast<const float4 *>(bias + n0 + e));
-                v[e] += b.x, v[e + 1] += b.y, v[e + 2] += b.z, v[e + 3] += b.w;
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) v[e] += __ldg(bias + min(n0 + e, cols - 1));
-        }
+        for (int e = 0; e < 16; ++e) v[e] += b[e];
     }
     if (act == B200_ACT_RELU2) {
 #pragma unroll
@@ -230,6 +221,55 @@ template <typename T> __device__ __forceinline__ void finish16(uint32_t (&r)[16]
     for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(v[e]);
 }
 
+__device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {  // the same shared-memory offset in CTA `rank` of the cluster
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Output columns [c0, c1) (steps of 16, counted from the tile's first) of row i of a tile in column tile tb, from accumulator columns that `get` fetches.
+template <typename T, typename GET> __device__ __forceinline__ void finish_tile(const GemmTcParams &p, int i, int tb, int c0, int c1, GET get) {
+    T *C = reinterpret_cast<T *>(p.C);
+    if (p.swiglu_inter) {
+        // gate in accumulator columns [0, hw), up in [hw, 2 hw): both rounded to T first (the reference's linear writes a T
+        // tensor that launchSiluAndMul reads back, src/kernels/silu_and_mul.cu:6-41), same expression as silu_and_mul_kernel
+        const int hw = p.swiglu_hw;
+        for (int c = c0; c < c1; c += 16) {
+            uint32_t g[16], u[16];
+            get(c, g);
+            get(hw + c, u);
+            if (p.scale) scale16(g, p.scale, tb * hw + c, p.rowsB), scale16(u, p.scale + p.swiglu_inter, tb * hw + c, p.rowsB);
+            const int valid = min(16, p.rowsB - (tb * hw + c));
+            if (i < p.rowsA && valid > 0) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    const float gf = round_to<T>(__uint_as_float(g[e])), uf = round_to<T>(__uint_as_float(u[e]));
+                    g[e] = __float_as_uint((gf / (1.0f + expf(-gf))) * uf);
+                }
+                store_row16<T>(C + (size_t)i * p.ldc + tb * hw + c, g, valid);
+            }
+        }
+        return;
+    }
+    const int j0 = tb * p.bn;
+    for (int c = c0; c < c1; c += 16) {
+        uint32_t r[16];
+        get(c, r);
+        if (p.scale) scale16(r, p.scale, j0 + c, p.rowsB);
+        if (p.finish) {
+            finish16<T>(r, p.bias, j0 + c, p.rowsB, p.act);
+        } else if (p.act >= 0) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(act_apply(__uint_as_float(r[e]), p.act));
+        }
+        const int valid = min(16, p.rowsB - (j0 + c));
+        if (i < p.rowsA && valid > 0) store_row16<T>(C + (size_t)i * p.ldc + j0 + c, r, valid);
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kTcThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmTcParams p) {
@@ -237,12 +277,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // carve: stages x [A tile | B tile] (1024-byte aligned), then barriers, then the TMEM base address
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int b_tile_bytes = p.bn * kBK * 2;
-    const int stage_bytes = kATileBytes + b_tile_bytes;
+    const int a_tile_bytes = p.a_rows * kBK * 2, stage_bytes = a_tile_bytes + b_tile_bytes;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (size_t)p.stages * stage_bytes);
     const uint32_t full0 = s_u32(bars), empty0 = full0 + 8 * kMaxStages;
     const uint32_t tfull0 = empty0 + 8 * kMaxStages, tempty0 = tfull0 + 16;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kMaxStages + 4);
-    int *flag_slot = reinterpret_cast<int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -276,23 +315,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (elect_one()) {
             SegIter si(p);
             Seg sg;
-            int it = 0;
+            int s = 0;  // (stage and phase by counting: a remainder and a quotient per k-block were a third of what a narrow tile's block took)
+            uint32_t ph = 1;
             while (si.next(sg)) {
                 const int ta = sg.tile % p.tilesA, tb = sg.tile / p.tilesA;
                 if (p.tile_expert && ta >= *p.n_live) continue;
                 const int brow = (p.tile_expert ? p.tile_expert[ta] * p.rowsB : 0) + tb * p.bn;
-                for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
-                    const int s = it % p.stages;
-                    bar_wait(empty0 + 8 * s, ((it / p.stages) & 1) ^ 1);
+                for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+                    bar_wait(empty0 + 8 * s, ph);
                     const uint32_t sa = s_u32(smem + (size_t)s * stage_bytes);
                     bar_expect_tx(full0 + 8 * s, (uint32_t)stage_bytes);
                     tma_load_2d(sa, &tmA, kb * kBK, ta * kBM, full0 + 8 * s);
                     if (p.swiglu_inter) {  // box = hw rows: the gate rows, then the up rows of the same columns
-                        tma_load_2d(sa + kATileBytes, &tmB, kb * kBK, tb * p.swiglu_hw, full0 + 8 * s);
-                        tma_load_2d(sa + kATileBytes + p.swiglu_hw * kBK * 2, &tmB, kb * kBK, p.swiglu_inter + tb * p.swiglu_hw, full0 + 8 * s);
+                        tma_load_2d(sa + a_tile_bytes, &tmB, kb * kBK, tb * p.swiglu_hw, full0 + 8 * s);
+                        tma_load_2d(sa + a_tile_bytes + p.swiglu_hw * kBK * 2, &tmB, kb * kBK, p.swiglu_inter + tb * p.swiglu_hw, full0 + 8 * s);
                     } else {
-                        tma_load_2d(sa + kATileBytes, &tmB, kb * kBK, brow, full0 + 8 * s);
+                        tma_load_2d(sa + a_tile_bytes, &tmB, kb * kBK, brow, full0 + 8 * s);
                     }
+                    if (++s == p.stages) s = 0, ph ^= 1;
                 }
             }
         }
@@ -301,8 +341,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const uint32_t idesc = instr_desc_f16(p.is_bf16 != 0, kBM, p.bn);
         SegIter si(p);
         Seg sg;
-        int it = 0, t = 0;
-        for (; si.next(sg); ++t) {
+        int s = 0, t = 0;
+        uint32_t ph = 0;
+        const bool issuer = elect_one();
+        for (; issuer && si.next(sg); ++t) {
             if (p.tile_expert && sg.tile % p.tilesA >= *p.n_live) {
                 --t;  // a row tile without rows: not a tile at all for the accumulator rotation
                 continue;
@@ -311,13 +353,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             bar_wait(tempty0 + 8 * acc, ((t / p.acc_bufs) & 1) ^ 1);  // the epilogue has drained this accumulator
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(acc * p.acc_stride);
-            for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
-                const int s = it % p.stages;
-                bar_wait(full0 + 8 * s, (it / p.stages) & 1);
+            for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+                bar_wait(full0 + 8 * s, ph);
                 tc_fence_after();
-                if (elect_one()) {
+                {
                     const uint32_t sa = s_u32(smem + (size_t)s * stage_bytes);
-                    const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + kATileBytes);
+                    const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + a_tile_bytes);
 #pragma unroll
                     for (int k = 0; k < kBK / kUmmaK; ++k) {
                         // advancing K inside the 128-byte swizzle row: +32 bytes = +2 in the (>>4) start-address field
@@ -326,14 +367,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     tc_commit(empty0 + 8 * s);                          // smem stage reusable once these MMAs have read it
                     if (kb == sg.kb1 - 1) tc_commit(tfull0 + 8 * acc);  // accumulator complete
                 }
-                __syncwarp();
+                if (++s == p.stages) s = 0, ph ^= 1;
             }
         }
     } else {
         // ================================================= epilogue (warps 2..5 -> TMEM lane quarters 2,3,0,1)
         const int q = warp & 3;
-        const int ep_tid = (warp - 2) * 32 + lane;  // 0..127
-        T *C = reinterpret_cast<T *>(p.C);
         SegIter si(p);
         Seg sg;
         int t = 0;
@@ -347,125 +386,50 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             bar_wait(tfull0 + 8 * acc, (t / p.acc_bufs) & 1);
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * p.acc_stride);
-            const int i = ta * kBM + q * 32 + lane;  // row of A this thread owns
-            const int j0 = tb * p.bn;
-            if (p.swiglu_inter) {
-                // gate in accumulator columns [0, hw), up in [hw, 2 hw): both rounded to T first (the reference's linear writes a T
-                // tensor that launchSiluAndMul reads back, src/kernels/silu_and_mul.cu:6-41), same expression as silu_and_mul_kernel
-                const int hw = p.swiglu_hw;
-                for (int c = 0; c < hw; c += 16) {
-                    uint32_t g[16], u[16];
-                    tc_ld16(taddr + c, g);
-                    tc_ld16(taddr + hw + c, u);
-                    tc_wait_ld();
-                    const int valid = min(16, p.rowsB - (tb * hw + c));
-                    if (i < p.rowsA && valid > 0) {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            const float gf = round_to<T>(__uint_as_float(g[e])), uf = round_to<T>(__uint_as_float(u[e]));
-                            g[e] = __float_as_uint((gf / (1.0f + expf(-gf))) * uf);
-                        }
-                        store_row16<T>(C + (size_t)i * p.ldc + tb * hw + c, g, valid);
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) bar_arrive(tempty0 + 8 * acc);
-            } else if (sg.nslots == 1) {
+            auto fetch = [&](int c, uint32_t (&r)[16]) {
+                tc_ld16(taddr + c, r);
+                tc_wait_ld();
+            };
+            if (p.splits > 1) {  // this CTA's part of the sums, [column][row], where its stages were
+                float *mine = reinterpret_cast<float *>(smem) + q * 32 + lane;
                 for (int c = 0; c < p.bn; c += 16) {
                     uint32_t r[16];
-                    tc_ld16(taddr + c, r);
-                    tc_wait_ld();
-                    if (p.finish) {
-                        finish16<T>(r, p.bias, j0 + c, p.rowsB, p.act);
-                    } else if (p.act >= 0) {
+                    fetch(c, r);
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(act_apply(__uint_as_float(r[e]), p.act));
-                    }
-                    if (i < p.rowsA) {
-                        if (!p.swap) {
-                            const int valid = min(16, p.rowsB - (j0 + c));
-                            if (valid > 0) store_row16<T>(C + (size_t)i * p.ldc + j0 + c, r, valid);
-                        } else {
-#pragma unroll
-                            for (int e = 0; e < 16; ++e)
-                                if (j0 + c + e < p.rowsB) C[(size_t)(j0 + c + e) * p.ldc + i] = Elem<T>::from_f(__uint_as_float(r[e]));
-                        }
-                    }
+                    for (int e = 0; e < 16; ++e) mine[(size_t)(c + e) * kBM] = __uint_as_float(r[e]);
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) bar_arrive(tempty0 + 8 * acc);
             } else {
-                // shared tile: publish this CTA's fp32 partial [bn][128] (coalesced over lanes); the last arriver reduces
-                const size_t tile_floats = (size_t)p.bn * kBM;
-                float *part = p.partial + ((size_t)sg.tile * p.maxslots + sg.slot) * tile_floats;
-                for (int c = 0; c < p.bn; c += 16) {
-                    uint32_t r[16];
-                    tc_ld16(taddr + c, r);
-                    tc_wait_ld();
+                finish_tile<T>(p, ta * kBM + q * 32 + lane, tb, 0, p.swiglu_inter ? p.swiglu_hw : p.bn, fetch);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) bar_arrive(tempty0 + 8 * acc);
+        }
+    }
+    if (p.splits > 1) {
+        // every CTA of the cluster adds up its part of the tile's columns, and stays until the others have read what it holds
+        __syncthreads();
+        cluster_sync_all();
+        const int tile = blockIdx.x / p.splits, rank = blockIdx.x % p.splits;
+        if (warp >= 2 && tile < p.tiles) {
+            const int q = warp & 3, cols = (p.swiglu_inter ? p.swiglu_hw : p.bn) / p.splits;
+            const uint32_t at = s_u32(smem) + (uint32_t)(q * 32 + lane) * 4;
+            finish_tile<T>(p, tile % p.tilesA * kBM + q * 32 + lane, tile / p.tilesA, rank * cols, (rank + 1) * cols, [&](int c, uint32_t (&r)[16]) {
+                float v[16];
+                for (int x = 0; x < p.splits; ++x) {
+                    const uint32_t from = in_cta(at + (uint32_t)c * kBM * 4, (uint32_t)x);
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) __stcg(part + (size_t)(c + e) * kBM + q * 32 + lane, __uint_as_float(r[e]));
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) bar_arrive(tempty0 + 8 * acc);  // the accumulator is free: the MMA warp may start the next segment
-                __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (ep_tid == 0) *flag_slot = atomicInc(&p.tickets[sg.tile], (unsigned)(sg.nslots - 1)) == (unsigned)(sg.nslots - 1);
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                const bool last = *flag_slot != 0;
-                asm volatile("bar.sync 1, 128;" ::: "memory");  // flag_slot may be rewritten by the next segment
-                if (last) {
-                    __threadfence();
-                    // 128 threads x float4: element f = (column c, 4 consecutive A rows); slots added in order (deterministic)
-                    const float4 *pt = reinterpret_cast<const float4 *>(p.partial + (size_t)sg.tile * p.maxslots * tile_floats);
-                    const int nf = p.bn * (kBM / 4), slot_f4 = (int)(tile_floats / 4);
-                    constexpr int U = 4;
-                    for (int f0 = ep_tid; f0 < nf; f0 += 128 * U) {
-                        float4 sum[U];
-#pragma unroll
-                        for (int u = 0; u < U; ++u) sum[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        for (int k2 = 0; k2 < sg.nslots; ++k2) {
-#pragma unroll
-                            for (int u = 0; u < U; ++u) {
-                                const int f = f0 + u * 128;
-                                if (f < nf) {
-                                    const float4 v = __ldcg(pt + (size_t)k2 * slot_f4 + f);
-                                    sum[u].x += v.x, sum[u].y += v.y, sum[u].z += v.z, sum[u].w += v.w;
-                                }
-                            }
-                        }
-#pragma unroll
-                        for (int u = 0; u < U; ++u) {
-                            const int f = f0 + u * 128;
-                            if (f >= nf) continue;
-                            const int c = f / (kBM / 4), ii = ta * kBM + (f % (kBM / 4)) * 4;
-                            if (j0 + c >= p.rowsB) continue;
-                            const float v[4] = {sum[u].x, sum[u].y, sum[u].z, sum[u].w};
-                            if (p.swap) {
-                                T *dst = C + (size_t)(j0 + c) * p.ldc + ii;
-                                if (ii + 3 < p.rowsA && (reinterpret_cast<uintptr_t>(dst) & 7) == 0 && sizeof(T) == 2) {
-                                    uint2 pk;
-                                    const T a0 = Elem<T>::from_f(v[0]), a1 = Elem<T>::from_f(v[1]), a2 = Elem<T>::from_f(v[2]), a3 = Elem<T>::from_f(v[3]);
-                                    pk.x = (uint32_t)(*reinterpret_cast<const unsigned short *>(&a0)) | ((uint32_t)(*reinterpret_cast<const unsigned short *>(&a1)) << 16);
-                                    pk.y = (uint32_t)(*reinterpret_cast<const unsigned short *>(&a2)) | ((uint32_t)(*reinterpret_cast<const unsigned short *>(&a3)) << 16);
-                                    *reinterpret_cast<uint2 *>(dst) = pk;
-                                } else {
-#pragma unroll
-                                    for (int e = 0; e < 4; ++e)
-                                        if (ii + e < p.rowsA) dst[e] = Elem<T>::from_f(v[e]);
-                                }
-                            } else {
-#pragma unroll
-                                for (int e = 0; e < 4; ++e)
-                                    if (ii + e < p.rowsA) C[(size_t)(ii + e) * p.ldc + j0 + c] = Elem<T>::from_f(v[e]);
-                            }
-                        }
+                    for (int e = 0; e < 16; ++e) {
+                        float f;
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f) : "r"(from + (uint32_t)e * kBM * 4) : "memory");
+                        v[e] = x == 0 ? f : v[e] + f;
                     }
                 }
-            }
+#pragma unroll
+                for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(v[e]);
+            });
         }
+        cluster_sync_all();
     }
 
     tc_fence_before();
@@ -491,6 +455,7 @@ struct GemmPairParams {
     int bn, bn2, n_wide;
     int stages, is_bf16;
     int swiglu_inter;  // as above: gate rows come from the leader's half of B, up rows from its peer's; tile widths count both
+    const float *scale;  // of every row of B, as above
     int finish, act;   // finish: bias_act on the result, as above
     const float *bias;
     WaitGuard wait;
@@ -498,11 +463,6 @@ struct GemmPairParams {
 constexpr int kPairThreads = 320;
 constexpr int kPairStageBytes = 2 * kATileBytes;  // 128 rows of A, up to 128 rows of B
 
-__device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {  // the same shared-memory offset in CTA `rank` of the cluster
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t leader_bar) {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
                  "l"(map), "r"(c0), "r"(c1), "r"(leader_bar)
@@ -522,10 +482,6 @@ __device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmB2, const GemmPairParams p) {
@@ -579,7 +535,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if (warp == 0) {
         // ================================================= TMA producer: this CTA's rows of A, its half of the B rows
         if (elect_one()) {
-            int it = 0;
+            int it = 0, s = 0;
+            uint32_t ph = 1;
             bool live = true;
             for (int item = pair; live && item < p.tiles; item += pairs) {
                 const int ta = item % p.tilesA, tb = item / p.tilesA, w = width_of(tb);
@@ -587,13 +544,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 const int brow = p.swiglu_inter ? (rank ? p.swiglu_inter : 0) + col_of(tb) : col_of(tb) + (int)rank * (w >> 1);
                 const CUtensorMap *mb = tb < p.n_wide ? &tmB : &tmB2;
                 for (int kb = 0; kb < p.kb_total; ++kb, ++it) {
-                    const int s = it % p.stages;
-                    live = wait(empty0 + 8 * s, ((it / p.stages) & 1) ^ 1);
+                    live = wait(empty0 + 8 * s, ph);
                     if (!live) break;
                     const uint32_t sa = s_u32(smem + (size_t)s * kPairStageBytes), bar = in_cta(full0 + 8 * s, 0);
                     if (rank == 0) bar_expect_tx(full0 + 8 * s, (uint32_t)(2 * (kATileBytes + (w >> 1) * kBK * 2)));
                     tma_load_2d_pair(sa, &tmA, kb * kBK, arow, bar);
                     tma_load_2d_pair(sa + kATileBytes, mb, kb * kBK, brow, bar);
+                    if (++s == p.stages) s = 0, ph ^= 1;
                 }
             }
             // The leader's last commits arrive at `empty` of both CTAs and nobody refills those stages: each CTA waits for its own here, since the
@@ -606,7 +563,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     } else if (warp == 1) {
         // ================================================= MMA issuer: the leader, for both
         if (rank == 0 && elect_one()) {
-            int it = 0, t = 0;
+            int s = 0, t = 0;
+            uint32_t ph = 0;
             bool live = true;
             for (int item = pair; live && item < p.tiles; item += pairs, ++t) {
                 const uint32_t idesc = instr_desc_f16(p.is_bf16 != 0, 2 * kBM, width_of(item / p.tilesA));
@@ -615,9 +573,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (!live) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
-                for (int kb = 0; kb < p.kb_total; ++kb, ++it) {
-                    const int s = it % p.stages;
-                    live = wait(full0 + 8 * s, (it / p.stages) & 1);
+                for (int kb = 0; kb < p.kb_total; ++kb) {
+                    live = wait(full0 + 8 * s, ph);
                     if (!live) break;
                     tc_fence_after();
                     const uint32_t sa = s_u32(smem + (size_t)s * kPairStageBytes);
@@ -626,6 +583,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     for (int k = 0; k < kBK / kUmmaK; ++k) tc_mma_f16_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     tc_commit_pair(empty0 + 8 * s);
                     if (kb == p.kb_total - 1) tc_commit_pair(tfull0 + 8 * acc);
+                    if (++s == p.stages) s = 0, ph ^= 1;
                 }
             }
             tc_commit_leader(drain);  // no product reads either CTA's shared memory when the pair leaves
@@ -653,6 +611,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     uint32_t u[16];
                     tc_ld16(taddr + out_w + c, u);
                     tc_wait_ld();
+                    if (p.scale) scale16(g, p.scale, col0 + c, p.rowsB), scale16(u, p.scale + p.swiglu_inter, col0 + c, p.rowsB);
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {  // (the same expression and roundings as the one-CTA epilogue)
                         const float gf = round_to<T>(__uint_as_float(g[e])), uf = round_to<T>(__uint_as_float(u[e]));
@@ -660,6 +619,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     }
                 } else {
                     tc_wait_ld();
+                    if (p.scale) scale16(g, p.scale, col0 + c, p.rowsB);
                     if (p.finish) finish16<T>(g, p.bias, col0 + c, p.rowsB, p.act);
                 }
                 if (!live) {
@@ -711,20 +671,50 @@ static PairWidths choose_widths(int tiles_a, int cols, int pairs) {  // cols: MM
     return best;
 }
 
-// CTA pairs when their busiest pair finishes before the one-CTA form's busiest SM would.  Both are counted in columns of a row tile (a pair multiplies 256
-// rows in the time an SM takes for 128); per column the one-CTA form is the slower by its doubled B traffic (7B at 2048 tokens, all eight linears:
-// 1235 us against 1158), so row counts that 256-row tiles pad (1084 tokens: 1280 rows against 1152) stay with it.
-static bool pair_takes(int M, int cols, int sms) {
-    const int t128 = (M + kBM - 1) / kBM, t256 = (M + 2 * kBM - 1) / (2 * kBM), pairs = sms / 2;
-    if (cols < 256 || t256 * ((cols + 255) / 256) * 2 < pairs) return false;
-    long long one = 1LL << 60;
-    for (int bn : {256, 240, 224, 208, 192}) one = std::min(one, (long long)((t128 * ((cols + bn - 1) / bn) + sms - 1) / sms) * (bn + 24));
-    return choose_widths(t256, cols, pairs).cost * 16 <= one * 17;
+// Tiles of the one-CTA form: the width and the number of CTAs per tile whose estimate is smallest, in nanoseconds.  A k-block costs its operand rows, but never less
+// than the issue of its copies and products (130); a wave ends on an epilogue; the weights come from memory at 6500 bytes a nanosecond.  Two CTAs on one tile's k pay
+// an exchange of 4.5 us: K = 11008, N = 4096 of 17 / 128 tokens 64 columns on two CTAs 20.5 / 23.1 us, 32 columns on one 24.1 / 26.0 (four CTAs: 22.0 / 23.6, and
+// behind two everywhere else).  Swept on a B200 (us, widths 16 to 256): K = 4096, N = 4096 of 128 tokens 32 columns 12.3, 64 14.0, 128 17.8; K = 2048, N = 6208 of 94:
+// 48 8.4, 128 10.7; K = 8192, N = 10240 of 400: 144 (two waves) 80, 192 89, 256 112; K = N = 8192 of 1084: 256 115, 192 131.
+// Against what was here (128 x 128 and wider tiles; up to 128 tokens the weights' rows as the tile's 128, their sums shared out through memory), us: 17 / 64 / 128 /
+// 267 / 600 tokens: K = 2048, N = 2048 12.1 / 17.6 / 28.4 / 13.0 / 14.4, K = 4096, N = 12288 25.8 / 31.4 / 40.4 / 35.4 / 57.1, K = 11008, N = 4096
+// 22.9 / 27.6 / 36.4 / 54.9 / 62.3.
+struct TilePlan {
+    int bn, splits;
+    double ns;
+};
+static TilePlan plan_tiles(int M, int cols, int K, int sms, int step, int only = 0) {  // only: this many CTAs per tile (0: any)
+    const int rows = std::min(kBM, (M + 7) / 8 * 8), tiles_a = (M + kBM - 1) / kBM, kb = (K + kBK - 1) / kBK, widest = std::min(256, (cols + step - 1) / step * step);
+    TilePlan best = {widest, 1, 1e30};
+    for (int splits : {1, 2}) {
+        if (only && splits != only) continue;
+        for (int bn = widest; bn >= step * splits; bn -= step) {
+            if (bn % (step * splits)) continue;
+            const long long tiles = (long long)tiles_a * ((cols + bn - 1) / bn);
+            if (splits > 1 && (tiles * splits > sms || kb < 4 * splits)) break;  // (narrower: more of them)
+            const int stages = std::min(kMaxStages, (int)(kRingBytes / ((rows + bn) * kBK * 2)));
+            if (splits > 1 && stages * (rows + bn) * kBK * 2 < 4 * bn * kBM) continue;  // (the exchange lies where the stages were)
+            const long long waves = (tiles * splits + sms - 1) / sms;
+            double ns = waves * ((kb + splits - 1) / splits * std::max(130.0, 1.1 * (rows + bn)) + 600) + (splits > 1 ? 4500 : 0);
+            ns = std::max(ns, cols * (double)K * 2 / 6500) + 0.05 * ns;
+            if (ns < best.ns) best = {bn, splits, ns};
+        }
+    }
+    return best;
+}
+
+// CTA pairs where their estimate (1.5 ns per column and k-block of the busiest pair) is smaller: large launches whose row tiles of 256 are nearly full.  A pair loads
+// half of a tile's B rows per CTA, which counts where all SMs load all the time (7B at 2048 tokens, all eight linears: 1235 us on one-CTA tiles, 1158 on pairs);
+// few waves of narrow tiles waste less (K = 2048, N = 6208 of 267 tokens: 15.1 on pairs, 12.2 here).
+static bool pair_takes(int M, int cols, int K, int sms, const TilePlan &one) {
+    const int t256 = (M + 2 * kBM - 1) / (2 * kBM), pairs = sms / 2;
+    if (M <= kBM || cols < 256 || t256 * ((cols + 255) / 256) * 2 < pairs) return false;
+    return choose_widths(t256, cols, pairs).cost * ((K + kBK - 1) / kBK) * 1.5 + 600 < one.ns;
 }
 
 struct Finish {
     int on, act;
-    const float *bias;
+    const float *bias, *scale;
 };
 static int launch_gemm_pair(const void *x, const void *w, void *y, int M, int N, int K, int dtype, int swiglu_inter, const Finish &fin, cudaStream_t st) {
     const bool bf16 = dtype == B200_BF16;
@@ -735,9 +725,9 @@ static int launch_gemm_pair(const void *x, const void *w, void *y, int M, int N,
     p.tilesA = (M + 2 * kBM - 1) / (2 * kBM);
     const PairWidths pw = choose_widths(p.tilesA, cols, pairs);
     p.bn = pw.bn, p.bn2 = pw.bn2, p.n_wide = pw.n_wide, p.tiles = p.tilesA * pw.n_tiles;
-    p.finish = fin.on, p.act = fin.act, p.bias = fin.bias;
+    p.finish = fin.on, p.act = fin.act, p.bias = fin.bias, p.scale = fin.scale;
     p.stages = 6, p.wait = wait_guard();
-    const size_t smem = (size_t)p.stages * kPairStageBytes + 1024 + (2 * kMaxStages + 4) * 8 + 16;
+    const size_t smem = (size_t)p.stages * kPairStageBytes + kTcExtra + 16;
     CUtensorMap tmA, tmB, tmB2;
     if (!tile_map(&tmA, x, M, K, kBM, bf16) || !tile_map(&tmB, w, cols, K, p.bn / 2, bf16) || !tile_map(&tmB2, w, cols, K, p.bn2 / 2, bf16)) {
         set_error("gemm_tc pair: cuTensorMapEncodeTiled failed (rows %d/%d, K %d)", M, cols, K);
@@ -757,109 +747,55 @@ static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int
     if (dtype != B200_BF16 && dtype != B200_F16) return B200_ERR_UNSUPPORTED;
     if (M < 1 || K % 8 != 0 || K < kBK || !aligned16(x) || !aligned16(w) || !y) return B200_ERR_UNSUPPORTED;
     const bool bf16 = dtype == B200_BF16;
-    const bool swap = M <= 128;
-    if (fin.on && swap) return B200_ERR_UNSUPPORTED;
-    if (swiglu_inter && (swap || swiglu_inter < 128)) return B200_ERR_UNSUPPORTED;  // the fused epilogue exists for prefill-sized token counts
-    if (!swap && pair_takes(M, swiglu_inter ? 2 * swiglu_inter : N, sm_count())) return launch_gemm_pair(x, w, y, M, N, K, dtype, swiglu_inter, fin, st);
+    if (swiglu_inter && swiglu_inter < 128) return B200_ERR_UNSUPPORTED;
+    const int sms = sm_count(), cols = swiglu_inter ? 2 * swiglu_inter : N;
+    TilePlan plan = plan_tiles(M, cols, K, sms, 16);
+    if (swiglu_inter) plan = plan_tiles(M, cols, K, sms, 32, plan.splits);  // (the plain linear's order of summation: the same bits)
+    if (pair_takes(M, cols, K, sms, plan)) return launch_gemm_pair(x, w, y, M, N, K, dtype, swiglu_inter, fin, st);
     GemmTcParams p = {};
-    p.C = y, p.ldc = N, p.K = K, p.swap = swap ? 1 : 0, p.is_bf16 = bf16 ? 1 : 0;
+    p.C = y, p.K = K, p.is_bf16 = bf16 ? 1 : 0;
     p.swiglu_inter = swiglu_inter;
-    p.finish = fin.on, p.act = fin.on ? fin.act : -1, p.bias = fin.bias;
+    p.finish = fin.on, p.act = fin.on ? fin.act : -1, p.bias = fin.bias, p.scale = fin.scale;
     p.kb_total = (K + kBK - 1) / kBK;
-    const void *a_ptr, *b_ptr;
-    int rows_b_map;  // rows of the B tensor as the TMA sees it
-    if (swap) {
-        a_ptr = w, b_ptr = x;
-        p.rowsA = N, p.rowsB = M;
-        p.bn = (M + 15) / 16 * 16;
-        rows_b_map = M;
-    } else {
-        a_ptr = x, b_ptr = w;
-        p.rowsA = M, p.rowsB = N;
-        p.bn = N >= 256 ? 256 : (N + 15) / 16 * 16;
-        rows_b_map = N;
-    }
-    const int sms = sm_count();
-    const int tiles_a = ((swap ? N : M) + kBM - 1) / kBM;
-    // Tile width of the prefill shapes: the widest tile is the most efficient one, but the number of waves is an integer -- 768 tiles of
-    // 256 columns on 148 SMs (7B QKV projection at 2048 tokens) take 6 waves for 5.19 waves of work.  Choose the width whose
-    // waves x width is smallest (ties: the wider one): 224 for that shape (880 tiles, 5.95 waves), 240 for N = 4096.  Measured gain 2-3 %
-    // per GEMM, not the 6-12 % of the wave count: a narrower MMA re-reads the 128-row A tile more often per flop.
-    auto waves_cost = [&](int cols, int width) { return (long long)((tiles_a * ((cols + width - 1) / width) + sms - 1) / sms) * width; };
-    if (swiglu_inter) {
-        // measured (7B, 2048 tokens): 2 x 112 columns (11 waves instead of 10 of 2 x 128) is 6 % SLOWER -- the narrower MMA re-reads the
-        // A tile more often per flop than the better wave count saves; the half width stays a parameter, the choice is 128
-        const int hw = 128;
-        p.swiglu_hw = hw;
-        p.bn = 2 * hw, p.rowsB = swiglu_inter, p.ldc = swiglu_inter;  // N = I output columns; the MMA tile is hw gate + hw up rows
-        rows_b_map = 2 * swiglu_inter;
-    } else if (!swap && p.bn == 256) {
-        if (tiles_a * ((N + 255) / 256) * 2 <= sms) {
-            p.bn = 128;  // under half a wave: more, smaller tiles
-        } else {
-            int bn = 256;
-            for (int cand : {240, 224, 208, 192})
-                if (waves_cost(N, cand) < waves_cost(N, bn)) bn = cand;
-            p.bn = bn;
-        }
-    }
-    p.tilesA = (p.rowsA + kBM - 1) / kBM;
-    const int tilesB = swiglu_inter ? (swiglu_inter + p.swiglu_hw - 1) / p.swiglu_hw : (p.rowsB + p.bn - 1) / p.bn;
-    p.tiles = p.tilesA * tilesB;
-    const long long total = (long long)p.tiles * p.kb_total;
-    int grid = p.tiles < sms ? p.tiles : sms;
-    // Few tiles relative to the SM count (HBM-bound decode shapes): stream-K -- the tiles x k-blocks space is cut into one equal
-    // contiguous range per SM, so every SM streams the same number of weight bytes.
-    p.streamk = 0;
-    if (swap && p.tiles < 4 * sms && total >= 2 * sms) {
-        const int g2 = (int)(total < sms ? total : sms);
-        const long long per = total / g2;  // >= 2 k-blocks per CTA
-        const int maxslots = (int)((p.kb_total + per - 1) / per) + 1;
-        Workspace ws;
-        if (!get_workspace(&ws)) return B200_ERR_WORKSPACE;
-        const size_t need = (size_t)p.tiles * maxslots * p.bn * kBM * sizeof(float);
-        if (need <= ws.scratch_bytes && (size_t)p.tiles <= ws.n_tickets) {
-            p.streamk = 1, p.maxslots = maxslots, grid = g2;
-            p.partial = reinterpret_cast<float *>(ws.scratch);
-            p.tickets = ws.tickets;
-        }
-    }
-    p.acc_bufs = 2 * p.bn <= 512 ? 2 : 1;
+    p.rowsA = M, p.rowsB = p.ldc = swiglu_inter ? swiglu_inter : N;  // (SwiGLU: I output columns; the MMA tile is hw gate + hw up rows)
+    p.bn = plan.bn, p.splits = plan.splits, p.swiglu_hw = swiglu_inter ? plan.bn / 2 : 0;
+    p.a_rows = std::min(kBM, (M + 7) / 8 * 8);
+    p.tilesA = (M + kBM - 1) / kBM;
+    p.tiles = p.tilesA * ((cols + p.bn - 1) / p.bn);
+    const int grid = p.splits > 1 ? p.tiles * p.splits : std::min(p.tiles, sms);
+    p.acc_bufs = 2;
     p.acc_stride = p.bn > 128 ? 256 : p.bn;
-    p.tmem_cols = pow2_cols(p.acc_bufs == 2 ? p.acc_stride + p.bn : p.bn);
-    const int stage_bytes = kATileBytes + p.bn * kBK * 2;
-    int stages = (int)((200 * 1024) / stage_bytes);  // (kTcSmem)
-    if (stages > kMaxStages) stages = kMaxStages;
-    if (stages < 2) return B200_ERR_UNSUPPORTED;
-    p.stages = stages;
-    const size_t smem = (size_t)stages * stage_bytes + 1024 /*alignment slack*/ + (2 * kMaxStages + 4) * 8 + 16;
+    p.tmem_cols = pow2_cols(p.acc_stride + p.bn);
+    const int stage_bytes = (p.a_rows + p.bn) * kBK * 2;
+    p.stages = std::min(kMaxStages, (int)(kRingBytes / stage_bytes));
+    const size_t smem = (size_t)p.stages * stage_bytes + (kATileBytes - p.a_rows * kBK * 2) + kTcExtra;
 
     CUtensorMap tmA, tmB;
-    if (!tile_map(&tmA, a_ptr, p.rowsA, K, kBM, bf16) || !tile_map(&tmB, b_ptr, rows_b_map, K, swiglu_inter ? p.swiglu_hw : p.bn, bf16)) {
-        set_error("gemm_tc: cuTensorMapEncodeTiled failed (rows %d/%d, K %d)", p.rowsA, p.rowsB, K);
+    if (!tile_map(&tmA, x, M, K, p.a_rows, bf16) || !tile_map(&tmB, w, cols, K, swiglu_inter ? p.swiglu_hw : p.bn, bf16)) {
+        set_error("gemm_tc: cuTensorMapEncodeTiled failed (rows %d/%d, K %d)", M, cols, K);
         return B200_ERR_CUDA;
     }
     auto launch = [&](auto kern) {
         allow_smem(reinterpret_cast<const void *>(kern), kTcSmem);
-        launch_pdl(kern, dim3(grid), dim3(kTcThreads), smem, st, true, tmA, tmB, p);
+        launch_pdl_cluster(kern, dim3(grid), dim3(kTcThreads), smem, st, true, (unsigned)p.splits, tmA, tmB, p);
     };
     if (bf16) launch(gemm_tc_kernel<__nv_bfloat16>);
     else launch(gemm_tc_kernel<__half>);
     return cuda_status("gemm_tc launch");
 }
 
-int launch_gemm_tc(const void *x, const void *w, void *y, int M, int N, int K, int dtype, cudaStream_t st) {
-    return launch_gemm_tc_impl(x, w, y, M, N, K, dtype, 0, Finish{0, -1, nullptr}, st);
+int launch_gemm_tc(const void *x, const void *w, void *y, int M, int N, int K, int dtype, cudaStream_t st, const float *row_scale) {
+    return launch_gemm_tc_impl(x, w, y, M, N, K, dtype, 0, Finish{0, -1, nullptr, row_scale}, st);
 }
 
 int launch_gemm_tc_act(const void *x, const void *w, void *y, int M, int N, int K, const float *bias, int act, int dtype, cudaStream_t st) {
-    return launch_gemm_tc_impl(x, w, y, M, N, K, dtype, 0, Finish{1, act, bias}, st);
+    return launch_gemm_tc_impl(x, w, y, M, N, K, dtype, 0, Finish{1, act, bias, nullptr}, st);
 }
 
 // act[M, inter] = silu(x . Wgate^T) * (x . Wup^T), w = [2 * inter, K] (gate rows, then up rows): the gate_up linear and launchSiluAndMul in one
-// kernel (prefill sizes, M > 128); the [M, 2 * inter] intermediate is never written.  B200_ERR_UNSUPPORTED: use the two launchers.
-int launch_gemm_tc_swiglu(const void *x, const void *w, void *act, int M, int inter, int K, int dtype, cudaStream_t st) {
-    return launch_gemm_tc_impl(x, w, act, M, inter, K, dtype, inter, Finish{0, -1, nullptr}, st);
+// kernel; the [M, 2 * inter] intermediate is never written.  B200_ERR_UNSUPPORTED: use the two launchers.
+int launch_gemm_tc_swiglu(const void *x, const void *w, void *act, int M, int inter, int K, int dtype, cudaStream_t st, const float *row_scale) {
+    return launch_gemm_tc_impl(x, w, act, M, inter, K, dtype, inter, Finish{0, -1, nullptr, row_scale}, st);
 }
 
 // c[row, :] = act?(a[row, :] . W_e^T) with e = tile_expert[row / 128]: the experts' up or down projection as ONE launch.  a [max_rows, K]
@@ -870,12 +806,12 @@ int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, 
     if (max_rows < kBM || max_rows % kBM != 0 || K % 8 != 0 || K < kBK || N < 16 || !aligned16(a) || !aligned16(w) || !c) return B200_ERR_UNSUPPORTED;
     const bool bf16 = dtype == B200_BF16;
     GemmTcParams p = {};
-    p.C = c, p.ldc = N, p.K = K, p.swap = 0, p.is_bf16 = bf16 ? 1 : 0;
+    p.C = c, p.ldc = N, p.K = K, p.splits = 1, p.is_bf16 = bf16 ? 1 : 0;
     p.act = act, p.tile_expert = tile_expert, p.n_live = n_live;
     p.kb_total = (K + kBK - 1) / kBK;
     p.rowsA = max_rows, p.rowsB = N;
     p.bn = N >= 256 ? 256 : (N + 15) / 16 * 16;
-    p.tilesA = max_rows / kBM;
+    p.tilesA = max_rows / kBM, p.a_rows = kBM;
     p.tiles = p.tilesA * ((N + p.bn - 1) / p.bn);
     const int sms = sm_count();
     const int grid = p.tiles < sms ? p.tiles : sms;
@@ -883,11 +819,8 @@ int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, 
     p.acc_stride = p.bn > 128 ? 256 : p.bn;
     p.tmem_cols = pow2_cols(p.acc_bufs == 2 ? p.acc_stride + p.bn : p.bn);
     const int stage_bytes = kATileBytes + p.bn * kBK * 2;
-    int stages = (int)((200 * 1024) / stage_bytes);  // (kTcSmem)
-    if (stages > kMaxStages) stages = kMaxStages;
-    if (stages < 2) return B200_ERR_UNSUPPORTED;
-    p.stages = stages;
-    const size_t smem = (size_t)stages * stage_bytes + 1024 + (2 * kMaxStages + 4) * 8 + 16;
+    p.stages = std::min(kMaxStages, (int)(kRingBytes / stage_bytes));
+    const size_t smem = (size_t)p.stages * stage_bytes + kTcExtra;
     CUtensorMap tmA, tmB;
     if (!tile_map(&tmA, a, max_rows, K, kBM, bf16) || !tile_map(&tmB, w, experts * N, K, p.bn, bf16)) {
         set_error("gemm_tc grouped: cuTensorMapEncodeTiled failed (rows %d, experts %d x %d, K %d)", max_rows, experts, N, K);

@@ -70,7 +70,7 @@ struct GemvArgs {
     // push.n > 0: y is this rank's PARTIAL sum of a row-sharded linear; the reducer stores it into every rank's exchange buffer
     // (peer-mapped memory: posted NVLink writes of LL words, common.cuh) instead of `y`, so that the consumers read only local memory
     TpPush push;
-    // finish: y = act(T(sum) + out_bias) (bias_act in common.cuh; gemv_qd.cuh and gemv_rs.cuh, not with SwiGLU, fp32 output or a partial)
+    // finish: y = act(T(sum) + out_bias) (bias_act in common.cuh; dense weights in gemv_qd.cuh, not with SwiGLU or fp32 output)
     int finish;
     int out_act;            // b200_act_t, -1: none
     const float *out_bias;  // [N] or NULL

@@ -192,7 +192,7 @@ gemv_qd_kernel(const GemvArgs a) {
                 }
             } else if (ok) {
                 const size_t o = (size_t)m * N + R * u + r;
-                if (a.finish) v = bias_act<T>(v, a.out_bias, R * u + r, a.out_act);
+                if (kDense && a.finish) v = bias_act<T>(v, a.out_bias, R * u + r, a.out_act);
                 if (a.y_f32) reinterpret_cast<float *>(a.y)[o] = v;
                 else reinterpret_cast<T *>(a.y)[o] = Elem<T>::from_f(v);
             }

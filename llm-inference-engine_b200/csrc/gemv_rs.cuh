@@ -218,7 +218,6 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
                         for (int i = 0; i < 4; ++i)
                             if (row_ok(u, r0 + i)) {
                                 const size_t idx = (size_t)m * N + R * u + r0 + i;
-                                if (a.finish) o[i] = bias_act<T>(o[i], a.out_bias, R * u + r0 + i, a.out_act);
                                 if (a.y_f32) reinterpret_cast<float *>(a.y)[idx] = o[i];
                                 else reinterpret_cast<T *>(a.y)[idx] = Elem<T>::from_f(o[i]);
                             }

@@ -271,7 +271,7 @@ dequant_vec_kernel(const uint8_t *__restrict__ w, const void *__restrict__ scale
         float f[8];
         if constexpr (FMT == B200_W_FP8E4M3) {
             const uint2 q = *reinterpret_cast<const uint2 *>(w + e0);
-            const float sc = reinterpret_cast<const float *>(scales)[n];
+            const float sc = scales ? reinterpret_cast<const float *>(scales)[n] : 1.0f;  // (none: the codes' own values, exact in T)
 #pragma unroll
             for (int j = 0; j < 8; ++j) f[j] = e4m3_to_f((uint8_t)(((j < 4 ? q.x : q.y) >> (8 * (j & 3))) & 0xffu)) * sc;
         } else {
@@ -373,7 +373,7 @@ int b200_linear(const void *x, const void *w, const void *scales, const void *ze
             if (rc == B200_OK) done = 1;
             else if (rc != B200_ERR_UNSUPPORTED) return rc;
         }
-        // dense 16-bit beyond that (and shapes the GEMV cannot take): tcgen05 GEMM (swap-AB + stream-K for M <= 128, 128x256 tiles above)
+        // dense 16-bit beyond that (and shapes the GEMV cannot take): tcgen05 GEMM
         if (!done && M > 4 && b16 && w_format == B200_W_DENSE) {
             rc = launch_gemm_tc(x, w, y, M, N, K, dtype, st);
             if (rc == B200_OK) done = 1;
@@ -493,7 +493,7 @@ int b200_transpose2d(const void *src, void *dst, int rows, int cols, int dtype, 
     return cuda_status("transpose2d launch");
 }
 
-// In the linear where its kernel has that ending, as a pass of its own over y elsewhere (fp32, 17 to 128 rows, one token of rows of more than 3072 k): the same
+// In the linear where its kernel has that ending, as a pass of its own over y elsewhere (fp32, up to 16 rows of more than 3072 k): the same
 // bits.  The pass took 16 us for 3085 x 8192 and 5 for 4096 x 2048 (with its launch 18 and 7), 2 to 4 us of launch for decoded tokens.
 int b200_linear_act(const void *x, const void *w, const float *bias, void *y, int M, int K, int N, int act, int dtype, b200_stream_t stream) {
     B200_REQUIRE(x && w && y, "linear_act: null pointer");
@@ -509,7 +509,7 @@ int b200_linear_act(const void *x, const void *w, const float *bias, void *y, in
         a.M = M, a.K = K, a.N = N;
         a.finish = 1, a.out_act = act, a.out_bias = bias;
         rc = launch_gemv_nk(a, dtype, WF_DENSE, false, st);
-    } else if (dtype != B200_F32 && M > 128) {
+    } else if (dtype != B200_F32) {
         rc = launch_gemm_tc_act(x, w, y, M, N, K, bias, act, dtype, st);
     }
     if (rc != B200_ERR_UNSUPPORTED) return rc;
@@ -522,7 +522,7 @@ int b200_linear_swiglu(const void *x, const void *w_gate_up, void *act, int M, i
     B200_REQUIRE(M >= 0 && K > 0 && inter_size > 0, "linear_swiglu: bad shape M=%d K=%d inter=%d", M, K, inter_size);
     B200_REQUIRE(dtype == B200_F16 || dtype == B200_BF16, "linear_swiglu: 16-bit activations only (dtype %d)", dtype);
     if (M == 0) return B200_OK;
-    const int rc = launch_gemm_tc_swiglu(x, w_gate_up, act, M, inter_size, K, dtype, as_stream(stream));
+    const int rc = M <= 128 ? B200_ERR_UNSUPPORTED : launch_gemm_tc_swiglu(x, w_gate_up, act, M, inter_size, K, dtype, as_stream(stream));
     if (rc == B200_ERR_UNSUPPORTED) set_error("linear_swiglu: shape M=%d K=%d inter=%d not served by the fused tensor-core kernel (M > 128, K %% 8 == 0, inter >= 128)", M, K, inter_size);
     return rc;
 }

@@ -149,7 +149,7 @@ def linear_plan(M, K, N, fmt, fused_rows=16, swiglu=False, push=False):
         if g:
             return ("norm_kernel + " + g["kernel"], 1, g)
     if fmt == "dense" and M > 4:
-        return ("un-fused gemm_tc (tcgen05, swap-AB stream-K)" if M <= 128 else "un-fused gemm_tc", 1, None)
+        return ("un-fused gemm_tc", 1, None)
     for step in (16, 8, 4):  # linear.cu: quantised weights in passes
         if M > (8 if step == 16 else 4) * step:
             continue
