@@ -33,7 +33,7 @@ struct GemmTcParams {
     void *C;
     int ldc;
     int rowsA, rowsB, K;
-    int tilesA, tiles, kb_total;
+    int tilesA, tilesB, kb_total;
     int splits;    // CTAs of a cluster that share the k of one tile (then a CTA has one tile), or 1: tiles are dealt round-robin
     int bn;        // UMMA N: rows of B per tile, multiple of 16, <= 256
     int a_rows;    // rows of A that a stage loads: all 128, or fewer where A has fewer (what lies below them in a stage fills accumulator rows that nobody stores)
@@ -47,9 +47,9 @@ struct GemmTcParams {
     // B stage), the epilogue reads both halves of the accumulator and writes silu(gate) * up: C [rowsA, I], rowsB = I.  0: plain GEMM.
     int swiglu_inter;
     int swiglu_hw;  // gate (and up) columns per tile: bn = 2 * swiglu_hw (128, 112 or 96: whichever wastes least of the last wave)
-    // Grouped GEMM (mixture of experts): every 128-row tile of A belongs to ONE expert, tile_expert[ta]; B = the experts' weights stacked
+    // Grouped GEMM (mixture of experts): every tile of a_rows rows of A (32, 64 or 128) belongs to ONE expert, tile_expert[ta]; B = the experts' weights stacked
     // [experts * rowsB, K], so tile (ta, tb) multiplies B rows [tile_expert[ta] * rowsB + tb * bn, +bn).  Only the first *n_live row
-    // tiles hold rows (a device-side count: the host launches the worst case); all three roles skip the others alike.  NULL: plain.
+    // tiles hold rows (a device-side count): those are dealt, and no others.  NULL: plain.
     const int *tile_expert;
     const int *n_live;
     int act;        // b200_act_t applied to the result before it is stored, -1: none (plain and grouped GEMM, not the SwiGLU epilogue)
@@ -60,16 +60,16 @@ struct GemmTcParams {
 
 // A CTA's pieces of work: k-blocks [kb0, kb1) of output tiles.
 struct Seg {
-    int tile, kb0, kb1;
+    int ta, tb, kb0, kb1;
 };
 struct SegIter {
     const GemmTcParams &p;
-    int item;
-    __device__ SegIter(const GemmTcParams &pp) : p(pp), item(blockIdx.x / pp.splits) {}
+    int item, tilesA, tiles;
+    __device__ SegIter(const GemmTcParams &pp) : p(pp), item(blockIdx.x / pp.splits), tilesA(pp.tile_expert ? *pp.n_live : pp.tilesA), tiles(tilesA * pp.tilesB) {}
     __device__ bool next(Seg &s) {
-        if (item >= p.tiles) return false;
+        if (item >= tiles) return false;
         const int rank = blockIdx.x % p.splits;
-        s.tile = item, s.kb0 = p.kb_total * rank / p.splits, s.kb1 = p.kb_total * (rank + 1) / p.splits;
+        s.ta = item % tilesA, s.tb = item / tilesA, s.kb0 = p.kb_total * rank / p.splits, s.kb1 = p.kb_total * (rank + 1) / p.splits;
         item += gridDim.x / p.splits;
         return true;
     }
@@ -192,18 +192,8 @@ __device__ __forceinline__ void scale16(uint32_t (&r)[16], const float *scale, i
     for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * b[e]);
 }
 
-// bias_act on 16 consecutive outputs of one row, the first of them column n0 of `cols`.  The choice of the activation stands outside the columns (inside, an
-// epilogue outlasted the products it should hide behind: a layer of 3085 rows with a biased up projection of 8192 columns 638 us, now 572), the biases come in 16-byte loads where they can.
-template <typename T> __device__ __forceinline__ void finish16(uint32_t (&r)[16], const float *bias, int n0, int cols, int act) {
-    float v[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e) v[e] = round_to<T>(__uint_as_float(r[e]));
-    if (bias) {
-        float b[16];
-        columns16(bias, n0, cols, b);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] += b[e];
-    }
+// an activation (-1: none) of 16 numbers, the choice outside of them
+__device__ __forceinline__ void act16(float (&v)[16], int act) {
     if (act == B200_ACT_RELU2) {
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = act_apply(v[e], B200_ACT_RELU2);
@@ -217,6 +207,21 @@ template <typename T> __device__ __forceinline__ void finish16(uint32_t (&r)[16]
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = act_apply(v[e], B200_ACT_GELU_TANH);
     }
+}
+
+// bias_act on 16 consecutive outputs of one row, the first of them column n0 of `cols`.  The choice of the activation stands outside the columns (inside, an
+// epilogue outlasted the products it should hide behind: a layer of 3085 rows with a biased up projection of 8192 columns 638 us, now 572), the biases come in 16-byte loads where they can.
+template <typename T> __device__ __forceinline__ void finish16(uint32_t (&r)[16], const float *bias, int n0, int cols, int act) {
+    float v[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) v[e] = round_to<T>(__uint_as_float(r[e]));
+    if (bias) {
+        float b[16];
+        columns16(bias, n0, cols, b);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] += b[e];
+    }
+    act16(v, act);
 #pragma unroll
     for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(v[e]);
 }
@@ -230,9 +235,10 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
-// Output columns [c0, c1) (steps of 16, counted from the tile's first) of row i of a tile in column tile tb, from accumulator columns that `get` fetches.
-template <typename T, typename GET> __device__ __forceinline__ void finish_tile(const GemmTcParams &p, int i, int tb, int c0, int c1, GET get) {
+// Output columns [c0, c1) (steps of 16, counted from the tile's first) of row `row` of tile (ta, tb), from accumulator columns that `get` fetches.
+template <typename T, typename GET> __device__ __forceinline__ void finish_tile(const GemmTcParams &p, int ta, int row, int tb, int c0, int c1, GET get) {
     T *C = reinterpret_cast<T *>(p.C);
+    const int i = row < p.a_rows ? ta * p.a_rows + row : p.rowsA;  // (accumulator rows below A's: nobody's)
     if (p.swiglu_inter) {
         // gate in accumulator columns [0, hw), up in [hw, 2 hw): both rounded to T first (the reference's linear writes a T
         // tensor that launchSiluAndMul reads back, src/kernels/silu_and_mul.cu:6-41), same expression as silu_and_mul_kernel
@@ -261,9 +267,13 @@ template <typename T, typename GET> __device__ __forceinline__ void finish_tile(
         if (p.scale) scale16(r, p.scale, j0 + c, p.rowsB);
         if (p.finish) {
             finish16<T>(r, p.bias, j0 + c, p.rowsB, p.act);
-        } else if (p.act >= 0) {
+        } else {
+            float v[16];
 #pragma unroll
-            for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(act_apply(__uint_as_float(r[e]), p.act));
+            for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r[e]);
+            act16(v, p.act);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(v[e]);
         }
         const int valid = min(16, p.rowsB - (j0 + c));
         if (i < p.rowsA && valid > 0) store_row16<T>(C + (size_t)i * p.ldc + j0 + c, r, valid);
@@ -318,14 +328,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int s = 0;  // (stage and phase by counting: a remainder and a quotient per k-block were a third of what a narrow tile's block took)
             uint32_t ph = 1;
             while (si.next(sg)) {
-                const int ta = sg.tile % p.tilesA, tb = sg.tile / p.tilesA;
-                if (p.tile_expert && ta >= *p.n_live) continue;
+                const int ta = sg.ta, tb = sg.tb;
                 const int brow = (p.tile_expert ? p.tile_expert[ta] * p.rowsB : 0) + tb * p.bn;
                 for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
                     bar_wait(empty0 + 8 * s, ph);
                     const uint32_t sa = s_u32(smem + (size_t)s * stage_bytes);
                     bar_expect_tx(full0 + 8 * s, (uint32_t)stage_bytes);
-                    tma_load_2d(sa, &tmA, kb * kBK, ta * kBM, full0 + 8 * s);
+                    tma_load_2d(sa, &tmA, kb * kBK, ta * p.a_rows, full0 + 8 * s);
                     if (p.swiglu_inter) {  // box = hw rows: the gate rows, then the up rows of the same columns
                         tma_load_2d(sa + a_tile_bytes, &tmB, kb * kBK, tb * p.swiglu_hw, full0 + 8 * s);
                         tma_load_2d(sa + a_tile_bytes + p.swiglu_hw * kBK * 2, &tmB, kb * kBK, p.swiglu_inter + tb * p.swiglu_hw, full0 + 8 * s);
@@ -345,10 +354,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         uint32_t ph = 0;
         const bool issuer = elect_one();
         for (; issuer && si.next(sg); ++t) {
-            if (p.tile_expert && sg.tile % p.tilesA >= *p.n_live) {
-                --t;  // a row tile without rows: not a tile at all for the accumulator rotation
-                continue;
-            }
             const int acc = t % p.acc_bufs;
             bar_wait(tempty0 + 8 * acc, ((t / p.acc_bufs) & 1) ^ 1);  // the epilogue has drained this accumulator
             tc_fence_after();
@@ -377,11 +382,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         Seg sg;
         int t = 0;
         for (; si.next(sg); ++t) {
-            const int ta = sg.tile % p.tilesA, tb = sg.tile / p.tilesA;
-            if (p.tile_expert && ta >= *p.n_live) {
-                --t;
-                continue;
-            }
             const int acc = t % p.acc_bufs;
             bar_wait(tfull0 + 8 * acc, (t / p.acc_bufs) & 1);
             tc_fence_after();
@@ -399,7 +399,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     for (int e = 0; e < 16; ++e) mine[(size_t)(c + e) * kBM] = __uint_as_float(r[e]);
                 }
             } else {
-                finish_tile<T>(p, ta * kBM + q * 32 + lane, tb, 0, p.swiglu_inter ? p.swiglu_hw : p.bn, fetch);
+                finish_tile<T>(p, sg.ta, q * 32 + lane, sg.tb, 0, p.swiglu_inter ? p.swiglu_hw : p.bn, fetch);
             }
             tc_fence_before();
             __syncwarp();
@@ -411,10 +411,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         __syncthreads();
         cluster_sync_all();
         const int tile = blockIdx.x / p.splits, rank = blockIdx.x % p.splits;
-        if (warp >= 2 && tile < p.tiles) {
+        if (warp >= 2) {
             const int q = warp & 3, cols = (p.swiglu_inter ? p.swiglu_hw : p.bn) / p.splits;
             const uint32_t at = s_u32(smem) + (uint32_t)(q * 32 + lane) * 4;
-            finish_tile<T>(p, tile % p.tilesA * kBM + q * 32 + lane, tile / p.tilesA, rank * cols, (rank + 1) * cols, [&](int c, uint32_t (&r)[16]) {
+            finish_tile<T>(p, tile % p.tilesA, q * 32 + lane, tile / p.tilesA, rank * cols, (rank + 1) * cols, [&](int c, uint32_t (&r)[16]) {
                 float v[16];
                 for (int x = 0; x < p.splits; ++x) {
                     const uint32_t from = in_cta(at + (uint32_t)c * kBM * 4, (uint32_t)x);
@@ -451,7 +451,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // Measured: see pair_takes.
 struct GemmPairParams {
     void *C;
-    int ldc, rowsA, rowsB, kb_total, tilesA, tiles;
+    int ldc, rowsA, rowsB, kb_total, tilesA, tilesB;
     int bn, bn2, n_wide;
     int stages, is_bf16;
     int swiglu_inter;  // as above: gate rows come from the leader's half of B, up rows from its peer's; tile widths count both
@@ -524,6 +524,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     pdl_wait();
     pdl_launch_dependents();
 
+    const int tilesA = p.tilesA, tiles = tilesA * p.tilesB;
     // a wait that runs out: no more copies, no more products, NaN for the tiles that are left, and the other CTA's waits on them run out in turn
     auto wait = [&](uint32_t bar, uint32_t parity) { return mbar_wait_guarded(bar, parity, p.wait, kWaitGemmPair); };
     auto width_of = [&](int tb) { return tb < p.n_wide ? p.bn : p.bn2; };
@@ -538,8 +539,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             int it = 0, s = 0;
             uint32_t ph = 1;
             bool live = true;
-            for (int item = pair; live && item < p.tiles; item += pairs) {
-                const int ta = item % p.tilesA, tb = item / p.tilesA, w = width_of(tb);
+            for (int item = pair; live && item < tiles; item += pairs) {
+                const int ta = item % tilesA, tb = item / tilesA, w = width_of(tb);
                 const int arow = ta * 2 * kBM + (int)rank * kBM;
                 const int brow = p.swiglu_inter ? (rank ? p.swiglu_inter : 0) + col_of(tb) : col_of(tb) + (int)rank * (w >> 1);
                 const CUtensorMap *mb = tb < p.n_wide ? &tmB : &tmB2;
@@ -566,8 +567,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             int s = 0, t = 0;
             uint32_t ph = 0;
             bool live = true;
-            for (int item = pair; live && item < p.tiles; item += pairs, ++t) {
-                const uint32_t idesc = instr_desc_f16(p.is_bf16 != 0, 2 * kBM, width_of(item / p.tilesA));
+            for (int item = pair; live && item < tiles; item += pairs, ++t) {
+                const uint32_t idesc = instr_desc_f16(p.is_bf16 != 0, 2 * kBM, width_of(item / tilesA));
                 const int acc = t & 1;
                 live = wait(tempty0 + 8 * acc, ((t >> 1) & 1) ^ 1);
                 if (!live) break;
@@ -595,8 +596,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         T *C = reinterpret_cast<T *>(p.C);
         int t = 0;
         bool live = true;
-        for (int item = pair; item < p.tiles; item += pairs, ++t) {
-            const int ta = item % p.tilesA, tb = item / p.tilesA, w = width_of(tb), acc = t & 1, col0 = col_of(tb);
+        for (int item = pair; item < tiles; item += pairs, ++t) {
+            const int ta = item % tilesA, tb = item / tilesA, w = width_of(tb), acc = t & 1, col0 = col_of(tb);
             live = live && __all_sync(0xffffffffu, wait(tfull0 + 8 * acc, (t >> 1) & 1));
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 256);
@@ -683,8 +684,9 @@ struct TilePlan {
     int bn, splits;
     double ns;
 };
-static TilePlan plan_tiles(int M, int cols, int K, int sms, int step, int only = 0) {  // only: this many CTAs per tile (0: any)
-    const int rows = std::min(kBM, (M + 7) / 8 * 8), tiles_a = (M + kBM - 1) / kBM, kb = (K + kBK - 1) / kBK, widest = std::min(256, (cols + step - 1) / step * step);
+// tiles_a row tiles that load `rows` rows each; only: this many CTAs per tile (0: any)
+static TilePlan plan_tiles(int tiles_a, int rows, int cols, int K, int sms, int step, int only = 0) {
+    const int kb = (K + kBK - 1) / kBK, widest = std::min(256, (cols + step - 1) / step * step);
     TilePlan best = {widest, 1, 1e30};
     for (int splits : {1, 2}) {
         if (only && splits != only) continue;
@@ -712,6 +714,25 @@ static bool pair_takes(int M, int cols, int K, int sms, const TilePlan &one) {
     return choose_widths(t256, cols, pairs).cost * ((K + kBK - 1) / kBK) * 1.5 + 600 < one.ns;
 }
 
+// the launch itself: `rows` rows of A, `cols` of B
+static int launch_pair(GemmPairParams &p, const void *x, const void *w, int rows, int cols, int K, cudaStream_t st) {
+    const bool bf16 = p.is_bf16;
+    const size_t smem = (size_t)p.stages * kPairStageBytes + kTcExtra + 16;
+    CUtensorMap tmA, tmB, tmB2;
+    if (!tile_map(&tmA, x, rows, K, kBM, bf16) || !tile_map(&tmB, w, cols, K, p.bn / 2, bf16) || !tile_map(&tmB2, w, cols, K, p.bn2 / 2, bf16)) {
+        set_error("gemm_tc pair: cuTensorMapEncodeTiled failed (rows %d/%d, K %d)", rows, cols, K);
+        return B200_ERR_CUDA;
+    }
+    const int grid = 2 * std::min(p.tilesA * p.tilesB, sm_count() / 2);
+    auto launch = [&](auto kern) {
+        allow_smem(reinterpret_cast<const void *>(kern), smem);
+        launch_pdl_cluster(kern, dim3(grid), dim3(kPairThreads), smem, st, true, 2u, tmA, tmB, tmB2, p);
+    };
+    if (bf16) launch(gemm_tc_pair_kernel<__nv_bfloat16>);
+    else launch(gemm_tc_pair_kernel<__half>);
+    return cuda_status("gemm_tc pair launch");
+}
+
 struct Finish {
     int on, act;
     const float *bias, *scale;
@@ -724,23 +745,10 @@ static int launch_gemm_pair(const void *x, const void *w, void *y, int M, int N,
     p.kb_total = (K + kBK - 1) / kBK, p.is_bf16 = bf16 ? 1 : 0, p.swiglu_inter = swiglu_inter;
     p.tilesA = (M + 2 * kBM - 1) / (2 * kBM);
     const PairWidths pw = choose_widths(p.tilesA, cols, pairs);
-    p.bn = pw.bn, p.bn2 = pw.bn2, p.n_wide = pw.n_wide, p.tiles = p.tilesA * pw.n_tiles;
+    p.bn = pw.bn, p.bn2 = pw.bn2, p.n_wide = pw.n_wide, p.tilesB = pw.n_tiles;
     p.finish = fin.on, p.act = fin.act, p.bias = fin.bias, p.scale = fin.scale;
     p.stages = 6, p.wait = wait_guard();
-    const size_t smem = (size_t)p.stages * kPairStageBytes + kTcExtra + 16;
-    CUtensorMap tmA, tmB, tmB2;
-    if (!tile_map(&tmA, x, M, K, kBM, bf16) || !tile_map(&tmB, w, cols, K, p.bn / 2, bf16) || !tile_map(&tmB2, w, cols, K, p.bn2 / 2, bf16)) {
-        set_error("gemm_tc pair: cuTensorMapEncodeTiled failed (rows %d/%d, K %d)", M, cols, K);
-        return B200_ERR_CUDA;
-    }
-    const int grid = 2 * std::min(p.tiles, pairs);
-    auto launch = [&](auto kern) {
-        allow_smem(reinterpret_cast<const void *>(kern), smem);
-        launch_pdl_cluster(kern, dim3(grid), dim3(kPairThreads), smem, st, true, 2u, tmA, tmB, tmB2, p);
-    };
-    if (bf16) launch(gemm_tc_pair_kernel<__nv_bfloat16>);
-    else launch(gemm_tc_pair_kernel<__half>);
-    return cuda_status("gemm_tc pair launch");
+    return launch_pair(p, x, w, M, cols, K, st);
 }
 
 static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int N, int K, int dtype, int swiglu_inter, const Finish &fin, cudaStream_t st) {
@@ -749,8 +757,9 @@ static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int
     const bool bf16 = dtype == B200_BF16;
     if (swiglu_inter && swiglu_inter < 128) return B200_ERR_UNSUPPORTED;
     const int sms = sm_count(), cols = swiglu_inter ? 2 * swiglu_inter : N;
-    TilePlan plan = plan_tiles(M, cols, K, sms, 16);
-    if (swiglu_inter) plan = plan_tiles(M, cols, K, sms, 32, plan.splits);  // (the plain linear's order of summation: the same bits)
+    const int a_rows = std::min(kBM, (M + 7) / 8 * 8), tiles_a = (M + kBM - 1) / kBM;
+    TilePlan plan = plan_tiles(tiles_a, a_rows, cols, K, sms, 16);
+    if (swiglu_inter) plan = plan_tiles(tiles_a, a_rows, cols, K, sms, 32, plan.splits);  // (the plain linear's order of summation: the same bits)
     if (pair_takes(M, cols, K, sms, plan)) return launch_gemm_pair(x, w, y, M, N, K, dtype, swiglu_inter, fin, st);
     GemmTcParams p = {};
     p.C = y, p.K = K, p.is_bf16 = bf16 ? 1 : 0;
@@ -759,10 +768,9 @@ static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int
     p.kb_total = (K + kBK - 1) / kBK;
     p.rowsA = M, p.rowsB = p.ldc = swiglu_inter ? swiglu_inter : N;  // (SwiGLU: I output columns; the MMA tile is hw gate + hw up rows)
     p.bn = plan.bn, p.splits = plan.splits, p.swiglu_hw = swiglu_inter ? plan.bn / 2 : 0;
-    p.a_rows = std::min(kBM, (M + 7) / 8 * 8);
-    p.tilesA = (M + kBM - 1) / kBM;
-    p.tiles = p.tilesA * ((cols + p.bn - 1) / p.bn);
-    const int grid = p.splits > 1 ? p.tiles * p.splits : std::min(p.tiles, sms);
+    p.a_rows = a_rows;
+    p.tilesA = tiles_a, p.tilesB = (cols + p.bn - 1) / p.bn;
+    const int tiles = p.tilesA * p.tilesB, grid = p.splits > 1 ? tiles * p.splits : std::min(tiles, sms);
     p.acc_bufs = 2;
     p.acc_stride = p.bn > 128 ? 256 : p.bn;
     p.tmem_cols = pow2_cols(p.acc_stride + p.bn);
@@ -798,31 +806,33 @@ int launch_gemm_tc_swiglu(const void *x, const void *w, void *act, int M, int in
     return launch_gemm_tc_impl(x, w, act, M, inter, K, dtype, inter, Finish{0, -1, nullptr, row_scale}, st);
 }
 
-// c[row, :] = act?(a[row, :] . W_e^T) with e = tile_expert[row / 128]: the experts' up or down projection as ONE launch.  a [max_rows, K]
-// (rows grouped by expert, every expert padded to whole 128-row tiles), w [experts * N, K], c [max_rows, N]; *n_live row tiles are live.
+// c[row, :] = act?(a[row, :] . W_e^T) with e = tile_expert[row / tile]: the experts' up or down projection as ONE launch.  a [max_rows, K]
+// (rows grouped by expert, every expert padded to whole tiles of `tile` rows: 32, 64 or 128), w [experts * N, K], c [max_rows, N]; *n_live row
+// tiles are live, of which the launch expects the even share (every expert pads half a tile).  (Tiles of 256 rows on CTA pairs: 64 us where
+// 128 take 48, 16384 rows of 32 experts, 2048 x 512.)
 int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, int N, int K, int experts, const int *tile_expert,
-                           const int *n_live, int act, int dtype, cudaStream_t st) {
+                           const int *n_live, int act, int dtype, cudaStream_t st, int tile) {
     if (dtype != B200_BF16 && dtype != B200_F16) return B200_ERR_UNSUPPORTED;
-    if (max_rows < kBM || max_rows % kBM != 0 || K % 8 != 0 || K < kBK || N < 16 || !aligned16(a) || !aligned16(w) || !c) return B200_ERR_UNSUPPORTED;
+    if (max_rows < tile || max_rows % tile != 0 || K % 8 != 0 || K < kBK || N < 16 || !aligned16(a) || !aligned16(w) || !c) return B200_ERR_UNSUPPORTED;
     const bool bf16 = dtype == B200_BF16;
+    const int sms = sm_count(), most = max_rows / tile, likely = std::max(1, most - experts / 2);
     GemmTcParams p = {};
     p.C = c, p.ldc = N, p.K = K, p.splits = 1, p.is_bf16 = bf16 ? 1 : 0;
     p.act = act, p.tile_expert = tile_expert, p.n_live = n_live;
     p.kb_total = (K + kBK - 1) / kBK;
     p.rowsA = max_rows, p.rowsB = N;
-    p.bn = N >= 256 ? 256 : (N + 15) / 16 * 16;
-    p.tilesA = max_rows / kBM, p.a_rows = kBM;
-    p.tiles = p.tilesA * ((N + p.bn - 1) / p.bn);
-    const int sms = sm_count();
-    const int grid = p.tiles < sms ? p.tiles : sms;
-    p.acc_bufs = 2 * p.bn <= 512 ? 2 : 1;
+    p.a_rows = tile, p.tilesA = most;
+    p.bn = plan_tiles(likely, tile, N, K, sms, 16, 1).bn;
+    p.tilesB = (N + p.bn - 1) / p.bn;
+    const int grid = std::min(most * p.tilesB, sms);
+    p.acc_bufs = 2;
     p.acc_stride = p.bn > 128 ? 256 : p.bn;
-    p.tmem_cols = pow2_cols(p.acc_bufs == 2 ? p.acc_stride + p.bn : p.bn);
-    const int stage_bytes = kATileBytes + p.bn * kBK * 2;
+    p.tmem_cols = pow2_cols(p.acc_stride + p.bn);
+    const int stage_bytes = (p.a_rows + p.bn) * kBK * 2;
     p.stages = std::min(kMaxStages, (int)(kRingBytes / stage_bytes));
-    const size_t smem = (size_t)p.stages * stage_bytes + kTcExtra;
+    const size_t smem = (size_t)p.stages * stage_bytes + (kATileBytes - p.a_rows * kBK * 2) + kTcExtra;
     CUtensorMap tmA, tmB;
-    if (!tile_map(&tmA, a, max_rows, K, kBM, bf16) || !tile_map(&tmB, w, experts * N, K, p.bn, bf16)) {
+    if (!tile_map(&tmA, a, max_rows, K, p.a_rows, bf16) || !tile_map(&tmB, w, experts * N, K, p.bn, bf16)) {
         set_error("gemm_tc grouped: cuTensorMapEncodeTiled failed (rows %d, experts %d x %d, K %d)", max_rows, experts, N, K);
         return B200_ERR_CUDA;
     }

@@ -870,9 +870,18 @@ int rec_cols(const b200_hybrid_layer_t &l) {
     return 0;
 }
 
+// Rows of an expert's tiles in the tcgen05 grouped GEMM.  A tile's k-block loads its rows and the expert's, so small tiles load fewer rows
+// that nobody needs.  Vasolix-shaped models of four layers, us a prompt
+// with its first token, 128-row tiles (from 1024 pairs) and 64-row tiles on mma.sync below -> now: 32 experts of 2048 x 512, 94 tokens 1016 -> 853, 267 1019 -> 952,
+// 600 1096 -> 1057; 16 experts of 1024 x 512, 300 tokens 745 -> 656.
+int expert_tile(int pairs, int experts) {
+    const int rows = pairs / std::max(experts, 1);
+    return rows > 48 ? 128 : rows > 20 ? 64 : 32;
+}
+
 int max_rows_of(const b200_hybrid_config_t &c, const b200_hybrid_layer_t &l) {
     const int pairs = c.max_tokens * l.top;
-    return ((pairs + 127) / 128 + l.experts) * 128;  // the larger of the two row-tile sizes
+    return ((pairs + 127) / 128 + l.experts) * 128;  // the largest of the row-tile sizes
 }
 
 int latent_gate_rows(const b200_hybrid_layer_t &l) { return l.head_gate == 2 ? 0 : (l.head_gate ? l.heads : l.heads * l.vdim); }
@@ -965,7 +974,7 @@ Carve carve(const b200_hybrid *m) {
     k.meta = align256((8 * (T / 64 + (size_t)c.max_seqs + 1) + 5 * T + 3 * (size_t)c.max_seqs + 1 + (size_t)c.max_seqs * c.max_pages_per_seq +
                        4 * T + 2 * lheads * (t_pad / 64) + 2 * (size_t)c.num_layers + kTokenShareCtas) * 4);
     // moe ints: sel_expert | pair_row [T*top each] | row_token [rows] | tile_expert [rows / tile] | n_tiles
-    k.moe_i = align256((2 * T * top + rows + rows / kMoeTileM + 4) * 4);
+    k.moe_i = align256((2 * T * top + rows + rows / 32 + 4) * 4);
     // moe floats: sel_weight [T*top] | row_weight [rows] | shared_gate [T]
     k.moe_f = align256((T * top + rows + T) * 4);
     k.rec = align256(T * n_rec * 4), k.f32c = align256(2 * T * n_heads * 4), k.cat = align256(T * n_cat * es);
@@ -1875,9 +1884,9 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         const int pairs = NT * l.top;
         const bool softmax = l.route == B200_ROUTE_SOFTMAX;
         const int outputs = softmax ? l.experts + l.identity : l.experts + (l.shared_ff > 0 ? 1 : 0);  // sigmoid: the shared expert's gate row comes last
-        // prompt-sized batches of a 16-bit engine: 128-row tiles on the tcgen05 grouped GEMM; otherwise 64-row tiles on mma.sync / SIMT
-        const bool tc = !f32 && pairs >= 1024 && width % 8 == 0 && l.expert_ff % 8 == 0 && width >= 64 && l.expert_ff >= 64;
-        const int tile = tc ? 128 : kMoeTileM;
+        // 16-bit engines beyond the decode batches: the tcgen05 grouped GEMM; otherwise 64-row tiles on mma.sync / SIMT
+        const bool tc = !f32 && (pairs >= 1024 || NT > 64) && width % 8 == 0 && l.expert_ff % 8 == 0 && width >= 64 && l.expert_ff >= 64;
+        const int tile = tc ? expert_tile(pairs, l.experts) : kMoeTileM;
         const int max_rows = ((pairs + tile - 1) / tile + std::min(l.experts, pairs)) * tile;
         const int max_tiles = max_rows / tile;
         int *sel_expert = m->moe_i, *pair_row = sel_expert + pairs, *row_token = pair_row + pairs, *tile_expert = row_token + max_rows,
@@ -1915,13 +1924,13 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         else if (!tile_live) RUN(launch_moe_gather(dt, m->x, row_token, row_weight, m->xg, n_live, max_rows, width, tile, st));
         const int up_act = l.gated ? -1 : l.act;
         char *inner = (char *)m->u;
-        if (tc) RUN(launch_gemm_tc_grouped(m->xg, l.w_up, m->u, max_rows, n_up, width, l.experts, tile_expert, n_live, up_act, dt, st));
+        if (tc) RUN(launch_gemm_tc_grouped(m->xg, l.w_up, m->u, max_rows, n_up, width, l.experts, tile_expert, n_live, up_act, dt, st, tile));
         else RUN(launch_moe_grouped_gemm(dt, m->xg, l.w_up, m->u, tile_expert, n_live, max_tiles, n_up, width, up_act, st, live_rows, tile_live));
         if (l.gated) {
             inner += (size_t)max_rows * n_up * es;
             RUN(launch_gated_activation(dt, m->u, inner, max_rows, l.expert_ff, l.act, n_live, tile, st, l.act_limit, l.act_slope));
         }
-        if (tc) RUN(launch_gemm_tc_grouped(inner, l.w_down, m->yrows, max_rows, width, l.expert_ff, l.experts, tile_expert, n_live, -1, dt, st));
+        if (tc) RUN(launch_gemm_tc_grouped(inner, l.w_down, m->yrows, max_rows, width, l.expert_ff, l.experts, tile_expert, n_live, -1, dt, st, tile));
         else RUN(launch_moe_grouped_gemm(dt, inner, l.w_down, m->yrows, tile_expert, n_live, max_tiles, width, l.expert_ff, -1, st, live_rows, tile_live));
         if (l.shared_ff > 0) {
             char *sin = (char *)m->us;

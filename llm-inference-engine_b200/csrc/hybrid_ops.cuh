@@ -263,9 +263,9 @@ int launch_gated_activation(int dtype, const void *in, void *out, int rows, int 
 int launch_poly_norm(int dtype, void *x, const float *coef, float eps, int rows, int cols, cudaStream_t st);
 // in place: x[r, c] = act(x[r, c] + bias[c]); bias NULL: none; act < 0: none
 int launch_bias_activation(int dtype, void *x, const float *bias, size_t rows, int cols, int act, cudaStream_t st);
-// gemm_tc.cu: the same product on tcgen05 for row tiles of 128 (16-bit dtypes, K >= 64 and a multiple of 8; B200_ERR_UNSUPPORTED otherwise)
+// gemm_tc.cu: the same product on tcgen05 for row tiles of `tile` rows (32, 64, 128; 16-bit dtypes, K >= 64 and a multiple of 8; B200_ERR_UNSUPPORTED otherwise)
 int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, int N, int K, int experts, const int *tile_expert,
-                           const int *n_live, int act, int dtype, cudaStream_t st);
+                           const int *n_live, int act, int dtype, cudaStream_t st, int tile = 128);
 // c[row, n] = act?(sum_k a[row, k] * w[tile_expert[row / kMoeTileM]][n, k]);  rows >= n_tiles * kMoeTileM are skipped
 // live_rows: rows at the head of every tile that a caller reads afterwards (the others may stay unwritten); tile_live (moe_few_rows_takes): each tile's own number, taken 8 or
 // 16 (live_rows) at a time
