@@ -15,9 +15,10 @@
 // partial, as in gemv_mma.cuh.
 // Measured, 4 layers of 7B size, us per decode step (the kernels before -> now): dense 2 tokens 430 -> 370, 8: 435 -> 375, 16 ragged 517 -> 447;
 // FP8 2: 328 -> 263, 4: 382 -> 261, 8: 388 -> 280, 16 ragged 520 -> 382; INT4 2: 383 -> 273, 4: 433 -> 276, 8: 573 -> 296, 16: 617 -> 451.  The gate / up
-// linear of 16 FP8 tokens (90 MB): 41 -> 25 us.  FP8, a lane's activations as consecutive eights and tiles of two tokens a line (before -> now, us per launch, 1 / 8 / 16
-// tokens): K = 4096, N = 4096 4.9 / 6.1 / 8.6 -> 4.8 / 5.6 / 8.0, N = 12288 9.7 / 11.1 / 14.4 -> 9.7 / 10.8 / 14.1, K = 11008, N = 4096 9.8 / 11.3 / 19.7 -> 9.7 / 10.5 / 17.9,
-// K = 8192, N = 7168 11.5 / 13.0 / 19.5 -> 11.7 / 12.4 / 17.8.  A norm on the fragments in front of the product was slower than a norm kernel: every CTA redid all rows
+// linear of 16 FP8 tokens (90 MB): 41 -> 25 us.  FP8, a lane's k as two sixteens 64 apart (before -> now, us per launch, 1 / 8 / 16
+// tokens): K = 4096, N = 4096 4.9 / 6.0 / 8.5 -> 4.8 / 5.4 / 7.3, N = 12288 9.7 / 11.1 / 14.4 -> 9.5 / 10.5 / 13.4, K = 11008, N = 4096 9.7 / 11.5 / 19.7 -> 9.5 / 10.5 / 17.2,
+// K = 8192, N = 7168 11.3 / 13.1 / 19.6 -> 11.3 / 12.0 / 17.3; the steps above, 16 ragged FP8 382 -> 351.  (As consecutive eights, in 8-byte reads of the weights: 1 token 1 to 3 %
+// slower than before, 16 tokens 7.8 / 13.8 / 18.3 / 18.5.)  A norm on the fragments in front of the product was slower than a norm kernel: every CTA redid all rows
 // (16 dense tokens 490 against 449).
 #pragma once
 #include "gemv_mma.cuh"
@@ -31,10 +32,8 @@ constexpr int kRsBlocks = 8;            // 32-k blocks of a part that a warp hol
 // weights are A -- up to 8 tokens fill B, more take a second one, the dequantised rows serve both -- so that what a unit costs beside its weights
 // (waits, hand-off, addresses: two thirds of the instructions of an INT4 unit of 8 rows) is paid half as often.
 __host__ __device__ constexpr int rs_rows(bool dense) { return dense ? kMmaRows : 16; }
-// fp32 values of one warp's tile: [16 tokens][8 rows]; quantised [8 NT tokens][16 rows], two tokens a line of 32 values that is turned by 8 a line: the lanes' stores
-// and the reducer's 16-byte reads fall on different banks, and three stages of 16 FP8 rows of 4096 k fit beside the tiles of 16 tokens (16 rows + 4: two)
-__host__ __device__ constexpr int rs_tile(bool dense, int nt) { return dense ? 16 * kMmaRows : 8 * nt * 16; }
-__device__ __forceinline__ int rs_tile_at(int token, int row) { return (token >> 1) * 32 + ((16 * (token & 1) + row + 8 * (token >> 1)) & 31); }
+// fp32 values of one warp's tile: [16 tokens][8 rows]; quantised [8 NT tokens][16 rows + 4]: the lanes' stores fall on different banks
+__host__ __device__ constexpr int rs_tile(bool dense, int nt) { return dense ? 16 * kMmaRows : 8 * nt * 20; }
 
 struct RsGeom {
     int part_k, parts;  // k per part (a multiple of 128)
@@ -163,7 +162,7 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
                 float4 sums[PASSES];
 #pragma unroll
                 for (int q = 0; q < PASSES; ++q) {
-                    const float *slot = tiles + (size_t)b * kMmaWarps * TILE + (kDense ? lane * 4 : rs_tile_at(m0 + 8 * q, r0));
+                    const float *slot = tiles + (size_t)b * kMmaWarps * TILE + (kDense ? lane * 4 : (m0 + 8 * q) * 20 + r0);
                     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                     for (int w2 = 0; w2 < kMmaWarps; ++w2) {  // fixed order: deterministic
@@ -249,10 +248,10 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
 
     const int ngroups_k = FMT == WF_INT4 ? K / 128 : 0;
     constexpr int NG = NB / 4;
-    // the k of a lane's 8 activations of block j, counted from the slice: the block's t-th eight, or (INT4) the j-th 8 of the 32 consecutive k of a group that the
-    // lane's 16-byte piece of a weight row holds.  (FP8 had the latter too, over two pieces: a load of activations then met 16 lines of the first-level cache instead
-    // of 8, and half of every sector, which is what 16 tokens waited for: see the file's header.)
-    auto k_of = [&](int j) -> int { return FMT != WF_INT4 ? 32 * j + 8 * t : 128 * (j >> 2) + 32 * t + 8 * (j & 3); };
+    // the k of a lane's 8 activations of block j, counted from the slice: the block's t-th eight (dense), or 8 of the 32 k of a group that the lane's pieces of 16 bytes
+    // of a weight row hold: consecutive ones (INT4, one piece), or two times 16, 64 apart (FP8; with 32 in a row there too a load of activations met 16 lines of the
+    // first-level cache instead of 8, which is what 16 tokens waited for: see the file's header)
+    auto k_of = [&](int j) -> int { return kDense ? 32 * j + 8 * t : FMT == WF_FP8 ? 64 * (j >> 1) + 16 * t + 8 * (j & 1) : 128 * (j >> 2) + 32 * t + 8 * (j & 3); };
     // INT4 parameters of the slice's groups.  A warp needs 16 rows x 2 groups of them per unit -- 2-byte and 1-byte loads a round trip to L2 away,
     // several units' worth of streaming.  So its 32 lanes fetch TWO units at once (lane: unit lane / 16 of the batch, row lane % 16), a batch ahead of
     // the one in use, and a unit's scales and zero points reach their lanes by shuffles.
@@ -337,16 +336,12 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
                 for (int q = 0; q < NG; ++q) {
                     if (4 * q >= nb) break;
                     // this lane's 32 weights of rows g and g + 8 in the group
-                    uint32_t wa[FMT == WF_FP8 ? 8 : 4], wb[FMT == WF_FP8 ? 8 : 4];
-                    if constexpr (FMT == WF_FP8) {
+                    constexpr int PIECES = FMT == WF_FP8 ? 2 : 1;
+                    uint32_t wa[4 * PIECES], wb[4 * PIECES];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            *reinterpret_cast<uint2 *>(wa + 2 * i) = *reinterpret_cast<const uint2 *>(wrow + 128 * q + 32 * i);
-                            *reinterpret_cast<uint2 *>(wb + 2 * i) = *reinterpret_cast<const uint2 *>(wrow8 + 128 * q + 32 * i);
-                        }
-                    } else {
-                        *reinterpret_cast<uint4 *>(wa) = *reinterpret_cast<const uint4 *>(wrow + 64 * q);
-                        *reinterpret_cast<uint4 *>(wb) = *reinterpret_cast<const uint4 *>(wrow8 + 64 * q);
+                    for (int i = 0; i < PIECES; ++i) {
+                        *reinterpret_cast<uint4 *>(wa + 4 * i) = *reinterpret_cast<const uint4 *>(wrow + 64 * (PIECES * q + i));
+                        *reinterpret_cast<uint4 *>(wb + 4 * i) = *reinterpret_cast<const uint4 *>(wrow8 + 64 * (PIECES * q + i));
                     }
                     float c0[4] = {}, c1[4] = {};  // two chains: the k-steps of the first tokens, or (16 tokens) the first and the second eight
                     uint32_t zpa = 0, nza = 0, zpb = 0, nzb = 0;
@@ -404,9 +399,9 @@ gemv_rs_kernel(const GemvArgs a, const RsGeom geo) {
             } else {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const int at = rs_tile_at(2 * t + (e & 1), g + 8 * (e >> 1));
+                    const int at = (2 * t + (e & 1)) * 20 + g + 8 * (e >> 1);
                     slot[at] = acc[e];
-                    if constexpr (NT == 2) slot[8 * 16 + at] = acc2[e];
+                    if constexpr (NT == 2) slot[8 * 20 + at] = acc2[e];
                 }
             }
             __syncwarp();
@@ -429,9 +424,8 @@ inline bool gemv_rs_geometry(int M, int K, int max_units, int fmt, RsGeom *out) 
     g.parts = (K + g.part_k - 1) / g.part_k;
     g.max_units = max_units;
     const size_t bytes = fmt == WF_DENSE ? (size_t)g.part_k * 2 : (fmt == WF_FP8 ? (size_t)g.part_k : (size_t)g.part_k / 2);
-    // rows of a stage 64 (dense, INT4) or 32 (FP8) bytes apart modulo 128: the 16-byte reads of the eight lanes of a phase -- two rows' four pieces, 64 bytes of
-    // each -- fall on different banks, and so do the 8-byte reads of sixteen lanes, four rows' 32 bytes
-    g.row_stride = (int)((bytes + 127) / 128 * 128) + (fmt == WF_FP8 ? 32 : 64);
+    // rows of a stage 64 bytes apart modulo 128: the 16-byte reads of the eight lanes of a phase -- two rows' four pieces, 64 bytes of each -- fall on different banks
+    g.row_stride = (int)((bytes + 127) / 128 * 128) + 64;
     g.stage_bytes = rs_rows(fmt == WF_DENSE) * g.row_stride;
     const size_t budget = kRsSmem, fixed = gemv_rs_fixed_smem(g, fmt == WF_DENSE, M > 8 ? 2 : 1);
     if (fixed + (size_t)2 * g.stage_bytes > budget) return false;

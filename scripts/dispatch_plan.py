@@ -90,8 +90,8 @@ def gemv_rs_plan(M, K, N, fmt, swiglu=False):
     part_k = -(-groups // parts) * 128
     parts = -(-K // part_k)
     row = {"dense": part_k * 2, "fp8": part_k, "int4": part_k // 2}[fmt]
-    stage = rows * (-(-row // 128) * 128 + (32 if fmt == "fp8" else 64))
-    tile, vals = (128, 128) if dense else (8 * nt * 16, 128 * nt)
+    stage = rows * (-(-row // 128) * 128 + 64)
+    tile, vals = (128, 128) if dense else (8 * nt * 20, 128 * nt)
     fixed = (2 * RS_STAGES + 4) * 8 + 2 * MMA_WARPS * tile * 4 + (max_units * vals * 4 if parts > 1 else 0)
     if fixed + 2 * stage > 226 * 1024:
         return None
