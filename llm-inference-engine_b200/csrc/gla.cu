@@ -419,6 +419,102 @@ gla_step_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ de
     }
 }
 
+// A decode batch's whole mixer between its projections in one launch, a CTA per (head, sequence): the decays of the head's channels (four lanes a channel), the step
+// over the state as above, and the head's norm and gate.  What bounds it: round trips.  As three launches the step of 16 requests x 8 heads (dim 128, vdim 256) was
+// 4.1 us of decays, 8.3 of state and 2.7 of norm, 6 us of launches between them; here the state's rows are on their way while the decays are formed.
+// Measured there (three launches and the gaps between them -> one): 21 -> 10 us.
+// Four columns a thread, 16 row groups: vdim * 4 threads.
+constexpr int kDecodeVdim = 256;
+template <typename T>
+__global__ void __launch_bounds__(4 * kDecodeVdim, 1)
+gla_decode_kernel(const T *__restrict__ proj, int ld, int rank_col, const T *__restrict__ w_decay, const float *__restrict__ bias, float inv_tau, int rank,
+                  float *__restrict__ state, const int *__restrict__ seq_start, const int *__restrict__ seq_pos0, const int *__restrict__ seq_slot, int heads, int dim,
+                  int vdim, const float *__restrict__ norm, float eps, int gate_col, T *__restrict__ out) {
+    extern __shared__ __align__(16) float smf[];  // {a, k, q, -}[dim] | part[kStepRowGroups][vdim] | the token's low-rank vector [rank]
+    __shared__ float red[32];
+    const int h = blockIdx.x, s = blockIdx.y, t = seq_start[s], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (seq_start[s + 1] - t != 1) return;  // (a sequence without a token)
+    float4 *akq = reinterpret_cast<float4 *>(smf);
+    float *part = smf + 4 * (size_t)dim, *lo = part + kStepRowGroups * vdim;
+    const T *row = proj + (size_t)t * ld;
+    const int groups = vdim / 4, cg = tid % groups, rg = tid / groups, c = 4 * cg;
+    const bool fresh = seq_pos0[s] == 0;
+    float *slot = state + (((size_t)seq_slot[s] * heads + h) * dim) * vdim + c;
+    float4 sv[kStepUnroll];
+    auto fetch = [&](int i0) {
+#pragma unroll
+        for (int u = 0; u < kStepUnroll; ++u) {
+            const int i = i0 + u * kStepRowGroups;
+            sv[u] = (!fresh && i < dim) ? *reinterpret_cast<const float4 *>(slot + (size_t)i * vdim) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    fetch(rg);
+    float v[4];
+    load_n<T, 4>(row + 2 * heads * dim + h * vdim + c, v);
+    if (tid < rank) lo[tid] = Elem<T>::to_f(row[rank_col + tid]);
+    const float gate = tid < vdim ? Elem<T>::to_f(row[gate_col + h * vdim + tid]) : 0.0f, gain = tid < vdim ? norm[tid] : 0.0f;
+    __syncthreads();
+    const float qscale = rsqrtf((float)dim);
+    const int sub = tid & 3;
+    for (int i0 = 0; i0 < dim; i0 += blockDim.x >> 2) {  // (whole warps: the shuffles take every lane)
+        const int i = min(i0 + (tid >> 2), dim - 1);
+        const T *wr = w_decay + (size_t)(h * dim + i) * rank;
+        float z = 0.0f;
+        for (int r = 8 * sub; r < rank; r += 32) {
+            float f[8];
+            load8<T>(wr + r, f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) z = fmaf(f[e], lo[r + e], z);
+        }
+        z += __shfl_xor_sync(0xffffffffu, z, 1);
+        z += __shfl_xor_sync(0xffffffffu, z, 2);
+        if (sub == 0 && i0 + (tid >> 2) < dim) {
+            if (bias) z += bias[h * dim + i];
+            // log sigmoid(z) = min(z, 0) - log1p(exp(-|z|));  a = exp(log sigmoid(z) / tau)
+            akq[i] = make_float4(expf((fminf(z, 0.0f) - log1pf(expf(-fabsf(z)))) * inv_tau), Elem<T>::to_f(row[heads * dim + h * dim + i]),
+                                 Elem<T>::to_f(row[h * dim + i]) * qscale, 0.0f);
+        }
+    }
+    __syncthreads();
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int i0 = rg; i0 < dim; i0 += kStepRowGroups * kStepUnroll) {
+        if (i0 != rg) fetch(i0);
+#pragma unroll
+        for (int u = 0; u < kStepUnroll; ++u) {
+            const int i = i0 + u * kStepRowGroups;
+            if (i < dim) {
+                const float4 x = akq[i];
+                float4 n;
+                n.x = fmaf(x.x, sv[u].x, x.y * v[0]);
+                n.y = fmaf(x.x, sv[u].y, x.y * v[1]);
+                n.z = fmaf(x.x, sv[u].z, x.y * v[2]);
+                n.w = fmaf(x.x, sv[u].w, x.y * v[3]);
+                *reinterpret_cast<float4 *>(slot + (size_t)i * vdim) = n;
+                acc[0] = fmaf(n.x, x.z, acc[0]);
+                acc[1] = fmaf(n.y, x.z, acc[1]);
+                acc[2] = fmaf(n.z, x.z, acc[2]);
+                acc[3] = fmaf(n.w, x.z, acc[3]);
+            }
+        }
+    }
+    *reinterpret_cast<float4 *>(part + rg * vdim + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    __syncthreads();
+    float o = 0.0f;
+    if (tid < vdim) {
+#pragma unroll
+        for (int g = 0; g < kStepRowGroups; ++g) o += part[g * vdim + tid];
+    }
+    const float ss = warp_sum(o * o);
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();
+    if (tid < vdim) {
+        float sum = 0.0f;
+        for (int w = 0; w < (vdim + 31) / 32; ++w) sum += red[w];
+        const float inv = rsqrtf(sum / (float)vdim + eps);
+        out[((size_t)t * heads + h) * vdim + tid] = Elem<T>::from_f(o * inv * gain * (gate / (1.0f + expf(-gate))));
+    }
+}
+
 template <typename T, int RR, int TB>
 static void launch_gla_reg(const void *proj, int ld, const float *decay, float *state, float *o, const int *seq_start, const int *seq_pos0,
                            const int *seq_slot, dim3 grid, int heads, int dim, int vdim, int min_tokens, int max_tokens, cudaStream_t st) {
@@ -512,6 +608,25 @@ int launch_gla_decay(int dtype, const void *proj, int ld, int col0, const void *
         launch_plain(gla_decay_kernel<T>, dim3(nb, cb), dim3(256), (size_t)kDecayTokens * rank * sizeof(float), st, (const T *)proj, ld, col0, (const T *)w_decay, bias, 1.0f / tau, decay, tokens, rank, channels);
     });
     return cuda_status("gla_decay launch");
+}
+
+// B200_ERR_UNSUPPORTED (nothing launched): fp32, sizes that its threads do not share evenly, rows off their 16-byte boundaries.  Every sequence has one token.
+int launch_gla_decode(int dtype, const void *proj, int ld, int rank_col, const void *w_decay, const float *bias, float tau, int rank, float *state, const int *seq_start,
+                      const int *seq_pos0, const int *seq_slot, int n_seqs, int heads, int dim, int vdim, const float *norm, float eps, int gate_col, void *out,
+                      cudaStream_t st) {
+    if (n_seqs == 0) return B200_OK;
+    const size_t smem = (4 * (size_t)dim + (size_t)kStepRowGroups * vdim + rank) * sizeof(float);
+    if (dtype == B200_F32 || vdim % 32 != 0 || vdim > kDecodeVdim || rank % 8 != 0 || rank < 8 || rank > 4 * vdim || dim % 4 != 0 || dim > 1024 || ld % 8 != 0 || n_seqs > 65535 ||
+        smem > 48 * 1024 || !all_aligned16({proj, w_decay, state}))
+        return B200_ERR_UNSUPPORTED;
+    auto go = [&](auto kern, auto *to) {
+        using T = std::remove_pointer_t<decltype(to)>;
+        launch_plain(kern, dim3(heads, n_seqs), dim3(4 * vdim), smem, st, (const T *)proj, ld, rank_col, (const T *)w_decay, bias, 1.0f / tau, rank, state, seq_start, seq_pos0, seq_slot,
+                     heads, dim, vdim, norm, eps, gate_col, to);
+    };
+    if (dtype == B200_BF16) go(gla_decode_kernel<__nv_bfloat16>, (__nv_bfloat16 *)out);
+    else go(gla_decode_kernel<__half>, (__half *)out);
+    return cuda_status("gla_decode launch");
 }
 
 int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay, float *state, float *o, const int *seq_start,

@@ -6,7 +6,7 @@
 // the fp32 residual stream.  Launch sequence per layer:
 //   fused input projection (b200_linear: tcgen05 GEMM / weight-streaming GEMV by token count)
 //   attention mixer:  q/k whole-projection norm + pool append -> chunked sink attention (gate fused) -> output projection
-//   gla mixer:        decay (low-rank, fp32) -> recurrence over the state slots -> head norm * silu(gate) -> output projection
+//   gla mixer:        decay (low-rank, fp32) -> recurrence over the state slots -> head norm * silu(gate), one launch for a decode batch -> output projection
 //   latent mixer:     split + rotation + latent-row norm + pool append -> grouped GEMM over the heads (q into the latent space) -> windowed
 //                     sink attention over the latent rows -> grouped GEMM over the heads (value up-projection) -> gate -> output projection
 //   post-norm + residual add (fp32)
@@ -1835,11 +1835,17 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         } else {
             const int hd = l.heads * l.dim, hv = l.heads * l.vdim;
             const char *gate = (const char *)m->proj + (size_t)(2 * hd + hv) * es;
-            RUN(launch_gla_decay(dt, m->proj, lp.n_in, 2 * hd + 2 * hv, l.w_decay, l.decay_bias, l.tau, m->f32a, NT, l.decay_rank, hd, st));
             float *state = (float *)(m->state_pool + lp.state_off);
-            RUN(recurrence(l, [&] { return launch_chunk_gla(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
-                           [&](int kinds, int most) { return launch_gla_recurrent(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, st, kinds, most); }));
-            RUN(launch_gla_output(dt, m->f32b, l.out_norm, c.norm_eps, gate, lp.n_in, m->mix2, NT, l.heads, l.vdim, st));
+            rc = gla_kinds != kGlaOneToken ? B200_ERR_UNSUPPORTED
+                                           : launch_gla_decode(dt, m->proj, lp.n_in, 2 * hd + 2 * hv, l.w_decay, l.decay_bias, l.tau, l.decay_rank, state, d_start, d_pos0, d_slot, S, l.heads,
+                                                               l.dim, l.vdim, l.out_norm, c.norm_eps, 2 * hd + hv, m->mix2, st);
+            if (rc != B200_OK && rc != B200_ERR_UNSUPPORTED) return rc;
+            if (rc == B200_ERR_UNSUPPORTED) {
+                RUN(launch_gla_decay(dt, m->proj, lp.n_in, 2 * hd + 2 * hv, l.w_decay, l.decay_bias, l.tau, m->f32a, NT, l.decay_rank, hd, st));
+                RUN(recurrence(l, [&] { return launch_chunk_gla(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
+                               [&](int kinds, int most) { return launch_gla_recurrent(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, st, kinds, most); }));
+                RUN(launch_gla_output(dt, m->f32b, l.out_norm, c.norm_eps, gate, lp.n_in, m->mix2, NT, l.heads, l.vdim, st));
+            }
             n_mixed = hv;
         }
         RUN(linear(m, m->mix2, l.w_out, m->y, NT, n_mixed, width, st));

@@ -194,6 +194,10 @@ int launch_gla_decay(int dtype, const void *proj, int ld, int col0, const void *
                      int tokens, int rank, int channels, cudaStream_t st);
 // kinds: which portions the batch holds, when the host knows (one-token portions have a kernel of their own; the default launches both)
 constexpr int kGlaOneToken = 1, kGlaManyTokens = 2;
+// a batch of one-token portions: decay, step, norm and gate in one launch (rank_col, gate_col: columns of the low-rank vector and of the gate in proj)
+int launch_gla_decode(int dtype, const void *proj, int ld, int rank_col, const void *w_decay, const float *bias, float tau, int rank, float *state, const int *seq_start,
+                      const int *seq_pos0, const int *seq_slot, int n_seqs, int heads, int dim, int vdim, const float *norm, float eps, int gate_col, void *out,
+                      cudaStream_t st);
 int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay, float *state, float *o, const int *seq_start,
                          const int *seq_pos0, const int *seq_slot, int n_seqs, int heads, int dim, int vdim, cudaStream_t st,
                          int kinds = kGlaOneToken | kGlaManyTokens, int max_tokens = kAnyTokens);
