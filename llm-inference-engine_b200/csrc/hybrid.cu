@@ -71,11 +71,16 @@ __global__ void embed_rows_kernel(const int *__restrict__ ids, const T *__restri
 
 // x[t, :] += rmsnorm(y[t, :]) * g (and h_out[t, :] = T(x[t, :]) for the next projection), where y is either a dense row (y_dense) or the mixture
 //   sum_k y_rows[pair_row[t*top + k], :] + shared_gate[t] * y_shared[t, :].   trace (optional) receives the new x.
-template <typename T>
+// ROUTE (16-byte pieces only): the CTA also multiplies the new row by the `outputs` rows of the router that reads it next, fp32, in proj_f32_small_kernel's order of
+// summation; the first two rows of every warp are on their way while the norm is summed.  As a launch of its own that was 5 us and 1.5 in front of it for a decode
+// batch of 16 tokens and 33 outputs of 2048 (6.4 for one token); here it adds 4.
+constexpr int kRoutePieces = 4;  // 16-byte pieces of a router row that a lane has on its way, of each of two rows
+template <typename T, bool ROUTE = false>
 __global__ void __launch_bounds__(256)
 postnorm_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, const T *__restrict__ y_rows, const int *__restrict__ pair_row,
                          int top, const T *__restrict__ y_shared, const float *__restrict__ shared_gate, const float *__restrict__ g, float eps,
-                         int width, float *__restrict__ trace, T *__restrict__ h_out) {
+                         int width, float *__restrict__ trace, T *__restrict__ h_out, const T *__restrict__ router = nullptr, float *__restrict__ logits = nullptr,
+                         int outputs = 0) {
     extern __shared__ __align__(16) float ys[];  // [width]
     __shared__ float red[33];
     const int t = blockIdx.x;
@@ -120,6 +125,7 @@ postnorm_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, c
             for (int i = 0; i < V; i += 4) {
                 const float4 r = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 *reinterpret_cast<float4 *>(x + (size_t)t * width + c + i) = r;
+                if (ROUTE) *reinterpret_cast<float4 *>(ys + c + i) = r;
                 if (trace) *reinterpret_cast<float4 *>(trace + (size_t)t * width + c + i) = r;
             }
             if (h_out) st_v4(h_out + (size_t)t * width + c, pack16<T>(v));  // what the next sublayer's projections read (16-bit engines)
@@ -130,6 +136,15 @@ postnorm_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, c
         };
         const int c0 = threadIdx.x * V;
         float y0[V], x0[V], g0[V];
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        uint4 rw[2][kRoutePieces];
+        auto request = [&](int o, int k0) {  // pieces k0, k0 + 256, ... of outputs o and o + 8 (past the end: live ones, not used)
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+                for (int i = 0; i < kRoutePieces; ++i) rw[u][i] = ld_v4(router + (size_t)min(o + 8 * u, outputs - 1) * width + min(k0 + 256 * i, width - 8));
+        };
+        if constexpr (ROUTE) request(warp, lane * 8);
         if (c0 < width) {
             fetch(x + (size_t)t * width + c0, x0);
             fetch(g + c0, g0);
@@ -149,6 +164,33 @@ postnorm_residual_kernel(float *__restrict__ x, const T *__restrict__ y_dense, c
             fetch(g + c, gs);
             fetch(ys + c, y);
             finish(c, xs, gs, y, inv);
+        }
+        if constexpr (ROUTE) {
+            __syncthreads();  // the new row is there
+            for (int o = warp; o < outputs; o += 16) {
+                float a[2][4] = {};
+                for (int k0 = lane * 8; k0 < width; k0 += 256 * kRoutePieces) {
+#pragma unroll
+                    for (int i = 0; i < kRoutePieces; ++i) {
+                        if (k0 + 256 * i >= width) break;
+                        float f[8], g[2][8];
+                        load_vec<8>(ys + k0 + 256 * i, f);
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            unpack16<T>(rw[u][i], g[u]);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) a[u][e & 3] = fmaf(f[e], g[u][e], a[u][e & 3]);
+                        }
+                    }
+                    if (k0 + 256 * kRoutePieces < width) request(o, k0 + 256 * kRoutePieces);
+                    else if (o + 16 < outputs) request(o + 16, lane * 8);
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const float v = warp_sum((a[u][0] + a[u][1]) + (a[u][2] + a[u][3]));
+                    if (lane == 0 && o + 8 * u < outputs) logits[(size_t)t * outputs + o + 8 * u] = v;
+                }
+            }
         }
         return;
     }
@@ -1708,11 +1750,21 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
 
     auto cast_x = [&]() -> const void * { return f32 ? (const void *)m->x : (const void *)m->h; };
     auto postnorm = [&](const void *y_dense, const void *y_rows, const int *pair_row, int top, const void *y_shared, const float *gate,
-                        const float *g, float *trace) -> int {
+                        const float *g, float *trace, const void *router = nullptr, int outputs = 0) -> int {
+        if (router) {  // (16-bit; every row on a 16-byte boundary: see its caller)
+            auto go = [&](auto *h) {
+                using T = std::remove_pointer_t<decltype(h)>;
+                launch_plain(postnorm_residual_kernel<T, true>, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, m->x, (const T *)y_dense, (const T *)y_rows, pair_row, top,
+                             (const T *)y_shared, gate, g, c.norm_eps, width, trace, h, (const T *)router, m->f32a, outputs);
+            };
+            if (dt == B200_BF16) go((__nv_bfloat16 *)m->h);
+            else go((__half *)m->h);
+            return cuda_status("postnorm_residual (router) launch");
+        }
         B200_DISPATCH_DTYPE(dt, {
             launch_plain(postnorm_residual_kernel<T>, dim3(NT), dim3(256), (size_t)width * sizeof(float), st, m->x, (const T *)y_dense, (const T *)y_rows, pair_row, top,
                                                                                       (const T *)y_shared, gate, g, c.norm_eps, width, trace,
-                                                                                      f32 ? nullptr : (T *)m->h);
+                                                                                      f32 ? nullptr : (T *)m->h, (const T *)nullptr, (float *)nullptr, 0);
         });
         return cuda_status("postnorm_residual launch");
     };
@@ -1849,6 +1901,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             n_mixed = hv;
         }
         RUN(linear(m, m->mix2, l.w_out, m->y, NT, n_mixed, width, st));
+        bool routed = false;  // m->f32a holds the router's logits
         if (sum_norm) {
             RUN(sum_step(li, 0, m->y, nullptr, nullptr, nullptr, nullptr, trace));
         } else if (ln_post) {
@@ -1858,7 +1911,11 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             RUN(residual(true, m->y, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, l.norm, l.post1, l.ls1, pre, trace));
             h_normed = pre != nullptr;
         } else {
-            RUN(postnorm(m->y, nullptr, nullptr, 0, nullptr, nullptr, l.norm1, trace));
+            // few tokens: the router's product with the row that has just been formed
+            const int outputs = l.experts + (l.shared_ff > 0 ? 1 : 0);
+            routed = !f32 && l.mlp == B200_MLP_MOE && l.route != B200_ROUTE_SOFTMAX && NT < 64 && (long long)NT * outputs <= 8192 && outputs <= 128 && width % 8 == 0 &&
+                     all_aligned16({m->x, m->y, l.norm1, trace, m->h, l.w_router});
+            RUN(postnorm(m->y, nullptr, nullptr, 0, nullptr, nullptr, l.norm1, trace, routed ? l.w_router : nullptr, outputs));
             h_normed = false;
         }
         if (l.mlp == B200_MLP_NONE) continue;
@@ -1901,7 +1958,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         // router logits (+ shared gate), fp32: 16-bit engines multiply the 16-bit copy of the input on the tensor cores (products of 16-bit
         // values are exact in fp32 and the sums are fp32), others -- and widths the tensor-core kernel does not take -- the fp32 kernel
         // (a decode batch is a single 64-row tile there -- one CTA walking all of K -- so few tokens take the fp32 kernel as well)
-        rc = NT >= 64 ? launch_dense_f32out(dt, h2, l.w_router, m->f32a, NT, outputs, width, st) : B200_ERR_UNSUPPORTED;
+        rc = routed ? B200_OK : NT >= 64 ? launch_dense_f32out(dt, h2, l.w_router, m->f32a, NT, outputs, width, st) : B200_ERR_UNSUPPORTED;
         if (rc == B200_ERR_UNSUPPORTED)
             rc = dyt || sum_norm ? launch_proj_f32(dt, m->h, width, dt, l.w_router, nullptr, m->f32a, outputs, NT, outputs, width, st)
                      : launch_proj_f32(B200_F32, m->x, width, dt, l.w_router, nullptr, m->f32a, outputs, NT, outputs, width, st);
