@@ -131,8 +131,9 @@ static int norm_linear(b200_decoder *d, const void *x, const void *res_in, void 
                        const b200_linear_weight_t &w, int K, int N, bool swiglu, void *y, int M, cudaStream_t st, const TpExchange *tp = nullptr) {
     const b200_decoder_config_t &c = d->cfg;
     const bool b16 = c.dtype != B200_F32;
-    // one dense token, fp32 up to 4 tokens: the prologue runs inside the GEMV (SIMT kernels)
-    if ((M == 1 && c.w_format == B200_W_DENSE) || (!b16 && M <= 4)) {
+    // one dense token, fp32 up to 4 tokens: the prologue runs inside the GEMV (SIMT kernels); one INT4 token: in gemv_qd.cuh
+    const bool int4 = b16 && M == 1 && c.w_format == B200_W_INT4 && !tp;
+    if ((M == 1 && c.w_format == B200_W_DENSE) || (!b16 && M <= 4) || int4) {
         GemvArgs a = {};
         a.w = w.w, a.scales = w.scales, a.zeros = w.zeros;
         a.x = x, a.y = y;

@@ -61,7 +61,7 @@ struct GemvArgs {
     const void *bias;
     const void *gamma;
     float eps;
-    int norm;
+    int norm;            // (INT4: gemv_qd.cuh, in the norm kernel's order of summation)
     int M, K, N;
     int group;
     int inter;  // SwiGLU: rows (i, inter + i) form a unit, n_out = inter

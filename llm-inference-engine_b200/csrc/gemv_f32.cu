@@ -24,6 +24,7 @@ int launch_gemv_nk(const GemvArgs &a, int dtype, int fmt, bool swiglu, cudaStrea
         const int rc = dtype == B200_BF16 ? launch_gemv_qd_bf16(a, fmt, swiglu, st) : launch_gemv_qd_f16(a, fmt, swiglu, st);
         if (rc != B200_ERR_UNSUPPORTED) return rc;
     }
+    if (a.norm && fmt == WF_INT4) return B200_ERR_UNSUPPORTED;  // (no other kernel keeps the norm kernel's bits)
     if (a.finish) return B200_ERR_UNSUPPORTED;  // (in gemv_rs.cuh the ending cost every other caller 0.6 to 1.1 %)
     // 16-bit activations, no prologue: 2..16 tokens, and one token of FP8 weights, past which the weights stream with the activations in registers
     // (gemv_rs.cuh).  One dense token keeps the SIMT kernel and its fused norm: its weights alone fill the memory pipe, and the norm launch would come on

@@ -49,7 +49,9 @@ enum { QD_TWO_SLICES, QD_SLICE, QD_PART, QD_DENSE, QD_DENSE_LARGE };
 // longer have all of theirs: K = 2048, N = 6176 of 1 / 8 / 16 tokens 5.8 / 6.5 / 6.7 us for 5.3 / 6.0 / 6.6; for K = 3072 and 16 tokens, which 108 KB do not hold, 5.9 (gemv_rs 7.1)
 __host__ __device__ constexpr size_t qd_smem(int mode, int warps) { return (size_t)(mode == QD_DENSE ? 108 : mode == QD_DENSE_LARGE ? 148 : 160) * 1024 * warps / 16; }
 
-template <typename T, int FMT, bool kSwiGLU, int NT, int NW, int MODE>
+// NORM: one INT4 token with the residual add and RMSNorm in front (GemvArgs), in the norm kernel's order and roundings: the same bits as with a launch in
+// between.  Four 7B layers, one token: 203.0 us with norm kernels, 199.2 here (202.4 with the gains asked for behind the sum).
+template <typename T, int FMT, bool kSwiGLU, int NT, int NW, int MODE, bool NORM = false>
 __global__ void __launch_bounds__(NW * 32, 16 / NW)
 gemv_qd_kernel(const GemvArgs a) {
     static_assert(FMT == WF_DENSE || (FMT == WF_INT4 && NT == 1 && (MODE == QD_PART) == (NW == 16)), "dense, or INT4 of up to 8 tokens");
@@ -127,12 +129,67 @@ gemv_qd_kernel(const GemvArgs a) {
 #pragma unroll
         for (int i = 0; i < kQdRing; ++i) load(ring[i], MODE == QD_SLICE ? i : lp);
     }
+    // (the gains do not depend on the kernel in front either: those of a thread's first rows of eight)
+    constexpr int GN = NORM ? 512 / (NW * 32) : 1;
+    uint4 gain[GN];
+    if constexpr (NORM) {
+#pragma unroll
+        for (int v = 0; v < GN; ++v) {
+            const int i = threadIdx.x + v * NW * 32;
+            if (a.gamma && i < K / 8) gain[v] = ld_v4(reinterpret_cast<const T *>(a.gamma) + (size_t)8 * i);
+        }
+    }
     pdl_wait();
     pdl_launch_dependents();
 
     // activations, [token][group][i][t] 16-byte pieces in the order in which a lane's loads meet them: the 8 k at 32 i + 8 t (dense), or (INT4, in f16) at
     // 32 t + 8 i.  One block of zeros for the slots past M
     const int xstride = 2 * K + 64;  // bytes: the rows of tokens g and g + 1 fall on different banks
+    if constexpr (NORM) {
+        __shared__ float sums[16];
+        constexpr int vt = 512;  // threads of the norm kernel: one of ours does the work of one or two of them
+        auto place = [&](int i) { return smem + ((i & ~15) + (i & 3) * 4 + ((i >> 2) & 3)) * 16; };
+#pragma unroll
+        for (int v = threadIdx.x; v < vt; v += NW * 32) {
+            float ss = 0.0f;
+            for (int i = v; i < K / 8; i += vt) {
+                float f[8];
+                unpack16<T>(ld_v4(reinterpret_cast<const T *>(a.x) + (size_t)8 * i), f);
+                if (a.res_in) {
+                    float r[8];
+                    unpack16<T>(ld_v4(reinterpret_cast<const T *>(a.res_in) + (size_t)8 * i), r);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) f[e] = round_to<T>(f[e] + r[e]);
+                }
+                if (a.res_out && blockIdx.x == 0) st_v4(reinterpret_cast<T *>(a.res_out) + (size_t)8 * i, pack16<T>(f));
+                if (a.bias) {
+                    float b[8];
+                    unpack16<T>(ld_v4(reinterpret_cast<const T *>(a.bias) + (size_t)8 * i), b);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) f[e] = round_to<T>(f[e] + b[e]);
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+                *reinterpret_cast<uint4 *>(place(i)) = pack16<T>(f);  // (exact: f is of T)
+            }
+            ss = warp_sum(ss);
+            if (lane == 0) sums[v >> 5] = ss;
+        }
+        __syncthreads();
+        const float scale = rsqrtf(warp_sum(lane < (vt >> 5) ? sums[lane & 15] : 0.0f) / (float)K + a.eps);
+#pragma unroll
+        for (int w = 0; w < GN; ++w)
+            for (int v = threadIdx.x + w * NW * 32, i = v; i < K / 8; i += vt) {
+                float f[8], g[8];
+                unpack16<T>(*reinterpret_cast<const uint4 *>(place(i)), f);
+                if (a.gamma) {
+                    unpack16<T>(i == v ? gain[w] : ld_v4(reinterpret_cast<const T *>(a.gamma) + (size_t)8 * i), g);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) f[e] = (f[e] * g[e]) * scale;
+                }
+                *reinterpret_cast<uint4 *>(place(i)) = rs_fragment<T, FMT>(pack16<T>(f));
+            }
+    } else
     for (int idx = threadIdx.x; idx < a.M * (K / 8); idx += NW * 32) {
         const int m = idx / (K / 8), p8 = idx - m * (K / 8);
         const uint4 f = rs_fragment<T, FMT>(ld_v4(reinterpret_cast<const T *>(a.x) + (size_t)8 * idx));
@@ -302,9 +359,9 @@ gemv_qd_kernel(const GemvArgs a) {
 inline size_t gemv_qd_smem(int M, int K, int fmt, int warps) {
     return (size_t)M * (2 * (size_t)K + 64) + 256 + (size_t)2 * (fmt == WF_INT4 ? 16 : warps) * (M > 8 ? 16 : 8) * kQdTileRow * sizeof(float);
 }
-template <typename T, int FMT, bool SW, int NT, int NW, int MODE>
+template <typename T, int FMT, bool SW, int NT, int NW, int MODE, bool NORM = false>
 static int launch_gemv_qd_inst(const GemvArgs &a, int units, cudaStream_t st) {
-    auto kern = gemv_qd_kernel<T, FMT, SW, NT, NW, MODE>;
+    auto kern = gemv_qd_kernel<T, FMT, SW, NT, NW, MODE, NORM>;
     const size_t smem = gemv_qd_smem(a.M, a.K, FMT, NW);
     if (smem > qd_smem(MODE, NW)) return B200_ERR_UNSUPPORTED;
     if (!allow_smem(reinterpret_cast<const void *>(kern), qd_smem(MODE, NW), qd_smem(MODE, 16) + 2048)) return cuda_status("gemv_qd cudaFuncSetAttribute");
@@ -317,14 +374,16 @@ static int launch_gemv_qd_inst(const GemvArgs &a, int units, cudaStream_t st) {
 template <typename T>
 static int launch_gemv_qd_t(const GemvArgs &a, int fmt, bool swiglu, cudaStream_t st) {
     if (fmt == WF_FP8 || (fmt == WF_INT4 && (a.group != 128 || a.M > 8)) || a.M < 1 || a.M > 16 || a.K % 128 != 0 || !aligned16(a.w) || !aligned16(a.x)) return B200_ERR_UNSUPPORTED;
-    if (a.tp.world > 1 || a.norm || a.push.n > 0 || (swiglu && a.inter % 8 != 0)) return B200_ERR_UNSUPPORTED;
+    if (a.norm && (fmt != WF_INT4 || a.M != 1 || a.K > 16384 || !all_aligned16({a.res_in, a.res_out, a.bias, a.gamma}))) return B200_ERR_UNSUPPORTED;
+    if (a.tp.world > 1 || a.push.n > 0 || (swiglu && a.inter % 8 != 0)) return B200_ERR_UNSUPPORTED;
     const int units = swiglu ? (a.inter + kQdRows / 2 - 1) / (kQdRows / 2) : (a.N + kQdRows - 1) / kQdRows;
     auto fits = [&](int mode, int warps) { return gemv_qd_smem(a.M, a.K, fmt, warps) <= qd_smem(mode, warps); };
     if (fmt == WF_INT4) {
         const int mode = a.K > 4096 || !fits(QD_SLICE, 8) ? QD_PART : a.K > 2048 ? QD_SLICE : QD_TWO_SLICES;
-#define B200_QD_GO(SW) (mode == QD_PART ? launch_gemv_qd_inst<T, WF_INT4, SW, 1, 16, QD_PART>(a, units, st) \
-                        : mode == QD_SLICE ? launch_gemv_qd_inst<T, WF_INT4, SW, 1, 8, QD_SLICE>(a, units, st) : launch_gemv_qd_inst<T, WF_INT4, SW, 1, 8, QD_TWO_SLICES>(a, units, st))
-        return swiglu ? B200_QD_GO(true) : B200_QD_GO(false);
+#define B200_QD_GO(SW, NORM) (mode == QD_PART ? launch_gemv_qd_inst<T, WF_INT4, SW, 1, 16, QD_PART, NORM>(a, units, st) \
+                        : mode == QD_SLICE ? launch_gemv_qd_inst<T, WF_INT4, SW, 1, 8, QD_SLICE, NORM>(a, units, st) : launch_gemv_qd_inst<T, WF_INT4, SW, 1, 8, QD_TWO_SLICES, NORM>(a, units, st))
+        if (a.norm) return swiglu ? B200_QD_GO(true, true) : B200_QD_GO(false, true);
+        return swiglu ? B200_QD_GO(true, false) : B200_QD_GO(false, false);
 #undef B200_QD_GO
     }
     // Dense rows of at most 3072 k: there the start is most of a launch.  Longer ones fill gemv_rs.cuh's 200 KB ring before their wait, behind an attention or a
