@@ -36,7 +36,24 @@ latent_prep_kernel(const T *__restrict__ proj, int ld, int q_col, int kv_col, T 
     __shared__ float red[33];
     const int t = blockIdx.x, half = rot_dims / 2;
     const int pos = tok_pos[t];
+    const int page = kv_col >= 0 ? block_table[(size_t)tok_seq[t] * mpps + pos / kPageL] : -1;  // (on its way)
     float *cosv = cs, *sinv = cs + half;
+    constexpr int V = Elem<T>::kVec;
+    const T *row = proj + (size_t)t * ld;
+    const int per = dim + rot_dim;
+    const bool vec = dim % V == 0 && rot_dim % V == 0 && ld % V == 0 && q_col % V == 0 && ((reinterpret_cast<size_t>(proj) | reinterpret_cast<size_t>(qn)) & 15) == 0;
+    const bool vec_r = vec && (reinterpret_cast<size_t>(qr) & 15) == 0;
+    // The angles are a chain of fp64 of a few microseconds in one warp: the others move the un-rotated parts meanwhile, and the rotated ones go by pieces (3085 tokens of
+    // 16 heads of 128 + 64: 20.7 -> 15.3 us, 2 tokens 8.4 -> 5.7)
+    const bool early = !rt.pairs && vec && half <= 32;
+    if (early && threadIdx.x >= 32) {
+        const int pieces = dim / V;
+#pragma unroll 4
+        for (int idx = threadIdx.x - 32; idx < heads * pieces; idx += blockDim.x - 32) {
+            const int h = idx / pieces, c = (idx - h * pieces) * V;
+            st_v4(qn + ((size_t)h * t_pad + t) * dim + c, ld_v4(row + q_col + (size_t)h * per + c));
+        }
+    }
     for (int i = threadIdx.x; i < half; i += blockDim.x) {
         if (rt.turns) {  // the angle in turns, in fp64; only its fraction goes to fp32, so that a far position costs no bits
             const double a = (double)pos * rt.turns[i];
@@ -51,7 +68,6 @@ latent_prep_kernel(const T *__restrict__ proj, int ld, int q_col, int kv_col, T 
         }
     }
     __syncthreads();
-    const T *row = proj + (size_t)t * ld;
     // r-th element of a rotated vector that starts at `v`
     auto rotated = [&](const T *v, int r) -> float {
         const float self = Elem<T>::to_f(v[r]);
@@ -64,8 +80,6 @@ latent_prep_kernel(const T *__restrict__ proj, int ld, int q_col, int kv_col, T 
         if (r < rot_dims) return self * cosv[r - half] + Elem<T>::to_f(v[r - half]) * sinv[r - half];
         return self;
     };
-    const int per = dim + rot_dim;
-    constexpr int V = Elem<T>::kVec;
     // neighbouring pairs lie inside one 16-byte piece: the piece at column c (from the rotated part's start) turns in registers
     auto rotate_piece = [&](float *v, int c) {
 #pragma unroll
@@ -76,8 +90,7 @@ latent_prep_kernel(const T *__restrict__ proj, int ld, int q_col, int kv_col, T 
             }
         }
     };
-    if (rt.pairs && dim % V == 0 && rot_dim % V == 0 && ld % V == 0 && q_col % V == 0 &&
-        ((reinterpret_cast<size_t>(proj) | reinterpret_cast<size_t>(qn) | reinterpret_cast<size_t>(qr)) & 15) == 0) {
+    if (rt.pairs && vec_r) {
         const int pieces = per / V;
 #pragma unroll 4
         for (int idx = threadIdx.x; idx < heads * pieces; idx += blockDim.x) {
@@ -92,16 +105,40 @@ latent_prep_kernel(const T *__restrict__ proj, int ld, int q_col, int kv_col, T 
                 st_v4(qr + ((size_t)t * heads + h) * rot_dim + (c - dim), pack16<T>(v));
             }
         }
-    } else if (dim % V == 0 && rot_dim % V == 0 && ld % V == 0 && q_col % V == 0 &&
-        ((reinterpret_cast<size_t>(proj) | reinterpret_cast<size_t>(qn)) & 15) == 0) {  // the un-rotated part moves in 16-byte pieces
-        const int pieces = dim / V;
-        for (int idx = threadIdx.x; idx < heads * pieces; idx += blockDim.x) {
-            const int h = idx / pieces, c = (idx - h * pieces) * V;
-            st_v4(qn + ((size_t)h * t_pad + t) * dim + c, ld_v4(row + q_col + (size_t)h * per + c));
+    } else if (vec) {  // the un-rotated part moves in 16-byte pieces
+        if (!early) {
+            const int pieces = dim / V;
+            for (int idx = threadIdx.x; idx < heads * pieces; idx += blockDim.x) {
+                const int h = idx / pieces, c = (idx - h * pieces) * V;
+                st_v4(qn + ((size_t)h * t_pad + t) * dim + c, ld_v4(row + q_col + (size_t)h * per + c));
+            }
         }
-        for (int idx = threadIdx.x; idx < heads * rot_dim; idx += blockDim.x) {
-            const int h = idx / rot_dim, r = idx - h * rot_dim;
-            qr[((size_t)t * heads + h) * rot_dim + r] = Elem<T>::from_f(rotated(row + q_col + (size_t)h * per + dim, r));
+        if (!rt.pairs && vec_r && half % V == 0 && half > 0) {  // a piece of the first half turns with its partner of the second; behind them nothing turns
+            const int turned = half / V, rest = (rot_dim - rot_dims) / V, units = turned + rest;
+            for (int idx = threadIdx.x; idx < heads * units; idx += blockDim.x) {
+                const int h = idx / units, p = idx - h * units;
+                const T *from = row + q_col + (size_t)h * per + dim;
+                T *to = qr + ((size_t)t * heads + h) * rot_dim;
+                if (p >= turned) {
+                    st_v4(to + rot_dims + (p - turned) * V, ld_v4(from + rot_dims + (p - turned) * V));
+                    continue;
+                }
+                float a[V], b[V], x[V], y[V];
+                unpack16<T>(ld_v4(from + p * V), a);
+                unpack16<T>(ld_v4(from + half + p * V), b);
+#pragma unroll
+                for (int e = 0; e < V; ++e) {
+                    const float cv = cosv[p * V + e], sv = sinv[p * V + e];
+                    x[e] = a[e] * cv - b[e] * sv, y[e] = b[e] * cv + a[e] * sv;
+                }
+                st_v4(to + p * V, pack16<T>(x));
+                st_v4(to + half + p * V, pack16<T>(y));
+            }
+        } else {
+            for (int idx = threadIdx.x; idx < heads * rot_dim; idx += blockDim.x) {
+                const int h = idx / rot_dim, r = idx - h * rot_dim;
+                qr[((size_t)t * heads + h) * rot_dim + r] = Elem<T>::from_f(rotated(row + q_col + (size_t)h * per + dim, r));
+            }
         }
     } else {
         for (int idx = threadIdx.x; idx < heads * per; idx += blockDim.x) {
@@ -125,7 +162,6 @@ latent_prep_kernel(const T *__restrict__ proj, int ld, int q_col, int kv_col, T 
             for (int e = 0; e < V; ++e) ss = fmaf(v[e], v[e], ss);
         }
         const float inv = rsqrtf(block_sum(ss, red) / (float)kv_rank + eps);
-        const int page = block_table[(size_t)tok_seq[t] * mpps + pos / kPageL];
         if (page < 0 || c >= kv_rank + rot_dim) return;  // no page held: nothing is written (the host refuses such a batch)
         if (c < kv_rank) {
             float w[V];
@@ -144,7 +180,6 @@ latent_prep_kernel(const T *__restrict__ proj, int ld, int q_col, int kv_col, T 
     }
     ss = block_sum(ss, red);
     const float inv = rsqrtf(ss / (float)kv_rank + eps);
-    const int page = block_table[(size_t)tok_seq[t] * mpps + pos / kPageL];
     if (page < 0) return;  // no page held: nothing is written (the host refuses such a batch)
     T *dst = pool + ((size_t)page * kPageL + (pos % kPageL)) * (kv_rank + rot_dim);
     for (int c = threadIdx.x; c < kv_rank + rot_dim; c += blockDim.x)
