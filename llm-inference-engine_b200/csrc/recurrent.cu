@@ -102,7 +102,8 @@ delta_prep_kernel(const T *__restrict__ proj, int ld, int col0, const float *__r
 // The same for prompt-sized batches of four taps: a thread takes EIGHT channels (one 16-byte piece of a projected row) of kPrepTokens consecutive
 // rows, `tiles` times.  It reads every row of its piece once -- the taps are rows it already holds -- and its channels' weights once, a channel's four in
 // one access: one CTA per token read each input once per tap and 64 KB of weights per token (100 us for 2911 tokens of 4096 channels, where the bytes
-// take 12), and weights fetched one by one for every eight rows still cost 1024 sectors a warp (65 us; now 44).  The unit norm of a head is a butterfly over the
+// take 12), and weights fetched one by one for every eight rows still cost 1024 sectors a warp (65 us; 44 with
+// two tiles a CTA in 1.2 waves and a tail of copies; now 35).  The unit norm of a head is a butterfly over the
 // dim / 8 lanes that hold it.  grid (row groups, channel groups + 1): the last group copies the low-rank inputs and the steps.
 constexpr int kPrepTokens = 8, kPrepTaps = 4;
 template <typename T>
@@ -131,11 +132,16 @@ delta_prep_tile_kernel(const T *__restrict__ proj, int ld, int col0, const float
         const int t0 = (blockIdx.x * tiles + tile) * kPrepTokens, nt = min(kPrepTokens, tokens - t0);
         if (nt <= 0) return;
         if (copies) {
-            for (int tt = 0; tt < nt; ++tt) {
-                const T *row = proj + (size_t)(t0 + tt) * ld + col0 + channels;  // step | decay-in | gate-in
-                for (int r = threadIdx.x; r < rank; r += blockDim.x) lr_a[(size_t)(t0 + tt) * rank + r] = row[heads + r];
-                for (int r = threadIdx.x; r < gate_rank; r += blockDim.x) lr_g[(size_t)(t0 + tt) * gate_rank + r] = row[heads + rank + r];
-                for (int h = threadIdx.x; h < heads; h += blockDim.x) rec[(size_t)(t0 + tt) * lay.ld + lay.beta + h] = sigmoid_r(Elem<T>::to_f(row[h]));
+            // step | decay-in | gate-in, all tokens of the tile at once (token by token, 16 tokens were 16 round trips, and these CTAs the launch's tail)
+            const int cols = heads + rank + gate_rank;
+#pragma unroll 4
+            for (int i = threadIdx.x; i < nt * cols; i += blockDim.x) {
+                const int tt = i / cols, r = i - tt * cols;
+                const size_t tok = (size_t)(t0 + tt);
+                const T x = proj[tok * ld + col0 + channels + r];
+                if (r < heads) rec[tok * lay.ld + lay.beta + r] = sigmoid_r(Elem<T>::to_f(x));
+                else if (r < heads + rank) lr_a[tok * rank + r - heads] = x;
+                else lr_g[tok * gate_rank + r - heads - rank] = x;
             }
             continue;
         }
@@ -837,7 +843,12 @@ int launch_delta_prep(int dtype, const void *proj, int ld, int col0, const float
                         (2 * kv_heads * dim) % 256 == 0 && ld % 8 == 0 && col0 % 8 == 0 && all_aligned16({proj, rec, conv_w});
     const int channels = 2 * kv_heads * dim + heads * vdim;
     const int row_tiles = (tokens + kPrepTokens - 1) / kPrepTokens, groups = (channels / 8 + 255) / 256;
-    const int per = std::max(1, std::min(4, row_tiles * groups / (2 * sm_count())));  // tiles per CTA, two CTAs per SM left
+    // tiles per CTA: two CTAs share an SM, and the device works in whole waves of them (2911 tokens, 4096 channels: three tiles in one wave 35 us);
+    // a CTA's weights cost about a third of a tile
+    int per = 1;
+    auto waves_cost = [&](int p) { return (double)((groups * ((row_tiles + p - 1) / p) + 2 * sm_count() - 1) / (2 * sm_count())) * (p + 0.3); };
+    for (int p = 2; p <= 8; ++p)
+        if (waves_cost(p) < waves_cost(per)) per = p;
     const dim3 tile_grid((row_tiles + per - 1) / per, groups + 1);
     if (pieces && dtype == B200_BF16)
         launch_plain(delta_prep_tile_kernel<__nv_bfloat16>, dim3(tile_grid), dim3(256), 0, st, (const __nv_bfloat16 *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__nv_bfloat16 *)lr_a,
