@@ -759,8 +759,10 @@ static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int
     const int sms = sm_count(), cols = swiglu_inter ? 2 * swiglu_inter : N;
     const int a_rows = std::min(kBM, (M + 7) / 8 * 8), tiles_a = (M + kBM - 1) / kBM;
     TilePlan plan = plan_tiles(tiles_a, a_rows, cols, K, sms, 16);
-    if (swiglu_inter) plan = plan_tiles(tiles_a, a_rows, cols, K, sms, 32, plan.splits);  // (the plain linear's order of summation: the same bits)
-    if (pair_takes(M, cols, K, sms, plan)) return launch_gemm_pair(x, w, y, M, N, K, dtype, swiglu_inter, fin, st);
+    // Whether two CTAs add up a tile's k is the plain linear's choice for SwiGLU too (the same bits); its widths, and pairs in place of whole tiles, are its own.
+    const bool split = plan.splits > 1 && !pair_takes(M, cols, K, sms, plan);
+    if (swiglu_inter) plan = plan_tiles(tiles_a, a_rows, cols, K, sms, 32, split ? plan.splits : 1);
+    if (!split && pair_takes(M, cols, K, sms, plan)) return launch_gemm_pair(x, w, y, M, N, K, dtype, swiglu_inter, fin, st);
     GemmTcParams p = {};
     p.C = y, p.K = K, p.is_bf16 = bf16 ? 1 : 0;
     p.swiglu_inter = swiglu_inter;

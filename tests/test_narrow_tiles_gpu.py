@@ -43,7 +43,8 @@ def test_two_ctas_share_a_tile(M, K, N):
     assert torch.equal(m.linear_act(x, w, bias, 3), torch.relu(got.float() + bias).bfloat16())
 
 
-@pytest.mark.parametrize("M,K,inter", [(200, 11008, 2048), (150, 16384, 512), (300, 8192, 1000)])
+# the last two: sizes at which the plain linear's widths leave two CTAs a tile and the SwiGLU ending's would have taken a CTA pair, which adds k up in one chain
+@pytest.mark.parametrize("M,K,inter", [(200, 11008, 2048), (150, 16384, 512), (300, 8192, 1000), (257, 5120, 2376), (257, 16384, 2320)])
 def test_swiglu_sums_in_the_same_order(M, K, inter):
     gen = torch.Generator(device=DEV).manual_seed(M + K)
     x, w = rand(gen, M, K), rand(gen, 2 * inter, K, scale=K ** -0.5)
