@@ -481,7 +481,7 @@ static int launch_mma_t(const void *q, const void *k_pool, const void *v_pool, c
                         const int *tiles, int n_tiles, const int *block_table, int mpps, int heads, int kv_heads, float scale, int chunk,
                         cudaStream_t st) {
     const size_t smem = (size_t)(kTileQ + 4 * kPage) * D * sizeof(T);
-    cudaFuncSetAttribute(chunked_attn_mma_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(chunked_attn_mma_kernel<T, D>);
     launch_plain(chunked_attn_mma_kernel<T, D>, dim3(n_tiles, heads), dim3(128), smem, st, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink, (const T *)gate_in,
                                                                             gate_ld, (T *)out, (const int4 *)tiles, block_table, mpps, heads, kv_heads,
                                                                             scale, chunk);
@@ -537,7 +537,7 @@ int launch_chunked_attention(int dtype, const void *q, const void *k_pool, const
         return B200_ERR_UNSUPPORTED;
     }
     B200_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(chunked_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 48 * 1024) allow_smem(chunked_attn_kernel<T>);
         launch_plain(chunked_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, (const T *)q, (const T *)k_pool, (const T *)v_pool, sink,
                                                                             (const T *)gate_in, gate_ld, (T *)out, tok_seq, tok_pos,
                                                                             block_table, mpps, heads, kv_heads, dim, scale, chunk, max_keys, tok_list);

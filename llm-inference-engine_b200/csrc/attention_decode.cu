@@ -641,29 +641,21 @@ static int launch_decode_attn_t(DecodeAttnArgs a, cudaStream_t st) {
         const size_t smem = (size_t)kAttnStages * 2 * kAttnTileBytes + sizeof(float) * ((size_t)GC * kAttnD + 2 * kAttnD + (size_t)RG * GC + 2 * GC + 2) +
                             2 * kAttnStages * 8 + 16;
         dim3 grid(a.nsplit, a.kv_head_num * (G / GC), a.batch);
-        auto go = [&](auto kern, int slot) {
-            // the three instantiations share one function-pointer type: the opt-in to large dynamic shared memory is per kernel and device
-            static thread_local bool attr_set[6][64] = {{false}};
-            int dev = 0;
-            cudaGetDevice(&dev);
-            dev &= 63;
-            if (!attr_set[slot][dev]) {
-                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                attr_set[slot][dev] = true;
-            }
+        auto go = [&](auto kern) {
+            allow_smem(kern);
             launch_pdl(kern, grid, dim3(kAttnThreads), smem, st, true, a);
         };
         if (a.block_table) {
             switch (GC) {
-                case 1: go(decode_attn_kernel<T, 1, true>, 3); break;
-                case 2: go(decode_attn_kernel<T, 2, true>, 4); break;
-                default: go(decode_attn_kernel<T, 4, true>, 5); break;
+                case 1: go(decode_attn_kernel<T, 1, true>); break;
+                case 2: go(decode_attn_kernel<T, 2, true>); break;
+                default: go(decode_attn_kernel<T, 4, true>); break;
             }
         } else {
             switch (GC) {
-                case 1: go(decode_attn_kernel<T, 1, false>, 0); break;
-                case 2: go(decode_attn_kernel<T, 2, false>, 1); break;
-                default: go(decode_attn_kernel<T, 4, false>, 2); break;
+                case 1: go(decode_attn_kernel<T, 1, false>); break;
+                case 2: go(decode_attn_kernel<T, 2, false>); break;
+                default: go(decode_attn_kernel<T, 4, false>); break;
             }
         }
         return cuda_status("decode_attn launch");
@@ -674,7 +666,7 @@ static int launch_decode_attn_t(DecodeAttnArgs a, cudaStream_t st) {
         set_error("decode_mha: step %d too long for the generic head-size path", a.step);
         return B200_ERR_UNSUPPORTED;
     }
-    cudaFuncSetAttribute(decode_attn_generic_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(decode_attn_generic_kernel<T>);
     launch_pdl(decode_attn_generic_kernel<T>, dim3(a.head_num, a.batch), dim3(128), smem, st, true, a);
     return cuda_status("decode_attn_generic launch");
 }

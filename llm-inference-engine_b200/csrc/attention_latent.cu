@@ -689,7 +689,7 @@ int launch_latent_attention(int dtype, const void *ql, const void *qr, const voi
         return B200_ERR_UNSUPPORTED;
     }
     B200_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(latent_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 48 * 1024) allow_smem(latent_attn_kernel<T>);
         launch_plain(latent_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, (const T *)ql, (const T *)qr, (const T *)pool, sink, (T *)ol, tok_seq,
                                                                            tok_pos, block_table, mpps, t_pad, heads, kv_rank, rot_dim, scale,
                                                                            window, max_keys, (int)part, tok_list);
@@ -716,7 +716,7 @@ static int launch_latent_mma_t(const void *ql, const void *qr, const void *pool,
                                int splits, float *part, cudaStream_t st) {
     const int ld = (kv_rank + rot_dim + 63) / 64 * 64;
     const size_t smem = (size_t)3 * kLatTileQ * ld * sizeof(T);
-    cudaFuncSetAttribute(latent_attn_mma_kernel<T, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(latent_attn_mma_kernel<T, NV>);
     launch_plain(latent_attn_mma_kernel<T, NV>, dim3(grid), dim3(128), smem, st, (const T *)ql, (const T *)qr, (const T *)pool, sink, (T *)ol, (const int4 *)tiles,
                                                            block_table, mpps, t_pad, heads, kv_rank, rot_dim, ld, scale, window, by_head, splits,
                                                            splits > 1 ? part : nullptr);

@@ -591,7 +591,7 @@ static int launch_scored_mma_t(const void *q, const void *k_pool, const void *v_
     const int pen_len = (!sigmoid && r1) ? window + kTileQS : 0;
     const size_t smem = (size_t)(kTileQS + 2 * kPageS) * DK * sizeof(T) + (size_t)2 * kPageS * DV * sizeof(T) + (size_t)pen_len * sizeof(float);
     auto kern = sigmoid ? scored_attn_mma_kernel<T, DK, DV, 1> : scored_attn_mma_kernel<T, DK, DV, 0>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(kern);
     launch_plain(kern, dim3(n_tiles, heads), dim3(128), smem, st, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, r1, r2, (const T *)gate_in, gate_ld,
                                                   (T *)out, out_ld, out_scale, (const int4 *)tiles, block_table, mpps, heads, kv_heads, scale, window,
                                                   pen_len, opt);
@@ -665,7 +665,7 @@ int launch_scored_attention(int dtype, const void *q, const void *k_pool, const 
         return B200_ERR_UNSUPPORTED;
     }
     B200_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(scored_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 48 * 1024) allow_smem(scored_attn_kernel<T>);
         launch_plain(scored_attn_kernel<T>, dim3(tokens, heads), dim3(threads), smem, st, (const T *)q, (const T *)k_pool, (const T *)v_pool, head_bias, dist_r1, dist_r2, (const T *)gate_in, gate_ld, (T *)out, out_ld, out_scale,
             tok_seq, tok_pos, block_table, mpps, heads, kv_heads, dim, vdim, scale, window, sigmoid, max_keys, (int)part, tok_list, opt);
     });

@@ -302,7 +302,7 @@ token_attn_kernel(const TokenAttnArgs args) {
 
 template <typename T, int G> int launch_token_t(const TokenAttnArgs &args, const dim3 &grid, size_t smem, cudaStream_t st) {
     auto kern = token_attn_kernel<T, G>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(kern);
     launch_plain(kern, grid, dim3(kThreads), smem, st, args);
     return cuda_status("token_attention launch");
 }

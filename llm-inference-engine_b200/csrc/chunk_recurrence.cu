@@ -627,8 +627,8 @@ int launch_chunks_t(const ChunkSource &src, ChunkMap map, float *scratch, size_t
     const size_t scan_smem = Scan<DK, DELTA>::kFloats * sizeof(float);
     auto fk = chunk_factors_kernel<TQ, DK, DELTA>;
     auto sk = chunk_scan_kernel<TQ, DK, DELTA>;
-    cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f);
-    cudaFuncSetAttribute(sk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem);
+    allow_smem(fk);
+    allow_smem(sk);
     for (map.first = 0; map.first < chunks; map.first += map.count) {
         const int n = std::min(map.count, chunks - map.first);
         launch_plain(fk, dim3(n, map.heads, n_seqs), dim3(256), smem_f, st, src, map, scratch);

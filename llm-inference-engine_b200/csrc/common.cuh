@@ -24,6 +24,8 @@ int sm_count();
 // l1: the kernel's loads in flight live in L1: ask for the smallest shared memory that holds `per_sm` bytes, whatever the kernel in front had (a kernel that fits
 // is otherwise run beside the 28 KB of L1 that a launch of 200 KB left: 17 rows of a head, whose last row runs alone, 96 -> 120 us).
 bool allow_smem(const void *kernel, size_t most, size_t per_sm = 0);
+// for kernels whose sizes follow a call's: all that a CTA of this device may have beside the kernel's own static arrays
+template <typename... Args> bool allow_smem(void (*kernel)(Args...)) { return allow_smem(reinterpret_cast<const void *>(kernel), 0); }
 }  // namespace b200
 struct CUtensorMap_st;
 namespace b200 {

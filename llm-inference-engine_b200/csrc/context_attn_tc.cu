@@ -494,7 +494,7 @@ int launch_context_attention_tc(const void *q, const void *k_layer, const void *
     const size_t smem = (size_t)(2 + 2 * kKvStages) * kTileBytes + 1024 + 18 * 8 + 16 + 2 * kRows * 4 * sizeof(float);
     dim3 grid((max_q_len + kRows - 1) / kRows, head_num, batch);
     auto go = [&](auto kern) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(kern);
         launch_pdl(kern, grid, dim3(kThreads), smem, st, true, tmQ, tmK, tmV, p);
     };
     if (bf16) go(context_attn_tc_kernel<__nv_bfloat16>);

@@ -519,7 +519,7 @@ template <typename T, int RR, int TB>
 static void launch_gla_reg(const void *proj, int ld, const float *decay, float *state, float *o, const int *seq_start, const int *seq_pos0,
                            const int *seq_slot, dim3 grid, int heads, int dim, int vdim, int min_tokens, int max_tokens, cudaStream_t st) {
     const size_t smem = 2 * ((size_t)TB * 32 * RR * 4 + (size_t)TB * kGlaCols) * sizeof(float);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(gla_recurrent_reg_kernel<T, RR, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(gla_recurrent_reg_kernel<T, RR, TB>);
     launch_plain(gla_recurrent_reg_kernel<T, RR, TB>, dim3(grid), dim3(256), smem, st, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim, min_tokens, max_tokens);
 }
 
@@ -639,7 +639,7 @@ int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay
         const size_t smem_step = (4 * (size_t)dim + kStepRowGroups * kStepCols) * sizeof(float);
         const dim3 grid_step((vdim + kStepCols - 1) / kStepCols, heads, n_seqs);
         B200_DISPATCH_DTYPE(dtype, {
-            if (smem_step > 48 * 1024) cudaFuncSetAttribute(gla_step_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_step);
+            if (smem_step > 48 * 1024) allow_smem(gla_step_kernel<T>);
             launch_plain(gla_step_kernel<T>, dim3(grid_step), dim3(256), smem_step, st, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim, vdim);
         });
         if (!(kinds & kGlaManyTokens)) return cuda_status("gla_step launch");
@@ -661,7 +661,7 @@ int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay
         return cuda_status("gla_recurrent launch");
     }
     B200_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(gla_recurrent_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 48 * 1024) allow_smem(gla_recurrent_kernel<T>);
         launch_plain(gla_recurrent_kernel<T>, dim3(grid), dim3(kGlaThreads), smem, st, (const T *)proj, ld, decay, state, o, seq_start, seq_pos0, seq_slot, heads, dim,
                                                                   vdim, min_tokens, max_tokens);
     });

@@ -512,7 +512,7 @@ static void launch_proj_f32_t(const void *x, int ldx, const void *w, const float
     const int mt = (M + PM - 1) / PM;
     int cols = (N * mt + 4 * 148 - 1) / (4 * 148);
     cols = cols < 8 ? 8 : (cols + 7) / 8 * 8;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(proj_f32_kernel<TX, TW, PM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(proj_f32_kernel<TX, TW, PM>);
     launch_plain(proj_f32_kernel<TX, TW, PM>, dim3((N + cols - 1) / cols, mt), dim3(256), smem, st, (const TX *)x, ldx, (const TW *)w, bias, y, ldy, M, N, K, cols);
 }
 

@@ -406,7 +406,7 @@ int b200_linear(const void *x, const void *w, const void *scales, const void *ze
             B200_DISPATCH_DTYPE(dtype, {
                 auto run = [&](auto mb) {
                     constexpr int kMB = decltype(mb)::value;
-                    cudaFuncSetAttribute(gemv_kn_kernel<T, kMB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                    allow_smem(gemv_kn_kernel<T, kMB>);
                     launch_pdl(gemv_kn_kernel<T, kMB>, dim3(tiles, ksplit), dim3(kKnWarps * 32), smem, st, true, (const T *)w,
                                (const T *)x, (T *)y, partial, ws.tickets, M, K, N, ksplit);
                 };

@@ -804,10 +804,10 @@ int launch_dense_f32out(int dtype, const void *x, const void *w, float *y, int M
     const dim3 grid((N + kMN - 1) / kMN, (M + kMoeTileM - 1) / kMoeTileM);
     const size_t smem = (size_t)kMStages * (kMoeTileM + kMN) * kMK * 2;
     if (dtype == B200_BF16) {
-        cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__nv_bfloat16, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(moe_grouped_gemm_mma_kernel<__nv_bfloat16, float>);
         launch_plain(moe_grouped_gemm_mma_kernel<__nv_bfloat16, float>, dim3(grid), dim3(128), smem, st, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, y, nullptr, nullptr, M, N, K, -1);
     } else {
-        cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__half, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(moe_grouped_gemm_mma_kernel<__half, float>);
         launch_plain(moe_grouped_gemm_mma_kernel<__half, float>, dim3(grid), dim3(128), smem, st, (const __half *)x, (const __half *)w, y, nullptr, nullptr, M, N, K, -1);
     }
     return cuda_status("dense_f32out launch");
@@ -868,7 +868,7 @@ int launch_moe_plan(const int *sel_expert, const float *sel_weight, int *row_tok
     const int pairs = tokens * top;
     const int warps = std::max(1, std::min({32, std::max(8, (pairs + 31) / 32), (int)(40 * 1024 / sizeof(int) / std::max(experts, 1))}));
     const size_t smem = ((size_t)(warps + 2) * experts + 1) * sizeof(int);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(moe_plan_kernel);
     launch_plain(moe_plan_kernel, dim3(1), dim3(warps * 32), smem, st, sel_expert, sel_weight, row_token, row_weight, tile_expert, pair_row, n_tiles, pairs, experts, top, tile);
     return cuda_status("moe_plan launch");
 }
@@ -932,11 +932,11 @@ int launch_moe_grouped_gemm(int dtype, const void *a, const void *w, void *c, co
         const dim3 grid((N + kMN - 1) / kMN, max_tiles);
         const size_t smem = (size_t)kMStages * (kMoeTileM + kMN) * kMK * 2;
         if (dtype == B200_BF16) {
-            cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__nv_bfloat16, __nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_smem(moe_grouped_gemm_mma_kernel<__nv_bfloat16, __nv_bfloat16>);
             launch_plain(moe_grouped_gemm_mma_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(grid), dim3(128), smem, st, (const __nv_bfloat16 *)a, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)c,
                                                                                                tile_expert, n_tiles, max_tiles * kMoeTileM, N, K, act);
         } else {
-            cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<__half, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_smem(moe_grouped_gemm_mma_kernel<__half, __half>);
             launch_plain(moe_grouped_gemm_mma_kernel<__half, __half>, dim3(grid), dim3(128), smem, st, (const __half *)a, (const __half *)w, (__half *)c, tile_expert, n_tiles,
                                                                                  max_tiles * kMoeTileM, N, K, act);
         }

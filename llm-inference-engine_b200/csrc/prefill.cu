@@ -507,7 +507,7 @@ static int context_attention_impl(const void *q, const void *k_cache, const void
     }
     dim3 grid((max_q_len + kCaRows - 1) / kCaRows, head_num, batch);
     B200_DISPATCH_DTYPE(dtype, {
-        cudaFuncSetAttribute(context_attention_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(context_attention_kernel<T>);
         launch_pdl(context_attention_kernel<T>, grid, dim3(kCaThreads), smem, st, true, (const T *)q,
                    (const T *)((const char *)k_cache + loff), (const T *)((const char *)v_cache + loff), (T *)out, (const int *)nullptr,
                    (const int *)seq_off, input_len, context_len, head_num, kv_head_num, max_q_len, max_seq_len, head_size, scale);

@@ -783,7 +783,7 @@ static int launch_colrec_t(const float *rec, int rec_ld, int q_off, int k_off, i
     constexpr int NV = MODE == 0 ? 3 : 2;
     const size_t smem = ((size_t)2 * kRecTB * (NV * DP + 4) + (size_t)2 * kRecTB * cb) * sizeof(float);
     auto kern = column_recurrence_kernel<DP, LANES, CPT, MODE>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(kern);
     launch_plain(kern, dim3((ncols + cb - 1) / cb, heads, n_seqs), dim3(block), smem, st, rec, rec_ld, q_off, k_off, v_off, a_off, b_off, S, n_state, m_state, o, nq, m_out,
                                                                         seq_start, seq_pos0, seq_slot, heads, kv_heads, dim, vdim, max_tokens);
     return cuda_status("column_recurrence launch");
@@ -857,7 +857,7 @@ int launch_delta_prep(int dtype, const void *proj, int ld, int col0, const float
         launch_plain(delta_prep_tile_kernel<__half>, dim3(tile_grid), dim3(256), 0, st, (const __half *)proj, ld, col0, conv_w, conv_state, rank, gate_rank, (__half *)lr_a, (__half *)lr_g, rec, lay,
                                                                   tok_seq, tok_pos, seq_pos0, seq_slot, tokens, heads, kv_heads, dim, vdim, per);
     else B200_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 48 * 1024) allow_smem(delta_prep_kernel<T>);
         // few tokens: few CTAs, so each gets more threads (a thread's channels are a chain of load latencies)
         launch_plain(delta_prep_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), smem, st, (const T *)proj, ld, col0, conv_w, taps, conv_state, rank, gate_rank, (T *)lr_a, (T *)lr_g, rec, lay,
                                                        tok_seq, tok_pos, seq_pos0, seq_slot, heads, kv_heads, dim, vdim);
@@ -930,7 +930,7 @@ int launch_delta_prep_direct(int dtype, const void *proj, int ld, int col0, cons
     const DeltaRow lay = delta_row(heads, kv_heads, dim, vdim);
     const size_t smem = ((size_t)2 * kv_heads * dim + heads * vdim) * sizeof(float);
     B200_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_direct_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 48 * 1024) allow_smem(delta_prep_direct_kernel<T>);
         launch_plain(delta_prep_direct_kernel<T>, dim3(tokens), dim3(tokens <= 64 ? 1024 : 256), smem, st, (const T *)proj, ld, col0, conv_w, taps, conv_state, decay_bias, a_log, rec,
                                                                                    lay, tok_seq, tok_pos, seq_pos0, seq_slot, heads, kv_heads, dim, vdim);
     });

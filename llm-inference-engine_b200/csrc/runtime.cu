@@ -102,6 +102,12 @@ bool allow_smem(const void *kernel, size_t most, size_t per_sm) {
     if (seen[dev].count(kernel)) return true;
     std::lock_guard<std::mutex> lk(mu);
     if (!raised[dev].count(kernel)) {
+        if (most == 0) {
+            int all = 0;
+            cudaFuncAttributes own;
+            if (cudaDeviceGetAttribute(&all, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess || cudaFuncGetAttributes(&own, kernel) != cudaSuccess) return false;
+            most = (size_t)all - own.sharedSizeBytes;
+        }
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return false;
         if (per_sm > 0 && cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)std::min<size_t>(100, (per_sm * 100 + (228 << 10) - 1) / (228 << 10))) != cudaSuccess) return false;
         raised[dev].insert(kernel);
