@@ -875,7 +875,7 @@ struct b200_hybrid {
     size_t chunk_floats = 0;
     int *meta = nullptr, *moe_i = nullptr;
     float *moe_f = nullptr;
-    float *tpart = nullptr;  // decoded tokens' key shares (attention_token.cu)
+    float *tpart = nullptr;  // sums of decoded tokens' blocks of keys (attention_token.cu)
     std::vector<int> host_meta;
 };
 
@@ -955,7 +955,7 @@ Carve carve(const b200_hybrid *m) {
                 n_chunk = std::max(n_chunk, chunk_scratch_floats(mx->heads, mx->dim, mx->mixer == B200_MIXER_DELTA, c.max_tokens, c.max_seqs));
         for (const b200_hybrid_layer_t *mx : {&l, l.side})
             if (mx && c.dtype != B200_F32 && (mx->mixer == B200_MIXER_ATTN_CHUNKED || mx->mixer == B200_MIXER_ATTN_SCORED))
-                n_tpart = std::max(n_tpart, token_attention_part_floats(mx->mixer == B200_MIXER_ATTN_CHUNKED ? mx->dim : mx->vdim));
+                n_tpart = std::max(n_tpart, token_attention_part_floats(mx->heads, mx->kv_heads, mx->mixer == B200_MIXER_ATTN_CHUNKED ? mx->dim : mx->vdim));
         n_mix = std::max(n_mix, (size_t)l.heads * std::max(l.dim, l.vdim));
         n_f32 = std::max(n_f32, (size_t)l.heads * std::max(l.dim, l.vdim));
         n_mix = std::max(n_mix, (size_t)l.heads * l.vdim);
@@ -1012,9 +1012,9 @@ Carve carve(const b200_hybrid *m) {
     //       | chunks of the minGRU mixer [4 * (T/64 + S)]
     //       | one-token tiles of the short portions [4 * T] | latent mixers: head of every row tile of 64 and of 128 [heads * t_pad / 64,
     //         heads * t_pad / 128] | live row tiles per layer, of 64 and of 128 [layers each]
-    //       | arrivals of the decoded tokens' key shares [kTokenShareCtas], zeros
+    //       | arrivals of the decoded tokens' runs of keys [kTokenTickets], zeros
     k.meta = align256((8 * (T / 64 + (size_t)c.max_seqs + 1) + 5 * T + 3 * (size_t)c.max_seqs + 1 + (size_t)c.max_seqs * c.max_pages_per_seq +
-                       4 * T + 2 * lheads * (t_pad / 64) + 2 * (size_t)c.num_layers + kTokenShareCtas) * 4);
+                       4 * T + 2 * lheads * (t_pad / 64) + 2 * (size_t)c.num_layers + kTokenTickets) * 4);
     // moe ints: sel_expert | pair_row [T*top each] | row_token [rows] | tile_expert [rows / tile] | n_tiles
     k.moe_i = align256((2 * T * top + rows + rows / 32 + 4) * 4);
     // moe floats: sel_weight [T*top] | row_weight [rows] | shared_gate [T]
@@ -1398,9 +1398,16 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     const int t_pad = lat_tc ? (NT + 127) / 128 * 128 : (NT + kMoeTileM - 1) / kMoeTileM * kMoeTileM;
     const int tph = t_pad / kMoeTileM, tph128 = lat_tc ? t_pad / 128 : 0;
     bool any_mingru = false;
-    for (int i = 0; i < c.num_layers; ++i) any_mingru |= m->layers[i].mixer == B200_MIXER_MINGRU;
+    size_t n_tickets = 0;
+    for (int i = 0; i < c.num_layers; ++i) {
+        const b200_hybrid_layer_t &l = m->layers[i];
+        any_mingru |= l.mixer == B200_MIXER_MINGRU;
+        for (const b200_hybrid_layer_t *mx : {&l, l.side})
+            if (mx && (mx->mixer == B200_MIXER_ATTN_CHUNKED || mx->mixer == B200_MIXER_ATTN_SCORED))
+                n_tickets = std::max(n_tickets, std::min((size_t)NT * mx->heads, (size_t)kTokenTickets));
+    }
     const size_t n_tile_ints = 4 * ((size_t)NT / 64 + S + 1), n_chunk_ints = any_mingru ? n_tile_ints : 0, n_stile_ints = (size_t)4 * NT;
-    hm.assign(n_tile_ints + n_chunk_ints + n_stile_ints + (size_t)5 * NT + 3 * S + 1 + (size_t)S * mpps + (size_t)lat_heads * (tph + tph128) + 2 * c.num_layers + kTokenShareCtas, 0);
+    hm.assign(n_tile_ints + n_chunk_ints + n_stile_ints + (size_t)5 * NT + 3 * S + 1 + (size_t)S * mpps + (size_t)lat_heads * (tph + tph128) + 2 * c.num_layers + n_tickets, 0);
     int *h_tiles = hm.data(), *h_chunks = h_tiles + n_tile_ints, *h_stiles = h_chunks + n_chunk_ints, *h_ids = h_stiles + n_stile_ints, *h_seq = h_ids + NT, *h_pos = h_seq + NT,
         *h_want = h_pos + NT, *h_short = h_want + NT, *h_start = h_short + NT, *h_pos0 = h_start + S + 1, *h_slot = h_pos0 + S, *h_bt = h_slot + S,
         *h_lat_head = h_bt + (size_t)S * mpps, *h_lat_head128 = h_lat_head + (size_t)lat_heads * tph,
@@ -1414,7 +1421,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     // prompt portions go to the tensor-core attention in tiles of <= 64 consecutive tokens, short ones (decoded tokens) to the per-token kernel
     constexpr int kShortPortion = 8;
     static_assert(kShortPortion == kMingruShort, "one list of short portions serves both");
-    int n_tiles = 0, n_short = 0, n_chunks = 0, gla_kinds = 0, last_short = 0;
+    int n_tiles = 0, n_short = 0, n_chunks = 0, gla_kinds = 0;
     // minGRU chunks: at most 64 per portion (a chunk composes the maps of all chunks before it), of whole multiples of kMingruChunk tokens
     int longest = 0, long_tokens = 0;  // long_tokens: of the portions that the token-parallel recurrences can take
     bool mid_portions = false;  // portions of several tokens that the token-parallel recurrences leave to the serial ones
@@ -1440,7 +1447,6 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                 int *tl = h_stiles + 4 * n_short;
                 tl[0] = s, tl[1] = t, tl[2] = 1, tl[3] = h_pos[t];
                 h_short[n_short++] = t;
-                last_short = std::max(last_short, h_pos[t]);
             }
         } else {
             for (int t = t0; t < t1; t += 64, ++n_tiles) {
@@ -1472,7 +1478,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
               *d_want = d_pos + NT, *d_short = d_want + NT, *d_start = d_short + NT, *d_pos0 = d_start + S + 1, *d_slot = d_pos0 + S, *d_bt = d_slot + S,
               *d_lat_head = d_bt + (size_t)S * mpps, *d_lat_head128 = d_lat_head + (size_t)lat_heads * tph,
               *d_lat_n = d_lat_head128 + (size_t)lat_heads * tph128, *d_lat_n128 = d_lat_n + c.num_layers;
-    unsigned int *const tickets = (unsigned int *)(m->meta + hm.size() - kTokenShareCtas);
+    unsigned int *const tickets = (unsigned int *)(m->meta + hm.size() - n_tickets);
 
     const int dt = c.dtype, width = c.width;
     const bool f32 = dt == B200_F32;
@@ -1566,13 +1572,12 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                                    l.kv_heads, l.dim, l.vdim, l.rot_dims, l.rot_base, st, opt, share));
             int max_keys = l.window > 0 ? std::min(l.window, mpps * kPageH) : mpps * kPageH;
             if (l.chunk > 0) max_keys = std::min(max_keys, l.chunk);
-            const int seen = std::min(max_keys, last_short + 1);  // keys of a decoded token, at most
-            TokenAttn ta{m->mix, kp, vp, l.head_bias, l.dist_r1, l.dist_r2, l.dist_slope, l.sink, gate, n_in, out, out_ld, out_scale, l.scale, l.softcap, (const int4 *)d_stiles, d_bt, mpps,
+            TokenAttn ta{m->mix, kp, vp, l.head_bias, l.dist_r1, l.dist_r2, l.dist_slope, l.sink, gate, n_in, out, out_ld, out_scale, l.scale, l.softcap, (const int4 *)d_stiles, (const int4 *)h_stiles, d_bt, mpps,
                          l.heads, l.kv_heads, l.dim, l.vdim, l.window, l.chunk, sig, m->tpart, tickets};
             if (scored_attention_tiles_supported(dt, l.dim, l.vdim, n_in, out_ld, l.window, l.dist_r1 != nullptr)) {
                 RUN(launch_scored_attention_tiles(dt, m->mix, kp, vp, l.head_bias, l.dist_r1, l.dist_r2, gate, n_in, out, out_ld, out_scale, d_tiles, n_tiles,
                                                   d_bt, mpps, l.heads, l.kv_heads, l.dim, l.vdim, l.scale, l.window, sig, st, so));
-                rc = launch_token_attention(dt, ta, n_short, seen, st);
+                rc = launch_token_attention(dt, ta, n_short, st);
                 if (rc == B200_ERR_UNSUPPORTED)
                     rc = launch_scored_attention(dt, m->mix, kp, vp, l.head_bias, l.dist_r1, l.dist_r2, gate, n_in, out, out_ld, out_scale, d_seq, d_pos, d_bt,
                                                  mpps, n_short, l.heads, l.kv_heads, l.dim, l.vdim, l.scale, l.window, sig, max_keys, st, d_short, so);
@@ -1821,9 +1826,9 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                                                    n_tiles, d_bt, mpps, l.heads, l.kv_heads, l.dim, l.scale, l.chunk, st));
                 TokenAttn ta{m->mix, m->kv_pool + lp.k_off, m->kv_pool + lp.v_off};
                 ta.sink = l.sink, ta.gate = gate, ta.gate_ld = lp.n_in, ta.out = m->mix2, ta.out_ld = hd, ta.scale = l.scale;
-                ta.tokens = (const int4 *)d_stiles, ta.block_table = d_bt, ta.mpps = mpps;
+                ta.tokens = (const int4 *)d_stiles, ta.listed = (const int4 *)h_stiles, ta.block_table = d_bt, ta.mpps = mpps;
                 ta.heads = l.heads, ta.kv_heads = l.kv_heads, ta.dim = ta.vdim = l.dim, ta.chunk = l.chunk, ta.part = m->tpart, ta.tickets = tickets;
-                rc = launch_token_attention(dt, ta, n_short, std::min(max_keys, last_short + 1), st);
+                rc = launch_token_attention(dt, ta, n_short, st);
                 if (rc == B200_ERR_UNSUPPORTED)
                     rc = launch_chunked_attention(dt, m->mix, m->kv_pool + lp.k_off, m->kv_pool + lp.v_off, l.sink, gate, lp.n_in, m->mix2, d_seq, d_pos,
                                                   d_bt, mpps, n_short, l.heads, l.kv_heads, l.dim, l.scale, l.chunk, max_keys, st, d_short);

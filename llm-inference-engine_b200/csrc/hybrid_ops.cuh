@@ -46,14 +46,16 @@ struct TokenAttn {
     int out_ld = 0;
     float out_scale = 1.0f, scale = 1.0f, softcap = 0.0f;
     const int4 *tokens = nullptr;     // {sequence, row, 1, position} of every token to do
+    const int4 *listed = nullptr;     // the same list on the host
     const int *block_table = nullptr;
     int mpps = 0, heads = 0, kv_heads = 0, dim = 0, vdim = 0, window = 0, chunk = 0, sigmoid = 0;
     float *part = nullptr;            // scratch of token_attention_part_floats
-    unsigned int *tickets = nullptr;  // [kTokenShareCtas], zero, and zero again afterwards
+    unsigned int *tickets = nullptr;  // one per token and block of query heads, kTokenTickets at most: zero, and zero again afterwards
 };
-constexpr int kMaxTokenShares = 16, kTokenShareCtas = 296;
-size_t token_attention_part_floats(int vdim);
-int launch_token_attention(int dtype, const TokenAttn &a, int tokens, int max_keys, cudaStream_t st);
+constexpr int kTokenCtas = 2 * 148;                                // CTAs that the blocks of a launch's tokens are shared out to
+constexpr int kTokenParts = 16 * 148, kTokenTickets = kTokenParts / 2;  // blocks whose sums the scratch holds; tokens x head blocks of more than one
+size_t token_attention_part_floats(int heads, int kv_heads, int vdim);
+int launch_token_attention(int dtype, const TokenAttn &a, int tokens, cudaStream_t st);
 
 // attention_latent.cu
 // other rotations than pairs (i, i + rot_dims/2) by pos * rot_base^(-2i/rot_dims): pairs: (2i, 2i+1); turns: DEVICE [rot_dims/2] turns per

@@ -1,6 +1,6 @@
 """Attention of decoded tokens by key head (csrc/attention_token.cu) against the float64 restatements: query heads per key head on both sides of every block of
-heads (1, 2, 3, 4, 5, 8, 9), head sizes of 64, 128 and 256, contexts of one key, of a share's edge (31, 32, 33), of a page's (63, 64, 65) and of more shares than
-one; batches whose tokens share out their keys beside batches that do not; portions of several decoded tokens; windows, blocks, a sink, distance penalties and
+heads (1, 2, 3, 4, 5, 8, 9), head sizes of 64 and 128 (256 keeps the per-token kernel), contexts of one key, of a page's edge (63, 64, 65), and of more blocks of keys
+than one; batches whose tokens share out their keys beside batches that do not; portions of several decoded tokens; windows, blocks, a sink, distance penalties and
 un-normalised weights."""
 import importlib
 
@@ -74,3 +74,35 @@ def test_unnormalised_weights(dtype, heads, kv, dim, vdim):
     config = fedovik_oracle.make_config([fedovik_oracle.attention_layer(heads=heads, kv_heads=kv, dim=dim, vdim=vdim)], width=64)
     run("fedovik", fedovik_oracle, config, dtype, EDGES, 5, 10)
     run("fedovik", fedovik_oracle, config, dtype, [400], 4, 1)
+
+
+@pytest.mark.parametrize("design,heads,kv,dim,size,contexts", [
+    ("vasolix", 16, 4, 128, 8192, [1, 100, 126, 127, 128, 254, 255, 256, 300, 511, 700, 1000, 1500, 2500, 4094, 4200]),  # one block of keys to 32, and longer ones
+    ("vasolix", 16, 2, 128, 1000, [40, 990, 1010, 2400]),  # blocks of positions
+    ("fedovik", 16, 4, 128, 0, [5, 300, 599, 601, 1200, 3000]),  # un-normalised weights
+    ("vasolix", 32, 16, 64, 4096, [2300 + 7 * i for i in range(16)])])  # more blocks than a launch's scratch holds
+def test_a_token_by_itself(design, heads, kv, dim, size, contexts):
+    """The keys of a decoded token are cut by its own context: its row has the same bits by itself, where its blocks of keys are shared out over the device, and in a
+    batch of up to sixteen, the range in which the linears around it have."""
+    if design == "vasolix":
+        ref, config = vasolix_oracle, vasolix_oracle.make_config([vasolix_oracle.attention_layer(heads=heads, kv_heads=kv, dim=dim, size=size, scale=dim ** -0.5)], width=128)
+    else:
+        ref, config = fedovik_oracle, fedovik_oracle.make_config([fedovik_oracle.attention_layer(heads=heads, kv_heads=kv, dim=dim, vdim=dim)], width=128)
+    _, packed = ref.make_weights(config, seed=9)
+    model = getattr(importlib.import_module("llm-inference-engine_b200.models." + design), design.capitalize() + "Model")(
+        config, packed, dtype="float16", device="cuda:0", max_tokens=2048, max_seqs=len(contexts), max_pages_per_seq=80)
+    serving = importlib.import_module("llm-inference-engine_b200.serving")
+    toks = [np.random.default_rng(i).integers(0, config["vocab"], n + 3).tolist() for i, n in enumerate(contexts)]
+    rows = {}
+    for how in ("alone", "together"):
+        sess = serving.Session(model, sum(n + 67 for n in contexts), max_seqs=len(contexts), max_batch_tokens=2048, poison=True)
+        ids = [sess.open() for _ in contexts]
+        for i, n in enumerate(contexts):
+            for a in range(0, n, 2000):
+                sess.feed([(ids[i], toks[i][a:min(a + 2000, n)], [])])
+        for k in range(3):
+            entries = [(ids[i], toks[i][n + k:n + k + 1], [0]) for i, n in enumerate(contexts)]
+            rows[how, k] = torch.cat([sess.feed([e]) for e in entries]) if how == "alone" else sess.feed(entries)
+    for k in range(3):
+        same = (rows["alone", k] == rows["together", k]).all(dim=-1)
+        assert same.all(), [contexts[i] for i in range(len(contexts)) if not same[i]]
