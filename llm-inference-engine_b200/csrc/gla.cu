@@ -419,12 +419,13 @@ gla_step_kernel(const T *__restrict__ proj, int ld, const float *__restrict__ de
     }
 }
 
-// A decode batch's whole mixer between its projections in one launch, a CTA per (head, sequence): the decays of the head's channels (four lanes a channel), the step
+// The whole mixer of decoded tokens between its projections in one launch, a CTA per (head, sequence of one token): the decays of the head's channels (four lanes a channel), the step
 // over the state as above, and the head's norm and gate.  What bounds it: round trips.  As three launches the step of 16 requests x 8 heads (dim 128, vdim 256) was
 // 4.1 us of decays, 8.3 of state and 2.7 of norm, 6 us of launches between them; here the state's rows are on their way while the decays are formed.
 // Measured there (three launches and the gaps between them -> one): 21 -> 10 us.
 // Four columns a thread, 16 row groups: vdim * 4 threads.
 constexpr int kDecodeVdim = 256;
+inline size_t gla_decode_smem(int dim, int vdim, int rank) { return (4 * (size_t)dim + (size_t)kStepRowGroups * vdim + rank) * sizeof(float); }
 template <typename T>
 __global__ void __launch_bounds__(4 * kDecodeVdim, 1)
 gla_decode_kernel(const T *__restrict__ proj, int ld, int rank_col, const T *__restrict__ w_decay, const float *__restrict__ bias, float inv_tau, int rank,
@@ -433,7 +434,7 @@ gla_decode_kernel(const T *__restrict__ proj, int ld, int rank_col, const T *__r
     extern __shared__ __align__(16) float smf[];  // {a, k, q, -}[dim] | part[kStepRowGroups][vdim] | the token's low-rank vector [rank]
     __shared__ float red[32];
     const int h = blockIdx.x, s = blockIdx.y, t = seq_start[s], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (seq_start[s + 1] - t != 1) return;  // (a sequence without a token)
+    if (seq_start[s + 1] - t != 1) return;  // (a prompt, or a sequence without a token)
     float4 *akq = reinterpret_cast<float4 *>(smf);
     float *part = smf + 4 * (size_t)dim, *lo = part + kStepRowGroups * vdim;
     const T *row = proj + (size_t)t * ld;
@@ -610,15 +611,19 @@ int launch_gla_decay(int dtype, const void *proj, int ld, int col0, const void *
     return cuda_status("gla_decay launch");
 }
 
-// B200_ERR_UNSUPPORTED (nothing launched): fp32, sizes that its threads do not share evenly, rows off their 16-byte boundaries.  Every sequence has one token.
+// Not fp32, sizes that its threads share evenly, rows on 16-byte boundaries.  Neither the batch nor what else is in it counts: a decoded token's sums are the same
+// beside a prompt.
+bool gla_decode_takes(int dtype, const void *proj, int ld, const void *w_decay, int rank, const float *state, int n_seqs, int dim, int vdim) {
+    return dtype != B200_F32 && vdim % 32 == 0 && vdim <= kDecodeVdim && rank % 8 == 0 && rank >= 8 && rank <= 4 * vdim && dim % 4 == 0 && dim <= 1024 && ld % 8 == 0 && n_seqs <= 65535 &&
+           gla_decode_smem(dim, vdim, rank) <= 48 * 1024 && all_aligned16({proj, w_decay, state});
+}
+
+// the sequences that bring one token; sizes that gla_decode_takes
 int launch_gla_decode(int dtype, const void *proj, int ld, int rank_col, const void *w_decay, const float *bias, float tau, int rank, float *state, const int *seq_start,
                       const int *seq_pos0, const int *seq_slot, int n_seqs, int heads, int dim, int vdim, const float *norm, float eps, int gate_col, void *out,
                       cudaStream_t st) {
     if (n_seqs == 0) return B200_OK;
-    const size_t smem = (4 * (size_t)dim + (size_t)kStepRowGroups * vdim + rank) * sizeof(float);
-    if (dtype == B200_F32 || vdim % 32 != 0 || vdim > kDecodeVdim || rank % 8 != 0 || rank < 8 || rank > 4 * vdim || dim % 4 != 0 || dim > 1024 || ld % 8 != 0 || n_seqs > 65535 ||
-        smem > 48 * 1024 || !all_aligned16({proj, w_decay, state}))
-        return B200_ERR_UNSUPPORTED;
+    const size_t smem = gla_decode_smem(dim, vdim, rank);
     auto go = [&](auto kern, auto *to) {
         using T = std::remove_pointer_t<decltype(to)>;
         launch_plain(kern, dim3(heads, n_seqs), dim3(4 * vdim), smem, st, (const T *)proj, ld, rank_col, (const T *)w_decay, bias, 1.0f / tau, rank, state, seq_start, seq_pos0, seq_slot,
@@ -644,7 +649,7 @@ int launch_gla_recurrent(int dtype, const void *proj, int ld, const float *decay
         });
         if (!(kinds & kGlaManyTokens)) return cuda_status("gla_step launch");
     }
-    const int min_tokens = step ? 2 : 1;
+    const int min_tokens = step || !(kinds & kGlaOneToken) ? 2 : 1;
     const size_t smem = ((size_t)dim * kGlaCols + 3 * (size_t)dim + kGlaCols + (kGlaThreads / kGlaCols) * kGlaCols) * sizeof(float);
     if (smem > 200 * 1024) {
         set_error("gla_recurrent: key size %d does not fit the shared-memory state tile", dim);

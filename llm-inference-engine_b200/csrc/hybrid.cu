@@ -6,7 +6,7 @@
 // the fp32 residual stream.  Launch sequence per layer:
 //   fused input projection (b200_linear: tcgen05 GEMM / weight-streaming GEMV by token count)
 //   attention mixer:  q/k whole-projection norm + pool append -> chunked sink attention (gate fused) -> output projection
-//   gla mixer:        decay (low-rank, fp32) -> recurrence over the state slots -> head norm * silu(gate), one launch for a decode batch -> output projection
+//   gla mixer:        decay (low-rank, fp32) -> recurrence over the state slots -> head norm * silu(gate), one launch for decoded tokens -> output projection
 //   latent mixer:     split + rotation + latent-row norm + pool append -> grouped GEMM over the heads (q into the latent space) -> windowed
 //                     sink attention over the latent rows -> grouped GEMM over the heads (value up-projection) -> gate -> output projection
 //   post-norm + residual add (fp32)
@@ -1533,8 +1533,8 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     }
 
     // a recurrence over the batch: its token-parallel form for the long portions, where it takes the layer's sizes and is the faster one, and the serial form for the rest
-    auto recurrence = [&](const b200_hybrid_layer_t &l, auto chunked, auto serial) -> int {
-        int kinds = gla_kinds, max_tokens = kAnyTokens;
+    auto recurrence = [&](const b200_hybrid_layer_t &l, int kinds, auto chunked, auto serial) -> int {
+        int max_tokens = kAnyTokens;
         if (chunk_pays(l.mixer == B200_MIXER_GLA, l.heads, l.vdim, longest, long_tokens, sm_count())) {
             rc = chunked();
             if (rc != B200_OK && rc != B200_ERR_UNSUPPORTED) return rc;
@@ -1547,7 +1547,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     };
     auto decay_recurrence = [&](const b200_hybrid_layer_t &l, const MixerPlan &mp, int key_heads) -> int {
         float *state = (float *)(m->state_pool + mp.state_off);
-        return recurrence(l, [&] { return launch_chunk_decay(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, key_heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
+        return recurrence(l, gla_kinds, [&] { return launch_chunk_decay(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, key_heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
                           [&](int, int most) { return launch_decay_recurrent(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, key_heads, l.dim, l.vdim, st, gla_kinds == kGlaOneToken, most); });
     };
 
@@ -1597,7 +1597,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
                                              NT, l.heads, l.kv_heads, l.dim, l.vdim, st));
             RUN(launch_conv_state_update(dt, m->proj, n_in, col, conv_state, l.conv, conv_channels(l), d_start, d_pos0, d_slot, S, st));
             float *state = (float *)(m->state_pool + mp.state_off);
-            RUN(recurrence(l, [&] { return launch_chunk_delta(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.kv_heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
+            RUN(recurrence(l, gla_kinds, [&] { return launch_chunk_delta(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.kv_heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
                            [&](int, int most) { return launch_delta_recurrent(m->rec, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.kv_heads, l.dim, l.vdim, st, one_token, most); }));
             if (l.decay_rank > 0) {
                 RUN(launch_head_output(dt, m->f32b, nullptr, nullptr, l.out_norm, 0, c.norm_eps, m->rec + lay.gate, lay.ld, nullptr, 0, out, out_ld, out_scale,
@@ -1893,16 +1893,18 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
             const int hd = l.heads * l.dim, hv = l.heads * l.vdim;
             const char *gate = (const char *)m->proj + (size_t)(2 * hd + hv) * es;
             float *state = (float *)(m->state_pool + lp.state_off);
-            rc = gla_kinds != kGlaOneToken ? B200_ERR_UNSUPPORTED
-                                           : launch_gla_decode(dt, m->proj, lp.n_in, 2 * hd + 2 * hv, l.w_decay, l.decay_bias, l.tau, l.decay_rank, state, d_start, d_pos0, d_slot, S, l.heads,
-                                                               l.dim, l.vdim, l.out_norm, c.norm_eps, 2 * hd + hv, m->mix2, st);
-            if (rc != B200_OK && rc != B200_ERR_UNSUPPORTED) return rc;
-            if (rc == B200_ERR_UNSUPPORTED) {
+            // decoded tokens in one launch, behind the others' (which leave rows of nothing in its place)
+            const bool ones = (gla_kinds & kGlaOneToken) && gla_decode_takes(dt, m->proj, lp.n_in, l.w_decay, l.decay_rank, state, S, l.dim, l.vdim);
+            const int rest = ones ? gla_kinds & ~kGlaOneToken : gla_kinds;
+            if (rest) {
                 RUN(launch_gla_decay(dt, m->proj, lp.n_in, 2 * hd + 2 * hv, l.w_decay, l.decay_bias, l.tau, m->f32a, NT, l.decay_rank, hd, st));
-                RUN(recurrence(l, [&] { return launch_chunk_gla(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
+                RUN(recurrence(l, rest, [&] { return launch_chunk_gla(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, m->chunk, m->chunk_floats, NT, longest, st); },
                                [&](int kinds, int most) { return launch_gla_recurrent(dt, m->proj, lp.n_in, m->f32a, state, m->f32b, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim, st, kinds, most); }));
                 RUN(launch_gla_output(dt, m->f32b, l.out_norm, c.norm_eps, gate, lp.n_in, m->mix2, NT, l.heads, l.vdim, st));
             }
+            if (ones)
+                RUN(launch_gla_decode(dt, m->proj, lp.n_in, 2 * hd + 2 * hv, l.w_decay, l.decay_bias, l.tau, l.decay_rank, state, d_start, d_pos0, d_slot, S, l.heads, l.dim, l.vdim,
+                                      l.out_norm, c.norm_eps, 2 * hd + hv, m->mix2, st));
             n_mixed = hv;
         }
         RUN(linear(m, m->mix2, l.w_out, m->y, NT, n_mixed, width, st));

@@ -194,9 +194,10 @@ int launch_mingru(int dtype, const void *proj, int ld, const float *bias, float 
 // decay[t, c] = sigmoid(z)^(1/tau), z = w_decay[c, :] . proj[t, col0 : col0 + rank] + bias[c]   (fp32 from the projection on)
 int launch_gla_decay(int dtype, const void *proj, int ld, int col0, const void *w_decay, const float *bias, float tau, float *decay,
                      int tokens, int rank, int channels, cudaStream_t st);
-// kinds: which portions the batch holds, when the host knows (one-token portions have a kernel of their own; the default launches both)
+// kinds: which portions to do (one-token portions have a kernel of their own; the default launches both)
 constexpr int kGlaOneToken = 1, kGlaManyTokens = 2;
-// a batch of one-token portions: decay, step, norm and gate in one launch (rank_col, gate_col: columns of the low-rank vector and of the gate in proj)
+// one-token portions: decay, step, norm and gate in one launch (rank_col, gate_col: columns of the low-rank vector and of the gate in proj)
+bool gla_decode_takes(int dtype, const void *proj, int ld, const void *w_decay, int rank, const float *state, int n_seqs, int dim, int vdim);
 int launch_gla_decode(int dtype, const void *proj, int ld, int rank_col, const void *w_decay, const float *bias, float tau, int rank, float *state, const int *seq_start,
                       const int *seq_pos0, const int *seq_slot, int n_seqs, int heads, int dim, int vdim, const float *norm, float eps, int gate_col, void *out,
                       cudaStream_t st);

@@ -38,3 +38,29 @@ def test_steps(dtype, tol, heads, dim, vdim, rank):
         assert not np.isnan(lg).any()
         err = np.linalg.norm(lg - want, axis=-1) / np.linalg.norm(want, axis=-1)
         assert err.max() < tol, (n, float(err.max()))
+
+
+@pytest.mark.parametrize("heads,dim,vdim,rank", [(8, 64, 128, 16), (8, 128, 256, 64)])
+def test_a_token_by_itself(heads, dim, vdim, rank):
+    """A decoded token's row has the same bits by itself, among others, and beside portions of several tokens (sixteen rows in all: the range in which the linears around
+    it have), step after step over the state that it leaves; and the portions beside it are what they are without it."""
+    config = ref.make_config([ref.gla_layer(heads=heads, dim=dim, vdim=vdim, tau=4.0) for _ in range(2)], width=128)
+    _, packed = ref.make_weights(config, seed=heads + dim, decay_rank=rank)
+    model = importlib.import_module("llm-inference-engine_b200.models.vasolix").VasolixModel(config, packed, dtype="float16", device="cuda:0", max_tokens=128, max_seqs=4,
+                                                                                              max_pages_per_seq=2)
+    serving = importlib.import_module("llm-inference-engine_b200.serving")
+    before, steps, beside = [0, 1, 5, 40], 4, [1, 5, 1, 7]  # tokens that each sequence brings to a step
+    toks = [np.random.default_rng(i).integers(0, config["vocab"], n + steps * k).tolist() for i, (n, k) in enumerate(zip(before, beside))]
+    rows = {}
+    for how in ("alone", "together"):
+        sess = serving.Session(model, 512, max_seqs=4, max_batch_tokens=128, poison=True)
+        ids = [sess.open() for _ in before]
+        for i, n in enumerate(before):
+            if n:
+                sess.feed([(ids[i], toks[i][:n], [])])
+        for s in range(steps):
+            entries = [(ids[i], toks[i][n + s * k:n + (s + 1) * k], list(range(k))) for i, (n, k) in enumerate(zip(before, beside))]
+            rows[how, s] = torch.cat([sess.feed([e]) for e in entries]) if how == "alone" else sess.feed(entries)
+    for s in range(steps):
+        assert not torch.isnan(rows["together", s]).any()
+        assert torch.equal(rows["alone", s], rows["together", s]), s
