@@ -1397,6 +1397,14 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
     const bool lat_tc = c.dtype != B200_F32 && NT >= 256;
     const int t_pad = lat_tc ? (NT + 127) / 128 * 128 : (NT + kMoeTileM - 1) / kMoeTileM * kMoeTileM;
     const int tph = t_pad / kMoeTileM, tph128 = lat_tc ? t_pad / 128 : 0;
+    // prompt portions go to the tensor-core attention in tiles of <= 64 consecutive tokens, short ones (decoded tokens) to the per-token kernel
+    constexpr int kShortPortion = 8;
+    static_assert(kShortPortion == kMingruShort, "one list of short portions serves both");
+    size_t n_listed = 0;  // tokens of short portions
+    for (int s = 0; s < S; ++s) {
+        const int n = b->seq_start[s + 1] - b->seq_start[s];
+        n_listed += n > 0 && n < kShortPortion ? n : 0;
+    }
     bool any_mingru = false;
     size_t n_tickets = 0;
     for (int i = 0; i < c.num_layers; ++i) {
@@ -1404,9 +1412,9 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         any_mingru |= l.mixer == B200_MIXER_MINGRU;
         for (const b200_hybrid_layer_t *mx : {&l, l.side})
             if (mx && (mx->mixer == B200_MIXER_ATTN_CHUNKED || mx->mixer == B200_MIXER_ATTN_SCORED))
-                n_tickets = std::max(n_tickets, std::min((size_t)NT * mx->heads, (size_t)kTokenTickets));
+                n_tickets = std::max(n_tickets, std::min(n_listed * mx->heads, (size_t)kTokenTickets));
     }
-    const size_t n_tile_ints = 4 * ((size_t)NT / 64 + S + 1), n_chunk_ints = any_mingru ? n_tile_ints : 0, n_stile_ints = (size_t)4 * NT;
+    const size_t n_tile_ints = 4 * ((size_t)NT / 64 + S + 1), n_chunk_ints = any_mingru ? n_tile_ints : 0, n_stile_ints = 4 * n_listed;
     hm.assign(n_tile_ints + n_chunk_ints + n_stile_ints + (size_t)5 * NT + 3 * S + 1 + (size_t)S * mpps + (size_t)lat_heads * (tph + tph128) + 2 * c.num_layers + n_tickets, 0);
     int *h_tiles = hm.data(), *h_chunks = h_tiles + n_tile_ints, *h_stiles = h_chunks + n_chunk_ints, *h_ids = h_stiles + n_stile_ints, *h_seq = h_ids + NT, *h_pos = h_seq + NT,
         *h_want = h_pos + NT, *h_short = h_want + NT, *h_start = h_short + NT, *h_pos0 = h_start + S + 1, *h_slot = h_pos0 + S, *h_bt = h_slot + S,
@@ -1418,9 +1426,6 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         const bool lat = m->layers[i].mixer == B200_MIXER_LATENT;
         h_lat_n[i] = lat ? m->layers[i].heads * tph : 0, h_lat_n128[i] = lat ? m->layers[i].heads * tph128 : 0;
     }
-    // prompt portions go to the tensor-core attention in tiles of <= 64 consecutive tokens, short ones (decoded tokens) to the per-token kernel
-    constexpr int kShortPortion = 8;
-    static_assert(kShortPortion == kMingruShort, "one list of short portions serves both");
     int n_tiles = 0, n_short = 0, n_chunks = 0, gla_kinds = 0;
     // minGRU chunks: at most 64 per portion (a chunk composes the maps of all chunks before it), of whole multiples of kMingruChunk tokens
     int longest = 0, long_tokens = 0;  // long_tokens: of the portions that the token-parallel recurrences can take

@@ -1,0 +1,38 @@
+"""What a call of the layer-list decoder copies to the device: the description of its batch (csrc/hybrid.cu, b200_hybrid_forward), in proportion to what is in it.  The
+list of decoded tokens (16 bytes each) and the counters of their runs of keys (one per token and query head) cost a prompt nothing."""
+import importlib
+import json
+
+import numpy as np
+import pytest
+import torch
+
+import vasolix_oracle as ref
+
+pytestmark = pytest.mark.gpu
+
+
+def uploaded(call, path):
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    p.export_chrome_trace(str(path))
+    return sum(e["args"]["bytes"] for e in json.load(open(path))["traceEvents"] if e.get("cat") == "gpu_memcpy" and "HtoD" in e["name"])
+
+
+def test_a_prompt_uploads_no_list_of_decoded_tokens(tmp_path):
+    heads, tokens, pages, layers = 4, 2048, 40, 1
+    config = ref.make_config([ref.attention_layer(heads=heads, kv_heads=2, dim=64, size=4096, scale=0.125) for _ in range(layers)], width=64)
+    _, packed = ref.make_weights(config, seed=2)
+    model = importlib.import_module("llm-inference-engine_b200.models.vasolix").VasolixModel(config, packed, dtype="bfloat16", device="cuda:0", max_tokens=tokens, max_seqs=1,
+                                                                                              max_pages_per_seq=pages)
+    sess = importlib.import_module("llm-inference-engine_b200.serving").Session(model, 2048 + 64, max_seqs=1, max_batch_tokens=tokens)
+    toks = np.random.default_rng(0).integers(0, config["vocab"], tokens + 1).tolist()
+    i = sess.open()
+    prompt = uploaded(lambda: sess.feed([(i, toks[:tokens], [])]), tmp_path / "p.json")
+    decode = uploaded(lambda: sess.feed([(i, toks[tokens:], [0])]), tmp_path / "d.json")
+    # ids, sequence, position, wanted rows and short rows of every token; tiles of 64 tokens; start, first position, slot; pages; two counts per layer
+    ints = lambda n, listed: 5 * n + 4 * (n // 64 + 2) + 4 + pages + 2 * layers + listed * (4 + heads)  # noqa: E731
+    assert prompt == 4 * ints(tokens, 0), (prompt, ints(tokens, 0) * 4)
+    assert decode == 4 * ints(1, 1), (decode, ints(1, 1) * 4)
