@@ -35,7 +35,7 @@ bool tile_map(CUtensorMap_st *map, const void *ptr, size_t rows, int cols, int b
 // Waits inside kernels have a limit: a fault elsewhere must not hang the device.  A kernel whose wait runs out stores NaN in place of what it could not
 // form, waits for its own copies, leaves its code in the process's wait word (mapped host memory) and returns; every later call of the library on the host
 // reports the word until b200_wait_error(1) clears it.  (Replayed graphs make no calls: their owner reads b200_wait_error().)
-enum WaitCode : unsigned int { kWaitGemvRs = 1, kWaitGemmPair = 2, kWaitPromptAttn = 3, kWaitProbe = 4 };
+enum WaitCode : unsigned int { kWaitGemvRs = 1, kWaitGemmPair = 2, kWaitPromptAttn = 3, kWaitProbe = 4, kWaitGemm = 5 };
 struct WaitGuard {          // kernel argument
     unsigned int *word;     // the wait word as the device sees it, or NULL
     unsigned int clocks;    // limit of one wait; 0: every wait runs out at once
@@ -205,6 +205,37 @@ static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity
 __device__ __forceinline__ bool mbar_wait_guarded(uint32_t bar, uint32_t parity, const WaitGuard &wg, unsigned int code) {
     if (wg.clocks != 0 && mbar_try(bar, parity)) return true;
     return mbar_wait_slow(bar, parity, wg.word, wg.clocks, code);
+}
+// The same where a wait is paid per k-block of a narrow tile: one piece of code without a call or a way out of the caller's loop.  `left`: the clocks that the
+// thread's waits may still take, one limit for all of them; zero: it has given up, and its waits return at once.  `flag`, in shared memory: set to 1 when the thread
+// gives up, with the numbers x and y behind it.
+__device__ __forceinline__ void mbar_wait_near(uint32_t bar, uint32_t parity, uint32_t &left, uint32_t flag, uint32_t x, uint32_t y) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        ".reg .u32 was, now, step;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE_%=;\n\t"
+        "setp.eq.u32 q, %0, 0;\n\t"
+        "@q bra DONE_%=;\n\t"
+        "mov.u32 was, %%clock;\n\t"
+        "WAIT_%=:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE_%=;\n\t"
+        "mov.u32 now, %%clock;\n\t"
+        "sub.u32 step, now, was;\n\t"
+        "min.u32 step, step, %3;\n\t"
+        "min.u32 step, step, %0;\n\t"
+        "sub.u32 %0, %0, step;\n\t"
+        "mov.u32 was, now;\n\t"
+        "setp.ne.u32 q, %0, 0;\n\t"
+        "@q bra WAIT_%=;\n\t"
+        "st.volatile.shared.v2.u32 [%4 + 8], {%5, %6};\n\t"
+        "st.volatile.shared.u32 [%4], 1;\n\t"
+        "membar.cta;\n\t"
+        "DONE_%=:\n\t}"
+        : "+r"(left)
+        : "r"(bar), "r"(parity), "n"(kWaitStep), "r"(flag), "r"(x), "r"(y)
+        : "memory");
 }
 // for what the CTA has under way itself when it leaves (copies into its shared memory, products that read it): whatever has run out before
 static __device__ __noinline__ bool mbar_drain(uint32_t bar, uint32_t parity) {

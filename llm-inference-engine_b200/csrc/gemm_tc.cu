@@ -39,8 +39,7 @@ struct GemmTcParams {
     int a_rows;    // rows of A that a stage loads: all 128, or fewer where A has fewer (what lies below them in a stage fills accumulator rows that nobody stores)
     int stages;
     int is_bf16;
-    int acc_bufs;  // TMEM accumulators (2 when 2*bn <= 512)
-    int acc_stride;  // TMEM columns between the accumulators: bn, or 256 for the 192..240-column tiles (power-of-two placement)
+    int acc_stride;  // TMEM columns between the two accumulators: bn, or 256 above 128 columns (power-of-two placement)
     unsigned int tmem_cols;
     // SwiGLU epilogue (gate_up linear of the prefill path, launchLinearGemm + launchSiluAndMul in one kernel): B = W [2I, K] with the gate
     // rows first; tile tb multiplies gate rows [hw tb, +hw) AND up rows [I + hw tb, +hw) as one N = 2 hw tile (two TMA boxes into one
@@ -56,6 +55,7 @@ struct GemmTcParams {
     const float *scale;  // of every row of B (fp32, NULL: none): the sums are multiplied by it, before anything else
     int finish;     // 1: the result is rounded and takes `bias` (bias_act) before its activation (plain GEMM, A = activations)
     const float *bias;
+    WaitGuard wait;
 };
 
 // A CTA's pieces of work: k-blocks [kb0, kb1) of output tiles.
@@ -86,26 +86,38 @@ __device__ __forceinline__ void bar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity) {
+// A stage's copies, two or three boxes at column c of their matrices, and what its barrier expects of them; yes == 0: nothing.
+__device__ __forceinline__ void tma_stage(uint32_t yes, uint32_t bar, uint32_t bytes, int c, uint32_t da, const CUtensorMap *ma, int ra, uint32_t db, const CUtensorMap *mb, int rb) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "WAIT_%=:\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t"
-        "@p bra DONE_%=;\n\t"
-        "bra WAIT_%=;\n\t"
-        "DONE_%=:\n\t}" ::"r"(bar),
-        "r"(parity)
+        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %0, 0;\n\t@p bra DONE_%=;\n\t"
+        "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %2;\n\t"
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%4], [%5, {%3, %6}], [%1];\n\t"
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%7], [%8, {%3, %9}], [%1];\n\t"
+        "DONE_%=:\n\t}" ::"r"(yes), "r"(bar), "r"(bytes), "r"(c), "r"(da), "l"(ma), "r"(ra), "r"(db), "l"(mb), "r"(rb)
         : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-                 "l"(map), "r"(c0), "r"(c1), "r"(bar)
-                 : "memory");
+__device__ __forceinline__ void tma_stage(uint32_t yes, uint32_t bar, uint32_t bytes, int c, uint32_t da, const CUtensorMap *ma, int ra, uint32_t db, const CUtensorMap *mb, int rb,
+                                          uint32_t dc, int rc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %0, 0;\n\t@p bra DONE_%=;\n\t"
+        "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %2;\n\t"
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%4], [%5, {%3, %6}], [%1];\n\t"
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%7], [%8, {%3, %9}], [%1];\n\t"
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%10], [%8, {%3, %11}], [%1];\n\t"
+        "DONE_%=:\n\t}" ::"r"(yes), "r"(bar), "r"(bytes), "r"(c), "r"(da), "l"(ma), "r"(ra), "r"(db), "l"(mb), "r"(rb), "r"(dc), "r"(rc)
+        : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(uint32_t yes, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %0, 0;\n\t@p bra DONE_%=;\n\t"
+        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t"
+        "DONE_%=:\n\t}" ::"r"(yes), "r"(bar)
+        : "memory");
 }
 __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -280,6 +292,13 @@ template <typename T, typename GET> __device__ __forceinline__ void finish_tile(
     }
 }
 
+// what a wait that ran out leaves of those columns
+template <typename T> __device__ __forceinline__ void lose_tile(const GemmTcParams &p, int ta, int row, int tb, int c0, int c1) {
+    const int i = ta * p.a_rows + row, j0 = tb * (p.swiglu_inter ? p.swiglu_hw : p.bn);
+    if (row >= p.a_rows || i >= p.rowsA) return;
+    for (int c = j0 + c0; c < min(j0 + c1, p.rowsB); ++c) reinterpret_cast<T *>(p.C)[(size_t)i * p.ldc + c] = Elem<T>::from_f(__uint_as_float(0x7fc00000u));
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kTcThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmTcParams p) {
@@ -292,6 +311,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t full0 = s_u32(bars), empty0 = full0 + 8 * kMaxStages;
     const uint32_t tfull0 = empty0 + 8 * kMaxStages, tempty0 = tfull0 + 16;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kMaxStages + 4);
+    const uint32_t drain = tempty0 + 24;  // (behind the TMEM slot)
+    __shared__ __align__(16) volatile int gave_up[8];  // the producer: {yes, -, its stage and phase then}; the issuer or the epilogue: {yes, -, -, -}
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -306,6 +327,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             bar_init(tfull0 + 8 * a, 1);
             bar_init(tempty0 + 8 * a, 4);  // one arrive per epilogue warp
         }
+        bar_init(drain, 1);
+        gave_up[0] = gave_up[4] = p.wait.clocks == 0, gave_up[2] = 0, gave_up[3] = 1;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -320,30 +343,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     pdl_wait();               // everything below reads (x) or overwrites (C) tensors of the previous kernel
     pdl_launch_dependents();
 
+    // A wait that runs out: the producer copies no more, the issuer hands nothing on (so that the others' waits run out in turn), and all of the CTA's tiles are NaN in the
+    // end.  The loops run on, and nothing that they need lives beyond them: an exit that hangs on a wait, or a stage counter that is read again at the end, takes
+    // the uniform registers from them.  Against waits without a limit, us: 2048 x 2048 of 94 tokens 6.8 -> 7.5 (with exits from the loops 9.6 to 10.7), K = 4096, N = 4096
+    // of 94 11.8 -> 12.4, K = 11008, N = 4096 of 267 36.0 -> 36.7.
+    const uint32_t flag = s_u32(const_cast<const int *>(gave_up));
     if (warp == 0) {
         // ================================================= TMA producer
         if (elect_one()) {
             SegIter si(p);
             Seg sg;
             int s = 0;  // (stage and phase by counting: a remainder and a quotient per k-block were a third of what a narrow tile's block took)
-            uint32_t ph = 1;
+            uint32_t ph = 1, left = p.wait.clocks;
             while (si.next(sg)) {
                 const int ta = sg.ta, tb = sg.tb;
                 const int brow = (p.tile_expert ? p.tile_expert[ta] * p.rowsB : 0) + tb * p.bn;
                 for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-                    bar_wait(empty0 + 8 * s, ph);
-                    const uint32_t sa = s_u32(smem + (size_t)s * stage_bytes);
-                    bar_expect_tx(full0 + 8 * s, (uint32_t)stage_bytes);
-                    tma_load_2d(sa, &tmA, kb * kBK, ta * p.a_rows, full0 + 8 * s);
-                    if (p.swiglu_inter) {  // box = hw rows: the gate rows, then the up rows of the same columns
-                        tma_load_2d(sa + a_tile_bytes, &tmB, kb * kBK, tb * p.swiglu_hw, full0 + 8 * s);
-                        tma_load_2d(sa + a_tile_bytes + p.swiglu_hw * kBK * 2, &tmB, kb * kBK, p.swiglu_inter + tb * p.swiglu_hw, full0 + 8 * s);
-                    } else {
-                        tma_load_2d(sa + a_tile_bytes, &tmB, kb * kBK, brow, full0 + 8 * s);
-                    }
+                    mbar_wait_near(empty0 + 8 * s, ph, left, flag, (uint32_t)s, ph);
+                    const uint32_t sa = s_u32(smem + (size_t)s * stage_bytes), sb = sa + a_tile_bytes, bar = full0 + 8 * s;
+                    if (p.swiglu_inter)  // box = hw rows: the gate rows, then the up rows of the same columns
+                        tma_stage(left, bar, stage_bytes, kb * kBK, sa, &tmA, ta * p.a_rows, sb, &tmB, tb * p.swiglu_hw, sb + p.swiglu_hw * kBK * 2, p.swiglu_inter + tb * p.swiglu_hw);
+                    else
+                        tma_stage(left, bar, stage_bytes, kb * kBK, sa, &tmA, ta * p.a_rows, sb, &tmB, brow);
                     if (++s == p.stages) s = 0, ph ^= 1;
                 }
             }
+            if (left) gave_up[2] = s, gave_up[3] = (int)ph;
         }
     } else if (warp == 1) {
         // ================================================= MMA issuer
@@ -351,15 +376,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         SegIter si(p);
         Seg sg;
         int s = 0, t = 0;
-        uint32_t ph = 0;
+        uint32_t ph = 0, left = p.wait.clocks;
+        auto wait = [&](uint32_t bar, uint32_t parity) { mbar_wait_near(bar, parity, left, flag + 16, 0, 0); };
         const bool issuer = elect_one();
         for (; issuer && si.next(sg); ++t) {
-            const int acc = t % p.acc_bufs;
-            bar_wait(tempty0 + 8 * acc, ((t / p.acc_bufs) & 1) ^ 1);  // the epilogue has drained this accumulator
+            const int acc = t & 1;
+            wait(tempty0 + 8 * acc, ((t >> 1) & 1) ^ 1);  // the epilogue has drained this accumulator
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(acc * p.acc_stride);
             for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-                bar_wait(full0 + 8 * s, ph);
+                wait(full0 + 8 * s, ph);
                 tc_fence_after();
                 {
                     const uint32_t sa = s_u32(smem + (size_t)s * stage_bytes);
@@ -369,8 +395,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         // advancing K inside the 128-byte swizzle row: +32 bytes = +2 in the (>>4) start-address field
                         tc_mma_f16(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > sg.kb0 || k > 0) ? 1u : 0u);
                     }
-                    tc_commit(empty0 + 8 * s);                          // smem stage reusable once these MMAs have read it
-                    if (kb == sg.kb1 - 1) tc_commit(tfull0 + 8 * acc);  // accumulator complete
+                    tc_commit_if(left, empty0 + 8 * s);                          // smem stage reusable once these MMAs have read it
+                    if (kb == sg.kb1 - 1) tc_commit_if(left, tfull0 + 8 * acc);  // accumulator complete
                 }
                 if (++s == p.stages) s = 0, ph ^= 1;
             }
@@ -381,9 +407,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         SegIter si(p);
         Seg sg;
         int t = 0;
+        uint32_t left = p.wait.clocks;
         for (; si.next(sg); ++t) {
-            const int acc = t % p.acc_bufs;
-            bar_wait(tfull0 + 8 * acc, (t / p.acc_bufs) & 1);
+            const int acc = t & 1;
+            mbar_wait_near(tfull0 + 8 * acc, (t >> 1) & 1, left, flag + 16, 0, 0);
+            __syncwarp();
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * p.acc_stride);
             auto fetch = [&](int c, uint32_t (&r)[16]) {
@@ -406,11 +434,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (lane == 0) bar_arrive(tempty0 + 8 * acc);
         }
     }
+    int lost = 0;
     if (p.splits > 1) {
         // every CTA of the cluster adds up its part of the tile's columns, and stays until the others have read what it holds
         __syncthreads();
         cluster_sync_all();
         const int tile = blockIdx.x / p.splits, rank = blockIdx.x % p.splits;
+        for (int x = 0; x < p.splits; ++x) {
+            int a, b;
+            asm volatile("ld.shared::cluster.s32 %0, [%2];\n\tld.shared::cluster.s32 %1, [%2 + 16];" : "=r"(a), "=r"(b) : "r"(in_cta(flag, (uint32_t)x)) : "memory");
+            lost |= a | b;
+        }
         if (warp >= 2) {
             const int q = warp & 3, cols = (p.swiglu_inter ? p.swiglu_hw : p.bn) / p.splits;
             const uint32_t at = s_u32(smem) + (uint32_t)(q * 32 + lane) * 4;
@@ -434,6 +468,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     tc_fence_before();
     __syncthreads();
+    if (lost | gave_up[0] | gave_up[4]) {  // the CTA stays until its copies have landed and its products have read them, and its tiles are NaN
+        uint32_t left = kWaitClocks;
+        if (warp == 0 && elect_one()) {  // (stages before the producer's last one in its round, the others in the round before)
+            for (int i = 0; i < p.stages; ++i) mbar_wait_near(full0 + 8 * i, (uint32_t)(i < gave_up[2] ? gave_up[3] ^ 1 : gave_up[3]), left, flag + 16, 0, 0);
+            if (p.wait.word) {
+                *reinterpret_cast<volatile unsigned int *>(p.wait.word) = kWaitGemm;
+                __threadfence_system();
+            }
+        } else if (warp == 1 && elect_one()) {  // (the same thread as above)
+            tc_commit(drain);
+            mbar_wait_near(drain, 0, left, flag + 16, 0, 0);
+        } else if (warp >= 2) {
+            const int cols = (p.swiglu_inter ? p.swiglu_hw : p.bn) / p.splits, c0 = blockIdx.x % p.splits * cols;
+            SegIter si(p);
+            Seg sg;
+            while (si.next(sg)) lose_tile<T>(p, sg.ta, (warp & 3) * 32 + lane, sg.tb, c0, c0 + cols);
+        }
+        __syncthreads();
+    }
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tmem_cols) : "memory");
@@ -767,13 +820,13 @@ static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int
     p.C = y, p.K = K, p.is_bf16 = bf16 ? 1 : 0;
     p.swiglu_inter = swiglu_inter;
     p.finish = fin.on, p.act = fin.on ? fin.act : -1, p.bias = fin.bias, p.scale = fin.scale;
+    p.wait = wait_guard();
     p.kb_total = (K + kBK - 1) / kBK;
     p.rowsA = M, p.rowsB = p.ldc = swiglu_inter ? swiglu_inter : N;  // (SwiGLU: I output columns; the MMA tile is hw gate + hw up rows)
     p.bn = plan.bn, p.splits = plan.splits, p.swiglu_hw = swiglu_inter ? plan.bn / 2 : 0;
     p.a_rows = a_rows;
     p.tilesA = tiles_a, p.tilesB = (cols + p.bn - 1) / p.bn;
     const int tiles = p.tilesA * p.tilesB, grid = p.splits > 1 ? tiles * p.splits : std::min(tiles, sms);
-    p.acc_bufs = 2;
     p.acc_stride = p.bn > 128 ? 256 : p.bn;
     p.tmem_cols = pow2_cols(p.acc_stride + p.bn);
     const int stage_bytes = (p.a_rows + p.bn) * kBK * 2;
@@ -820,14 +873,13 @@ int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, 
     const int sms = sm_count(), most = max_rows / tile, likely = std::max(1, most - experts / 2);
     GemmTcParams p = {};
     p.C = c, p.ldc = N, p.K = K, p.splits = 1, p.is_bf16 = bf16 ? 1 : 0;
-    p.act = act, p.tile_expert = tile_expert, p.n_live = n_live;
+    p.act = act, p.tile_expert = tile_expert, p.n_live = n_live, p.wait = wait_guard();
     p.kb_total = (K + kBK - 1) / kBK;
     p.rowsA = max_rows, p.rowsB = N;
     p.a_rows = tile, p.tilesA = most;
     p.bn = plan_tiles(likely, tile, N, K, sms, 16, 1).bn;
     p.tilesB = (N + p.bn - 1) / p.bn;
     const int grid = std::min(most * p.tilesB, sms);
-    p.acc_bufs = 2;
     p.acc_stride = p.bn > 128 ? 256 : p.bn;
     p.tmem_cols = pow2_cols(p.acc_stride + p.bn);
     const int stage_bytes = (p.a_rows + p.bn) * kBK * 2;

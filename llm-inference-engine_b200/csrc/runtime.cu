@@ -63,8 +63,8 @@ static unsigned int wait_code() {
 int wait_status(const char *what) {
     const unsigned int code = wait_code();
     if (code == 0) return B200_OK;
-    static const char *const names[] = {"", "the streaming GEMV", "the CTA-pair GEMM", "the prompt attention", "the wait probe"};
-    set_error("%s: a wait inside %s ran out; results since then are not valid (b200_wait_error(1) clears this)", what, code <= kWaitProbe ? names[code] : "a kernel");
+    static const char *const names[] = {"", "the streaming GEMV", "the CTA-pair GEMM", "the prompt attention", "the wait probe", "the one-CTA GEMM"};
+    set_error("%s: a wait inside %s ran out; results since then are not valid (b200_wait_error(1) clears this)", what, code <= kWaitGemm ? names[code] : "a kernel");
     return B200_ERR_CUDA;
 }
 

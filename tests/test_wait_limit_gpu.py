@@ -12,7 +12,7 @@ import util
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 b200 = util.b200()
-GEMV, PAIR, PROMPT, PROBE = 1, 2, 3, 4
+GEMV, PAIR, PROMPT, PROBE, GEMM = 1, 2, 3, 4, 5
 
 
 @pytest.fixture(autouse=True)
@@ -105,6 +105,41 @@ def test_pair_gemm(m, k, n):
         got = run_out(call, PAIR)
         assert bool(torch.isnan(got).all())
         assert torch.equal(call(), want) and not bool(torch.isnan(want).any())
+
+
+@pytest.mark.parametrize("m,k,n", [(17, 64, 16), (94, 2048, 2048), (300, 2048, 512), (100, 512, 64000), (17, 11008, 4096), (256, 28672, 1024)])
+def test_one_cta_gemm(m, k, n):
+    """Tiles of their own, one and several a CTA, and (the last two) tiles whose k two CTAs share."""
+    gen = torch.Generator(device=DEV).manual_seed(k + n + m)
+    x, w = (torch.randn(r, k, generator=gen, device=DEV).bfloat16() for r in (m, n))
+    bias = torch.randn(n, generator=gen, device=DEV)
+    calls = [lambda: b200.linear(x, w), lambda: b200.linear_act(x, w, bias, 3)]  # (a rectifier would make a number of NaN)
+    if m > 128 and n >= 256:
+        calls.append(lambda: b200.linear_swiglu(x, w))
+    for call in calls:
+        want = call()
+        got = run_out(call, GEMM)
+        assert bool(torch.isnan(got).all())
+        assert torch.equal(call(), want) and not bool(torch.isnan(want).any())
+
+
+@pytest.mark.parametrize("m,k,n", [(94, 2048, 2048), (100, 512, 64000), (300, 4096, 12288), (17, 11008, 4096), (256, 28672, 1024)])
+def test_one_cta_gemm_that_gives_up_halfway(m, k, n):
+    """Limits of the order of what a launch waits for, so that some CTAs give up with copies and products under way: what a CTA stores is either right or NaN, and the
+    next call is what it was."""
+    gen = torch.Generator(device=DEV).manual_seed(k + n + m)
+    x, w = (torch.randn(r, k, generator=gen, device=DEV).bfloat16() for r in (m, n))
+    want = b200.linear(x, w)
+    for clocks in (1, 300, 1000, 2000, 4000, 8000, 2 ** 31 - 1):
+        b200.lib().b200_wait_limit(clocks)
+        got = b200.linear(x, w)
+        b200.lib().b200_wait_limit(2 ** 32 - 1)
+        torch.cuda.synchronize()
+        code = b200.wait_error(clear=True)
+        lost = torch.isnan(got)
+        assert code in (0, GEMM) and bool((lost | (got == want)).all())
+        assert bool(lost.any()) == (code == GEMM) and (clocks < 2 ** 30 or code == 0)
+        assert torch.equal(b200.linear(x, w), want)
 
 
 @pytest.mark.parametrize("window", [0, 100])
