@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Which kernel, how many passes over the weights and which ring geometry each linear of a decode step gets -- a Python MODEL of the host-side
-dispatch (no GPU): decoder.cu norm_linear (norm inside the GEMV for one dense token, a norm kernel in front otherwise), gemv_f32.cu launch_gemv_nk
+dispatch (no GPU): decoder.cu norm_linear (norm inside the GEMV for one dense or INT4 token, a norm kernel in front otherwise) and plain_linear, gemv_f32.cu launch_gemv_nk
 (gemv_qd for up to 8 tokens of INT4 and short dense rows, gemv_rs, what its ring refuses on gemv_mma, gemv_sr for one token of short rows, the SIMT GEMV for up
 to 4 tokens), linear.cu (GEMV passes, tcgen05 GEMM for dense M > 16), gemv_inst.cuh, gemv_qd.cuh launch_gemv_qd_t, gemv_sr.cuh launch_gemv_sr_t, gemv_rs.cuh
 gemv_rs_geometry and gemv_mma.cuh gemv_mma_geometry.  It restates those few formulas; when they change, this file must follow
@@ -138,16 +138,20 @@ def gemv_any(M, K, N, fmt, swiglu=False, push=False):
     return (fmt == "dense" and not push and gemv_sr_plan(M, K)) or gemv_nk_plan(M, K, fmt)
 
 
-def linear_plan(M, K, N, fmt, fused_rows=16, swiglu=False, push=False):
-    """One linear of the decode step: (path, passes over the weights, geometry)."""
-    if M == 1 and fmt == "dense":  # the norm / residual / tensor-parallel prologue inside the GEMV
+def linear_plan(M, K, N, fmt, fused_rows=16, swiglu=False, push=False, norm=True, tp=False):
+    """One linear of the decode step: (path, passes over the weights, geometry).  norm: residual and norm in front (QKV, gate-up); tp: a tensor-parallel exchange too."""
+    if norm and M == 1 and fmt == "dense":  # the norm / residual / tensor-parallel prologue inside the GEMV
         g = (not push and gemv_sr_plan(M, K)) or gemv_nk_plan(M, K, fmt)
+        if g:
+            return ("fused " + g["kernel"], 1, g)
+    if norm and M == 1 and fmt == "int4" and not tp and not push and K <= 16384:  # residual and norm in the norm kernel's order of summation
+        g = gemv_qd_plan(M, K, N, fmt, swiglu)
         if g:
             return ("fused " + g["kernel"], 1, g)
     if M <= fused_rows:
         g = gemv_any(M, K, N, fmt, swiglu, push)
         if g:
-            return ("norm_kernel + " + g["kernel"], 1, g)
+            return (("norm_kernel + " if norm else "") + g["kernel"], 1, g)
     if fmt == "dense" and M > 4:
         return ("un-fused gemm_tc", 1, None)
     for step in (16, 8, 4):  # linear.cu: quantised weights in passes
@@ -165,7 +169,7 @@ def step_plan(name, hidden, heads, kv_heads, d, inter, tp, batch, fmt):
               ("down", inter // tp, hidden)]
     lines = [f"{name}, batch {batch}, weights {fmt}" + (f", TP-{tp} (one rank)" if tp > 1 else "")]
     for lin, K, N in shapes:
-        path, passes, g = linear_plan(batch, K, N, fmt, fused_rows, lin == "gate_up", tp > 1 and lin in ("o", "down"))
+        path, passes, g = linear_plan(batch, K, N, fmt, fused_rows, lin == "gate_up", tp > 1 and lin in ("o", "down"), lin in ("qkv", "gate_up"), tp > 1)
         if g and g["kernel"] == "gemv_qd":
             geo = f"ring of registers, {16 // g['warps']} CTAs of {g['warps']} warps per SM, barriers per 16 rows: {g['barriers']}"
         elif g and g["kernel"] == "gemv_sr":

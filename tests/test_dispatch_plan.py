@@ -30,7 +30,7 @@ def test_streaming_gemv_geometry(fmt, k, m):
     assert g["parts"] == max(1, -(-k // 4096)) and g["part_k"] % 128 == 0 and g["part_k"] <= 16 * 8 * 32
     assert g["parts"] * g["part_k"] >= k > (g["parts"] - 1) * g["part_k"]
     rows, nt = (8 if fmt == "dense" else 16), (2 if m > 8 else 1)
-    stage = rows * (-(-g["piece_bytes"] // 128) * 128 + (16 if fmt == "fp8" else 64))
+    stage = rows * (-(-g["piece_bytes"] // 128) * 128 + 64)
     tile, sums = (128, 128) if fmt == "dense" else (160 * nt, 128 * nt)
     units = -(-(-(-4096 // rows)) // 148)
     assert 2 <= g["stages"] <= 12
@@ -45,14 +45,18 @@ def test_streaming_gemv_stages():
 
 
 def test_decode_batches_read_the_weights_once():
-    """Every decode batch up to 16 is ONE pass over the weights, in every format, behind a norm kernel; one dense token keeps the norm inside the GEMV."""
+    """Every decode batch up to 16 is ONE pass over the weights, in every format, behind a norm kernel; one dense or INT4 token has the norm inside the GEMV."""
     for fmt in ("dense", "fp8", "int4"):
         for m in (1, 2, 4, 8, 16):
             for k, n in ((4096, 12288), (11008, 4096), (8192, 1280)):
                 path, passes, geo = dp.linear_plan(m, k, n, fmt)
                 streamed = fmt == "int4" and m <= 8 and not (k == 11008 and m == 8)  # (whose 8 tokens leave no room for what is in flight)
-                want = "fused gemv_nk" if fmt == "dense" and m == 1 else "norm_kernel + gemv_qd" if streamed else "norm_kernel + gemv_rs"
+                want = "fused gemv_nk" if fmt == "dense" and m == 1 else "fused gemv_qd" if streamed and m == 1 else "norm_kernel + gemv_qd" if streamed else "norm_kernel + gemv_rs"
                 assert passes == 1 and path == want, (fmt, m, k, path)
+    # the linears without a norm in front (O, down), one behind a tensor-parallel exchange, and rows too long for the norm's registers
+    assert dp.linear_plan(1, 4096, 4096, "int4", norm=False)[0] == "gemv_qd" and dp.linear_plan(1, 11008, 4096, "fp8", norm=False)[0] == "gemv_rs"
+    assert dp.linear_plan(1, 2048, 4096, "dense", norm=False)[0] == "gemv_qd" and dp.linear_plan(1, 4096, 4096, "dense", norm=False)[0] == "gemv_nk"
+    assert dp.linear_plan(1, 4096, 1536, "int4", tp=True)[0] == "norm_kernel + gemv_qd" and dp.linear_plan(1, 28672, 4096, "int4")[0] == "norm_kernel + gemv_qd"
     path, passes, _ = dp.linear_plan(32, 4096, 4096, "fp8")
     assert passes == 2 and path == "un-fused gemv_rs x 2 passes of <= 16 tokens"
 
