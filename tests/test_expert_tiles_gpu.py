@@ -14,7 +14,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype,tol,u", [("bfloat16", 4e-2, 2.0 ** -8), ("float16", 6e-3, 2.0 ** -11)])
 @pytest.mark.parametrize("tokens,experts,top,width,ff", [(65, 16, 2, 64, 72), (65, 3, 1, 128, 64), (85, 8, 2, 64, 64), (170, 8, 2, 128, 200), (196, 8, 2, 64, 64), (250, 16, 3, 64, 520),
-                                                         (767, 8, 2, 64, 64), (769, 8, 2, 128, 136), (1500, 5, 1, 64, 264), (600, 3, 3, 64, 64)])
+                                                         (767, 8, 2, 64, 64), (769, 8, 2, 128, 136), (1500, 5, 1, 64, 264), (600, 3, 3, 64, 64),
+                                                         # 32 rows an expert or fewer, planned by many CTAs (512 tokens and more)
+                                                         (512, 26, 1, 64, 64), (700, 128, 3, 64, 72)])
 def test_row_tiles(monkeypatch, dtype, tol, u, tokens, experts, top, width, ff):
     layer = ref.attention_layer(heads=2, kv_heads=1, dim=16, size=50, mlp=ref.moe(experts=experts, top=top, ff=ff, shared_ff=64))
     config = ref.make_config([layer], width=width, vocab=80)

@@ -93,3 +93,41 @@ def test_fp8_prompts_keep_their_scales_in_32_bits(dtype, T):
     anyscale, _ = engine("fp8", False)
     a, b = run(anyscale, [T]), run(anyscale, [16] * (T // 16) + ([T % 16] if T % 16 else []))
     assert (a - b).norm() <= 4 * u * b.norm()
+
+
+def fp8_scales(n, dt, gen):
+    """Scales that a rounding to 16 bits moves by a quarter to a half of its unit."""
+    u = torch.finfo(dt).eps
+    return ((1 + u * (torch.randint(0, 64, (n,), generator=gen, device=DEV) + 0.25 + 0.25 * torch.rand(n, generator=gen, device=DEV))) * 0.03).float()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T", [48, 49, 128, 129, 300])
+def test_fp8_scales_are_not_rounded(dtype, T):
+    """The value rows that a prompt leaves in the cache are one FP8 linear's outputs.  Its inputs are made +-1 (a norm of +-1 rows), so that the codes' sums are exact
+    in fp32 and the only roundings are the product's with the scale and the result's: half a unit of the type and 2^-23.  Scales folded into rounded 16-bit weights
+    break that bound."""
+    h, heads, kv, inter, d = 512, 4, 2, 768, 128
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    code = m.BF16 if dtype == torch.bfloat16 else m.F16
+    dec = m.Decoder(m.DecoderConfig(h, heads, kv, d, inter, 1, 320, 1, code, m.W_FP8, 128, 1e-6, d, 10000.0, 1, 0), DEV)
+    layer = {"g1": torch.ones(h, device=DEV, dtype=dtype), "g2": torch.ones(h, device=DEV, dtype=dtype)}
+    for name, n, k in (("qkv", (heads + 2 * kv) * d, h), ("o", h, heads * d), ("gate_up", 2 * inter, h), ("down", h, inter)):
+        layer[name] = (torch.randn(n, k, generator=gen, device=DEV).to(torch.float8_e4m3fn).view(torch.uint8), fp8_scales(n, dtype, gen), None)
+    dec.set_layer(0, layer)
+    x = torch.randint(0, 2, (T, h), generator=gen, device=DEV).to(dtype) * 2 - 1
+    k, v = (torch.zeros(1, 5, kv, 64, d, device=DEV, dtype=dtype) for _ in range(2))
+    i32 = lambda *a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    dec.prefill_paged(x.clone(), k, v, torch.arange(5, dtype=torch.int32, device=DEV).reshape(1, 5), i32(T), i32(0), i32(T), T)
+    got = v[0].permute(0, 2, 1, 3).reshape(-1, kv * d)[:T].double()
+    codes, scales, _ = layer["qkv"]
+    codes, scales = codes[(heads + kv) * d:].view(torch.float8_e4m3fn).double(), scales[(heads + kv) * d:].double()
+    want = (x.double() @ codes.T) * scales
+    bound = (0.5 * torch.finfo(dtype).eps + 2.0 ** -22) * want.abs() + torch.finfo(dtype).tiny
+
+    def broken(rows):
+        return float(((rows - want).abs() > bound).double().mean())
+
+    folded = (x.double() @ (codes * scales[:, None]).to(dtype).double().T).to(dtype).double()
+    assert broken(folded) > 0.05  # (so many outputs are more than that bound off with folded scales: 0.15 of fp16, more of bf16)
+    assert broken(got) == 0.0, broken(got)
