@@ -582,10 +582,10 @@ def dominant_linear_kernel(batch, wformat):
     if batch == 1 and wformat == "bf16":
         return "gemv_nk_kernel"
     if batch <= 16:
-        return "gemv_rs_kernel"
+        return "gemv_qd_kernel" if wformat == "int4" and batch <= 8 else "gemv_rs_kernel"
     if wformat == "bf16":
-        return "gemm_tc_kernel (tcgen05, swap-AB + stream-K)" if batch <= 128 else "gemm_tc_kernel (tcgen05)"
-    return "gemv_rs_kernel (passes of <= 16 tokens)" if batch <= 64 else "generic SIMT fallback"
+        return "gemm_tc_kernel (tcgen05)"
+    return "gemv_rs_kernel (passes of <= 16 tokens)" if batch <= 128 else "generic SIMT fallback"
 
 
 def run_prefill(args, cfg, mod, dec, dev, dt, kc, vc, rank):

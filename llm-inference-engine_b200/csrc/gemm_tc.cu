@@ -32,7 +32,7 @@ constexpr size_t kTcSmem = kRingBytes + kATileBytes + kTcExtra;  // of a CTA, at
 struct GemmTcParams {
     void *C;
     int ldc;
-    int rowsA, rowsB, K;
+    int rowsA, rowsB;
     int tilesA, tilesB, kb_total;
     int splits;    // CTAs of a cluster that share the k of one tile (then a CTA has one tile), or 1: tiles are dealt round-robin
     int bn;        // UMMA N: rows of B per tile, multiple of 16, <= 256
@@ -45,7 +45,7 @@ struct GemmTcParams {
     // rows first; tile tb multiplies gate rows [hw tb, +hw) AND up rows [I + hw tb, +hw) as one N = 2 hw tile (two TMA boxes into one
     // B stage), the epilogue reads both halves of the accumulator and writes silu(gate) * up: C [rowsA, I], rowsB = I.  0: plain GEMM.
     int swiglu_inter;
-    int swiglu_hw;  // gate (and up) columns per tile: bn = 2 * swiglu_hw (128, 112 or 96: whichever wastes least of the last wave)
+    int swiglu_hw;  // gate (and up) columns per tile: bn = 2 * swiglu_hw (a multiple of 16 up to 128)
     // Grouped GEMM (mixture of experts): every tile of a_rows rows of A (32, 64 or 128) belongs to ONE expert, tile_expert[ta]; B = the experts' weights stacked
     // [experts * rowsB, K], so tile (ta, tb) multiplies B rows [tile_expert[ta] * rowsB + tb * bn, +bn).  Only the first *n_live row
     // tiles hold rows (a device-side count): those are dealt, and no others.  NULL: plain.
@@ -817,7 +817,7 @@ static int launch_gemm_tc_impl(const void *x, const void *w, void *y, int M, int
     if (swiglu_inter) plan = plan_tiles(tiles_a, a_rows, cols, K, sms, 32, split ? plan.splits : 1);
     if (!split && pair_takes(M, cols, K, sms, plan)) return launch_gemm_pair(x, w, y, M, N, K, dtype, swiglu_inter, fin, st);
     GemmTcParams p = {};
-    p.C = y, p.K = K, p.is_bf16 = bf16 ? 1 : 0;
+    p.C = y, p.is_bf16 = bf16 ? 1 : 0;
     p.swiglu_inter = swiglu_inter;
     p.finish = fin.on, p.act = fin.on ? fin.act : -1, p.bias = fin.bias, p.scale = fin.scale;
     p.wait = wait_guard();
@@ -872,7 +872,7 @@ int launch_gemm_tc_grouped(const void *a, const void *w, void *c, int max_rows, 
     const bool bf16 = dtype == B200_BF16;
     const int sms = sm_count(), most = max_rows / tile, likely = std::max(1, most - experts / 2);
     GemmTcParams p = {};
-    p.C = c, p.ldc = N, p.K = K, p.splits = 1, p.is_bf16 = bf16 ? 1 : 0;
+    p.C = c, p.ldc = N, p.splits = 1, p.is_bf16 = bf16 ? 1 : 0;
     p.act = act, p.tile_expert = tile_expert, p.n_live = n_live, p.wait = wait_guard();
     p.kb_total = (K + kBK - 1) / kBK;
     p.rowsA = max_rows, p.rowsB = N;

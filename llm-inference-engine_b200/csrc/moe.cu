@@ -1,4 +1,4 @@
-// moe.cu -- mixture-of-experts feed-forward for ragged token batches.  (Row tiles are 64 rows for the kernels of this file, 128 for the
+// moe.cu -- mixture-of-experts feed-forward for ragged token batches.  (Row tiles are 64 rows for the kernels of this file, 32, 64 or 128 for the
 // tcgen05 grouped GEMM of gemm_tc.cu, which serves prompt-sized batches of 16-bit engines; the engine chooses per call.)
 //   route:   scores = sigmoid(router logits) (fp32); the `top` largest are chosen, their scores ARE the weights (no renormalisation);
 //            a separate sigmoid gate scales the shared expert.

@@ -43,7 +43,7 @@ private:
 
     void buildEngine() {
         if (engine) return;
-        B200_CALL(b200_workspace_ensure(0));  // split-K / stream-K partials of the prefill's tensor-core linears (library-owned)
+        B200_CALL(b200_workspace_ensure(0));  // partial sums of [K, N] weights' linears (library-owned)
         b200_decoder_config_t c = {};
         c.hidden = hidden_units, c.head_num = head_num, c.kv_head_num = kv_head_num, c.head_size = head_size;
         c.inter_size = inter_size, c.num_layers = num_layers, c.max_seq_len = max_seq_len, c.max_batch = 1;  // the reference is batch 1

@@ -124,7 +124,7 @@ def test_sparse_choices_of_decode_batches(monkeypatch, dtype, tol, u, experts, t
 @pytest.mark.parametrize("dtype,tol", [("bfloat16", 4e-2), ("float16", 6e-3)])
 @pytest.mark.parametrize("n", [511, 512, 1000, 1023])
 def test_prompts_of_one_expert_each(monkeypatch, dtype, tol, n):
-    """16-bit prompts of fewer than 1024 pairs, whose experts run on 64-row tiles: from 512 tokens on their choice and their plan run in many CTAs."""
+    """16-bit prompts of one expert each: from 512 tokens on their choice and their plan run in many CTAs (expert tiles of 128 rows)."""
     layer = ref.attention_layer(heads=2, kv_heads=1, dim=16, size=50, mlp=ref.moe(experts=5, top=1, ff=64, shared_ff=64))
     config = ref.make_config([layer], width=64, vocab=80)
     W, packed = ref.make_weights(config, seed=2)

@@ -125,10 +125,10 @@ def test_linear_dense(M, K, N, layout, dtype):
                                    (300, 4096, 1024), (1024, 1024, 776), (2048, 4096, 512), (2048, 4096, 4096), (2048, 1024, 12288),
                                    (1100, 704, 4900)])
 def test_linear_tensor_core_gemm(M, K, N, dtype):
-    """M > 4, dense 16-bit, [N,K] weights: the tcgen05 / TMEM GEMM (gemm_tc.cu) -- swap-AB + split-K up to 128 rows, 128x256 tiles
-    above -- against an fp32 matmul of the same (rounded) inputs.  Integer-valued inputs must come out exact.  The last three shapes have
-    more 256-column tiles than SMs and not a multiple of them (256, 768 and 180 tiles on 148 SMs): the launcher picks the tile width
-    (240 / 224 / ... columns) whose whole waves waste least, with ragged M / N edges."""
+    """M > 4, dense 16-bit, [N,K] weights: the decode linears up to 16 rows (gemv_qd, gemv_rs), the tcgen05 / TMEM GEMM (gemm_tc.cu) above -- against an fp32
+    matmul of the same (rounded) inputs.  Integer-valued inputs must come out exact.  The last three shapes have more 256-column tiles than
+    SMs and not a multiple of them (256, 768 and 180 tiles on 148 SMs): CTA pairs, or the width whose whole waves waste least, with ragged
+    M / N edges."""
     import torch
 
     mod = b200()
