@@ -292,6 +292,12 @@ template <typename T, typename GET> __device__ __forceinline__ void finish_tile(
     }
 }
 
+// Rows that a product multiplies: 64 where a tile has no more.  (With 128 for everybody, tokens of a small batch kept the tensor cores at work on rows of nothing until the
+// board's power limit took the clock down: a 70B-shaped layer over 21 tokens, run back to back, 342 us at 1545 MHz where 128 weights' rows by 24 tokens took 333.)
+__device__ __forceinline__ int mma_rows(const GemmTcParams &p) { return p.a_rows <= kBM / 2 ? kBM / 2 : kBM; }
+// the tile's row in a lane of an accumulator's quarter q: 32 of them each, or (64 rows) 16 in the lower half
+__device__ __forceinline__ int acc_row(const GemmTcParams &p, int q, int lane) { return p.a_rows > kBM / 2 ? q * 32 + lane : lane < 16 ? q * 16 + lane : kBM; }
+
 // what a wait that ran out leaves of those columns
 template <typename T> __device__ __forceinline__ void lose_tile(const GemmTcParams &p, int ta, int row, int tb, int c0, int c1) {
     const int i = ta * p.a_rows + row, j0 = tb * (p.swiglu_inter ? p.swiglu_hw : p.bn);
@@ -372,7 +378,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else if (warp == 1) {
         // ================================================= MMA issuer
-        const uint32_t idesc = instr_desc_f16(p.is_bf16 != 0, kBM, p.bn);
+        const uint32_t idesc = instr_desc_f16(p.is_bf16 != 0, mma_rows(p), p.bn);
         SegIter si(p);
         Seg sg;
         int s = 0, t = 0;
@@ -427,7 +433,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     for (int e = 0; e < 16; ++e) mine[(size_t)(c + e) * kBM] = __uint_as_float(r[e]);
                 }
             } else {
-                finish_tile<T>(p, sg.ta, q * 32 + lane, sg.tb, 0, p.swiglu_inter ? p.swiglu_hw : p.bn, fetch);
+                finish_tile<T>(p, sg.ta, acc_row(p, q, lane), sg.tb, 0, p.swiglu_inter ? p.swiglu_hw : p.bn, fetch);
             }
             tc_fence_before();
             __syncwarp();
@@ -448,7 +454,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (warp >= 2) {
             const int q = warp & 3, cols = (p.swiglu_inter ? p.swiglu_hw : p.bn) / p.splits;
             const uint32_t at = s_u32(smem) + (uint32_t)(q * 32 + lane) * 4;
-            finish_tile<T>(p, tile % p.tilesA, q * 32 + lane, tile / p.tilesA, rank * cols, (rank + 1) * cols, [&](int c, uint32_t (&r)[16]) {
+            finish_tile<T>(p, tile % p.tilesA, acc_row(p, q, lane), tile / p.tilesA, rank * cols, (rank + 1) * cols, [&](int c, uint32_t (&r)[16]) {
                 float v[16];
                 for (int x = 0; x < p.splits; ++x) {
                     const uint32_t from = in_cta(at + (uint32_t)c * kBM * 4, (uint32_t)x);
@@ -483,7 +489,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int cols = (p.swiglu_inter ? p.swiglu_hw : p.bn) / p.splits, c0 = blockIdx.x % p.splits * cols;
             SegIter si(p);
             Seg sg;
-            while (si.next(sg)) lose_tile<T>(p, sg.ta, (warp & 3) * 32 + lane, sg.tb, c0, c0 + cols);
+            while (si.next(sg)) lose_tile<T>(p, sg.ta, acc_row(p, warp & 3, lane), sg.tb, c0, c0 + cols);
         }
         __syncthreads();
     }

@@ -23,7 +23,7 @@ def close(got, x, w, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("M", [17, 24, 25, 64, 127, 128, 129, 200, 256, 257, 300])
+@pytest.mark.parametrize("M", [17, 24, 25, 64, 65, 127, 128, 129, 200, 256, 257, 300])  # (64 | 65: rows of a product)
 @pytest.mark.parametrize("K,N", [(64, 16), (72, 40), (2048, 2056), (1000, 4104), (4096, 1024)])
 def test_tiles(dtype, M, K, N):
     gen = torch.Generator(device=DEV).manual_seed(M * 7 + K + N)
