@@ -662,15 +662,21 @@ static int prefill_impl(b200_decoder_t *dec, void *hidden, void *k_cache, void *
     int rc = b200_cal_padding_offset(padding_offset, cum, input_len, batch, max_q_len, stream);
     if (rc != B200_OK) return rc;
     void *wdq = base + off[11];
-    // quantised weights through scratch: FP8 from where its passes cost more (7B, two layers: 70 tokens 478 us against 627 in five passes, 48 about 460 in three),
-    // INT4 where the passes end (its weights lose bits on this way)
+    // Quantised weights through scratch: FP8 from where its passes of 16 tokens cost more, INT4 where the passes end (its weights lose bits on this way).  A linear's
+    // 16-bit codes are written and read again: three passes' worth while the device's second-level cache holds most of them or rows are so long that a pass reads them
+    // slowly, five beyond.  us, four passes (60 tokens) / through codes: K = 4096, N = 12288 50 / 47, N = 4096 26 / 22, K = 11008, N = 4096 65 / 44, K = 28672, N = 8192
+    // 214 / 210; but K = 4096, N = 22016 76 / 88 (five passes 91), K = 8192, N = 10240 78 / 82, N = 57344 320 / 433 (five 390, six 470).
     const bool fp8 = c.w_format == B200_W_FP8E4M3;
-    const bool quant_gemm = c.w_format != B200_W_DENSE && c.dtype != B200_F32 && T > (fp8 ? 48 : 128);
+    auto through_16_bits = [&](int K, int N) {
+        if (c.w_format == B200_W_DENSE || c.dtype == B200_F32) return false;
+        const size_t codes = (size_t)K * N * 2;
+        return T > (!fp8 ? 128 : K > 8192 || codes <= 150000000 ? 48 : codes <= 400000000 ? 64 : 80);
+    };
     auto linear = [&](const void *x, const b200_linear_weight_t &w, void *out, int K, int N) {
         // FP8 / INT4 at prefill sizes: the linear's weights into scratch as 16-bit numbers (one vectorised pass), then the tcgen05 GEMM.  FP8 codes are exact there and
         // the rows' scales multiply the GEMM's sums; INT4 weights are rounded with their groups' scales.  Fewer tokens: the decode kernels' passes of 16 tokens over
         // the packed weights.
-        if (quant_gemm) {
+        if (through_16_bits(K, N)) {
             int r = launch_dequant_vec(w.w, fp8 ? nullptr : w.scales, w.zeros, wdq, N, K, c.w_format, c.group, c.dtype, st);
             if (r == B200_OK) r = launch_gemm_tc(x, wdq, out, T, N, K, c.dtype, st, fp8 ? (const float *)w.scales : nullptr);
             if (r != B200_ERR_UNSUPPORTED) return r;
@@ -720,7 +726,7 @@ static int prefill_impl(b200_decoder_t *dec, void *hidden, void *k_cache, void *
         if (rc != B200_OK) return rc;
         // gate_up + SwiGLU: one tensor-core GEMM whose epilogue applies the activation (16-bit, T > 16; quantised weights as above); otherwise the two launchers
         rc = B200_ERR_UNSUPPORTED;
-        if (c.dtype != B200_F32 && (c.w_format == B200_W_DENSE ? T > 16 : quant_gemm)) {
+        if (c.dtype != B200_F32 && (c.w_format == B200_W_DENSE ? T > 16 : through_16_bits(h, 2 * c.inter_size))) {
             const void *wgu = w.gate_up.w;
             if (c.w_format != B200_W_DENSE) {
                 rc = launch_dequant_vec(w.gate_up.w, fp8 ? nullptr : w.gate_up.scales, w.gate_up.zeros, wdq, 2 * c.inter_size, h, c.w_format, c.group, c.dtype, st);

@@ -101,13 +101,14 @@ def fp8_scales(n, dt, gen):
     return ((1 + u * (torch.randint(0, 64, (n,), generator=gen, device=DEV) + 0.25 + 0.25 * torch.rand(n, generator=gen, device=DEV))) * 0.03).float()
 
 
+# the large layer: QKV of 151 MB in 16 bits, which leaves the passes at 65 tokens, gate-up of 411 MB, at 81
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("T", [48, 49, 128, 129, 300])
-def test_fp8_scales_are_not_rounded(dtype, T):
+@pytest.mark.parametrize("T,size", [(T, (512, 4, 2, 768)) for T in (48, 49, 128, 129, 300)] + [(T, (8192, 64, 4, 12544)) for T in (64, 65, 80, 81)])
+def test_fp8_scales_are_not_rounded(dtype, T, size):
     """The value rows that a prompt leaves in the cache are one FP8 linear's outputs.  Its inputs are made +-1 (a norm of +-1 rows), so that the codes' sums are exact
     in fp32 and the only roundings are the product's with the scale and the result's: half a unit of the type and 2^-23.  Scales folded into rounded 16-bit weights
-    break that bound."""
-    h, heads, kv, inter, d = 512, 4, 2, 768, 128
+    break that bound.  The whole layer agrees with the same prompt sixteen tokens at a time."""
+    (h, heads, kv, inter), d = size, 128
     gen = torch.Generator(device=DEV).manual_seed(T)
     code = m.BF16 if dtype == torch.bfloat16 else m.F16
     dec = m.Decoder(m.DecoderConfig(h, heads, kv, d, inter, 1, 320, 1, code, m.W_FP8, 128, 1e-6, d, 10000.0, 1, 0), DEV)
@@ -116,9 +117,15 @@ def test_fp8_scales_are_not_rounded(dtype, T):
         layer[name] = (torch.randn(n, k, generator=gen, device=DEV).to(torch.float8_e4m3fn).view(torch.uint8), fp8_scales(n, dtype, gen), None)
     dec.set_layer(0, layer)
     x = torch.randint(0, 2, (T, h), generator=gen, device=DEV).to(dtype) * 2 - 1
-    k, v = (torch.zeros(1, 5, kv, 64, d, device=DEV, dtype=dtype) for _ in range(2))
+    k, v, k2, v2 = (torch.zeros(1, 5, kv, 64, d, device=DEV, dtype=dtype) for _ in range(4))
     i32 = lambda *a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
-    dec.prefill_paged(x.clone(), k, v, torch.arange(5, dtype=torch.int32, device=DEV).reshape(1, 5), i32(T), i32(0), i32(T), T)
+    table = torch.arange(5, dtype=torch.int32, device=DEV).reshape(1, 5)
+    whole, parts = x.clone(), x.clone()
+    dec.prefill_paged(whole, k, v, table, i32(T), i32(0), i32(T), T)
+    for a in range(0, T, 16):
+        n = min(16, T - a)
+        dec.prefill_paged(parts[a:a + n], k2, v2, table, i32(n), i32(a), i32(a + n), n)
+    assert (whole.double() - parts.double()).norm() <= 4 * torch.finfo(dtype).eps * parts.double().norm()
     got = v[0].permute(0, 2, 1, 3).reshape(-1, kv * d)[:T].double()
     codes, scales, _ = layer["qkv"]
     codes, scales = codes[(heads + kv) * d:].view(torch.float8_e4m3fn).double(), scales[(heads + kv) * d:].double()
