@@ -44,7 +44,8 @@ __host__ __device__ inline int first_key(int pos, int window, int chunk) {
 // Keys of a block: of the token's own number of keys and of nothing else.  128 are what the lanes take in one round.
 __host__ __device__ inline int block_keys(int nkeys) {
     if (nkeys <= kBlocks * kBlock) return kBlock;
-    const int blocks = nkeys > kBlocks * kMostKeys ? (nkeys + kMostKeys - 1) / kMostKeys : kBlocks;
+    int blocks = nkeys > kBlocks * kMostKeys ? (nkeys + kMostKeys - 1) / kMostKeys : kBlocks;
+    if (blocks > kMostBlocks) blocks = kMostBlocks;
     return ((nkeys + blocks - 1) / blocks + 7) & ~7;
 }
 
@@ -382,7 +383,7 @@ int launch_token_attention(int dtype, const TokenAttn &a, int tokens, cudaStream
     };
     int longest = 1;
     for (int i = 0; i < tokens; ++i) longest = std::max(longest, keys_of(i));
-    if (rows > 65535 || blocks_of(longest) > kMostBlocks || smem_of(std::max(block_keys(longest), kBlock), longest) > 110 * 1024) return B200_ERR_UNSUPPORTED;
+    if (rows > 65535 || smem_of(std::max(block_keys(longest), kBlock), longest) > 110 * 1024) return B200_ERR_UNSUPPORTED;
     for (int i0 = 0, i1; i0 < tokens; i0 = i1) {
         long long all = 0;
         int per = kBlock, most = 1, keys = 1, run = 1;

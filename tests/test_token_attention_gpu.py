@@ -106,3 +106,30 @@ def test_a_token_by_itself(design, heads, kv, dim, size, contexts):
     for k in range(3):
         same = (rows["alone", k] == rows["together", k]).all(dim=-1)
         assert same.all(), [contexts[i] for i in range(len(contexts)) if not same[i]]
+
+
+@pytest.mark.parametrize("heads,kv", [(1, 1), (8, 1)])
+def test_long_contexts(heads, kv):
+    """Contexts beyond the sizes at which blocks of keys change their number and their length (4096, 32768 and 131072 keys): the last tokens of a prompt decoded one by
+    one against the same tokens as a portion of eight, which the prompt kernel takes.  Both round their rows to 16 bits."""
+    config = vasolix_oracle.make_config([vasolix_oracle.attention_layer(heads=heads, kv_heads=kv, dim=64, size=1 << 20, scale=0.125)], width=64)
+    _, packed = vasolix_oracle.make_weights(config, seed=3)
+    model = importlib.import_module("llm-inference-engine_b200.models.vasolix").VasolixModel(config, packed, dtype="float16", device="cuda:0", max_tokens=4096, max_seqs=1,
+                                                                                              max_pages_per_seq=2200)
+    serving = importlib.import_module("llm-inference-engine_b200.serving")
+    toks = np.random.default_rng(0).integers(0, config["vocab"], 140000).tolist()
+    rows = {}
+    for how in ("portions", "decoded"):
+        sess = serving.Session(model, len(toks) + 64, max_seqs=1, max_batch_tokens=4096, poison=True)
+        i, at = sess.open(), 0
+        for stop in (5000, 33000, 140000):
+            while at < stop - 8:
+                n = min(4096, stop - 8 - at)
+                sess.feed([(i, toks[at:at + n], [])])
+                at += n
+            part = toks[at:stop]
+            rows[how, stop] = sess.feed([(i, part, list(range(8)))]) if how == "portions" else torch.cat([sess.feed([(i, [x], [0])]) for x in part])
+            at = stop
+    for stop in (5000, 33000, 140000):
+        a, b = rows["portions", stop].double(), rows["decoded", stop].double()
+        assert not torch.isnan(b).any() and ((a - b).norm(dim=-1) / a.norm(dim=-1)).max() < TOL["float16"], stop
