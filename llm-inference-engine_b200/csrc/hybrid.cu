@@ -1437,7 +1437,7 @@ int b200_hybrid_forward(b200_hybrid_t *m, const b200_hybrid_batch_t *b, float *l
         mid_portions |= t1 - t0 > 1 && t1 - t0 < kChunkMinTokens;
         if (t1 - t0 >= kChunkMinTokens) long_tokens += t1 - t0;
         gla_kinds |= t1 - t0 == 1 ? kGlaOneToken : (t1 - t0 > 1 ? kGlaManyTokens : 0);
-        B200_REQUIRE(t1 >= t0 && b->seq_pos0[s] >= 0, "hybrid_forward: bad portion of sequence %d", s);
+        B200_REQUIRE(t1 >= t0 && t1 <= NT && b->seq_pos0[s] >= 0, "hybrid_forward: bad portion of sequence %d", s);
         B200_REQUIRE(b->seq_slot[s] >= 0 && b->seq_slot[s] < m->num_slots, "hybrid_forward: state slot %d outside [0, %d)", b->seq_slot[s], m->num_slots);
         for (int s2 = 0; s2 < s; ++s2) B200_REQUIRE(b->seq_slot[s2] != b->seq_slot[s], "hybrid_forward: state slot %d given to two sequences", b->seq_slot[s]);
         const int last = b->seq_pos0[s] + (t1 - t0) - 1;

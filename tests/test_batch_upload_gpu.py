@@ -36,3 +36,18 @@ def test_a_prompt_uploads_no_list_of_decoded_tokens(tmp_path):
     ints = lambda n, listed: 5 * n + 4 * (n // 64 + 2) + 4 + pages + 2 * layers + listed * (4 + heads)  # noqa: E731
     assert prompt == 4 * ints(tokens, 0), (prompt, ints(tokens, 0) * 4)
     assert decode == 4 * ints(1, 1), (decode, ints(1, 1) * 4)
+
+
+@pytest.mark.parametrize("starts", [[0, 9, 4], [0, 400, 4], [0, 2, 9, 4], [0, 3, 2, 4]])
+def test_portions_outside_the_batch_are_refused(starts):
+    """Starts that pass the number of tokens and come back, or that fall: refused before anything is written for them."""
+    config = ref.make_config([ref.attention_layer(heads=2, kv_heads=1, dim=64, size=100, scale=0.125)], width=64)
+    _, packed = ref.make_weights(config, seed=2)
+    model = importlib.import_module("llm-inference-engine_b200.models.vasolix").VasolixModel(config, packed, dtype="bfloat16", device="cuda:0", max_tokens=16, max_seqs=4,
+                                                                                              max_pages_per_seq=8)
+    engine, seqs = model.engine, len(starts) - 1
+    engine.set_pools(8 * seqs, seqs)
+    call = lambda st: engine.forward([1, 2, 3, 4], st, [0] * seqs, range(seqs), np.arange(8 * seqs), [3])  # noqa: E731
+    with pytest.raises(importlib.import_module("llm-inference-engine_b200").B200Error, match="bad portion"):
+        call(starts)
+    assert torch.isfinite(call([0] * seqs + [4])).all()
