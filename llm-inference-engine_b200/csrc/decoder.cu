@@ -583,8 +583,10 @@ int b200_decoder_linears_only(b200_decoder_t *dec, int batch, int *n_launches, b
         if (rc != B200_OK) return rc;
         dec->cur = next_res(dec->cur);
         if ((rc = plain_linear(dec, dec->act, w.down, c.inter_size, c.hidden, dec->y_ffn, batch, st)) != B200_OK) return rc;
-        // 4 linears; for 2+ tokens of a 16-bit model (5+ in fp32) each of the two prologues is its own small kernel (norm_linear)
-        launches += (batch == 1 || ((c.dtype == B200_F32 || c.w_format != B200_W_DENSE) && batch <= 4)) ? 4 : 6;
+        // 4 linears in their passes; each of the two prologues is a kernel but for one dense or INT4 token and up to 4 in fp32 (norm_linear), the activation beyond one pass
+        const bool f32 = c.dtype == B200_F32;
+        const int rows = f32 ? 4 : 16, passes = f32 && batch > 16 ? 1 : f32 || c.w_format != B200_W_DENSE ? (batch + rows - 1) / rows : 1;
+        launches += 4 * passes + (f32 ? batch > 4 : batch > 1 || c.w_format == B200_W_FP8E4M3) * 2 + (batch > rows);
     }
     if (n_launches) *n_launches = launches;
     return B200_OK;
