@@ -1,5 +1,6 @@
-"""b200_decoder_linears_only says how many kernels it launched (include/b200llm.h): counted by the profiler for every weight format on both sides of the sizes at which
+"""b200_decoder_linears_only says how many kernels it launched (include/b200llm.h): counted in a captured graph for every weight format on both sides of the sizes at which
 a norm leaves its linear and a linear goes in passes."""
+import ctypes
 import importlib
 
 import pytest
@@ -33,8 +34,9 @@ def test_the_number_of_launches(fmt, batch):
     k, v = (torch.zeros(layers, batch, heads, 64, d, device=DEV, dtype=dtype) for _ in range(2))
     dec.step(torch.randn(batch, h, generator=gen, device=DEV).to(dtype), k, v, 1)
     torch.cuda.synchronize()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
         said = dec.linears_only(batch)
-        torch.cuda.synchronize()
-    names = [e.name for e in p.events() if "b200::" in e.name]
-    assert said == len(names), (said, names)
+    nodes = ctypes.c_size_t(0)  # (kernels are all that it launches)
+    assert ctypes.CDLL("libcuda.so.1").cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(nodes)) == 0
+    assert said == nodes.value
