@@ -93,8 +93,8 @@ token_attn_kernel(const TokenAttnArgs args) {
     if (b0 >= b1) return;  // (fewer blocks than another token has)
     const int run0 = b0 * per, run1 = min(b1 * per, nkeys);  // this CTA's keys, counted from the first
 
-    float *const qs = sm, *const sc = qs + G * dim, *const part = sc + (size_t)args.block_max * G, *const red = part + kWarpsT * G * vdim;  // maxima and sums [2][warps][G]
-    float *const whole = red + 2 * kWarpsT * G;                               // [G]: the factors of the result
+    float *const qs = sm, *const sc = qs + G * dim, *const part = sc + (size_t)args.block_max * G, *const red = part + kWarpsT * G * vdim;  // sums of weights and the maxima of every other block [3][warps][G]
+    float *const whole = red + 3 * kWarpsT * G;                               // [G]: the factors of the result
     int *const pages = reinterpret_cast<int *>(whole + G);
     __shared__ int last_one;
     const int page0 = (first + run0) / kPageT;
@@ -136,16 +136,17 @@ token_attn_kernel(const TokenAttnArgs args) {
         for (int w = 0; w < kWarpsT; ++w) v += part[(size_t)w * G * vdim + i];
         return v;
     };
-    auto largest = [&](int h) {
+    auto maxima = [&](int b) { return red + (1 + (b & 1)) * kWarpsT * G; };  // (a warp may form the next block's while another still folds this one's)
+    auto largest = [&](int b, int h) {
         float m = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < kWarpsT; ++w) m = fmaxf(m, red[w * G + h]);
+        for (int w = 0; w < kWarpsT; ++w) m = fmaxf(m, maxima(b)[w * G + h]);
         return m;
     };
     auto total = [&](int h) {
         float l = 0.0f;
 #pragma unroll
-        for (int w = 0; w < kWarpsT; ++w) l += red[(kWarpsT + w) * G + h];
+        for (int w = 0; w < kWarpsT; ++w) l += red[w * G + h];
         return l;
     };
     const int item = blockIdx.x * gridDim.y + blockIdx.y, stride = G * (vdim + 2);
@@ -218,10 +219,10 @@ token_attn_kernel(const TokenAttnArgs args) {
             for (int h = 0; h < HQ; ++h) {
 #pragma unroll
                 for (int x = G >= 2 ? 2 : 1; x < 32; x <<= 1) mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], x));
-                if (lane < (G >= 2 ? 2 : 1)) red[warp * G + hq + h] = mx[h];
+                if (lane < (G >= 2 ? 2 : 1)) maxima(b)[warp * G + hq + h] = mx[h];
             }
             __syncthreads();
-            const float m = largest(tid % G), top = m == -INFINITY ? 0.0f : m;  // (a block whose scores are all minus infinity has weights of zero, another may not)
+            const float m = largest(b, tid % G), top = m == -INFINITY ? 0.0f : m;  // (a block whose scores are all minus infinity has weights of zero, another may not)
             float sum = 0.0f;  // of head tid % G
             for (int i = tid; i < n * G; i += kThreads) {
                 const float e = expf(sc[i] - top);
@@ -230,7 +231,7 @@ token_attn_kernel(const TokenAttnArgs args) {
             }
 #pragma unroll
             for (int x = G; x < 32; x <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
-            if (lane < G) red[(kWarpsT + warp) * G + lane] = sum;
+            if (lane < G) red[warp * G + lane] = sum;
         }
         __syncthreads();
 
@@ -282,13 +283,13 @@ token_attn_kernel(const TokenAttnArgs args) {
                 if (a.sigmoid) {
                     out[e] += p;
                 } else {
-                    const Fold f(out_m[e], largest(i >> vshift));
+                    const Fold f(out_m[e], largest(b, i >> vshift));
                     out[e] = fold(out[e], f.of_old, p, f.of_new), out_l[e] = fold(out_l[e], f.of_old, total(i >> vshift), f.of_new), out_m[e] = f.top;
                 }
             }
         } else {
             float *const mine = all + (size_t)b * stride;
-            if (!a.sigmoid && tid < G) __stcg(mine + tid, largest(tid)), __stcg(mine + G + tid, total(tid));
+            if (!a.sigmoid && tid < G) __stcg(mine + tid, largest(b, tid)), __stcg(mine + G + tid, total(tid));
             for (int i = tid; i < G * vdim; i += kThreads) __stcg(mine + 2 * G + i, folded(i));
         }
     }
@@ -379,7 +380,7 @@ int launch_token_attention(int dtype, const TokenAttn &a, int tokens, cudaStream
     auto keys_of = [&](int i) { return a.listed[i].w - first_key(a.listed[i].w, a.window, a.chunk) + 1; };
     auto blocks_of = [&](int keys) { return (keys + block_keys(keys) - 1) / block_keys(keys); };
     auto smem_of = [&](int per, int run) {
-        return ((size_t)G * a.dim + (size_t)per * G + (size_t)kWarpsT * G * a.vdim + 2 * kWarpsT * G + G) * sizeof(float) + (run / kPageT + 2) * sizeof(int);
+        return ((size_t)G * a.dim + (size_t)per * G + (size_t)kWarpsT * G * a.vdim + 3 * kWarpsT * G + G) * sizeof(float) + (run / kPageT + 2) * sizeof(int);
     };
     int longest = 1;
     for (int i = 0; i < tokens; ++i) longest = std::max(longest, keys_of(i));

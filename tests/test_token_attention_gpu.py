@@ -133,3 +133,27 @@ def test_long_contexts(heads, kv):
     for stop in (5000, 33000, 140000):
         a, b = rows["portions", stop].double(), rows["decoded", stop].double()
         assert not torch.isnan(b).any() and ((a - b).norm(dim=-1) / a.norm(dim=-1)).max() < TOL["float16"], stop
+
+
+@pytest.mark.parametrize("each", [1, 7])
+def test_the_same_every_time(each):
+    """Forty sequences of a dozen blocks of keys, shared out over two CTAs a token and key head (one token each) or all of them in one CTA (seven): a step repeated from
+    the same state gives every bit again, whatever the order in which warps and CTAs come to their sums."""
+    config = vasolix_oracle.make_config([vasolix_oracle.attention_layer(heads=16, kv_heads=4, dim=128, size=4096, scale=128 ** -0.5)], width=128)
+    _, packed = vasolix_oracle.make_weights(config, seed=4)
+    seqs, pages = 40, 25
+    model = importlib.import_module("llm-inference-engine_b200.models.vasolix").VasolixModel(config, packed, dtype="float16", device="cuda:0", max_tokens=2048, max_seqs=seqs,
+                                                                                              max_pages_per_seq=pages)
+    engine = model.engine
+    engine.set_pools(seqs * pages, seqs)
+    rng = np.random.default_rng(each)
+    table = np.arange(seqs * pages).reshape(seqs, pages)
+    lens = [1400 + 4 * i for i in range(seqs)]
+    for i, n in enumerate(lens):
+        engine.forward(rng.integers(0, config["vocab"], n), [0, n], [0], [i], table[i], [])
+    ids, starts, rows = rng.integers(0, config["vocab"], seqs * each), [each * i for i in range(seqs + 1)], range(seqs * each)
+    step = lambda: engine.forward(ids, starts, lens, range(seqs), table.reshape(-1), rows)  # noqa: E731
+    want = step()
+    assert not torch.isnan(want).any()
+    for _ in range(150):
+        assert torch.equal(step(), want)
